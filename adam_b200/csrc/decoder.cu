@@ -76,7 +76,7 @@ struct Decoder {
 constexpr uint32_t MAX_DECODERS = 8;
 constexpr uint32_t ATTN_SPLIT = 64;        // fewest tokens an attention CTA takes before another CTA is added
 constexpr uint32_t ATTN_MAX_SPLITS = 64;   // attention CTAs per (sequence, kv head)
-constexpr uint32_t PREFILL_ROWS = 64;      // rows (sequences x tokens) of one prefill chunk
+constexpr uint32_t PREFILL_ROWS = 1024;    // rows (sequences x tokens) of one prefill chunk
 static Decoder* g_dec[MAX_DECODERS];
 
 static Decoder* get_dec(uint32_t id) {
@@ -1218,10 +1218,13 @@ extern "C" int adam_b200_decoder_create(const adam_b200_decoder_desc* desc, uint
     D->page_elems = (size_t)d.n_layer * 2 * d.n_head_kv * d.page_size * d.head_dim;
     D->n_splits = (d.kv_cap + ATTN_SPLIT - 1) / ATTN_SPLIT;      // ATTN_SPLIT = ATTN_CP * ATTN_CHUNKS_PER_CTA
     if (D->n_splits > ATTN_MAX_SPLITS) D->n_splits = ATTN_MAX_SPLITS;
-    D->rows_cap = d.max_batch > PREFILL_ROWS ? d.max_batch : PREFILL_ROWS;
-    gemm_tc_prepare();                          // workspace of the many-row GEMM (without it those rows run on the GEMV kernels)
+    const uint64_t most = (uint64_t)d.max_batch * d.kv_cap;     // no more prompt rows than that exist
+    D->rows_cap = (uint32_t)(most < PREFILL_ROWS ? (most > 64 ? most : 64) : PREFILL_ROWS);
+    if (D->rows_cap < d.max_batch) D->rows_cap = d.max_batch;
     const size_t B = d.max_batch, R = D->rows_cap, E = d.n_embd, q_dim = (size_t)d.n_head * d.head_dim, k_dim = (size_t)d.n_head_kv * d.head_dim;
     const uint32_t gs = d.n_head / d.n_head_kv;
+    // workspace of the many-row GEMM (without it those rows run on the GEMV kernels)
+    gemm_tc_prepare((int)D->rows_cap, (int)(d.n_ff > E ? (d.n_ff > q_dim ? d.n_ff : q_dim) : (E > q_dim ? E : q_dim)));
     g_dec[id] = D;
 #define DALLOC(p, bytes) do { cudaError_t e__ = cudaMalloc((void**)&(p), (bytes)); if (e__ != cudaSuccess) { destroy(D); g_dec[id] = nullptr; \
         return fail(ADAMAH_ERR_MEMORY, "decoder_create: cudaMalloc(%zu) failed: %s", (size_t)(bytes), cudaGetErrorString(e__)); } } while (0)

@@ -1,251 +1,215 @@
-// Dequant-fused GEMM  y[b][n] = sum_k W[n][k] x[b][k]  for 9..64 activation rows b (a prefill chunk
-// or a large decode batch) on the 5th-generation tensor cores: tcgen05.mma with the accumulator in
-// tensor memory (TMEM).  Same operator as the GEMV kernels (the reference's Q4 mat-vec shader
-// adamah-MAIN/adamah/shaders/src/f32/map_matvec_t_xq4.comp and map_fused_gateup_t_xq4.comp run once
-// per row by adamah.c:8606-8691).  Arithmetic: a row's activations become integers of up to 23 bits
-// with one power-of-two scale per row, split into two signed parts that fp16 holds exactly
-// (x = 2048 x_hi + x_lo); a weight is dequantised in fp32 (block scale and offset applied) and split
-// into two fp16 terms (22 bits); the three significant cross products are accumulated over all of K in
-// fp32 in TMEM and combined once per output.  Measured error ~5e-7 of max |y| (operator tolerance 1e-3).
+// Dequant-fused GEMM  y[b][n] = sum_k W[n][k] x[b][k]  for many activation rows b (prompt rows, decode batches) on the
+// 5th-generation tensor cores: tcgen05.mma with the weight operand and the accumulator in tensor memory (TMEM).  Same
+// operator as the GEMV kernels (the reference's Q4 mat-vec shader adamah-MAIN/adamah/shaders/src/f32/map_matvec_t_xq4.comp
+// and map_fused_gateup_t_xq4.comp run once per row by adamah.c:8606-8691).
+//
+// Arithmetic.  A row of activations is scaled by a power of two (largest element near 2^15) and split into two fp16
+// terms, x = x_hi + x_lo (22 bits of every element).  A weight is rebuilt exactly as two fp16 terms, w = w_hi + w_lo:
+//   Q4_0  w = d (q - 8): w_hi = RN16(d (q - 8)), w_lo = fma(d, q - 8, -w_hi), exact because d (q - 8) has 14 bits
+//   Q4_K  w = d (sc q) - dmin m: the first product has 21 bits and splits the same way; the second is the same for 32
+//         neighbouring weights, so it becomes one more "weight" per 32 that multiplies the sum of their 32 activations
+//         (a few extra steps of K, 1/32 of the work)
+// and w_hi x_hi + w_lo x_hi + w_hi x_lo is accumulated over K in fp32 (w_lo x_lo lies below 2^-22 of the product).
+// Limit: |w| < 65504, what fp16 holds.
 //
 // Two kernels:
-//   k_quant_rows   one CTA per activation row: the optional input chain (residual add + RMS norms,
-//                  as the GEMV prologue; the row stays in registers and all loads are issued before
-//                  the first use), the row's scale, and the row's two fp16 planes written straight
-//                  into the B-operand image in global memory: K-major with the 128-byte swizzle,
-//                  two 32-wide K blocks per 128-byte operand row, 128 operand rows (row n = plane *
-//                  64 + activation row) = 16 KB per block pair (behind each chunk of two pairs the
-//                  4 x 64 per-row integer sums are kept as floats for callers that want them).
-//   k_gemm_tc      256 threads, two CTAs per SM (256 TMEM columns and 97 KB of shared memory each), a
-//                  grid that fills the GPU twice over and takes work items (tile of 128 weight rows
-//                  x K split) round-robin; see the comment at the kernel.  K splits leave partial
-//                  sums in a workspace; the last CTA of a tile (atomic ticket) adds them in split
-//                  order and runs the epilogue (store, or GeGLU / SwiGLU over a tile of 64 gate
-//                  rows + 64 up rows).
-// Every wait (bulk copy, tensor-core completion) is bounded: when one runs out the kernel records
-// DEVERR_WAIT, stops waiting, and still frees its tensor memory.  The shared-memory request keeps a
-// third CTA off an SM, so a TMEM allocation never waits on a CTA that cannot run.
+//   k_quant_rows  one CTA per activation row: the optional input chain (residual add + RMS norms, as the GEMV prologue),
+//                 the row's scale, and its two fp16 planes written in the B operand's shared-memory order (K-major,
+//                 128-byte swizzle), so that the GEMM fetches operand tiles with plain bulk copies.
+//   k_gemm_tc     see there.
+// Every wait is bounded: when one runs out the kernel records DEVERR_WAIT, stops waiting, and still frees its tensor memory.
 #include "gemm_tc.cuh"
 #include "gemv_mma.cuh"
 
+#include <cmath>
 #include <cstdlib>
+#include <vector>
 
 namespace ab {
 
-constexpr int TC_PLANES = 2;
-constexpr int TC_N = TC_PLANES * TC_COLS;                // 128 B-operand rows
-constexpr int TC_CH = 4;                                 // K blocks per chunk of the B image (two pair images + the sums)
-// Operand images, K-major with the 128-byte swizzle: a "pair" image holds two K blocks (64 fp16 = 128
-// bytes per operand row) of 128 operand rows = 16 KB: 8-row groups of 1024 bytes, a row's 128 bytes
-// contiguous, and the 16-byte piece c of row r stored at piece c ^ (r & 7).  Images start at
-// multiples of 1024 bytes (the swizzle works on address bits).
-constexpr int TC_PAIR_IMG = 128 * 128;                   // 16384
-constexpr int TC_A_CHUNK = (TC_CH / 2) * TC_PAIR_IMG;    // 32768
-constexpr int TC_B_SUMS = TC_A_CHUNK;                    // offset of the chunk's [4][64] row sums in the B chunk image
-constexpr int TC_B_CHUNK = TC_A_CHUNK + TC_CH * TC_COLS * 4;        // 33792 = 33 * 1024
-constexpr int TC_TMEM_COLS = 256;
-constexpr int TC_THREADS = 256;                         // two warps per TMEM lane quarter: each takes 32 of the 64 columns
-constexpr int TC_MYCOLS = TC_COLS / 2;
+// ---- workspace: the operand image of the activations and the rows' inverse scales -----------------------------
+constexpr int TC_GROUP = 64;                            // rows of one image group
+constexpr int TC_STEP_IMG = TC_GROUP * 128;             // one plane of one group and step (64 values of K): 8 KB
+constexpr size_t TC_IMG_MAX = 256u << 20;               // largest image kept; longer calls run in row chunks
 constexpr int TC_MAX_K = 32768;
-constexpr int TC_MAX_CTAS = 1536;                        // workspace: 32 KB of partial sums per CTA
-constexpr int TC_MAX_TILES = 4096;
 
-struct TcWork { uint8_t* bimg; float* inv; float* part; unsigned int* tickets; bool ok; };
+struct TcWork { uint8_t* img; size_t img_cap; float* inv; int inv_cap; std::vector<void*> retired; };
 static TcWork g_tc = {};
 static uint64_t g_tc_calls = 0;
 static int g_tc_policy = -1;             // 0 never, 1 where it is expected to be faster, 2 whenever the shape allows; -1 = take it from ADAM_B200_TC
 
-bool gemm_tc_prepare() {
-    if (g_tc.ok) return true;
-    const size_t bimg_bytes = (size_t)(TC_MAX_K / 32 / TC_CH) * TC_B_CHUNK;
-    if (cudaMalloc(&g_tc.bimg, bimg_bytes) != cudaSuccess || cudaMalloc(&g_tc.inv, TC_COLS * 4) != cudaSuccess ||
-        cudaMalloc(&g_tc.part, (size_t)TC_MAX_CTAS * TC_COLS * 128 * 4) != cudaSuccess ||
-        cudaMalloc(&g_tc.tickets, TC_MAX_TILES * 4) != cudaSuccess) {
-        cudaGetLastError();
-        gemm_tc_release();
-        return false;
+static int tc_main_steps(int K) { return (K + 63) / 64; }
+static int tc_min_steps(int wtype, int K) { return wtype == WT_Q4_K ? (K / 32 + 63) / 64 : 0; }
+static size_t tc_group_bytes(int wtype, int K) { return (size_t)(tc_main_steps(K) + tc_min_steps(wtype, K)) * 2 * TC_STEP_IMG; }
+static int tc_pad_rows(int rows) { return (rows + 127) / 128 * 128; }
+
+// Room for `rows` activation rows of length K (either block type); false when out of memory.  Recorded graphs hold the
+// buffers' addresses, so a buffer that is outgrown stays until the release; sizes at least double, which bounds the sum.
+bool gemm_tc_prepare(int rows, int K) {
+    if (rows < 1 || K < 1 || K > TC_MAX_K) return false;
+    const int pad = tc_pad_rows(rows);
+    size_t need = (size_t)(pad / TC_GROUP) * tc_group_bytes(WT_Q4_K, K);
+    if (need > TC_IMG_MAX) need = TC_IMG_MAX;
+    auto grow = [&](void** p, size_t bytes) {
+        void* q = nullptr;
+        if (cudaMalloc(&q, bytes) != cudaSuccess) { cudaGetLastError(); return false; }
+        cudaMemsetAsync(q, 0, bytes, g.stream);
+        if (*p) g_tc.retired.push_back(*p);
+        *p = q;
+        return true;
+    };
+    if (need > g_tc.img_cap) {
+        size_t cap = need > 2 * g_tc.img_cap ? need : 2 * g_tc.img_cap;
+        if (cap > TC_IMG_MAX) cap = TC_IMG_MAX;
+        if (!grow((void**)&g_tc.img, cap)) return false;
+        g_tc.img_cap = cap;
     }
-    cudaMemset(g_tc.tickets, 0, TC_MAX_TILES * 4);
-    cudaMemset(g_tc.bimg, 0, bimg_bytes);
-    g_tc.ok = true;
+    if (pad > g_tc.inv_cap) {
+        const int cap = pad > 2 * g_tc.inv_cap ? pad : 2 * g_tc.inv_cap;
+        if (!grow((void**)&g_tc.inv, (size_t)cap * 4)) return false;
+        g_tc.inv_cap = cap;
+    }
     return true;
 }
 
 void gemm_tc_release() {
-    cudaFree(g_tc.bimg); cudaFree(g_tc.inv); cudaFree(g_tc.part); cudaFree(g_tc.tickets);
+    cudaFree(g_tc.img); cudaFree(g_tc.inv);
+    for (void* p : g_tc.retired) cudaFree(p);
     g_tc = TcWork{};
 }
-
-// Byte offset of (operand row n, byte kb of the row's 128) in a pair image.
-__device__ __forceinline__ int swz_off(int n, int kb) { return (n >> 3) * 1024 + (n & 7) * 128 + ((((kb >> 4) ^ n) & 7) << 4) + (kb & 15); }
-// Byte offset in the B image of the 4 values k0 .. k0+3 (k0 a multiple of 4) of operand row n, and of block kb's row sums.
-__device__ __forceinline__ size_t bimg_off(int n, int k0) {
-    const int kb = k0 >> 5;
-    return (size_t)(kb >> 2) * TC_B_CHUNK + ((kb >> 1) & 1) * TC_PAIR_IMG + swz_off(n, (kb & 1) * 64 + (k0 & 31) * 2);
-}
-__device__ __forceinline__ size_t bsum_off(int kb) { return (size_t)(kb >> 2) * TC_B_CHUNK + TC_B_SUMS + (kb & 3) * (TC_COLS * 4); }
-
-// ---- activations: chain, scale, two fp16 planes in B-operand order -------------------------------
-// Four consecutive activations (k = 4i .. 4i+3) of column `col`, already scaled: round to integers,
-// split into the two planes, store them, and leave the block's integer sum behind the block's image.
-// Called by all threads of a warp together (the eight threads of one 32-wide block are eight
-// neighbouring lanes); threads with on == false only take part in the shuffles.
-__device__ __forceinline__ void put_planes(uint8_t* __restrict__ bimg, int col, int i, bool on, float4 v, float s) {
-    const float f[4] = {v.x * s, v.y * s, v.z * s, v.w * s};
-    __align__(8) __half hi[4], lo[4];
-    int sum = 0;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const int xi = on ? __float2int_rn(f[e]) : 0;       // |xi| <= 2^22
-        const int l = ((xi + 1024) & 2047) - 1024;          // [-1024, 1023]
-        const int h = (xi - l) >> 11;                       // [-2048, 2048]: exact in fp16
-        hi[e] = __int2half_rn(h); lo[e] = __int2half_rn(l);
-        sum += xi;
-    }
-    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-    if (on) {
-        const int k0 = 4 * i;
-        *reinterpret_cast<uint2*>(bimg + bimg_off(col, k0)) = *reinterpret_cast<const uint2*>(hi);
-        *reinterpret_cast<uint2*>(bimg + bimg_off(TC_COLS + col, k0)) = *reinterpret_cast<const uint2*>(lo);
-        if ((k0 & 31) == 0) reinterpret_cast<float*>(bimg + bsum_off(k0 >> 5))[col] = (float)sum;
-    }
+static int tc_rows_fit(int wtype, int K) {              // rows of one pass: whole 128-row tiles
+    const long long fit = (long long)(g_tc.img_cap / (2 * tc_group_bytes(wtype, K))) * 128;
+    return (int)(fit < g_tc.inv_cap ? fit : g_tc.inv_cap / 128 * 128);
 }
 
-constexpr int QR_THREADS = 512;
-constexpr int QR_MAXV = 4;             // float4 per thread held in registers: rows of up to 8192 values
+// ---- activations: chain, scale, two fp16 planes in B-operand order -------------------------------------------
+// Bound by the latency of its chain (one row per CTA: load, up to three reductions, store), not by its 12 bytes per
+// value; the row stays in registers (MAXV float4 per thread) and all loads are issued before the first use.
+// Four consecutive values of K are stored in the order 0, 2, 1, 3: the order in which a word of nibbles is taken apart
+// two at a time (see k_gemm_tc); K order is free as long as both operands agree.
+__device__ __forceinline__ uint32_t swz_off(int r, int kb) { return (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((((kb >> 4) ^ r) & 7) << 4) + (kb & 15)); }
 
-__global__ void __launch_bounds__(QR_THREADS) k_quant_rows(const GemvArgs a, uint8_t* __restrict__ bimg, float* __restrict__ inv_out) {
-    extern __shared__ float xs[];                       // the row, K floats
+__device__ __forceinline__ void split_half(float v, __half& hi, __half& lo) {
+    hi = __float2half_rn(v);
+    lo = __float2half_rn(v - __half2float(hi));
+}
+
+template <int MAXV, bool CHAIN>
+__global__ void __launch_bounds__(512) k_quant_rows(const GemvArgs a, uint8_t* __restrict__ img, float* __restrict__ inv_out, int n_min, int n_steps) {
     __shared__ float red[66];
-    const int col = blockIdx.x, tid = threadIdx.x, K = a.K, n4 = K >> 2;
+    const int r = blockIdx.x, tid = threadIdx.x, K = a.K, n4 = K >> 2, nt = blockDim.x;
+    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f), o4 = make_float4(1.f, 1.f, 1.f, 1.f);
+    const bool post = CHAIN && a.add_src && a.w_post, pre = CHAIN && a.w_pre;
+    float4 v[MAXV];
     pdl_launch_dependents();
     pdl_wait();
-    if (col >= a.B) {                                   // unused columns multiply as zeros
-        for (int i = tid; i < n4; i += blockDim.x) {
-            const int k0 = 4 * i;
+    const size_t row = (size_t)r * a.ldx;
+    if constexpr (CHAIN) {
+        const float* ap = a.add_src ? a.add_src + row : nullptr;
+        float4 va[MAXV], vp[MAXV], vw[MAXV];
 #pragma unroll
-            for (int p = 0; p < TC_PLANES; ++p) *reinterpret_cast<uint2*>(bimg + bimg_off(p * TC_COLS + col, k0)) = make_uint2(0u, 0u);
-            if ((k0 & 31) == 0) reinterpret_cast<float*>(bimg + bsum_off(k0 >> 5))[col] = 0.f;
-        }
-        if (tid == 0) inv_out[col] = 0.f;
-        return;
-    }
-    const size_t row = (size_t)col * a.ldx;
-    if (n4 <= (int)blockDim.x * QR_MAXV) {
-        // the row lives in registers: every load of the chain is issued before the first use
-        const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f), o4 = make_float4(1.f, 1.f, 1.f, 1.f);
-        const float* ap = a.h_in && a.add_src ? a.add_src + row : nullptr;
-        const bool post = ap && a.w_post, pre = a.h_in && a.w_pre;
-        float4 v[QR_MAXV], va[QR_MAXV], vp[QR_MAXV], vw[QR_MAXV];
-#pragma unroll
-        for (int j = 0; j < QR_MAXV; ++j) {
-            const int i = tid + j * (int)blockDim.x;
+        for (int j = 0; j < MAXV; ++j) {
+            const int i = tid + j * nt;
             const bool in = i < n4;
-            v[j] = in ? reinterpret_cast<const float4*>((a.h_in ? a.h_in : a.x) + row)[i] : z4;
+            v[j] = in ? reinterpret_cast<const float4*>(a.h_in + row)[i] : z4;
             va[j] = (in && ap) ? reinterpret_cast<const float4*>(ap)[i] : z4;
             vp[j] = (in && post) ? reinterpret_cast<const float4*>(a.w_post)[i] : o4;
             vw[j] = (in && pre) ? reinterpret_cast<const float4*>(a.w_pre)[i] : o4;
         }
-        if (a.h_in) {
-            float rms_a = 1.f;
-            if (post) {
-                float ss = 0.f;
-#pragma unroll
-                for (int j = 0; j < QR_MAXV; ++j) { ss = fmaf(va[j].x, va[j].x, ss); ss = fmaf(va[j].y, va[j].y, ss); ss = fmaf(va[j].z, va[j].z, ss); ss = fmaf(va[j].w, va[j].w, ss); }
-                ss = block_sum(ss, red);
-                rms_a = sqrtf(ss / (float)K + a.eps);
-            }
-            const float rcp_a = __frcp_rn(rms_a);
-            float ss = 0.f;
-#pragma unroll
-            for (int j = 0; j < QR_MAXV; ++j) {
-                if (ap) {
-                    if (post) {
-                        v[j].x += div_by(va[j].x, rms_a, rcp_a) * vp[j].x; v[j].y += div_by(va[j].y, rms_a, rcp_a) * vp[j].y;
-                        v[j].z += div_by(va[j].z, rms_a, rcp_a) * vp[j].z; v[j].w += div_by(va[j].w, rms_a, rcp_a) * vp[j].w;
-                    } else { v[j].x += va[j].x; v[j].y += va[j].y; v[j].z += va[j].z; v[j].w += va[j].w; }
-                }
-                ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss); ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
-                const int i = tid + j * (int)blockDim.x;
-                if (i < n4 && a.h_out) reinterpret_cast<float4*>(a.h_out + row)[i] = v[j];
-            }
-            if (pre) {
-                ss = block_sum(ss, red);
-                const float rms = sqrtf(ss / (float)K + a.eps), rcp = __frcp_rn(rms);
-#pragma unroll
-                for (int j = 0; j < QR_MAXV; ++j) {
-                    v[j].x = div_by(v[j].x, rms, rcp) * vw[j].x; v[j].y = div_by(v[j].y, rms, rcp) * vw[j].y;
-                    v[j].z = div_by(v[j].z, rms, rcp) * vw[j].z; v[j].w = div_by(v[j].w, rms, rcp) * vw[j].w;
-                }
-            }
-        }
-        float am = 0.f;
-#pragma unroll
-        for (int j = 0; j < QR_MAXV; ++j) am = fmaxf(am, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
-        am = block_max(am, red);
-        float s, inv;
-        pow2_scale(am, s, inv);
-        if (tid == 0) inv_out[col] = inv;
-#pragma unroll
-        for (int j = 0; j < QR_MAXV; ++j) {
-            const int i = tid + j * (int)blockDim.x;
-            if (j * (int)blockDim.x < n4) put_planes(bimg, col, i, i < n4, v[j], s);     // warp-uniform: whole warps skip together only past the row's end
-        }
-        return;
-    }
-    float am = 0.f;
-    if (a.h_in) {
-        const float* hp = a.h_in + row;
-        const float* ap = a.add_src ? a.add_src + row : nullptr;
         float rms_a = 1.f;
-        if (ap && a.w_post) {
+        if (post) {
             float ss = 0.f;
-            for (int i = tid; i < K; i += blockDim.x) ss = fmaf(ap[i], ap[i], ss);
+#pragma unroll
+            for (int j = 0; j < MAXV; ++j) { ss = fmaf(va[j].x, va[j].x, ss); ss = fmaf(va[j].y, va[j].y, ss); ss = fmaf(va[j].z, va[j].z, ss); ss = fmaf(va[j].w, va[j].w, ss); }
             ss = block_sum(ss, red);
             rms_a = sqrtf(ss / (float)K + a.eps);
         }
         const float rcp_a = __frcp_rn(rms_a);
         float ss = 0.f;
-        for (int i = tid; i < K; i += blockDim.x) {
-            float h = hp[i];
-            if (ap) h += a.w_post ? div_by(ap[i], rms_a, rcp_a) * a.w_post[i] : ap[i];
-            if (a.h_out) a.h_out[row + i] = h;
-            xs[i] = h;
-            ss = fmaf(h, h, ss);
+#pragma unroll
+        for (int j = 0; j < MAXV; ++j) {
+            if (ap) {
+                if (post) {
+                    v[j].x += div_by(va[j].x, rms_a, rcp_a) * vp[j].x; v[j].y += div_by(va[j].y, rms_a, rcp_a) * vp[j].y;
+                    v[j].z += div_by(va[j].z, rms_a, rcp_a) * vp[j].z; v[j].w += div_by(va[j].w, rms_a, rcp_a) * vp[j].w;
+                } else { v[j].x += va[j].x; v[j].y += va[j].y; v[j].z += va[j].z; v[j].w += va[j].w; }
+            }
+            ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss); ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
+            const int i = tid + j * nt;
+            if (i < n4 && a.h_out) reinterpret_cast<float4*>(a.h_out + row)[i] = v[j];
         }
-        ss = block_sum(ss, red);
-        if (a.w_pre) {
+        if (pre) {
+            ss = block_sum(ss, red);
             const float rms = sqrtf(ss / (float)K + a.eps), rcp = __frcp_rn(rms);
-            for (int i = tid; i < K; i += blockDim.x) xs[i] = div_by(xs[i], rms, rcp) * a.w_pre[i];
+#pragma unroll
+            for (int j = 0; j < MAXV; ++j) {
+                v[j].x = div_by(v[j].x, rms, rcp) * vw[j].x; v[j].y = div_by(v[j].y, rms, rcp) * vw[j].y;
+                v[j].z = div_by(v[j].z, rms, rcp) * vw[j].z; v[j].w = div_by(v[j].w, rms, rcp) * vw[j].w;
+            }
         }
-        for (int i = tid; i < K; i += blockDim.x) am = fmaxf(am, fabsf(xs[i]));
     } else {
-        for (int i = tid; i < K; i += blockDim.x) { const float v = a.x[row + i]; xs[i] = v; am = fmaxf(am, fabsf(v)); }
+#pragma unroll
+        for (int j = 0; j < MAXV; ++j) {
+            const int i = tid + j * nt;
+            v[j] = i < n4 ? reinterpret_cast<const float4*>(a.x + row)[i] : z4;
+        }
     }
+    float am = 0.f;
+#pragma unroll
+    for (int j = 0; j < MAXV; ++j) am = fmaxf(am, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
     am = block_max(am, red);
     float s, inv;
-    pow2_scale(am, s, inv);
-    if (tid == 0) inv_out[col] = inv;
-    for (int i0 = 0; i0 < n4; i0 += blockDim.x) {
-        const int i = i0 + tid;
-        const bool on = i < n4;
-        put_planes(bimg, col, i, on, on ? reinterpret_cast<const float4*>(xs)[i] : make_float4(0.f, 0.f, 0.f, 0.f), s);
+    pow2_scale(am, s, inv);                             // largest element in (2^21, 2^22] ...
+    s *= 0.0078125f; inv *= 128.f;                      // ... in (2^14, 2^15]
+    if (tid == 0) inv_out[r] = inv;
+    const int r64 = r & 63;
+    uint8_t* base = img + (size_t)(r >> 6) * n_steps * (2 * TC_STEP_IMG);
+    auto put4 = [&](int k0, float4 f) {                 // values k0 .. k0+3, already scaled
+        __half h[4], l[4];
+        split_half(f.x, h[0], l[0]); split_half(f.z, h[1], l[1]); split_half(f.y, h[2], l[2]); split_half(f.w, h[3], l[3]);
+        uint8_t* d = base + (size_t)(n_min + (k0 >> 6)) * (2 * TC_STEP_IMG) + swz_off(r64, (k0 & 63) * 2);
+        *reinterpret_cast<uint2*>(d) = *reinterpret_cast<const uint2*>(h);
+        *reinterpret_cast<uint2*>(d + TC_STEP_IMG) = *reinterpret_cast<const uint2*>(l);
+    };
+#pragma unroll
+    for (int j = 0; j < MAXV; ++j) {
+        const int i = tid + j * nt;
+        const float4 f = make_float4(v[j].x * s, v[j].y * s, v[j].z * s, v[j].w * s);
+        if (i < n4) put4(4 * i, f);
+        if (n_min) {                                    // sums over 32 neighbouring values (eight lanes), over 32: what Q4_K's block minimum multiplies
+            float t = (f.x + f.y) + (f.z + f.w);
+            t += __shfl_xor_sync(0xffffffffu, t, 1);
+            t += __shfl_xor_sync(0xffffffffu, t, 2);
+            t += __shfl_xor_sync(0xffffffffu, t, 4);
+            if (i < n4 && (i & 7) == 0) {
+                const int sub = i >> 3;
+                __half h, l;
+                split_half(t * 0.03125f, h, l);
+                uint8_t* d = base + (size_t)(sub >> 6) * (2 * TC_STEP_IMG) + swz_off(r64, (sub & 63) * 2);
+                *reinterpret_cast<__half*>(d) = h;
+                *reinterpret_cast<__half*>(d + TC_STEP_IMG) = l;
+            }
+        }
+    }
+    // what the last steps hold beyond the row's end multiplies as zero
+    for (int i = n4 + tid; i < (n_steps - n_min) * 16; i += nt) put4(4 * i, z4);
+    for (int sub = (K >> 5) + tid; sub < n_min * 64; sub += nt) {
+        uint8_t* d = base + (size_t)(sub >> 6) * (2 * TC_STEP_IMG) + swz_off(r64, (sub & 63) * 2);
+        *reinterpret_cast<__half*>(d) = __half(0.f);
+        *reinterpret_cast<__half*>(d + TC_STEP_IMG) = __half(0.f);
     }
 }
 
-// ---- tcgen05 primitives --------------------------------------------------------------------------
-// Shared-memory matrix descriptor, K-major with the 128-byte swizzle (layout 2 at bit 61): start
-// address and the distance between 8-row groups (1024 bytes), in 16-byte units, plus the descriptor
-// version of this architecture (bit 46).  The 16 values of K of one instruction are 32 bytes of a
-// row: the next instruction's descriptor starts 32 bytes further.
+// ---- tcgen05 primitives --------------------------------------------------------------------------------------
+// Shared-memory matrix descriptor, K-major with the 128-byte swizzle (layout 2 at bit 61): start address and the
+// distance between 8-row groups (1024 bytes), in 16-byte units, plus the descriptor version of this architecture (bit 46).
+// The 16 values of K of one instruction are 32 bytes of a row: the next instruction's descriptor starts 32 bytes further.
 __device__ __forceinline__ uint64_t tc_desc(uint32_t saddr) {
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-// Instruction descriptor of kind::f16: D = f32 (1 at bit 4), A = B = f16 (0 at bits 7 and 10), both
-// operands K-major, N / 8 at bit 17, M / 16 at bit 24.
-constexpr uint32_t TC_IDESC = (1u << 4) | ((uint32_t)(TC_N >> 3) << 17) | ((128u >> 4) << 24);
+// Instruction descriptor of kind::f16: D = f32 (1 at bit 4), A = B = f16 (0 at bits 7 and 10), both operands K-major,
+// N / 8 at bit 17, M / 16 at bit 24.
+template <int N> constexpr uint32_t TC_IDESC = (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((128u >> 4) << 24);
 
 __device__ __forceinline__ void tc_alloc(uint32_t* slot, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(slot)), "r"(cols) : "memory");
@@ -256,345 +220,596 @@ __device__ __forceinline__ void tc_dealloc(uint32_t taddr, uint32_t cols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// D[tmem] = A * B (accumulate == 0) or D += A * B; one instruction covers 16 values of K
-__device__ __forceinline__ void tc_mma_f16(uint32_t taddr, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[tmem] * B[smem]; one instruction covers 16 values of K.
+__device__ __forceinline__ void tc_mma_ts(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 :: "r"(taddr), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 :: "r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // The mbarrier gets one arrival when all tensor-core operations issued so far by this thread are done.
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(bar)) : "memory");
 }
-// 32 consecutive 32-bit columns of this thread's TMEM lane.
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&r)[32]) {
-    // the registers hold the values only after tc_ld_wait(): nothing may touch them before
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                 : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]), "=f"(r[8]), "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15]), "=f"(r[16]), "=f"(r[17]), "=f"(r[18]), "=f"(r[19]), "=f"(r[20]), "=f"(r[21]), "=f"(r[22]), "=f"(r[23]), "=f"(r[24]), "=f"(r[25]), "=f"(r[26]), "=f"(r[27]), "=f"(r[28]), "=f"(r[29]), "=f"(r[30]), "=f"(r[31])
-                 : "r"(taddr) : "memory");
+// 16 consecutive 32-bit columns of this thread's TMEM lane, to and from registers.
+__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+                    "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&r)[16]) {       // valid after tc_ld_wait()
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]), "=f"(r[8]), "=f"(r[9]),
+                   "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15]) : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// ---- the GEMM ---------------------------------------------------------------------------------
-// Weights enter the tensor core already scaled: w = 64 * (sa * q + sb) in fp32 (the factor keeps the low
-// term of typical weights out of the fp16 subnormals; |sa * q + sb| must stay below 1000) (sa, sb the block's
-// scale and offset: d and -8 d for Q4_0, d*sc and -dmin*m for Q4_K), split into two fp16 terms
-// w_hi + w_lo (22 bits).  With the activations' planes x_hi, x_lo the product is
-//   sum_k w x = 2048 * (sum w_hi x_hi + sum w_lo x_hi) + sum w_hi x_lo      (w_lo x_lo is below fp32 resolution)
-// and all of a work item's K is accumulated in TMEM: D1 (128 columns) = w_hi x [x_hi | x_lo],
-// D2 (64 columns) = w_lo x x_hi.  Nothing is read back per block.
-//
-// Per step of two K blocks (64 values of K, one 128-byte operand row): the threads expand one 16-byte
-// unit of nibbles each into the two A images of buffer b (the unit was requested one step ahead), one
-// thread waits for the step's B image (16 KB bulk copy, requested one step ahead into buffer b) and
-// issues 4 x 2 tcgen05.mma (K 16 each; N 128 and N 64) and a commit that frees buffer b two steps later.
-// grid = min(items, 2 per SM); item = (tile of 128 weight rows, K split) dealt round-robin.
-// PAIR: a tile is 64 rows of w0 (gate) in TMEM lanes 0..63 and the same 64 rows of w1 (up) in lanes 64..127.
-constexpr uint32_t TC_IDESC_N64 = (1u << 4) | ((uint32_t)(TC_COLS >> 3) << 17) | ((128u >> 4) << 24);
-constexpr int TC_A_BUF = 2 * TC_PAIR_IMG;               // w_hi image + w_lo image of one step
-constexpr int TC_SMEM2 = 2 * TC_A_BUF + 2 * TC_PAIR_IMG + 1024;     // 99328: two A buffers, two B buffers, alignment slack
-
-// Four nibbles-as-bytes of t -> sa * q + sb (the callers pass scales times 64) as fp16 high and low terms (two packed pairs each).
-__device__ __forceinline__ void nib4_split(uint32_t t, float sa, float sb, uint32_t (&hi)[2], uint32_t (&lo)[2]) {
-    float w[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        // byte i of t into mantissa bits 16..23 of 2^7: the float 128 + q, exactly
-        const float f = __uint_as_float(__byte_perm(t, 0x43000000u, 0x7054u | ((uint32_t)i << 8)));
-        w[i] = fmaf(sa, f - 128.f, sb);
-    }
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-        const __half2 h = __floats2half2_rn(w[2 * p], w[2 * p + 1]);
-        const float2 hf = __half22float2(h);
-        const __half2 l = __floats2half2_rn(w[2 * p] - hf.x, w[2 * p + 1] - hf.y);
-        hi[p] = *reinterpret_cast<const uint32_t*>(&h);
-        lo[p] = *reinterpret_cast<const uint32_t*>(&l);
-    }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16_l1(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
+__device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ float ld_cluster(uint32_t saddr, uint32_t rank) {
+    uint32_t a; float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
 }
 
-template <int WT, bool PAIR>
-__global__ void __launch_bounds__(TC_THREADS, 2) k_gemm_tc(const GemvArgs a, const uint8_t* __restrict__ bimg, const float* __restrict__ inv,
-                                                           float* __restrict__ part, unsigned int* __restrict__ tickets, int S, int items) {
+// ---- nibbles -> two fp16 terms ----------------------------------------------------------------------------------
+__device__ __forceinline__ __half2 as_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
+__device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
+// The eight nibbles of a word, two at a time, as halves: low nibbles of bytes (0, 2) and (1, 3) as 1024 + q, high ones
+// as 1024 + 16 q, by masking them into the mantissa of 1024.0.
+__device__ __forceinline__ void nib_pairs(uint32_t w, uint32_t (&lo)[2], uint32_t (&hi)[2]) {
+    const uint32_t w8 = w >> 8;
+    lo[0] = (w & 0x000F000Fu) | 0x64006400u; lo[1] = (w8 & 0x000F000Fu) | 0x64006400u;
+    hi[0] = (w & 0x00F000F0u) | 0x64006400u; hi[1] = (w8 & 0x00F000F0u) | 0x64006400u;
+}
+// v * d as w_hi + w_lo (v two exact small integers)
+__device__ __forceinline__ void split_h2(__half2 v, __half2 d, uint32_t& whi, uint32_t& wlo) {
+    const __half2 h = __hmul2_rn(v, d);                    // rounded once, not contracted
+    whi = as_u32(h);
+    wlo = as_u32(__hfma2(v, d, __hneg2(h)));
+}
+// Scales and minima of group g (64 weights = sub-blocks 2g, 2g+1) of a Q4_K header: sub-block 2g in bits 0..7, 2g+1 in 8..15.
+__device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, uint32_t& mp) {
+    const int sh = (g & 1) * 16;
+    const uint32_t s16 = (h.y >> sh) & 0xFFFFu, m16 = (h.z >> sh) & 0xFFFFu, t16 = (h.w >> sh) & 0xFFFFu;
+    if (g < 2) { sp = s16 & 0x3F3Fu; mp = m16 & 0x3F3Fu; }
+    else { sp = (t16 & 0x0F0Fu) | ((s16 >> 2) & 0x3030u); mp = ((t16 >> 4) & 0x0F0Fu) | ((m16 >> 2) & 0x3030u); }
+}
+
+// ---- the GEMM ---------------------------------------------------------------------------------------------------
+// One CTA per SM, 10 warps: 0..7 rebuild weights, 8 fetches activation tiles, 9 issues the tensor-core instructions.
+// A CTA's tile is NA x 128 weight rows (NA = 2: either 128 gate + 128 up rows of one GeGLU tile, or 256 rows of one
+// matrix, which share an activation tile) by NT activation rows; per 128 rows D is 2 NT columns of TMEM, the rest of TMEM
+// is a ring of four weight tiles (128 rows x 64 values of K as w_hi | w_lo, 64 columns).
+//   weights      A lane owns a row.  Its 32 bytes of nibbles per step come by cp.async into the warp's own ring in shared
+//                memory (R steps ahead, across the end of a tile, two lanes per row so that a sector is fetched whole), are
+//                taken apart in fp16 pairs (4.25 instructions per two weights) and go to TMEM with tcgen05.st: no
+//                shared-memory operand image, no swizzle, no bank conflicts, and the shared memory's 128 bytes per cycle
+//                are left to the activation operand.  Warps 0..3 take the even weight tiles, 4..7 the odd ones.
+//   activations  x_hi | x_lo tiles of 64 values of K by bulk copies from the image, a ring of NB stages shared by the NA
+//                weight tiles of a step.
+//   products     per tile and 16 values of K two tcgen05.mma (M 128): w_hi x [x_hi | x_lo] with N = 2 NT into D1 | D2, and
+//                w_lo x x_hi with N = NT into D2; 384 cycles per tile at NT = 64, which is the tensor core's rate.  One
+//                elected lane issues, but the whole warp walks the loop: inside a one-lane branch the same loop took 628
+//                cycles per tile instead of 413 (waits and descriptors leave the uniform datapath).
+//   rounding     The tensor core rounds its running sum towards zero, an error that grows with the number of instructions
+//                added up (measured: 5e-9 of the result each).  So the cross terms, 2^-11 of the result, have D2 to
+//                themselves, and every `period` steps D1 is added to registers and restarted.  Relative error of a
+//                1152 x 6912 product: 6.1e-6 with one accumulator for all of K, 4e-7 with this.
+//   read-out     The warps that rebuild weight tile i read D1 of tile i (half of the columns each where NA = 1), after
+//                they have produced the first tile of the next period, so the tensor core works on the other tile meanwhile.
+//   K splits     where the tiles alone leave SMs idle, S CTAs of a cluster take a part of K each, leave their sums in their
+//                own shared memory and add each other's columns through distributed shared memory (in split order: results
+//                do not depend on timing).
+// The request for shared memory is at least 120 KB, so that an SM never holds two of these CTAs: one that waits for
+// tensor memory held by a cluster that waits for it would never end.
+constexpr int TC_WARPS = 10, TC_THREADS = TC_WARPS * 32;
+constexpr int TC_SMEM_MIN = 120 * 1024;
+constexpr int TC_PERIOD = 6;                            // most steps (64 values of K) accumulated in D1 before it is read out
+struct TcGemm {
+    WeightRef w0, w1;
+    float* y; int ldy;
+    const uint8_t* img; const float* inv; uint32_t* err;
+    int N, units, B, swiglu;                            // units = K / 32
+    int n_min, n_main, tiles_n, items;                  // items = tiles_n * tiles of NT rows
+    int S, period;                                      // K splits; steps per accumulation period
+};
+template <int WT, int NT, bool PAIR> struct TcGeo {
+    static constexpr int R = 8;                                              // weight ring: steps ahead per warp
+    static constexpr int SLOT = 1024 + (WT == WT_Q4_0 ? 128 : 512);          // 32 rows: nibbles, then block scales / superblock headers
+    static constexpr int NB = 4;
+    static constexpr int BSTAGE = NT * 256;
+    static constexpr int XCH = PAIR ? NT * 512 : 0;                          // gate / up exchange: half of the columns each way
+    static constexpr int SMEM_USED = NB * BSTAGE + 8 * R * SLOT + XCH + 1024;
+    static constexpr int SMEM = SMEM_USED > TC_SMEM_MIN ? SMEM_USED : TC_SMEM_MIN;
+};
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+    return p != 0;
+}
+template <int WT, int NA, int NT, bool PAIR>
+__global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
+    using G = TcGeo<WT, NT, PAIR>;
+    static_assert(!PAIR || NA == 2, "a gate/up tile holds both matrices");
     extern __shared__ __align__(1024) uint8_t sm_raw[];
-    uint8_t* sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);     // the swizzle needs images at multiples of 1024 bytes
-    uint8_t* smA = sm;                                  // [2 buffers][w_hi image, w_lo image]
-    uint8_t* smB = sm + 2 * TC_A_BUF;                   // [2 buffers][pair image]
-    __shared__ __align__(8) uint64_t bar_b[2], bar_free[2];
+    uint8_t* sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);     // the swizzle works on address bits
+    uint8_t* smB = sm;
+    __shared__ __align__(8) uint64_t b_full[G::NB], b_empty[G::NB], a_full[4], a_empty[4], d_full[NA], d_empty[NA];
     __shared__ uint32_t s_tmem;
-    __shared__ bool s_last;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int lane_row = tid & 127, chalf = tid >> 7;          // TMEM lane (row of the tile) and column half this thread reads back
-    const int urow = tid >> 1, uu = tid & 1;                    // operand row and 16-byte unit (of the step's two) this thread expands
-    const int units = a.K >> 5, n_steps = (units + 1) >> 1;
-    constexpr int TILE_ROWS = PAIR ? 64 : 128;
-    int tile = 0;
-    auto row_of = [&](int l, const WeightRef*& w) -> int {      // the weight row behind TMEM lane l of this tile
-        if constexpr (PAIR) { w = (l >> 6) ? &a.w1 : &a.w0; return min(tile * 64 + (l & 63), a.N - 1); }
-        else { w = &a.w0; return min(tile * 128 + l, a.N - 1); }
-    };
-    if (tid == 0) { mbar_init(&bar_b[0], 1); mbar_init(&bar_b[1], 1); mbar_init(&bar_free[0], 1); mbar_init(&bar_free[1], 1); }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (warp == 0) tc_alloc(&s_tmem, TC_TMEM_COLS);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int S = a.S, split = S > 1 ? (int)(blockIdx.x % (uint32_t)S) : 0;     // a cluster's CTAs are neighbours along x
+    const int first = S > 1 ? (int)(blockIdx.x / (uint32_t)S) : (int)blockIdx.x, stride = (int)gridDim.x / S;
+    // this split's share of the steps: first those of the block minima, then those of the products
+    const int mn0 = split * a.n_min / S, mn1 = (split + 1) * a.n_min / S;
+    const int ma0 = split * a.n_main / S, ma1 = (split + 1) * a.n_main / S;
+    const int nmn = mn1 - mn0, nst = nmn + ma1 - ma0, n_steps = a.n_min + a.n_main;
+    if (tid == 0) {
+        for (int i = 0; i < G::NB; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
+        for (int i = 0; i < 4; ++i) { mbar_init(&a_full[i], 4); mbar_init(&a_empty[i], 1); }
+        for (int i = 0; i < NA; ++i) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], NA == 2 ? 4 : 8); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 9) tc_alloc(&s_tmem, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
-    const uint32_t tlane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    constexpr uint32_t A_COL = NA * 2 * NT;             // first column of the weight ring
+    static_assert(A_COL + 256 <= 512, "tensor memory");
     bool dead = false;
     auto wait_on = [&](uint64_t* bar, uint32_t parity) {
         if (!dead && !mbar_wait(bar, parity)) { dead = true; atomicOr(a.err, DEVERR_WAIT); }
     };
-
-    struct Raw { uint4 q; uint4 h; unsigned short d; };
-    const WeightRef* wu = nullptr;
-    int r_u = 0;
-    auto fetch = [&](int st, Raw& r) {                      // this thread's unit of step st (weights only: no dependency on earlier kernels)
-        if constexpr (WT == WT_Q4_0) {
-            const int blk = min(2 * st + uu, units - 1);
-            r.q = ld_stream(wu->q + (size_t)r_u * units + blk);
-            r.d = __ldg(reinterpret_cast<const unsigned short*>(wu->d) + (size_t)r_u * units + blk);
-        } else {
-            const uint4* sb = wu->q + ((size_t)r_u * (units >> 3) + (st >> 2)) * 9;
-            r.h = __ldg(sb);
-            r.q = ld_stream(sb + 1 + (st & 3) * 2 + uu);
-        }
-    };
-    auto fetch_b = [&](int st, int b) {                     // thread 0: the step's B pair image into buffer b
-        mbar_expect_tx(&bar_b[b], (uint32_t)TC_PAIR_IMG);
-        bulk_g2s(smB + b * TC_PAIR_IMG, bimg + (size_t)(st >> 1) * TC_B_CHUNK + (size_t)(st & 1) * TC_PAIR_IMG, (uint32_t)TC_PAIR_IMG, &bar_b[b]);
-    };
-
-    Raw cur, nxt;
-    bool first = true;
-    uint32_t it = 0;                                        // steps done by this CTA: buffer = it & 1, use number of the buffer = it >> 1
     pdl_launch_dependents();
-    for (int item = (int)blockIdx.x; item < items; item += (int)gridDim.x) {
-        const int sp = item % S;
-        tile = item / S;
-        const int st0 = (int)((long long)sp * n_steps / S), st1 = (int)((long long)(sp + 1) * n_steps / S);
-        r_u = row_of(urow, wu);
-        if (st0 < st1) fetch(st0, cur);
-        if (first) { pdl_wait(); first = false; }           // the B image comes from the kernel before this one; weights were requested above
-        if (tid == 0 && st0 < st1) {
-            if ((it >> 1) >= 1u) wait_on(&bar_free[it & 1u], ((it >> 1) - 1u) & 1u);
-            fetch_b(st0, (int)(it & 1u));
-        }
-        for (int st = st0; st < st1; ++st, ++it) {
-            const uint32_t b = it & 1u, n = it >> 1;
-            if (st + 1 < st1) fetch(st + 1, nxt);
-            // scales of the unit's low-nibble and high-nibble halves, times 64
-            float sa0, sb0, sa1, sb1;
-            int p_lo, p_hi;                                 // first 16-byte piece (8 values of K) of the two halves in the 128-byte row
-            if constexpr (WT == WT_Q4_0) {
-                // unit = block 2 st + uu = half uu of the row: low nibbles are its values 0..15, high nibbles 16..31
-                const float d = (2 * st + uu < units) ? 64.f * __half2float(__ushort_as_half(cur.d)) : 0.f;
-                sa0 = sa1 = d; sb0 = sb1 = -8.f * d;
-                p_lo = uu * 4; p_hi = p_lo + 2;
-            } else {
-                // units 2g, 2g+1 = bytes 0..15, 16..31 of group g = this step: low nibbles sub-block 2g (first half
-                // of the row), high nibbles sub-block 2g+1 (second half)
-                float m0, m1;
-                q4k_scales(cur.h, st & 3, sa0, m0, sa1, m1);
-                sa0 *= 64.f; sa1 *= 64.f; sb0 = -64.f * m0; sb1 = -64.f * m1;
-                p_lo = uu * 2; p_hi = 4 + p_lo;
+
+    if (warp == 8) {
+        // ---- activation tiles ----
+        pdl_wait();                                     // the image comes from the kernel before this one
+        const bool lead = elect_one();
+        uint32_t n = 0;
+        for (int item = first; item < a.items; item += stride) {
+            const uint8_t* group = a.img + (size_t)(item / a.tiles_n) * n_steps * (2 * TC_STEP_IMG);
+            for (int st = 0; st < nst; ++st, ++n) {
+                const int bs = (int)(n % G::NB);
+                const uint8_t* src = group + (size_t)(st < nmn ? mn0 + st : a.n_min + ma0 + st - nmn) * (2 * TC_STEP_IMG);
+                uint8_t* dst = smB + bs * G::BSTAGE;
+                if (n >= (uint32_t)G::NB) wait_on(&b_empty[bs], (n / G::NB - 1u) & 1u);
+                if (lead) {
+                    mbar_expect_tx(&b_full[bs], (uint32_t)G::BSTAGE);
+                    if constexpr (NT == TC_GROUP) bulk_g2s(dst, src, G::BSTAGE, &b_full[bs]);
+                    else {                              // the first NT rows of both planes
+                        bulk_g2s(dst, src, NT * 128, &b_full[bs]);
+                        bulk_g2s(dst + NT * 128, src + TC_STEP_IMG, NT * 128, &b_full[bs]);
+                    }
+                }
+                __syncwarp();
             }
-            if (n >= 1u) wait_on(&bar_free[b], (n - 1u) & 1u);  // the tensor core has finished with buffer b
-            {
-                const uint32_t l[4] = {cur.q.x & 0x0F0F0F0Fu, cur.q.y & 0x0F0F0F0Fu, cur.q.z & 0x0F0F0F0Fu, cur.q.w & 0x0F0F0F0Fu};
-                const uint32_t h[4] = {(cur.q.x >> 4) & 0x0F0F0F0Fu, (cur.q.y >> 4) & 0x0F0F0F0Fu, (cur.q.z >> 4) & 0x0F0F0F0Fu, (cur.q.w >> 4) & 0x0F0F0F0Fu};
-                uint8_t* rowp = smA + b * TC_A_BUF + (urow >> 3) * 1024 + (urow & 7) * 128;
-                const int x7 = urow & 7;
+        }
+    } else if (warp == 9) {
+        // ---- products ----
+        pdl_wait();                                     // so that no bounded wait below spans an earlier kernel
+        const bool lead = elect_one();
+        uint32_t n = 0, t = 0, period = 0;              // steps, weight tiles, accumulation periods so far
+        for (int item = first; item < a.items; item += stride) {
+            int left = 0;                               // steps left in the period
+            for (int st = 0; st < nst; ++st, ++n) {
+                const bool fresh = left == 0;
+                if (fresh) { left = min(a.period, nst - st); ++period; }
+                --left;
+                const int bs = (int)(n % G::NB);
+                wait_on(&b_full[bs], (n / G::NB) & 1u);
+                const uint32_t bh = smem_u32(smB + bs * G::BSTAGE);
 #pragma unroll
-                for (int pc = 0; pc < 2; ++pc) {            // 16-byte pieces: words 2 pc, 2 pc + 1 of each nibble half
-                    uint32_t ha[2], la[2], hb[2], lb[2];
-                    nib4_split(l[2 * pc], sa0, sb0, ha, la); nib4_split(l[2 * pc + 1], sa0, sb0, hb, lb);
-                    *reinterpret_cast<uint4*>(rowp + (((p_lo + pc) ^ x7) << 4)) = make_uint4(ha[0], ha[1], hb[0], hb[1]);
-                    *reinterpret_cast<uint4*>(rowp + TC_PAIR_IMG + (((p_lo + pc) ^ x7) << 4)) = make_uint4(la[0], la[1], lb[0], lb[1]);
-                    nib4_split(h[2 * pc], sa1, sb1, ha, la); nib4_split(h[2 * pc + 1], sa1, sb1, hb, lb);
-                    *reinterpret_cast<uint4*>(rowp + (((p_hi + pc) ^ x7) << 4)) = make_uint4(ha[0], ha[1], hb[0], hb[1]);
-                    *reinterpret_cast<uint4*>(rowp + TC_PAIR_IMG + (((p_hi + pc) ^ x7) << 4)) = make_uint4(la[0], la[1], lb[0], lb[1]);
+                for (int i = 0; i < NA; ++i, ++t) {
+                    const uint32_t as = t & 3u, ac = tmem + A_COL + as * 64u, d1 = tmem + (uint32_t)(i * 2 * NT), d2 = d1 + NT;
+                    if (fresh && period > 1) wait_on(&d_empty[i], (period - 2u) & 1u);      // D of the period before is read
+                    wait_on(&a_full[as], (t >> 2) & 1u);
+                    tc_fence_after();
+                    if (lead) {
+                        if (fresh && st > 0) {          // D1 starts again, D2 goes on
+                            tc_mma_ts(d1, ac, tc_desc(bh), TC_IDESC<NT>, 0u);
+                            tc_mma_ts(d2, ac, tc_desc(bh + NT * 128), TC_IDESC<NT>, 1u);
+                        } else tc_mma_ts(d1, ac, tc_desc(bh), TC_IDESC<2 * NT>, st > 0 ? 1u : 0u);
+                        tc_mma_ts(d2, ac + 32u, tc_desc(bh), TC_IDESC<NT>, 1u);
+#pragma unroll
+                        for (uint32_t q = 1; q < 4; ++q) {
+                            tc_mma_ts(d1, ac + q * 8u, tc_desc(bh + q * 32u), TC_IDESC<2 * NT>, 1u);
+                            tc_mma_ts(d2, ac + 32u + q * 8u, tc_desc(bh + q * 32u), TC_IDESC<NT>, 1u);
+                        }
+                        tc_commit(&a_empty[as]);
+                        if (left == 0) tc_commit(&d_full[i]);
+                        if (i == NA - 1) tc_commit(&b_empty[bs]);
+                    }
+                    __syncwarp();
                 }
             }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncthreads();
-            if (tid == 0) {
-                if (st + 1 < st1) {                         // next step's B image into the other buffer (free once the step before this one is done)
-                    const uint32_t b1 = (it + 1u) & 1u, n1 = (it + 1u) >> 1;
-                    if (n1 >= 1u) wait_on(&bar_free[b1], (n1 - 1u) & 1u);
-                    fetch_b(st + 1, (int)b1);
-                }
-                wait_on(&bar_b[b], n & 1u);
-                tc_fence_after();
-                const uint32_t ahi = smem_u32(smA + b * TC_A_BUF), alo = ahi + TC_PAIR_IMG, bb = smem_u32(smB + b * TC_PAIR_IMG);
-#pragma unroll
-                for (uint32_t t = 0; t < 4; ++t) {
-                    const uint32_t accf = (st > st0 || t > 0) ? 1u : 0u;
-                    tc_mma_f16(tmem, tc_desc(ahi + t * 32u), tc_desc(bb + t * 32u), TC_IDESC, accf);
-                    tc_mma_f16(tmem + TC_N, tc_desc(alo + t * 32u), tc_desc(bb + t * 32u), TC_IDESC_N64, accf);
-                }
-                tc_commit(&bar_free[b]);
-            }
-            cur = nxt;
-        }
-        // ---- all of this item's K is in TMEM: read it back once ----
-        float acc[TC_MYCOLS];
-        if (st0 < st1) {
-            const uint32_t last = it - 1u;
-            wait_on(&bar_free[last & 1u], (last >> 1) & 1u);    // the last commit covers every instruction before it
-            tc_fence_after();
-            float hh[32], hl[32], lh[32];
-            tc_ld32(tlane + chalf * 32, hh);                    // w_hi x x_hi
-            tc_ld32(tlane + TC_COLS + chalf * 32, hl);          // w_hi x x_lo
-            tc_ld32(tlane + TC_N + chalf * 32, lh);             // w_lo x x_hi
-            tc_ld_wait();
-#pragma unroll
-            for (int c = 0; c < 32; ++c) acc[c] = fmaf(hh[c] + lh[c], 2048.f, hl[c]);
-            tc_fence_before();
-        } else {
-#pragma unroll
-            for (int c = 0; c < 32; ++c) acc[c] = 0.f;
-        }
-    // ---- epilogue ----
-    const int r_out = PAIR ? (tid & 63) : lane_row;             // row of the tile this thread finishes
-    const int row = tile * TILE_ROWS + r_out;
-    auto finish = [&](int c, float v0, float v1) {              // column c: scale back, activation, store
-        if (c < a.B && row < a.N) {
-            const float sc = inv[c] * (1.f / 64.f);             // the weights went in times 64
-            float out = v0 * sc;
-            if constexpr (PAIR) out = (a.epi == EPI_GEGLU ? gelu_tanh(out) : silu_clip(out)) * (v1 * sc);
-            a.y[(size_t)c * a.ldy + row] = out;
-        }
-    };
-    if (S == 1) {
-        if constexpr (!PAIR) {
-#pragma unroll
-            for (int c = 0; c < TC_MYCOLS; ++c) finish(chalf * TC_MYCOLS + c, acc[c], 0.f);
-        } else {
-            // gate (lanes 0..63) and up (lanes 64..127) of a row meet through shared memory
-            float* ex = reinterpret_cast<float*>(sm);           // [64 columns][128 lanes]; the images are no longer read
-#pragma unroll
-            for (int c = 0; c < TC_MYCOLS; ++c) ex[(chalf * TC_MYCOLS + c) * 128 + lane_row] = acc[c];
-            __syncthreads();
-            for (int c = tid >> 6; c < a.B; c += TC_THREADS / 64) finish(c, ex[c * 128 + r_out], ex[c * 128 + 64 + r_out]);
         }
     } else {
-        // partial sums of this (tile, split): [64 columns][128 lanes]
-        float* mine = part + (size_t)item * TC_COLS * 128;
+        // ---- weights, and the end of a tile ----
+        const int grp = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane;       // row = this lane's TMEM lane
+        const int mine = NA == 2 ? grp : 0;             // which 128 rows of the tile this group rebuilds and reads back
+        const uint32_t tlane = tmem + ((uint32_t)(quarter * 32) << 16);
+        uint8_t* ring = sm + G::NB * G::BSTAGE + warp * G::R * G::SLOT;
+        const uint32_t ring_s = smem_u32(ring);
+        const WeightRef w = (PAIR && grp) ? a.w1 : a.w0;
+        const bool scales_async = WT == WT_Q4_K || ((a.units & 1) == 0 && ((uintptr_t)w.d & 3) == 0);
+        const int n_own = NA == 2 ? nst : (nst + 1 - grp) / 2;                          // this group's weight tiles of an item
+        auto step_of = [&](int j) { return NA == 2 ? j : grp + 2 * j; };
+        auto row_of = [&](int tn, int r) { return min((PAIR ? tn * 128 : (tn * NA + mine) * 128) + r, a.N - 1); };
+        const int rpu = WT == WT_Q4_0 ? a.units : (a.units >> 3) * 9;                   // uint4 per weight row
+        const int n_items = first < a.items ? (a.items - first + stride - 1) / stride : 0;
+
+        // fetch cursor, R tiles ahead of the production cursor
+        int f_item = 0, f_j = 0; uint32_t f_n = 0;
+        const uint4 *f_q[2] = {nullptr, nullptr}, *f_h = nullptr; const __half* f_d = nullptr;
+        auto fetch = [&]() {
+            if (f_item < n_items && n_own > 0) {
+                if (f_j == 0) {
+                    const int tn = (first + f_item * stride) % a.tiles_n;
 #pragma unroll
-        for (int c = 0; c < TC_MYCOLS; ++c) mine[(chalf * TC_MYCOLS + c) * 128 + lane_row] = acc[c];
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) {
-            const unsigned int t = atomicAdd(&tickets[tile], 1u);
-            s_last = t == (unsigned int)(S - 1);
-            if (s_last) tickets[tile] = 0u;
-        }
-        __syncthreads();
-        if (s_last) {
-            // the last CTA of the tile adds the splits in order, 8 columns x 4 splits of loads in flight
-            __threadfence();
-            const float* base = part + (size_t)tile * S * TC_COLS * 128;
-            constexpr int CG = 8;
-            constexpr int GSTEP = TC_THREADS / TILE_ROWS;       // column groups worked on side by side
-            for (int g8 = tid / TILE_ROWS; g8 * CG < a.B; g8 += GSTEP) {
-                float v0[CG], v1[CG];
+                    for (int h = 0; h < 2; ++h) f_q[h] = w.q + (size_t)row_of(tn, quarter * 32 + 16 * h + (lane >> 1)) * rpu;
+                    if constexpr (WT == WT_Q4_0) f_d = w.d + (size_t)row_of(tn, row) * a.units;
+                    else f_h = w.q + (size_t)row_of(tn, row) * rpu;
+                }
+                const int st = step_of(f_j), ks = ma0 + st - nmn;
+                if (st >= nmn) {
+                    const uint32_t dst = ring_s + (f_n % G::R) * G::SLOT;
+                    const int half = lane & 1;
+                    const int off = WT == WT_Q4_0 ? min(2 * ks + half, a.units - 1) : (ks >> 2) * 9 + 1 + (ks & 3) * 2 + half;
 #pragma unroll
-                for (int e = 0; e < CG; ++e) { v0[e] = 0.f; v1[e] = 0.f; }
-                for (int s0 = 0; s0 < S; s0 += 4) {
-                    float t0[4][CG], t1[4][CG];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float* p = base + ((size_t)min(s0 + i, S - 1) * TC_COLS + g8 * CG) * 128;
-#pragma unroll
-                        for (int e = 0; e < CG; ++e) {
-                            t0[i][e] = __ldcg(p + e * 128 + r_out);
-                            if constexpr (PAIR) t1[i][e] = __ldcg(p + e * 128 + 64 + r_out);
-                        }
+                    for (int h = 0; h < 2; ++h) {
+                        const int rl = 16 * h + (lane >> 1);
+                        cp_async16(dst + rl * 32 + ((half ^ ((rl >> 2) & 1)) << 4), f_q[h] + off);
                     }
+                    if constexpr (WT == WT_Q4_0) { if (scales_async) cp_async4(dst + 1024 + lane * 4, f_d + 2 * ks); }
+                    else cp_async16_l1(dst + 1024 + lane * 16, f_h + (ks >> 2) * 9);
+                }
+                if (++f_j == n_own) { f_j = 0; ++f_item; }
+            }
+            ++f_n;
+            cp_commit();
+        };
+
+        // D1 (and, with the item's last period, D2) into acc; the end of an item: scale back, activation, store
+        constexpr int COLS = NA == 2 ? NT : (NT >= 32 ? NT / 2 : 16);                   // columns this group reads back
+        const bool reads = NA == 2 || NT >= 32 || grp == 0;
+        const int c0 = NA == 2 ? 0 : grp * COLS;
+        const int np = (nst + a.period - 1) / a.period;                                 // periods per item
+        bool waited = false;
+        int done = 0, done_item = 0, done_p = 0;        // periods read out: in all, as (item, period of the item)
+        float acc[COLS];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        if (s0 + i < S) {
+        for (int c = 0; c < COLS; ++c) acc[c] = 0.f;
+        auto read_out = [&]() {
+            if (!waited) { pdl_wait(); waited = true; }
+            const bool last = done_p == np - 1;
+            wait_on(&d_full[mine], (uint32_t)done & 1u);
+            tc_fence_after();
+            if (reads) {
+                const uint32_t col = tlane + (uint32_t)(mine * 2 * NT + c0);
 #pragma unroll
-                            for (int e = 0; e < CG; ++e) { v0[e] += t0[i][e]; if constexpr (PAIR) v1[e] += t1[i][e]; }
-                        }
+                for (int ch = 0; ch < COLS / 16; ++ch) {
+                    float v[16];
+                    tc_ld16(col + ch * 16, v);
+                    tc_ld_wait();
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) acc[ch * 16 + c] += v[c];
+                }
+                if (last) {
+#pragma unroll
+                    for (int ch = 0; ch < COLS / 16; ++ch) {
+                        float v[16];
+                        tc_ld16(col + NT + ch * 16, v);
+                        tc_ld_wait();
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) acc[ch * 16 + c] += v[c];
                     }
                 }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&d_empty[mine]);
+            ++done; ++done_p;
+            if (!last) return;
+            const int item = first + done_item * stride, tn = item % a.tiles_n, m0 = item / a.tiles_n * NT;
+            done_p = 0; ++done_item;
+            const int n_out = (PAIR ? tn * 128 : (tn * NA + mine) * 128) + row, n_col = min(NT, a.B - m0);
+            const float inv0 = m0 + lane < a.B ? a.inv[m0 + lane] : 0.f, inv1 = NT > 32 && m0 + 32 + lane < a.B ? a.inv[m0 + 32 + lane] : 0.f;
+            float* yp = a.y + (size_t)m0 * a.ldy + n_out;
+            auto inv_of = [&](int c) { return __shfl_sync(0xffffffffu, c < 32 ? inv0 : inv1, c & 31); };
+            auto act = [&](float gate, float up) { return (a.swiglu ? silu_clip(gate) : gelu_tanh(gate)) * up; };
+            if (S > 1) {
+                // one item per cluster: sums into the exchange (the activation ring is drained), then every CTA finishes the
+                // columns c = split, split + S, ... from all S parts
+                float* ex = reinterpret_cast<float*>(smB);
+                if (reads) {
 #pragma unroll
-                for (int e = 0; e < CG; ++e) finish(g8 * CG + e, v0[e], v1[e]);
+                    for (int c = 0; c < COLS; ++c) ex[(mine * NT + c0 + c) * 128 + row] = acc[c];
+                }
+                cl_arrive();
+                cl_wait();
+                const uint32_t ex_s = smem_u32(ex);
+                auto total_of = [&](int i, int c) {             // all loads in flight, then one order of addition
+                    float p[8], v = 0.f;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) p[q] = q < S ? ld_cluster(ex_s + (uint32_t)((i * NT + c) * 128 + row) * 4u, (uint32_t)q) : 0.f;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) v += p[q];
+                    return v;
+                };
+                if constexpr (PAIR || NA == 1) {                // both groups share the columns
+                    for (int c = split + S * grp; c < n_col; c += 2 * S) {
+                        const float sc = inv_of(c), v = total_of(0, c);
+                        if constexpr (PAIR) { const float u = total_of(1, c); if (n_out < a.N) yp[(size_t)c * a.ldy] = act(v * sc, u * sc); }
+                        else if (n_out < a.N) yp[(size_t)c * a.ldy] = v * sc;
+                    }
+                } else {
+                    for (int c = split; c < n_col; c += S) {
+                        const float v = total_of(mine, c) * inv_of(c);
+                        if (n_out < a.N) yp[(size_t)c * a.ldy] = v;
+                    }
+                }
+                cl_arrive();
+                cl_wait();
+            } else if constexpr (PAIR) {
+                // gate (group 0) and up (group 1) swap half of their columns; group 0 finishes the first half
+                float* x0 = reinterpret_cast<float*>(sm + G::NB * G::BSTAGE + 8 * G::R * G::SLOT);
+                constexpr int H = NT / 2;
+                float* put = x0 + (grp ? 0 : H * 128) + row;
+                const float* get = x0 + (grp ? H * 128 : 0) + row;
+#pragma unroll
+                for (int c = 0; c < H; ++c) put[c * 128] = grp ? acc[c] : acc[H + c];
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+#pragma unroll
+                for (int c = 0; c < H; ++c) {
+                    const int col = grp * H + c;
+                    const float o = get[c * 128], sc = inv_of(col), m = grp ? acc[H + c] : acc[c];
+                    if (col < n_col && n_out < a.N) yp[(size_t)col * a.ldy] = grp ? act(o * sc, m * sc) : act(m * sc, o * sc);
+                }
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+            } else if (reads) {
+#pragma unroll
+                for (int c = 0; c < COLS; ++c) {
+                    const float v = acc[c] * inv_of(c0 + c);
+                    if (c0 + c < n_col && n_out < a.N) yp[(size_t)(c0 + c) * a.ldy] = v;
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) acc[c] = 0.f;
+        };
+        // ---- production ----
+        for (int j = 0; j < G::R; ++j) fetch();
+        uint32_t t = (uint32_t)grp, n = 0;              // tile number in the order of the products; tiles of this group
+        for (int k = 0; k < n_items; ++k) {
+            const int tn = (first + k * stride) % a.tiles_n;
+            for (int j = 0; j < n_own; ++j, ++n) {
+                const int st = step_of(j), ks = ma0 + st - nmn;
+                if constexpr (NA == 2) t = 2u * n + (uint32_t)grp;
+                else t = (uint32_t)(k * nst + st);
+                const uint32_t as = t & 3u, acol = tlane + A_COL + as * 64u;
+                cp_wait<G::R - 1>();
+                __syncwarp();
+                const uint8_t* slot = ring + (n % G::R) * G::SLOT;
+                const uint4 q0 = *reinterpret_cast<const uint4*>(slot + lane * 32 + (((lane >> 2) & 1) << 4));
+                const uint4 q1 = *reinterpret_cast<const uint4*>(slot + lane * 32 + (((~lane >> 2) & 1) << 4));
+                uint32_t d01 = 0; uint4 hdr = make_uint4(0, 0, 0, 0);
+                if constexpr (WT == WT_Q4_0) d01 = *reinterpret_cast<const uint32_t*>(slot + 1024 + lane * 4);
+                else hdr = *reinterpret_cast<const uint4*>(slot + 1024 + lane * 16);
+                __syncwarp();
+                fetch();
+                if (t >= 4u) {
+                    if (!waited) { pdl_wait(); waited = true; }
+                    wait_on(&a_empty[as], ((t >> 2) - 1u) & 1u);
+                    tc_fence_after();
+                }
+                const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+                if constexpr (WT == WT_Q4_0) {
+                    if (!scales_async) {                // odd number of blocks per row: their scales are not pairs of aligned halves
+                        const unsigned short* dp = reinterpret_cast<const unsigned short*>(w.d) + (size_t)row_of(tn, row) * a.units + 2 * ks;
+                        d01 = (uint32_t)dp[0] | (2 * ks + 1 < a.units ? (uint32_t)dp[1] << 16 : 0u);
+                    }
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        const uint32_t dd = b ? d01 >> 16 : d01 & 0xFFFFu;
+                        const __half2 d = as_h2(dd * 0x10001u);
+                        uint32_t whi[16], wlo[16];
+#pragma unroll
+                        for (int x = 0; x < 4; ++x) {
+                            uint32_t l[2], h[2];
+                            nib_pairs(qw[4 * b + x], l, h);
+#pragma unroll
+                            for (int p = 0; p < 2; ++p) {
+                                split_h2(__hadd2(as_h2(l[p]), __float2half2_rn(-1032.f)), d, whi[2 * x + p], wlo[2 * x + p]);
+                                split_h2(__hfma2(as_h2(h[p]), __float2half2_rn(0.0625f), __float2half2_rn(-72.f)), d, whi[8 + 2 * x + p], wlo[8 + 2 * x + p]);
+                            }
+                        }
+                        tc_st16(acol + b * 16u, whi);
+                        tc_st16(acol + 32u + b * 16u, wlo);
+                    }
+                } else if (st >= nmn) {
+                    uint32_t sp, mp;
+                    q4k_codes(hdr, ks & 3, sp, mp);
+                    const __half2 d = as_h2((hdr.x & 0xFFFFu) * 0x10001u);
+                    uint32_t lo_[8][2], hi_[8][2];
+#pragma unroll
+                    for (int x = 0; x < 8; ++x) nib_pairs(qw[x], lo_[x], hi_[x]);
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {       // low nibbles = sub-block 2g, high nibbles = sub-block 2g + 1
+                        const uint32_t code = b ? sp >> 8 : sp & 0xFFu;
+                        const __half2 sc = __hsub2(as_h2((code * 0x10001u) | 0x64006400u), __float2half2_rn(1024.f));
+                        const __half2 mul = b ? __hmul2(sc, __float2half2_rn(0.0625f)) : sc;
+                        const __half2 off = __hmul2(sc, __float2half2_rn(b ? -64.f : -1024.f));
+                        uint32_t whi[16], wlo[16];
+#pragma unroll
+                        for (int x = 0; x < 8; ++x)
+#pragma unroll
+                            for (int p = 0; p < 2; ++p)   // sc * q, an integer below 946, exactly
+                                split_h2(__hfma2(as_h2(b ? hi_[x][p] : lo_[x][p]), mul, off), d, whi[2 * x + p], wlo[2 * x + p]);
+                        tc_st16(acol + b * 16u, whi);
+                        tc_st16(acol + 32u + b * 16u, wlo);
+                    }
+                } else {
+                    // a step of block minima: -32 dmin m of 64 sub-blocks (the image holds the sums over 32 activations / 32)
+                    const int sb0 = (mn0 + st) * 8, n_sb = a.units >> 3;
+                    const uint4* src = w.q + (size_t)row_of(tn, row) * rpu;
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        uint32_t whi[16], wlo[16];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int sb = sb0 + 4 * b + e;
+                            const uint4 h = __ldg(src + (size_t)min(sb, n_sb - 1) * 9);
+                            const float dm = sb < n_sb ? -32.f * __half2float(__ushort_as_half((unsigned short)(h.x >> 16))) : 0.f;
+#pragma unroll
+                            for (int gq = 0; gq < 4; ++gq) {
+                                uint32_t sp, mp;
+                                q4k_codes(h, gq, sp, mp);
+                                const float v0 = dm * (float)(mp & 0xFFu), v1 = dm * (float)(mp >> 8);
+                                const __half2 h2 = __floats2half2_rn(v0, v1);
+                                const float2 f2 = __half22float2(h2);
+                                whi[4 * e + gq] = as_u32(h2);
+                                wlo[4 * e + gq] = as_u32(__floats2half2_rn(v0 - f2.x, v1 - f2.y));
+                            }
+                        }
+                        tc_st16(acol + b * 16u, whi);
+                        tc_st16(acol + 32u + b * 16u, wlo);
+                    }
+                }
+                tc_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&a_full[as]);
+                while (done < k * np + st / a.period) read_out();       // what ended before this tile's period
             }
         }
+        while (done < n_items * np) read_out();
+        cp_wait<0>();
     }
-    __syncthreads();                                    // the images, s_last and the exchange buffer are free again
-    }   // work items
-    if (warp == 0) tc_dealloc(tmem, TC_TMEM_COLS);
+    if (S > 1 && warp >= 8) { cl_arrive(); cl_wait(); cl_arrive(); cl_wait(); }
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 9) tc_dealloc(tmem, 512);
 }
 
-// ---- host ----------------------------------------------------------------------------------------
+// ---- host ----------------------------------------------------------------------------------------------------------
+static bool tc_policy_takes(int wtype, const GemvArgs& a, bool pair) {
+    if (g_tc_policy < 0) g_tc_policy = getenv("ADAM_B200_TC") ? atoi(getenv("ADAM_B200_TC")) : 1;
+    if (g_tc_policy == 0) return false;
+    if (g_tc_policy == 2) return true;
+    (void)wtype; (void)a; (void)pair;
+    return true;
+}
+
 bool gemm_tc_supports(int wtype, const GemvArgs& a) {
     if (wtype != WT_Q4_0 && wtype != WT_Q4_K) return false;
-    if (g_tc_policy < 0) g_tc_policy = getenv("ADAM_B200_TC") ? atoi(getenv("ADAM_B200_TC")) : 1;
-    if (g_tc_policy == 0 || !g_tc.ok) return false;
-    if (a.B < TC_MIN_ROWS || a.B > TC_COLS) return false;
-    if (a.epi != EPI_STORE && a.epi != EPI_GEGLU && a.epi != EPI_SWIGLU) return false;
-    if (a.K <= 0 || a.K > TC_MAX_K || a.N < 16 || !a.y) return false;
-    if (wtype == WT_Q4_0 ? (a.K % 32) != 0 : (a.K % 256) != 0) return false;
-    if ((a.ldx & 3) || (!a.h_in && !a.x)) return false;
-    const bool pair = a.epi != EPI_STORE;
-    if (g_tc_policy == 1) {
-        // The GEMV kernels pass over the weights once per 4 rows; this kernel passes once but has a fixed
-        // cost of 10-15 us.  Measured cross-over: weights x passes of about 2e8 (Q4_0) / 1e8 (Q4_K) elements.
-        const double work = (double)a.N * a.K * (pair ? 2 : 1) * ((a.B + 3) / 4);
-        if (work < (wtype == WT_Q4_0 ? 2.0e8 : 1.0e8)) return false;
-    }
-    const int tiles = pair ? (a.N + 63) / 64 : (a.N + 127) / 128;
-    return tiles <= TC_MAX_CTAS && tiles <= TC_MAX_TILES && (size_t)a.K * 4 <= 160 * 1024;
+    if (a.B < TC_MIN_ROWS || (a.epi != EPI_STORE && a.epi != EPI_GEGLU && a.epi != EPI_SWIGLU)) return false;
+    if (a.K <= 0 || a.K > TC_MAX_K || a.N < 16 || !a.y || (wtype == WT_Q4_0 ? (a.K % 32) : (a.K % 256))) return false;
+    if ((a.ldx & 3) || (!a.h_in && (!a.x || ((uintptr_t)a.x & 15)))) return false;
+    if (!tc_policy_takes(wtype, a, a.epi != EPI_STORE)) return false;
+    return tc_rows_fit(wtype, a.K) >= 128;
 }
 
-int launch_gemm_tc(int wtype, const GemvArgs& a_in, cudaStream_t stream) {
-    GemvArgs a = a_in;
-    a.err = g.dev_err;
+typedef void (*TcKernel)(const TcGemm);
+struct TcPick { TcKernel k; int smem; bool attr; };
+template <int WT, int NA, int NT, bool PAIR> static TcPick& tc_pick() {
+    static TcPick p = {k_gemm_tc<WT, NA, NT, PAIR>, TcGeo<WT, NT, PAIR>::SMEM, false};
+    return p;
+}
+template <int WT> static TcPick& tc_pick(int nt, int na, bool pair) {
+    if (pair) return nt == 16 ? tc_pick<WT, 2, 16, true>() : nt == 32 ? tc_pick<WT, 2, 32, true>() : tc_pick<WT, 2, 64, true>();
+    if (na == 2) return tc_pick<WT, 2, 64, false>();
+    return nt == 16 ? tc_pick<WT, 1, 16, false>() : nt == 32 ? tc_pick<WT, 1, 32, false>() : tc_pick<WT, 1, 64, false>();
+}
+
+static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
     const bool pair = a.epi != EPI_STORE;
-    const int tiles = pair ? (a.N + 63) / 64 : (a.N + 127) / 128;
-    const int n_chunks = (a.K / 32 + TC_CH - 1) / TC_CH;
-    // Splits per tile: the cheapest of 1..32 under a simple model (time in chunks: the items are dealt to
-    // 2 CTAs per SM; every item costs its chunks plus about two chunks of fixed work, the last CTA of a
-    // tile also reads every split's partial sums).
-    const int slots = 2 * g.sm_count;
-    int S = 1;
-    {
-        double best = 1e30;
-        for (int c = 1; c <= 32 && c <= n_chunks; ++c) {
-            const long long it = (long long)tiles * c;
-            if (it > TC_MAX_CTAS) break;
-            const double rounds = (double)((it + slots - 1) / slots);
-            const double cost = rounds * ((double)((n_chunks + c - 1) / c) + 2.0) + (c > 1 ? 0.5 + 0.1 * c : 0.0);
-            if (cost < best - 1e-9) { best = cost; S = c; }
+    const int n_min = tc_min_steps(wtype, a.K), n_main = tc_main_steps(a.K), n4 = a.K / 4;
+    {   // one CTA per row; the fewest float4 per thread that 512 threads allow
+        const int cand[5] = {1, 2, 4, 8, 16};
+        int mv = 16;
+        for (int c : cand) if ((n4 + c - 1) / c <= 512) { mv = c; break; }
+        const int threads = ((n4 + mv - 1) / mv + 31) / 32 * 32;
+        auto go = [&](auto kern) { launch_k(kern, dim3(a.B), dim3(threads), 0, stream, g.pdl, a, g_tc.img, g_tc.inv, n_min, n_min + n_main); };
+        const bool chain = a.h_in != nullptr;
+        switch (mv) {
+        case 1: if (chain) go(k_quant_rows<1, true>); else go(k_quant_rows<1, false>); break;
+        case 2: if (chain) go(k_quant_rows<2, true>); else go(k_quant_rows<2, false>); break;
+        case 4: if (chain) go(k_quant_rows<4, true>); else go(k_quant_rows<4, false>); break;
+        case 8: if (chain) go(k_quant_rows<8, true>); else go(k_quant_rows<8, false>); break;
+        default: if (chain) go(k_quant_rows<16, true>); else go(k_quant_rows<16, false>); break;
+        }
+        count_launch();
+    }
+    // Tile and K splits: the cheapest of the candidates under an estimate in SM cycles.  A weight tile costs the larger of
+    // its tensor-core time (6 cycles per activation row), its rebuilding (about 200 issue cycles) and the fetch of its
+    // activation tile (NT * 256 bytes, shared by NA weight tiles, at about 40 bytes per cycle and SM out of L2); a CTA
+    // costs about 3000 cycles besides, a K split about 1500 more.
+    const int nt = a.B <= 16 ? 16 : a.B <= 32 ? 32 : 64;
+    const int tiles_m = (a.B + nt - 1) / nt;
+    int na = pair ? 2 : 1, S = 1;
+    double best = 1e300;
+    for (int c_na = pair ? 2 : 1; c_na <= (pair || nt == 64 ? 2 : 1); ++c_na) {
+        const long long items = (long long)(pair ? (a.N + 127) / 128 : (a.N + 128 * c_na - 1) / (128 * c_na)) * tiles_m;
+        const double tile = fmax(fmax(6.0 * nt, 200.0), nt * 256.0 / c_na / 40.0);
+        for (int s = 1; s <= 8 && s <= n_main; s *= 2) {
+            const double waves = (double)((items * s + g.sm_count - 1) / g.sm_count);
+            const int steps = (n_main + s - 1) / s + (n_min + s - 1) / s;
+            const double cost = waves * (steps * c_na * tile + (s > 1 ? 4500.0 : 3000.0));
+            if (cost < best * 0.999) { best = cost; na = c_na; S = s; }
         }
     }
-    const int items = tiles * S;
-    static bool attr_done = false;
-    if (!attr_done) {
-        cudaFuncSetAttribute(k_quant_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-        cudaFuncSetAttribute(k_gemm_tc<WT_Q4_0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM2);
-        cudaFuncSetAttribute(k_gemm_tc<WT_Q4_0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM2);
-        cudaFuncSetAttribute(k_gemm_tc<WT_Q4_K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM2);
-        cudaFuncSetAttribute(k_gemm_tc<WT_Q4_K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM2);
-        attr_done = true;
+    TcGemm t = {};
+    t.w0 = a.w0; t.w1 = a.w1; t.y = a.y; t.ldy = a.ldy; t.img = g_tc.img; t.inv = g_tc.inv; t.err = g.dev_err;
+    t.N = a.N; t.units = a.K / 32; t.B = a.B; t.swiglu = a.epi == EPI_SWIGLU;
+    t.n_min = n_min; t.n_main = n_main; t.S = S;
+    const int longest = (n_main + S - 1) / S + (n_min + S - 1) / S, n_periods = (longest + TC_PERIOD - 1) / TC_PERIOD;
+    t.period = (longest + n_periods - 1) / n_periods;
+    t.tiles_n = pair ? (a.N + 127) / 128 : (a.N + 128 * na - 1) / (128 * na);
+    t.items = t.tiles_n * tiles_m;
+    TcPick& p = wtype == WT_Q4_0 ? tc_pick<WT_Q4_0>(nt, na, pair) : tc_pick<WT_Q4_K>(nt, na, pair);
+    if (!p.attr) {
+        if (cudaFuncSetAttribute((const void*)p.k, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem) != cudaSuccess)
+            return fail(ADAMAH_ERR_BACKEND, "gemm_tc: cannot raise the shared-memory limit");
+        p.attr = true;
     }
-    launch_k(k_quant_rows, dim3(TC_COLS), dim3(QR_THREADS), (a.K >> 2) <= QR_THREADS * QR_MAXV ? (size_t)0 : (size_t)a.K * 4, stream, g.pdl, a, g_tc.bimg, g_tc.inv);
+    cudaError_t e;
+    if (S == 1) e = launch_k(p.k, dim3((unsigned)(t.items < g.sm_count ? t.items : g.sm_count)), dim3(TC_THREADS), (size_t)p.smem, stream, g.pdl, t);
+    else e = launch_k_cluster(p.k, dim3((unsigned)(t.items * S)), dim3(TC_THREADS), (size_t)p.smem, stream, g.pdl, (unsigned)S, t);
+    if (e != cudaSuccess) return fail(ADAMAH_ERR_BACKEND, "gemm_tc: launch failed: %s", cudaGetErrorString(e));
     count_launch();
-    const dim3 grid((unsigned)(items < slots ? items : slots)), block(TC_THREADS);
-    if (wtype == WT_Q4_0) {
-        if (pair) launch_k(k_gemm_tc<WT_Q4_0, true>, grid, block, (size_t)TC_SMEM2, stream, g.pdl, a, (const uint8_t*)g_tc.bimg, (const float*)g_tc.inv, g_tc.part, g_tc.tickets, S, items);
-        else launch_k(k_gemm_tc<WT_Q4_0, false>, grid, block, (size_t)TC_SMEM2, stream, g.pdl, a, (const uint8_t*)g_tc.bimg, (const float*)g_tc.inv, g_tc.part, g_tc.tickets, S, items);
-    } else {
-        if (pair) launch_k(k_gemm_tc<WT_Q4_K, true>, grid, block, (size_t)TC_SMEM2, stream, g.pdl, a, (const uint8_t*)g_tc.bimg, (const float*)g_tc.inv, g_tc.part, g_tc.tickets, S, items);
-        else launch_k(k_gemm_tc<WT_Q4_K, false>, grid, block, (size_t)TC_SMEM2, stream, g.pdl, a, (const uint8_t*)g_tc.bimg, (const float*)g_tc.inv, g_tc.part, g_tc.tickets, S, items);
+    return ADAMAH_OK;
+}
+
+// Rows that exceed the workspace run in chunks of whole 128-row tiles.
+int launch_gemm_tc(int wtype, const GemvArgs& a, cudaStream_t stream) {
+    const int fit = tc_rows_fit(wtype, a.K);
+    for (int b0 = 0; b0 < a.B; b0 += fit) {
+        GemvArgs c = a;
+        c.B = a.B - b0 < fit ? a.B - b0 : fit;
+        if (a.x) c.x = a.x + (size_t)b0 * a.ldx;
+        if (a.h_in) c.h_in = a.h_in + (size_t)b0 * a.ldx;
+        if (a.add_src) c.add_src = a.add_src + (size_t)b0 * a.ldx;
+        if (a.h_out) c.h_out = a.h_out + (size_t)b0 * a.ldx;
+        c.y = a.y + (size_t)b0 * a.ldy;
+        const int rc = launch_rows(wtype, c, stream);
+        if (rc) return rc;
     }
-    count_launch();
     ++g_tc_calls;
     return check_launch("gemm_tc");
 }

@@ -562,7 +562,7 @@ int run_gemv(uint32_t map_id, uint64_t off, int wtype, GemvArgs& ga) {
     if (ga.B >= TC_MIN_ROWS) {
         // many rows: the tcgen05 GEMM (its workspace is allocated on first use, never inside a capture)
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(g.stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) gemm_tc_prepare();
+        if (cudaStreamIsCapturing(g.stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) gemm_tc_prepare(ga.B, ga.K);
         if (gemm_tc_supports(wtype, ga)) return launch_gemm_tc(wtype, ga, g.stream);
     }
     if (ga.epi != EPI_GEGLU && ga.epi != EPI_SWIGLU) {
