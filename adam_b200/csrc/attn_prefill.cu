@@ -1,0 +1,499 @@
+// Attention of a prefill chunk: causal soft-max attention of many query rows over the paged cache
+// (map_qk_norm_rope_x.comp, map_row_copy.comp, map_matmul_t.comp + map_attn_softmax_value.comp for every prompt position;
+// adam/models/engine.py:3838-3847 walks the prompt one position at a time).
+//
+// The decode attention (k_attention in decoder.cu) gives every row its own pass over the cache on the fp32 pipe; for a
+// prompt that is rows x context cache reads.  Here 64 or 128 query rows (positions x the query heads of one kv head)
+// share each tile of the cache, and both products run on mma.sync tensor instructions with the operands kept at the
+// precision of the fp32 path: the cache's fp16 values are exact operands, and a query row or a row of probabilities goes
+// in as two fp16 terms (22 bits); an fp32 cache takes three tf32 products (x_hi y_hi + x_hi y_lo + x_lo y_hi) instead.
+// mma.sync rather than tcgen05: the rows of a chunk are a few dozen tiles per layer, about a tenth of the chunk's
+// arithmetic, and the score tile needs a tanh and an exponential per element between the two products, which keeps it in
+// registers here.  A tile's P.V goes into fresh accumulators and is added to the running output in fp32 with the
+// rescaling that the online soft-max needs anyway, so the tensor core's round-to-zero sums stay a few instructions long.
+// 1B shape, fp16 cache, 1024 rows of 32 prompts x 512: see the figures at launch_attn_prefill.
+#include "attn_prefill.cuh"
+
+namespace ab {
+
+constexpr float AP_NEG = -1.0e30f;
+
+// ---- QK-norm + RoPE + append: one warp per (row, head); the arithmetic of k_attention's row prologue ----------------
+template <typename T, int HD>
+__global__ void __launch_bounds__(256) k_qkv_prep(const AttnPrefillArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t lane = threadIdx.x & 31, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, per_row = a.n_head + 2 * a.geo.n_kv;
+    if (w >= a.n_rows * per_row) return;
+    const uint32_t r = w / per_row, h = w % per_row;
+    const bool is_q = h < a.n_head, is_v = h >= a.n_head + a.geo.n_kv;
+    const int32_t p = a.row_pos[r];
+    float* src = a.qkv + (size_t)r * a.qkv_ld + (size_t)h * HD;
+    T* dst = nullptr;
+    if (!is_q) {
+        const uint32_t page_no = (uint32_t)p / a.geo.page;
+        const int32_t page_id = page_no < a.geo.max_pages ? a.block_table[(size_t)a.row_seq[r] * a.geo.max_pages + page_no] : -1;
+        if (page_id < 0 || (uint32_t)p >= a.n_pos) { if (lane == 0) atomicOr(a.err, DEVERR_OOB_MAP); return; }
+        dst = reinterpret_cast<T*>(a.kv_pool) + kv_index(a.geo, (uint32_t)page_id, a.layer, is_v ? 1u : 0u, (h - a.n_head) % a.geo.n_kv, (uint32_t)p % a.geo.page);
+    }
+    if (is_v) {
+        for (uint32_t i = lane; i < HD; i += 32) st_kv(dst + i, src[i]);
+        return;
+    }
+    constexpr uint32_t half = HD / 2;
+    constexpr int NP = (HD / 2 + 31) / 32;
+    const uint32_t pp = (uint32_t)p < a.n_pos ? (uint32_t)p : a.n_pos - 1;
+    const float *ct = a.cos_t + (size_t)pp * half, *sn_t = a.sin_t + (size_t)pp * half, *wt = is_q ? a.q_norm : a.k_norm;
+    float x0[NP], x1[NP], ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < NP; ++j) {
+        const uint32_t i = lane + 32 * j;
+        x0[j] = i < half ? src[i] : 0.f;
+        x1[j] = i < half ? src[i + half] : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < NP; ++j) ss = fmaf(x0[j], x0[j], ss);
+#pragma unroll
+    for (int j = 0; j < NP; ++j) ss = fmaf(x1[j], x1[j], ss);
+    float rms = 1.f;
+    if (wt) { ss = warp_sum(ss); rms = sqrtf(ss / (float)HD + a.eps); }
+    const float rcp = __frcp_rn(rms);
+#pragma unroll
+    for (int j = 0; j < NP; ++j) {
+        const uint32_t i = lane + 32 * j;
+        if (i < half) {
+            float a0 = x0[j], a1 = x1[j];
+            if (wt) { a0 = div_by(a0, rms, rcp) * wt[i]; a1 = div_by(a1, rms, rcp) * wt[i + half]; }
+            const float c = ct[i], sn = sn_t[i];
+            const float y0 = __fsub_rn(__fmul_rn(a0, c), __fmul_rn(a1, sn)), y1 = __fadd_rn(__fmul_rn(a0, sn), __fmul_rn(a1, c));
+            if (is_q) { src[i] = y0; src[i + half] = y1; }
+            else { st_kv(dst + i, y0); st_kv(dst + i + half, y1); }
+        }
+    }
+}
+
+// ---- small helpers -------------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t ap_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ap_cp16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void ap_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void ap_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void mma_h(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_t(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void tf32_split(float x, uint32_t& hi, uint32_t& lo) {
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(x - __uint_as_float(hi)));
+}
+__device__ __forceinline__ void half_split(float x, float y, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(x, y);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h); lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// What a query row of a tile is: row r -> position r / group, head r % group of the kv head's group.
+struct ApRow { int pos; bool ok; size_t q, o; };
+__device__ __forceinline__ ApRow ap_row(const AttnPrefillArgs& a, const AttnTile& t, uint32_t kvh, uint32_t group, uint32_t r, uint32_t HD) {
+    const uint32_t tok = r / group, head = kvh * group + r % group;
+    ApRow x;
+    x.ok = tok < (uint32_t)t.n_tok && r < (uint32_t)t.n_tok * group;
+    const uint32_t tk = x.ok ? tok : 0u;
+    x.pos = t.pos + (int)tk;
+    x.q = (size_t)(t.row + tk) * a.qkv_ld + (size_t)head * HD;
+    x.o = (size_t)(t.row + tk) * a.n_head * HD + (size_t)head * HD;
+    return x;
+}
+
+// Online soft-max of one tile of scores (NT tiles of 8 positions from kv0): c becomes the probabilities, alpha the factor
+// of the rows' earlier sums.  Row h of this thread is rows g + 8 h of the warp.
+template <int NT>
+__device__ __forceinline__ void ap_softmax(float (&c)[NT][4], const AttnPrefillArgs& a, const float (&scl)[2], const int (&pos)[2], int kv0, bool edge,
+                                           float (&m)[2], float (&l)[2], float (&alpha)[2]) {
+    const int lane = threadIdx.x & 31, q = lane & 3;
+    const float rcap = a.cap > 0.f ? __frcp_rn(a.cap) : 0.f;
+    float mx[2] = {AP_NEG, AP_NEG};
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int h = e >> 1, kp = kv0 + 8 * j + 2 * q + (e & 1);
+            float s = c[j][e] * scl[h];
+            if (a.cap > 0.f) s = tanhf(div_by(s, a.cap, rcap)) * a.cap;
+            if (edge && (kp > pos[h] || (a.window > 0 && kp + (int)a.window <= pos[h]))) s = AP_NEG;
+            c[j][e] = s;
+            mx[h] = fmaxf(mx[h], s);
+        }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
+        mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
+        const float mn = fmaxf(m[h], mx[h]);
+        alpha[h] = expf(m[h] - mn);
+        m[h] = mn;
+        l[h] *= alpha[h];
+    }
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float p = c[j][e] > 0.5f * AP_NEG ? expf(c[j][e] - m[e >> 1]) : 0.f;
+            c[j][e] = p;
+            l[e >> 1] += p;
+        }
+}
+
+// ---- fp16 cache: m16n8k16, two terms on the query / probability side ------------------------------------------------
+// NW warps of 16 query rows; tiles of 64 positions.  Shared memory: the query rows' two terms, one K and one V tile; the
+// next K tile is requested when the scores are done, the next V tile after P.V.
+template <int HD, int NW>
+__global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_h(const AttnPrefillArgs a) {
+    constexpr int ROWS = NW * 16, BN = 64, NCH = HD / 8, NTH = NW * 32;
+    extern __shared__ __align__(128) uint8_t sm[];
+    __half* sQh = reinterpret_cast<__half*>(sm);
+    __half* sQl = sQh + ROWS * HD;
+    const uint32_t qh_s = ap_smem(sQh), ql_s = ap_smem(sQl), k_s = ql_s + ROWS * HD * 2, v_s = k_s + BN * HD * 2;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2;
+    pdl_launch_dependents();
+    pdl_wait();
+    const AttnTile t = a.tiles[blockIdx.x];
+    const uint32_t kvh = blockIdx.y, group = a.n_head / a.geo.n_kv;
+    const __half* pool = reinterpret_cast<const __half*>(a.kv_pool);
+    const int32_t* bt = a.block_table + (size_t)t.seq * a.geo.max_pages;
+    auto sw = [](int r, int ch) { return NCH >= 8 ? ch ^ (r & 7) : ch ^ ((r >> 1) & (NCH - 1)); };
+    const int kv_hi = t.pos + t.n_tok;                                                  // positions [.., kv_hi)
+    const int kv_lo = a.window > 0 && t.pos + 1 > (int)a.window ? (t.pos + 1 - (int)a.window) / BN * BN : 0;
+    auto load = [&](uint32_t dst, uint32_t kv, int kv0) {
+        for (int i = tid; i < BN * NCH; i += NTH) {
+            const int r = i / NCH, ch = i % NCH, p = min(kv0 + r, kv_hi - 1);
+            const uint32_t pn = (uint32_t)p / a.geo.page;
+            const int32_t page = pn < a.geo.max_pages ? max(bt[pn], 0) : 0;
+            ap_cp16(dst + (uint32_t)(r * HD + sw(r, ch) * 8) * 2u, pool + kv_index(a.geo, (uint32_t)page, a.layer, kv, kvh, (uint32_t)p % a.geo.page) + ch * 8);
+        }
+        ap_commit();
+    };
+    load(k_s, 0, kv_lo);
+    load(v_s, 1, kv_lo);
+    // this warp's query rows: power-of-two scale per row, two fp16 terms
+    float inv_row[16];
+    constexpr int EPL = HD / 32;                                                        // values per lane
+#pragma unroll
+    for (int r0 = 0; r0 < 16; r0 += 4) {
+        float x[4][EPL];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const ApRow row = ap_row(a, t, kvh, group, warp * 16 + r0 + r, HD);
+#pragma unroll
+            for (int e = 0; e < EPL; ++e) x[r][e] = row.ok ? a.qkv[row.q + lane * EPL + e] : 0.f;
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            float mxv = 0.f;
+#pragma unroll
+            for (int e = 0; e < EPL; ++e) mxv = fmaxf(mxv, fabsf(x[r][e]));
+            mxv = warp_max(mxv);
+            int ex = 0;                                                                 // largest element into [2^7, 2^8)
+            if (mxv > 0.f && mxv < 3.0e38f) ex = max(-100, min(100, 134 - (int)((__float_as_uint(mxv) >> 23) & 0xFFu)));
+            const float s = __uint_as_float((uint32_t)(127 + ex) << 23);
+            inv_row[r0 + r] = __uint_as_float((uint32_t)(127 - ex) << 23);
+            const int rr = warp * 16 + r0 + r;
+#pragma unroll
+            for (int e = 0; e < EPL; ++e) {
+                const int d = lane * EPL + e;
+                const float v = x[r][e] * s;
+                const __half h = __float2half_rn(v);
+                const int at = rr * HD + sw(rr, d >> 3) * 8 + (d & 7);
+                sQh[at] = h;
+                sQl[at] = __float2half_rn(v - __half2float(h));
+            }
+        }
+    }
+    float scl[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        float v = 0.f;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) v = r == g ? inv_row[8 * h + r] : v;
+        scl[h] = v * a.scale;
+    }
+    const ApRow row0 = ap_row(a, t, kvh, group, warp * 16 + g, HD), row1 = ap_row(a, t, kvh, group, warp * 16 + g + 8, HD);
+    const int pos[2] = {row0.pos, row1.pos};
+    // the warp's range of positions, to leave out tiles that it does not attend to
+    const int tok_lo = (warp * 16) / (int)group, tok_hi = min((warp * 16 + 15) / (int)group, t.n_tok - 1);
+    const bool live = tok_lo < t.n_tok;
+    const int p_lo = t.pos + tok_lo, p_hi = t.pos + tok_hi;
+    float o[HD / 8][4], m[2] = {AP_NEG, AP_NEG}, l[2] = {0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < HD / 8; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
+
+    for (int kv0 = kv_lo; kv0 < kv_hi; kv0 += BN) {
+        const bool work = live && kv0 <= p_hi && !(a.window > 0 && kv0 + BN - 1 + (int)a.window <= p_lo);
+        const bool edge = kv0 + BN - 1 > p_lo || (a.window > 0 && kv0 + (int)a.window <= p_hi);
+        float c[8][4], alpha[2] = {1.f, 1.f};
+        ap_wait<1>();
+        __syncthreads();
+        if (work) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) c[j][e] = 0.f;
+#pragma unroll 2
+            for (int k = 0; k < HD / 16; ++k) {
+                uint32_t qh[4], ql[4];
+                const int qr = warp * 16 + (lane & 15), qc = 2 * k + (lane >> 4);
+                const uint32_t qo = (uint32_t)(qr * HD + sw(qr, qc) * 8) * 2u;
+                ldsm4(qh_s + qo, qh);
+                ldsm4(ql_s + qo, ql);
+#pragma unroll
+                for (int n = 0; n < 4; ++n) {
+                    uint32_t b[4];
+                    const int kr = n * 16 + (lane >> 4) * 8 + (lane & 7), kc = 2 * k + ((lane >> 3) & 1);
+                    ldsm4(k_s + (uint32_t)(kr * HD + sw(kr, kc) * 8) * 2u, b);
+                    mma_h(c[2 * n], ql, b[0], b[1]); mma_h(c[2 * n + 1], ql, b[2], b[3]);
+                    mma_h(c[2 * n], qh, b[0], b[1]); mma_h(c[2 * n + 1], qh, b[2], b[3]);
+                }
+            }
+        }
+        __syncthreads();
+        if (kv0 + BN < kv_hi) load(k_s, 0, kv0 + BN); else ap_commit();
+        uint32_t ph[4][4], pl[4][4];
+        if (work) {
+            ap_softmax<8>(c, a, scl, pos, kv0, edge, m, l, alpha);
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+#pragma unroll
+                for (int f = 0; f < 4; ++f) {           // times 256: the low terms stay clear of the fp16 subnormals
+                    const float* p = &c[2 * s + (f >> 1)][2 * (f & 1)];
+                    half_split(p[0] * 256.f, p[1] * 256.f, ph[s][f], pl[s][f]);
+                }
+        }
+        ap_wait<1>();
+        __syncthreads();
+        if (work) {
+            constexpr int DC = HD == 256 ? 32 : HD >= 64 ? 64 : HD;     // dims per round: what the registers beside `o` allow
+#pragma unroll
+            for (int d0 = 0; d0 < HD; d0 += DC) {
+                float acc[DC / 8][4];
+#pragma unroll
+                for (int j = 0; j < DC / 8; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+#pragma unroll
+                    for (int n = 0; n < DC / 16; ++n) {
+                        uint32_t b[4];
+                        const int vr = s * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), vc = d0 / 8 + 2 * n + (lane >> 4);
+                        ldsm4t(v_s + (uint32_t)(vr * HD + sw(vr, vc) * 8) * 2u, b);
+                        mma_h(acc[2 * n], pl[s], b[0], b[1]); mma_h(acc[2 * n + 1], pl[s], b[2], b[3]);
+                        mma_h(acc[2 * n], ph[s], b[0], b[1]); mma_h(acc[2 * n + 1], ph[s], b[2], b[3]);
+                    }
+#pragma unroll
+                for (int j = 0; j < DC / 8; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) o[d0 / 8 + j][e] = fmaf(o[d0 / 8 + j][e], alpha[e >> 1], acc[j][e]);
+            }
+        }
+        __syncthreads();
+        if (kv0 + BN < kv_hi) load(v_s, 1, kv0 + BN); else ap_commit();
+    }
+    ap_wait<0>();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
+        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
+        const ApRow& r = h ? row1 : row0;
+        if (!r.ok) continue;
+        const float d = l[h] * 256.f, rd = __frcp_rn(d);
+#pragma unroll
+        for (int j = 0; j < HD / 8; ++j)
+            *reinterpret_cast<float2*>(a.out + r.o + 8 * j + 2 * (lane & 3)) = make_float2(div_by(o[j][2 * h], d, rd), div_by(o[j][2 * h + 1], d, rd));
+    }
+}
+
+// ---- fp32 cache: m16n8k8 tf32, three products per pair --------------------------------------------------------------
+// Operands stay fp32 in shared memory (rows padded by 4 floats: the fragment reads below are free of bank conflicts) and
+// are split into two tf32 terms as they are read.  Tiles of 32 positions.
+template <int HD, int NW>
+__global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_f(const AttnPrefillArgs a) {
+    constexpr int ROWS = NW * 16, BN = 32, LD = HD + 4, NTH = NW * 32;
+    extern __shared__ __align__(128) uint8_t sm[];
+    float *sQ = reinterpret_cast<float*>(sm), *sK = sQ + ROWS * LD, *sV = sK + BN * LD;
+    const uint32_t k_s = ap_smem(sK), v_s = ap_smem(sV);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+    pdl_launch_dependents();
+    pdl_wait();
+    const AttnTile t = a.tiles[blockIdx.x];
+    const uint32_t kvh = blockIdx.y, group = a.n_head / a.geo.n_kv;
+    const float* pool = reinterpret_cast<const float*>(a.kv_pool);
+    const int32_t* bt = a.block_table + (size_t)t.seq * a.geo.max_pages;
+    const int kv_hi = t.pos + t.n_tok;
+    const int kv_lo = a.window > 0 && t.pos + 1 > (int)a.window ? (t.pos + 1 - (int)a.window) / BN * BN : 0;
+    auto load = [&](uint32_t dst, uint32_t kv, int kv0) {
+        for (int i = tid; i < BN * (HD / 4); i += NTH) {
+            const int r = i / (HD / 4), ch = i % (HD / 4), p = min(kv0 + r, kv_hi - 1);
+            const uint32_t pn = (uint32_t)p / a.geo.page;
+            const int32_t page = pn < a.geo.max_pages ? max(bt[pn], 0) : 0;
+            ap_cp16(dst + (uint32_t)(r * LD + ch * 4) * 4u, pool + kv_index(a.geo, (uint32_t)page, a.layer, kv, kvh, (uint32_t)p % a.geo.page) + ch * 4);
+        }
+        ap_commit();
+    };
+    load(k_s, 0, kv_lo);
+    load(v_s, 1, kv_lo);
+#pragma unroll 4
+    for (int r = 0; r < 16; ++r) {
+        const ApRow row = ap_row(a, t, kvh, group, warp * 16 + r, HD);
+#pragma unroll
+        for (int d = lane; d < HD; d += 32) sQ[(warp * 16 + r) * LD + d] = row.ok ? a.qkv[row.q + d] : 0.f;
+    }
+    const float scl[2] = {a.scale, a.scale};
+    const ApRow row0 = ap_row(a, t, kvh, group, warp * 16 + g, HD), row1 = ap_row(a, t, kvh, group, warp * 16 + g + 8, HD);
+    const int pos[2] = {row0.pos, row1.pos};
+    const int tok_lo = (warp * 16) / (int)group, tok_hi = min((warp * 16 + 15) / (int)group, t.n_tok - 1);
+    const bool live = tok_lo < t.n_tok;
+    const int p_lo = t.pos + tok_lo, p_hi = t.pos + tok_hi;
+    float o[HD / 8][4], m[2] = {AP_NEG, AP_NEG}, l[2] = {0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < HD / 8; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
+
+    for (int kv0 = kv_lo; kv0 < kv_hi; kv0 += BN) {
+        const bool work = live && kv0 <= p_hi && !(a.window > 0 && kv0 + BN - 1 + (int)a.window <= p_lo);
+        const bool edge = kv0 + BN - 1 > p_lo || (a.window > 0 && kv0 + (int)a.window <= p_hi);
+        float c[4][4], alpha[2] = {1.f, 1.f};
+        ap_wait<1>();
+        __syncthreads();
+        if (work) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) c[j][e] = 0.f;
+#pragma unroll 2
+            for (int k = 0; k < HD; k += 8) {
+                const float* qp = sQ + (warp * 16 + g) * LD + k + q;
+                uint32_t ah[4], al[4];
+                tf32_split(qp[0], ah[0], al[0]); tf32_split(qp[8 * LD], ah[1], al[1]);
+                tf32_split(qp[4], ah[2], al[2]); tf32_split(qp[8 * LD + 4], ah[3], al[3]);
+#pragma unroll
+                for (int n = 0; n < 4; ++n) {
+                    const float* kp = sK + (n * 8 + g) * LD + k + q;
+                    uint32_t b0h, b0l, b1h, b1l;
+                    tf32_split(kp[0], b0h, b0l); tf32_split(kp[4], b1h, b1l);
+                    mma_t(c[n], al, b0h, b1h); mma_t(c[n], ah, b0l, b1l); mma_t(c[n], ah, b0h, b1h);
+                }
+            }
+        }
+        __syncthreads();
+        if (kv0 + BN < kv_hi) load(k_s, 0, kv0 + BN); else ap_commit();
+        if (work) ap_softmax<4>(c, a, scl, pos, kv0, edge, m, l, alpha);
+        ap_wait<1>();
+        __syncthreads();
+        if (work) {
+            // the order of the positions inside a step of 8 is free: slots t and t + 4 are positions 2 t and 2 t + 1, which is
+            // how the scores lie in the registers
+            uint32_t ph[4][4], pl[4][4];
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                tf32_split(c[s][0], ph[s][0], pl[s][0]); tf32_split(c[s][2], ph[s][1], pl[s][1]);
+                tf32_split(c[s][1], ph[s][2], pl[s][2]); tf32_split(c[s][3], ph[s][3], pl[s][3]);
+            }
+            constexpr int DC = HD >= 64 ? 64 : HD;
+#pragma unroll
+            for (int d0 = 0; d0 < HD; d0 += DC) {
+                float acc[DC / 8][4];
+#pragma unroll
+                for (int j = 0; j < DC / 8; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+#pragma unroll
+                    for (int n = 0; n < DC / 8; ++n) {
+                        const float* vp = sV + (s * 8 + 2 * q) * LD + d0 + n * 8 + g;
+                        uint32_t b0h, b0l, b1h, b1l;
+                        tf32_split(vp[0], b0h, b0l); tf32_split(vp[LD], b1h, b1l);
+                        mma_t(acc[n], pl[s], b0h, b1h); mma_t(acc[n], ph[s], b0l, b1l); mma_t(acc[n], ph[s], b0h, b1h);
+                    }
+#pragma unroll
+                for (int j = 0; j < DC / 8; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) o[d0 / 8 + j][e] = fmaf(o[d0 / 8 + j][e], alpha[e >> 1], acc[j][e]);
+            }
+        }
+        __syncthreads();
+        if (kv0 + BN < kv_hi) load(v_s, 1, kv0 + BN); else ap_commit();
+    }
+    ap_wait<0>();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
+        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
+        const ApRow& r = h ? row1 : row0;
+        if (!r.ok) continue;
+        const float rd = __frcp_rn(l[h]);
+#pragma unroll
+        for (int j = 0; j < HD / 8; ++j)
+            *reinterpret_cast<float2*>(a.out + r.o + 8 * j + 2 * q) = make_float2(div_by(o[j][2 * h], l[h], rd), div_by(o[j][2 * h + 1], l[h], rd));
+    }
+}
+
+// ---- host ----------------------------------------------------------------------------------------------------------
+template <typename T>
+static int prep_t(const AttnPrefillArgs& a, cudaStream_t stream, bool pdl) {
+    const uint32_t warps = a.n_rows * (a.n_head + 2 * a.geo.n_kv);
+    const dim3 grid((warps + 7) / 8);
+    switch (a.head_dim) {
+    case 32: launch_k(k_qkv_prep<T, 32>, grid, dim3(256), 0, stream, pdl, a); break;
+    case 64: launch_k(k_qkv_prep<T, 64>, grid, dim3(256), 0, stream, pdl, a); break;
+    case 128: launch_k(k_qkv_prep<T, 128>, grid, dim3(256), 0, stream, pdl, a); break;
+    default: launch_k(k_qkv_prep<T, 256>, grid, dim3(256), 0, stream, pdl, a); break;
+    }
+    count_launch();
+    return check_launch("qkv_prep");
+}
+int launch_qkv_prep(const AttnPrefillArgs& a, bool kv_half, cudaStream_t stream, bool pdl) {
+    return kv_half ? prep_t<__half>(a, stream, pdl) : prep_t<float>(a, stream, pdl);
+}
+
+template <int HD, int NW>
+static int attn_t(const AttnPrefillArgs& a, bool kv_half, cudaStream_t stream, bool pdl) {
+    constexpr size_t smem_h = (size_t)(2 * NW * 16 + 2 * 64) * HD * 2, smem_f = (size_t)(NW * 16 + 2 * 32) * (HD + 4) * 4;
+    void (*k)(const AttnPrefillArgs) = kv_half ? k_attn_prefill_h<HD, NW> : k_attn_prefill_f<HD, NW>;
+    const size_t smem = kv_half ? smem_h : smem_f;
+    static bool set[2] = {false, false};
+    if (!set[kv_half]) {
+        if (cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+            return fail(ADAMAH_ERR_BACKEND, "attn_prefill: cannot raise the shared-memory limit");
+        set[kv_half] = true;
+    }
+    launch_k(k, dim3(a.n_tiles, a.geo.n_kv), dim3(NW * 32), smem, stream, pdl, a);
+    count_launch();
+    return check_launch("attn_prefill");
+}
+template <int HD>
+static int attn_r(const AttnPrefillArgs& a, bool kv_half, uint32_t rows, cudaStream_t stream, bool pdl) {
+    return rows == 128 ? attn_t<HD, 8>(a, kv_half, stream, pdl) : attn_t<HD, 4>(a, kv_half, stream, pdl);
+}
+int launch_attn_prefill(const AttnPrefillArgs& a, bool kv_half, uint32_t tile_rows, cudaStream_t stream, bool pdl) {
+    switch (a.head_dim) {
+    case 32: return attn_r<32>(a, kv_half, tile_rows, stream, pdl);
+    case 64: return attn_r<64>(a, kv_half, tile_rows, stream, pdl);
+    case 128: return attn_r<128>(a, kv_half, tile_rows, stream, pdl);
+    default: return attn_r<256>(a, kv_half, tile_rows, stream, pdl);
+    }
+}
+
+}  // namespace ab

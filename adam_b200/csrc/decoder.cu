@@ -18,7 +18,9 @@
 #include "gemm_tc.cuh"
 #include "token.cuh"
 #include "blocks8.cuh"
+#include "attn_prefill.cuh"
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <vector>
@@ -44,6 +46,9 @@ struct Layer {
     const uint8_t* qkv_tiled;   // row-tiled copy of the q,k,v rows as one tensor
 };
 
+// One pass of prefill: rows (sequence, position) of the plan and the attention tiles they are cut into.
+struct PrefillChunk { uint32_t n_rows, n_tiles, tile_rows; const int32_t *row_seq, *row_pos; const AttnTile* tiles; };
+
 struct Decoder {
     bool used;
     adam_b200_decoder_desc d;
@@ -57,8 +62,10 @@ struct Decoder {
     void* kv_pool; size_t page_elems;
     float *hbuf[2], *qkv, *attn_out, *proj, *act, *logits; int h_final;
     float *part_o, *part_ml; unsigned int* attn_ticket; uint32_t n_splits;
-    int32_t *row_seq, *row_pos; // chunked prefill: (sequence, position) of every row of the chunk
-    uint32_t rows_cap;          // rows the activation buffers hold: max(max_batch, PREFILL_ROWS)
+    // chunked prefill: what the rows of all chunks are (device copy and pinned source of one call; see PrefillPlan)
+    uint8_t *plan, *plan_pin; size_t plan_cap; cudaEvent_t plan_read;
+    std::vector<PrefillChunk> chunks; const int32_t* plan_n;
+    uint32_t rows_cap;          // rows the activation buffers hold
     std::vector<uint32_t> hpos, hplen, hres;   // host mirror of positions, prompt lengths and reserved tokens (argument checks)
     std::vector<int32_t> hbt;            // host mirror of the block table
     int32_t* tok_ring[4]; cudaEvent_t tok_event[4]; uint32_t tok_next;   // pinned slots for asynchronous token reads
@@ -208,8 +215,7 @@ __global__ void __launch_bounds__(256) k_attention(const float* __restrict__ qkv
                                                    const int32_t* __restrict__ block_table, const int32_t* __restrict__ pos,
                                                    uint32_t n_head, uint32_t layer, uint32_t window, float scale, float cap,
                                                    float* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
-                                                   unsigned int* __restrict__ ticket, uint32_t n_splits_max, uint32_t hpc,
-                                                   const int32_t* __restrict__ row_seq, const int32_t* __restrict__ row_pos, uint32_t* err STEP_TRACE_PARAM) {
+                                                   unsigned int* __restrict__ ticket, uint32_t n_splits_max, uint32_t hpc, uint32_t* err STEP_TRACE_PARAM) {
 #ifdef ADAM_B200_STEP_TRACE
 #define AT_STAMP(slot) do { if (threadIdx.x == 0 && blockIdx.z == 0 && (blockIdx.y * gridDim.x + blockIdx.x) < 32) STEP_STAMP(trace, (blockIdx.y * gridDim.x + blockIdx.x) * 8 + (slot)); } while (0)
 #else
@@ -220,9 +226,6 @@ __global__ void __launch_bounds__(256) k_attention(const float* __restrict__ qkv
     // through CTA 0's shared memory instead of global memory, a ticket and the last CTA to arrive.
     const bool cmerge = n_splits_max == 0;
     if (cmerge) cluster_arrive();               // "this CTA runs": waited for before the first store into CTA 0
-    // row_seq / row_pos != NULL: chunked prefill.  Row b of qkv/out belongs to sequence row_seq[b] at position
-    // row_pos[b], and the keys and values of the whole chunk are already in the cache (k_kv_append ran before).
-    const bool appended = row_pos != nullptr;
     const uint32_t cpc_min = (hpc >> 16) ? (hpc >> 16) : ATTN_CHUNKS_PER_CTA;     // chunks per CTA before another CTA joins
     hpc &= 0xFFFFu;
     T* __restrict__ kv_pool = reinterpret_cast<T*>(kv_pool_v);
@@ -245,8 +248,7 @@ __global__ void __launch_bounds__(256) k_attention(const float* __restrict__ qkv
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // The block table is written by the host before the step's first kernel, so it can be
     // read ahead of the dependency wait: up to 128 entries sit in registers across the warp.
-    const uint32_t sq = row_seq ? (uint32_t)row_seq[b] : b;
-    const int32_t* bt = block_table + (size_t)sq * geo.max_pages;
+    const int32_t* bt = block_table + (size_t)b * geo.max_pages;
     const bool bt_regs = geo.max_pages <= 128;
     int32_t btr[4];
 #pragma unroll
@@ -273,11 +275,8 @@ __global__ void __launch_bounds__(256) k_attention(const float* __restrict__ qkv
     // Positions only change in the step's last kernel, and the step's first kernel is
     // launched with a full dependency on it, so the position, and everything in the cache
     // older than this step, can be read ahead of the wait as well.
-    // In chunked prefill the chunk's own keys and values were written by the kernel just before
-    // this one, so the wait comes first there.
-    if (appended) { pdl_launch_dependents(); pdl_wait(); }
     const uint32_t hd = HD, half = HD / 2, gs = hpc;
-    const int32_t p = appended ? row_pos[b] : pos[b];
+    const int32_t p = pos[b];
     const uint32_t seq = (uint32_t)p + 1;
     const uint32_t start = (window > 0 && seq > window) ? seq - window : 0;
     const uint32_t c_first = start / CP, n_chunks = (seq - 1) / CP - c_first + 1;
@@ -285,8 +284,8 @@ __global__ void __launch_bounds__(256) k_attention(const float* __restrict__ qkv
     if (split >= n_act) { if (cmerge) { cluster_wait(); cluster_arrive(); } return; }
     const uint32_t cpc = (n_chunks + n_act - 1) / n_act;
     const uint32_t c0 = min(c_first + split * cpc, c_first + n_chunks), c1 = min(c_first + n_chunks, c0 + cpc);
-    const uint32_t c_new = appended ? 0xFFFFFFFFu : (uint32_t)p / CP;      // chunk whose newest row comes from this step's q/k/v
-    const bool owner = !appended && c_new >= c0 && c_new < c1;
+    const uint32_t c_new = (uint32_t)p / CP;      // chunk whose newest row comes from this step's q/k/v
+    const bool owner = c_new >= c0 && c_new < c1;
     float* s_q = sm;                            // [gs][hd]
     float* s_kn = s_q + gs * hd;                // [hd] newest key (as stored)
     float* s_vn = s_kn + hd;                    // [hd] newest value (as stored)
@@ -344,7 +343,8 @@ __global__ void __launch_bounds__(256) k_attention(const float* __restrict__ qkv
         sn[j] = i < half ? st[i] : 0.f;
     }
     AT_STAMP(1);
-    if (!appended) { pdl_launch_dependents(); pdl_wait(); }     // this step's q/k/v rows come from the previous kernel
+    pdl_launch_dependents();
+    pdl_wait();                                 // this step's q/k/v rows come from the previous kernel
     AT_STAMP(2);
     const float* row_q = qkv + (size_t)b * qkv_ld + (size_t)head0 * hd;
     const float* row_k = qkv + (size_t)b * qkv_ld + (size_t)n_head * hd + (size_t)kvh * hd;
@@ -639,77 +639,12 @@ __global__ void __launch_bounds__(256) k_attention(const float* __restrict__ qkv
     if (tid == 0) *tkt = 0u;
 }
 
-// Chunked prefill: QK-norm + RoPE of the key row and append of key and value to the paged
-// cache for every row of the chunk, one warp per (row, kv head, K|V); the same arithmetic as
-// the key/value part of k_attention.
-template <typename T, int HD>
-__global__ void __launch_bounds__(256) k_kv_append(const float* __restrict__ qkv, uint32_t qkv_ld, const float* __restrict__ k_norm, float eps,
-                                                   const float* __restrict__ cos_t, const float* __restrict__ sin_t, uint32_t n_pos,
-                                                   void* __restrict__ kv_pool_v, KvGeom geo, const int32_t* __restrict__ block_table,
-                                                   const int32_t* __restrict__ row_seq, const int32_t* __restrict__ row_pos,
-                                                   uint32_t n_rows, uint32_t n_head, uint32_t layer, uint32_t* err) {
-    T* __restrict__ kv_pool = reinterpret_cast<T*>(kv_pool_v);
-    pdl_launch_dependents();
-    pdl_wait();
-    const uint32_t lane = threadIdx.x & 31, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (w >= n_rows * geo.n_kv * 2) return;
-    const uint32_t kv = w & 1u, kvh = (w >> 1) % geo.n_kv, r = (w >> 1) / geo.n_kv;
-    const uint32_t sq = (uint32_t)row_seq[r];
-    const int32_t p = row_pos[r];
-    const uint32_t page_no = (uint32_t)p / geo.page;
-    const int32_t page_id = page_no < geo.max_pages ? block_table[(size_t)sq * geo.max_pages + page_no] : -1;
-    if (page_id < 0 || (uint32_t)p >= n_pos) { if (lane == 0) atomicOr(err, DEVERR_OOB_MAP); return; }
-    T* dst = kv_pool + kv_index(geo, (uint32_t)page_id, layer, kv, kvh, (uint32_t)p % geo.page);
-    const float* src = qkv + (size_t)r * qkv_ld + (size_t)n_head * HD + (size_t)kv * geo.n_kv * HD + (size_t)kvh * HD;
-    if (kv == 1) {
-        for (uint32_t i = lane; i < HD; i += 32) st_kv(dst + i, src[i]);
-        return;
-    }
-    constexpr uint32_t half = HD / 2;
-    constexpr int NP = (HD / 2 + 31) / 32;
-    const float* ct = cos_t + (size_t)p * half;
-    const float* st = sin_t + (size_t)p * half;
-    float x0[NP], x1[NP];
-    float ss = 0.f;
-#pragma unroll
-    for (int j = 0; j < NP; ++j) {
-        const uint32_t i = lane + 32 * j;
-        x0[j] = i < half ? src[i] : 0.f;
-        x1[j] = i < half ? src[i + half] : 0.f;
-    }
-#pragma unroll
-    for (int j = 0; j < NP; ++j) ss = fmaf(x0[j], x0[j], ss);
-#pragma unroll
-    for (int j = 0; j < NP; ++j) ss = fmaf(x1[j], x1[j], ss);
-    float rms = 1.f;
-    if (k_norm) { ss = warp_sum(ss); rms = sqrtf(ss / (float)HD + eps); }
-    const float rcp = __frcp_rn(rms);
-#pragma unroll
-    for (int j = 0; j < NP; ++j) {
-        const uint32_t i = lane + 32 * j;
-        if (i < half) {
-            float a0 = x0[j], a1 = x1[j];
-            if (k_norm) { a0 = div_by(a0, rms, rcp) * k_norm[i]; a1 = div_by(a1, rms, rcp) * k_norm[i + half]; }
-            const float c = ct[i], sn = st[i];
-            st_kv(dst + i, __fsub_rn(__fmul_rn(a0, c), __fmul_rn(a1, sn)));
-            st_kv(dst + i + half, __fadd_rn(__fmul_rn(a0, sn), __fmul_rn(a1, c)));
-        }
-    }
-}
-
-// Chunked prefill: row r = (sequence r / T, position pos[sequence] + r % T).
-__global__ void k_prefill_rows(const int32_t* __restrict__ pos, uint32_t batch, uint32_t T, int32_t* __restrict__ row_seq, int32_t* __restrict__ row_pos) {
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= batch * T) return;
-    const uint32_t s = r / T;
-    row_seq[r] = (int32_t)s;
-    row_pos[r] = pos[s] + (int32_t)(r % T);
-}
-__global__ void k_advance_n(int32_t* __restrict__ pos, uint32_t batch, int32_t n) {
+// End of a prefill: every sequence moves on by its own number of tokens.
+__global__ void k_advance_by(int32_t* __restrict__ pos, const int32_t* __restrict__ n, uint32_t batch) {
     pdl_launch_dependents();
     pdl_wait();
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b < batch) pos[b] += n;
+    if (b < batch) pos[b] += n[b];
 }
 
 // End of a step: advance positions; when the LM head ran, log the sampled token.
@@ -755,9 +690,11 @@ static void destroy(Decoder* D) {
     free_token_kernel(D);
     for (int i = 0; i < 4; ++i) { if (D->tok_ring[i]) cudaFreeHost(D->tok_ring[i]); if (D->tok_event[i]) cudaEventDestroy(D->tok_event[i]); }
     void* ptrs[] = {D->pos, D->cur_tok, D->cur_val, D->prompt_len, D->prompt_tok, D->gen_log, D->block_table, D->kv_pool, D->hbuf[0], D->hbuf[1], D->qkv,
-                    D->attn_out, D->proj, D->act, D->logits, D->part_o, D->part_ml, D->attn_ticket, D->row_seq, D->row_pos,
+                    D->attn_out, D->proj, D->act, D->logits, D->part_o, D->part_ml, D->attn_ticket, D->plan,
                     D->rope_cos[0], D->rope_sin[0], D->rope_cos[1], D->rope_sin[1]};
     for (void* p : ptrs) cudaFree(p);
+    cudaFreeHost(D->plan_pin);
+    if (D->plan_read) cudaEventDestroy(D->plan_read);
     delete D;
 }
 
@@ -773,7 +710,7 @@ static size_t kv_elem_size(const adam_b200_decoder_desc& d) { return d.kv_dtype 
 
 typedef void (*AttnKernel)(const float*, uint32_t, const float*, const float*, float, const float*, const float*, uint32_t, void*, KvGeom,
                            const int32_t*, const int32_t*, uint32_t, uint32_t, uint32_t, float, float, float*, float*, float*,
-                           unsigned int*, uint32_t, uint32_t, const int32_t*, const int32_t*, uint32_t* STEP_TRACE_PARAM);
+                           unsigned int*, uint32_t, uint32_t, uint32_t* STEP_TRACE_PARAM);
 
 template <typename T, int GS>
 static AttnKernel pick_attn_hd(uint32_t hd) {
@@ -786,7 +723,7 @@ static AttnKernel pick_attn_hd(uint32_t hd) {
 }
 
 template <typename T>
-static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch, bool prefill = false) {
+static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
     const adam_b200_decoder_desc& d = D->d;
     KvGeom geo{d.n_layer, d.n_head_kv, d.head_dim, d.page_size, D->max_pages_per_seq, D->page_elems};
     const uint32_t gs = d.n_head / d.n_head_kv;
@@ -825,7 +762,7 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch, bool prefill = 
     // The kernels behind a cluster launch start later (their prologues no longer overlap it); that costs more than the merge
     // saves once the o-proj behind it has more than about a megabyte of tiles to request (27B shape, 4-way shard: 2 % slower).
     const size_t o_bytes = (size_t)ly.m[MAT_O].rows * ly.m[MAT_O].cols * 9 / 16;
-    if (cluster_env != 0 && !prefill && work <= cluster_work && reach <= 2048u && o_bytes <= (1u << 20)) {
+    if (cluster_env != 0 && work <= cluster_work && reach <= 2048u && o_bytes <= (1u << 20)) {
         struct Known { AttnKernel k; unsigned cs; };
         static Known known[16]; static int n_known = 0;
         int cs = -1;
@@ -854,8 +791,7 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch, bool prefill = 
             if (launch_k_cluster(kern, grid, dim3(256), smem_for((unsigned)cs), g.stream, g.pdl, (unsigned)cs, D->qkv, qkv_ld, ly.norm[NORM_Q], ly.norm[NORM_K], d.norm_eps,
                                  D->rope_cos[which], D->rope_sin[which], D->rope_pos[which],
                                  D->kv_pool, geo, D->block_table, D->pos, d.n_head, L, window, d.attn_scale,
-                                 d.attn_softcap, D->attn_out, D->part_o, D->part_ml, D->attn_ticket, 0u, hpc | (cpc << 16),
-                                 (const int32_t*)nullptr, (const int32_t*)nullptr, g.dev_err STEP_TRACE_ARG((g_step_trace && L == g_step_trace_layer) ? g_step_trace + 4 * 64 : nullptr)) != cudaSuccess)
+                                 d.attn_softcap, D->attn_out, D->part_o, D->part_ml, D->attn_ticket, 0u, hpc | (cpc << 16), g.dev_err STEP_TRACE_ARG((g_step_trace && L == g_step_trace_layer) ? g_step_trace + 4 * 64 : nullptr)) != cudaSuccess)
                 return fail(ADAMAH_ERR_BACKEND, "attention: cluster launch failed: %s", cudaGetErrorString(cudaGetLastError()));
             count_launch();
             return ADAMAH_OK;
@@ -865,8 +801,7 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch, bool prefill = 
     launch_k(kern, grid, dim3(256), smem, g.stream, g.pdl, D->qkv, qkv_ld, ly.norm[NORM_Q], ly.norm[NORM_K], d.norm_eps,
              D->rope_cos[which], D->rope_sin[which], D->rope_pos[which],
              D->kv_pool, geo, D->block_table, D->pos, d.n_head, L, window, d.attn_scale,
-             d.attn_softcap, D->attn_out, D->part_o, D->part_ml, D->attn_ticket, D->n_splits, hpc | (cpc << 16),
-             prefill ? D->row_seq : nullptr, prefill ? D->row_pos : nullptr, g.dev_err STEP_TRACE_ARG((g_step_trace && L == g_step_trace_layer && !prefill) ? g_step_trace + 4 * 64 : nullptr));
+             d.attn_softcap, D->attn_out, D->part_o, D->part_ml, D->attn_ticket, D->n_splits, hpc | (cpc << 16), g.dev_err STEP_TRACE_ARG((g_step_trace && L == g_step_trace_layer) ? g_step_trace + 4 * 64 : nullptr));
     count_launch();
     return ADAMAH_OK;
 }
@@ -1235,12 +1170,11 @@ extern "C" int adam_b200_decoder_create(const adam_b200_decoder_desc* desc, uint
     DALLOC(D->hbuf[0], R * E * 4); DALLOC(D->hbuf[1], R * E * 4); DALLOC(D->qkv, R * (q_dim + 2 * k_dim) * 4);
     DALLOC(D->attn_out, R * q_dim * 4); DALLOC(D->proj, R * E * 4);
     DALLOC(D->act, R * d.n_ff * 4); DALLOC(D->logits, B * (size_t)d.n_vocab * 4);
-    DALLOC(D->part_o, R * d.n_head_kv * D->n_splits * gs * d.head_dim * 4);
-    DALLOC(D->part_ml, R * d.n_head_kv * D->n_splits * gs * 2 * 4);
-    DALLOC(D->attn_ticket, R * d.n_head * 4);
-    DALLOC(D->row_seq, R * 4); DALLOC(D->row_pos, R * 4);
+    DALLOC(D->part_o, B * d.n_head_kv * D->n_splits * gs * d.head_dim * 4);
+    DALLOC(D->part_ml, B * d.n_head_kv * D->n_splits * gs * 2 * 4);
+    DALLOC(D->attn_ticket, B * d.n_head * 4);
 #undef DALLOC
-    cudaMemsetAsync(D->attn_ticket, 0, R * d.n_head * 4, g.stream);
+    cudaMemsetAsync(D->attn_ticket, 0, B * d.n_head * 4, g.stream);
     cudaMemsetAsync(D->pos, 0, B * 4, g.stream);
     cudaMemsetAsync(D->cur_tok, 0, B * 4, g.stream);
     cudaMemsetAsync(D->cur_val, 0, B * 4, g.stream);
@@ -1565,51 +1499,87 @@ extern "C" int adam_b200_decoder_set_tokens(uint32_t id, const int32_t* tokens) 
     return ADAMAH_OK;
 }
 
-// Chunked prefill: consume the next n_tokens prompt tokens of every active sequence, several
-// positions per pass: the rows of a chunk (sequence x token) go through the GEMVs together as
-// batch rows, their keys and values are appended first and attention then reads the whole
-// chunk from the cache (causal by position).  No LM head: the token after the prompt's last one
-// comes from a normal step.  Every sequence must still have n_tokens prompt tokens ahead.
-// Same results as n_tokens single steps (the reference consumes prompts token by token,
-// engine.py:3838-3847).
-template <typename T>
-static int launch_kv_append_t(Decoder* D, uint32_t L, uint32_t rows) {
+// Chunked prefill: consume the next n_tokens[b] prompt tokens of every active sequence, many rows (sequence, position)
+// per pass: the rows of a chunk go through the products together, their keys and values are appended first and attention
+// then reads the whole chunk from the cache (causal by position).  No LM head: the token after a prompt's last one comes
+// from a normal step.  Same results as single steps (the reference consumes prompts token by token, engine.py:3838-3847).
+//
+// The plan of a call lists its rows sequence by sequence, cut into chunks of equal size, and each sequence's run inside a
+// chunk is cut into attention tiles; one copy takes it to the device.
+static int plan_prefill(Decoder* D, const uint32_t* n_tokens) {
     const adam_b200_decoder_desc& d = D->d;
-    KvGeom geo{d.n_layer, d.n_head_kv, d.head_dim, d.page_size, D->max_pages_per_seq, D->page_elems};
-    const int which = is_global_layer(d, L) ? 1 : 0;
-    const uint32_t warps = rows * d.n_head_kv * 2, qkv_ld = (d.n_head + 2 * d.n_head_kv) * d.head_dim;
-    const dim3 grid((warps * 32 + 255) / 256);
-    const Layer& ly = D->layers[L];
-#define KVA(HD_) launch_k(k_kv_append<T, HD_>, grid, dim3(256), 0, g.stream, g.pdl, (const float*)D->qkv, qkv_ld, ly.norm[NORM_K], d.norm_eps, \
-        (const float*)D->rope_cos[which], (const float*)D->rope_sin[which], D->rope_pos[which], D->kv_pool, geo, (const int32_t*)D->block_table, \
-        (const int32_t*)D->row_seq, (const int32_t*)D->row_pos, rows, d.n_head, L, g.dev_err)
-    switch (d.head_dim) { case 32: KVA(32); break; case 64: KVA(64); break; case 128: KVA(128); break; default: KVA(256); break; }
-#undef KVA
-    count_launch();
+    const uint32_t group = d.n_head / d.n_head_kv;
+    uint64_t total = 0;
+    for (uint32_t b = 0; b < D->batch; ++b) total += n_tokens[b];
+    D->chunks.clear();
+    if (!total) return ADAMAH_OK;
+    const uint64_t n_chunks = (total + D->rows_cap - 1) / D->rows_cap;
+    uint64_t size = ((total + n_chunks - 1) / n_chunks + 63) / 64 * 64;
+    if (size > D->rows_cap) size = D->rows_cap;
+    std::vector<int32_t> seq, pos;
+    std::vector<AttnTile> tiles;
+    seq.reserve(total); pos.reserve(total);
+    struct Cut { uint32_t row, rows, tile, n_tiles, tile_rows; };
+    std::vector<Cut> cuts;
+    uint32_t b = 0, at = 0;                             // sequence and how many of its tokens are placed
+    while (seq.size() < total) {
+        Cut c = {(uint32_t)seq.size(), 0, (uint32_t)tiles.size(), 0, 128};
+        struct Run { uint32_t row, b, pos, n; };
+        std::vector<Run> runs;
+        while (c.rows < size && b < D->batch) {
+            const uint32_t n = std::min<uint32_t>(n_tokens[b] - at, (uint32_t)size - c.rows);
+            if (n) runs.push_back(Run{c.rows, b, D->hpos[b] + at, n});
+            for (uint32_t i = 0; i < n; ++i) { seq.push_back((int32_t)b); pos.push_back((int32_t)(D->hpos[b] + at + i)); }
+            c.rows += n; at += n;
+            if (at == n_tokens[b]) { ++b; at = 0; }
+        }
+        // 128 query rows per attention tile while that still fills the SMs (each tile of the cache is then read half as often)
+        uint32_t wide = 0;
+        for (const Run& r : runs) wide += (r.n + attn_prefill_tokens(group, 128) - 1) / attn_prefill_tokens(group, 128);
+        if (wide * d.n_head_kv < (uint32_t)g.sm_count) c.tile_rows = 64;
+        const uint32_t step = attn_prefill_tokens(group, c.tile_rows);
+        for (const Run& r : runs)
+            for (uint32_t i = 0; i < r.n; i += step)
+                tiles.push_back(AttnTile{(int32_t)(r.row + i), (int32_t)r.b, (int32_t)(r.pos + i), (int32_t)std::min(step, r.n - i)});
+        c.n_tiles = (uint32_t)tiles.size() - c.tile;
+        // the tiles with the longest reach first: they end last otherwise
+        std::sort(tiles.begin() + c.tile, tiles.end(), [](const AttnTile& x, const AttnTile& y) { return x.pos > y.pos; });
+        cuts.push_back(c);
+    }
+    const size_t o_pos = seq.size() * 4, o_tiles = (2 * seq.size() * 4 + 15) & ~(size_t)15, o_n = o_tiles + tiles.size() * sizeof(AttnTile), bytes = o_n + (size_t)D->batch * 4;
+    if (bytes > D->plan_cap) {
+        DCU(cudaStreamSynchronize(g.stream));
+        cudaFree(D->plan); cudaFreeHost(D->plan_pin);
+        D->plan = D->plan_pin = nullptr; D->plan_cap = 0;
+        const size_t cap = bytes * 2;
+        DCU(cudaMalloc((void**)&D->plan, cap));
+        DCU(cudaMallocHost((void**)&D->plan_pin, cap));
+        D->plan_cap = cap;
+    } else if (D->plan_read) DCU(cudaEventSynchronize(D->plan_read));       // the copy of the call before has left the pinned source
+    if (!D->plan_read) DCU(cudaEventCreateWithFlags(&D->plan_read, cudaEventDisableTiming));
+    memcpy(D->plan_pin, seq.data(), seq.size() * 4);
+    memcpy(D->plan_pin + o_pos, pos.data(), pos.size() * 4);
+    memcpy(D->plan_pin + o_tiles, tiles.data(), tiles.size() * sizeof(AttnTile));
+    memcpy(D->plan_pin + o_n, n_tokens, (size_t)D->batch * 4);
+    DCU(cudaMemcpyAsync(D->plan, D->plan_pin, bytes, cudaMemcpyHostToDevice, g.stream));
+    DCU(cudaEventRecord(D->plan_read, g.stream));
+    for (const Cut& c : cuts)
+        D->chunks.push_back(PrefillChunk{c.rows, c.n_tiles, c.tile_rows, (const int32_t*)D->plan + c.row, (const int32_t*)(D->plan + o_pos) + c.row,
+                                         (const AttnTile*)(D->plan + o_tiles) + c.tile});
+    D->plan_n = (const int32_t*)(D->plan + o_n);
     return ADAMAH_OK;
 }
 
-// One part of a prefill chunk of T tokens per sequence; parts as in enqueue_part (2L = attention half
-// of layer L, preceded by the row set-up and the embedding for L = 0; 2L+1 = FFN half), and part
-// 2*n_layer advances the positions by T.
-static int enqueue_prefill_part(Decoder* D, uint32_t batch, uint32_t T, uint32_t part) {
+// Part 2L / 2L+1 of one chunk: the attention half of layer L (preceded by the embedding for L = 0) / its FFN half.
+static int enqueue_prefill_part(Decoder* D, const PrefillChunk& c, uint32_t part) {
     const adam_b200_decoder_desc& d = D->d;
-    const uint32_t rows = batch * T;
+    const uint32_t rows = c.n_rows;
     const uint32_t E = d.n_embd, q_dim = d.n_head * d.head_dim, k_dim = d.n_head_kv * d.head_dim, qkv_ld = q_dim + 2 * k_dim;
     int rc;
-    if (part == 2 * d.n_layer) {
-        launch_k(k_advance_n, dim3((batch + 63) / 64), dim3(64), 0, g.stream, g.pdl, D->pos, batch, (int32_t)T);
-        count_launch();
-        return check_launch("decoder prefill");
-    }
     const uint32_t L = part / 2;
     const Layer& ly = D->layers[L];
     if (!(part & 1u)) {
-        if (L == 0) {
-            k_prefill_rows<<<(rows + 63) / 64, 64, 0, g.stream>>>(D->pos, batch, T, D->row_seq, D->row_pos);
-            count_launch();
-            launch_embed(D, rows, (const int32_t*)D->row_seq, (const int32_t*)D->row_pos);
-        }
+        if (L == 0) launch_embed(D, rows, c.row_seq, c.row_pos);
         const int cur = L == 0 ? 0 : 1;
         GemvArgs in = {};
         in.ldx = (int)E; in.eps = d.norm_eps; in.h_in = D->hbuf[cur]; in.w_pre = ly.norm[NORM_ATTN];
@@ -1626,10 +1596,17 @@ static int enqueue_prefill_part(Decoder* D, uint32_t batch, uint32_t T, uint32_t
             in2.y = D->qkv + q_dim + k_dim;
             if ((rc = gemv(ly.m[MAT_V], nullptr, in2, rows, EPI_STORE))) return rc;
         }
-        rc = d.kv_dtype == 1 ? launch_kv_append_t<__half>(D, L, rows) : launch_kv_append_t<float>(D, L, rows);
-        if (rc) return rc;
-        rc = d.kv_dtype == 1 ? launch_attn_t<__half>(D, L, rows, true) : launch_attn_t<float>(D, L, rows, true);
-        if (rc) return rc;
+        const int which = is_global_layer(d, L) ? 1 : 0;
+        AttnPrefillArgs a = {};
+        a.qkv = D->qkv; a.qkv_ld = qkv_ld; a.q_norm = ly.norm[NORM_Q]; a.k_norm = ly.norm[NORM_K]; a.eps = d.norm_eps;
+        a.cos_t = D->rope_cos[which]; a.sin_t = D->rope_sin[which]; a.n_pos = D->rope_pos[which];
+        a.kv_pool = D->kv_pool; a.geo = KvGeom{d.n_layer, d.n_head_kv, d.head_dim, d.page_size, D->max_pages_per_seq, D->page_elems};
+        a.block_table = D->block_table; a.row_seq = c.row_seq; a.row_pos = c.row_pos; a.tiles = c.tiles; a.n_tiles = c.n_tiles;
+        a.n_rows = rows; a.n_head = d.n_head; a.head_dim = d.head_dim; a.layer = L;
+        a.window = ((d.flags & 1u) && d.sliding_window > 0 && !which) ? d.sliding_window : 0;
+        a.scale = d.attn_scale; a.cap = d.attn_softcap; a.out = D->attn_out; a.err = g.dev_err;
+        if ((rc = launch_qkv_prep(a, d.kv_dtype == 1, g.stream, g.pdl))) return rc;
+        if ((rc = launch_attn_prefill(a, d.kv_dtype == 1, c.tile_rows, g.stream, g.pdl))) return rc;
         GemvArgs o = {};
         o.x = D->attn_out; o.ldx = (int)q_dim; o.y = D->proj; o.ldy = (int)E;
         if ((rc = gemv(ly.m[MAT_O], nullptr, o, rows, EPI_STORE))) return rc;
@@ -1645,32 +1622,62 @@ static int enqueue_prefill_part(Decoder* D, uint32_t batch, uint32_t T, uint32_t
     return check_launch("decoder prefill");
 }
 
-static int enqueue_prefill_chunk(Decoder* D, uint32_t batch, uint32_t T) {
-    for (uint32_t part = 0; part <= 2 * D->d.n_layer; ++part) {
-        const int rc = enqueue_prefill_part(D, batch, T, part);
-        if (rc) return rc;
-    }
-    return ADAMAH_OK;
+static void enqueue_prefill_end(Decoder* D) {
+    launch_k(k_advance_by, dim3((D->batch + 63) / 64), dim3(64), 0, g.stream, g.pdl, D->pos, D->plan_n, D->batch);
+    count_launch();
 }
 
-// One part of one prefill chunk of n_tokens (<= 64 / batch) tokens per sequence, for tensor-parallel
-// callers: parts 0 .. 2*n_layer-1 as in adam_b200_decoder_step_part (all-reduce the projection
-// buffer, batch * n_tokens rows, after each), part 2*n_layer advances the positions.
+static int check_prefill(Decoder* D, const uint32_t* n_tokens, const char* name) {
+    if (D->batch == 0) return fail(ADAMAH_ERR_INVALID, "%s: call decoder_begin first", name);
+    for (uint32_t b = 0; b < D->batch; ++b)
+        if ((uint64_t)D->hpos[b] + n_tokens[b] > D->hplen[b])
+            return fail(ADAMAH_ERR_INVALID, "%s: sequence %u has only %u prompt tokens left", name, b, D->hplen[b] - D->hpos[b]);
+    return ADAMAH_OK;
+}
+static bool pdl_allowed() {
+    static const bool allow = !(getenv("ADAM_B200_PDL") && atoi(getenv("ADAM_B200_PDL")) == 0);
+    return allow;
+}
+
+// One part of one prefill chunk of n_tokens (n_tokens * batch rows, at most what buffer 0 of
+// adam_b200_decoder_buffer_ptr holds) tokens per sequence, for tensor-parallel callers: parts 0 .. 2*n_layer-1 as in
+// adam_b200_decoder_step_part (all-reduce the projection buffer, batch * n_tokens rows, after each), part 2*n_layer
+// advances the positions.
 extern "C" int adam_b200_decoder_prefill_part(uint32_t id, uint32_t n_tokens, uint32_t part) {
     Decoder* D = get_dec(id);
     if (!D) return ADAMAH_ERR_NOT_FOUND;
-    if (D->batch == 0) return fail(ADAMAH_ERR_INVALID, "decoder_prefill_part: call decoder_begin first");
     if (part > 2 * D->d.n_layer) return fail(ADAMAH_ERR_INVALID, "decoder_prefill_part: part %u of %u", part, 2 * D->d.n_layer + 1);
-    if (n_tokens == 0 || (uint64_t)n_tokens * D->batch > D->rows_cap) return fail(ADAMAH_ERR_INVALID, "decoder_prefill_part: a chunk holds at most %u rows", D->rows_cap);
-    if (part == 0)
-        for (uint32_t b = 0; b < D->batch; ++b)
-            if ((uint64_t)D->hpos[b] + n_tokens > D->hplen[b])
-                return fail(ADAMAH_ERR_INVALID, "decoder_prefill_part: sequence %u has only %u prompt tokens left", b, D->hplen[b] - D->hpos[b]);
-    static const bool allow = !(getenv("ADAM_B200_PDL") && atoi(getenv("ADAM_B200_PDL")) == 0);
-    g.pdl = allow;
-    const int rc = enqueue_prefill_part(D, D->batch, n_tokens, part);
+    if (D->batch && (n_tokens == 0 || (uint64_t)n_tokens * D->batch > D->rows_cap)) return fail(ADAMAH_ERR_INVALID, "decoder_prefill_part: a chunk holds at most %u rows", D->rows_cap);
+    const std::vector<uint32_t> n(D->batch, n_tokens);
+    int rc = ADAMAH_OK;
+    if (part == 0 && ((rc = check_prefill(D, n.data(), "decoder_prefill_part")) || (rc = plan_prefill(D, n.data())))) return rc;
+    if (D->chunks.size() != 1 || D->chunks[0].n_rows != n_tokens * D->batch) return fail(ADAMAH_ERR_INVALID, "decoder_prefill_part: begin with part 0");
+    g.pdl = pdl_allowed();
+    if (part < 2 * D->d.n_layer) rc = enqueue_prefill_part(D, D->chunks[0], part);
+    else { enqueue_prefill_end(D); rc = check_launch("decoder prefill"); }
     g.pdl = false;
-    if (rc == ADAMAH_OK && part == 2 * D->d.n_layer) for (uint32_t& hp : D->hpos) hp += n_tokens;
+    if (rc == ADAMAH_OK && part == 2 * D->d.n_layer) { for (uint32_t& hp : D->hpos) hp += n_tokens; D->chunks.clear(); }
+    end_of_op();
+    return rc;
+}
+
+// n_tokens[b] prompt tokens of every active sequence b; none for a sequence is fine.
+extern "C" int adam_b200_decoder_prefill_ragged(uint32_t id, const uint32_t* n_tokens) {
+    Decoder* D = get_dec(id);
+    if (!D) return ADAMAH_ERR_NOT_FOUND;
+    if (!n_tokens) return fail(ADAMAH_ERR_INVALID, "decoder_prefill: null argument");
+    if (capturing()) return fail(ADAMAH_ERR_INVALID, "decoder_prefill: not allowed while a graph is being captured");
+    int rc = check_prefill(D, n_tokens, "decoder_prefill");
+    if (rc || (rc = plan_prefill(D, n_tokens))) return rc;
+    if (!D->chunks.empty()) {
+        g.pdl = pdl_allowed();
+        for (const PrefillChunk& c : D->chunks)
+            for (uint32_t part = 0; part < 2 * D->d.n_layer && rc == ADAMAH_OK; ++part) rc = enqueue_prefill_part(D, c, part);
+        if (rc == ADAMAH_OK) { enqueue_prefill_end(D); rc = check_launch("decoder prefill"); }
+        g.pdl = false;
+        D->chunks.clear();
+    }
+    if (rc == ADAMAH_OK) for (uint32_t b = 0; b < D->batch; ++b) D->hpos[b] += n_tokens[b];
     end_of_op();
     return rc;
 }
@@ -1678,26 +1685,8 @@ extern "C" int adam_b200_decoder_prefill_part(uint32_t id, uint32_t n_tokens, ui
 extern "C" int adam_b200_decoder_prefill(uint32_t id, uint32_t n_tokens) {
     Decoder* D = get_dec(id);
     if (!D) return ADAMAH_ERR_NOT_FOUND;
-    if (D->batch == 0) return fail(ADAMAH_ERR_INVALID, "decoder_prefill: call decoder_begin first");
-    if (capturing()) return fail(ADAMAH_ERR_INVALID, "decoder_prefill: not allowed while a graph is being captured");
-    for (uint32_t b = 0; b < D->batch; ++b)
-        if ((uint64_t)D->hpos[b] + n_tokens > D->hplen[b])
-            return fail(ADAMAH_ERR_INVALID, "decoder_prefill: sequence %u has only %u prompt tokens left", b, D->hplen[b] - D->hpos[b]);
-    const uint32_t t_max = D->rows_cap / D->batch;
-    if (t_max == 0) return fail(ADAMAH_ERR_INVALID, "decoder_prefill: batch larger than the row buffers");
-    static const bool allow = !(getenv("ADAM_B200_PDL") && atoi(getenv("ADAM_B200_PDL")) == 0);
-    int rc = ADAMAH_OK;
-    uint32_t left = n_tokens;
-    while (left && rc == ADAMAH_OK) {
-        const uint32_t T = left < t_max ? left : t_max;
-        g.pdl = allow;
-        rc = enqueue_prefill_chunk(D, D->batch, T);
-        g.pdl = false;
-        left -= T;
-    }
-    if (rc == ADAMAH_OK) for (uint32_t& hp : D->hpos) hp += n_tokens;
-    end_of_op();
-    return rc;
+    const std::vector<uint32_t> n(D->batch ? D->batch : 1, n_tokens);
+    return adam_b200_decoder_prefill_ragged(id, n.data());
 }
 
 // Where the time of a one-sequence step on the graph of per-operation kernels goes (diagnostics build only):
@@ -1802,7 +1791,7 @@ extern "C" int adam_b200_decoder_test_wait_expiry(uint32_t id, uint32_t wait_us)
 // Device address and size of one of the decoder's buffers, for callers that run their own
 // kernels or collectives on them (same stream, see adam_b200_set_stream):
 //   0 = projection output [rows][n_embd] f32 (what a tensor-parallel caller all-reduces; rows =
-//       batch in a decode step, batch * n_tokens in a prefill chunk; sized for max(max_batch, 64) rows)
+//       batch in a decode step, batch * n_tokens in a prefill chunk; at least max(max_batch, 64) rows)
 //   1 = current token ids [max_batch] i32     2 = their logit values [max_batch] f32
 //   3 = positions [max_batch] i32
 extern "C" int adam_b200_decoder_buffer_ptr(uint32_t id, uint32_t which, uint64_t* ptr_out, uint64_t* bytes_out) {

@@ -229,6 +229,13 @@ class ADAMEngine:
         if n_tokens > 0:
             self._check(self._lib.adam_b200_decoder_prefill(self._dec, int(n_tokens)), "adam_b200_decoder_prefill")
 
+    def prefill_prompts(self, prompts: Sequence[Sequence[int]], reuse: int) -> List[int]:
+        """Consume every prompt but for its last token (the first ``reuse`` positions are cached already), each sequence its
+        own number of tokens in the same passes; returns the positions that are then in the cache."""
+        n = np.array([len(p) - 1 - reuse for p in prompts], np.uint32)
+        self._check(self._lib.adam_b200_decoder_prefill_ragged(self._dec, n.ctypes.data), "adam_b200_decoder_prefill_ragged")
+        return [len(p) - 1 for p in prompts]
+
     def read_state(self):
         pos = np.empty(self._max_batch, np.int32)
         tok = np.empty(self._max_batch, np.int32)
@@ -357,7 +364,7 @@ class ADAMEngine:
         g = self.gpu
         g.reset_native_stats()
         tp = time.perf_counter()
-        # all sequences step together, so each needs room up to the longest one's end
+        # room up to the longest sequence's end: where prompts end at different steps, all step until the last one is done
         max_len, min_len = max(lens), min(lens)
         # reuse_prefix (one sequence): the first tokens' keys and values are still cached from the previous call
         reuse = int(reuse_prefix or 0)
@@ -367,13 +374,12 @@ class ADAMEngine:
             self.continue_with(prompts[0], max_len + config.max_tokens, reuse)
         else:
             self.begin(prompts, [max_len + config.max_tokens] * len(prompts))
-        # prefill: every sequence consumes its own prompt; shorter ones start decoding earlier
         with g.batch():
-            if min_len - 1 > reuse:
-                self.prefill(min_len - 1 - reuse)
+            cached = self.prefill_prompts(prompts, reuse)
         t_pre = time.perf_counter() - tp
         td = time.perf_counter()
-        n_steps = (max_len - min_len) + config.max_tokens          # steps that run the LM head
+        ahead = [n - c for n, c in zip(lens, cached)]              # steps until a sequence's first sampled token
+        n_steps = max(ahead) - 1 + config.max_tokens               # steps that run the LM head
         eos = set(int(e) for e in config.eos_token_ids)
         steps_done = 0
         d2h = 0
@@ -386,11 +392,10 @@ class ADAMEngine:
             while steps_done < n_steps and not all(finished):
                 with g.batch():
                     self.step(1, lm_head=True, logits=True)
-                new_pos = min_len + steps_done              # position of the token this step produced
                 steps_done += 1
                 toks = np.zeros(len(prompts), np.int32)
                 for b, n in enumerate(lens):
-                    if finished[b] or new_pos < n:
+                    if finished[b] or steps_done < ahead[b]:     # still inside its prompt
                         continue
                     lg = self.read_logits(b)
                     d2h += lg.nbytes
@@ -418,7 +423,7 @@ class ADAMEngine:
                 self._check(self._lib.adam_b200_decoder_tokens_wait(self._dec, slot, buf.ctypes.data), "adam_b200_decoder_tokens_wait")
                 d2h += 4 * len(prompts)
                 for b, n in enumerate(lens):
-                    if finished[b] or min_len + step_no < n:          # still inside its prompt
+                    if finished[b] or step_no + 1 < ahead[b]:          # still inside its prompt
                         continue
                     t = int(buf[b])
                     if t in eos:

@@ -297,6 +297,12 @@ class ADAMEngineTP(ADAMEngine):
                         self._reduce_proj(self._batch * T)
                 left -= T
 
+    def prefill_prompts(self, prompts, reuse):
+        """Every sequence consumes as many positions as the shortest prompt has; the rest of a longer one runs step by step."""
+        n = min(len(p) for p in prompts) - 1
+        self.prefill(n - reuse)
+        return [n] * len(prompts)
+
     def begin(self, prompts, reserve):
         super().begin(prompts, reserve)
         self._graphs = {k: g for k, g in self._graphs.items() if k[1] == self._batch}

@@ -362,11 +362,13 @@ int adam_b200_decoder_set_tokens(uint32_t id, const int32_t* tokens);
  * the cache (generate(reuse_prefix=..), adam/models/engine.py:3815-3833): positions restart at
  * n_reuse (which must not exceed the positions computed so far), pages are kept and extended. */
 int adam_b200_decoder_continue(uint32_t id, const int32_t* prompt_tokens, uint32_t prompt_len, uint32_t reserve, uint32_t n_reuse);
-/* Chunked prefill: consume the next n_tokens prompt tokens of every active sequence, up to 64
- * rows (sequences x tokens) per pass through the layers; same results as n_tokens steps without
+/* Chunked prefill: consume the next n_tokens prompt tokens of every active sequence, many rows
+ * (sequences x tokens) per pass through the layers; same results as n_tokens steps without
  * the LM head.  Every sequence must still have n_tokens prompt tokens ahead.  The reference
  * consumes prompts token by token (adam/models/engine.py:3838-3847). */
 int adam_b200_decoder_prefill(uint32_t id, uint32_t n_tokens);
+/* The same with a number of tokens of its own for every active sequence ([batch], 0 allowed). */
+int adam_b200_decoder_prefill_ragged(uint32_t id, const uint32_t* n_tokens);
 /* The same step in parts, each enqueued directly on the stream, for callers that put their
  * own work between them (tensor parallelism).  Parts 2L / 2L+1 = attention half (embedding
  * for L = 0, QKV, attention, o-proj) / FFN half (gate+up, down) of layer L; then the LM head
@@ -375,12 +377,12 @@ int adam_b200_decoder_prefill(uint32_t id, uint32_t n_tokens);
 int adam_b200_decoder_n_parts(uint32_t id);                                   /* 2*n_layer + 2, or a negative status */
 int adam_b200_decoder_step_part(uint32_t id, uint32_t part, uint32_t flags);
 /* Number of matrix products enqueued so far on the tcgen05 (tensor memory) GEMM, which takes calls
- * with 9..64 activation rows; calls with fewer rows run on the GEMV kernels. */
+ * with many activation rows; calls with fewer rows run on the GEMV kernels. */
 uint64_t adam_b200_tc_gemm_count(void);
 /* Which calls take it: 0 = none, 1 = those expected to be faster than the GEMV kernels (default; also the
  * initial value of environment variable ADAM_B200_TC), 2 = every call whose shape allows. */
 int adam_b200_tc_gemm_policy(int policy);
-/* One part of one prefill chunk of n_tokens (batch * n_tokens <= 64 rows) tokens per sequence: parts
+/* One part of one prefill chunk of n_tokens (batch * n_tokens rows, at least 64 are accepted) tokens per sequence: parts
  * 0 .. 2*n_layer-1 as above (the projection buffer then holds batch * n_tokens rows of partial
  * sums), part 2*n_layer advances the positions by n_tokens. */
 int adam_b200_decoder_prefill_part(uint32_t id, uint32_t n_tokens, uint32_t part);
