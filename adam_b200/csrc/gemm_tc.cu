@@ -236,6 +236,10 @@ __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16])
                  :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
                     "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
+__device__ __forceinline__ void tc_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
 __device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&r)[16]) {       // valid after tc_ld_wait()
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -269,12 +273,12 @@ __device__ __forceinline__ float ld_cluster(uint32_t saddr, uint32_t rank) {
 // ---- nibbles -> two fp16 terms ----------------------------------------------------------------------------------
 __device__ __forceinline__ __half2 as_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
 __device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
-// The eight nibbles of a word, two at a time, as halves: low nibbles of bytes (0, 2) and (1, 3) as 1024 + q, high ones
-// as 1024 + 16 q, by masking them into the mantissa of 1024.0.
-__device__ __forceinline__ void nib_pairs(uint32_t w, uint32_t (&lo)[2], uint32_t (&hi)[2]) {
-    const uint32_t w8 = w >> 8;
-    lo[0] = (w & 0x000F000Fu) | 0x64006400u; lo[1] = (w8 & 0x000F000Fu) | 0x64006400u;
-    hi[0] = (w & 0x00F000F0u) | 0x64006400u; hi[1] = (w8 & 0x00F000F0u) | 0x64006400u;
+// The low or high nibbles of a word's four bytes, two at a time, as halves: bytes (0, 2) and (1, 3) as 1024 + q (low) or
+// 1024 + 16 q (high), by masking them into the mantissa of 1024.0.
+template <bool HIGH> __device__ __forceinline__ void nib_pairs(uint32_t w, uint32_t (&p)[2]) {
+    constexpr uint32_t M = HIGH ? 0x00F000F0u : 0x000F000Fu;
+    p[0] = (w & M) | 0x64006400u;
+    p[1] = ((w >> 8) & M) | 0x64006400u;
 }
 // v * d as w_hi + w_lo (v two exact small integers)
 __device__ __forceinline__ void split_h2(__half2 v, __half2 d, uint32_t& whi, uint32_t& wlo) {
@@ -291,7 +295,7 @@ __device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, u
 }
 
 // ---- the GEMM ---------------------------------------------------------------------------------------------------
-// One CTA per SM, 10 warps: 0..7 rebuild weights, 8 fetches activation tiles, 9 issues the tensor-core instructions.
+// One CTA per SM, 18 warps: 0..15 rebuild weights, 16 fetches activation tiles, 17 issues the tensor-core instructions.
 // A CTA's tile is NA x 128 weight rows (NA = 2: either 128 gate + 128 up rows of one GeGLU tile, or 256 rows of one
 // matrix, which share an activation tile) by NT activation rows; per 128 rows D is 2 NT columns of TMEM, the rest of TMEM
 // is a ring of four weight tiles (128 rows x 64 values of K as w_hi | w_lo, 64 columns).
@@ -299,7 +303,9 @@ __device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, u
 //                memory (R steps ahead, across the end of a tile, two lanes per row so that a sector is fetched whole), are
 //                taken apart in fp16 pairs (4.25 instructions per two weights) and go to TMEM with tcgen05.st: no
 //                shared-memory operand image, no swizzle, no bank conflicts, and the shared memory's 128 bytes per cycle
-//                are left to the activation operand.  Warps 0..3 take the even weight tiles, 4..7 the odd ones.
+//                are left to the activation operand.  Four groups of four warps take the weight tiles in turn, one ring
+//                slot each: rebuilding a tile is a chain of about 1000 cycles (two groups: 1125 cycles per tile and SM;
+//                four: see the figures at launch_rows), and what the four schedulers lack is warps, not issue slots.
 //   activations  x_hi | x_lo tiles of 64 values of K by bulk copies from the image, a ring of NB stages shared by the NA
 //                weight tiles of a step.
 //   products     per tile and 16 values of K two tcgen05.mma (M 128): w_hi x [x_hi | x_lo] with N = 2 NT into D1 | D2, and
@@ -310,14 +316,15 @@ __device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, u
 //                added up (measured: 5e-9 of the result each).  So the cross terms, 2^-11 of the result, have D2 to
 //                themselves, and every `period` steps D1 is added to registers and restarted.  Relative error of a
 //                1152 x 6912 product: 6.1e-6 with one accumulator for all of K, 4e-7 with this.
-//   read-out     The warps that rebuild weight tile i read D1 of tile i (half of the columns each where NA = 1), after
-//                they have produced the first tile of the next period, so the tensor core works on the other tile meanwhile.
+//   read-out     The same warps read D1, each group its share of the columns, after it has produced its first tile of the
+//                next period, so the tensor core has work meanwhile.
 //   K splits     where the tiles alone leave SMs idle, S CTAs of a cluster take a part of K each, leave their sums in their
 //                own shared memory and add each other's columns through distributed shared memory (in split order: results
 //                do not depend on timing).
 // The request for shared memory is at least 120 KB, so that an SM never holds two of these CTAs: one that waits for
 // tensor memory held by a cluster that waits for it would never end.
-constexpr int TC_WARPS = 10, TC_THREADS = TC_WARPS * 32;
+constexpr int TC_GROUPS = 4, TC_WARPS = TC_GROUPS * 4 + 2, TC_THREADS = TC_WARPS * 32;
+constexpr int TC_LOADER = TC_GROUPS * 4, TC_ISSUER = TC_LOADER + 1;
 constexpr int TC_SMEM_MIN = 120 * 1024;
 constexpr int TC_PERIOD = 6;                            // most steps (64 values of K) accumulated in D1 before it is read out
 struct TcGemm {
@@ -329,12 +336,12 @@ struct TcGemm {
     int S, period;                                      // K splits; steps per accumulation period
 };
 template <int WT, int NT, bool PAIR> struct TcGeo {
-    static constexpr int R = 8;                                              // weight ring: steps ahead per warp
+    static constexpr int R = 4;                                              // weight ring: tiles ahead per warp
     static constexpr int SLOT = 1024 + (WT == WT_Q4_0 ? 128 : 512);          // 32 rows: nibbles, then block scales / superblock headers
     static constexpr int NB = 4;
     static constexpr int BSTAGE = NT * 256;
-    static constexpr int XCH = PAIR ? NT * 512 : 0;                          // gate / up exchange: half of the columns each way
-    static constexpr int SMEM_USED = NB * BSTAGE + 8 * R * SLOT + XCH + 1024;
+    static constexpr int XCH = PAIR ? (NT < 32 ? 32 : NT) * 512 : 0;         // gate / up exchange: half of the columns each way
+    static constexpr int SMEM_USED = NB * BSTAGE + TC_GROUPS * 4 * R * SLOT + XCH + 1024;
     static constexpr int SMEM = SMEM_USED > TC_SMEM_MIN ? SMEM_USED : TC_SMEM_MIN;
 };
 __device__ __forceinline__ bool elect_one() {
@@ -352,6 +359,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
     __shared__ __align__(8) uint64_t b_full[G::NB], b_empty[G::NB], a_full[4], a_empty[4], d_full[NA], d_empty[NA];
     __shared__ uint32_t s_tmem;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // columns that a group reads back, and how many groups read
+    constexpr int COLS = NA * NT / TC_GROUPS < 16 ? 16 : NA * NT / TC_GROUPS, READERS = NA * NT / COLS;
     const int S = a.S, split = S > 1 ? (int)(blockIdx.x % (uint32_t)S) : 0;     // a cluster's CTAs are neighbours along x
     const int first = S > 1 ? (int)(blockIdx.x / (uint32_t)S) : (int)blockIdx.x, stride = (int)gridDim.x / S;
     // this split's share of the steps: first those of the block minima, then those of the products
@@ -361,11 +370,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
     if (tid == 0) {
         for (int i = 0; i < G::NB; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
         for (int i = 0; i < 4; ++i) { mbar_init(&a_full[i], 4); mbar_init(&a_empty[i], 1); }
-        for (int i = 0; i < NA; ++i) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], NA == 2 ? 4 : 8); }
+        for (int i = 0; i < NA; ++i) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], 4 * READERS / NA); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 9) tc_alloc(&s_tmem, 512);
+    if (warp == TC_ISSUER) tc_alloc(&s_tmem, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -378,7 +387,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
     };
     pdl_launch_dependents();
 
-    if (warp == 8) {
+    if (warp == TC_LOADER) {
         // ---- activation tiles ----
         pdl_wait();                                     // the image comes from the kernel before this one
         const bool lead = elect_one();
@@ -401,11 +410,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                 __syncwarp();
             }
         }
-    } else if (warp == 9) {
+        // no copy may be in flight when the CTA ends, whatever became of the waits above
+        for (uint32_t i = n > (uint32_t)G::NB ? n - G::NB : 0; i < n; ++i) mbar_wait(&b_full[i % G::NB], (i / G::NB) & 1u);
+    } else if (warp == TC_ISSUER) {
         // ---- products ----
         pdl_wait();                                     // so that no bounded wait below spans an earlier kernel
         const bool lead = elect_one();
-        uint32_t n = 0, t = 0, period = 0;              // steps, weight tiles, accumulation periods so far
+        uint32_t n = 0, period = 0, phase = 0;          // steps and accumulation periods so far; parities of the weight ring's slots
         for (int item = first; item < a.items; item += stride) {
             int left = 0;                               // steps left in the period
             for (int st = 0; st < nst; ++st, ++n) {
@@ -416,10 +427,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                 wait_on(&b_full[bs], (n / G::NB) & 1u);
                 const uint32_t bh = smem_u32(smB + bs * G::BSTAGE);
 #pragma unroll
-                for (int i = 0; i < NA; ++i, ++t) {
-                    const uint32_t as = t & 3u, ac = tmem + A_COL + as * 64u, d1 = tmem + (uint32_t)(i * 2 * NT), d2 = d1 + NT;
+                for (int i = 0; i < NA; ++i) {
+                    const uint32_t as = (uint32_t)(st * NA + i) & 3u, ac = tmem + A_COL + as * 64u, d1 = tmem + (uint32_t)(i * 2 * NT), d2 = d1 + NT;
                     if (fresh && period > 1) wait_on(&d_empty[i], (period - 2u) & 1u);      // D of the period before is read
-                    wait_on(&a_full[as], (t >> 2) & 1u);
+                    wait_on(&a_full[as], (phase >> as) & 1u);
+                    phase ^= 1u << as;
                     tc_fence_after();
                     if (lead) {
                         if (fresh && st > 0) {          // D1 starts again, D2 goes on
@@ -443,14 +455,18 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
     } else {
         // ---- weights, and the end of a tile ----
         const int grp = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane;       // row = this lane's TMEM lane
-        const int mine = NA == 2 ? grp : 0;             // which 128 rows of the tile this group rebuilds and reads back
+        const int mine = NA == 2 ? grp & 1 : 0;         // which 128 rows of the tile this group rebuilds and reads back
         const uint32_t tlane = tmem + ((uint32_t)(quarter * 32) << 16);
         uint8_t* ring = sm + G::NB * G::BSTAGE + warp * G::R * G::SLOT;
         const uint32_t ring_s = smem_u32(ring);
-        const WeightRef w = (PAIR && grp) ? a.w1 : a.w0;
+        const WeightRef w = (PAIR && mine) ? a.w1 : a.w0;
         const bool scales_async = WT == WT_Q4_K || ((a.units & 1) == 0 && ((uintptr_t)w.d & 3) == 0);
-        const int n_own = NA == 2 ? nst : (nst + 1 - grp) / 2;                          // this group's weight tiles of an item
-        auto step_of = [&](int j) { return NA == 2 ? j : grp + 2 * j; };
+        // Tiles of an item in the order of the products: number t = step * NA + i.  This group takes t = grp, grp + 4, ... of
+        // every item and always uses ring slot grp: a slot that changed hands could be waited for by a group that has not
+        // followed its phases, and a wait on a phase two ahead returns at once.
+        constexpr int SS = TC_GROUPS / NA;              // steps from one to the next
+        const int s0 = grp / NA, n_own = (nst - s0 + SS - 1) / SS;
+        auto step_of = [&](int j) { return s0 + SS * j; };
         auto row_of = [&](int tn, int r) { return min((PAIR ? tn * 128 : (tn * NA + mine) * 128) + r, a.N - 1); };
         const int rpu = WT == WT_Q4_0 ? a.units : (a.units >> 3) * 9;                   // uint4 per weight row
         const int n_items = first < a.items ? (a.items - first + stride - 1) / stride : 0;
@@ -487,9 +503,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
         };
 
         // D1 (and, with the item's last period, D2) into acc; the end of an item: scale back, activation, store
-        constexpr int COLS = NA == 2 ? NT : (NT >= 32 ? NT / 2 : 16);                   // columns this group reads back
-        const bool reads = NA == 2 || NT >= 32 || grp == 0;
-        const int c0 = NA == 2 ? 0 : grp * COLS;
+        const bool reads = grp < READERS;
+        const int c0 = grp / NA * COLS;
         const int np = (nst + a.period - 1) / a.period;                                 // periods per item
         bool waited = false;
         int done = 0, done_item = 0, done_p = 0;        // periods read out: in all, as (item, period of the item)
@@ -501,7 +516,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
             const bool last = done_p == np - 1;
             wait_on(&d_full[mine], (uint32_t)done & 1u);
             tc_fence_after();
-            if (reads) {
+            {
                 const uint32_t col = tlane + (uint32_t)(mine * 2 * NT + c0);
 #pragma unroll
                 for (int ch = 0; ch < COLS / 16; ++ch) {
@@ -538,6 +553,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                 // one item per cluster: sums into the exchange (the activation ring is drained), then every CTA finishes the
                 // columns c = split, split + S, ... from all S parts
                 float* ex = reinterpret_cast<float*>(smB);
+                if constexpr (NA == 2) wait_on(&d_full[mine ^ 1], (uint32_t)(done - 1) & 1u);      // the other tile's last products read the ring too
                 if (reads) {
 #pragma unroll
                     for (int c = 0; c < COLS; ++c) ex[(mine * NT + c0 + c) * 128 + row] = acc[c];
@@ -553,14 +569,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                     for (int q = 0; q < 8; ++q) v += p[q];
                     return v;
                 };
-                if constexpr (PAIR || NA == 1) {                // both groups share the columns
-                    for (int c = split + S * grp; c < n_col; c += 2 * S) {
+                if constexpr (PAIR || NA == 1) {                // all groups share the columns
+                    for (int c = split + S * grp; c < n_col; c += READERS * S) {
                         const float sc = inv_of(c), v = total_of(0, c);
                         if constexpr (PAIR) { const float u = total_of(1, c); if (n_out < a.N) yp[(size_t)c * a.ldy] = act(v * sc, u * sc); }
                         else if (n_out < a.N) yp[(size_t)c * a.ldy] = v * sc;
                     }
                 } else {
-                    for (int c = split; c < n_col; c += S) {
+                    for (int c = split + S * (grp >> 1); c < n_col; c += READERS / 2 * S) {
                         const float v = total_of(mine, c) * inv_of(c);
                         if (n_out < a.N) yp[(size_t)c * a.ldy] = v;
                     }
@@ -568,22 +584,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                 cl_arrive();
                 cl_wait();
             } else if constexpr (PAIR) {
-                // gate (group 0) and up (group 1) swap half of their columns; group 0 finishes the first half
-                float* x0 = reinterpret_cast<float*>(sm + G::NB * G::BSTAGE + 8 * G::R * G::SLOT);
-                constexpr int H = NT / 2;
-                float* put = x0 + (grp ? 0 : H * 128) + row;
-                const float* get = x0 + (grp ? H * 128 : 0) + row;
+                // the gate group and the up group of the same columns swap half of them; the gate group finishes the first half
+                constexpr int H = COLS / 2;
+                float* x0 = reinterpret_cast<float*>(sm + G::NB * G::BSTAGE + TC_GROUPS * 4 * G::R * G::SLOT) + (grp >> 1) * COLS * 128;
+                float* put = x0 + (mine ? 0 : H * 128) + row;
+                const float* get = x0 + (mine ? H * 128 : 0) + row;
 #pragma unroll
-                for (int c = 0; c < H; ++c) put[c * 128] = grp ? acc[c] : acc[H + c];
-                asm volatile("bar.sync 1, 256;" ::: "memory");
+                for (int c = 0; c < H; ++c) put[c * 128] = mine ? acc[c] : acc[H + c];
+                asm volatile("bar.sync %0, 256;" :: "r"(1 + (grp >> 1)) : "memory");
 #pragma unroll
                 for (int c = 0; c < H; ++c) {
-                    const int col = grp * H + c;
-                    const float o = get[c * 128], sc = inv_of(col), m = grp ? acc[H + c] : acc[c];
-                    if (col < n_col && n_out < a.N) yp[(size_t)col * a.ldy] = grp ? act(o * sc, m * sc) : act(m * sc, o * sc);
+                    const int col = c0 + mine * H + c;
+                    const float o = get[c * 128], sc = inv_of(col), m = mine ? acc[H + c] : acc[c];
+                    if (col < n_col && n_out < a.N) yp[(size_t)col * a.ldy] = mine ? act(o * sc, m * sc) : act(m * sc, o * sc);
                 }
-                asm volatile("bar.sync 1, 256;" ::: "memory");
-            } else if (reads) {
+                asm volatile("bar.sync %0, 256;" :: "r"(1 + (grp >> 1)) : "memory");
+            } else {
 #pragma unroll
                 for (int c = 0; c < COLS; ++c) {
                     const float v = acc[c] * inv_of(c0 + c);
@@ -595,14 +611,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
         };
         // ---- production ----
         for (int j = 0; j < G::R; ++j) fetch();
-        uint32_t t = (uint32_t)grp, n = 0;              // tile number in the order of the products; tiles of this group
+        uint32_t n = 0;                                 // tiles of this group
         for (int k = 0; k < n_items; ++k) {
             const int tn = (first + k * stride) % a.tiles_n;
             for (int j = 0; j < n_own; ++j, ++n) {
                 const int st = step_of(j), ks = ma0 + st - nmn;
-                if constexpr (NA == 2) t = 2u * n + (uint32_t)grp;
-                else t = (uint32_t)(k * nst + st);
-                const uint32_t as = t & 3u, acol = tlane + A_COL + as * 64u;
+                const uint32_t acol = tlane + A_COL + grp * 64u;
                 cp_wait<G::R - 1>();
                 __syncwarp();
                 const uint8_t* slot = ring + (n % G::R) * G::SLOT;
@@ -613,9 +627,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                 else hdr = *reinterpret_cast<const uint4*>(slot + 1024 + lane * 16);
                 __syncwarp();
                 fetch();
-                if (t >= 4u) {
+                if (n) {                                // the tensor core is done with this group's tile before
                     if (!waited) { pdl_wait(); waited = true; }
-                    wait_on(&a_empty[as], ((t >> 2) - 1u) & 1u);
+                    wait_on(&a_empty[grp], (n - 1u) & 1u);
                     tc_fence_after();
                 }
                 const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
@@ -625,44 +639,49 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                         d01 = (uint32_t)dp[0] | (2 * ks + 1 < a.units ? (uint32_t)dp[1] << 16 : 0u);
                     }
 #pragma unroll
-                    for (int b = 0; b < 2; ++b) {
-                        const uint32_t dd = b ? d01 >> 16 : d01 & 0xFFFFu;
-                        const __half2 d = as_h2(dd * 0x10001u);
-                        uint32_t whi[16], wlo[16];
+                    for (int b = 0; b < 2; ++b) {       // columns 16 b ..: values 0..15 of the block from the low nibbles, 16..31 from the high ones
+                        const __half2 d = as_h2((b ? d01 >> 16 : d01 & 0xFFFFu) * 0x10001u);
+                        uint32_t whi[8], wlo[8], v[2];
 #pragma unroll
                         for (int x = 0; x < 4; ++x) {
-                            uint32_t l[2], h[2];
-                            nib_pairs(qw[4 * b + x], l, h);
+                            nib_pairs<false>(qw[4 * b + x], v);
 #pragma unroll
-                            for (int p = 0; p < 2; ++p) {
-                                split_h2(__hadd2(as_h2(l[p]), __float2half2_rn(-1032.f)), d, whi[2 * x + p], wlo[2 * x + p]);
-                                split_h2(__hfma2(as_h2(h[p]), __float2half2_rn(0.0625f), __float2half2_rn(-72.f)), d, whi[8 + 2 * x + p], wlo[8 + 2 * x + p]);
-                            }
+                            for (int p = 0; p < 2; ++p) split_h2(__hadd2(as_h2(v[p]), __float2half2_rn(-1032.f)), d, whi[2 * x + p], wlo[2 * x + p]);
                         }
-                        tc_st16(acol + b * 16u, whi);
-                        tc_st16(acol + 32u + b * 16u, wlo);
+                        tc_st8(acol + b * 16u, whi);
+                        tc_st8(acol + 32u + b * 16u, wlo);
+#pragma unroll
+                        for (int x = 0; x < 4; ++x) {
+                            nib_pairs<true>(qw[4 * b + x], v);
+#pragma unroll
+                            for (int p = 0; p < 2; ++p) split_h2(__hfma2(as_h2(v[p]), __float2half2_rn(0.0625f), __float2half2_rn(-72.f)), d, whi[2 * x + p], wlo[2 * x + p]);
+                        }
+                        tc_st8(acol + 8u + b * 16u, whi);
+                        tc_st8(acol + 40u + b * 16u, wlo);
                     }
                 } else if (st >= nmn) {
                     uint32_t sp, mp;
                     q4k_codes(hdr, ks & 3, sp, mp);
                     const __half2 d = as_h2((hdr.x & 0xFFFFu) * 0x10001u);
-                    uint32_t lo_[8][2], hi_[8][2];
-#pragma unroll
-                    for (int x = 0; x < 8; ++x) nib_pairs(qw[x], lo_[x], hi_[x]);
 #pragma unroll
                     for (int b = 0; b < 2; ++b) {       // low nibbles = sub-block 2g, high nibbles = sub-block 2g + 1
                         const uint32_t code = b ? sp >> 8 : sp & 0xFFu;
                         const __half2 sc = __hsub2(as_h2((code * 0x10001u) | 0x64006400u), __float2half2_rn(1024.f));
                         const __half2 mul = b ? __hmul2(sc, __float2half2_rn(0.0625f)) : sc;
                         const __half2 off = __hmul2(sc, __float2half2_rn(b ? -64.f : -1024.f));
-                        uint32_t whi[16], wlo[16];
 #pragma unroll
-                        for (int x = 0; x < 8; ++x)
+                        for (int y = 0; y < 2; ++y) {
+                            uint32_t whi[8], wlo[8], v[2];
 #pragma unroll
-                            for (int p = 0; p < 2; ++p)   // sc * q, an integer below 946, exactly
-                                split_h2(__hfma2(as_h2(b ? hi_[x][p] : lo_[x][p]), mul, off), d, whi[2 * x + p], wlo[2 * x + p]);
-                        tc_st16(acol + b * 16u, whi);
-                        tc_st16(acol + 32u + b * 16u, wlo);
+                            for (int x = 0; x < 4; ++x) {
+                                if (b) nib_pairs<true>(qw[4 * y + x], v); else nib_pairs<false>(qw[4 * y + x], v);
+#pragma unroll
+                                for (int p = 0; p < 2; ++p)       // sc * q, an integer below 946, exactly
+                                    split_h2(__hfma2(as_h2(v[p]), mul, off), d, whi[2 * x + p], wlo[2 * x + p]);
+                            }
+                            tc_st8(acol + b * 16u + y * 8u, whi);
+                            tc_st8(acol + 32u + b * 16u + y * 8u, wlo);
+                        }
                     }
                 } else {
                     // a step of block minima: -32 dmin m of 64 sub-blocks (the image holds the sums over 32 activations / 32)
@@ -694,17 +713,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                 tc_st_wait();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&a_full[as]);
-                while (done < k * np + st / a.period) read_out();       // what ended before this tile's period
+                if (lane == 0) mbar_arrive(&a_full[grp]);
+                if (reads) while (done < k * np + st / a.period) read_out();    // what ended before this tile's period
             }
         }
-        while (done < n_items * np) read_out();
+        if (reads) while (done < n_items * np) read_out();
         cp_wait<0>();
     }
-    if (S > 1 && warp >= 8) { cl_arrive(); cl_wait(); cl_arrive(); cl_wait(); }
+    if (S > 1 && (warp >= TC_LOADER || (warp >> 2) >= READERS)) { cl_arrive(); cl_wait(); cl_arrive(); cl_wait(); }
     __syncthreads();
     tc_fence_after();
-    if (warp == 9) tc_dealloc(tmem, 512);
+    if (warp == TC_ISSUER) tc_dealloc(tmem, 512);
 }
 
 // ---- host ----------------------------------------------------------------------------------------------------------
