@@ -204,9 +204,7 @@ __global__ void __launch_bounds__(512) k_quant_rows(const GemvArgs a, uint8_t* _
 // Shared-memory matrix descriptor, K-major with the 128-byte swizzle (layout 2 at bit 61): start address and the
 // distance between 8-row groups (1024 bytes), in 16-byte units, plus the descriptor version of this architecture (bit 46).
 // The 16 values of K of one instruction are 32 bytes of a row: the next instruction's descriptor starts 32 bytes further.
-__device__ __forceinline__ uint64_t tc_desc(uint32_t saddr) {
-    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
+#define TC_DESC_HI ((uint32_t)(1024u >> 4) | (1u << 14) | (2u << 29))
 // Instruction descriptor of kind::f16: D = f32 (1 at bit 4), A = B = f16 (0 at bits 7 and 10), both operands K-major,
 // N / 8 at bit 17, M / 16 at bit 24.
 template <int N> constexpr uint32_t TC_IDESC = (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((128u >> 4) << 24);
@@ -230,12 +228,7 @@ __device__ __forceinline__ void tc_mma_ts(uint32_t d, uint32_t a, uint64_t bdesc
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(smem_u32(bar)) : "memory");
 }
-// 16 consecutive 32-bit columns of this thread's TMEM lane, to and from registers.
-__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-                    "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-}
+// 16 and 8 consecutive 32-bit columns of this thread's TMEM lane, to and from registers.
 __device__ __forceinline__ void tc_st8(uint32_t taddr, const uint32_t (&r)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
                  :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
@@ -296,28 +289,28 @@ __device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, u
 
 // ---- the GEMM ---------------------------------------------------------------------------------------------------
 // One CTA per SM, 18 warps: 0..15 rebuild weights, 16 fetches activation tiles, 17 issues the tensor-core instructions.
-// A CTA's tile is NA x 128 weight rows (NA = 2: either 128 gate + 128 up rows of one GeGLU tile, or 256 rows of one
-// matrix, which share an activation tile) by NT activation rows; per 128 rows D is 2 NT columns of TMEM, the rest of TMEM
-// is a ring of four weight tiles (128 rows x 64 values of K as w_hi | w_lo, 64 columns).
+// A CTA's tile is 128 weight rows (or 64 gate rows in TMEM lanes 0..63 and the same 64 up rows in lanes 64..127) by NT
+// activation rows: D is 2 NT columns of TMEM, the upper half of TMEM is a ring of four weight tiles (128 rows x 64 values
+// of K as w_hi | w_lo, 64 columns).
 //   weights      A lane owns a row.  Its 32 bytes of nibbles per step come by cp.async into the warp's own ring in shared
-//                memory (R steps ahead, across the end of a tile, two lanes per row so that a sector is fetched whole), are
+//                memory (R tiles ahead, across the end of a tile, two lanes per row so that a sector is fetched whole), are
 //                taken apart in fp16 pairs (4.25 instructions per two weights) and go to TMEM with tcgen05.st: no
 //                shared-memory operand image, no swizzle, no bank conflicts, and the shared memory's 128 bytes per cycle
-//                are left to the activation operand.  Four groups of four warps take the weight tiles in turn, one ring
-//                slot each: rebuilding a tile is a chain of about 1000 cycles (two groups: 1125 cycles per tile and SM;
-//                four: see the figures at launch_rows), and what the four schedulers lack is warps, not issue slots.
-//   activations  x_hi | x_lo tiles of 64 values of K by bulk copies from the image, a ring of NB stages shared by the NA
-//                weight tiles of a step.
-//   products     per tile and 16 values of K two tcgen05.mma (M 128): w_hi x [x_hi | x_lo] with N = 2 NT into D1 | D2, and
-//                w_lo x x_hi with N = NT into D2; 384 cycles per tile at NT = 64, which is the tensor core's rate.  One
-//                elected lane issues, but the whole warp walks the loop: inside a one-lane branch the same loop took 628
-//                cycles per tile instead of 413 (waits and descriptors leave the uniform datapath).
+//                are left to the activation operand.  Four groups of four warps take the steps in turn, one ring slot
+//                each: rebuilding a tile is a chain of about 1000 cycles, and what the four schedulers lack is warps.
+//                It takes some 330 issue slots of each scheduler, which is why a tile has up to 128 activation rows (768
+//                cycles of the tensor core per step): with 64 (384 cycles) the same kernel ran at half the rate.
+//   activations  x_hi | x_lo tiles of 64 values of K by bulk copies from the image, a ring of NB stages.
+//   products     per 16 values of K two tcgen05.mma (M 128): w_hi x [x_hi | x_lo] with N = 2 NT into D1 | D2, and
+//                w_lo x x_hi with N = NT into D2; 6 cycles per step and activation row, the tensor core's rate.  One
+//                elected lane issues, but the whole warp walks the loop: inside a one-lane branch a step took 628 cycles
+//                instead of 413 (NT = 64; waits and descriptors leave the uniform datapath).
 //   rounding     The tensor core rounds its running sum towards zero, an error that grows with the number of instructions
 //                added up (measured: 5e-9 of the result each).  So the cross terms, 2^-11 of the result, have D2 to
 //                themselves, and every `period` steps D1 is added to registers and restarted.  Relative error of a
 //                1152 x 6912 product: 6.1e-6 with one accumulator for all of K, 4e-7 with this.
 //   read-out     The same warps read D1, each group its share of the columns, after it has produced its first tile of the
-//                next period, so the tensor core has work meanwhile.
+//                next period, so that the pause of the tensor core is short.
 //   K splits     where the tiles alone leave SMs idle, S CTAs of a cluster take a part of K each, leave their sums in their
 //                own shared memory and add each other's columns through distributed shared memory (in split order: results
 //                do not depend on timing).
@@ -335,13 +328,13 @@ struct TcGemm {
     int n_min, n_main, tiles_n, items;                  // items = tiles_n * tiles of NT rows
     int S, period;                                      // K splits; steps per accumulation period
 };
-template <int WT, int NT, bool PAIR> struct TcGeo {
+template <int WT, int NT> struct TcGeo {
     static constexpr int R = 4;                                              // weight ring: tiles ahead per warp
     static constexpr int SLOT = 1024 + (WT == WT_Q4_0 ? 128 : 512);          // 32 rows: nibbles, then block scales / superblock headers
-    static constexpr int NB = 4;
+    static constexpr int NB = NT == 128 ? 3 : 4;
     static constexpr int BSTAGE = NT * 256;
-    static constexpr int XCH = PAIR ? (NT < 32 ? 32 : NT) * 512 : 0;         // gate / up exchange: half of the columns each way
-    static constexpr int SMEM_USED = NB * BSTAGE + TC_GROUPS * 4 * R * SLOT + XCH + 1024;
+    static constexpr int RING = NB * BSTAGE, XCH = RING + TC_GROUPS * 4 * R * SLOT;     // offsets: weight rings, gate / up exchange (4 KB per group)
+    static constexpr int SMEM_USED = XCH + TC_GROUPS * 4096 + 1024;
     static constexpr int SMEM = SMEM_USED > TC_SMEM_MIN ? SMEM_USED : TC_SMEM_MIN;
 };
 __device__ __forceinline__ bool elect_one() {
@@ -349,18 +342,17 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
     return p != 0;
 }
-template <int WT, int NA, int NT, bool PAIR>
+template <int WT, int NT, bool PAIR>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
-    using G = TcGeo<WT, NT, PAIR>;
-    static_assert(!PAIR || NA == 2, "a gate/up tile holds both matrices");
+    using G = TcGeo<WT, NT>;
     extern __shared__ __align__(1024) uint8_t sm_raw[];
     uint8_t* sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);     // the swizzle works on address bits
     uint8_t* smB = sm;
-    __shared__ __align__(8) uint64_t b_full[G::NB], b_empty[G::NB], a_full[4], a_empty[4], d_full[NA], d_empty[NA];
+    __shared__ __align__(8) uint64_t b_full[G::NB], b_empty[G::NB], a_full[TC_GROUPS], a_empty[TC_GROUPS], d_full, d_empty;
     __shared__ uint32_t s_tmem;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // columns that a group reads back, and how many groups read
-    constexpr int COLS = NA * NT / TC_GROUPS < 16 ? 16 : NA * NT / TC_GROUPS, READERS = NA * NT / COLS;
+    constexpr int COLS = NT / TC_GROUPS < 16 ? 16 : NT / TC_GROUPS, READERS = NT / COLS;
     const int S = a.S, split = S > 1 ? (int)(blockIdx.x % (uint32_t)S) : 0;     // a cluster's CTAs are neighbours along x
     const int first = S > 1 ? (int)(blockIdx.x / (uint32_t)S) : (int)blockIdx.x, stride = (int)gridDim.x / S;
     // this split's share of the steps: first those of the block minima, then those of the products
@@ -369,8 +361,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
     const int nmn = mn1 - mn0, nst = nmn + ma1 - ma0, n_steps = a.n_min + a.n_main;
     if (tid == 0) {
         for (int i = 0; i < G::NB; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
-        for (int i = 0; i < 4; ++i) { mbar_init(&a_full[i], 4); mbar_init(&a_empty[i], 1); }
-        for (int i = 0; i < NA; ++i) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], 4 * READERS / NA); }
+        for (int i = 0; i < TC_GROUPS; ++i) { mbar_init(&a_full[i], 4); mbar_init(&a_empty[i], 1); }
+        mbar_init(&d_full, 1); mbar_init(&d_empty, 4 * READERS);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -379,8 +371,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
-    constexpr uint32_t A_COL = NA * 2 * NT;             // first column of the weight ring
-    static_assert(A_COL + 256 <= 512, "tensor memory");
+    constexpr uint32_t A_COL = 256;                     // first column of the weight ring
     bool dead = false;
     auto wait_on = [&](uint64_t* bar, uint32_t parity) {
         if (!dead && !mbar_wait(bar, parity)) { dead = true; atomicOr(a.err, DEVERR_WAIT); }
@@ -393,7 +384,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
         const bool lead = elect_one();
         uint32_t n = 0;
         for (int item = first; item < a.items; item += stride) {
-            const uint8_t* group = a.img + (size_t)(item / a.tiles_n) * n_steps * (2 * TC_STEP_IMG);
+            const size_t group_bytes = (size_t)n_steps * (2 * TC_STEP_IMG);
+            const uint8_t* group = a.img + (size_t)(item / a.tiles_n) * (NT == 128 ? 2 : 1) * group_bytes;
             for (int st = 0; st < nst; ++st, ++n) {
                 const int bs = (int)(n % G::NB);
                 const uint8_t* src = group + (size_t)(st < nmn ? mn0 + st : a.n_min + ma0 + st - nmn) * (2 * TC_STEP_IMG);
@@ -402,9 +394,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                 if (lead) {
                     mbar_expect_tx(&b_full[bs], (uint32_t)G::BSTAGE);
                     if constexpr (NT == TC_GROUP) bulk_g2s(dst, src, G::BSTAGE, &b_full[bs]);
-                    else {                              // the first NT rows of both planes
-                        bulk_g2s(dst, src, NT * 128, &b_full[bs]);
-                        bulk_g2s(dst + NT * 128, src + TC_STEP_IMG, NT * 128, &b_full[bs]);
+                    else {                              // both planes of the first NT rows, or of two groups
+                        constexpr int ROWS = NT < TC_GROUP ? NT : TC_GROUP;
+                        bulk_g2s(dst, src, ROWS * 128, &b_full[bs]);
+                        bulk_g2s(dst + NT * 128, src + TC_STEP_IMG, ROWS * 128, &b_full[bs]);
+                        if constexpr (NT > TC_GROUP) {
+                            bulk_g2s(dst + TC_STEP_IMG, src + group_bytes, TC_STEP_IMG, &b_full[bs]);
+                            bulk_g2s(dst + NT * 128 + TC_STEP_IMG, src + group_bytes + TC_STEP_IMG, TC_STEP_IMG, &b_full[bs]);
+                        }
                     }
                 }
                 __syncwarp();
@@ -416,58 +413,60 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
         // ---- products ----
         pdl_wait();                                     // so that no bounded wait below spans an earlier kernel
         const bool lead = elect_one();
-        uint32_t n = 0, period = 0, phase = 0;          // steps and accumulation periods so far; parities of the weight ring's slots
+        // the issuer shares its scheduler with four busy warps: few instructions per step
+        const uint32_t b_lo = (smem_u32(smB) & 0x3FFFFu) >> 4, d1 = tmem, d2 = tmem + NT;
+        auto desc = [&](uint32_t lo) { return ((uint64_t)TC_DESC_HI << 32) | lo; };
+        uint32_t bs = 0, b_par = 0, g_at = 0, a_par = 0, periods = 0;       // ring positions and parities
         for (int item = first; item < a.items; item += stride) {
             int left = 0;                               // steps left in the period
-            for (int st = 0; st < nst; ++st, ++n) {
+            g_at = 0;
+            for (int st = 0; st < nst; ++st) {
                 const bool fresh = left == 0;
-                if (fresh) { left = min(a.period, nst - st); ++period; }
-                --left;
-                const int bs = (int)(n % G::NB);
-                wait_on(&b_full[bs], (n / G::NB) & 1u);
-                const uint32_t bh = smem_u32(smB + bs * G::BSTAGE);
-#pragma unroll
-                for (int i = 0; i < NA; ++i) {
-                    const uint32_t as = (uint32_t)(st * NA + i) & 3u, ac = tmem + A_COL + as * 64u, d1 = tmem + (uint32_t)(i * 2 * NT), d2 = d1 + NT;
-                    if (fresh && period > 1) wait_on(&d_empty[i], (period - 2u) & 1u);      // D of the period before is read
-                    wait_on(&a_full[as], (phase >> as) & 1u);
-                    phase ^= 1u << as;
-                    tc_fence_after();
-                    if (lead) {
-                        if (fresh && st > 0) {          // D1 starts again, D2 goes on
-                            tc_mma_ts(d1, ac, tc_desc(bh), TC_IDESC<NT>, 0u);
-                            tc_mma_ts(d2, ac, tc_desc(bh + NT * 128), TC_IDESC<NT>, 1u);
-                        } else tc_mma_ts(d1, ac, tc_desc(bh), TC_IDESC<2 * NT>, st > 0 ? 1u : 0u);
-                        tc_mma_ts(d2, ac + 32u, tc_desc(bh), TC_IDESC<NT>, 1u);
-#pragma unroll
-                        for (uint32_t q = 1; q < 4; ++q) {
-                            tc_mma_ts(d1, ac + q * 8u, tc_desc(bh + q * 32u), TC_IDESC<2 * NT>, 1u);
-                            tc_mma_ts(d2, ac + 32u + q * 8u, tc_desc(bh + q * 32u), TC_IDESC<NT>, 1u);
-                        }
-                        tc_commit(&a_empty[as]);
-                        if (left == 0) tc_commit(&d_full[i]);
-                        if (i == NA - 1) tc_commit(&b_empty[bs]);
-                    }
-                    __syncwarp();
+                if (fresh) {                            // D of the period before must have been read
+                    if (periods) wait_on(&d_empty, (periods - 1u) & 1u);
+                    left = min(a.period, nst - st);
+                    ++periods;
                 }
+                --left;
+                wait_on(&b_full[bs], b_par);
+                wait_on(&a_full[g_at], (a_par >> g_at) & 1u);
+                tc_fence_after();
+                const uint32_t ac = tmem + A_COL + g_at * 64u, bh = b_lo + bs * (uint32_t)(G::BSTAGE / 16);
+                if (lead) {
+                    if (fresh && st > 0) {              // D1 starts again, D2 goes on
+                        tc_mma_ts(d1, ac, desc(bh), TC_IDESC<NT>, 0u);
+                        tc_mma_ts(d2, ac, desc(bh + NT * 8), TC_IDESC<NT>, 1u);
+                    } else tc_mma_ts(d1, ac, desc(bh), TC_IDESC<2 * NT>, st > 0 ? 1u : 0u);
+                    tc_mma_ts(d2, ac + 32u, desc(bh), TC_IDESC<NT>, 1u);
+#pragma unroll
+                    for (uint32_t q = 1; q < 4; ++q) {
+                        tc_mma_ts(d1, ac + q * 8u, desc(bh + q * 2u), TC_IDESC<2 * NT>, 1u);
+                        tc_mma_ts(d2, ac + 32u + q * 8u, desc(bh + q * 2u), TC_IDESC<NT>, 1u);
+                    }
+                    tc_commit(&a_empty[g_at]);
+                    tc_commit(&b_empty[bs]);
+                    if (left == 0) tc_commit(&d_full);
+                }
+                a_par ^= 1u << g_at;
+                g_at = (g_at + 1u) % TC_GROUPS;
+                if (++bs == (uint32_t)G::NB) { bs = 0; b_par ^= 1u; }
+                __syncwarp();
             }
         }
     } else {
         // ---- weights, and the end of a tile ----
         const int grp = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane;       // row = this lane's TMEM lane
-        const int mine = NA == 2 ? grp & 1 : 0;         // which 128 rows of the tile this group rebuilds and reads back
         const uint32_t tlane = tmem + ((uint32_t)(quarter * 32) << 16);
-        uint8_t* ring = sm + G::NB * G::BSTAGE + warp * G::R * G::SLOT;
+        uint8_t* ring = sm + G::RING + warp * G::R * G::SLOT;
+        [[maybe_unused]] float* xch = reinterpret_cast<float*>(sm + G::XCH) + grp * 1024;
         const uint32_t ring_s = smem_u32(ring);
-        const WeightRef w = (PAIR && mine) ? a.w1 : a.w0;
+        const WeightRef w = (PAIR && quarter >= 2) ? a.w1 : a.w0;                      // lanes 64..127 of a pair: up rows
         const bool scales_async = WT == WT_Q4_K || ((a.units & 1) == 0 && ((uintptr_t)w.d & 3) == 0);
-        // Tiles of an item in the order of the products: number t = step * NA + i.  This group takes t = grp, grp + 4, ... of
-        // every item and always uses ring slot grp: a slot that changed hands could be waited for by a group that has not
-        // followed its phases, and a wait on a phase two ahead returns at once.
-        constexpr int SS = TC_GROUPS / NA;              // steps from one to the next
-        const int s0 = grp / NA, n_own = (nst - s0 + SS - 1) / SS;
-        auto step_of = [&](int j) { return s0 + SS * j; };
-        auto row_of = [&](int tn, int r) { return min((PAIR ? tn * 128 : (tn * NA + mine) * 128) + r, a.N - 1); };
+        // This group takes steps grp, grp + 4, ... of every item and always uses ring slot grp: a slot that changed hands
+        // could be waited for by a group that has not followed its phases, and a wait on a phase two ahead returns at once.
+        const int n_own = (nst - grp + TC_GROUPS - 1) / TC_GROUPS;
+        auto step_of = [&](int j) { return grp + TC_GROUPS * j; };
+        auto row_of = [&](int tn, int r) { return min(PAIR ? tn * 64 + (r & 63) : tn * 128 + r, a.N - 1); };
         const int rpu = WT == WT_Q4_0 ? a.units : (a.units >> 3) * 9;                   // uint4 per weight row
         const int n_items = first < a.items ? (a.items - first + stride - 1) / stride : 0;
 
@@ -504,7 +503,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
 
         // D1 (and, with the item's last period, D2) into acc; the end of an item: scale back, activation, store
         const bool reads = grp < READERS;
-        const int c0 = grp / NA * COLS;
+        const int c0 = grp * COLS;
         const int np = (nst + a.period - 1) / a.period;                                 // periods per item
         bool waited = false;
         int done = 0, done_item = 0, done_p = 0;        // periods read out: in all, as (item, period of the item)
@@ -514,10 +513,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
         auto read_out = [&]() {
             if (!waited) { pdl_wait(); waited = true; }
             const bool last = done_p == np - 1;
-            wait_on(&d_full[mine], (uint32_t)done & 1u);
+            wait_on(&d_full, (uint32_t)done & 1u);
             tc_fence_after();
             {
-                const uint32_t col = tlane + (uint32_t)(mine * 2 * NT + c0);
+                const uint32_t col = tlane + (uint32_t)c0;
 #pragma unroll
                 for (int ch = 0; ch < COLS / 16; ++ch) {
                     float v[16];
@@ -539,70 +538,63 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&d_empty[mine]);
+            if (lane == 0) mbar_arrive(&d_empty);
             ++done; ++done_p;
             if (!last) return;
             const int item = first + done_item * stride, tn = item % a.tiles_n, m0 = item / a.tiles_n * NT;
             done_p = 0; ++done_item;
-            const int n_out = (PAIR ? tn * 128 : (tn * NA + mine) * 128) + row, n_col = min(NT, a.B - m0);
-            const float inv0 = m0 + lane < a.B ? a.inv[m0 + lane] : 0.f, inv1 = NT > 32 && m0 + 32 + lane < a.B ? a.inv[m0 + 32 + lane] : 0.f;
+            const int n_out = PAIR ? tn * 64 + (row & 63) : tn * 128 + row, n_col = min(NT, a.B - m0);
             float* yp = a.y + (size_t)m0 * a.ldy + n_out;
-            auto inv_of = [&](int c) { return __shfl_sync(0xffffffffu, c < 32 ? inv0 : inv1, c & 31); };
+            const float inv_mine = m0 + c0 + lane < a.B ? a.inv[m0 + c0 + lane] : 0.f;         // of this group's columns (COLS <= 32)
             auto act = [&](float gate, float up) { return (a.swiglu ? silu_clip(gate) : gelu_tanh(gate)) * up; };
             if (S > 1) {
                 // one item per cluster: sums into the exchange (the activation ring is drained), then every CTA finishes the
                 // columns c = split, split + S, ... from all S parts
                 float* ex = reinterpret_cast<float*>(smB);
-                if constexpr (NA == 2) wait_on(&d_full[mine ^ 1], (uint32_t)(done - 1) & 1u);      // the other tile's last products read the ring too
-                if (reads) {
 #pragma unroll
-                    for (int c = 0; c < COLS; ++c) ex[(mine * NT + c0 + c) * 128 + row] = acc[c];
-                }
+                for (int c = 0; c < COLS; ++c) ex[(c0 + c) * 128 + row] = acc[c];
                 cl_arrive();
                 cl_wait();
                 const uint32_t ex_s = smem_u32(ex);
-                auto total_of = [&](int i, int c) {             // all loads in flight, then one order of addition
+                auto total_of = [&](int c, int r) {             // all loads in flight, then one order of addition
                     float p[8], v = 0.f;
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) p[q] = q < S ? ld_cluster(ex_s + (uint32_t)((i * NT + c) * 128 + row) * 4u, (uint32_t)q) : 0.f;
+                    for (int q = 0; q < 8; ++q) p[q] = q < S ? ld_cluster(ex_s + (uint32_t)(c * 128 + r) * 4u, (uint32_t)q) : 0.f;
 #pragma unroll
                     for (int q = 0; q < 8; ++q) v += p[q];
                     return v;
                 };
-                if constexpr (PAIR || NA == 1) {                // all groups share the columns
-                    for (int c = split + S * grp; c < n_col; c += READERS * S) {
-                        const float sc = inv_of(c), v = total_of(0, c);
-                        if constexpr (PAIR) { const float u = total_of(1, c); if (n_out < a.N) yp[(size_t)c * a.ldy] = act(v * sc, u * sc); }
-                        else if (n_out < a.N) yp[(size_t)c * a.ldy] = v * sc;
-                    }
-                } else {
-                    for (int c = split + S * (grp >> 1); c < n_col; c += READERS / 2 * S) {
-                        const float v = total_of(mine, c) * inv_of(c);
-                        if (n_out < a.N) yp[(size_t)c * a.ldy] = v;
-                    }
+                // a pair's 64 rows: each half of the lanes takes its own columns
+                const int lanes = PAIR ? 2 : 1, sub = PAIR ? row >> 6 : 0;
+                for (int c = split + S * (grp * lanes + sub); c < n_col; c += READERS * lanes * S) {
+                    const float sc = a.inv[m0 + c], v = total_of(c, PAIR ? row & 63 : row);
+                    if constexpr (PAIR) { const float u = total_of(c, 64 + (row & 63)); if (n_out < a.N) yp[(size_t)c * a.ldy] = act(v * sc, u * sc); }
+                    else if (n_out < a.N) yp[(size_t)c * a.ldy] = v * sc;
                 }
                 cl_arrive();
                 cl_wait();
             } else if constexpr (PAIR) {
-                // the gate group and the up group of the same columns swap half of them; the gate group finishes the first half
-                constexpr int H = COLS / 2;
-                float* x0 = reinterpret_cast<float*>(sm + G::NB * G::BSTAGE + TC_GROUPS * 4 * G::R * G::SLOT) + (grp >> 1) * COLS * 128;
-                float* put = x0 + (mine ? 0 : H * 128) + row;
-                const float* get = x0 + (mine ? H * 128 : 0) + row;
+                // gate lanes (quarters 0, 1) and up lanes (2, 3) of a row swap half of this group's columns, eight at a time,
+                // through shared memory
+                constexpr int H = COLS / 2, CH = H < 8 ? H : 8;
+                const bool up = row >= 64;
 #pragma unroll
-                for (int c = 0; c < H; ++c) put[c * 128] = mine ? acc[c] : acc[H + c];
-                asm volatile("bar.sync %0, 256;" :: "r"(1 + (grp >> 1)) : "memory");
+                for (int h0 = 0; h0 < H; h0 += CH) {
 #pragma unroll
-                for (int c = 0; c < H; ++c) {
-                    const int col = c0 + mine * H + c;
-                    const float o = get[c * 128], sc = inv_of(col), m = mine ? acc[H + c] : acc[c];
-                    if (col < n_col && n_out < a.N) yp[(size_t)col * a.ldy] = mine ? act(o * sc, m * sc) : act(m * sc, o * sc);
+                    for (int c = 0; c < CH; ++c) xch[c * 128 + row] = up ? acc[h0 + c] : acc[H + h0 + c];
+                    asm volatile("bar.sync %0, 128;" :: "r"(1 + grp) : "memory");
+#pragma unroll
+                    for (int c = 0; c < CH; ++c) {
+                        const int lc = (up ? H : 0) + h0 + c;   // gate lanes finish the first half of the columns
+                        const float o = xch[c * 128 + (row ^ 64)], sc = __shfl_sync(0xffffffffu, inv_mine, lc), m = up ? acc[H + h0 + c] : acc[h0 + c];
+                        if (c0 + lc < n_col && n_out < a.N) yp[(size_t)(c0 + lc) * a.ldy] = up ? act(o * sc, m * sc) : act(m * sc, o * sc);
+                    }
+                    asm volatile("bar.sync %0, 128;" :: "r"(1 + grp) : "memory");
                 }
-                asm volatile("bar.sync %0, 256;" :: "r"(1 + (grp >> 1)) : "memory");
             } else {
 #pragma unroll
                 for (int c = 0; c < COLS; ++c) {
-                    const float v = acc[c] * inv_of(c0 + c);
+                    const float v = acc[c] * __shfl_sync(0xffffffffu, inv_mine, c);
                     if (c0 + c < n_col && n_out < a.N) yp[(size_t)(c0 + c) * a.ldy] = v;
                 }
             }
@@ -687,12 +679,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                     // a step of block minima: -32 dmin m of 64 sub-blocks (the image holds the sums over 32 activations / 32)
                     const int sb0 = (mn0 + st) * 8, n_sb = a.units >> 3;
                     const uint4* src = w.q + (size_t)row_of(tn, row) * rpu;
+#pragma unroll 1
+                    for (int b = 0; b < 4; ++b) {
+                        uint32_t whi[8], wlo[8];
 #pragma unroll
-                    for (int b = 0; b < 2; ++b) {
-                        uint32_t whi[16], wlo[16];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const int sb = sb0 + 4 * b + e;
+                        for (int e = 0; e < 2; ++e) {
+                            const int sb = sb0 + 2 * b + e;
                             const uint4 h = __ldg(src + (size_t)min(sb, n_sb - 1) * 9);
                             const float dm = sb < n_sb ? -32.f * __half2float(__ushort_as_half((unsigned short)(h.x >> 16))) : 0.f;
 #pragma unroll
@@ -706,8 +698,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                                 wlo[4 * e + gq] = as_u32(__floats2half2_rn(v0 - f2.x, v1 - f2.y));
                             }
                         }
-                        tc_st16(acol + b * 16u, whi);
-                        tc_st16(acol + 32u + b * 16u, wlo);
+                        tc_st8(acol + b * 8u, whi);
+                        tc_st8(acol + 32u + b * 8u, wlo);
                     }
                 }
                 tc_st_wait();
@@ -746,14 +738,12 @@ bool gemm_tc_supports(int wtype, const GemvArgs& a) {
 
 typedef void (*TcKernel)(const TcGemm);
 struct TcPick { TcKernel k; int smem; bool attr; };
-template <int WT, int NA, int NT, bool PAIR> static TcPick& tc_pick() {
-    static TcPick p = {k_gemm_tc<WT, NA, NT, PAIR>, TcGeo<WT, NT, PAIR>::SMEM, false};
+template <int WT, int NT, bool PAIR> static TcPick& tc_pick() {
+    static TcPick p = {k_gemm_tc<WT, NT, PAIR>, TcGeo<WT, NT>::SMEM, false};
     return p;
 }
-template <int WT> static TcPick& tc_pick(int nt, int na, bool pair) {
-    if (pair) return nt == 16 ? tc_pick<WT, 2, 16, true>() : nt == 32 ? tc_pick<WT, 2, 32, true>() : tc_pick<WT, 2, 64, true>();
-    if (na == 2) return tc_pick<WT, 2, 64, false>();
-    return nt == 16 ? tc_pick<WT, 1, 16, false>() : nt == 32 ? tc_pick<WT, 1, 32, false>() : tc_pick<WT, 1, 64, false>();
+template <int WT, bool PAIR> static TcPick& tc_pick(int nt) {
+    return nt == 16 ? tc_pick<WT, 16, PAIR>() : nt == 32 ? tc_pick<WT, 32, PAIR>() : nt == 64 ? tc_pick<WT, 64, PAIR>() : tc_pick<WT, 128, PAIR>();
 }
 
 static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
@@ -775,23 +765,18 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
         }
         count_launch();
     }
-    // Tile and K splits: the cheapest of the candidates under an estimate in SM cycles.  A weight tile costs the larger of
-    // its tensor-core time (6 cycles per activation row), its rebuilding (about 200 issue cycles) and the fetch of its
-    // activation tile (NT * 256 bytes, shared by NA weight tiles, at about 40 bytes per cycle and SM out of L2); a CTA
-    // costs about 3000 cycles besides, a K split about 1500 more.
-    const int nt = a.B <= 16 ? 16 : a.B <= 32 ? 32 : 64;
-    const int tiles_m = (a.B + nt - 1) / nt;
-    int na = pair ? 2 : 1, S = 1;
+    // K splits: the cheapest under an estimate in SM cycles.  A step costs the larger of its tensor-core time (6 cycles per
+    // activation row) and its rebuilding (about 330 issue slots); a CTA costs about 3000 cycles besides, a split 1500 more.
+    const int nt = a.B <= 16 ? 16 : a.B <= 32 ? 32 : a.B <= 64 ? 64 : 128;
+    const int tiles_n = pair ? (a.N + 63) / 64 : (a.N + 127) / 128, tiles_m = (a.B + nt - 1) / nt;
+    const long long items = (long long)tiles_n * tiles_m;
+    int S = 1;
     double best = 1e300;
-    for (int c_na = pair ? 2 : 1; c_na <= (pair || nt == 64 ? 2 : 1); ++c_na) {
-        const long long items = (long long)(pair ? (a.N + 127) / 128 : (a.N + 128 * c_na - 1) / (128 * c_na)) * tiles_m;
-        const double tile = fmax(fmax(6.0 * nt, 200.0), nt * 256.0 / c_na / 40.0);
-        for (int s = 1; s <= 8 && s <= n_main; s *= 2) {
-            const double waves = (double)((items * s + g.sm_count - 1) / g.sm_count);
-            const int steps = (n_main + s - 1) / s + (n_min + s - 1) / s;
-            const double cost = waves * (steps * c_na * tile + (s > 1 ? 4500.0 : 3000.0));
-            if (cost < best * 0.999) { best = cost; na = c_na; S = s; }
-        }
+    for (int s = 1; s <= 8 && s <= n_main; s *= 2) {
+        const double waves = (double)((items * s + g.sm_count - 1) / g.sm_count);
+        const int steps = (n_main + s - 1) / s + (n_min + s - 1) / s;
+        const double cost = waves * (steps * fmax(6.0 * nt, 330.0) + (s > 1 ? 4500.0 : 3000.0));
+        if (cost < best * 0.999) { best = cost; S = s; }
     }
     TcGemm t = {};
     t.w0 = a.w0; t.w1 = a.w1; t.y = a.y; t.ldy = a.ldy; t.img = g_tc.img; t.inv = g_tc.inv; t.err = g.dev_err;
@@ -799,9 +784,9 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
     t.n_min = n_min; t.n_main = n_main; t.S = S;
     const int longest = (n_main + S - 1) / S + (n_min + S - 1) / S, n_periods = (longest + TC_PERIOD - 1) / TC_PERIOD;
     t.period = (longest + n_periods - 1) / n_periods;
-    t.tiles_n = pair ? (a.N + 127) / 128 : (a.N + 128 * na - 1) / (128 * na);
-    t.items = t.tiles_n * tiles_m;
-    TcPick& p = wtype == WT_Q4_0 ? tc_pick<WT_Q4_0>(nt, na, pair) : tc_pick<WT_Q4_K>(nt, na, pair);
+    t.tiles_n = tiles_n;
+    t.items = (int)items;
+    TcPick& p = wtype == WT_Q4_0 ? (pair ? tc_pick<WT_Q4_0, true>(nt) : tc_pick<WT_Q4_0, false>(nt)) : (pair ? tc_pick<WT_Q4_K, true>(nt) : tc_pick<WT_Q4_K, false>(nt));
     if (!p.attr) {
         if (cudaFuncSetAttribute((const void*)p.k, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem) != cudaSuccess)
             return fail(ADAMAH_ERR_BACKEND, "gemm_tc: cannot raise the shared-memory limit");
