@@ -309,8 +309,7 @@ __device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, u
 //                added up (measured: 5e-9 of the result each).  So the cross terms, 2^-11 of the result, have D2 to
 //                themselves, and every `period` steps D1 is added to registers and restarted.  Relative error of a
 //                1152 x 6912 product: 6.1e-6 with one accumulator for all of K, 4e-7 with this.
-//   read-out     The same warps read D1, each group its share of the columns, after it has produced its first tile of the
-//                next period, so that the pause of the tensor core is short.
+//   read-out     The same warps read D1, each group its share of the columns, as soon as it is complete.
 //   K splits     where the tiles alone leave SMs idle, S CTAs of a cluster take a part of K each, leave their sums in their
 //                own shared memory and add each other's columns through distributed shared memory (in split order: results
 //                do not depend on timing).
@@ -619,6 +618,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                 else hdr = *reinterpret_cast<const uint4*>(slot + 1024 + lane * 16);
                 __syncwarp();
                 fetch();
+                if (reads) {
+                    // Where this group's tile before was the last of a period, D is read first: the tensor core waits for that,
+                    // while the tile that comes now is four steps away (producing first: 3300 idle cycles per period).
+                    const int ended = st >= TC_GROUPS ? k * np + (st - TC_GROUPS + 1) / a.period : (nst - 1 - grp) % TC_GROUPS == 0 ? k * np : 0;
+                    while (done < ended) read_out();
+                }
                 if (n) {                                // the tensor core is done with this group's tile before
                     if (!waited) { pdl_wait(); waited = true; }
                     wait_on(&a_empty[grp], (n - 1u) & 1u);
