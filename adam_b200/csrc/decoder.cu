@@ -909,6 +909,17 @@ static int enqueue_part(Decoder* D, uint32_t batch, uint32_t part, bool with_lm,
     } else if (part == 2 * d.n_layer) {
         if (with_lm) {
             const Mat& lm = D->output.bound ? D->output : D->embd;
+            GemvArgs a = {};
+            a.ldx = (int)E; a.eps = d.norm_eps; a.h_in = D->hbuf[1]; a.add_src = D->proj;
+            a.w_post = D->layers[d.n_layer - 1].norm[NORM_POST_FFW]; a.w_pre = D->output_norm; a.h_out = D->hbuf[0];
+            a.y = want_logits ? D->logits : nullptr; a.ldy = (int)lm.rows; a.softcap = d.final_softcap;
+            a.out_tok = D->cur_tok; a.out_val = D->cur_val;
+            a.w0 = lm.w; a.N = (int)lm.rows; a.K = (int)lm.cols; a.B = (int)batch; a.epi = EPI_ARGMAX;
+            if (gemm_tc_supports(lm.wtype, a)) {
+                if ((rc = launch_gemm_tc(lm.wtype, a, g.stream))) return rc;
+                D->h_final = 0;
+                return check_launch("decoder step");
+            }
             if (wt_is_b8(lm.wtype)) {
                 // Q8_0 / Q5_0 LM head: the norm chain, the products and the arg-max as three kernels; the products land
                 // in the logits buffer (soft-capped afterwards only when the caller wants them)
@@ -919,11 +930,6 @@ static int enqueue_part(Decoder* D, uint32_t batch, uint32_t part, bool with_lm,
                 D->h_final = 0;
                 return check_launch("decoder step");
             }
-            GemvArgs a = {};
-            a.ldx = (int)E; a.eps = d.norm_eps; a.h_in = D->hbuf[1]; a.add_src = D->proj;
-            a.w_post = D->layers[d.n_layer - 1].norm[NORM_POST_FFW]; a.w_pre = D->output_norm; a.h_out = D->hbuf[0];
-            a.y = want_logits ? D->logits : nullptr; a.ldy = (int)lm.rows; a.softcap = d.final_softcap;
-            a.out_tok = D->cur_tok; a.out_val = D->cur_val;
             if ((rc = argmax_scratch(&a.part_val, &a.part_idx, &a.ticket))) return rc;
             if ((rc = gemv(lm, nullptr, a, batch, EPI_ARGMAX))) return rc;
             D->h_final = 0;

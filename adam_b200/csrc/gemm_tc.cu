@@ -9,6 +9,7 @@
 //   Q4_K  w = d (sc q) - dmin m: the first product has 21 bits and splits the same way; the second is the same for 32
 //         neighbouring weights, so it becomes one more "weight" per 32 that multiplies the sum of their 32 activations
 //         (a few extra steps of K, 1/32 of the work)
+//   Q8_0  w = d q: 19 bits, as Q4_0
 // and w_hi x_hi + w_lo x_hi + w_hi x_lo is accumulated over K in fp32 (w_lo x_lo lies below 2^-22 of the product).
 // Limit: |w| < 65504, what fp16 holds.
 //
@@ -33,7 +34,7 @@ constexpr int TC_STEP_IMG = TC_GROUP * 128;             // one plane of one grou
 constexpr size_t TC_IMG_MAX = 256u << 20;               // largest image kept; longer calls run in row chunks
 constexpr int TC_MAX_K = 32768;
 
-struct TcWork { uint8_t* img; size_t img_cap; float* inv; int inv_cap; std::vector<void*> retired; };
+struct TcWork { uint8_t* img; size_t img_cap; float* inv; int inv_cap; unsigned long long* best; std::vector<void*> retired; };   // best: arg-max keys [inv_cap], then a ticket
 static TcWork g_tc = {};
 static uint64_t g_tc_calls = 0;
 static int g_tc_policy = -1;             // 0 never, 1 where it is expected to be faster, 2 whenever the shape allows; -1 = take it from ADAM_B200_TC
@@ -66,6 +67,7 @@ bool gemm_tc_prepare(int rows, int K) {
     }
     if (pad > g_tc.inv_cap) {
         const int cap = pad > 2 * g_tc.inv_cap ? pad : 2 * g_tc.inv_cap;
+        if (!grow((void**)&g_tc.best, (size_t)cap * 8 + 8)) return false;
         if (!grow((void**)&g_tc.inv, (size_t)cap * 4)) return false;
         g_tc.inv_cap = cap;
     }
@@ -73,7 +75,7 @@ bool gemm_tc_prepare(int rows, int K) {
 }
 
 void gemm_tc_release() {
-    cudaFree(g_tc.img); cudaFree(g_tc.inv);
+    cudaFree(g_tc.img); cudaFree(g_tc.inv); cudaFree(g_tc.best);
     for (void* p : g_tc.retired) cudaFree(p);
     g_tc = TcWork{};
 }
@@ -326,10 +328,14 @@ struct TcGemm {
     int N, units, B, swiglu;                            // units = K / 32
     int n_min, n_main, tiles_n, items;                  // items = tiles_n * tiles of NT rows
     int S, period;                                      // K splits; steps per accumulation period
+    unsigned long long* best; unsigned int* ticket;     // arg-max: one key per activation row (0 between launches), CTAs that are done
+    int* out_tok; float *out_val, *out_tok_f32, softcap;
 };
+enum { TC_STORE = 0, TC_PAIR = 1, TC_ARGMAX = 2 };       // what becomes of a product: stored, gate/up pairs, arg-max per activation row (and stored)
 template <int WT, int NT> struct TcGeo {
-    static constexpr int R = 4;                                              // weight ring: tiles ahead per warp
-    static constexpr int SLOT = 1024 + (WT == WT_Q4_0 ? 128 : 512);          // 32 rows: nibbles, then block scales / superblock headers
+    static constexpr int R = WT == WT_Q8_0 && NT == 128 ? 2 : 4;             // weight ring: tiles ahead per warp
+    static constexpr int QB = WT == WT_Q8_0 ? 64 : 32;                       // bytes of a row's codes per step
+    static constexpr int SLOT = 32 * QB + (WT == WT_Q4_K ? 512 : 128);       // 32 rows: codes, then block scales / superblock headers
     static constexpr int NB = NT == 128 ? 3 : 4;
     static constexpr int BSTAGE = NT * 256;
     static constexpr int RING = NB * BSTAGE, XCH = RING + TC_GROUPS * 4 * R * SLOT;     // offsets: weight rings, gate / up exchange (4 KB per group)
@@ -341,9 +347,10 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
     return p != 0;
 }
-template <int WT, int NT, bool PAIR>
+template <int WT, int NT, int MODE>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
     using G = TcGeo<WT, NT>;
+    constexpr bool PAIR = MODE == TC_PAIR;
     extern __shared__ __align__(1024) uint8_t sm_raw[];
     uint8_t* sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);     // the swizzle works on address bits
     uint8_t* smB = sm;
@@ -466,33 +473,34 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
         const int n_own = (nst - grp + TC_GROUPS - 1) / TC_GROUPS;
         auto step_of = [&](int j) { return grp + TC_GROUPS * j; };
         auto row_of = [&](int tn, int r) { return min(PAIR ? tn * 64 + (r & 63) : tn * 128 + r, a.N - 1); };
-        const int rpu = WT == WT_Q4_0 ? a.units : (a.units >> 3) * 9;                   // uint4 per weight row
+        const int rpu = WT == WT_Q4_0 ? a.units : WT == WT_Q8_0 ? 2 * a.units : (a.units >> 3) * 9;     // uint4 per weight row
         const int n_items = first < a.items ? (a.items - first + stride - 1) / stride : 0;
 
         // fetch cursor, R tiles ahead of the production cursor
         int f_item = 0, f_j = 0; uint32_t f_n = 0;
-        const uint4 *f_q[2] = {nullptr, nullptr}, *f_h = nullptr; const __half* f_d = nullptr;
+        constexpr int LPR = G::QB / 16, FI = LPR;       // lanes per row and copies per lane of a step's codes
+        const uint4 *f_q[FI], *f_h = nullptr; const __half* f_d = nullptr;
         auto fetch = [&]() {
             if (f_item < n_items && n_own > 0) {
                 if (f_j == 0) {
                     const int tn = (first + f_item * stride) % a.tiles_n;
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) f_q[h] = w.q + (size_t)row_of(tn, quarter * 32 + 16 * h + (lane >> 1)) * rpu;
-                    if constexpr (WT == WT_Q4_0) f_d = w.d + (size_t)row_of(tn, row) * a.units;
+                    for (int h = 0; h < FI; ++h) f_q[h] = w.q + (size_t)row_of(tn, quarter * 32 + (32 / FI) * h + lane / LPR) * rpu;
+                    if constexpr (WT != WT_Q4_K) f_d = w.d + (size_t)row_of(tn, row) * a.units;
                     else f_h = w.q + (size_t)row_of(tn, row) * rpu;
                 }
                 const int st = step_of(f_j), ks = ma0 + st - nmn;
                 if (st >= nmn) {
                     const uint32_t dst = ring_s + (f_n % G::R) * G::SLOT;
-                    const int half = lane & 1;
-                    const int off = WT == WT_Q4_0 ? min(2 * ks + half, a.units - 1) : (ks >> 2) * 9 + 1 + (ks & 3) * 2 + half;
+                    const int piece = lane % LPR;
+                    const int off = WT == WT_Q4_K ? (ks >> 2) * 9 + 1 + (ks & 3) * 2 + piece : min(LPR * ks + piece, rpu - 1);
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int rl = 16 * h + (lane >> 1);
-                        cp_async16(dst + rl * 32 + ((half ^ ((rl >> 2) & 1)) << 4), f_q[h] + off);
+                    for (int h = 0; h < FI; ++h) {      // 16-byte pieces are stored rotated: the reads below are free of bank conflicts
+                        const int rl = (32 / FI) * h + lane / LPR;
+                        cp_async16(dst + rl * G::QB + ((LPR == 2 ? piece ^ ((rl >> 2) & 1) : piece ^ ((rl >> 1) & 3)) << 4), f_q[h] + off);
                     }
-                    if constexpr (WT == WT_Q4_0) { if (scales_async) cp_async4(dst + 1024 + lane * 4, f_d + 2 * ks); }
-                    else cp_async16_l1(dst + 1024 + lane * 16, f_h + (ks >> 2) * 9);
+                    if constexpr (WT != WT_Q4_K) { if (scales_async) cp_async4(dst + 32 * G::QB + lane * 4, f_d + 2 * ks); }
+                    else cp_async16_l1(dst + 32 * G::QB + lane * 16, f_h + (ks >> 2) * 9);
                 }
                 if (++f_j == n_own) { f_j = 0; ++f_item; }
             }
@@ -507,6 +515,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
         bool waited = false;
         int done = 0, done_item = 0, done_p = 0;        // periods read out: in all, as (item, period of the item)
         float acc[COLS];
+        [[maybe_unused]] unsigned long long best = 0;
 #pragma unroll
         for (int c = 0; c < COLS; ++c) acc[c] = 0.f;
         auto read_out = [&]() {
@@ -594,8 +603,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
 #pragma unroll
                 for (int c = 0; c < COLS; ++c) {
                     const float v = acc[c] * __shfl_sync(0xffffffffu, inv_mine, c);
-                    if (c0 + c < n_col && n_out < a.N) yp[(size_t)(c0 + c) * a.ldy] = v;
+                    if constexpr (MODE == TC_ARGMAX) {
+                        // best of the warp's rows: NaN counts as -FLT_MAX, ties go to the lower row; lane c keeps column c's
+                        const float f = (v == v ? v : -3.402823466e+38f) + 0.f;
+                        const uint32_t bits = __float_as_uint(f), ord = n_out < a.N ? bits ^ ((uint32_t)((int)bits >> 31) | 0x80000000u) : 0u;
+                        const uint32_t top = __reduce_max_sync(0xffffffffu, ord);
+                        const uint32_t at = __reduce_min_sync(0xffffffffu, ord == top ? (uint32_t)n_out : 0xffffffffu);
+                        const unsigned long long key = ((unsigned long long)top << 32) | (0xffffffffu - at);
+                        if (lane == c && key > best) best = key;
+                        if (a.y && c0 + c < n_col && n_out < a.N) yp[(size_t)(c0 + c) * a.ldy] = a.softcap > 0.f ? tanhf(v / a.softcap) * a.softcap : v;
+                    } else if (c0 + c < n_col && n_out < a.N) yp[(size_t)(c0 + c) * a.ldy] = v;
                 }
+                if constexpr (MODE == TC_ARGMAX)
+                    if (a.B > NT || done_item == n_items) {     // the columns change with the next item, or there is none
+                        if (lane < COLS && c0 + lane < n_col) atomicMax(a.best + m0 + c0 + lane, best);
+                        best = 0;
+                    }
             }
 #pragma unroll
             for (int c = 0; c < COLS; ++c) acc[c] = 0.f;
@@ -611,11 +634,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                 cp_wait<G::R - 1>();
                 __syncwarp();
                 const uint8_t* slot = ring + (n % G::R) * G::SLOT;
-                const uint4 q0 = *reinterpret_cast<const uint4*>(slot + lane * 32 + (((lane >> 2) & 1) << 4));
-                const uint4 q1 = *reinterpret_cast<const uint4*>(slot + lane * 32 + (((~lane >> 2) & 1) << 4));
+                uint32_t qw[G::QB / 4];                 // this row's codes of the step
+#pragma unroll
+                for (int p = 0; p < LPR; ++p) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(slot + lane * G::QB + ((LPR == 2 ? p ^ ((lane >> 2) & 1) : p ^ ((lane >> 1) & 3)) << 4));
+                    qw[4 * p] = v.x; qw[4 * p + 1] = v.y; qw[4 * p + 2] = v.z; qw[4 * p + 3] = v.w;
+                }
                 uint32_t d01 = 0; uint4 hdr = make_uint4(0, 0, 0, 0);
-                if constexpr (WT == WT_Q4_0) d01 = *reinterpret_cast<const uint32_t*>(slot + 1024 + lane * 4);
-                else hdr = *reinterpret_cast<const uint4*>(slot + 1024 + lane * 16);
+                if constexpr (WT != WT_Q4_K) d01 = *reinterpret_cast<const uint32_t*>(slot + 32 * G::QB + lane * 4);
+                else hdr = *reinterpret_cast<const uint4*>(slot + 32 * G::QB + lane * 16);
                 __syncwarp();
                 fetch();
                 if (reads) {
@@ -629,8 +656,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                     wait_on(&a_empty[grp], (n - 1u) & 1u);
                     tc_fence_after();
                 }
-                const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-                if constexpr (WT == WT_Q4_0) {
+                if constexpr (WT != WT_Q4_K) {
                     if (!scales_async) {                // odd number of blocks per row: their scales are not pairs of aligned halves
                         const unsigned short* dp = reinterpret_cast<const unsigned short*>(w.d) + (size_t)row_of(tn, row) * a.units + 2 * ks;
                         d01 = (uint32_t)dp[0] | (2 * ks + 1 < a.units ? (uint32_t)dp[1] << 16 : 0u);
@@ -639,6 +665,21 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                     for (int b = 0; b < 2; ++b) {       // columns 16 b ..: values 0..15 of the block from the low nibbles, 16..31 from the high ones
                         const __half2 d = as_h2((b ? d01 >> 16 : d01 & 0xFFFFu) * 0x10001u);
                         uint32_t whi[8], wlo[8], v[2];
+                        if constexpr (WT == WT_Q8_0) {  // bytes + 128 into the mantissa of 1024, two at a time
+#pragma unroll
+                            for (int y = 0; y < 2; ++y) {
+#pragma unroll
+                                for (int x = 0; x < 4; ++x) {
+                                    const uint32_t u = qw[8 * b + 4 * y + x] ^ 0x80808080u;
+                                    v[0] = (u & 0x00FF00FFu) | 0x64006400u; v[1] = ((u >> 8) & 0x00FF00FFu) | 0x64006400u;
+#pragma unroll
+                                    for (int p = 0; p < 2; ++p) split_h2(__hadd2(as_h2(v[p]), __float2half2_rn(-1152.f)), d, whi[2 * x + p], wlo[2 * x + p]);
+                                }
+                                tc_st8(acol + b * 16u + y * 8u, whi);
+                                tc_st8(acol + 32u + b * 16u + y * 8u, wlo);
+                            }
+                            continue;
+                        }
 #pragma unroll
                         for (int x = 0; x < 4; ++x) {
                             nib_pairs<false>(qw[4 * b + x], v);
@@ -718,9 +759,26 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
         cp_wait<0>();
     }
     if (S > 1 && (warp >= TC_LOADER || (warp >> 2) >= READERS)) { cl_arrive(); cl_wait(); cl_arrive(); cl_wait(); }
+    if constexpr (MODE == TC_ARGMAX) __threadfence();
     __syncthreads();
     tc_fence_after();
     if (warp == TC_ISSUER) tc_dealloc(tmem, 512);
+    if constexpr (MODE == TC_ARGMAX) {                  // the last CTA to end decodes the winners and clears the keys
+        if (tid == 0) s_tmem = atomicAdd(a.ticket, 1u);
+        __syncthreads();
+        if (s_tmem != gridDim.x - 1) return;
+        __threadfence();
+        for (int b = tid; b < a.B; b += TC_THREADS) {
+            const unsigned long long key = __ldcg(a.best + b);
+            const uint32_t ord = (uint32_t)(key >> 32);
+            const int tok = (int)(0xffffffffu - (uint32_t)key);
+            if (a.out_tok) a.out_tok[b] = tok;
+            if (a.out_tok_f32) a.out_tok_f32[b] = (float)tok;
+            if (a.out_val) a.out_val[b] = __uint_as_float(ord & 0x80000000u ? ord ^ 0x80000000u : ~ord);
+            a.best[b] = 0;
+        }
+        if (tid == 0) *a.ticket = 0u;
+    }
 }
 
 // ---- host ----------------------------------------------------------------------------------------------------------
@@ -728,31 +786,38 @@ static bool tc_policy_takes(int wtype, const GemvArgs& a, bool pair) {
     if (g_tc_policy < 0) g_tc_policy = getenv("ADAM_B200_TC") ? atoi(getenv("ADAM_B200_TC")) : 1;
     if (g_tc_policy == 0) return false;
     if (g_tc_policy == 2) return true;
-    (void)wtype; (void)a; (void)pair;
-    return true;
+    (void)wtype; (void)pair;
+    static const int mr = getenv("TCMIN") ? atoi(getenv("TCMIN")) : 9;
+    static const int ml = getenv("TCLM") ? atoi(getenv("TCLM")) : 9;
+    return a.B >= (a.epi == EPI_ARGMAX ? ml : mr);
 }
 
 bool gemm_tc_supports(int wtype, const GemvArgs& a) {
-    if (wtype != WT_Q4_0 && wtype != WT_Q4_K) return false;
-    if (a.B < TC_MIN_ROWS || (a.epi != EPI_STORE && a.epi != EPI_GEGLU && a.epi != EPI_SWIGLU)) return false;
-    if (a.K <= 0 || a.K > TC_MAX_K || a.N < 16 || !a.y || (wtype == WT_Q4_0 ? (a.K % 32) : (a.K % 256))) return false;
+    const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU;
+    if (wtype != WT_Q4_0 && wtype != WT_Q4_K && (wtype != WT_Q8_0 || pair)) return false;
+    if (a.B < TC_MIN_ROWS || a.K <= 0 || a.K > TC_MAX_K || a.N < 16 || (!a.y && a.epi != EPI_ARGMAX) || (wtype == WT_Q4_K ? (a.K % 256) : (a.K % 32))) return false;
+    if (a.epi == EPI_ARGMAX && a.B > tc_rows_fit(wtype, a.K)) return false;
     if ((a.ldx & 3) || (!a.h_in && (!a.x || ((uintptr_t)a.x & 15)))) return false;
-    if (!tc_policy_takes(wtype, a, a.epi != EPI_STORE)) return false;
+    if (!tc_policy_takes(wtype, a, pair)) return false;
     return tc_rows_fit(wtype, a.K) >= 128;
 }
 
 typedef void (*TcKernel)(const TcGemm);
 struct TcPick { TcKernel k; int smem; bool attr; };
-template <int WT, int NT, bool PAIR> static TcPick& tc_pick() {
-    static TcPick p = {k_gemm_tc<WT, NT, PAIR>, TcGeo<WT, NT>::SMEM, false};
+template <int WT, int NT, int MODE> static TcPick& tc_pick() {
+    static TcPick p = {k_gemm_tc<WT, NT, MODE>, TcGeo<WT, NT>::SMEM, false};
     return p;
 }
-template <int WT, bool PAIR> static TcPick& tc_pick(int nt) {
-    return nt == 16 ? tc_pick<WT, 16, PAIR>() : nt == 32 ? tc_pick<WT, 32, PAIR>() : nt == 64 ? tc_pick<WT, 64, PAIR>() : tc_pick<WT, 128, PAIR>();
+template <int WT, int MODE> static TcPick& tc_pick(int nt) {
+    return nt == 16 ? tc_pick<WT, 16, MODE>() : nt == 32 ? tc_pick<WT, 32, MODE>() : nt == 64 ? tc_pick<WT, 64, MODE>() : tc_pick<WT, 128, MODE>();
+}
+template <int WT> static TcPick& tc_pick(int nt, int mode) {
+    if constexpr (WT != WT_Q8_0) { if (mode == TC_PAIR) return tc_pick<WT, TC_PAIR>(nt); }
+    return mode == TC_ARGMAX ? tc_pick<WT, TC_ARGMAX>(nt) : tc_pick<WT, TC_STORE>(nt);
 }
 
 static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
-    const bool pair = a.epi != EPI_STORE;
+    const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU;
     const int n_min = tc_min_steps(wtype, a.K), n_main = tc_main_steps(a.K), n4 = a.K / 4;
     {   // one CTA per row; the fewest float4 per thread that 512 threads allow
         const int cand[5] = {1, 2, 4, 8, 16};
@@ -777,7 +842,7 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
     const long long items = (long long)tiles_n * tiles_m;
     int S = 1;
     double best = 1e300;
-    for (int s = 1; s <= 8 && s <= n_main; s *= 2) {
+    for (int s = 1; s <= (a.epi == EPI_ARGMAX ? 1 : 8) && s <= n_main; s *= 2) {
         const double waves = (double)((items * s + g.sm_count - 1) / g.sm_count);
         const int steps = (n_main + s - 1) / s + (n_min + s - 1) / s;
         const double cost = waves * (steps * fmax(6.0 * nt, 330.0) + (s > 1 ? 4500.0 : 3000.0));
@@ -791,7 +856,12 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
     t.period = (longest + n_periods - 1) / n_periods;
     t.tiles_n = tiles_n;
     t.items = (int)items;
-    TcPick& p = wtype == WT_Q4_0 ? (pair ? tc_pick<WT_Q4_0, true>(nt) : tc_pick<WT_Q4_0, false>(nt)) : (pair ? tc_pick<WT_Q4_K, true>(nt) : tc_pick<WT_Q4_K, false>(nt));
+    const int mode = pair ? TC_PAIR : a.epi == EPI_ARGMAX ? TC_ARGMAX : TC_STORE;
+    if (mode == TC_ARGMAX) {
+        t.best = g_tc.best; t.ticket = (unsigned int*)(g_tc.best + g_tc.inv_cap);
+        t.out_tok = a.out_tok; t.out_val = a.out_val; t.out_tok_f32 = a.out_tok_f32; t.softcap = a.softcap;
+    }
+    TcPick& p = wtype == WT_Q4_0 ? tc_pick<WT_Q4_0>(nt, mode) : wtype == WT_Q4_K ? tc_pick<WT_Q4_K>(nt, mode) : tc_pick<WT_Q8_0>(nt, mode);
     if (!p.attr) {
         if (cudaFuncSetAttribute((const void*)p.k, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem) != cudaSuccess)
             return fail(ADAMAH_ERR_BACKEND, "gemm_tc: cannot raise the shared-memory limit");
@@ -815,7 +885,7 @@ int launch_gemm_tc(int wtype, const GemvArgs& a, cudaStream_t stream) {
         if (a.h_in) c.h_in = a.h_in + (size_t)b0 * a.ldx;
         if (a.add_src) c.add_src = a.add_src + (size_t)b0 * a.ldx;
         if (a.h_out) c.h_out = a.h_out + (size_t)b0 * a.ldx;
-        c.y = a.y + (size_t)b0 * a.ldy;
+        if (a.y) c.y = a.y + (size_t)b0 * a.ldy;
         const int rc = launch_rows(wtype, c, stream);
         if (rc) return rc;
     }

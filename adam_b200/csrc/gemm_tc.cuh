@@ -6,7 +6,7 @@
 
 namespace ab {
 
-constexpr int TC_MIN_ROWS = 9;         // fewer rows than this stay on the GEMV kernels
+constexpr int TC_MIN_ROWS = 2;         // fewer rows than this stay on the GEMV kernels
 
 // Can this problem run on the tcgen05 path?  (STORE / GEGLU / SWIGLU epilogues, TC_MIN_ROWS rows and more.)
 bool gemm_tc_supports(int wtype, const GemvArgs& a);

@@ -548,6 +548,12 @@ int weight_ref(const Map* m, uint64_t off, uint64_t n_elems, int* wtype, WeightR
 // Run a GEMV on the tensor at (map, off): the tensor-core kernel when a row-tiled
 // copy of exactly this tensor is registered and the shape fits, the generic one otherwise.
 int run_gemv(uint32_t map_id, uint64_t off, int wtype, GemvArgs& ga) {
+    if (ga.B >= TC_MIN_ROWS) {
+        // many rows: the tcgen05 GEMM (its workspace is allocated on first use, never inside a capture)
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(g.stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) gemm_tc_prepare(ga.B, ga.K);
+        if (gemm_tc_supports(wtype, ga)) return launch_gemm_tc(wtype, ga, g.stream);
+    }
     if (wt_is_b8(wtype)) {
         // Q8_0 / Q5_0: plain products from their own kernel; an arg-max is a second small kernel over the logits
         if (ga.h_in || ga.epi == EPI_GEGLU || ga.epi == EPI_SWIGLU) return fail(ADAMAH_ERR_INVALID, "Q8_0 / Q5_0 tensors take plain products and arg-max only");
@@ -558,12 +564,6 @@ int run_gemv(uint32_t map_id, uint64_t off, int wtype, GemvArgs& ga) {
         if (rc || ga.epi != EPI_ARGMAX) return rc;
         if (ldy != ga.N) return fail(ADAMAH_ERR_INVALID, "arg-max over Q8_0 / Q5_0 products needs densely stored logits");
         return launch_argmax_rows(y, ga.N, ga.B, ga.softcap, ga.y != nullptr, ga.out_tok, ga.out_val, ga.out_tok_f32, g.stream, false);
-    }
-    if (ga.B >= TC_MIN_ROWS) {
-        // many rows: the tcgen05 GEMM (its workspace is allocated on first use, never inside a capture)
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(g.stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) gemm_tc_prepare(ga.B, ga.K);
-        if (gemm_tc_supports(wtype, ga)) return launch_gemm_tc(wtype, ga, g.stream);
     }
     if (ga.epi != EPI_GEGLU && ga.epi != EPI_SWIGLU) {
         const void* t = find_tiled(map_id, off, (uint32_t)ga.N, (uint32_t)ga.K);
