@@ -290,208 +290,364 @@ __device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, u
 }
 
 // ---- the GEMM ---------------------------------------------------------------------------------------------------
-// One CTA per SM, 18 warps: 0..15 rebuild weights, 16 fetches activation tiles, 17 issues the tensor-core instructions.
-// A CTA's tile is 128 weight rows (or 64 gate rows in TMEM lanes 0..63 and the same 64 up rows in lanes 64..127) by NT
-// activation rows: D is 2 NT columns of TMEM, the upper half of TMEM is a ring of four weight tiles (128 rows x 64 values
-// of K as w_hi | w_lo, 64 columns).
-//   weights      A lane owns a row.  Its 32 bytes of nibbles per step come by cp.async into the warp's own ring in shared
-//                memory (R tiles ahead, across the end of a tile, two lanes per row so that a sector is fetched whole), are
-//                taken apart in fp16 pairs (4.25 instructions per two weights) and go to TMEM with tcgen05.st: no
-//                shared-memory operand image, no swizzle, no bank conflicts, and the shared memory's 128 bytes per cycle
-//                are left to the activation operand.  Four groups of four warps take the steps in turn, one ring slot
-//                each: rebuilding a tile is a chain of about 1000 cycles, and what the four schedulers lack is warps.
-//                It takes some 330 issue slots of each scheduler, which is why a tile has up to 128 activation rows (768
-//                cycles of the tensor core per step): with 64 (384 cycles) the same kernel ran at half the rate.
-//   activations  x_hi | x_lo tiles of 64 values of K by bulk copies from the image, a ring of NB stages.
+// One CTA per SM.  A CTA's tile is 128 weight rows (or 64 gate rows in TMEM lanes 0..63 and the same 64 up rows in lanes
+// 64..127) by NT activation rows: D is 2 NT columns of TMEM, the rest a ring of weight tiles (128 rows x 64 values of K as
+// w_hi | w_lo, 64 columns each).  K is walked in stages of SP steps of 64 values, NS stages in flight; a stage has one
+// barrier for everything that fills it (its activation tiles, and the warps that rebuild its weight tiles) and one that
+// the tensor core's commit releases.
+//   warp roles   Warpgroup 0: warp 0 issues the tensor-core instructions, warp 1 fetches activation tiles.  Warpgroup 1 reads
+//                results back.  The others rebuild weights, one warpgroup for each weight tile in flight.  setmaxnreg moves
+//                registers from warpgroup 0 to the reader, which holds NT sums per thread.
+//   weights      A lane owns a row.  Its codes come by cp.async into the warp's own ring in shared memory (R tiles ahead,
+//                across the end of a tile, two lanes per row so that a sector is fetched whole), are taken apart in fp16
+//                pairs (4.25 instructions per two weights) and go to TMEM with tcgen05.st: no shared-memory operand image,
+//                no swizzle, and the shared memory's 128 bytes per cycle are left to the activation operand.
+//   activations  x_hi | x_lo tiles of 64 values of K by bulk copies from the image.
 //   products     per 16 values of K two tcgen05.mma (M 128): w_hi x [x_hi | x_lo] with N = 2 NT into D1 | D2, and
-//                w_lo x x_hi with N = NT into D2; 6 cycles per step and activation row, the tensor core's rate.  One
-//                elected lane issues, but the whole warp walks the loop: inside a one-lane branch a step took 628 cycles
-//                instead of 413 (NT = 64; waits and descriptors leave the uniform datapath).
+//                w_lo x x_hi with N = NT into D2; 6 cycles per step and activation row, the tensor core's rate.
+//                What the loop costs besides is the issuing warp's own latency, about 100 cycles per barrier and 20 per
+//                instruction, because the queue in front of the tensor core is short: with two barriers and two commits per
+//                step the bare loop took 671 cycles at NT = 64 and 520 at NT = 16, with one of each per two steps 448 and
+//                246 (NT = 128: 878 and 772, the rate of the instructions).  One elected lane issues, but the whole warp
+//                walks the loop: inside a one-lane branch it took half as long again.
 //   rounding     The tensor core rounds its running sum towards zero, an error that grows with the number of instructions
 //                added up (measured: 5e-9 of the result each).  So the cross terms, 2^-11 of the result, have D2 to
-//                themselves, and every `period` steps D1 is added to registers and restarted.  Relative error of a
-//                1152 x 6912 product: 6.1e-6 with one accumulator for all of K, 4e-7 with this.
-//   read-out     The same warps read D1, each group its share of the columns, as soon as it is complete.
+//                themselves, and every `period` stages D1 is added to registers and restarted.  Relative error of a
+//                1152 x 6912 product: 6.1e-6 with one accumulator for all of K, 5e-7 with this.
 //   K splits     where the tiles alone leave SMs idle, S CTAs of a cluster take a part of K each, leave their sums in their
 //                own shared memory and add each other's columns through distributed shared memory (in split order: results
 //                do not depend on timing).
 // The request for shared memory is at least 120 KB, so that an SM never holds two of these CTAs: one that waits for
 // tensor memory held by a cluster that waits for it would never end.
-constexpr int TC_GROUPS = 4, TC_WARPS = TC_GROUPS * 4 + 2, TC_THREADS = TC_WARPS * 32;
-constexpr int TC_LOADER = TC_GROUPS * 4, TC_ISSUER = TC_LOADER + 1;
 constexpr int TC_SMEM_MIN = 120 * 1024;
-constexpr int TC_PERIOD = 6;                            // most steps (64 values of K) accumulated in D1 before it is read out
+constexpr int TC_PERIOD = 10;                           // most steps (64 values of K) accumulated in D1 before it is read out
 struct TcGemm {
     WeightRef w0, w1;
     float* y; int ldy;
     const uint8_t* img; const float* inv; uint32_t* err;
     int N, units, B, swiglu;                            // units = K / 32
     int n_min, n_main, tiles_n, items;                  // items = tiles_n * tiles of NT rows
-    int S, period;                                      // K splits; steps per accumulation period
+    int S, period;                                      // K splits; stages per accumulation period
     unsigned long long* best; unsigned int* ticket;     // arg-max: one key per activation row (0 between launches), CTAs that are done
     int* out_tok; float *out_val, *out_tok_f32, softcap;
 };
 enum { TC_STORE = 0, TC_PAIR = 1, TC_ARGMAX = 2 };       // what becomes of a product: stored, gate/up pairs, arg-max per activation row (and stored)
 template <int WT, int NT> struct TcGeo {
-    static constexpr int R = WT == WT_Q8_0 && NT == 128 ? 2 : 4;             // weight ring: tiles ahead per warp
+    static constexpr int SP = NT == 128 ? 1 : 2, NS = NT == 128 ? 3 : 2;     // steps per stage, stages
+    static constexpr int GROUPS = NS * SP, THREADS = (2 + GROUPS) * 128;     // weight tiles in flight = warpgroups that rebuild them
+    static constexpr int REG_LOW = 40, REG_READ = NT == 128 ? 200 : 120, REG_MAKE = 80;    // sum = what the CTA is launched with
+    static constexpr int R = WT == WT_Q8_0 && NT == 128 ? 3 : 4;             // weight ring: tiles ahead per warp
     static constexpr int QB = WT == WT_Q8_0 ? 64 : 32;                       // bytes of a row's codes per step
     static constexpr int SLOT = 32 * QB + (WT == WT_Q4_K ? 512 : 128);       // 32 rows: codes, then block scales / superblock headers
-    static constexpr int NB = NT == 128 ? 3 : 4;
-    static constexpr int BSTAGE = NT * 256;
-    static constexpr int RING = NB * BSTAGE, XCH = RING + TC_GROUPS * 4 * R * SLOT;     // offsets: weight rings, gate / up exchange (4 KB per group)
-    static constexpr int SMEM_USED = XCH + TC_GROUPS * 4096 + 1024;
+    static constexpr int BSTEP = NT * 256;                                   // both planes of one step
+    static constexpr int RING = GROUPS * BSTEP, XCH = RING + GROUPS * 4 * R * SLOT;     // offsets: weight rings, gate / up exchange (4 KB)
+    static constexpr int SMEM_USED = XCH + 4096 + 1024;
     static constexpr int SMEM = SMEM_USED > TC_SMEM_MIN ? SMEM_USED : TC_SMEM_MIN;
+    static_assert(SMEM <= 226 * 1024 && 2 * NT + 64 * GROUPS <= 512, "shared or tensor memory");
+    static_assert(REG_LOW + REG_READ + GROUPS * REG_MAKE <= 65536 / THREADS / 8 * 8 * (2 + GROUPS), "registers");
 };
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
     return p != 0;
 }
+template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(N)); }
+template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(N)); }
+template <int N, int HAVE> __device__ __forceinline__ void reg_set() { if constexpr (N > HAVE) reg_inc<N>(); else if constexpr (N < HAVE) reg_dec<N>(); }
 template <int WT, int NT, int MODE>
-__global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
+__global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcGemm a) {
     using G = TcGeo<WT, NT>;
     constexpr bool PAIR = MODE == TC_PAIR;
+    constexpr int SP = G::SP, NS = G::NS;
     extern __shared__ __align__(1024) uint8_t sm_raw[];
     uint8_t* sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);     // the swizzle works on address bits
     uint8_t* smB = sm;
-    __shared__ __align__(8) uint64_t b_full[G::NB], b_empty[G::NB], a_full[TC_GROUPS], a_empty[TC_GROUPS], d_full, d_empty;
+    __shared__ __align__(8) uint64_t full[NS], empty[NS], d_full, d_empty;
     __shared__ uint32_t s_tmem;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // columns that a group reads back, and how many groups read
-    constexpr int COLS = NT / TC_GROUPS < 16 ? 16 : NT / TC_GROUPS, READERS = NT / COLS;
+    [[maybe_unused]] __shared__ bool s_last;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = warp >> 2;
     const int S = a.S, split = S > 1 ? (int)(blockIdx.x % (uint32_t)S) : 0;     // a cluster's CTAs are neighbours along x
     const int first = S > 1 ? (int)(blockIdx.x / (uint32_t)S) : (int)blockIdx.x, stride = (int)gridDim.x / S;
     // this split's share of the steps: first those of the block minima, then those of the products
     const int mn0 = split * a.n_min / S, mn1 = (split + 1) * a.n_min / S;
     const int ma0 = split * a.n_main / S, ma1 = (split + 1) * a.n_main / S;
     const int nmn = mn1 - mn0, nst = nmn + ma1 - ma0, n_steps = a.n_min + a.n_main;
+    const int spi = (nst + SP - 1) / SP;                                        // stages per item; the last may hold one step only
+    const int n_items = first < a.items ? (a.items - first + stride - 1) / stride : 0;
     if (tid == 0) {
-        for (int i = 0; i < G::NB; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
-        for (int i = 0; i < TC_GROUPS; ++i) { mbar_init(&a_full[i], 4); mbar_init(&a_empty[i], 1); }
-        mbar_init(&d_full, 1); mbar_init(&d_empty, 4 * READERS);
+        for (int i = 0; i < NS; ++i) { mbar_init(&full[i], 4 * SP + 1); mbar_init(&empty[i], 1); }
+        mbar_init(&d_full, 1); mbar_init(&d_empty, 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == TC_ISSUER) tc_alloc(&s_tmem, 512);
+    if (warp == 0) tc_alloc(&s_tmem, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
-    constexpr uint32_t A_COL = 256;                     // first column of the weight ring
+    constexpr uint32_t A_COL = 2 * NT;                  // first column of the weight ring
     bool dead = false;
     auto wait_on = [&](uint64_t* bar, uint32_t parity) {
         if (!dead && !mbar_wait(bar, parity)) { dead = true; atomicOr(a.err, DEVERR_WAIT); }
     };
+    const int row = (warp & 3) * 32 + lane;             // this lane's TMEM lane
+    const uint32_t tlane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    auto act = [&](float gate, float up) { return (a.swiglu ? silu_clip(gate) : gelu_tanh(gate)) * up; };
+    // The end of a split item: the cluster's sums lie in the exchange; every CTA finishes the columns c = split, split + S, ...
+    auto finish_split = [&]() {
+        cl_arrive();
+        cl_wait();
+        const uint32_t ex_s = smem_u32(smB);
+        auto total_of = [&](int c, int r) {             // all loads in flight, then one order of addition
+            float p[8], v = 0.f;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) p[q] = q < S ? ld_cluster(ex_s + (uint32_t)(c * 128 + r) * 4u, (uint32_t)q) : 0.f;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v += p[q];
+            return v;
+        };
+        const int tn = first % a.tiles_n, m0 = first / a.tiles_n * NT, n_col = min(NT, a.B - m0);
+        const int n_out = PAIR ? tn * 64 + (row & 63) : tn * 128 + row;
+        float* yp = a.y + (size_t)m0 * a.ldy + n_out;
+        constexpr int LANES = PAIR ? 2 : 1;             // a pair's 64 rows: each half of the lanes takes its own columns
+        for (int c = split + S * ((wg - 1) * LANES + (PAIR ? row >> 6 : 0)); c < n_col; c += (G::GROUPS + 1) * LANES * S) {
+            const float sc = a.inv[m0 + c], v = total_of(c, PAIR ? row & 63 : row);
+            if constexpr (PAIR) { const float u = total_of(c, 64 + (row & 63)); if (n_out < a.N) yp[(size_t)c * a.ldy] = act(v * sc, u * sc); }
+            else if (n_out < a.N) yp[(size_t)c * a.ldy] = v * sc;
+        }
+        cl_arrive();
+        cl_wait();
+    };
     pdl_launch_dependents();
 
-    if (warp == TC_LOADER) {
-        // ---- activation tiles ----
-        pdl_wait();                                     // the image comes from the kernel before this one
+    if (wg == 0) {
+        reg_dec<G::REG_LOW>();
+        pdl_wait();                                     // the image comes from the kernel before this one; no bounded wait below spans that kernel
         const bool lead = elect_one();
-        uint32_t n = 0;
-        for (int item = first; item < a.items; item += stride) {
+        if (warp == 1) {
+            // ---- activation tiles ----
+            uint32_t s = 0, par = 1, n = 0;
             const size_t group_bytes = (size_t)n_steps * (2 * TC_STEP_IMG);
-            const uint8_t* group = a.img + (size_t)(item / a.tiles_n) * (NT == 128 ? 2 : 1) * group_bytes;
-            for (int st = 0; st < nst; ++st, ++n) {
-                const int bs = (int)(n % G::NB);
-                const uint8_t* src = group + (size_t)(st < nmn ? mn0 + st : a.n_min + ma0 + st - nmn) * (2 * TC_STEP_IMG);
-                uint8_t* dst = smB + bs * G::BSTAGE;
-                if (n >= (uint32_t)G::NB) wait_on(&b_empty[bs], (n / G::NB - 1u) & 1u);
-                if (lead) {
-                    mbar_expect_tx(&b_full[bs], (uint32_t)G::BSTAGE);
-                    if constexpr (NT == TC_GROUP) bulk_g2s(dst, src, G::BSTAGE, &b_full[bs]);
-                    else {                              // both planes of the first NT rows, or of two groups
-                        constexpr int ROWS = NT < TC_GROUP ? NT : TC_GROUP;
-                        bulk_g2s(dst, src, ROWS * 128, &b_full[bs]);
-                        bulk_g2s(dst + NT * 128, src + TC_STEP_IMG, ROWS * 128, &b_full[bs]);
-                        if constexpr (NT > TC_GROUP) {
-                            bulk_g2s(dst + TC_STEP_IMG, src + group_bytes, TC_STEP_IMG, &b_full[bs]);
-                            bulk_g2s(dst + NT * 128 + TC_STEP_IMG, src + group_bytes + TC_STEP_IMG, TC_STEP_IMG, &b_full[bs]);
+            for (int item = first; item < a.items; item += stride) {
+                const uint8_t* group = a.img + (size_t)(item / a.tiles_n) * (NT == 128 ? 2 : 1) * group_bytes;
+                for (int j = 0; j < spi; ++j, ++n) {
+                    if (n >= (uint32_t)NS) wait_on(&empty[s], par);
+                    const int st0 = j * SP, n_sub = SP == 1 ? 1 : min(SP, nst - st0);
+                    if (lead) {
+                        mbar_expect_tx(&full[s], (uint32_t)(n_sub * G::BSTEP));
+                        for (int t = 0; t < n_sub; ++t) {
+                            const int st = st0 + t;
+                            const uint8_t* src = group + (size_t)(st < nmn ? mn0 + st : a.n_min + ma0 + st - nmn) * (2 * TC_STEP_IMG);
+                            uint8_t* dst = smB + (s * SP + t) * G::BSTEP;
+                            if constexpr (NT == TC_GROUP) bulk_g2s(dst, src, G::BSTEP, &full[s]);
+                            else {                      // both planes of the first NT rows, or of two groups
+                                constexpr int ROWS = NT < TC_GROUP ? NT : TC_GROUP;
+                                bulk_g2s(dst, src, ROWS * 128, &full[s]);
+                                bulk_g2s(dst + NT * 128, src + TC_STEP_IMG, ROWS * 128, &full[s]);
+                                if constexpr (NT > TC_GROUP) {
+                                    bulk_g2s(dst + TC_STEP_IMG, src + group_bytes, TC_STEP_IMG, &full[s]);
+                                    bulk_g2s(dst + NT * 128 + TC_STEP_IMG, src + group_bytes + TC_STEP_IMG, TC_STEP_IMG, &full[s]);
+                                }
+                            }
                         }
                     }
+                    __syncwarp();
+                    if (++s == (uint32_t)NS) { s = 0; par ^= 1u; }
                 }
-                __syncwarp();
+            }
+            // no copy may be in flight when the CTA ends, whatever became of the waits above
+            for (uint32_t i = n > (uint32_t)NS ? n - NS : 0; i < n; ++i) mbar_wait(&full[i % NS], (i / NS) & 1u);
+        } else if (warp == 0) {
+            // ---- products ----
+            const uint32_t b_lo = (smem_u32(smB) & 0x3FFFFu) >> 4, d1 = tmem, d2 = tmem + NT;
+            auto desc = [&](uint32_t lo) { return ((uint64_t)TC_DESC_HI << 32) | lo; };
+            uint32_t s = 0, par = 0, periods = 0;
+            for (int k = 0; k < n_items; ++k) {
+                int left = 0;                           // stages left in the period
+                for (int j = 0; j < spi; ++j) {
+                    const bool fresh = left == 0;
+                    if (fresh) {                        // D of the period before must have been read
+                        if (periods) wait_on(&d_empty, (periods - 1u) & 1u);
+                        left = min(a.period, spi - j);
+                        ++periods;
+                    }
+                    --left;
+                    wait_on(&full[s], par);
+                    tc_fence_after();
+                    if (lead) {
+#pragma unroll
+                        for (int t = 0; t < SP; ++t) {
+                            if (SP == 2 && t == 1 && 2 * j + 1 >= nst) break;
+                            const uint32_t slot = s * SP + t, ac = tmem + A_COL + slot * 64u, bh = b_lo + slot * (uint32_t)(G::BSTEP / 16);
+                            if (t == 0 && fresh && j > 0) {     // D1 starts again, D2 goes on
+                                tc_mma_ts(d1, ac, desc(bh), TC_IDESC<NT>, 0u);
+                                tc_mma_ts(d2, ac, desc(bh + NT * 8), TC_IDESC<NT>, 1u);
+                            } else tc_mma_ts(d1, ac, desc(bh), TC_IDESC<2 * NT>, (t > 0 || j > 0) ? 1u : 0u);
+                            tc_mma_ts(d2, ac + 32u, desc(bh), TC_IDESC<NT>, 1u);
+#pragma unroll
+                            for (uint32_t q = 1; q < 4; ++q) {
+                                tc_mma_ts(d1, ac + q * 8u, desc(bh + q * 2u), TC_IDESC<2 * NT>, 1u);
+                                tc_mma_ts(d2, ac + 32u + q * 8u, desc(bh + q * 2u), TC_IDESC<NT>, 1u);
+                            }
+                        }
+                        tc_commit(&empty[s]);
+                        if (left == 0) tc_commit(&d_full);
+                    }
+                    __syncwarp();
+                    if (++s == (uint32_t)NS) { s = 0; par ^= 1u; }
+                }
             }
         }
-        // no copy may be in flight when the CTA ends, whatever became of the waits above
-        for (uint32_t i = n > (uint32_t)G::NB ? n - G::NB : 0; i < n; ++i) mbar_wait(&b_full[i % G::NB], (i / G::NB) & 1u);
-    } else if (warp == TC_ISSUER) {
-        // ---- products ----
-        pdl_wait();                                     // so that no bounded wait below spans an earlier kernel
-        const bool lead = elect_one();
-        // the issuer shares its scheduler with four busy warps: few instructions per step
-        const uint32_t b_lo = (smem_u32(smB) & 0x3FFFFu) >> 4, d1 = tmem, d2 = tmem + NT;
-        auto desc = [&](uint32_t lo) { return ((uint64_t)TC_DESC_HI << 32) | lo; };
-        uint32_t bs = 0, b_par = 0, g_at = 0, a_par = 0, periods = 0;       // ring positions and parities
-        for (int item = first; item < a.items; item += stride) {
-            int left = 0;                               // steps left in the period
-            g_at = 0;
-            for (int st = 0; st < nst; ++st) {
-                const bool fresh = left == 0;
-                if (fresh) {                            // D of the period before must have been read
-                    if (periods) wait_on(&d_empty, (periods - 1u) & 1u);
-                    left = min(a.period, nst - st);
-                    ++periods;
-                }
-                --left;
-                wait_on(&b_full[bs], b_par);
-                wait_on(&a_full[g_at], (a_par >> g_at) & 1u);
-                tc_fence_after();
-                const uint32_t ac = tmem + A_COL + g_at * 64u, bh = b_lo + bs * (uint32_t)(G::BSTAGE / 16);
-                if (lead) {
-                    if (fresh && st > 0) {              // D1 starts again, D2 goes on
-                        tc_mma_ts(d1, ac, desc(bh), TC_IDESC<NT>, 0u);
-                        tc_mma_ts(d2, ac, desc(bh + NT * 8), TC_IDESC<NT>, 1u);
-                    } else tc_mma_ts(d1, ac, desc(bh), TC_IDESC<2 * NT>, st > 0 ? 1u : 0u);
-                    tc_mma_ts(d2, ac + 32u, desc(bh), TC_IDESC<NT>, 1u);
+        __syncwarp();
+        if (S > 1) { cl_arrive(); cl_wait(); cl_arrive(); cl_wait(); }
+    } else if (wg == 1) {
+        // ---- results: D1 (and, with an item's last period, D2) into registers; an item's end: scale back, activation, store ----
+        reg_inc<G::REG_READ>();
+        pdl_wait();
+        [[maybe_unused]] float* xch = reinterpret_cast<float*>(sm + G::XCH);
+        const int np = (spi + a.period - 1) / a.period;                                 // periods per item
+        uint32_t par = 0;
+        [[maybe_unused]] unsigned long long best[(NT + 31) / 32] = {};
+        for (int k = 0; k < n_items; ++k) {
+            const int item = first + k * stride, tn = item % a.tiles_n, m0 = item / a.tiles_n * NT;
+            float acc[NT];
 #pragma unroll
-                    for (uint32_t q = 1; q < 4; ++q) {
-                        tc_mma_ts(d1, ac + q * 8u, desc(bh + q * 2u), TC_IDESC<2 * NT>, 1u);
-                        tc_mma_ts(d2, ac + 32u + q * 8u, desc(bh + q * 2u), TC_IDESC<NT>, 1u);
-                    }
-                    tc_commit(&a_empty[g_at]);
-                    tc_commit(&b_empty[bs]);
-                    if (left == 0) tc_commit(&d_full);
+            for (int c = 0; c < NT; ++c) acc[c] = 0.f;
+#pragma unroll 1
+            for (int p = 0; p < np; ++p) {
+                wait_on(&d_full, par);
+                par ^= 1u;
+                tc_fence_after();
+#pragma unroll
+                for (int ch = 0; ch < NT; ch += 16) {
+                    float v[16];
+                    tc_ld16(tlane + ch, v);
+                    tc_ld_wait();
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) acc[ch + c] += v[c];
                 }
-                a_par ^= 1u << g_at;
-                g_at = (g_at + 1u) % TC_GROUPS;
-                if (++bs == (uint32_t)G::NB) { bs = 0; b_par ^= 1u; }
+                if (p == np - 1) {
+#pragma unroll
+                    for (int ch = 0; ch < NT; ch += 16) {
+                        float v[16];
+                        tc_ld16(tlane + NT + ch, v);
+                        tc_ld_wait();
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) acc[ch + c] += v[c];
+                    }
+                }
+                tc_fence_before();
                 __syncwarp();
+                if (lane == 0) mbar_arrive(&d_empty);
+            }
+            if (S > 1) {                                // one item per cluster, and the activation ring is drained: it becomes the exchange
+                float* ex = reinterpret_cast<float*>(smB);
+#pragma unroll
+                for (int c = 0; c < NT; ++c) ex[c * 128 + row] = acc[c];
+                break;
+            }
+            const int n_out = PAIR ? tn * 64 + (row & 63) : tn * 128 + row, n_col = min(NT, a.B - m0);
+            float* yp = a.y + (size_t)m0 * a.ldy + n_out;
+            float inv[(NT + 31) / 32];                  // lane l of part i: column 32 i + l
+#pragma unroll
+            for (int i = 0; i < (NT + 31) / 32; ++i) inv[i] = 32 * i + lane < n_col ? a.inv[m0 + 32 * i + lane] : 0.f;
+            if constexpr (PAIR) {
+                // gate lanes (quarters 0, 1) and up lanes (2, 3) of a row swap half of their columns, eight at a time, through
+                // shared memory; gate lanes finish the first half of the columns
+                constexpr int H = NT / 2;
+                const bool up = row >= 64;
+#pragma unroll
+                for (int h0 = 0; h0 < H; h0 += 8) {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) xch[c * 128 + row] = up ? acc[h0 + c] : acc[H + h0 + c];
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const int cg = h0 + c, cu = H + h0 + c, col = up ? cu : cg;
+                        const float sg = __shfl_sync(0xffffffffu, inv[cg / 32], cg & 31), su = __shfl_sync(0xffffffffu, inv[cu / 32], cu & 31), sc = up ? su : sg;
+                        const float o = xch[c * 128 + (row ^ 64)], m = up ? acc[cu] : acc[cg];
+                        if (col < n_col && n_out < a.N) yp[(size_t)col * a.ldy] = up ? act(o * sc, m * sc) : act(m * sc, o * sc);
+                    }
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < NT; ++c) {
+                    const float v = acc[c] * __shfl_sync(0xffffffffu, inv[c / 32], c & 31);
+                    if constexpr (MODE == TC_ARGMAX) {
+                        // best of the warp's rows: NaN counts as -FLT_MAX, ties go to the lower row; lane c % 32 keeps column c's
+                        const float f = (v == v ? v : -3.402823466e+38f) + 0.f;
+                        const uint32_t bits = __float_as_uint(f), ord = n_out < a.N ? bits ^ ((uint32_t)((int)bits >> 31) | 0x80000000u) : 0u;
+                        const uint32_t top = __reduce_max_sync(0xffffffffu, ord);
+                        const uint32_t at = __reduce_min_sync(0xffffffffu, ord == top ? (uint32_t)n_out : 0xffffffffu);
+                        const unsigned long long key = ((unsigned long long)top << 32) | (0xffffffffu - at);
+                        if (lane == (c & 31) && key > best[c / 32]) best[c / 32] = key;
+                        if (a.y && c < n_col && n_out < a.N) yp[(size_t)c * a.ldy] = a.softcap > 0.f ? tanhf(v / a.softcap) * a.softcap : v;
+                    } else if (c < n_col && n_out < a.N) yp[(size_t)c * a.ldy] = v;
+                }
+                if constexpr (MODE == TC_ARGMAX)
+                    if (a.B > NT || k == n_items - 1) {         // the columns change with the next item, or there is none
+#pragma unroll
+                        for (int i = 0; i < (NT + 31) / 32; ++i) {
+                            if (32 * i + lane < n_col) atomicMax(a.best + m0 + 32 * i + lane, best[i]);
+                            best[i] = 0;
+                        }
+                    }
+            }
+        }
+        if (S > 1) finish_split();
+        if constexpr (MODE == TC_ARGMAX) {              // the last CTA to end decodes the winners and clears the keys
+            __threadfence();
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (tid == 128) s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (s_last) {
+                __threadfence();
+                for (int b = tid - 128; b < a.B; b += 128) {
+                    const unsigned long long key = __ldcg(a.best + b);
+                    const uint32_t ord = (uint32_t)(key >> 32);
+                    const int tok = (int)(0xffffffffu - (uint32_t)key);
+                    if (a.out_tok) a.out_tok[b] = tok;
+                    if (a.out_tok_f32) a.out_tok_f32[b] = (float)tok;
+                    if (a.out_val) a.out_val[b] = __uint_as_float(ord & 0x80000000u ? ord ^ 0x80000000u : ~ord);
+                    a.best[b] = 0;
+                }
+                if (tid == 128) *a.ticket = 0u;
             }
         }
     } else {
-        // ---- weights, and the end of a tile ----
-        const int grp = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane;       // row = this lane's TMEM lane
-        const uint32_t tlane = tmem + ((uint32_t)(quarter * 32) << 16);
-        uint8_t* ring = sm + G::RING + warp * G::R * G::SLOT;
-        [[maybe_unused]] float* xch = reinterpret_cast<float*>(sm + G::XCH) + grp * 1024;
+        // ---- weights ----
+        reg_set<G::REG_MAKE, 65536 / G::THREADS / 8 * 8>();
+        const int grp = wg - 2, quarter = warp & 3;
+        const uint32_t stage = (uint32_t)(grp / SP);    // this group fills step grp % SP of every NS-th stage, counted over all items
+        uint8_t* ring = sm + G::RING + (warp - 8) * G::R * G::SLOT;
         const uint32_t ring_s = smem_u32(ring);
         const WeightRef w = (PAIR && quarter >= 2) ? a.w1 : a.w0;                      // lanes 64..127 of a pair: up rows
         const bool scales_async = WT == WT_Q4_K || ((a.units & 1) == 0 && ((uintptr_t)w.d & 3) == 0);
-        // This group takes steps grp, grp + 4, ... of every item and always uses ring slot grp: a slot that changed hands
-        // could be waited for by a group that has not followed its phases, and a wait on a phase two ahead returns at once.
-        const int n_own = (nst - grp + TC_GROUPS - 1) / TC_GROUPS;
-        auto step_of = [&](int j) { return grp + TC_GROUPS * j; };
         auto row_of = [&](int tn, int r) { return min(PAIR ? tn * 64 + (r & 63) : tn * 128 + r, a.N - 1); };
         const int rpu = WT == WT_Q4_0 ? a.units : WT == WT_Q8_0 ? 2 * a.units : (a.units >> 3) * 9;     // uint4 per weight row
-        const int n_items = first < a.items ? (a.items - first + stride - 1) / stride : 0;
+        struct Cursor { int k, j; };                    // item, stage of the item
+        auto settle = [&](Cursor& c) { while (c.j >= spi && c.k < n_items) { c.j -= spi; ++c.k; } };
 
         // fetch cursor, R tiles ahead of the production cursor
-        int f_item = 0, f_j = 0; uint32_t f_n = 0;
+        Cursor f = {0, (int)stage};
+        settle(f);
+        int f_k = -1; uint32_t f_n = 0;                 // item that the row pointers belong to; ring slot
         constexpr int LPR = G::QB / 16, FI = LPR;       // lanes per row and copies per lane of a step's codes
         const uint4 *f_q[FI], *f_h = nullptr; const __half* f_d = nullptr;
         auto fetch = [&]() {
-            if (f_item < n_items && n_own > 0) {
-                if (f_j == 0) {
-                    const int tn = (first + f_item * stride) % a.tiles_n;
+            if (f.k < n_items) {
+                if (f_k != f.k) {
+                    f_k = f.k;
+                    const int tn = (first + f.k * stride) % a.tiles_n;
 #pragma unroll
                     for (int h = 0; h < FI; ++h) f_q[h] = w.q + (size_t)row_of(tn, quarter * 32 + (32 / FI) * h + lane / LPR) * rpu;
                     if constexpr (WT != WT_Q4_K) f_d = w.d + (size_t)row_of(tn, row) * a.units;
                     else f_h = w.q + (size_t)row_of(tn, row) * rpu;
                 }
-                const int st = step_of(f_j), ks = ma0 + st - nmn;
-                if (st >= nmn) {
-                    const uint32_t dst = ring_s + (f_n % G::R) * G::SLOT;
+                const int st = f.j * SP + grp % SP, ks = ma0 + st - nmn;
+                if (st >= nmn && st < nst) {
+                    const uint32_t dst = ring_s + f_n * G::SLOT;
                     const int piece = lane % LPR;
                     const int off = WT == WT_Q4_K ? (ks >> 2) * 9 + 1 + (ks & 3) * 2 + piece : min(LPR * ks + piece, rpu - 1);
 #pragma unroll
@@ -502,160 +658,41 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                     if constexpr (WT != WT_Q4_K) { if (scales_async) cp_async4(dst + 32 * G::QB + lane * 4, f_d + 2 * ks); }
                     else cp_async16_l1(dst + 32 * G::QB + lane * 16, f_h + (ks >> 2) * 9);
                 }
-                if (++f_j == n_own) { f_j = 0; ++f_item; }
+                f.j += NS;
+                settle(f);
             }
-            ++f_n;
+            if (++f_n == (uint32_t)G::R) f_n = 0;
             cp_commit();
         };
-
-        // D1 (and, with the item's last period, D2) into acc; the end of an item: scale back, activation, store
-        const bool reads = grp < READERS;
-        const int c0 = grp * COLS;
-        const int np = (nst + a.period - 1) / a.period;                                 // periods per item
-        bool waited = false;
-        int done = 0, done_item = 0, done_p = 0;        // periods read out: in all, as (item, period of the item)
-        float acc[COLS];
-        [[maybe_unused]] unsigned long long best = 0;
-#pragma unroll
-        for (int c = 0; c < COLS; ++c) acc[c] = 0.f;
-        auto read_out = [&]() {
-            if (!waited) { pdl_wait(); waited = true; }
-            const bool last = done_p == np - 1;
-            wait_on(&d_full, (uint32_t)done & 1u);
-            tc_fence_after();
-            {
-                const uint32_t col = tlane + (uint32_t)c0;
-#pragma unroll
-                for (int ch = 0; ch < COLS / 16; ++ch) {
-                    float v[16];
-                    tc_ld16(col + ch * 16, v);
-                    tc_ld_wait();
-#pragma unroll
-                    for (int c = 0; c < 16; ++c) acc[ch * 16 + c] += v[c];
-                }
-                if (last) {
-#pragma unroll
-                    for (int ch = 0; ch < COLS / 16; ++ch) {
-                        float v[16];
-                        tc_ld16(col + NT + ch * 16, v);
-                        tc_ld_wait();
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) acc[ch * 16 + c] += v[c];
-                    }
-                }
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&d_empty);
-            ++done; ++done_p;
-            if (!last) return;
-            const int item = first + done_item * stride, tn = item % a.tiles_n, m0 = item / a.tiles_n * NT;
-            done_p = 0; ++done_item;
-            const int n_out = PAIR ? tn * 64 + (row & 63) : tn * 128 + row, n_col = min(NT, a.B - m0);
-            float* yp = a.y + (size_t)m0 * a.ldy + n_out;
-            const float inv_mine = m0 + c0 + lane < a.B ? a.inv[m0 + c0 + lane] : 0.f;         // of this group's columns (COLS <= 32)
-            auto act = [&](float gate, float up) { return (a.swiglu ? silu_clip(gate) : gelu_tanh(gate)) * up; };
-            if (S > 1) {
-                // one item per cluster: sums into the exchange (the activation ring is drained), then every CTA finishes the
-                // columns c = split, split + S, ... from all S parts
-                float* ex = reinterpret_cast<float*>(smB);
-#pragma unroll
-                for (int c = 0; c < COLS; ++c) ex[(c0 + c) * 128 + row] = acc[c];
-                cl_arrive();
-                cl_wait();
-                const uint32_t ex_s = smem_u32(ex);
-                auto total_of = [&](int c, int r) {             // all loads in flight, then one order of addition
-                    float p[8], v = 0.f;
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) p[q] = q < S ? ld_cluster(ex_s + (uint32_t)(c * 128 + r) * 4u, (uint32_t)q) : 0.f;
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) v += p[q];
-                    return v;
-                };
-                // a pair's 64 rows: each half of the lanes takes its own columns
-                const int lanes = PAIR ? 2 : 1, sub = PAIR ? row >> 6 : 0;
-                for (int c = split + S * (grp * lanes + sub); c < n_col; c += READERS * lanes * S) {
-                    const float sc = a.inv[m0 + c], v = total_of(c, PAIR ? row & 63 : row);
-                    if constexpr (PAIR) { const float u = total_of(c, 64 + (row & 63)); if (n_out < a.N) yp[(size_t)c * a.ldy] = act(v * sc, u * sc); }
-                    else if (n_out < a.N) yp[(size_t)c * a.ldy] = v * sc;
-                }
-                cl_arrive();
-                cl_wait();
-            } else if constexpr (PAIR) {
-                // gate lanes (quarters 0, 1) and up lanes (2, 3) of a row swap half of this group's columns, eight at a time,
-                // through shared memory
-                constexpr int H = COLS / 2, CH = H < 8 ? H : 8;
-                const bool up = row >= 64;
-#pragma unroll
-                for (int h0 = 0; h0 < H; h0 += CH) {
-#pragma unroll
-                    for (int c = 0; c < CH; ++c) xch[c * 128 + row] = up ? acc[h0 + c] : acc[H + h0 + c];
-                    asm volatile("bar.sync %0, 128;" :: "r"(1 + grp) : "memory");
-#pragma unroll
-                    for (int c = 0; c < CH; ++c) {
-                        const int lc = (up ? H : 0) + h0 + c;   // gate lanes finish the first half of the columns
-                        const float o = xch[c * 128 + (row ^ 64)], sc = __shfl_sync(0xffffffffu, inv_mine, lc), m = up ? acc[H + h0 + c] : acc[h0 + c];
-                        if (c0 + lc < n_col && n_out < a.N) yp[(size_t)(c0 + lc) * a.ldy] = up ? act(o * sc, m * sc) : act(m * sc, o * sc);
-                    }
-                    asm volatile("bar.sync %0, 128;" :: "r"(1 + grp) : "memory");
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < COLS; ++c) {
-                    const float v = acc[c] * __shfl_sync(0xffffffffu, inv_mine, c);
-                    if constexpr (MODE == TC_ARGMAX) {
-                        // best of the warp's rows: NaN counts as -FLT_MAX, ties go to the lower row; lane c keeps column c's
-                        const float f = (v == v ? v : -3.402823466e+38f) + 0.f;
-                        const uint32_t bits = __float_as_uint(f), ord = n_out < a.N ? bits ^ ((uint32_t)((int)bits >> 31) | 0x80000000u) : 0u;
-                        const uint32_t top = __reduce_max_sync(0xffffffffu, ord);
-                        const uint32_t at = __reduce_min_sync(0xffffffffu, ord == top ? (uint32_t)n_out : 0xffffffffu);
-                        const unsigned long long key = ((unsigned long long)top << 32) | (0xffffffffu - at);
-                        if (lane == c && key > best) best = key;
-                        if (a.y && c0 + c < n_col && n_out < a.N) yp[(size_t)(c0 + c) * a.ldy] = a.softcap > 0.f ? tanhf(v / a.softcap) * a.softcap : v;
-                    } else if (c0 + c < n_col && n_out < a.N) yp[(size_t)(c0 + c) * a.ldy] = v;
-                }
-                if constexpr (MODE == TC_ARGMAX)
-                    if (a.B > NT || done_item == n_items) {     // the columns change with the next item, or there is none
-                        if (lane < COLS && c0 + lane < n_col) atomicMax(a.best + m0 + c0 + lane, best);
-                        best = 0;
-                    }
-            }
-#pragma unroll
-            for (int c = 0; c < COLS; ++c) acc[c] = 0.f;
-        };
-        // ---- production ----
         for (int j = 0; j < G::R; ++j) fetch();
-        uint32_t n = 0;                                 // tiles of this group
-        for (int k = 0; k < n_items; ++k) {
-            const int tn = (first + k * stride) % a.tiles_n;
-            for (int j = 0; j < n_own; ++j, ++n) {
-                const int st = step_of(j), ks = ma0 + st - nmn;
-                const uint32_t acol = tlane + A_COL + grp * 64u;
-                cp_wait<G::R - 1>();
-                __syncwarp();
-                const uint8_t* slot = ring + (n % G::R) * G::SLOT;
-                uint32_t qw[G::QB / 4];                 // this row's codes of the step
+        const uint32_t acol = tlane + A_COL + (uint32_t)grp * 64u;
+        uint32_t at = 0, par = 1;                       // ring slot; parity of the next wait for an empty stage
+        bool again = false;                             // this group has filled its slot before
+        Cursor c = {0, (int)stage};
+        settle(c);
+        while (c.k < n_items) {
+            const int tn = (first + c.k * stride) % a.tiles_n;
+            const int st = c.j * SP + grp % SP, ks = ma0 + st - nmn;
+            cp_wait<G::R - 1>();
+            __syncwarp();
+            const uint8_t* slot = ring + at * G::SLOT;
+            uint32_t qw[G::QB / 4];                     // this row's codes of the step
 #pragma unroll
-                for (int p = 0; p < LPR; ++p) {
-                    const uint4 v = *reinterpret_cast<const uint4*>(slot + lane * G::QB + ((LPR == 2 ? p ^ ((lane >> 2) & 1) : p ^ ((lane >> 1) & 3)) << 4));
-                    qw[4 * p] = v.x; qw[4 * p + 1] = v.y; qw[4 * p + 2] = v.z; qw[4 * p + 3] = v.w;
-                }
-                uint32_t d01 = 0; uint4 hdr = make_uint4(0, 0, 0, 0);
-                if constexpr (WT != WT_Q4_K) d01 = *reinterpret_cast<const uint32_t*>(slot + 32 * G::QB + lane * 4);
-                else hdr = *reinterpret_cast<const uint4*>(slot + 32 * G::QB + lane * 16);
-                __syncwarp();
-                fetch();
-                if (reads) {
-                    // Where this group's tile before was the last of a period, D is read first: the tensor core waits for that,
-                    // while the tile that comes now is four steps away (producing first: 3300 idle cycles per period).
-                    const int ended = st >= TC_GROUPS ? k * np + (st - TC_GROUPS + 1) / a.period : (nst - 1 - grp) % TC_GROUPS == 0 ? k * np : 0;
-                    while (done < ended) read_out();
-                }
-                if (n) {                                // the tensor core is done with this group's tile before
-                    if (!waited) { pdl_wait(); waited = true; }
-                    wait_on(&a_empty[grp], (n - 1u) & 1u);
-                    tc_fence_after();
-                }
+            for (int p = 0; p < LPR; ++p) {
+                const uint4 v = *reinterpret_cast<const uint4*>(slot + lane * G::QB + ((LPR == 2 ? p ^ ((lane >> 2) & 1) : p ^ ((lane >> 1) & 3)) << 4));
+                qw[4 * p] = v.x; qw[4 * p + 1] = v.y; qw[4 * p + 2] = v.z; qw[4 * p + 3] = v.w;
+            }
+            uint32_t d01 = 0; uint4 hdr = make_uint4(0, 0, 0, 0);
+            if constexpr (WT != WT_Q4_K) d01 = *reinterpret_cast<const uint32_t*>(slot + 32 * G::QB + lane * 4);
+            else hdr = *reinterpret_cast<const uint4*>(slot + 32 * G::QB + lane * 16);
+            __syncwarp();
+            fetch();
+            if (again) {                                // the tensor core is done with this group's tile before
+                wait_on(&empty[stage], par);
+                tc_fence_after();
+            } else { pdl_wait(); again = true; }        // (nothing was awaited before; from here on bounded waits span no earlier kernel)
+            par ^= 1u;
+            if (st < nst) {
                 if constexpr (WT != WT_Q4_K) {
                     if (!scales_async) {                // odd number of blocks per row: their scales are not pairs of aligned halves
                         const unsigned short* dp = reinterpret_cast<const unsigned short*>(w.d) + (size_t)row_of(tn, row) * a.units + 2 * ks;
@@ -750,35 +787,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_tc(const TcGemm a) {
                 }
                 tc_st_wait();
                 tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&a_full[grp]);
-                if (reads) while (done < k * np + st / a.period) read_out();    // what ended before this tile's period
             }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[stage]);
+            if (++at == (uint32_t)G::R) at = 0;
+            c.j += NS;
+            settle(c);
         }
-        if (reads) while (done < n_items * np) read_out();
         cp_wait<0>();
+        if (S > 1) finish_split();
     }
-    if (S > 1 && (warp >= TC_LOADER || (warp >> 2) >= READERS)) { cl_arrive(); cl_wait(); cl_arrive(); cl_wait(); }
-    if constexpr (MODE == TC_ARGMAX) __threadfence();
     __syncthreads();
     tc_fence_after();
-    if (warp == TC_ISSUER) tc_dealloc(tmem, 512);
-    if constexpr (MODE == TC_ARGMAX) {                  // the last CTA to end decodes the winners and clears the keys
-        if (tid == 0) s_tmem = atomicAdd(a.ticket, 1u);
-        __syncthreads();
-        if (s_tmem != gridDim.x - 1) return;
-        __threadfence();
-        for (int b = tid; b < a.B; b += TC_THREADS) {
-            const unsigned long long key = __ldcg(a.best + b);
-            const uint32_t ord = (uint32_t)(key >> 32);
-            const int tok = (int)(0xffffffffu - (uint32_t)key);
-            if (a.out_tok) a.out_tok[b] = tok;
-            if (a.out_tok_f32) a.out_tok_f32[b] = (float)tok;
-            if (a.out_val) a.out_val[b] = __uint_as_float(ord & 0x80000000u ? ord ^ 0x80000000u : ~ord);
-            a.best[b] = 0;
-        }
-        if (tid == 0) *a.ticket = 0u;
-    }
+    if (warp == 0) tc_dealloc(tmem, 512);
 }
 
 // ---- host ----------------------------------------------------------------------------------------------------------
@@ -803,9 +824,9 @@ bool gemm_tc_supports(int wtype, const GemvArgs& a) {
 }
 
 typedef void (*TcKernel)(const TcGemm);
-struct TcPick { TcKernel k; int smem; bool attr; };
+struct TcPick { TcKernel k; int smem, threads; bool attr; };
 template <int WT, int NT, int MODE> static TcPick& tc_pick() {
-    static TcPick p = {k_gemm_tc<WT, NT, MODE>, TcGeo<WT, NT>::SMEM, false};
+    static TcPick p = {k_gemm_tc<WT, NT, MODE>, TcGeo<WT, NT>::SMEM, TcGeo<WT, NT>::THREADS, false};
     return p;
 }
 template <int WT, int MODE> static TcPick& tc_pick(int nt) {
@@ -852,8 +873,8 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
     t.w0 = a.w0; t.w1 = a.w1; t.y = a.y; t.ldy = a.ldy; t.img = g_tc.img; t.inv = g_tc.inv; t.err = g.dev_err;
     t.N = a.N; t.units = a.K / 32; t.B = a.B; t.swiglu = a.epi == EPI_SWIGLU;
     t.n_min = n_min; t.n_main = n_main; t.S = S;
-    const int longest = (n_main + S - 1) / S + (n_min + S - 1) / S, n_periods = (longest + TC_PERIOD - 1) / TC_PERIOD;
-    t.period = (longest + n_periods - 1) / n_periods;
+    const int sp = nt == 128 ? 1 : 2, stages = ((n_main + S - 1) / S + (n_min + S - 1) / S + sp - 1) / sp, n_periods = (stages * sp + TC_PERIOD - 1) / TC_PERIOD;
+    t.period = (stages + n_periods - 1) / n_periods;
     t.tiles_n = tiles_n;
     t.items = (int)items;
     const int mode = pair ? TC_PAIR : a.epi == EPI_ARGMAX ? TC_ARGMAX : TC_STORE;
@@ -868,8 +889,8 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
         p.attr = true;
     }
     cudaError_t e;
-    if (S == 1) e = launch_k(p.k, dim3((unsigned)(t.items < g.sm_count ? t.items : g.sm_count)), dim3(TC_THREADS), (size_t)p.smem, stream, g.pdl, t);
-    else e = launch_k_cluster(p.k, dim3((unsigned)(t.items * S)), dim3(TC_THREADS), (size_t)p.smem, stream, g.pdl, (unsigned)S, t);
+    if (S == 1) e = launch_k(p.k, dim3((unsigned)(t.items < g.sm_count ? t.items : g.sm_count)), dim3(p.threads), (size_t)p.smem, stream, g.pdl, t);
+    else e = launch_k_cluster(p.k, dim3((unsigned)(t.items * S)), dim3(p.threads), (size_t)p.smem, stream, g.pdl, (unsigned)S, t);
     if (e != cudaSuccess) return fail(ADAMAH_ERR_BACKEND, "gemm_tc: launch failed: %s", cudaGetErrorString(e));
     count_launch();
     return ADAMAH_OK;
