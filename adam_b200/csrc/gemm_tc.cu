@@ -320,7 +320,7 @@ __device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, u
 // The request for shared memory is at least 120 KB, so that an SM never holds two of these CTAs: one that waits for
 // tensor memory held by a cluster that waits for it would never end.
 constexpr int TC_SMEM_MIN = 120 * 1024;
-constexpr int TC_PERIOD = 10;                           // most steps (64 values of K) accumulated in D1 before it is read out
+constexpr int TC_PERIOD = 8;                            // most steps (64 values of K) accumulated in D1 before it is read out
 struct TcGemm {
     WeightRef w0, w1;
     float* y; int ldy;
@@ -845,7 +845,7 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
         int mv = 16;
         for (int c : cand) if ((n4 + c - 1) / c <= 512) { mv = c; break; }
         const int threads = ((n4 + mv - 1) / mv + 31) / 32 * 32;
-        auto go = [&](auto kern) { launch_k(kern, dim3(a.B), dim3(threads), 0, stream, g.pdl, a, g_tc.img, g_tc.inv, n_min, n_min + n_main); };
+        auto go = [&](auto kern) { launch_k(kern, dim3(a.B), dim3(threads), 0, stream, true, a, g_tc.img, g_tc.inv, n_min, n_min + n_main); };
         const bool chain = a.h_in != nullptr;
         switch (mv) {
         case 1: if (chain) go(k_quant_rows<1, true>); else go(k_quant_rows<1, false>); break;
@@ -889,8 +889,8 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
         p.attr = true;
     }
     cudaError_t e;
-    if (S == 1) e = launch_k(p.k, dim3((unsigned)(t.items < g.sm_count ? t.items : g.sm_count)), dim3(p.threads), (size_t)p.smem, stream, g.pdl, t);
-    else e = launch_k_cluster(p.k, dim3((unsigned)(t.items * S)), dim3(p.threads), (size_t)p.smem, stream, g.pdl, (unsigned)S, t);
+    if (S == 1) e = launch_k(p.k, dim3((unsigned)(t.items < g.sm_count ? t.items : g.sm_count)), dim3(p.threads), (size_t)p.smem, stream, true, t);
+    else e = launch_k_cluster(p.k, dim3((unsigned)(t.items * S)), dim3(p.threads), (size_t)p.smem, stream, true, (unsigned)S, t);
     if (e != cudaSuccess) return fail(ADAMAH_ERR_BACKEND, "gemm_tc: launch failed: %s", cudaGetErrorString(e));
     count_launch();
     return ADAMAH_OK;
