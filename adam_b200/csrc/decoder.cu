@@ -829,7 +829,7 @@ static int gemv(const Mat& m, const Mat* m2, GemvArgs a, int B, int epi) {
 #endif
     a.w0 = m.w; if (m2) a.w1 = m2->w;
     a.N = (int)m.rows; a.K = (int)m.cols; a.B = B; a.epi = epi;
-    if (B >= TC_MIN_ROWS && (!m2 || m2->wtype == m.wtype) && gemm_tc_supports(m.wtype, a)) return launch_gemm_tc(m.wtype, a, g.stream);
+    if (B >= TC_MIN_ROWS && (!m2 || m2->wtype == m.wtype) && gemm_tc_supports(m.wtype, a, m.tiled && (!m2 || m2->tiled))) return launch_gemm_tc(m.wtype, a, g.stream);
     if (m.tiled && (!m2 || (m2->tiled && m2->wtype == m.wtype)) && gemv_mma_supports(m.wtype, a))
         return launch_gemv_mma(m.wtype, m.tiled, m2 ? m2->tiled : nullptr, a, g.stream);
     return launch_gemv(m.wtype, a, g.stream);
@@ -915,7 +915,7 @@ static int enqueue_part(Decoder* D, uint32_t batch, uint32_t part, bool with_lm,
             a.y = want_logits ? D->logits : nullptr; a.ldy = (int)lm.rows; a.softcap = d.final_softcap;
             a.out_tok = D->cur_tok; a.out_val = D->cur_val;
             a.w0 = lm.w; a.N = (int)lm.rows; a.K = (int)lm.cols; a.B = (int)batch; a.epi = EPI_ARGMAX;
-            if (gemm_tc_supports(lm.wtype, a)) {
+            if (gemm_tc_supports(lm.wtype, a, lm.tiled != nullptr)) {
                 if ((rc = launch_gemm_tc(lm.wtype, a, g.stream))) return rc;
                 D->h_final = 0;
                 return check_launch("decoder step");

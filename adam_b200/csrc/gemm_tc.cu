@@ -34,7 +34,7 @@ constexpr int TC_STEP_IMG = TC_GROUP * 128;             // one plane of one grou
 constexpr size_t TC_IMG_MAX = 256u << 20;               // largest image kept; longer calls run in row chunks
 constexpr int TC_MAX_K = 32768;
 
-struct TcWork { uint8_t* img; size_t img_cap; float* inv; int inv_cap; unsigned long long* best; std::vector<void*> retired; };   // best: arg-max keys [inv_cap], then a ticket
+struct TcWork { uint8_t* img; size_t img_cap; float* inv; int inv_cap; unsigned long long* best; float* part; unsigned int* tickets; std::vector<void*> retired; };   // best: arg-max keys [inv_cap], then a ticket
 static TcWork g_tc = {};
 static uint64_t g_tc_calls = 0;
 static int g_tc_policy = -1;             // 0 never, 1 where it is expected to be faster, 2 whenever the shape allows; -1 = take it from ADAM_B200_TC
@@ -59,6 +59,9 @@ bool gemm_tc_prepare(int rows, int K) {
         *p = q;
         return true;
     };
+    if (!g_tc.part) {                                   // two tiles of 128 x 128 sums and a ticket per CTA
+        if (!grow((void**)&g_tc.tickets, (size_t)g.sm_count * 4) || !grow((void**)&g_tc.part, (size_t)g.sm_count * 2 * 128 * 128 * 4)) return false;
+    }
     if (need > g_tc.img_cap) {
         size_t cap = need > 2 * g_tc.img_cap ? need : 2 * g_tc.img_cap;
         if (cap > TC_IMG_MAX) cap = TC_IMG_MAX;
@@ -75,7 +78,7 @@ bool gemm_tc_prepare(int rows, int K) {
 }
 
 void gemm_tc_release() {
-    cudaFree(g_tc.img); cudaFree(g_tc.inv); cudaFree(g_tc.best);
+    cudaFree(g_tc.img); cudaFree(g_tc.inv); cudaFree(g_tc.best); cudaFree(g_tc.part); cudaFree(g_tc.tickets);
     for (void* p : g_tc.retired) cudaFree(p);
     g_tc = TcWork{};
 }
@@ -296,8 +299,8 @@ __device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, u
 // barrier for everything that fills it (its activation tiles, and the warps that rebuild its weight tiles) and one that
 // the tensor core's commit releases.
 //   warp roles   Warpgroup 0: warp 0 issues the tensor-core instructions, warp 1 fetches activation tiles.  Warpgroup 1 reads
-//                results back.  The others rebuild weights, one warpgroup for each weight tile in flight.  setmaxnreg moves
-//                registers from warpgroup 0 to the reader, which holds NT sums per thread.
+//                results back.  The others rebuild weights, a weight tile each in turn.  setmaxnreg moves registers from
+//                warpgroup 0 to the reader, which holds NT sums per thread.
 //   weights      A lane owns a row.  Its codes come by cp.async into the warp's own ring in shared memory (R tiles ahead,
 //                across the end of a tile, two lanes per row so that a sector is fetched whole), are taken apart in fp16
 //                pairs (4.25 instructions per two weights) and go to TMEM with tcgen05.st: no shared-memory operand image,
@@ -314,9 +317,12 @@ __device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, u
 //                added up (measured: 5e-9 of the result each).  So the cross terms, 2^-11 of the result, have D2 to
 //                themselves, and every `period` stages D1 is added to registers and restarted.  Relative error of a
 //                1152 x 6912 product: 6.1e-6 with one accumulator for all of K, 5e-7 with this.
-//   K splits     where the tiles alone leave SMs idle, S CTAs of a cluster take a part of K each, leave their sums in their
-//                own shared memory and add each other's columns through distributed shared memory (in split order: results
-//                do not depend on timing).
+//   work split   Three ways, by an estimate of their times (launch_rows).  Whole tiles, dealt in turn.  Or all stages
+//                of all tiles in a row, dealt out evenly: a tile that several CTAs share is added up by the one that ends
+//                last (atomic ticket, partial sums in a workspace), in the order of K; 168 tiles on 148 SMs take 1.14 tiles'
+//                time, not 2, but the adding up costs 2 to 5 us.  Or, where the tiles alone leave SMs idle, clusters of S
+//                CTAs that take a part of K each, leave their sums in their own shared memory and add each other's columns
+//                through distributed shared memory, again in the order of K: results do not depend on timing.
 // The request for shared memory is at least 120 KB, so that an SM never holds two of these CTAs: one that waits for
 // tensor memory held by a cluster that waits for it would never end.
 constexpr int TC_SMEM_MIN = 120 * 1024;
@@ -326,24 +332,25 @@ struct TcGemm {
     float* y; int ldy;
     const uint8_t* img; const float* inv; uint32_t* err;
     int N, units, B, swiglu;                            // units = K / 32
-    int n_min, n_main, tiles_n, items;                  // items = tiles_n * tiles of NT rows
-    int S, period;                                      // K splits; stages per accumulation period
+    int n_min, n_main, tiles_n, items;                  // items = tiles_n (weight tiles) * tiles of NT rows
+    int S, period, shared;                              // K splits; stages per accumulation period; whether CTAs share tiles
+    float* part; unsigned int* tickets;                 // shared tiles: per CTA the sums of its first and last one; arrivals, by the CTA in which a tile begins
     unsigned long long* best; unsigned int* ticket;     // arg-max: one key per activation row (0 between launches), CTAs that are done
     int* out_tok; float *out_val, *out_tok_f32, softcap;
 };
 enum { TC_STORE = 0, TC_PAIR = 1, TC_ARGMAX = 2 };       // what becomes of a product: stored, gate/up pairs, arg-max per activation row (and stored)
 template <int WT, int NT> struct TcGeo {
-    static constexpr int SP = NT == 128 ? 1 : 2, NS = NT == 128 ? 3 : 2;     // steps per stage, stages
-    static constexpr int GROUPS = NS * SP, THREADS = (2 + GROUPS) * 128;     // weight tiles in flight = warpgroups that rebuild them
+    static constexpr int SP = NT == 128 ? 1 : 2, NS = NT == 128 ? 4 : 2;     // steps per stage, stages
+    static constexpr int GROUPS = NT == 128 ? 3 : 4, THREADS = (2 + GROUPS) * 128;     // warpgroups that rebuild weights, a step each in turn
     static constexpr int REG_LOW = 40, REG_READ = NT == 128 ? 200 : 120, REG_MAKE = 80;    // sum = what the CTA is launched with
     static constexpr int R = WT == WT_Q8_0 && NT == 128 ? 3 : 4;             // weight ring: tiles ahead per warp
     static constexpr int QB = WT == WT_Q8_0 ? 64 : 32;                       // bytes of a row's codes per step
     static constexpr int SLOT = 32 * QB + (WT == WT_Q4_K ? 512 : 128);       // 32 rows: codes, then block scales / superblock headers
     static constexpr int BSTEP = NT * 256;                                   // both planes of one step
-    static constexpr int RING = GROUPS * BSTEP, XCH = RING + GROUPS * 4 * R * SLOT;     // offsets: weight rings, gate / up exchange (4 KB)
+    static constexpr int RING = NS * SP * BSTEP, XCH = RING + GROUPS * 4 * R * SLOT;     // offsets: weight rings, gate / up exchange (4 KB)
     static constexpr int SMEM_USED = XCH + 4096 + 1024;
     static constexpr int SMEM = SMEM_USED > TC_SMEM_MIN ? SMEM_USED : TC_SMEM_MIN;
-    static_assert(SMEM <= 226 * 1024 && 2 * NT + 64 * GROUPS <= 512, "shared or tensor memory");
+    static_assert(SMEM <= 226 * 1024 && 2 * NT + 64 * NS * SP <= 512 && GROUPS % SP == 0 && GROUPS <= NS * SP, "shared or tensor memory");
     static_assert(REG_LOW + REG_READ + GROUPS * REG_MAKE <= 65536 / THREADS / 8 * 8 * (2 + GROUPS), "registers");
 };
 __device__ __forceinline__ bool elect_one() {
@@ -367,13 +374,20 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
     [[maybe_unused]] __shared__ bool s_last;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = warp >> 2;
     const int S = a.S, split = S > 1 ? (int)(blockIdx.x % (uint32_t)S) : 0;     // a cluster's CTAs are neighbours along x
-    const int first = S > 1 ? (int)(blockIdx.x / (uint32_t)S) : (int)blockIdx.x, stride = (int)gridDim.x / S;
     // this split's share of the steps: first those of the block minima, then those of the products
     const int mn0 = split * a.n_min / S, mn1 = (split + 1) * a.n_min / S;
     const int ma0 = split * a.n_main / S, ma1 = (split + 1) * a.n_main / S;
     const int nmn = mn1 - mn0, nst = nmn + ma1 - ma0, n_steps = a.n_min + a.n_main;
     const int spi = (nst + SP - 1) / SP;                                        // stages per item; the last may hold one step only
-    const int n_items = first < a.items ? (a.items - first + stride - 1) / stride : 0;
+    // This CTA's stages [q0, q1), counted through its items; the i-th of them is item_of(i).  Whole tiles are dealt in turn, so
+    // that CTAs side by side read the same activation tile at about the same time.
+    const long long all = (long long)a.items * spi;
+    auto q_begin = [&](int cta) { return (int)(cta * all / gridDim.x); };       // shared tiles: stages of all items in a row
+    const int cta = (int)blockIdx.x, n_cta = (int)gridDim.x;
+    const int q0 = a.shared ? q_begin(cta) : 0, q1 = a.shared ? q_begin(cta + 1) : S > 1 ? spi : (a.items - cta + n_cta - 1) / n_cta * spi;
+    auto item_of = [&](int i) { return a.shared ? i : S > 1 ? cta / S : cta + i * n_cta; };
+    auto m_of = [&](int item) { return item / a.tiles_n * NT; };                // first activation row and weight tile of an item
+    auto n_of = [&](int item) { return item % a.tiles_n; };
     if (tid == 0) {
         for (int i = 0; i < NS; ++i) { mbar_init(&full[i], 4 * SP + 1); mbar_init(&empty[i], 1); }
         mbar_init(&d_full, 1); mbar_init(&d_empty, 4);
@@ -406,7 +420,7 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
             for (int q = 0; q < 8; ++q) v += p[q];
             return v;
         };
-        const int tn = first % a.tiles_n, m0 = first / a.tiles_n * NT, n_col = min(NT, a.B - m0);
+        const int item = item_of(0), tn = n_of(item), m0 = m_of(item), n_col = min(NT, a.B - m0);
         const int n_out = PAIR ? tn * 64 + (row & 63) : tn * 128 + row;
         float* yp = a.y + (size_t)m0 * a.ldy + n_out;
         constexpr int LANES = PAIR ? 2 : 1;             // a pair's 64 rows: each half of the lanes takes its own columns
@@ -428,9 +442,11 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
             // ---- activation tiles ----
             uint32_t s = 0, par = 1, n = 0;
             const size_t group_bytes = (size_t)n_steps * (2 * TC_STEP_IMG);
-            for (int item = first; item < a.items; item += stride) {
-                const uint8_t* group = a.img + (size_t)(item / a.tiles_n) * (NT == 128 ? 2 : 1) * group_bytes;
-                for (int j = 0; j < spi; ++j, ++n) {
+            for (int q = q0; q < q1;) {
+                const int i = q / spi, j0 = q - i * spi, j1 = min(spi, j0 + q1 - q);
+                q += j1 - j0;
+                const uint8_t* group = a.img + (size_t)(item_of(i) / a.tiles_n) * (NT == 128 ? 2 : 1) * group_bytes;
+                for (int j = j0; j < j1; ++j, ++n) {
                     if (n >= (uint32_t)NS) wait_on(&empty[s], par);
                     const int st0 = j * SP, n_sub = SP == 1 ? 1 : min(SP, nst - st0);
                     if (lead) {
@@ -462,13 +478,15 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
             const uint32_t b_lo = (smem_u32(smB) & 0x3FFFFu) >> 4, d1 = tmem, d2 = tmem + NT;
             auto desc = [&](uint32_t lo) { return ((uint64_t)TC_DESC_HI << 32) | lo; };
             uint32_t s = 0, par = 0, periods = 0;
-            for (int k = 0; k < n_items; ++k) {
+            for (int q = q0; q < q1;) {
+                const int j0 = q % spi, j1 = min(spi, j0 + q1 - q);
+                q += j1 - j0;
                 int left = 0;                           // stages left in the period
-                for (int j = 0; j < spi; ++j) {
+                for (int j = j0; j < j1; ++j) {
                     const bool fresh = left == 0;
                     if (fresh) {                        // D of the period before must have been read
                         if (periods) wait_on(&d_empty, (periods - 1u) & 1u);
-                        left = min(a.period, spi - j);
+                        left = min(a.period, j1 - j);
                         ++periods;
                     }
                     --left;
@@ -479,10 +497,10 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                         for (int t = 0; t < SP; ++t) {
                             if (SP == 2 && t == 1 && 2 * j + 1 >= nst) break;
                             const uint32_t slot = s * SP + t, ac = tmem + A_COL + slot * 64u, bh = b_lo + slot * (uint32_t)(G::BSTEP / 16);
-                            if (t == 0 && fresh && j > 0) {     // D1 starts again, D2 goes on
+                            if (t == 0 && fresh && j > j0) {    // D1 starts again, D2 goes on
                                 tc_mma_ts(d1, ac, desc(bh), TC_IDESC<NT>, 0u);
                                 tc_mma_ts(d2, ac, desc(bh + NT * 8), TC_IDESC<NT>, 1u);
-                            } else tc_mma_ts(d1, ac, desc(bh), TC_IDESC<2 * NT>, (t > 0 || j > 0) ? 1u : 0u);
+                            } else tc_mma_ts(d1, ac, desc(bh), TC_IDESC<2 * NT>, (t > 0 || j > j0) ? 1u : 0u);
                             tc_mma_ts(d2, ac + 32u, desc(bh), TC_IDESC<NT>, 1u);
 #pragma unroll
                             for (uint32_t q = 1; q < 4; ++q) {
@@ -505,11 +523,19 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
         reg_inc<G::REG_READ>();
         pdl_wait();
         [[maybe_unused]] float* xch = reinterpret_cast<float*>(sm + G::XCH);
-        const int np = (spi + a.period - 1) / a.period;                                 // periods per item
         uint32_t par = 0;
         [[maybe_unused]] unsigned long long best[(NT + 31) / 32] = {};
-        for (int k = 0; k < n_items; ++k) {
-            const int item = first + k * stride, tn = item % a.tiles_n, m0 = item / a.tiles_n * NT;
+        [[maybe_unused]] auto flush_best = [&](int m0) {
+#pragma unroll
+            for (int i = 0; i < (NT + 31) / 32; ++i) {
+                if (32 * i + lane < min(NT, a.B - m0) && best[i]) atomicMax(a.best + m0 + 32 * i + lane, best[i]);
+                best[i] = 0;
+            }
+        };
+        for (int q = q0; q < q1;) {
+            const int i0 = q / spi, j0 = q - i0 * spi, j1 = min(spi, j0 + q1 - q), item = item_of(i0), tn = n_of(item), m0 = m_of(item);
+            const int np = (j1 - j0 + a.period - 1) / a.period;                         // accumulation periods
+            q += j1 - j0;
             float acc[NT];
 #pragma unroll
             for (int c = 0; c < NT; ++c) acc[c] = 0.f;
@@ -518,24 +544,20 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                 wait_on(&d_full, par);
                 par ^= 1u;
                 tc_fence_after();
+                auto take = [&](uint32_t col) {         // the tensor core may wait for this: few round trips
+                    constexpr int CH = NT < 32 ? NT : 32;
 #pragma unroll
-                for (int ch = 0; ch < NT; ch += 16) {
-                    float v[16];
-                    tc_ld16(tlane + ch, v);
-                    tc_ld_wait();
+                    for (int ch = 0; ch < NT; ch += CH) {
+                        float v[CH / 16][16];
 #pragma unroll
-                    for (int c = 0; c < 16; ++c) acc[ch + c] += v[c];
-                }
-                if (p == np - 1) {
-#pragma unroll
-                    for (int ch = 0; ch < NT; ch += 16) {
-                        float v[16];
-                        tc_ld16(tlane + NT + ch, v);
+                        for (int h = 0; h < CH / 16; ++h) tc_ld16(col + ch + 16 * h, v[h]);
                         tc_ld_wait();
 #pragma unroll
-                        for (int c = 0; c < 16; ++c) acc[ch + c] += v[c];
+                        for (int c = 0; c < CH; ++c) acc[ch + c] += v[c / 16][c % 16];
                     }
-                }
+                };
+                take(tlane);
+                if (p == np - 1) take(tlane + NT);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&d_empty);
@@ -545,6 +567,51 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
 #pragma unroll
                 for (int c = 0; c < NT; ++c) ex[c * 128 + row] = acc[c];
                 break;
+            }
+            if (j1 - j0 < spi) {
+                // a tile that several CTAs share: leave the partial sums; the CTA that arrives last adds all of them
+                auto cta_of = [&](int qq) {
+                    int c = (int)((long long)qq * n_cta / all);
+                    while (q_begin(c) > qq) --c;
+                    while (q_begin(c + 1) <= qq) ++c;
+                    return c;
+                };
+                const int c_lo = cta_of(item * spi), c_hi = cta_of(item * spi + spi - 1);
+                auto slot_of = [&](int c) { return a.part + (size_t)(2 * c + (c == c_lo ? 1 : 0)) * (NT * 128) + row; };   // it begins here, or before
+                float* out = slot_of(cta);
+#pragma unroll
+                for (int c = 0; c < NT; ++c) out[c * 128] = acc[c];
+                __threadfence();
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (tid == 128) {
+                    const unsigned int seen = atomicAdd(a.tickets + c_lo, 1u);
+                    s_last = seen == (unsigned int)(c_hi - c_lo);
+                    if (s_last) a.tickets[c_lo] = 0u;
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                const bool last = s_last;
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (!last) continue;
+                __threadfence();
+                constexpr int CH = NT < 32 ? NT : 32;           // columns whose loads are in flight together
+#pragma unroll
+                for (int ch = 0; ch < NT; ch += CH) {
+                    const float* in = slot_of(c_lo) + ch * 128;
+#pragma unroll
+                    for (int c = 0; c < CH; ++c) acc[ch + c] = __ldcg(in + c * 128);
+                }
+#pragma unroll 1
+                for (int other = c_lo + 1; other <= c_hi; ++other) {
+                    const float* in = slot_of(other);
+#pragma unroll
+                    for (int ch = 0; ch < NT; ch += CH) {
+                        float t[CH];
+#pragma unroll
+                        for (int c = 0; c < CH; ++c) t[c] = __ldcg(in + (ch + c) * 128);
+#pragma unroll
+                        for (int c = 0; c < CH; ++c) acc[ch + c] += t[c];
+                    }
+                }
             }
             const int n_out = PAIR ? tn * 64 + (row & 63) : tn * 128 + row, n_col = min(NT, a.B - m0);
             float* yp = a.y + (size_t)m0 * a.ldy + n_out;
@@ -586,17 +653,12 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                     } else if (c < n_col && n_out < a.N) yp[(size_t)c * a.ldy] = v;
                 }
                 if constexpr (MODE == TC_ARGMAX)
-                    if (a.B > NT || k == n_items - 1) {         // the columns change with the next item, or there is none
-#pragma unroll
-                        for (int i = 0; i < (NT + 31) / 32; ++i) {
-                            if (32 * i + lane < n_col) atomicMax(a.best + m0 + 32 * i + lane, best[i]);
-                            best[i] = 0;
-                        }
-                    }
+                    if (a.B > NT) flush_best(m0);          // the columns change with the next item
             }
         }
         if (S > 1) finish_split();
         if constexpr (MODE == TC_ARGMAX) {              // the last CTA to end decodes the winners and clears the keys
+            flush_best(0);
             __threadfence();
             asm volatile("bar.sync 1, 128;" ::: "memory");
             if (tid == 128) s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
@@ -619,33 +681,37 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
         // ---- weights ----
         reg_set<G::REG_MAKE, 65536 / G::THREADS / 8 * 8>();
         const int grp = wg - 2, quarter = warp & 3;
-        const uint32_t stage = (uint32_t)(grp / SP);    // this group fills step grp % SP of every NS-th stage, counted over all items
+        // This group fills step `sub` of every GROUPS / SP-th stage of the CTA's range.  It waits for a ring slot to be emptied
+        // without having followed every phase of it, which is sound because the slots empty in order: it has seen a later
+        // one than the slot's last but one use empty (GROUPS <= NS * SP).
+        const int sub = grp % SP;
         uint8_t* ring = sm + G::RING + (warp - 8) * G::R * G::SLOT;
         const uint32_t ring_s = smem_u32(ring);
         const WeightRef w = (PAIR && quarter >= 2) ? a.w1 : a.w0;                      // lanes 64..127 of a pair: up rows
         const bool scales_async = WT == WT_Q4_K || ((a.units & 1) == 0 && ((uintptr_t)w.d & 3) == 0);
         auto row_of = [&](int tn, int r) { return min(PAIR ? tn * 64 + (r & 63) : tn * 128 + r, a.N - 1); };
         const int rpu = WT == WT_Q4_0 ? a.units : WT == WT_Q8_0 ? 2 * a.units : (a.units >> 3) * 9;     // uint4 per weight row
-        struct Cursor { int k, j; };                    // item, stage of the item
-        auto settle = [&](Cursor& c) { while (c.j >= spi && c.k < n_items) { c.j -= spi; ++c.k; } };
+        struct Cursor { int q, i, j; };                 // stage: of the range, item of the range and stage of the item
+        constexpr int HOP = G::GROUPS / SP;
+        auto next = [&](Cursor& c) { c.q += HOP; c.j += HOP; while (c.j >= spi) { c.j -= spi; ++c.i; } };
 
         // fetch cursor, R tiles ahead of the production cursor
-        Cursor f = {0, (int)stage};
-        settle(f);
+        const int q_first = q0 + grp / SP;
+        Cursor f = {q_first, q_first / spi, q_first % spi};
         int f_k = -1; uint32_t f_n = 0;                 // item that the row pointers belong to; ring slot
         constexpr int LPR = G::QB / 16, FI = LPR;       // lanes per row and copies per lane of a step's codes
         const uint4 *f_q[FI], *f_h = nullptr; const __half* f_d = nullptr;
         auto fetch = [&]() {
-            if (f.k < n_items) {
-                if (f_k != f.k) {
-                    f_k = f.k;
-                    const int tn = (first + f.k * stride) % a.tiles_n;
+            if (f.q < q1) {
+                if (f_k != f.i) {
+                    f_k = f.i;
+                    const int tn = n_of(item_of(f.i));
 #pragma unroll
                     for (int h = 0; h < FI; ++h) f_q[h] = w.q + (size_t)row_of(tn, quarter * 32 + (32 / FI) * h + lane / LPR) * rpu;
                     if constexpr (WT != WT_Q4_K) f_d = w.d + (size_t)row_of(tn, row) * a.units;
                     else f_h = w.q + (size_t)row_of(tn, row) * rpu;
                 }
-                const int st = f.j * SP + grp % SP, ks = ma0 + st - nmn;
+                const int st = f.j * SP + sub, ks = ma0 + st - nmn;
                 if (st >= nmn && st < nst) {
                     const uint32_t dst = ring_s + f_n * G::SLOT;
                     const int piece = lane % LPR;
@@ -658,21 +724,17 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                     if constexpr (WT != WT_Q4_K) { if (scales_async) cp_async4(dst + 32 * G::QB + lane * 4, f_d + 2 * ks); }
                     else cp_async16_l1(dst + 32 * G::QB + lane * 16, f_h + (ks >> 2) * 9);
                 }
-                f.j += NS;
-                settle(f);
+                next(f);
             }
             if (++f_n == (uint32_t)G::R) f_n = 0;
             cp_commit();
         };
         for (int j = 0; j < G::R; ++j) fetch();
-        const uint32_t acol = tlane + A_COL + (uint32_t)grp * 64u;
-        uint32_t at = 0, par = 1;                       // ring slot; parity of the next wait for an empty stage
-        bool again = false;                             // this group has filled its slot before
-        Cursor c = {0, (int)stage};
-        settle(c);
-        while (c.k < n_items) {
-            const int tn = (first + c.k * stride) % a.tiles_n;
-            const int st = c.j * SP + grp % SP, ks = ma0 + st - nmn;
+        uint32_t at = 0;                                // weight ring slot
+        bool waited = false;
+        for (Cursor c = {q_first, q_first / spi, q_first % spi}; c.q < q1; next(c)) {
+            const int st = c.j * SP + sub, ks = ma0 + st - nmn;
+            const uint32_t nth = (uint32_t)(c.q - q0), stage = nth % NS, acol = tlane + A_COL + (stage * SP + sub) * 64u;
             cp_wait<G::R - 1>();
             __syncwarp();
             const uint8_t* slot = ring + at * G::SLOT;
@@ -685,17 +747,15 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
             uint32_t d01 = 0; uint4 hdr = make_uint4(0, 0, 0, 0);
             if constexpr (WT != WT_Q4_K) d01 = *reinterpret_cast<const uint32_t*>(slot + 32 * G::QB + lane * 4);
             else hdr = *reinterpret_cast<const uint4*>(slot + 32 * G::QB + lane * 16);
-            __syncwarp();
-            fetch();
-            if (again) {                                // the tensor core is done with this group's tile before
-                wait_on(&empty[stage], par);
+            if (!waited) { pdl_wait(); waited = true; } // no bounded wait below spans an earlier kernel
+            if (nth >= (uint32_t)NS) {                  // the tensor core is done with what the slot held
+                wait_on(&empty[stage], (nth / NS - 1u) & 1u);
                 tc_fence_after();
-            } else { pdl_wait(); again = true; }        // (nothing was awaited before; from here on bounded waits span no earlier kernel)
-            par ^= 1u;
+            }
             if (st < nst) {
                 if constexpr (WT != WT_Q4_K) {
                     if (!scales_async) {                // odd number of blocks per row: their scales are not pairs of aligned halves
-                        const unsigned short* dp = reinterpret_cast<const unsigned short*>(w.d) + (size_t)row_of(tn, row) * a.units + 2 * ks;
+                        const unsigned short* dp = reinterpret_cast<const unsigned short*>(w.d) + (size_t)row_of(n_of(item_of(c.i)), row) * a.units + 2 * ks;
                         d01 = (uint32_t)dp[0] | (2 * ks + 1 < a.units ? (uint32_t)dp[1] << 16 : 0u);
                     }
 #pragma unroll
@@ -761,7 +821,7 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                 } else {
                     // a step of block minima: -32 dmin m of 64 sub-blocks (the image holds the sums over 32 activations / 32)
                     const int sb0 = (mn0 + st) * 8, n_sb = a.units >> 3;
-                    const uint4* src = w.q + (size_t)row_of(tn, row) * rpu;
+                    const uint4* src = w.q + (size_t)row_of(n_of(item_of(c.i)), row) * rpu;
 #pragma unroll 1
                     for (int b = 0; b < 4; ++b) {
                         uint32_t whi[8], wlo[8];
@@ -785,14 +845,14 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                         tc_st8(acol + 32u + b * 8u, wlo);
                     }
                 }
-                tc_st_wait();
-                tc_fence_before();
             }
+            __syncwarp();
+            fetch();                                    // into the slot just taken, while the stores are under way
+            tc_st_wait();
+            tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&full[stage]);
             if (++at == (uint32_t)G::R) at = 0;
-            c.j += NS;
-            settle(c);
         }
         cp_wait<0>();
         if (S > 1) finish_split();
@@ -803,23 +863,28 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
 }
 
 // ---- host ----------------------------------------------------------------------------------------------------------
-static bool tc_policy_takes(int wtype, const GemvArgs& a, bool pair) {
-    if (g_tc_policy < 0) g_tc_policy = getenv("ADAM_B200_TC") ? atoi(getenv("ADAM_B200_TC")) : 1;
-    if (g_tc_policy == 0) return false;
-    if (g_tc_policy == 2) return true;
-    (void)wtype; (void)pair;
-    static const int mr = getenv("TCMIN") ? atoi(getenv("TCMIN")) : 9;
-    static const int ml = getenv("TCLM") ? atoi(getenv("TCLM")) : 9;
-    return a.B >= (a.epi == EPI_ARGMAX ? ml : mr);
+// Fewest rows from which the GEMM is faster than the GEMV kernels, measured in decode steps and single calls.  The GEMV
+// passes over the weights once per 1, 2 or 4 rows; where the passes run side by side on idle SMs (matrices of a few MB) that
+// costs little (1B shape, 9 rows: 1.22 against 1.31 ms per step; 12: equal; 16: 1.39 against 1.33), where they fill the GPU
+// it costs their number (27B shape, 4 rows: 1.62 against 1.88 ms, 6: 2.16 against 2.03, 12: 3.93 against 2.08).  An LM head of a
+// narrow model is bound by rebuilding weights here (262144 x 1152: 75 us whatever the rows, the GEMV 43 us at 4 and 71 at 8).
+// Without a row-tiled copy a GEMV takes one launch per four rows (7 us each), and Q8_0 / Q5_0 have no tensor-core GEMV.
+static int tc_rows_from(int wtype, const GemvArgs& a, bool pair, bool tiled) {
+    if (wtype == WT_Q8_0) return 4;
+    if (!tiled) return 5;
+    const double bytes = (double)a.N * a.K * 0.5625 * (pair ? 2 : 1);
+    if (a.epi == EPI_ARGMAX && a.K < 4096) return 9;
+    return bytes > 16.0e6 ? 6 : 13;
 }
 
-bool gemm_tc_supports(int wtype, const GemvArgs& a) {
+bool gemm_tc_supports(int wtype, const GemvArgs& a, bool tiled) {
     const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU;
     if (wtype != WT_Q4_0 && wtype != WT_Q4_K && (wtype != WT_Q8_0 || pair)) return false;
     if (a.B < TC_MIN_ROWS || a.K <= 0 || a.K > TC_MAX_K || a.N < 16 || (!a.y && a.epi != EPI_ARGMAX) || (wtype == WT_Q4_K ? (a.K % 256) : (a.K % 32))) return false;
     if (a.epi == EPI_ARGMAX && a.B > tc_rows_fit(wtype, a.K)) return false;
     if ((a.ldx & 3) || (!a.h_in && (!a.x || ((uintptr_t)a.x & 15)))) return false;
-    if (!tc_policy_takes(wtype, a, pair)) return false;
+    if (g_tc_policy < 0) g_tc_policy = getenv("ADAM_B200_TC") ? atoi(getenv("ADAM_B200_TC")) : 1;
+    if (g_tc_policy == 0 || (g_tc_policy == 1 && a.B < tc_rows_from(wtype, a, pair, tiled))) return false;
     return tc_rows_fit(wtype, a.K) >= 128;
 }
 
@@ -835,6 +900,25 @@ template <int WT, int MODE> static TcPick& tc_pick(int nt) {
 template <int WT> static TcPick& tc_pick(int nt, int mode) {
     if constexpr (WT != WT_Q8_0) { if (mode == TC_PAIR) return tc_pick<WT, TC_PAIR>(nt); }
     return mode == TC_ARGMAX ? tc_pick<WT, TC_ARGMAX>(nt) : tc_pick<WT, TC_STORE>(nt);
+}
+
+// Clusters of `s` CTAs that run at the same time, one CTA per SM (clusters stay inside a GPC).
+static int tc_clusters_at_once(int s) {
+    static int known[9] = {};
+    if (!known[s]) {
+        TcPick& p = tc_pick<WT_Q4_0, 16, TC_STORE>();
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)s); cfg.blockDim = dim3((unsigned)p.threads); cfg.dynamicSmemBytes = (size_t)p.smem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)s; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        cfg.attrs = at; cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaFuncSetAttribute((const void*)p.k, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, (const void*)p.k, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+        known[s] = n > 0 ? n : -1;
+    }
+    return known[s];
 }
 
 static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
@@ -856,27 +940,40 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
         }
         count_launch();
     }
-    // K splits: the cheapest under an estimate in SM cycles.  A step costs the larger of its tensor-core time (6 cycles per
-    // activation row) and its rebuilding (about 330 issue slots); a CTA costs about 3000 cycles besides, a split 1500 more.
-    const int nt = a.B <= 16 ? 16 : a.B <= 32 ? 32 : a.B <= 64 ? 64 : 128;
+    // Work split: the cheapest under an estimate in SM cycles.  A step costs the larger of its tensor-core time and what
+    // the rebuilding of a weight tile allows.  Dealt out evenly, a CTA costs its stages and, where tiles are shared, the
+    // adding up of P partial results of nt columns; as clusters of S, waves of CTAs and one exchange.
+    const int nt = a.B <= 16 ? 16 : a.B <= 32 ? 32 : a.B <= 64 ? 64 : 128, sp = nt == 128 ? 1 : 2;
     const int tiles_n = pair ? (a.N + 63) / 64 : (a.N + 127) / 128, tiles_m = (a.B + nt - 1) / nt;
     const long long items = (long long)tiles_n * tiles_m;
-    int S = 1;
+    const double step = nt == 128 ? 900.0 : nt == 64 ? 620.0 : 500.0;
+    const int spi1 = (n_min + n_main + sp - 1) / sp;
+    int S = 1, grid = 1;
+    bool shared = false;
     double best = 1e300;
-    for (int s = 1; s <= (a.epi == EPI_ARGMAX ? 1 : 8) && s <= n_main; s *= 2) {
-        const double waves = (double)((items * s + g.sm_count - 1) / g.sm_count);
+    auto offer = [&](double cost, int s, int ctas, bool sh) { if (cost < best * 0.999) { best = cost; S = s; grid = ctas; shared = sh; } };
+    const long long all = items * spi1;
+    const int whole = (int)(items < g.sm_count ? items : g.sm_count);
+    offer((double)((items + whole - 1) / whole) * spi1 * sp * step, 1, whole, false);
+    if (all >= g.sm_count) {
+        const double per = (double)((all + g.sm_count - 1) / g.sm_count), sharers = 2.0 + spi1 / per;
+        offer(per * sp * step + 3000.0 + nt * (20.0 + 40.0 * sharers), 1, g.sm_count, true);
+    }
+    for (int s = 2; s <= (a.epi == EPI_ARGMAX ? 1 : 8) && s <= n_main; ++s) {
+        const int at_once = tc_clusters_at_once(s);
+        if (at_once < 1) continue;
         const int steps = (n_main + s - 1) / s + (n_min + s - 1) / s;
-        const double cost = waves * (steps * fmax(6.0 * nt, 330.0) + (s > 1 ? 4500.0 : 3000.0));
-        if (cost < best * 0.999) { best = cost; S = s; }
+        offer((double)((items + at_once - 1) / at_once) * ((steps + sp - 1) / sp * sp * step + 2000.0), s, (int)items * s, false);
     }
     TcGemm t = {};
     t.w0 = a.w0; t.w1 = a.w1; t.y = a.y; t.ldy = a.ldy; t.img = g_tc.img; t.inv = g_tc.inv; t.err = g.dev_err;
     t.N = a.N; t.units = a.K / 32; t.B = a.B; t.swiglu = a.epi == EPI_SWIGLU;
     t.n_min = n_min; t.n_main = n_main; t.S = S;
-    const int sp = nt == 128 ? 1 : 2, stages = ((n_main + S - 1) / S + (n_min + S - 1) / S + sp - 1) / sp, n_periods = (stages * sp + TC_PERIOD - 1) / TC_PERIOD;
+    const int stages = ((n_main + S - 1) / S + (n_min + S - 1) / S + sp - 1) / sp, n_periods = (stages * sp + TC_PERIOD - 1) / TC_PERIOD;
     t.period = (stages + n_periods - 1) / n_periods;
     t.tiles_n = tiles_n;
     t.items = (int)items;
+    t.part = g_tc.part; t.tickets = g_tc.tickets; t.shared = shared ? 1 : 0;
     const int mode = pair ? TC_PAIR : a.epi == EPI_ARGMAX ? TC_ARGMAX : TC_STORE;
     if (mode == TC_ARGMAX) {
         t.best = g_tc.best; t.ticket = (unsigned int*)(g_tc.best + g_tc.inv_cap);
@@ -889,8 +986,8 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
         p.attr = true;
     }
     cudaError_t e;
-    if (S == 1) e = launch_k(p.k, dim3((unsigned)(t.items < g.sm_count ? t.items : g.sm_count)), dim3(p.threads), (size_t)p.smem, stream, true, t);
-    else e = launch_k_cluster(p.k, dim3((unsigned)(t.items * S)), dim3(p.threads), (size_t)p.smem, stream, true, (unsigned)S, t);
+    if (S == 1) e = launch_k(p.k, dim3((unsigned)grid), dim3(p.threads), (size_t)p.smem, stream, true, t);
+    else e = launch_k_cluster(p.k, dim3((unsigned)grid), dim3(p.threads), (size_t)p.smem, stream, true, (unsigned)S, t);
     if (e != cudaSuccess) return fail(ADAMAH_ERR_BACKEND, "gemm_tc: launch failed: %s", cudaGetErrorString(e));
     count_launch();
     return ADAMAH_OK;

@@ -6,10 +6,10 @@
 
 namespace ab {
 
-constexpr int TC_MIN_ROWS = 2;         // fewer rows than this stay on the GEMV kernels
+constexpr int TC_MIN_ROWS = 2;         // fewer rows than this never leave the GEMV kernels
 
-// Can this problem run on the tcgen05 path?  (STORE / GEGLU / SWIGLU epilogues, TC_MIN_ROWS rows and more.)
-bool gemm_tc_supports(int wtype, const GemvArgs& a);
+// Does this problem run on the tcgen05 path?  `tiled`: the GEMV kernels would have row-tiled copies of the weights.
+bool gemm_tc_supports(int wtype, const GemvArgs& a, bool tiled);
 // Makes room for calls with up to `rows` activation rows of length K (outside any stream capture; longer calls run in
 // chunks).  The workspace only grows; false when out of memory.
 bool gemm_tc_prepare(int rows, int K);
