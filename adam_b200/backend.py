@@ -16,6 +16,7 @@ import numpy as np
 from . import _lib
 from ._lib import DecodePlanOp  # noqa: F401  (re-exported)
 from . import constants as C
+from .host_arrays import HostArrays
 
 _SCHED_NAMES = {0: "legacy", 1: "alias_safe", 2: "level_batched"}
 
@@ -51,6 +52,7 @@ class Adamah:
         self._has_map_upload_gguf_blocks = True
         self._has_decoder = True
         self._is_integrated_gpu = False
+        self.host_arrays = HostArrays(self._lib)
         dev, sms, mem = ctypes.c_int(), ctypes.c_int(), ctypes.c_uint64()
         self._lib.adam_b200_device_info(ctypes.byref(dev), ctypes.byref(sms), ctypes.byref(mem))
         self.device_index, self.sm_count, self.total_mem = dev.value, sms.value, mem.value
@@ -470,6 +472,7 @@ class Adamah:
     def shutdown(self):
         if not self._closed:
             self._closed = True
+            self.host_arrays.close()
             self._lib.adamah_shutdown()
 
     def __repr__(self):

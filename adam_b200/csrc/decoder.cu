@@ -65,6 +65,7 @@ struct Decoder {
     // chunked prefill: what the rows of all chunks are (device copy and pinned source of one call; see PrefillPlan)
     uint8_t *plan, *plan_pin; size_t plan_cap; cudaEvent_t plan_read;
     std::vector<PrefillChunk> chunks; const int32_t* plan_n;
+    float* score_logits; cudaEvent_t score_ev[4]; cudaStream_t score_copy;      // adam_b200_decoder_score: two groups of rows of logits, and their copies to the host
     uint32_t rows_cap;          // rows the activation buffers hold
     std::vector<uint32_t> hpos, hplen, hres;   // host mirror of positions, prompt lengths and reserved tokens (argument checks)
     std::vector<int32_t> hbt;            // host mirror of the block table
@@ -695,6 +696,9 @@ static void destroy(Decoder* D) {
     for (void* p : ptrs) cudaFree(p);
     cudaFreeHost(D->plan_pin);
     if (D->plan_read) cudaEventDestroy(D->plan_read);
+    cudaFree(D->score_logits);
+    for (cudaEvent_t e : D->score_ev) if (e) cudaEventDestroy(e);
+    if (D->score_copy) cudaStreamDestroy(D->score_copy);
     delete D;
 }
 
@@ -854,6 +858,32 @@ static int enqueue_step(Decoder* D, uint32_t batch, bool with_lm, bool want_logi
 // QKV, attention, o-proj) and the FFN half (gate/up, down) of layer L; part 2*n_layer is the
 // LM head, part 2*n_layer + 1 advances the positions.  A tensor-parallel caller all-reduces
 // `proj` after every layer part and merges the arg-max pairs after the LM-head part.
+// The LM head over rows r0 .. r0 + rows of the step's or chunk's residual stream: winners to tok / val ([rows]), the
+// soft-capped logits to `logits` ([rows][n_vocab]) where it is given.
+static int enqueue_head(Decoder* D, uint32_t r0, uint32_t rows, float* logits, int32_t* tok, float* val) {
+    const adam_b200_decoder_desc& d = D->d;
+    const uint32_t E = d.n_embd;
+    const Mat& lm = D->output.bound ? D->output : D->embd;
+    int rc;
+    GemvArgs a = {};
+    a.ldx = (int)E; a.eps = d.norm_eps; a.h_in = D->hbuf[1] + (size_t)r0 * E; a.add_src = D->proj + (size_t)r0 * E;
+    a.w_post = D->layers[d.n_layer - 1].norm[NORM_POST_FFW]; a.w_pre = D->output_norm; a.h_out = D->hbuf[0] + (size_t)r0 * E;
+    a.y = logits; a.ldy = (int)lm.rows; a.softcap = d.final_softcap;
+    a.out_tok = tok; a.out_val = val;
+    a.w0 = lm.w; a.N = (int)lm.rows; a.K = (int)lm.cols; a.B = (int)rows; a.epi = EPI_ARGMAX;
+    D->h_final = 0;
+    if (gemm_tc_supports(lm.wtype, a, lm.tiled != nullptr)) return launch_gemm_tc(lm.wtype, a, g.stream);
+    if (wt_is_b8(lm.wtype)) {
+        // Q8_0 / Q5_0 LM head: the norm chain, the products and the arg-max as three kernels; the products land in the
+        // logits buffer (soft-capped afterwards only when the caller wants them)
+        float* y = logits ? logits : D->logits;
+        if ((rc = launch_chain_rows(a.h_in, a.add_src, a.w_post, a.w_pre, a.h_out, D->act, (int)E, (int)rows, d.norm_eps, g.stream, g.pdl))) return rc;
+        if ((rc = launch_gemv_b8(lm.wtype, lm.w, D->act, (int)E, y, (int)lm.rows, (int)lm.rows, (int)E, (int)rows, g.stream))) return rc;
+        return launch_argmax_rows(y, (int)lm.rows, (int)rows, d.final_softcap, logits != nullptr, tok, val, nullptr, g.stream, false);
+    }
+    if ((rc = argmax_scratch(&a.part_val, &a.part_idx, &a.ticket))) return rc;
+    return gemv(lm, nullptr, a, (int)rows, EPI_ARGMAX);
+}
 static uint32_t n_parts(const Decoder* D) { return 2 * D->d.n_layer + 2; }
 static int enqueue_part(Decoder* D, uint32_t batch, uint32_t part, bool with_lm, bool want_logits) {
     const adam_b200_decoder_desc& d = D->d;
@@ -908,31 +938,7 @@ static int enqueue_part(Decoder* D, uint32_t batch, uint32_t part, bool with_lm,
         if ((rc = gemv(ly.m[MAT_DOWN], nullptr, dn, batch, EPI_STORE))) return rc;
     } else if (part == 2 * d.n_layer) {
         if (with_lm) {
-            const Mat& lm = D->output.bound ? D->output : D->embd;
-            GemvArgs a = {};
-            a.ldx = (int)E; a.eps = d.norm_eps; a.h_in = D->hbuf[1]; a.add_src = D->proj;
-            a.w_post = D->layers[d.n_layer - 1].norm[NORM_POST_FFW]; a.w_pre = D->output_norm; a.h_out = D->hbuf[0];
-            a.y = want_logits ? D->logits : nullptr; a.ldy = (int)lm.rows; a.softcap = d.final_softcap;
-            a.out_tok = D->cur_tok; a.out_val = D->cur_val;
-            a.w0 = lm.w; a.N = (int)lm.rows; a.K = (int)lm.cols; a.B = (int)batch; a.epi = EPI_ARGMAX;
-            if (gemm_tc_supports(lm.wtype, a, lm.tiled != nullptr)) {
-                if ((rc = launch_gemm_tc(lm.wtype, a, g.stream))) return rc;
-                D->h_final = 0;
-                return check_launch("decoder step");
-            }
-            if (wt_is_b8(lm.wtype)) {
-                // Q8_0 / Q5_0 LM head: the norm chain, the products and the arg-max as three kernels; the products land
-                // in the logits buffer (soft-capped afterwards only when the caller wants them)
-                if ((rc = launch_chain_rows(D->hbuf[1], D->proj, D->layers[d.n_layer - 1].norm[NORM_POST_FFW], D->output_norm, D->hbuf[0], D->act,
-                                            (int)E, (int)batch, d.norm_eps, g.stream, g.pdl))) return rc;
-                if ((rc = launch_gemv_b8(lm.wtype, lm.w, D->act, (int)E, D->logits, (int)lm.rows, (int)lm.rows, (int)E, (int)batch, g.stream))) return rc;
-                if ((rc = launch_argmax_rows(D->logits, (int)lm.rows, (int)batch, d.final_softcap, want_logits, D->cur_tok, D->cur_val, nullptr, g.stream, false))) return rc;
-                D->h_final = 0;
-                return check_launch("decoder step");
-            }
-            if ((rc = argmax_scratch(&a.part_val, &a.part_idx, &a.ticket))) return rc;
-            if ((rc = gemv(lm, nullptr, a, batch, EPI_ARGMAX))) return rc;
-            D->h_final = 0;
+            if ((rc = enqueue_head(D, 0, batch, want_logits ? D->logits : nullptr, D->cur_tok, D->cur_val))) return rc;
         }
     } else {
         launch_k(k_advance, dim3((batch + 63) / 64), dim3(64), 0, g.stream, g.pdl, D->pos, D->cur_tok, D->gen_log, d.kv_cap, batch, with_lm ? 1 : 0);
@@ -1685,6 +1691,70 @@ extern "C" int adam_b200_decoder_prefill_ragged(uint32_t id, const uint32_t* n_t
     }
     if (rc == ADAMAH_OK) for (uint32_t b = 0; b < D->batch; ++b) D->hpos[b] += n_tokens[b];
     end_of_op();
+    return rc;
+}
+
+// Logits after every one of the next n_tokens prompt tokens of the single active sequence (a text under evaluation): the
+// positions go through the layers together like a prompt, then the LM head runs over the chunk's rows, and the logits of
+// one group of rows travel to the host while the next is computed.  Bound by the copy (1 MB per position at the 1B shape)
+// and the latency of the layers' kernels.
+// Leaves the decoder as n_tokens steps would: positions, log, current token, and the last position's rows in the buffers
+// that adam_b200_decoder_read_buffer reads.
+extern "C" int adam_b200_decoder_score(uint32_t id, uint32_t n_tokens, float* out) {
+    Decoder* D = get_dec(id);
+    if (!D) return ADAMAH_ERR_NOT_FOUND;
+    if (capturing()) return fail(ADAMAH_ERR_INVALID, "decoder_score: not allowed while a graph is being captured");
+    if (!out || n_tokens == 0 || D->batch != 1) return fail(ADAMAH_ERR_INVALID, "decoder_score: needs one active sequence, tokens and a destination");
+    const adam_b200_decoder_desc& d = D->d;
+    if (d.tp_size > 1) return fail(ADAMAH_ERR_INVALID, "decoder_score: not available with tensor parallelism");
+    int rc = check_prefill(D, &n_tokens, "decoder_score");
+    if (rc || (rc = plan_prefill(D, &n_tokens))) return rc;
+    constexpr uint32_t GROUP = 64;                      // rows per LM-head call: one arg-max scratch, one buffer of logits
+    if (!D->score_logits) {
+        DCU(cudaMalloc((void**)&D->score_logits, (size_t)2 * GROUP * d.n_vocab * 4 + 2 * GROUP * 8));
+        for (cudaEvent_t& e : D->score_ev) DCU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        DCU(cudaStreamCreateWithFlags(&D->score_copy, cudaStreamNonBlocking));
+    }
+    int32_t* tok = (int32_t*)(D->score_logits + (size_t)2 * GROUP * d.n_vocab);
+    float* val = (float*)(tok + GROUP);
+    { float* pv; int* pi; unsigned int* tk; if ((rc = argmax_scratch(&pv, &pi, &tk))) return rc; }
+    uint32_t done = 0, n_group = 0, last_row = 0, in_group = 0;
+    const uint32_t p0 = D->hpos[0];
+    g.pdl = pdl_allowed();
+    for (const PrefillChunk& c : D->chunks) {
+        for (uint32_t part = 0; part < 2 * d.n_layer && rc == ADAMAH_OK; ++part) rc = enqueue_prefill_part(D, c, part);
+        for (uint32_t r0 = 0; r0 < c.n_rows && rc == ADAMAH_OK; r0 += GROUP, ++n_group) {
+            const uint32_t m = std::min(GROUP, c.n_rows - r0), half = n_group & 1u;
+            float* lg = D->score_logits + (size_t)half * GROUP * d.n_vocab;
+            if (n_group >= 2) cudaStreamWaitEvent(g.stream, D->score_ev[2 + half], 0);      // the half's copy has left
+            if ((rc = enqueue_head(D, r0, m, lg, tok, val))) break;
+            // logged as the token of the position behind, as a step's
+            const uint32_t fits = p0 + done + 1 < d.kv_cap ? std::min(m, d.kv_cap - p0 - done - 1) : 0;
+            if (fits) cudaMemcpyAsync(D->gen_log + p0 + done + 1, tok, (size_t)fits * 4, cudaMemcpyDeviceToDevice, g.stream);
+            cudaEventRecord(D->score_ev[half], g.stream);
+            cudaStreamWaitEvent(D->score_copy, D->score_ev[half], 0);
+            cudaMemcpyAsync(out + (size_t)done * d.n_vocab, lg, (size_t)m * d.n_vocab * 4, cudaMemcpyDeviceToHost, D->score_copy);
+            cudaEventRecord(D->score_ev[2 + half], D->score_copy);
+            done += m; last_row = r0 + m - 1; in_group = m - 1;
+        }
+        if (rc) break;
+    }
+    if (rc == ADAMAH_OK) {
+        enqueue_prefill_end(D);
+        cudaMemcpyAsync(D->cur_tok, tok + in_group, 4, cudaMemcpyDeviceToDevice, g.stream);
+        cudaMemcpyAsync(D->cur_val, val + in_group, 4, cudaMemcpyDeviceToDevice, g.stream);
+        const uint32_t q_dim = d.n_head * d.head_dim, qkv_ld = q_dim + 2 * d.n_head_kv * d.head_dim;
+        float* bufs[5] = {D->hbuf[0], D->qkv, D->attn_out, D->proj, D->act};
+        const uint32_t lds[5] = {d.n_embd, qkv_ld, q_dim, d.n_embd, d.n_ff};
+        if (last_row) for (int i = 0; i < 5; ++i) cudaMemcpyAsync(bufs[i], bufs[i] + (size_t)last_row * lds[i], (size_t)lds[i] * 4, cudaMemcpyDeviceToDevice, g.stream);
+        rc = check_launch("decoder score");
+    }
+    g.pdl = false;
+    D->chunks.clear();
+    if (rc == ADAMAH_OK) D->hpos[0] += n_tokens;
+    cudaStreamSynchronize(D->score_copy);
+    DCU(cudaStreamSynchronize(g.stream));               // the caller reads `out` on return
+    g.submits++;
     return rc;
 }
 

@@ -279,6 +279,14 @@ extern "C" int adam_b200_set_stream(uint64_t stream) {
     return ADAMAH_OK;
 }
 
+extern "C" void* adam_b200_host_alloc(uint64_t n_bytes) {
+    void* p = nullptr;
+    if (!ready() || n_bytes == 0) return nullptr;
+    if (cudaMallocHost(&p, n_bytes) != cudaSuccess) { cudaGetLastError(); fail(ADAMAH_ERR_MEMORY, "host_alloc: %llu bytes", (unsigned long long)n_bytes); return nullptr; }
+    return p;
+}
+extern "C" void adam_b200_host_free(void* p) { if (p) cudaFreeHost(p); }
+
 extern "C" void adamah_sync(void) { if (g.inited) cudaStreamSynchronize(g.stream); }
 extern "C" void adamah_synchronize(uint64_t) { adamah_sync(); }
 extern "C" void adamah_synchronize_all(void) { adamah_sync(); }

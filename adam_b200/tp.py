@@ -303,6 +303,14 @@ class ADAMEngineTP(ADAMEngine):
         self.prefill(n - reuse)
         return [n] * len(prompts)
 
+    def _score(self, n, direct):
+        """Position by position: the collectives sit between the parts of a step."""
+        out = np.empty((n, self.cfg.n_vocab), np.float32)
+        for i in range(n):
+            self.step(1, lm_head=True, logits=True, direct=direct)
+            out[i] = self.read_logits(0)
+        return out
+
     def begin(self, prompts, reserve):
         super().begin(prompts, reserve)
         self._graphs = {k: g for k, g in self._graphs.items() if k[1] == self._batch}

@@ -369,6 +369,13 @@ int adam_b200_decoder_continue(uint32_t id, const int32_t* prompt_tokens, uint32
 int adam_b200_decoder_prefill(uint32_t id, uint32_t n_tokens);
 /* The same with a number of tokens of its own for every active sequence ([batch], 0 allowed). */
 int adam_b200_decoder_prefill_ragged(uint32_t id, const uint32_t* n_tokens);
+/* Soft-capped logits after each of the next n_tokens prompt tokens of the single active sequence, to the host buffer
+ * `out` ([n_tokens][n_vocab] float32): the positions run together, like a prompt's.  Leaves the decoder as n_tokens
+ * steps with logits would. */
+int adam_b200_decoder_score(uint32_t id, uint32_t n_tokens, float* out);
+/* Page-locked host memory, which copies from the device reach at full speed (NULL on failure). */
+void* adam_b200_host_alloc(uint64_t n_bytes);
+void adam_b200_host_free(void* p);
 /* The same step in parts, each enqueued directly on the stream, for callers that put their
  * own work between them (tensor parallelism).  Parts 2L / 2L+1 = attention half (embedding
  * for L = 0, QKV, attention, o-proj) / FFN half (gate+up, down) of layer L; then the LM head
