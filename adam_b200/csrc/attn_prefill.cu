@@ -115,6 +115,17 @@ __device__ __forceinline__ ApRow ap_row(const AttnPrefillArgs& a, const AttnTile
     return x;
 }
 
+// tanh(x) for soft-capped scores: where the whole warp is below 1/4 (scores below a quarter of the cap, nearly always) its
+// power series (the first term left out is 9e-9 of the value), else 1 - 2 / (1 + e^2x).
+__device__ __forceinline__ float ap_tanh_small(float x) {
+    const float y = x * x;
+    return fmaf(x * y, fmaf(y, fmaf(y, fmaf(y, 62.f / 2835.f, -17.f / 315.f), 2.f / 15.f), -1.f / 3.f), x);
+}
+__device__ __forceinline__ float ap_tanh(float x) {
+    const float d = 1.f + expf(fminf(2.f * x, 80.f));
+    return fabsf(x) < 0.25f ? ap_tanh_small(x) : 1.f - div_by(2.f, d, __frcp_rn(d));
+}
+
 // Online soft-max of one tile of scores (NT tiles of 8 positions from kv0): c becomes the probabilities, alpha the factor
 // of the rows' earlier sums.  Row h of this thread is rows g + 8 h of the warp.
 template <int NT>
@@ -123,13 +134,36 @@ __device__ __forceinline__ void ap_softmax(float (&c)[NT][4], const AttnPrefillA
     const int lane = threadIdx.x & 31, q = lane & 3;
     const float rcap = a.cap > 0.f ? __frcp_rn(a.cap) : 0.f;
     float mx[2] = {AP_NEG, AP_NEG};
+    if (a.cap > 0.f) {
+        float big = 0.f;
+        const float sx[2] = {scl[0] * rcap, scl[1] * rcap};
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { c[j][e] *= sx[e >> 1]; big = fmaxf(big, fabsf(c[j][e])); }
+        if (__all_sync(0xffffffffu, big < 0.25f)) {
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) c[j][e] = ap_tanh_small(c[j][e]) * a.cap;
+        } else {
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) c[j][e] = ap_tanh(c[j][e]) * a.cap;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) c[j][e] *= scl[e >> 1];
+    }
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int h = e >> 1, kp = kv0 + 8 * j + 2 * q + (e & 1);
-            float s = c[j][e] * scl[h];
-            if (a.cap > 0.f) s = tanhf(div_by(s, a.cap, rcap)) * a.cap;
+            float s = c[j][e];
             if (edge && (kp > pos[h] || (a.window > 0 && kp + (int)a.window <= pos[h]))) s = AP_NEG;
             c[j][e] = s;
             mx[h] = fmaxf(mx[h], s);
@@ -160,6 +194,7 @@ template <int HD, int NW>
 __global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_h(const AttnPrefillArgs a) {
     constexpr int ROWS = NW * 16, BN = 64, NCH = HD / 8, NTH = NW * 32;
     extern __shared__ __align__(128) uint8_t sm[];
+    __shared__ size_t s_row[2][BN];
     __half* sQh = reinterpret_cast<__half*>(sm);
     __half* sQl = sQh + ROWS * HD;
     const uint32_t qh_s = ap_smem(sQh), ql_s = ap_smem(sQl), k_s = ql_s + ROWS * HD * 2, v_s = k_s + BN * HD * 2;
@@ -173,15 +208,29 @@ __global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_h(const AttnPrefill
     auto sw = [](int r, int ch) { return NCH >= 8 ? ch ^ (r & 7) : ch ^ ((r >> 1) & (NCH - 1)); };
     const int kv_hi = t.pos + t.n_tok;                                                  // positions [.., kv_hi)
     const int kv_lo = a.window > 0 && t.pos + 1 > (int)a.window ? (t.pos + 1 - (int)a.window) / BN * BN : 0;
-    auto load = [&](uint32_t dst, uint32_t kv, int kv0) {
-        for (int i = tid; i < BN * NCH; i += NTH) {
-            const int r = i / NCH, ch = i % NCH, p = min(kv0 + r, kv_hi - 1);
+    // Where a tile's rows lie in the cache: looked up once per row and a tile ahead (a look-up per 16-byte copy, with its
+    // dependent load of the page table, made a tile take 12 us).
+    const size_t v_off = (size_t)a.geo.n_kv * a.geo.page * HD;                          // a value row lies this far behind its key row
+    auto locate = [&](int kv0) {
+        if (tid < BN) {
+            const int p = min(kv0 + tid, kv_hi - 1);
             const uint32_t pn = (uint32_t)p / a.geo.page;
             const int32_t page = pn < a.geo.max_pages ? max(bt[pn], 0) : 0;
-            ap_cp16(dst + (uint32_t)(r * HD + sw(r, ch) * 8) * 2u, pool + kv_index(a.geo, (uint32_t)page, a.layer, kv, kvh, (uint32_t)p % a.geo.page) + ch * 8);
+            s_row[(kv0 / BN) & 1][tid] = kv_index(a.geo, (uint32_t)page, a.layer, 0, kvh, (uint32_t)p % a.geo.page);
+        }
+    };
+    auto load = [&](uint32_t dst, uint32_t kv, int kv0) {
+        const __half* src = pool + (kv ? v_off : 0);
+        const size_t* rows = s_row[(kv0 / BN) & 1];
+#pragma unroll 8
+        for (int i = tid; i < BN * NCH; i += NTH) {
+            const int r = i / NCH, ch = i % NCH;
+            ap_cp16(dst + (uint32_t)(r * HD + sw(r, ch) * 8) * 2u, src + rows[r] + ch * 8);
         }
         ap_commit();
     };
+    locate(kv_lo);
+    __syncthreads();
     load(k_s, 0, kv_lo);
     load(v_s, 1, kv_lo);
     // this warp's query rows: power-of-two scale per row, two fp16 terms
@@ -242,6 +291,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_h(const AttnPrefill
         const bool work = live && kv0 <= p_hi && !(a.window > 0 && kv0 + BN - 1 + (int)a.window <= p_lo);
         const bool edge = kv0 + BN - 1 > p_lo || (a.window > 0 && kv0 + (int)a.window <= p_hi);
         float c[8][4], alpha[2] = {1.f, 1.f};
+        if (kv0 + BN < kv_hi) locate(kv0 + BN);
         ap_wait<1>();
         __syncthreads();
         if (work) {
@@ -330,6 +380,7 @@ template <int HD, int NW>
 __global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_f(const AttnPrefillArgs a) {
     constexpr int ROWS = NW * 16, BN = 32, LD = HD + 4, NTH = NW * 32;
     extern __shared__ __align__(128) uint8_t sm[];
+    __shared__ size_t s_row[2][BN];
     float *sQ = reinterpret_cast<float*>(sm), *sK = sQ + ROWS * LD, *sV = sK + BN * LD;
     const uint32_t k_s = ap_smem(sK), v_s = ap_smem(sV);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
@@ -341,15 +392,27 @@ __global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_f(const AttnPrefill
     const int32_t* bt = a.block_table + (size_t)t.seq * a.geo.max_pages;
     const int kv_hi = t.pos + t.n_tok;
     const int kv_lo = a.window > 0 && t.pos + 1 > (int)a.window ? (t.pos + 1 - (int)a.window) / BN * BN : 0;
-    auto load = [&](uint32_t dst, uint32_t kv, int kv0) {
-        for (int i = tid; i < BN * (HD / 4); i += NTH) {
-            const int r = i / (HD / 4), ch = i % (HD / 4), p = min(kv0 + r, kv_hi - 1);
+    const size_t v_off = (size_t)a.geo.n_kv * a.geo.page * HD;                          // see k_attn_prefill_h
+    auto locate = [&](int kv0) {
+        if (tid < BN) {
+            const int p = min(kv0 + tid, kv_hi - 1);
             const uint32_t pn = (uint32_t)p / a.geo.page;
             const int32_t page = pn < a.geo.max_pages ? max(bt[pn], 0) : 0;
-            ap_cp16(dst + (uint32_t)(r * LD + ch * 4) * 4u, pool + kv_index(a.geo, (uint32_t)page, a.layer, kv, kvh, (uint32_t)p % a.geo.page) + ch * 4);
+            s_row[(kv0 / BN) & 1][tid] = kv_index(a.geo, (uint32_t)page, a.layer, 0, kvh, (uint32_t)p % a.geo.page);
+        }
+    };
+    auto load = [&](uint32_t dst, uint32_t kv, int kv0) {
+        const float* src = pool + (kv ? v_off : 0);
+        const size_t* rows = s_row[(kv0 / BN) & 1];
+#pragma unroll 8
+        for (int i = tid; i < BN * (HD / 4); i += NTH) {
+            const int r = i / (HD / 4), ch = i % (HD / 4);
+            ap_cp16(dst + (uint32_t)(r * LD + ch * 4) * 4u, src + rows[r] + ch * 4);
         }
         ap_commit();
     };
+    locate(kv_lo);
+    __syncthreads();
     load(k_s, 0, kv_lo);
     load(v_s, 1, kv_lo);
 #pragma unroll 4
@@ -374,6 +437,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_f(const AttnPrefill
         const bool work = live && kv0 <= p_hi && !(a.window > 0 && kv0 + BN - 1 + (int)a.window <= p_lo);
         const bool edge = kv0 + BN - 1 > p_lo || (a.window > 0 && kv0 + (int)a.window <= p_hi);
         float c[4][4], alpha[2] = {1.f, 1.f};
+        if (kv0 + BN < kv_hi) locate(kv0 + BN);
         ap_wait<1>();
         __syncthreads();
         if (work) {

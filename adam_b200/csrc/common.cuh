@@ -189,17 +189,17 @@ __device__ __forceinline__ float block_max(float v, float* red) {
     return red[32];
 }
 
-// tanh-approximated GELU exactly as the reference's numpy decoder writes it
-// (tests/diagnostics/diag_inference.py:941-943).
+// x / (1 + e^-z), without the branches of the IEEE division (z >= -80 keeps the divisor finite).
+__device__ __forceinline__ float gated(float x, float z) {
+    const float d = 1.0f + expf(-fmaxf(z, -80.f));
+    return div_by(x, d, __frcp_rn(d));
+}
+// GELU in its tanh form (tests/diagnostics/diag_inference.py:941-943), 0.5 x (1 + tanh u), written as x / (1 + e^-2u): the
+// same function without tanhf's branches, and without the cancellation in 1 + tanh u for negative u.
 __device__ __forceinline__ float gelu_tanh(float x) {
     const float k = 0.7978845608028654f;        // float32(sqrt(2/pi))
-    float x3 = x * x * x;
-    float inner = k * (x + 0.044715f * x3);
-    return 0.5f * x * (1.0f + tanhf(inner));
+    return gated(x, 2.0f * (k * (x + 0.044715f * (x * x * x))));
 }
-__device__ __forceinline__ float silu_clip(float x) {
-    float c = fminf(fmaxf(x, -80.f), 80.f);     // diag_inference.py:945-946
-    return x * (1.0f / (1.0f + expf(-c)));
-}
+__device__ __forceinline__ float silu_clip(float x) { return gated(x, fminf(fmaxf(x, -80.f), 80.f)); }      // diag_inference.py:945-946
 
 }  // namespace ab

@@ -347,8 +347,9 @@ template <int WT, int NT> struct TcGeo {
     static constexpr int QB = WT == WT_Q8_0 ? 64 : 32;                       // bytes of a row's codes per step
     static constexpr int SLOT = 32 * QB + (WT == WT_Q4_K ? 512 : 128);       // 32 rows: codes, then block scales / superblock headers
     static constexpr int BSTEP = NT * 256;                                   // both planes of one step
-    static constexpr int RING = NS * SP * BSTEP, XCH = RING + GROUPS * 4 * R * SLOT;     // offsets: weight rings, gate / up exchange (4 KB)
-    static constexpr int SMEM_USED = XCH + 4096 + 1024;
+    static constexpr int RING = NS * SP * BSTEP, XCH = RING + GROUPS * 4 * R * SLOT;     // offsets: weight rings, gate / up exchange
+    static constexpr int XCOLS = NT < 32 ? NT : 32;                          // columns exchanged at a time
+    static constexpr int SMEM_USED = XCH + (WT == WT_Q8_0 ? 0 : XCOLS * 512) + 1024;
     static constexpr int SMEM = SMEM_USED > TC_SMEM_MIN ? SMEM_USED : TC_SMEM_MIN;
     static_assert(SMEM <= 226 * 1024 && 2 * NT + 64 * NS * SP <= 512 && GROUPS % SP == 0 && GROUPS <= NS * SP, "shared or tensor memory");
     static_assert(REG_LOW + REG_READ + GROUPS * REG_MAKE <= 65536 / THREADS / 8 * 8 * (2 + GROUPS), "registers");
@@ -613,31 +614,34 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                     }
                 }
             }
-            const int n_out = PAIR ? tn * 64 + (row & 63) : tn * 128 + row, n_col = min(NT, a.B - m0);
-            float* yp = a.y + (size_t)m0 * a.ldy + n_out;
-            float inv[(NT + 31) / 32];                  // lane l of part i: column 32 i + l
-#pragma unroll
-            for (int i = 0; i < (NT + 31) / 32; ++i) inv[i] = 32 * i + lane < n_col ? a.inv[m0 + 32 * i + lane] : 0.f;
+            const int n_col = min(NT, a.B - m0);
             if constexpr (PAIR) {
-                // gate lanes (quarters 0, 1) and up lanes (2, 3) of a row swap half of their columns, eight at a time, through
-                // shared memory; gate lanes finish the first half of the columns
-                constexpr int H = NT / 2;
-                const bool up = row >= 64;
+                // gate (lanes 0..63) and up rows meet in shared memory, XCOLS columns at a time, and all lanes share the outputs.
+                // A rolled loop: unrolled over the columns, the activations' code did not fit the instruction cache (264 us
+                // instead of 88 for 1024 rows of 2 x 6912 x 1152 Q4_0).
+                constexpr int XC = G::XCOLS;
+                const int r = row & 63, n = tn * 64 + r;
+                float* yp = a.y + (size_t)m0 * a.ldy + n;
 #pragma unroll
-                for (int h0 = 0; h0 < H; h0 += 8) {
+                for (int h0 = 0; h0 < NT; h0 += XC) {
+                    if (h0 >= n_col) break;
+                    const float inv = h0 + lane < n_col ? a.inv[m0 + h0 + lane] : 0.f;         // lane c: column h0 + c
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) xch[c * 128 + row] = up ? acc[h0 + c] : acc[H + h0 + c];
+                    for (int c = 0; c < XC; ++c) xch[c * 128 + row] = acc[h0 + c] * __shfl_sync(0xffffffffu, inv, c);
                     asm volatile("bar.sync 1, 128;" ::: "memory");
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const int cg = h0 + c, cu = H + h0 + c, col = up ? cu : cg;
-                        const float sg = __shfl_sync(0xffffffffu, inv[cg / 32], cg & 31), su = __shfl_sync(0xffffffffu, inv[cu / 32], cu & 31), sc = up ? su : sg;
-                        const float o = xch[c * 128 + (row ^ 64)], m = up ? acc[cu] : acc[cg];
-                        if (col < n_col && n_out < a.N) yp[(size_t)col * a.ldy] = up ? act(o * sc, m * sc) : act(m * sc, o * sc);
+#pragma unroll 4
+                    for (int c = row >> 6; c < XC; c += 2) {
+                        const float v = act(xch[c * 128 + r], xch[c * 128 + 64 + r]);
+                        if (h0 + c < n_col && n < a.N) yp[(size_t)(h0 + c) * a.ldy] = v;
                     }
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                 }
             } else {
+                const int n_out = tn * 128 + row;
+                float* yp = a.y + (size_t)m0 * a.ldy + n_out;
+                float inv[(NT + 31) / 32];              // lane l of part i: column 32 i + l
+#pragma unroll
+                for (int i = 0; i < (NT + 31) / 32; ++i) inv[i] = 32 * i + lane < n_col ? a.inv[m0 + 32 * i + lane] : 0.f;
 #pragma unroll
                 for (int c = 0; c < NT; ++c) {
                     const float v = acc[c] * __shfl_sync(0xffffffffu, inv[c / 32], c & 31);
