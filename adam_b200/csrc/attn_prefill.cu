@@ -123,7 +123,7 @@ __device__ __forceinline__ float ap_tanh_small(float x) {
 }
 __device__ __forceinline__ float ap_tanh(float x) {
     const float d = 1.f + expf(fminf(2.f * x, 80.f));
-    return fabsf(x) < 0.25f ? ap_tanh_small(x) : 1.f - div_by(2.f, d, __frcp_rn(d));
+    return fabsf(x) < 0.25f ? ap_tanh_small(x) : 1.f - div_by(2.f, d, rcp_newton(d));
 }
 
 // Online soft-max of one tile of scores (NT tiles of 8 positions from kv0): c becomes the probabilities, alpha the factor

@@ -189,17 +189,23 @@ __device__ __forceinline__ float block_max(float v, float* red) {
     return red[32];
 }
 
-// x / (1 + e^-z), without the branches of the IEEE division (z >= -80 keeps the divisor finite).
+// 1 / d for a normal d whose reciprocal is normal too: the approximation and one Newton step (no branches, unlike the
+// correctly rounded reciprocal; a quotient formed with it by div_by is within an ulp).
+__device__ __forceinline__ float rcp_newton(float d) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return fmaf(r, fmaf(-d, r, 1.0f), r);
+}
+// x / (1 + e^-z), without branches (z >= -80 keeps the divisor finite).
 __device__ __forceinline__ float gated(float x, float z) {
     const float d = 1.0f + expf(-fmaxf(z, -80.f));
-    return div_by(x, d, __frcp_rn(d));
+    return div_by(x, d, rcp_newton(d));
 }
 // GELU in its tanh form (tests/diagnostics/diag_inference.py:941-943), 0.5 x (1 + tanh u), written as x / (1 + e^-2u): the
 // same function without tanhf's branches, and without the cancellation in 1 + tanh u for negative u.
-__device__ __forceinline__ float gelu_tanh(float x) {
-    const float k = 0.7978845608028654f;        // float32(sqrt(2/pi))
-    return gated(x, 2.0f * (k * (x + 0.044715f * (x * x * x))));
-}
-__device__ __forceinline__ float silu_clip(float x) { return gated(x, fminf(fmaxf(x, -80.f), 80.f)); }      // diag_inference.py:945-946
+__device__ __forceinline__ float gelu_arg(float x) { return 2.0f * (0.7978845608028654f * (x + 0.044715f * (x * x * x))); }   // float32(sqrt(2/pi))
+__device__ __forceinline__ float silu_arg(float x) { return fminf(fmaxf(x, -80.f), 80.f); }      // diag_inference.py:945-946
+__device__ __forceinline__ float gelu_tanh(float x) { return gated(x, gelu_arg(x)); }
+__device__ __forceinline__ float silu_clip(float x) { return gated(x, silu_arg(x)); }
 
 }  // namespace ab

@@ -323,6 +323,10 @@ __device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, u
 //                time, not 2, but the adding up costs 2 to 5 us.  Or, where the tiles alone leave SMs idle, clusters of S
 //                CTAs that take a part of K each, leave their sums in their own shared memory and add each other's columns
 //                through distributed shared memory, again in the order of K: results do not depend on timing.
+//   code size    Every launch finds the instruction cache cold, and fetching code costs about 12 cycles per instruction executed
+//                for the first time: with every loop unrolled and an instance per kind of result, 6000 to 15000 of a layer's
+//                15000 to 25000 cycles.  So stored and gate/up products share an instance (the flag is uniform), and
+//                loops whose registers allow it are rolled.
 // The request for shared memory is at least 120 KB, so that an SM never holds two of these CTAs: one that waits for
 // tensor memory held by a cluster that waits for it would never end.
 constexpr int TC_SMEM_MIN = 120 * 1024;
@@ -331,14 +335,14 @@ struct TcGemm {
     WeightRef w0, w1;
     float* y; int ldy;
     const uint8_t* img; const float* inv; uint32_t* err;
-    int N, units, B, swiglu;                            // units = K / 32
+    int N, units, B;                                    // units = K / 32
+    int pair, swiglu;                                   // gate / up tiles, and which activation
     int n_min, n_main, tiles_n, items;                  // items = tiles_n (weight tiles) * tiles of NT rows
     int S, period, shared;                              // K splits; stages per accumulation period; whether CTAs share tiles
     float* part; unsigned int* tickets;                 // shared tiles: per CTA the sums of its first and last one; arrivals, by the CTA in which a tile begins
     unsigned long long* best; unsigned int* ticket;     // arg-max: one key per activation row (0 between launches), CTAs that are done
     int* out_tok; float *out_val, *out_tok_f32, softcap;
 };
-enum { TC_STORE = 0, TC_PAIR = 1, TC_ARGMAX = 2 };       // what becomes of a product: stored, gate/up pairs, arg-max per activation row (and stored)
 template <int WT, int NT> struct TcGeo {
     static constexpr int SP = NT == 128 ? 1 : 2, NS = NT == 128 ? 4 : 2;     // steps per stage, stages
     static constexpr int GROUPS = NT == 128 ? 3 : 4, THREADS = (2 + GROUPS) * 128;     // warpgroups that rebuild weights, a step each in turn
@@ -347,9 +351,9 @@ template <int WT, int NT> struct TcGeo {
     static constexpr int QB = WT == WT_Q8_0 ? 64 : 32;                       // bytes of a row's codes per step
     static constexpr int SLOT = 32 * QB + (WT == WT_Q4_K ? 512 : 128);       // 32 rows: codes, then block scales / superblock headers
     static constexpr int BSTEP = NT * 256;                                   // both planes of one step
-    static constexpr int RING = NS * SP * BSTEP, XCH = RING + GROUPS * 4 * R * SLOT;     // offsets: weight rings, gate / up exchange
-    static constexpr int XCOLS = NT < 32 ? NT : 32;                          // columns exchanged at a time
-    static constexpr int SMEM_USED = XCH + (WT == WT_Q8_0 ? 0 : XCOLS * 512) + 1024;
+    static constexpr int RING = NS * SP * BSTEP, XCH = RING + GROUPS * 4 * R * SLOT;     // offsets: weight rings, columns of results on their way out
+    static constexpr int XCOLS = NT < 32 ? NT : 32;                          // so many columns at a time
+    static constexpr int SMEM_USED = XCH + XCOLS * 512 + 1024;
     static constexpr int SMEM = SMEM_USED > TC_SMEM_MIN ? SMEM_USED : TC_SMEM_MIN;
     static_assert(SMEM <= 226 * 1024 && 2 * NT + 64 * NS * SP <= 512 && GROUPS % SP == 0 && GROUPS <= NS * SP, "shared or tensor memory");
     static_assert(REG_LOW + REG_READ + GROUPS * REG_MAKE <= 65536 / THREADS / 8 * 8 * (2 + GROUPS), "registers");
@@ -362,17 +366,19 @@ __device__ __forceinline__ bool elect_one() {
 template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(N)); }
 template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(N)); }
 template <int N, int HAVE> __device__ __forceinline__ void reg_set() { if constexpr (N > HAVE) reg_inc<N>(); else if constexpr (N < HAVE) reg_dec<N>(); }
-template <int WT, int NT, int MODE>
+template <int WT, int NT, bool HEAD>
 __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcGemm a) {
     using G = TcGeo<WT, NT>;
-    constexpr bool PAIR = MODE == TC_PAIR;
+    const bool pair = !HEAD && WT != WT_Q8_0 && a.pair != 0;
     constexpr int SP = G::SP, NS = G::NS;
     extern __shared__ __align__(1024) uint8_t sm_raw[];
     uint8_t* sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);     // the swizzle works on address bits
     uint8_t* smB = sm;
     __shared__ __align__(8) uint64_t full[NS], empty[NS], d_full, d_empty;
     __shared__ uint32_t s_tmem;
-    [[maybe_unused]] __shared__ bool s_last;
+    __shared__ bool s_last;
+    __shared__ float s_inv[NT];
+    [[maybe_unused]] __shared__ unsigned long long s_best[HEAD ? NT : 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = warp >> 2;
     const int S = a.S, split = S > 1 ? (int)(blockIdx.x % (uint32_t)S) : 0;     // a cluster's CTAs are neighbours along x
     // this split's share of the steps: first those of the block minima, then those of the products
@@ -407,7 +413,7 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
     };
     const int row = (warp & 3) * 32 + lane;             // this lane's TMEM lane
     const uint32_t tlane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    auto act = [&](float gate, float up) { return (a.swiglu ? silu_clip(gate) : gelu_tanh(gate)) * up; };
+    auto act = [&](float gate, float up) { return gated(gate, a.swiglu ? silu_arg(gate) : gelu_arg(gate)) * up; };     // no branch
     // The end of a split item: the cluster's sums lie in the exchange; every CTA finishes the columns c = split, split + S, ...
     auto finish_split = [&]() {
         cl_arrive();
@@ -422,13 +428,15 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
             return v;
         };
         const int item = item_of(0), tn = n_of(item), m0 = m_of(item), n_col = min(NT, a.B - m0);
-        const int n_out = PAIR ? tn * 64 + (row & 63) : tn * 128 + row;
+        const int r = pair ? row & 63 : row, n_out = pair ? tn * 64 + r : tn * 128 + r;
         float* yp = a.y + (size_t)m0 * a.ldy + n_out;
-        constexpr int LANES = PAIR ? 2 : 1;             // a pair's 64 rows: each half of the lanes takes its own columns
-        for (int c = split + S * ((wg - 1) * LANES + (PAIR ? row >> 6 : 0)); c < n_col; c += (G::GROUPS + 1) * LANES * S) {
-            const float sc = a.inv[m0 + c], v = total_of(c, PAIR ? row & 63 : row);
-            if constexpr (PAIR) { const float u = total_of(c, 64 + (row & 63)); if (n_out < a.N) yp[(size_t)c * a.ldy] = act(v * sc, u * sc); }
-            else if (n_out < a.N) yp[(size_t)c * a.ldy] = v * sc;
+        const int lanes = pair ? 2 : 1;                 // a pair's 64 rows: each half of the lanes takes its own columns
+#pragma unroll 1
+        for (int c = split + S * ((wg - 1) * lanes + (pair ? row >> 6 : 0)); c < n_col; c += (G::GROUPS + 1) * lanes * S) {
+            const float sc = a.inv[m0 + c];
+            float v = total_of(c, r) * sc;
+            if (pair) v = act(v, total_of(c, 64 + r) * sc);
+            if (n_out < a.N) yp[(size_t)c * a.ldy] = v;
         }
         cl_arrive();
         cl_wait();
@@ -523,15 +531,19 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
         // ---- results: D1 (and, with an item's last period, D2) into registers; an item's end: scale back, activation, store ----
         reg_inc<G::REG_READ>();
         pdl_wait();
-        [[maybe_unused]] float* xch = reinterpret_cast<float*>(sm + G::XCH);
+        float* xch = reinterpret_cast<float*>(sm + G::XCH);
         uint32_t par = 0;
-        [[maybe_unused]] unsigned long long best[(NT + 31) / 32] = {};
+        if constexpr (HEAD) {
+            if (tid - 128 < NT) s_best[tid - 128] = 0;
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+        }
         [[maybe_unused]] auto flush_best = [&](int m0) {
-#pragma unroll
-            for (int i = 0; i < (NT + 31) / 32; ++i) {
-                if (32 * i + lane < min(NT, a.B - m0) && best[i]) atomicMax(a.best + m0 + 32 * i + lane, best[i]);
-                best[i] = 0;
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (const int c = tid - 128; c < min(NT, a.B - m0)) {
+                if (s_best[c]) atomicMax(a.best + m0 + c, s_best[c]);
+                s_best[c] = 0;
             }
+            asm volatile("bar.sync 1, 128;" ::: "memory");
         };
         for (int q = q0; q < q1;) {
             const int i0 = q / spi, j0 = q - i0 * spi, j1 = min(spi, j0 + q1 - q), item = item_of(i0), tn = n_of(item), m0 = m_of(item);
@@ -557,8 +569,8 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                         for (int c = 0; c < CH; ++c) acc[ch + c] += v[c / 16][c % 16];
                     }
                 };
-                take(tlane);
-                if (p == np - 1) take(tlane + NT);
+#pragma unroll 1
+                for (int h = 0; h < (p == np - 1 ? 2 : 1); ++h) take(tlane + h * NT);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&d_empty);
@@ -614,54 +626,51 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                     }
                 }
             }
+            // Out through shared memory, XC columns at a time, by rolled loops.
+            constexpr int XC = G::XCOLS;
             const int n_col = min(NT, a.B - m0);
-            if constexpr (PAIR) {
-                // gate (lanes 0..63) and up rows meet in shared memory, XCOLS columns at a time, and all lanes share the outputs.
-                // A rolled loop: unrolled over the columns, the activations' code did not fit the instruction cache (264 us
-                // instead of 88 for 1024 rows of 2 x 6912 x 1152 Q4_0).
-                constexpr int XC = G::XCOLS;
-                const int r = row & 63, n = tn * 64 + r;
-                float* yp = a.y + (size_t)m0 * a.ldy + n;
+            const int r = pair ? row & 63 : row, n = pair ? tn * 64 + r : tn * 128 + r;
+            float* yp = a.y + (size_t)m0 * a.ldy + n;
+            if (tid - 128 < n_col) s_inv[tid - 128] = a.inv[m0 + tid - 128];
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+#pragma unroll 1
+            for (int h0 = 0; h0 < n_col; h0 += XC) {
+                const int m = min(XC, n_col - h0);
 #pragma unroll
-                for (int h0 = 0; h0 < NT; h0 += XC) {
-                    if (h0 >= n_col) break;
-                    const float inv = h0 + lane < n_col ? a.inv[m0 + h0 + lane] : 0.f;         // lane c: column h0 + c
-#pragma unroll
-                    for (int c = 0; c < XC; ++c) xch[c * 128 + row] = acc[h0 + c] * __shfl_sync(0xffffffffu, inv, c);
+                for (int c = 0; c < XC; ++c) xch[c * 128 + row] = acc[c];
+                if (pair) {                             // gate (lanes 0..63) and up rows meet; all lanes share the outputs
                     asm volatile("bar.sync 1, 128;" ::: "memory");
 #pragma unroll 4
-                    for (int c = row >> 6; c < XC; c += 2) {
-                        const float v = act(xch[c * 128 + r], xch[c * 128 + 64 + r]);
-                        if (h0 + c < n_col && n < a.N) yp[(size_t)(h0 + c) * a.ldy] = v;
+                    for (int c = row >> 6; c < m; c += 2) {
+                        const float sc = s_inv[h0 + c], v = act(xch[c * 128 + r] * sc, xch[c * 128 + 64 + r] * sc);
+                        if (n < a.N) yp[(size_t)(h0 + c) * a.ldy] = v;
                     }
                     asm volatile("bar.sync 1, 128;" ::: "memory");
-                }
-            } else {
-                const int n_out = tn * 128 + row;
-                float* yp = a.y + (size_t)m0 * a.ldy + n_out;
-                float inv[(NT + 31) / 32];              // lane l of part i: column 32 i + l
-#pragma unroll
-                for (int i = 0; i < (NT + 31) / 32; ++i) inv[i] = 32 * i + lane < n_col ? a.inv[m0 + 32 * i + lane] : 0.f;
-#pragma unroll
-                for (int c = 0; c < NT; ++c) {
-                    const float v = acc[c] * __shfl_sync(0xffffffffu, inv[c / 32], c & 31);
-                    if constexpr (MODE == TC_ARGMAX) {
-                        // best of the warp's rows: NaN counts as -FLT_MAX, ties go to the lower row; lane c % 32 keeps column c's
-                        const float f = (v == v ? v : -3.402823466e+38f) + 0.f;
-                        const uint32_t bits = __float_as_uint(f), ord = n_out < a.N ? bits ^ ((uint32_t)((int)bits >> 31) | 0x80000000u) : 0u;
+                } else if constexpr (HEAD) {
+                    // best of the warp's rows per column: NaN counts as -FLT_MAX, ties go to the lower row
+                    unsigned long long mine = 0;        // lane c: column h0 + c
+#pragma unroll 2
+                    for (int c = 0; c < m; ++c) {
+                        const float v = xch[c * 128 + row] * s_inv[h0 + c], f = (v == v ? v : -3.402823466e+38f) + 0.f;
+                        const uint32_t bits = __float_as_uint(f), ord = n < a.N ? bits ^ ((uint32_t)((int)bits >> 31) | 0x80000000u) : 0u;
                         const uint32_t top = __reduce_max_sync(0xffffffffu, ord);
-                        const uint32_t at = __reduce_min_sync(0xffffffffu, ord == top ? (uint32_t)n_out : 0xffffffffu);
-                        const unsigned long long key = ((unsigned long long)top << 32) | (0xffffffffu - at);
-                        if (lane == (c & 31) && key > best[c / 32]) best[c / 32] = key;
-                        if (a.y && c < n_col && n_out < a.N) yp[(size_t)c * a.ldy] = a.softcap > 0.f ? tanhf(v / a.softcap) * a.softcap : v;
-                    } else if (c < n_col && n_out < a.N) yp[(size_t)c * a.ldy] = v;
+                        const uint32_t at = __reduce_min_sync(0xffffffffu, ord == top ? (uint32_t)n : 0xffffffffu);
+                        if (lane == c) mine = ((unsigned long long)top << 32) | (0xffffffffu - at);
+                        if (a.y && n < a.N) yp[(size_t)(h0 + c) * a.ldy] = a.softcap > 0.f ? tanhf(v / a.softcap) * a.softcap : v;
+                    }
+                    if (lane < m) atomicMax(&s_best[h0 + lane], mine);
+                } else if (n < a.N) {
+#pragma unroll 4
+                    for (int c = 0; c < m; ++c) yp[(size_t)(h0 + c) * a.ldy] = xch[c * 128 + row] * s_inv[h0 + c];
                 }
-                if constexpr (MODE == TC_ARGMAX)
-                    if (a.B > NT) flush_best(m0);          // the columns change with the next item
+#pragma unroll
+                for (int c = 0; c < NT - XC; ++c) acc[c] = acc[c + XC];
             }
+            if constexpr (HEAD) { if (a.B > NT) flush_best(m0); }       // the columns change with the next item
+            asm volatile("bar.sync 1, 128;" ::: "memory");              // s_inv is free again
         }
         if (S > 1) finish_split();
-        if constexpr (MODE == TC_ARGMAX) {              // the last CTA to end decodes the winners and clears the keys
+        if constexpr (HEAD) {                           // the last CTA to end decodes the winners and clears the keys
             flush_best(0);
             __threadfence();
             asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -691,9 +700,9 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
         const int sub = grp % SP;
         uint8_t* ring = sm + G::RING + (warp - 8) * G::R * G::SLOT;
         const uint32_t ring_s = smem_u32(ring);
-        const WeightRef w = (PAIR && quarter >= 2) ? a.w1 : a.w0;                      // lanes 64..127 of a pair: up rows
+        const WeightRef w = (pair && quarter >= 2) ? a.w1 : a.w0;                      // lanes 64..127 of a pair: up rows
         const bool scales_async = WT == WT_Q4_K || ((a.units & 1) == 0 && ((uintptr_t)w.d & 3) == 0);
-        auto row_of = [&](int tn, int r) { return min(PAIR ? tn * 64 + (r & 63) : tn * 128 + r, a.N - 1); };
+        auto row_of = [&](int tn, int r) { return min(pair ? tn * 64 + (r & 63) : tn * 128 + r, a.N - 1); };
         const int rpu = WT == WT_Q4_0 ? a.units : WT == WT_Q8_0 ? 2 * a.units : (a.units >> 3) * 9;     // uint4 per weight row
         struct Cursor { int q, i, j; };                 // stage: of the range, item of the range and stage of the item
         constexpr int HOP = G::GROUPS / SP;
@@ -733,130 +742,132 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
             if (++f_n == (uint32_t)G::R) f_n = 0;
             cp_commit();
         };
-        for (int j = 0; j < G::R; ++j) fetch();
         uint32_t at = 0;                                // weight ring slot
         bool waited = false;
-        for (Cursor c = {q_first, q_first / spi, q_first % spi}; c.q < q1; next(c)) {
+        Cursor c = {q_first, q_first / spi, q_first % spi};
+        // One copy of the loop body serves the start too: R - 1 fetches before the first tile is taken.
+#pragma unroll 1
+        for (int turn = 0; c.q < q1; ++turn) {
+            fetch();
+            if (turn < G::R - 1) continue;
             const int st = c.j * SP + sub, ks = ma0 + st - nmn;
             const uint32_t nth = (uint32_t)(c.q - q0), stage = nth % NS, acol = tlane + A_COL + (stage * SP + sub) * 64u;
             cp_wait<G::R - 1>();
             __syncwarp();
             const uint8_t* slot = ring + at * G::SLOT;
-            uint32_t qw[G::QB / 4];                     // this row's codes of the step
-#pragma unroll
-            for (int p = 0; p < LPR; ++p) {
-                const uint4 v = *reinterpret_cast<const uint4*>(slot + lane * G::QB + ((LPR == 2 ? p ^ ((lane >> 2) & 1) : p ^ ((lane >> 1) & 3)) << 4));
-                qw[4 * p] = v.x; qw[4 * p + 1] = v.y; qw[4 * p + 2] = v.z; qw[4 * p + 3] = v.w;
-            }
-            uint32_t d01 = 0; uint4 hdr = make_uint4(0, 0, 0, 0);
-            if constexpr (WT != WT_Q4_K) d01 = *reinterpret_cast<const uint32_t*>(slot + 32 * G::QB + lane * 4);
-            else hdr = *reinterpret_cast<const uint4*>(slot + 32 * G::QB + lane * 16);
+            const uint8_t* codes = slot + lane * G::QB;
+            auto piece_at = [&](int p) { return *reinterpret_cast<const uint4*>(codes + ((LPR == 2 ? p ^ ((lane >> 2) & 1) : p ^ ((lane >> 1) & 3)) << 4)); };
             if (!waited) { pdl_wait(); waited = true; } // no bounded wait below spans an earlier kernel
             if (nth >= (uint32_t)NS) {                  // the tensor core is done with what the slot held
                 wait_on(&empty[stage], (nth / NS - 1u) & 1u);
                 tc_fence_after();
             }
-            if (st < nst) {
+            if (WT == WT_Q4_K ? st >= nmn && st < nst : st < nst) {
+                uint32_t d01 = 0, sp = 0;               // two block scales; or a superblock's, and two sub-blocks' factors
                 if constexpr (WT != WT_Q4_K) {
-                    if (!scales_async) {                // odd number of blocks per row: their scales are not pairs of aligned halves
+                    if (scales_async) d01 = *reinterpret_cast<const uint32_t*>(slot + 32 * G::QB + lane * 4);
+                    else {                              // odd number of blocks per row: their scales are not pairs of aligned halves
                         const unsigned short* dp = reinterpret_cast<const unsigned short*>(w.d) + (size_t)row_of(n_of(item_of(c.i)), row) * a.units + 2 * ks;
                         d01 = (uint32_t)dp[0] | (2 * ks + 1 < a.units ? (uint32_t)dp[1] << 16 : 0u);
                     }
+                } else {
+                    const uint4 hdr = *reinterpret_cast<const uint4*>(slot + 32 * G::QB + lane * 16);
+                    uint32_t mp;
+                    q4k_codes(hdr, ks & 3, sp, mp);
+                    d01 = (hdr.x & 0xFFFFu) * 0x10001u;
+                }
+#pragma unroll (NT == 128 ? 2 : 1)
+                for (int b = 0; b < 2; ++b) {           // 32 values of K: columns 16 b .. of w_hi and of w_lo
+                    const uint32_t col = acol + b * 16u;
+                    uint32_t whi[8], wlo[8], v[2];
+                    if constexpr (WT == WT_Q8_0) {      // bytes + 128 into the mantissa of 1024, two at a time
+                        const __half2 d = as_h2((d01 >> (16 * b) & 0xFFFFu) * 0x10001u);
 #pragma unroll
-                    for (int b = 0; b < 2; ++b) {       // columns 16 b ..: values 0..15 of the block from the low nibbles, 16..31 from the high ones
-                        const __half2 d = as_h2((b ? d01 >> 16 : d01 & 0xFFFFu) * 0x10001u);
-                        uint32_t whi[8], wlo[8], v[2];
-                        if constexpr (WT == WT_Q8_0) {  // bytes + 128 into the mantissa of 1024, two at a time
+                        for (int y = 0; y < 2; ++y) {
+                            const uint4 p4 = piece_at(2 * b + y);
+                            const uint32_t qw[4] = {p4.x, p4.y, p4.z, p4.w};
 #pragma unroll
-                            for (int y = 0; y < 2; ++y) {
+                            for (int x = 0; x < 4; ++x) {
+                                const uint32_t u = qw[x] ^ 0x80808080u;
+                                v[0] = (u & 0x00FF00FFu) | 0x64006400u; v[1] = ((u >> 8) & 0x00FF00FFu) | 0x64006400u;
 #pragma unroll
-                                for (int x = 0; x < 4; ++x) {
-                                    const uint32_t u = qw[8 * b + 4 * y + x] ^ 0x80808080u;
-                                    v[0] = (u & 0x00FF00FFu) | 0x64006400u; v[1] = ((u >> 8) & 0x00FF00FFu) | 0x64006400u;
-#pragma unroll
-                                    for (int p = 0; p < 2; ++p) split_h2(__hadd2(as_h2(v[p]), __float2half2_rn(-1152.f)), d, whi[2 * x + p], wlo[2 * x + p]);
-                                }
-                                tc_st8(acol + b * 16u + y * 8u, whi);
-                                tc_st8(acol + 32u + b * 16u + y * 8u, wlo);
+                                for (int p = 0; p < 2; ++p) split_h2(__hadd2(as_h2(v[p]), __float2half2_rn(-1152.f)), d, whi[2 * x + p], wlo[2 * x + p]);
                             }
-                            continue;
+                            tc_st8(col + y * 8u, whi);
+                            tc_st8(col + 32u + y * 8u, wlo);
                         }
+                    } else if constexpr (WT == WT_Q4_0) {       // block b: values 0..15 in the low nibbles, 16..31 in the high ones
+                        const __half2 d = as_h2((d01 >> (16 * b) & 0xFFFFu) * 0x10001u);
+                        const uint4 p4 = piece_at(b);
+                        const uint32_t qw[4] = {p4.x, p4.y, p4.z, p4.w};
 #pragma unroll
                         for (int x = 0; x < 4; ++x) {
-                            nib_pairs<false>(qw[4 * b + x], v);
+                            nib_pairs<false>(qw[x], v);
 #pragma unroll
                             for (int p = 0; p < 2; ++p) split_h2(__hadd2(as_h2(v[p]), __float2half2_rn(-1032.f)), d, whi[2 * x + p], wlo[2 * x + p]);
                         }
-                        tc_st8(acol + b * 16u, whi);
-                        tc_st8(acol + 32u + b * 16u, wlo);
+                        tc_st8(col, whi);
+                        tc_st8(col + 32u, wlo);
 #pragma unroll
                         for (int x = 0; x < 4; ++x) {
-                            nib_pairs<true>(qw[4 * b + x], v);
+                            nib_pairs<true>(qw[x], v);
 #pragma unroll
                             for (int p = 0; p < 2; ++p) split_h2(__hfma2(as_h2(v[p]), __float2half2_rn(0.0625f), __float2half2_rn(-72.f)), d, whi[2 * x + p], wlo[2 * x + p]);
                         }
-                        tc_st8(acol + 8u + b * 16u, whi);
-                        tc_st8(acol + 40u + b * 16u, wlo);
-                    }
-                } else if (st >= nmn) {
-                    uint32_t sp, mp;
-                    q4k_codes(hdr, ks & 3, sp, mp);
-                    const __half2 d = as_h2((hdr.x & 0xFFFFu) * 0x10001u);
-#pragma unroll
-                    for (int b = 0; b < 2; ++b) {       // low nibbles = sub-block 2g, high nibbles = sub-block 2g + 1
-                        const uint32_t code = b ? sp >> 8 : sp & 0xFFu;
-                        const __half2 sc = __hsub2(as_h2((code * 0x10001u) | 0x64006400u), __float2half2_rn(1024.f));
-                        const __half2 mul = b ? __hmul2(sc, __float2half2_rn(0.0625f)) : sc;
-                        const __half2 off = __hmul2(sc, __float2half2_rn(b ? -64.f : -1024.f));
+                        tc_st8(col + 8u, whi);
+                        tc_st8(col + 40u, wlo);
+                    } else {                            // low nibbles = sub-block 2g, high nibbles = sub-block 2g + 1
+                        const uint32_t code = sp >> (8 * b) & 0xFFu;
+                        const __half2 sc = __hsub2(as_h2((code * 0x10001u) | 0x64006400u), __float2half2_rn(1024.f)), off = __hmul2(sc, __float2half2_rn(-1024.f));
 #pragma unroll
                         for (int y = 0; y < 2; ++y) {
-                            uint32_t whi[8], wlo[8], v[2];
+                            const uint4 p4 = piece_at(y);
+                            const uint32_t qw[4] = {p4.x >> (4 * b), p4.y >> (4 * b), p4.z >> (4 * b), p4.w >> (4 * b)};
 #pragma unroll
                             for (int x = 0; x < 4; ++x) {
-                                if (b) nib_pairs<true>(qw[4 * y + x], v); else nib_pairs<false>(qw[4 * y + x], v);
+                                nib_pairs<false>(qw[x], v);
 #pragma unroll
                                 for (int p = 0; p < 2; ++p)       // sc * q, an integer below 946, exactly
-                                    split_h2(__hfma2(as_h2(v[p]), mul, off), d, whi[2 * x + p], wlo[2 * x + p]);
+                                    split_h2(__hfma2(as_h2(v[p]), sc, off), as_h2(d01), whi[2 * x + p], wlo[2 * x + p]);
                             }
-                            tc_st8(acol + b * 16u + y * 8u, whi);
-                            tc_st8(acol + 32u + b * 16u + y * 8u, wlo);
+                            tc_st8(col + y * 8u, whi);
+                            tc_st8(col + 32u + y * 8u, wlo);
                         }
-                    }
-                } else {
-                    // a step of block minima: -32 dmin m of 64 sub-blocks (the image holds the sums over 32 activations / 32)
-                    const int sb0 = (mn0 + st) * 8, n_sb = a.units >> 3;
-                    const uint4* src = w.q + (size_t)row_of(n_of(item_of(c.i)), row) * rpu;
-#pragma unroll 1
-                    for (int b = 0; b < 4; ++b) {
-                        uint32_t whi[8], wlo[8];
-#pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            const int sb = sb0 + 2 * b + e;
-                            const uint4 h = __ldg(src + (size_t)min(sb, n_sb - 1) * 9);
-                            const float dm = sb < n_sb ? -32.f * __half2float(__ushort_as_half((unsigned short)(h.x >> 16))) : 0.f;
-#pragma unroll
-                            for (int gq = 0; gq < 4; ++gq) {
-                                uint32_t sp, mp;
-                                q4k_codes(h, gq, sp, mp);
-                                const float v0 = dm * (float)(mp & 0xFFu), v1 = dm * (float)(mp >> 8);
-                                const __half2 h2 = __floats2half2_rn(v0, v1);
-                                const float2 f2 = __half22float2(h2);
-                                whi[4 * e + gq] = as_u32(h2);
-                                wlo[4 * e + gq] = as_u32(__floats2half2_rn(v0 - f2.x, v1 - f2.y));
-                            }
-                        }
-                        tc_st8(acol + b * 8u, whi);
-                        tc_st8(acol + 32u + b * 8u, wlo);
                     }
                 }
+            } else if (WT == WT_Q4_K && st < nmn) {
+                // a step of block minima: -32 dmin m of 64 sub-blocks (the image holds the sums over 32 activations / 32)
+                const int sb0 = (mn0 + st) * 8, n_sb = a.units >> 3;
+                const uint4* src = w.q + (size_t)row_of(n_of(item_of(c.i)), row) * rpu;
+#pragma unroll 1
+                for (int b = 0; b < 4; ++b) {
+                    uint32_t whi[8], wlo[8];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int sb = sb0 + 2 * b + e;
+                        const uint4 h = __ldg(src + (size_t)min(sb, n_sb - 1) * 9);
+                        const float dm = sb < n_sb ? -32.f * __half2float(__ushort_as_half((unsigned short)(h.x >> 16))) : 0.f;
+#pragma unroll
+                        for (int gq = 0; gq < 4; ++gq) {
+                            uint32_t sp, mp;
+                            q4k_codes(h, gq, sp, mp);
+                            const float v0 = dm * (float)(mp & 0xFFu), v1 = dm * (float)(mp >> 8);
+                            const __half2 h2 = __floats2half2_rn(v0, v1);
+                            const float2 f2 = __half22float2(h2);
+                            whi[4 * e + gq] = as_u32(h2);
+                            wlo[4 * e + gq] = as_u32(__floats2half2_rn(v0 - f2.x, v1 - f2.y));
+                        }
+                    }
+                    tc_st8(acol + b * 8u, whi);
+                    tc_st8(acol + 32u + b * 8u, wlo);
+                }
             }
-            __syncwarp();
-            fetch();                                    // into the slot just taken, while the stores are under way
             tc_st_wait();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&full[stage]);
             if (++at == (uint32_t)G::R) at = 0;
+            next(c);
         }
         cp_wait<0>();
         if (S > 1) finish_split();
@@ -894,23 +905,20 @@ bool gemm_tc_supports(int wtype, const GemvArgs& a, bool tiled) {
 
 typedef void (*TcKernel)(const TcGemm);
 struct TcPick { TcKernel k; int smem, threads; bool attr; };
-template <int WT, int NT, int MODE> static TcPick& tc_pick() {
-    static TcPick p = {k_gemm_tc<WT, NT, MODE>, TcGeo<WT, NT>::SMEM, TcGeo<WT, NT>::THREADS, false};
+template <int WT, int NT, bool HEAD> static TcPick& tc_pick() {
+    static TcPick p = {k_gemm_tc<WT, NT, HEAD>, TcGeo<WT, NT>::SMEM, TcGeo<WT, NT>::THREADS, false};
     return p;
 }
-template <int WT, int MODE> static TcPick& tc_pick(int nt) {
-    return nt == 16 ? tc_pick<WT, 16, MODE>() : nt == 32 ? tc_pick<WT, 32, MODE>() : nt == 64 ? tc_pick<WT, 64, MODE>() : tc_pick<WT, 128, MODE>();
+template <int WT, bool HEAD> static TcPick& tc_pick(int nt) {
+    return nt == 16 ? tc_pick<WT, 16, HEAD>() : nt == 32 ? tc_pick<WT, 32, HEAD>() : nt == 64 ? tc_pick<WT, 64, HEAD>() : tc_pick<WT, 128, HEAD>();
 }
-template <int WT> static TcPick& tc_pick(int nt, int mode) {
-    if constexpr (WT != WT_Q8_0) { if (mode == TC_PAIR) return tc_pick<WT, TC_PAIR>(nt); }
-    return mode == TC_ARGMAX ? tc_pick<WT, TC_ARGMAX>(nt) : tc_pick<WT, TC_STORE>(nt);
-}
+template <int WT> static TcPick& tc_pick(int nt, bool head) { return head ? tc_pick<WT, true>(nt) : tc_pick<WT, false>(nt); }
 
 // Clusters of `s` CTAs that run at the same time, one CTA per SM (clusters stay inside a GPC).
 static int tc_clusters_at_once(int s) {
     static int known[9] = {};
     if (!known[s]) {
-        TcPick& p = tc_pick<WT_Q4_0, 16, TC_STORE>();
+        TcPick& p = tc_pick<WT_Q4_0, 16, false>();
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)s); cfg.blockDim = dim3((unsigned)p.threads); cfg.dynamicSmemBytes = (size_t)p.smem;
         cudaLaunchAttribute at[1];
@@ -973,17 +981,17 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
     t.w0 = a.w0; t.w1 = a.w1; t.y = a.y; t.ldy = a.ldy; t.img = g_tc.img; t.inv = g_tc.inv; t.err = g.dev_err;
     t.N = a.N; t.units = a.K / 32; t.B = a.B; t.swiglu = a.epi == EPI_SWIGLU;
     t.n_min = n_min; t.n_main = n_main; t.S = S;
-    const int stages = ((n_main + S - 1) / S + (n_min + S - 1) / S + sp - 1) / sp, n_periods = (stages * sp + TC_PERIOD - 1) / TC_PERIOD;
-    t.period = (stages + n_periods - 1) / n_periods;
+    t.period = TC_PERIOD / sp;
     t.tiles_n = tiles_n;
     t.items = (int)items;
     t.part = g_tc.part; t.tickets = g_tc.tickets; t.shared = shared ? 1 : 0;
-    const int mode = pair ? TC_PAIR : a.epi == EPI_ARGMAX ? TC_ARGMAX : TC_STORE;
-    if (mode == TC_ARGMAX) {
+    const bool head = a.epi == EPI_ARGMAX;
+    t.pair = pair;
+    if (head) {
         t.best = g_tc.best; t.ticket = (unsigned int*)(g_tc.best + g_tc.inv_cap);
         t.out_tok = a.out_tok; t.out_val = a.out_val; t.out_tok_f32 = a.out_tok_f32; t.softcap = a.softcap;
     }
-    TcPick& p = wtype == WT_Q4_0 ? tc_pick<WT_Q4_0>(nt, mode) : wtype == WT_Q4_K ? tc_pick<WT_Q4_K>(nt, mode) : tc_pick<WT_Q8_0>(nt, mode);
+    TcPick& p = wtype == WT_Q4_0 ? tc_pick<WT_Q4_0>(nt, head) : wtype == WT_Q4_K ? tc_pick<WT_Q4_K>(nt, head) : tc_pick<WT_Q8_0>(nt, head);
     if (!p.attr) {
         if (cudaFuncSetAttribute((const void*)p.k, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem) != cudaSuccess)
             return fail(ADAMAH_ERR_BACKEND, "gemm_tc: cannot raise the shared-memory limit");
