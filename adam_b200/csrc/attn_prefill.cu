@@ -187,18 +187,85 @@ __device__ __forceinline__ void ap_softmax(float (&c)[NT][4], const AttnPrefillA
         }
 }
 
-// ---- fp16 cache: m16n8k16, two terms on the query / probability side ------------------------------------------------
-// NW warps of 16 query rows; tiles of 64 positions.  Shared memory: the query rows' two terms, one K and one V tile; the
-// next K tile is requested when the scores are done, the next V tile after P.V.
-template <int HD, int NW>
-__global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_h(const AttnPrefillArgs a) {
-    constexpr int ROWS = NW * 16, BN = 64, NCH = HD / 8, NTH = NW * 32;
+// The KH warps of a row group hold soft-max sums over different positions of the same rows: added up through shared memory
+// (`ex`: KH / 2 slots per row group of m, l and the output, lane by lane), the result in the warps kh = 0.
+template <int HD, int RG, int KH>
+__device__ __forceinline__ void ap_merge(float4* ex, int rg, int kh, int lane, float (&o)[HD / 8][4], float (&m)[2], float (&l)[2]) {
+#pragma unroll 1
+    for (int step = KH / 2; step > 0; step >>= 1) {
+        float4* at = ex + (size_t)((kh & (step - 1)) * RG + rg) * (HD / 8 + 1) * 32 + lane;
+        __syncthreads();
+        if (kh >= step && kh < 2 * step) {
+            at[0] = make_float4(m[0], m[1], l[0], l[1]);
+#pragma unroll
+            for (int j = 0; j < HD / 8; ++j) at[(j + 1) * 32] = make_float4(o[j][0], o[j][1], o[j][2], o[j][3]);
+        }
+        __syncthreads();
+        if (kh < step) {
+            const float4 y = at[0];
+            const float ym[2] = {y.x, y.y}, yl[2] = {y.z, y.w};
+            float s0[2], s1[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float mn = fmaxf(m[h], ym[h]);
+                s0[h] = expf(m[h] - mn); s1[h] = expf(ym[h] - mn);
+                m[h] = mn;
+                l[h] = l[h] * s0[h] + yl[h] * s1[h];
+            }
+#pragma unroll
+            for (int j = 0; j < HD / 8; ++j) {
+                const float4 v = at[(j + 1) * 32];
+                o[j][0] = o[j][0] * s0[0] + v.x * s1[0]; o[j][1] = o[j][1] * s0[0] + v.y * s1[0];
+                o[j][2] = o[j][2] * s0[1] + v.z * s1[1]; o[j][3] = o[j][3] * s0[1] + v.w * s1[1];
+            }
+        }
+    }
+}
+template <int HD>
+__device__ __forceinline__ void ap_store(const AttnPrefillArgs& a, const AttnTile& t, uint32_t kvh, uint32_t group, int r0, int lane, const float (&o)[HD / 8][4],
+                                         const float (&l_part)[2], float unit) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        float l = l_part[h];
+        l += __shfl_xor_sync(0xffffffffu, l, 1);
+        l += __shfl_xor_sync(0xffffffffu, l, 2);
+        const ApRow r = ap_row(a, t, kvh, group, r0 + (lane >> 2) + 8 * h, HD);
+        if (!r.ok) continue;
+        const float d = l * unit, rd = __frcp_rn(d);
+#pragma unroll
+        for (int j = 0; j < HD / 8; ++j)
+            *reinterpret_cast<float2*>(a.out + r.o + 8 * j + 2 * (lane & 3)) = make_float2(div_by(o[j][2 * h], d, rd), div_by(o[j][2 * h + 1], d, rd));
+    }
+}
+
+// Where a tile's rows lie in the cache: looked up once per row and an iteration ahead (a look-up per 16-byte copy, with its
+// dependent load of the page table, made a tile take 12 us).
+template <int BN>
+__device__ __forceinline__ void ap_locate(const AttnPrefillArgs& a, const int32_t* bt, uint32_t kvh, int kv0, int kv_hi, size_t (&rows)[2][BN]) {
+    if (threadIdx.x < BN) {
+        const int p = min(kv0 + (int)threadIdx.x, kv_hi - 1);
+        const uint32_t pn = (uint32_t)p / a.geo.page;
+        const int32_t page = pn < a.geo.max_pages ? max(bt[pn], 0) : 0;
+        rows[(kv0 / BN) & 1][threadIdx.x] = kv_index(a.geo, (uint32_t)page, a.layer, 0, kvh, (uint32_t)p % a.geo.page);
+    }
+}
+
+// The kernels below: RG groups of 16 query rows, KH warps to a group, each with its share of every tile's positions.  Two
+// tiles of K and V in shared memory.  The loop's first two turns only request tiles (one copy of the code: a launch runs
+// through most of it once or twice, and each instruction's first fetch counts).
+
+// ---- fp16 cache: m16n8k16, two terms on the query / probability side; tiles of 64 positions -------------------------
+template <int HD, int RG, int KH>
+__global__ void __launch_bounds__(RG * KH * 32, 1) k_attn_prefill_h(const AttnPrefillArgs a) {
+    constexpr int ROWS = RG * 16, BN = 64, PB = BN / KH, NCH = HD / 8, NTH = RG * KH * 32;
     extern __shared__ __align__(128) uint8_t sm[];
     __shared__ size_t s_row[2][BN];
+    __shared__ float s_inv[ROWS];
     __half* sQh = reinterpret_cast<__half*>(sm);
     __half* sQl = sQh + ROWS * HD;
-    const uint32_t qh_s = ap_smem(sQh), ql_s = ap_smem(sQl), k_s = ql_s + ROWS * HD * 2, v_s = k_s + BN * HD * 2;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2;
+    const uint32_t qh_s = ap_smem(sQh), ql_s = ap_smem(sQl), kv_s = ql_s + ROWS * HD * 2;
+    constexpr uint32_t TILE = BN * HD * 2;                                              // stage s: K at kv_s + 2 s TILE, V behind it
+    const int tid = threadIdx.x, warp = tid >> 5, rg = warp % RG, kh = warp / RG, lane = tid & 31, g = lane >> 2;
     pdl_launch_dependents();
     pdl_wait();
     const AttnTile t = a.tiles[blockIdx.x];
@@ -208,77 +275,10 @@ __global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_h(const AttnPrefill
     auto sw = [](int r, int ch) { return NCH >= 8 ? ch ^ (r & 7) : ch ^ ((r >> 1) & (NCH - 1)); };
     const int kv_hi = t.pos + t.n_tok;                                                  // positions [.., kv_hi)
     const int kv_lo = a.window > 0 && t.pos + 1 > (int)a.window ? (t.pos + 1 - (int)a.window) / BN * BN : 0;
-    // Where a tile's rows lie in the cache: looked up once per row and a tile ahead (a look-up per 16-byte copy, with its
-    // dependent load of the page table, made a tile take 12 us).
     const size_t v_off = (size_t)a.geo.n_kv * a.geo.page * HD;                          // a value row lies this far behind its key row
-    auto locate = [&](int kv0) {
-        if (tid < BN) {
-            const int p = min(kv0 + tid, kv_hi - 1);
-            const uint32_t pn = (uint32_t)p / a.geo.page;
-            const int32_t page = pn < a.geo.max_pages ? max(bt[pn], 0) : 0;
-            s_row[(kv0 / BN) & 1][tid] = kv_index(a.geo, (uint32_t)page, a.layer, 0, kvh, (uint32_t)p % a.geo.page);
-        }
-    };
-    auto load = [&](uint32_t dst, uint32_t kv, int kv0) {
-        const __half* src = pool + (kv ? v_off : 0);
-        const size_t* rows = s_row[(kv0 / BN) & 1];
-#pragma unroll 8
-        for (int i = tid; i < BN * NCH; i += NTH) {
-            const int r = i / NCH, ch = i % NCH;
-            ap_cp16(dst + (uint32_t)(r * HD + sw(r, ch) * 8) * 2u, src + rows[r] + ch * 8);
-        }
-        ap_commit();
-    };
-    locate(kv_lo);
-    __syncthreads();
-    load(k_s, 0, kv_lo);
-    load(v_s, 1, kv_lo);
-    // this warp's query rows: power-of-two scale per row, two fp16 terms
-    float inv_row[16];
-    constexpr int EPL = HD / 32;                                                        // values per lane
-#pragma unroll
-    for (int r0 = 0; r0 < 16; r0 += 4) {
-        float x[4][EPL];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const ApRow row = ap_row(a, t, kvh, group, warp * 16 + r0 + r, HD);
-#pragma unroll
-            for (int e = 0; e < EPL; ++e) x[r][e] = row.ok ? a.qkv[row.q + lane * EPL + e] : 0.f;
-        }
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            float mxv = 0.f;
-#pragma unroll
-            for (int e = 0; e < EPL; ++e) mxv = fmaxf(mxv, fabsf(x[r][e]));
-            mxv = warp_max(mxv);
-            int ex = 0;                                                                 // largest element into [2^7, 2^8)
-            if (mxv > 0.f && mxv < 3.0e38f) ex = max(-100, min(100, 134 - (int)((__float_as_uint(mxv) >> 23) & 0xFFu)));
-            const float s = __uint_as_float((uint32_t)(127 + ex) << 23);
-            inv_row[r0 + r] = __uint_as_float((uint32_t)(127 - ex) << 23);
-            const int rr = warp * 16 + r0 + r;
-#pragma unroll
-            for (int e = 0; e < EPL; ++e) {
-                const int d = lane * EPL + e;
-                const float v = x[r][e] * s;
-                const __half h = __float2half_rn(v);
-                const int at = rr * HD + sw(rr, d >> 3) * 8 + (d & 7);
-                sQh[at] = h;
-                sQl[at] = __float2half_rn(v - __half2float(h));
-            }
-        }
-    }
-    float scl[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        float v = 0.f;
-#pragma unroll
-        for (int r = 0; r < 8; ++r) v = r == g ? inv_row[8 * h + r] : v;
-        scl[h] = v * a.scale;
-    }
-    const ApRow row0 = ap_row(a, t, kvh, group, warp * 16 + g, HD), row1 = ap_row(a, t, kvh, group, warp * 16 + g + 8, HD);
-    const int pos[2] = {row0.pos, row1.pos};
+    const int pos[2] = {ap_row(a, t, kvh, group, rg * 16 + g, HD).pos, ap_row(a, t, kvh, group, rg * 16 + g + 8, HD).pos};
     // the warp's range of positions, to leave out tiles that it does not attend to
-    const int tok_lo = (warp * 16) / (int)group, tok_hi = min((warp * 16 + 15) / (int)group, t.n_tok - 1);
+    const int tok_lo = (rg * 16) / (int)group, tok_hi = min((rg * 16 + 15) / (int)group, t.n_tok - 1);
     const bool live = tok_lo < t.n_tok;
     const int p_lo = t.pos + tok_lo, p_hi = t.pos + tok_hi;
     float o[HD / 8][4], m[2] = {AP_NEG, AP_NEG}, l[2] = {0.f, 0.f};
@@ -287,51 +287,83 @@ __global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_h(const AttnPrefill
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
 
-    for (int kv0 = kv_lo; kv0 < kv_hi; kv0 += BN) {
-        const bool work = live && kv0 <= p_hi && !(a.window > 0 && kv0 + BN - 1 + (int)a.window <= p_lo);
-        const bool edge = kv0 + BN - 1 > p_lo || (a.window > 0 && kv0 + (int)a.window <= p_hi);
-        float c[8][4], alpha[2] = {1.f, 1.f};
-        if (kv0 + BN < kv_hi) locate(kv0 + BN);
-        ap_wait<1>();
+    ap_locate<BN>(a, bt, kvh, kv_lo, kv_hi, s_row);
+#pragma unroll 1
+    for (int kv0 = kv_lo - 2 * BN; kv0 < kv_hi; kv0 += BN) {
+        if (kv0 >= kv_lo) ap_wait<1>();
         __syncthreads();
-        if (work) {
+        if (kv0 + 3 * BN < kv_hi) ap_locate<BN>(a, bt, kvh, kv0 + 3 * BN, kv_hi, s_row);
+        const uint32_t k_s = kv_s + (uint32_t)((kv0 / BN) & 1) * 2u * TILE, v_s = k_s + TILE;
+        const int part = kv0 + kh * PB;
+        const bool work = kv0 >= kv_lo && live && part <= p_hi && !(a.window > 0 && part + PB - 1 + (int)a.window <= p_lo);
+        if (kv0 == kv_lo - BN) {
+            // the query rows: power-of-two scale per row, two fp16 terms; the row group's warps share them out
+            constexpr int EPL = HD / 32, RB = KH == 4 ? 4 : 2;                          // values per lane, rows at a time
+#pragma unroll 1
+            for (int r0 = kh * (16 / KH); r0 < (kh + 1) * (16 / KH); r0 += RB) {
+                float x[RB][EPL];
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
+                for (int r = 0; r < RB; ++r) {
+                    const ApRow row = ap_row(a, t, kvh, group, rg * 16 + r0 + r, HD);
+#pragma unroll
+                    for (int e = 0; e < EPL; ++e) x[r][e] = row.ok ? a.qkv[row.q + lane * EPL + e] : 0.f;
+                }
+#pragma unroll
+                for (int r = 0; r < RB; ++r) {
+                    float mxv = 0.f;
+#pragma unroll
+                    for (int e = 0; e < EPL; ++e) mxv = fmaxf(mxv, fabsf(x[r][e]));
+                    mxv = warp_max(mxv);
+                    int ex = 0;                                                         // largest element into [2^7, 2^8)
+                    if (mxv > 0.f && mxv < 3.0e38f) ex = max(-100, min(100, 134 - (int)((__float_as_uint(mxv) >> 23) & 0xFFu)));
+                    const float s = __uint_as_float((uint32_t)(127 + ex) << 23);
+                    const int rr = rg * 16 + r0 + r;
+                    if (lane == 0) s_inv[rr] = __uint_as_float((uint32_t)(127 - ex) << 23);
+#pragma unroll
+                    for (int e = 0; e < EPL; ++e) {
+                        const int d = lane * EPL + e;
+                        const float v = x[r][e] * s;
+                        const __half h = __float2half_rn(v);
+                        const int at = rr * HD + sw(rr, d >> 3) * 8 + (d & 7);
+                        sQh[at] = h;
+                        sQl[at] = __float2half_rn(v - __half2float(h));
+                    }
+                }
+            }
+        }
+        if (work) {
+            const bool edge = part + PB - 1 > p_lo || (a.window > 0 && part + (int)a.window <= p_hi);
+            float c[PB / 8][4], alpha[2] = {1.f, 1.f};
+            const float scl[2] = {s_inv[rg * 16 + g] * a.scale, s_inv[rg * 16 + g + 8] * a.scale};
+#pragma unroll
+            for (int j = 0; j < PB / 8; ++j)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) c[j][e] = 0.f;
-#pragma unroll 2
+#pragma unroll KH
             for (int k = 0; k < HD / 16; ++k) {
                 uint32_t qh[4], ql[4];
-                const int qr = warp * 16 + (lane & 15), qc = 2 * k + (lane >> 4);
+                const int qr = rg * 16 + (lane & 15), qc = 2 * k + (lane >> 4);
                 const uint32_t qo = (uint32_t)(qr * HD + sw(qr, qc) * 8) * 2u;
                 ldsm4(qh_s + qo, qh);
                 ldsm4(ql_s + qo, ql);
 #pragma unroll
-                for (int n = 0; n < 4; ++n) {
+                for (int n = 0; n < PB / 16; ++n) {
                     uint32_t b[4];
-                    const int kr = n * 16 + (lane >> 4) * 8 + (lane & 7), kc = 2 * k + ((lane >> 3) & 1);
+                    const int kr = kh * PB + n * 16 + (lane >> 4) * 8 + (lane & 7), kc = 2 * k + ((lane >> 3) & 1);
                     ldsm4(k_s + (uint32_t)(kr * HD + sw(kr, kc) * 8) * 2u, b);
                     mma_h(c[2 * n], ql, b[0], b[1]); mma_h(c[2 * n + 1], ql, b[2], b[3]);
                     mma_h(c[2 * n], qh, b[0], b[1]); mma_h(c[2 * n + 1], qh, b[2], b[3]);
                 }
             }
-        }
-        __syncthreads();
-        if (kv0 + BN < kv_hi) load(k_s, 0, kv0 + BN); else ap_commit();
-        uint32_t ph[4][4], pl[4][4];
-        if (work) {
-            ap_softmax<8>(c, a, scl, pos, kv0, edge, m, l, alpha);
+            uint32_t ph[PB / 16][4], pl[PB / 16][4];
+            ap_softmax<PB / 8>(c, a, scl, pos, part, edge, m, l, alpha);
 #pragma unroll
-            for (int s = 0; s < 4; ++s)
+            for (int s = 0; s < PB / 16; ++s)
 #pragma unroll
                 for (int f = 0; f < 4; ++f) {           // times 256: the low terms stay clear of the fp16 subnormals
                     const float* p = &c[2 * s + (f >> 1)][2 * (f & 1)];
                     half_split(p[0] * 256.f, p[1] * 256.f, ph[s][f], pl[s][f]);
                 }
-        }
-        ap_wait<1>();
-        __syncthreads();
-        if (work) {
             constexpr int DC = HD == 256 ? 32 : HD >= 64 ? 64 : HD;     // dims per round: what the registers beside `o` allow
 #pragma unroll
             for (int d0 = 0; d0 < HD; d0 += DC) {
@@ -341,11 +373,11 @@ __global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_h(const AttnPrefill
 #pragma unroll
                     for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
 #pragma unroll
-                for (int s = 0; s < 4; ++s)
+                for (int s = 0; s < PB / 16; ++s)
 #pragma unroll
                     for (int n = 0; n < DC / 16; ++n) {
                         uint32_t b[4];
-                        const int vr = s * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), vc = d0 / 8 + 2 * n + (lane >> 4);
+                        const int vr = kh * PB + s * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), vc = d0 / 8 + 2 * n + (lane >> 4);
                         ldsm4t(v_s + (uint32_t)(vr * HD + sw(vr, vc) * 8) * 2u, b);
                         mma_h(acc[2 * n], pl[s], b[0], b[1]); mma_h(acc[2 * n + 1], pl[s], b[2], b[3]);
                         mma_h(acc[2 * n], ph[s], b[0], b[1]); mma_h(acc[2 * n + 1], ph[s], b[2], b[3]);
@@ -357,33 +389,34 @@ __global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_h(const AttnPrefill
             }
         }
         __syncthreads();
-        if (kv0 + BN < kv_hi) load(v_s, 1, kv0 + BN); else ap_commit();
+        if (kv0 + 2 * BN < kv_hi) {
+            const size_t* rows = s_row[(kv0 / BN) & 1];
+#pragma unroll 4
+            for (int i = tid; i < BN * NCH; i += NTH) {
+                const int r = i / NCH, ch = i % NCH;
+                const __half* src = pool + rows[r] + ch * 8;
+                const uint32_t dst = (uint32_t)(r * HD + sw(r, ch) * 8) * 2u;
+                ap_cp16(k_s + dst, src);
+                ap_cp16(v_s + dst, src + v_off);
+            }
+        }
+        ap_commit();
     }
     ap_wait<0>();
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
-        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
-        const ApRow& r = h ? row1 : row0;
-        if (!r.ok) continue;
-        const float d = l[h] * 256.f, rd = __frcp_rn(d);
-#pragma unroll
-        for (int j = 0; j < HD / 8; ++j)
-            *reinterpret_cast<float2*>(a.out + r.o + 8 * j + 2 * (lane & 3)) = make_float2(div_by(o[j][2 * h], d, rd), div_by(o[j][2 * h + 1], d, rd));
-    }
+    ap_merge<HD, RG, KH>(reinterpret_cast<float4*>(sm), rg, kh, lane, o, m, l);
+    if (kh == 0) ap_store<HD>(a, t, kvh, group, rg * 16, lane, o, l, 256.f);
 }
 
-// ---- fp32 cache: m16n8k8 tf32, three products per pair --------------------------------------------------------------
+// ---- fp32 cache: m16n8k8 tf32, three products per pair; tiles of 32 positions ---------------------------------------
 // Operands stay fp32 in shared memory (rows padded by 4 floats: the fragment reads below are free of bank conflicts) and
-// are split into two tf32 terms as they are read.  Tiles of 32 positions.
-template <int HD, int NW>
-__global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_f(const AttnPrefillArgs a) {
-    constexpr int ROWS = NW * 16, BN = 32, LD = HD + 4, NTH = NW * 32;
+// are split into two tf32 terms as they are read.
+template <int HD, int RG, int KH>
+__global__ void __launch_bounds__(RG * KH * 32, 1) k_attn_prefill_f(const AttnPrefillArgs a) {
+    constexpr int ROWS = RG * 16, BN = 32, PB = BN / KH, LD = HD + 4, NTH = RG * KH * 32;
     extern __shared__ __align__(128) uint8_t sm[];
     __shared__ size_t s_row[2][BN];
-    float *sQ = reinterpret_cast<float*>(sm), *sK = sQ + ROWS * LD, *sV = sK + BN * LD;
-    const uint32_t k_s = ap_smem(sK), v_s = ap_smem(sV);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+    float *sQ = reinterpret_cast<float*>(sm), *sKV = sQ + ROWS * LD;                    // stage s: K at sKV + 2 s BN LD, V behind it
+    const int tid = threadIdx.x, warp = tid >> 5, rg = warp % RG, kh = warp / RG, lane = tid & 31, g = lane >> 2, q = lane & 3;
     pdl_launch_dependents();
     pdl_wait();
     const AttnTile t = a.tiles[blockIdx.x];
@@ -392,39 +425,10 @@ __global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_f(const AttnPrefill
     const int32_t* bt = a.block_table + (size_t)t.seq * a.geo.max_pages;
     const int kv_hi = t.pos + t.n_tok;
     const int kv_lo = a.window > 0 && t.pos + 1 > (int)a.window ? (t.pos + 1 - (int)a.window) / BN * BN : 0;
-    const size_t v_off = (size_t)a.geo.n_kv * a.geo.page * HD;                          // see k_attn_prefill_h
-    auto locate = [&](int kv0) {
-        if (tid < BN) {
-            const int p = min(kv0 + tid, kv_hi - 1);
-            const uint32_t pn = (uint32_t)p / a.geo.page;
-            const int32_t page = pn < a.geo.max_pages ? max(bt[pn], 0) : 0;
-            s_row[(kv0 / BN) & 1][tid] = kv_index(a.geo, (uint32_t)page, a.layer, 0, kvh, (uint32_t)p % a.geo.page);
-        }
-    };
-    auto load = [&](uint32_t dst, uint32_t kv, int kv0) {
-        const float* src = pool + (kv ? v_off : 0);
-        const size_t* rows = s_row[(kv0 / BN) & 1];
-#pragma unroll 8
-        for (int i = tid; i < BN * (HD / 4); i += NTH) {
-            const int r = i / (HD / 4), ch = i % (HD / 4);
-            ap_cp16(dst + (uint32_t)(r * LD + ch * 4) * 4u, src + rows[r] + ch * 4);
-        }
-        ap_commit();
-    };
-    locate(kv_lo);
-    __syncthreads();
-    load(k_s, 0, kv_lo);
-    load(v_s, 1, kv_lo);
-#pragma unroll 4
-    for (int r = 0; r < 16; ++r) {
-        const ApRow row = ap_row(a, t, kvh, group, warp * 16 + r, HD);
-#pragma unroll
-        for (int d = lane; d < HD; d += 32) sQ[(warp * 16 + r) * LD + d] = row.ok ? a.qkv[row.q + d] : 0.f;
-    }
+    const size_t v_off = (size_t)a.geo.n_kv * a.geo.page * HD;
     const float scl[2] = {a.scale, a.scale};
-    const ApRow row0 = ap_row(a, t, kvh, group, warp * 16 + g, HD), row1 = ap_row(a, t, kvh, group, warp * 16 + g + 8, HD);
-    const int pos[2] = {row0.pos, row1.pos};
-    const int tok_lo = (warp * 16) / (int)group, tok_hi = min((warp * 16 + 15) / (int)group, t.n_tok - 1);
+    const int pos[2] = {ap_row(a, t, kvh, group, rg * 16 + g, HD).pos, ap_row(a, t, kvh, group, rg * 16 + g + 8, HD).pos};
+    const int tok_lo = (rg * 16) / (int)group, tok_hi = min((rg * 16 + 15) / (int)group, t.n_tok - 1);
     const bool live = tok_lo < t.n_tok;
     const int p_lo = t.pos + tok_lo, p_hi = t.pos + tok_hi;
     float o[HD / 8][4], m[2] = {AP_NEG, AP_NEG}, l[2] = {0.f, 0.f};
@@ -433,44 +437,49 @@ __global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_f(const AttnPrefill
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
 
-    for (int kv0 = kv_lo; kv0 < kv_hi; kv0 += BN) {
-        const bool work = live && kv0 <= p_hi && !(a.window > 0 && kv0 + BN - 1 + (int)a.window <= p_lo);
-        const bool edge = kv0 + BN - 1 > p_lo || (a.window > 0 && kv0 + (int)a.window <= p_hi);
-        float c[4][4], alpha[2] = {1.f, 1.f};
-        if (kv0 + BN < kv_hi) locate(kv0 + BN);
-        ap_wait<1>();
+    ap_locate<BN>(a, bt, kvh, kv_lo, kv_hi, s_row);
+#pragma unroll 1
+    for (int kv0 = kv_lo - 2 * BN; kv0 < kv_hi; kv0 += BN) {
+        if (kv0 >= kv_lo) ap_wait<1>();
         __syncthreads();
-        if (work) {
+        if (kv0 + 3 * BN < kv_hi) ap_locate<BN>(a, bt, kvh, kv0 + 3 * BN, kv_hi, s_row);
+        float *sK = sKV + (size_t)((kv0 / BN) & 1) * 2 * BN * LD, *sV = sK + BN * LD;
+        const int part = kv0 + kh * PB;
+        const bool work = kv0 >= kv_lo && live && part <= p_hi && !(a.window > 0 && part + PB - 1 + (int)a.window <= p_lo);
+        if (kv0 == kv_lo - BN)
+#pragma unroll 2
+            for (int r = kh * (16 / KH); r < (kh + 1) * (16 / KH); ++r) {
+                const ApRow row = ap_row(a, t, kvh, group, rg * 16 + r, HD);
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+                for (int d = lane; d < HD; d += 32) sQ[(rg * 16 + r) * LD + d] = row.ok ? a.qkv[row.q + d] : 0.f;
+            }
+        if (work) {
+            const bool edge = part + PB - 1 > p_lo || (a.window > 0 && part + (int)a.window <= p_hi);
+            float c[PB / 8][4], alpha[2] = {1.f, 1.f};
+#pragma unroll
+            for (int j = 0; j < PB / 8; ++j)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) c[j][e] = 0.f;
-#pragma unroll 2
+#pragma unroll KH
             for (int k = 0; k < HD; k += 8) {
-                const float* qp = sQ + (warp * 16 + g) * LD + k + q;
+                const float* qp = sQ + (rg * 16 + g) * LD + k + q;
                 uint32_t ah[4], al[4];
                 tf32_split(qp[0], ah[0], al[0]); tf32_split(qp[8 * LD], ah[1], al[1]);
                 tf32_split(qp[4], ah[2], al[2]); tf32_split(qp[8 * LD + 4], ah[3], al[3]);
 #pragma unroll
-                for (int n = 0; n < 4; ++n) {
-                    const float* kp = sK + (n * 8 + g) * LD + k + q;
+                for (int n = 0; n < PB / 8; ++n) {
+                    const float* kp = sK + (kh * PB + n * 8 + g) * LD + k + q;
                     uint32_t b0h, b0l, b1h, b1l;
                     tf32_split(kp[0], b0h, b0l); tf32_split(kp[4], b1h, b1l);
                     mma_t(c[n], al, b0h, b1h); mma_t(c[n], ah, b0l, b1l); mma_t(c[n], ah, b0h, b1h);
                 }
             }
-        }
-        __syncthreads();
-        if (kv0 + BN < kv_hi) load(k_s, 0, kv0 + BN); else ap_commit();
-        if (work) ap_softmax<4>(c, a, scl, pos, kv0, edge, m, l, alpha);
-        ap_wait<1>();
-        __syncthreads();
-        if (work) {
+            ap_softmax<PB / 8>(c, a, scl, pos, part, edge, m, l, alpha);
             // the order of the positions inside a step of 8 is free: slots t and t + 4 are positions 2 t and 2 t + 1, which is
             // how the scores lie in the registers
-            uint32_t ph[4][4], pl[4][4];
+            uint32_t ph[PB / 8][4], pl[PB / 8][4];
 #pragma unroll
-            for (int s = 0; s < 4; ++s) {
+            for (int s = 0; s < PB / 8; ++s) {
                 tf32_split(c[s][0], ph[s][0], pl[s][0]); tf32_split(c[s][2], ph[s][1], pl[s][1]);
                 tf32_split(c[s][1], ph[s][2], pl[s][2]); tf32_split(c[s][3], ph[s][3], pl[s][3]);
             }
@@ -483,10 +492,10 @@ __global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_f(const AttnPrefill
 #pragma unroll
                     for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
 #pragma unroll
-                for (int s = 0; s < 4; ++s)
+                for (int s = 0; s < PB / 8; ++s)
 #pragma unroll
                     for (int n = 0; n < DC / 8; ++n) {
-                        const float* vp = sV + (s * 8 + 2 * q) * LD + d0 + n * 8 + g;
+                        const float* vp = sV + (kh * PB + s * 8 + 2 * q) * LD + d0 + n * 8 + g;
                         uint32_t b0h, b0l, b1h, b1l;
                         tf32_split(vp[0], b0h, b0l); tf32_split(vp[LD], b1h, b1l);
                         mma_t(acc[n], pl[s], b0h, b1h); mma_t(acc[n], ph[s], b0l, b1l); mma_t(acc[n], ph[s], b0h, b1h);
@@ -498,20 +507,23 @@ __global__ void __launch_bounds__(NW * 32, 1) k_attn_prefill_f(const AttnPrefill
             }
         }
         __syncthreads();
-        if (kv0 + BN < kv_hi) load(v_s, 1, kv0 + BN); else ap_commit();
+        if (kv0 + 2 * BN < kv_hi) {
+            const size_t* rows = s_row[(kv0 / BN) & 1];
+            const uint32_t k_s = ap_smem(sK), v_s = ap_smem(sV);
+#pragma unroll 4
+            for (int i = tid; i < BN * (HD / 4); i += NTH) {
+                const int r = i / (HD / 4), ch = i % (HD / 4);
+                const float* src = pool + rows[r] + ch * 4;
+                const uint32_t dst = (uint32_t)(r * LD + ch * 4) * 4u;
+                ap_cp16(k_s + dst, src);
+                ap_cp16(v_s + dst, src + v_off);
+            }
+        }
+        ap_commit();
     }
     ap_wait<0>();
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
-        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
-        const ApRow& r = h ? row1 : row0;
-        if (!r.ok) continue;
-        const float rd = __frcp_rn(l[h]);
-#pragma unroll
-        for (int j = 0; j < HD / 8; ++j)
-            *reinterpret_cast<float2*>(a.out + r.o + 8 * j + 2 * q) = make_float2(div_by(o[j][2 * h], l[h], rd), div_by(o[j][2 * h + 1], l[h], rd));
-    }
+    ap_merge<HD, RG, KH>(reinterpret_cast<float4*>(sm), rg, kh, lane, o, m, l);
+    if (kh == 0) ap_store<HD>(a, t, kvh, group, rg * 16, lane, o, l, 1.f);
 }
 
 // ---- host ----------------------------------------------------------------------------------------------------------
@@ -532,10 +544,12 @@ int launch_qkv_prep(const AttnPrefillArgs& a, bool kv_half, cudaStream_t stream,
     return kv_half ? prep_t<__half>(a, stream, pdl) : prep_t<float>(a, stream, pdl);
 }
 
-template <int HD, int NW>
+template <int HD, int RG, int KH>
 static int attn_t(const AttnPrefillArgs& a, bool kv_half, cudaStream_t stream, bool pdl) {
-    constexpr size_t smem_h = (size_t)(2 * NW * 16 + 2 * 64) * HD * 2, smem_f = (size_t)(NW * 16 + 2 * 32) * (HD + 4) * 4;
-    void (*k)(const AttnPrefillArgs) = kv_half ? k_attn_prefill_h<HD, NW> : k_attn_prefill_f<HD, NW>;
+    constexpr size_t rows = RG * 16, smem_h = (2 * rows + 4 * 64) * HD * 2, smem_f = (rows + 4 * 32) * (HD + 4) * 4;
+    constexpr size_t merge = (size_t)(KH / 2) * RG * (HD / 8 + 1) * 32 * 16;
+    static_assert(merge <= smem_h && merge <= smem_f && smem_h <= 225 * 1024 && smem_f <= 225 * 1024, "shared memory");
+    void (*k)(const AttnPrefillArgs) = kv_half ? k_attn_prefill_h<HD, RG, KH> : k_attn_prefill_f<HD, RG, KH>;
     const size_t smem = kv_half ? smem_h : smem_f;
     static bool set[2] = {false, false};
     if (!set[kv_half]) {
@@ -543,13 +557,15 @@ static int attn_t(const AttnPrefillArgs& a, bool kv_half, cudaStream_t stream, b
             return fail(ADAMAH_ERR_BACKEND, "attn_prefill: cannot raise the shared-memory limit");
         set[kv_half] = true;
     }
-    launch_k(k, dim3(a.n_tiles, a.geo.n_kv), dim3(NW * 32), smem, stream, pdl, a);
+    launch_k(k, dim3(a.n_tiles, a.geo.n_kv), dim3(RG * KH * 32), smem, stream, pdl, a);
     count_launch();
     return check_launch("attn_prefill");
 }
 template <int HD>
 static int attn_r(const AttnPrefillArgs& a, bool kv_half, uint32_t rows, cudaStream_t stream, bool pdl) {
-    return rows == 128 ? attn_t<HD, 8>(a, kv_half, stream, pdl) : attn_t<HD, 4>(a, kv_half, stream, pdl);
+    if constexpr (HD <= 128)
+        if (rows == 128) return attn_t<HD, 8, 1>(a, kv_half, stream, pdl);
+    return rows == 64 ? attn_t<HD, 4, 2>(a, kv_half, stream, pdl) : attn_t<HD, 2, 4>(a, kv_half, stream, pdl);
 }
 int launch_attn_prefill(const AttnPrefillArgs& a, bool kv_half, uint32_t tile_rows, cudaStream_t stream, bool pdl) {
     switch (a.head_dim) {

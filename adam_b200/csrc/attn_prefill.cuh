@@ -21,8 +21,15 @@ struct AttnPrefillArgs {
     uint32_t* err;
 };
 
-// Positions per attention tile for this group size (query heads per kv head); `rows` = 64 or 128 query rows per tile.
-inline uint32_t attn_prefill_tokens(uint32_t group, uint32_t rows) { return rows / group; }
+// Query rows per attention tile: the widest of 128 (head_dim <= 128: shared memory), 64 and 32 whose tiles still give every
+// SM one.  A wide tile reads the cache less often; below one tile per SM the chunk's time is that of its longest tile, which
+// a narrow tile, with more warps to each query row, gets through faster.  `positions`: rows of the chunk's sequences.
+inline uint32_t attn_prefill_tokens(uint32_t group, uint32_t rows) { return rows / group; }     // positions per tile
+inline uint32_t attn_prefill_rows(uint32_t positions, uint32_t group, uint32_t n_kv, uint32_t head_dim, uint32_t sms) {
+    for (uint32_t rows = head_dim <= 128 ? 128 : 64; rows > 32; rows /= 2)
+        if ((uint64_t)positions * group / rows * n_kv >= sms || rows / 2 < group) return rows;
+    return 32;
+}
 // QK-norm + RoPE of the chunk's query rows (in place) and key rows, append of keys and values to the cache.
 int launch_qkv_prep(const AttnPrefillArgs& a, bool kv_half, cudaStream_t stream, bool pdl);
 // Causal (and windowed) soft-max attention of every chunk row over the cache, which already holds the chunk's rows.

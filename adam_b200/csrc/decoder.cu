@@ -1535,7 +1535,7 @@ static int plan_prefill(Decoder* D, const uint32_t* n_tokens) {
     std::vector<Cut> cuts;
     uint32_t b = 0, at = 0;                             // sequence and how many of its tokens are placed
     while (seq.size() < total) {
-        Cut c = {(uint32_t)seq.size(), 0, (uint32_t)tiles.size(), 0, 128};
+        Cut c = {(uint32_t)seq.size(), 0, (uint32_t)tiles.size(), 0, 0};
         struct Run { uint32_t row, b, pos, n; };
         std::vector<Run> runs;
         while (c.rows < size && b < D->batch) {
@@ -1545,10 +1545,7 @@ static int plan_prefill(Decoder* D, const uint32_t* n_tokens) {
             c.rows += n; at += n;
             if (at == n_tokens[b]) { ++b; at = 0; }
         }
-        // 128 query rows per attention tile while that still fills the SMs (each tile of the cache is then read half as often)
-        uint32_t wide = 0;
-        for (const Run& r : runs) wide += (r.n + attn_prefill_tokens(group, 128) - 1) / attn_prefill_tokens(group, 128);
-        if (wide * d.n_head_kv < (uint32_t)g.sm_count) c.tile_rows = 64;
+        c.tile_rows = attn_prefill_rows(c.rows, group, d.n_head_kv, d.head_dim, (uint32_t)g.sm_count);
         const uint32_t step = attn_prefill_tokens(group, c.tile_rows);
         for (const Run& r : runs)
             for (uint32_t i = 0; i < r.n; i += step)
