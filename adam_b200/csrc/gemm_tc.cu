@@ -879,17 +879,18 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
 
 // ---- host ----------------------------------------------------------------------------------------------------------
 // Fewest rows from which the GEMM is faster than the GEMV kernels, measured in decode steps and single calls.  The GEMV
-// passes over the weights once per 1, 2 or 4 rows; where the passes run side by side on idle SMs (matrices of a few MB) that
-// costs little (1B shape, 9 rows: 1.22 against 1.31 ms per step; 12: equal; 16: 1.39 against 1.33), where they fill the GPU
-// it costs their number (27B shape, 4 rows: 1.62 against 1.88 ms, 6: 2.16 against 2.03, 12: 3.93 against 2.08).  An LM head of a
-// narrow model is bound by rebuilding weights here (262144 x 1152: 75 us whatever the rows, the GEMV 43 us at 4 and 71 at 8).
+// passes over the weights once per 1, 2 or 4 rows.  Where the passes run side by side on idle SMs (matrices below some 10 MB)
+// that costs little (1B shape: 8 rows 1.11 against 1.10 ms per step, a chunk of 8 prompt rows 1.39 against 1.45 ms; 10 rows:
+// 1.22 against 1.15; 12: 1.35 against 1.16); where they fill the GPU it costs their number (27B shape with every matrix on
+// one path, 4 rows: 1.62 against 2.02 ms, 6: 2.5 against 2.04, 12: 3.9 against 2.08).  An LM head of a narrow model is bound by
+// rebuilding weights here (262144 x 1152: 75 us whatever the rows, the GEMV 43 us at 4 and 71 at 8).
 // Without a row-tiled copy a GEMV takes one launch per four rows (7 us each), and Q8_0 / Q5_0 have no tensor-core GEMV.
 static int tc_rows_from(int wtype, const GemvArgs& a, bool pair, bool tiled) {
     if (wtype == WT_Q8_0) return 4;
     if (!tiled) return 5;
     const double bytes = (double)a.N * a.K * 0.5625 * (pair ? 2 : 1);
     if (a.epi == EPI_ARGMAX && a.K < 4096) return 9;
-    return bytes > 16.0e6 ? 6 : 13;
+    return bytes > 10.0e6 ? 6 : 9;
 }
 
 bool gemm_tc_supports(int wtype, const GemvArgs& a, bool tiled) {
