@@ -147,7 +147,7 @@ class Adamah:
         locs = np.ascontiguousarray(locs, dtype=np.uint32)
         n = n_locs if n_locs is not None else (n_packs if n_packs is not None else len(locs))
         pack = self._maps.get(map_id, (4, 1, 0, 0))[1]
-        out = np.empty(n * pack, dtype=np.uint32)
+        out = self.host_arrays.empty((n * pack,), np.uint32)
         self._metrics["gather_calls"] += 1
         self._check(self._lib.map_gather(map_id, self._ptr(locs), self._ptr(out), n), "map_gather")
         self._metrics["total_bytes_gpu_to_cpu"] += out.nbytes

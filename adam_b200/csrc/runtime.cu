@@ -425,7 +425,7 @@ namespace ab { bool capturing(); }
 // ring, one pinned download buffer and one device scratch buffer for its lifetime (bounded below; larger requests take
 // the plain path).  An upload is read into the ring before the call returns and needs no synchronisation: everything
 // that reads its destination is behind it on the stream.  One gather of 1152 floats: 500 -> 12 us.
-constexpr size_t RING_BYTES = 4u << 20, RING_MAX = 1u << 20, DOWN_BYTES = 4u << 20, SCRATCH_KEEP = 16u << 20;
+constexpr size_t RING_BYTES = 4u << 20, RING_MAX = 1u << 20, DOWN_BYTES = 4u << 20, DIRECT_MIN = 64u << 10, SCRATCH_KEEP = 16u << 20;
 struct IoStage { uint8_t* ring; size_t ring_at; uint8_t* down; uint8_t* scratch; size_t scratch_cap; };
 static IoStage g_io = {};
 
@@ -450,18 +450,23 @@ static cudaError_t upload(void* dst, const void* src, size_t n) {
     const cudaError_t e = cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, g.stream);
     return e == cudaSuccess ? cudaStreamSynchronize(g.stream) : e;
 }
-// Device bytes -> host; returns when they are there.
-static cudaError_t download(void* dst, const void* src, size_t n) {
-    if (n <= DOWN_BYTES && (g_io.down || cudaMallocHost((void**)&g_io.down, DOWN_BYTES) == cudaSuccess)) {
-        cudaError_t e = cudaMemcpyAsync(g_io.down, src, n, cudaMemcpyDeviceToHost, g.stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream);
-        if (e == cudaSuccess) memcpy(dst, g_io.down, n);
-        return e;
+// Device bytes -> host; returns when they are there.  `meanwhile` runs while the copy does.
+template <typename F>
+static cudaError_t download(void* dst, const void* src, size_t n, F meanwhile) {
+    bool direct = false;                                        // page-locked by the caller (adam_b200_host_alloc, for one)
+    if (n >= DIRECT_MIN) {
+        cudaPointerAttributes at = {};
+        direct = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeHost;
     }
-    cudaGetLastError();
-    const cudaError_t e = cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, g.stream);
-    return e == cudaSuccess ? cudaStreamSynchronize(g.stream) : e;
+    const bool staged = !direct && n <= DOWN_BYTES && (g_io.down || cudaMallocHost((void**)&g_io.down, DOWN_BYTES) == cudaSuccess);
+    if (!staged) cudaGetLastError();
+    cudaError_t e = cudaMemcpyAsync(staged ? g_io.down : dst, src, n, cudaMemcpyDeviceToHost, g.stream);
+    meanwhile();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream);
+    if (e == cudaSuccess && staged) memcpy(dst, g_io.down, n);
+    return e;
 }
+static cudaError_t download(void* dst, const void* src, size_t n) { return download(dst, src, n, [] {}); }
 // Device scratch of one call, released on every way out of it: the kept buffer, or a stream-ordered allocation of its own.
 struct Scratch {
     uint8_t* p = nullptr; bool own = false;
@@ -540,14 +545,17 @@ extern "C" int map_gather(uint32_t id, const uint32_t* locs, void* out, uint32_t
     if (m->dtype != ADAMAH_DTYPE_F32 && m->dtype != ADAMAH_DTYPE_Q4)
         return fail(ADAMAH_ERR_INVALID, "gather: map %u holds GGUF blocks; use map_dequant_gguf", id);
     uint64_t n = (uint64_t)n_locs * m->pack_size;
-    if (m->dtype == ADAMAH_DTYPE_F32 && (uint64_t)locs[0] + n_locs <= m->n_packs) {
-        // neighbouring packs (a whole result vector): one copy, no locs on the device, no kernel
-        uint32_t apart = 0;
-        for (uint32_t i = 0; i < n_locs; ++i) apart |= locs[i] ^ (locs[0] + i);
-        if (!apart) {
-            CU(download(out, (const float*)m->buf + (uint64_t)locs[0] * m->pack_size, n * 4));
-            return check_launch("map_gather");
-        }
+    if (m->dtype == ADAMAH_DTYPE_F32 && (uint64_t)locs[0] + n_locs <= m->n_packs && locs[n_locs - 1] == locs[0] + n_locs - 1) {
+        // neighbouring packs (a whole result vector): one copy, no locs on the device, no kernel; the locs between the first
+        // and the last are looked at while it is under way
+        bool apart = false;
+        CU(download(out, (const float*)m->buf + (uint64_t)locs[0] * m->pack_size, n * 4, [&] {
+            const uint32_t first = locs[0];
+            uint32_t d = 0;
+            for (uint32_t i = 0; i < n_locs; ++i) d |= locs[i] ^ (first + i);
+            apart = d != 0;
+        }));
+        if (!apart) return check_launch("map_gather");
     }
     Scratch tmp;
     CU(tmp.get(pad256(n * 4) + (size_t)n_locs * 4));

@@ -7,6 +7,7 @@ fault for every 4 KB of a fresh array (68 MB of logits: 15 ms and more); into pa
 from __future__ import annotations
 
 import ctypes
+import math
 import threading
 import weakref
 
@@ -14,18 +15,21 @@ import numpy as np
 
 
 class HostArrays:
-    MIN = 1 << 20                   # smaller arrays are ordinary ones
+    MIN = 1 << 16                   # smaller arrays are ordinary ones
+    LARGE = 1 << 20
+    SMALL_LIMIT = 16 << 20          # bytes of the blocks below LARGE, in use or kept
     LIMIT = 512 << 20               # bytes of unused blocks kept
 
     def __init__(self, lib):
         self._lib, self._lock = lib, threading.Lock()
         self._free = []             # (bytes, address)
         self._kept = 0
+        self._small = 0             # bytes of the blocks below LARGE
         self._closed = False
 
     def empty(self, shape, dtype) -> np.ndarray:
         dtype = np.dtype(dtype)
-        n = int(np.prod(shape)) * dtype.itemsize
+        n = math.prod(shape) * dtype.itemsize
         if n < self.MIN:
             return np.empty(shape, dtype)
         block = None
@@ -35,10 +39,17 @@ class HostArrays:
                 block = min(fits)
                 self._free.remove(block)
                 self._kept -= block[0]
+            step = self.LARGE if n >= self.LARGE else self.MIN
+            size = (n + step - 1) // step * step
+            if block is None and size < self.LARGE:
+                if self._small + size > self.SMALL_LIMIT:
+                    return np.empty(shape, dtype)
+                self._small += size
         if block is None:
-            size = (n + self.MIN - 1) // self.MIN * self.MIN
             address = self._lib.adam_b200_host_alloc(size)
             if not address:
+                with self._lock:
+                    self._small -= size if size < self.LARGE else 0
                 return np.empty(shape, dtype)
             block = (size, address)
         raw = (ctypes.c_char * n).from_address(block[1])
@@ -51,6 +62,7 @@ class HostArrays:
                 self._free.append(block)
                 self._kept += block[0]
                 return
+            self._small -= block[0] if block[0] < self.LARGE else 0
         self._lib.adam_b200_host_free(block[1])
 
     def close(self):
