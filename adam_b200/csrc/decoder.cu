@@ -752,7 +752,12 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
     static const uint32_t cpc_env = getenv("ADAM_B200_ATTN_CPC") ? (uint32_t)atoi(getenv("ADAM_B200_ATTN_CPC")) : 0u;
     const uint32_t pairs = grid.y * grid.z;
     const uint32_t cpc = cpc_env ? cpc_env : (work <= 64u ? 8u : ATTN_CHUNKS_PER_CTA);
-    (void)pairs;
+    // Position splits launched: no more than this layer can reach (a split without positions still costs a CTA its start and the
+    // read of the position: 15 of 16 CTAs of the 27B shape's 64 sequences, 60 of the launch's 75 us), and no more than four
+    // CTAs per SM in all -- beyond that the pairs alone fill the GPU and a CTA takes more chunks instead.
+    const uint32_t reach = window ? (window < d.kv_cap ? window : d.kv_cap) : d.kv_cap;
+    const uint32_t useful = ((reach + ATTN_CP - 1) / ATTN_CP + 1 + cpc - 1) / cpc, fill = (4u * (uint32_t)g.sm_count + pairs - 1) / pairs;
+    grid.x = std::min(D->n_splits, std::min(useful, fill));
     AttnKernel kern = hpc <= 1 ? pick_attn_hd<T, 1>(d.head_dim) : hpc <= 2 ? pick_attn_hd<T, 2>(d.head_dim)
                     : hpc <= 4 ? pick_attn_hd<T, 4>(d.head_dim) : pick_attn_hd<T, 8>(d.head_dim);
     // Few (sequence, head) pairs in flight (at most 12): the position splits of a pair form one thread-block cluster of 8 CTAs and merge
@@ -762,7 +767,6 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
     // and so does every kernel behind them.)  ADAM_B200_ATTN_CLUSTER=0 turns the path off, =16 allows clusters of 16.
     static const int cluster_env = getenv("ADAM_B200_ATTN_CLUSTER") ? atoi(getenv("ADAM_B200_ATTN_CLUSTER")) : 8;
     static const uint32_t cluster_work = getenv("ADAM_B200_ATTN_CLUSTER_WORK") ? (uint32_t)atoi(getenv("ADAM_B200_ATTN_CLUSTER_WORK")) : 12u;
-    const uint32_t reach = window ? (window < d.kv_cap ? window : d.kv_cap) : d.kv_cap;
     // The kernels behind a cluster launch start later (their prologues no longer overlap it); that costs more than the merge
     // saves once the o-proj behind it has more than about a megabyte of tiles to request (27B shape, 4-way shard: 2 % slower).
     const size_t o_bytes = (size_t)ly.m[MAT_O].rows * ly.m[MAT_O].cols * 9 / 16;
