@@ -776,7 +776,7 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                     q4k_codes(hdr, ks & 3, sp, mp);
                     d01 = (hdr.x & 0xFFFFu) * 0x10001u;
                 }
-#pragma unroll (NT == 128 ? 2 : 1)
+#pragma unroll (NT == 128 || WT == WT_Q4_K ? 2 : 1)
                 for (int b = 0; b < 2; ++b) {           // 32 values of K: columns 16 b .. of w_hi and of w_lo
                     const uint32_t col = acol + b * 16u;
                     uint32_t whi[8], wlo[8], v[2];
