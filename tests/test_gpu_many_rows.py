@@ -1,0 +1,135 @@
+"""Calls of many rows at the sizes where their kernels change tiles: the tcgen05 GEMM, the LM head's arg-max on it, the
+attention of prompt chunks, scoring a text, and the host side of large results."""
+import gc
+from dataclasses import replace
+
+import numpy as np
+import pytest
+
+import adam_b200 as A
+from adam_b200 import gguf_blocks as gb
+from adam_b200 import synth
+from adam_b200.config import GenerationConfig, tiny_gemma3
+from adam_b200.engine import ADAMEngine
+from oracle import q4_blocks
+from oracle.decoder import OracleDecoder, dequant_model
+
+from tests.test_gpu_blocks8 import _matmul
+from tests.test_gpu_decoder import GREEDY
+from tests.test_gpu_gemv import _gemv
+
+pytestmark = pytest.mark.gpu
+
+
+# Rows around the tiles of 16, 32, 64 and 128; weight rows that are not whole tiles of 128; an odd number of blocks per row; one
+# tile on a cluster of CTAs (long K); more tiles than SMs, shared between CTAs or dealt in turn.
+@pytest.mark.parametrize("ggml_type,N,K,B", [
+    (2, 128, 64, 16), (2, 100, 96, 17), (2, 256, 6912, 33), (2, 1152, 1056, 65), (2, 19200, 256, 9), (2, 6000, 320, 129), (2, 1536, 1152, 200),
+    (2, 200, 128, 1025), (8, 256, 6912, 40), (8, 300, 96, 70), (8, 130, 1152, 300), (12, 256, 256, 16), (12, 129, 2304, 65), (12, 21504, 512, 32), (12, 384, 5376, 257)])
+def test_gemm_tiles(gpu, ggml_type, N, K, B):
+    """Relative error of a row below 5e-6: activations keep 22 bits (2^-22), and up to 33 additions of the tensor core are
+    rounded towards zero, each by less than 2^-23 of the running sum, before the sum moves to registers."""
+    rng = np.random.default_rng(N + K + B)
+    raw = {2: gb.random_q4_0_blocks, 8: gb.random_q8_0_blocks, 12: gb.random_q4_k_blocks}[ggml_type](rng, N, K)
+    x = rng.standard_normal((B, K), dtype=np.float32) * rng.uniform(0.01, 100.0, (B, 1)).astype(np.float32)
+    gpu.tc_gemm_policy(2)
+    try:
+        y = (_matmul(gpu, 8, A.DTYPE_GGUF_Q8_0, raw, N, K, x) if ggml_type == 8 else _gemv(gpu, ggml_type, raw, N, K, x)).astype(np.float64)
+    finally:
+        gpu.tc_gemm_policy(1)
+    ref = x.astype(np.float64) @ q4_blocks.dequant(raw.reshape(-1), ggml_type, N, K).astype(np.float64).T
+    assert (np.linalg.norm(y - ref, axis=1) / np.linalg.norm(ref, axis=1)).max() < 5e-6
+    assert gpu.device_error() == 0
+
+
+@pytest.mark.parametrize("batch", [9, 17, 40])
+def test_batched_head_and_ragged_prefill_match_the_oracle(gpu, batch):
+    """Prompts of 1 to 70 tokens through one ragged prefill, then steps whose products and arg-max are the GEMM's."""
+    cfg = tiny_gemma3(n_layer=2, n_vocab=1000)
+    tensors = synth.build_model(cfg, gb.GGML_TYPE_Q4_0, seed=61, tied=False)
+    f32 = dequant_model(tensors)
+    lens = [1 + (23 * i) % 70 for i in range(batch)]
+    prompts = [synth.random_prompt(cfg.n_vocab, n, seed=100 + i) for i, n in enumerate(lens)]
+    eng = ADAMEngine(gpu, cfg, tensors, kv_cap=80, kv_dtype="f32", max_batch=batch)
+    try:
+        outs, _ = eng.generate_batch(prompts, GenerationConfig(max_tokens=3, **GREEDY))
+        for p, o in list(zip(prompts, outs))[:: max(1, batch // 8)]:
+            assert o == OracleDecoder(cfg, f32, kv_cap=80).generate(p, 3)[0]
+        assert gpu.device_error() == 0
+    finally:
+        eng.close()
+
+
+# Query rows per attention tile: 32 (a chunk that does not fill the GPU), 64 and 128 (it does); windows and pages whose edges
+# lie inside a cache tile; a prompt longer than one chunk of 1024 rows.
+@pytest.mark.parametrize("kv_dtype", ["f16", "f32"])
+@pytest.mark.parametrize("head_dim,n_head,n_kv,window,lens", [
+    (256, 4, 1, 0, (14, 66, 193)), (128, 2, 1, 40, (129, 3, 64)), (64, 8, 1, 0, (65, 33)), (32, 4, 4, 24, (100, 2)),
+    (64, 16, 8, 0, (700, 500)), (32, 32, 16, 100, (1300,))])
+def test_prompt_attention_tiles(gpu, head_dim, n_head, n_kv, window, lens, kv_dtype):
+    """The token after the prompts has the logits of single steps.  f32 cache: 2e-5 (both sides sum in fp32, in different
+    orders); f16: a last-bit difference can move a cached value by one f16 step."""
+    cfg = tiny_gemma3(n_layer=2, n_embd=128, n_head=n_head, n_head_kv=n_kv, head_dim=head_dim, n_ff=128, n_vocab=256, sliding_window=window)
+    tensors = synth.build_model(cfg, gb.GGML_TYPE_Q4_0, seed=62)
+    prompts = [synth.random_prompt(cfg.n_vocab, n, seed=70 + n) for n in lens]
+    eng = ADAMEngine(gpu, cfg, tensors, kv_cap=max(lens) + 8, kv_dtype=kv_dtype, max_batch=len(lens), window=window > 0)
+    try:
+        want = []
+        for p in prompts:
+            eng.begin([p], [len(p) + 2])
+            gpu.batch_begin(); eng.step(len(p) - 1, lm_head=False); eng.step(1, lm_head=True, logits=True); gpu.batch_end()
+            want.append(eng.read_logits(0))
+        eng.begin(prompts, [max(lens) + 2] * len(lens))
+        gpu.batch_begin(); eng.prefill_prompts(prompts, 0); eng.step(1, lm_head=True, logits=True); gpu.batch_end()
+        tol = 1e-3 if kv_dtype == "f16" else 2e-5
+        for b, w in enumerate(want):
+            assert np.abs(eng.read_logits(b) - w).max() <= tol * np.abs(w).max()
+        assert gpu.device_error() == 0
+    finally:
+        eng.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 65, 130])
+def test_score_equals_steps(gpu, n):
+    cfg = replace(tiny_gemma3(n_layer=2), n_vocab=512)
+    tensors = synth.build_model(cfg, gb.GGML_TYPE_Q4_0, seed=63)
+    toks = synth.random_prompt(cfg.n_vocab, n, seed=5)
+    eng = ADAMEngine(gpu, cfg, tensors, kv_cap=160, kv_dtype="f32")
+    try:
+        eng.begin([toks], [n])
+        want = []
+        for _ in range(n):
+            eng.step(1, lm_head=True, logits=True)
+            want.append(eng.read_logits(0))
+        got, want = eng.logits_trace(toks), np.stack(want)
+        assert np.abs(got - want).max() <= 2e-5 * np.abs(want).max()
+    finally:
+        eng.close()
+
+
+@pytest.mark.parametrize("n", [1, 16383, 16384, 262144, 262145, 1200000])
+def test_large_results_and_uploads(gpu, n):
+    """Around the sizes where results move to page-locked blocks and uploads leave the ring; neighbouring locs and others; arrays
+    that outlive the next call keep their values."""
+    gpu.map_create_typed(90, A.DTYPE_F32, 1, 1300000)
+    try:
+        x = np.random.default_rng(n).standard_normal(n + 7).astype(np.float32)
+        gpu.scatter_contiguous(90, 0, x)
+        locs = np.arange(n, dtype=np.uint32)
+        first = gpu.gather(90, locs + 7).view(np.float32)
+        swapped = locs.copy()
+        swapped[n // 2:] = swapped[n // 2:][::-1]
+        mixed = gpu.gather(90, swapped).view(np.float32)
+        near = locs.copy()
+        if n > 2:
+            near[n // 2] = 0                            # first and last as if they were neighbours
+        almost = gpu.gather(90, near).view(np.float32)
+        assert np.array_equal(first, x[7:]) and np.array_equal(mixed, x[swapped]) and np.array_equal(almost, x[near])
+        del first, mixed, almost
+        gc.collect()
+        kept = [gpu.gather(90, locs).view(np.float32) for _ in range(3)]
+        gpu.scatter_contiguous(90, 0, -x)
+        again = gpu.gather(90, locs).view(np.float32)
+        assert all(np.array_equal(k, x[:n]) for k in kept) and np.array_equal(again, -x[:n])
+    finally:
+        gpu.map_destroy(90)
