@@ -284,50 +284,75 @@ int launch_chain_rows(const float* h_in, const float* add_src, const float* w_po
     return ADAMAH_OK;
 }
 
+// Arg-max of rows of logits (and their soft-cap in place).  A row is cut over gridDim.x CTAs, the last of them to be done picks
+// among their winners: with one CTA per row a step of the 1B shape with a Q8_0 head took 0.686 ms, with 32 it takes 0.663.
+constexpr int AM_CTAS = 32, AM_ROWS = 256;
+__device__ float g_am_val[AM_ROWS * AM_CTAS];
+__device__ int g_am_idx[AM_ROWS * AM_CTAS];
+__device__ unsigned int g_am_done[AM_ROWS];     // CTAs of a row that are done; zero between launches
 __global__ void __launch_bounds__(1024) k_argmax_rows(float* __restrict__ logits, int V, float cap, int store_capped, int32_t* __restrict__ tok,
                                                       float* __restrict__ val, float* __restrict__ tok_f32) {
     __shared__ float sv[32]; __shared__ int si[32];
+    __shared__ bool s_last;
     pdl_launch_dependents();
     pdl_wait();
-    float* lg = logits + (size_t)blockIdx.x * V;
+    const int row = blockIdx.y, P = gridDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float* lg = logits + (size_t)row * V;
+    const int i0 = (int)((long long)V * blockIdx.x / P), i1 = (int)((long long)V * (blockIdx.x + 1) / P);
     float bv = B8_SNEG; int bi = -1;
-    for (int i = threadIdx.x; i < V; i += 1024) {
+    const bool capped = store_capped && cap > 0.f;
+#pragma unroll 4
+    for (int i = i0 + threadIdx.x; i < i1; i += 1024) {
         float v = lg[i];
+        if (capped) lg[i] = tanhf(v / cap) * cap;
         if (!(v == v)) v = B8_SNEG;
         if (better(v, i, bv, bi)) { bv = v; bi = i; }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) { sv[warp] = bv; si[warp] = bi; }
-    __syncthreads();
-    if (warp == 0) {
-        bv = sv[lane]; bi = si[lane];
+    auto warp_best = [&]() {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
             const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
             if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
         }
+    };
+    warp_best();
+    if (lane == 0) { sv[warp] = bv; si[warp] = bi; }
+    __syncthreads();
+    if (warp != 0) return;
+    bv = sv[lane]; bi = si[lane];
+    warp_best();
+    if (P > 1) {
         if (lane == 0) {
-            const int t = bi < 0 ? 0 : bi;
-            if (tok) tok[blockIdx.x] = t;
-            if (val) val[blockIdx.x] = bv;
-            if (tok_f32) tok_f32[blockIdx.x] = (float)t;
+            g_am_val[row * AM_CTAS + blockIdx.x] = bv; g_am_idx[row * AM_CTAS + blockIdx.x] = bi;
+            __threadfence();
+            s_last = atomicAdd(&g_am_done[row], 1u) == (unsigned)P - 1u;
         }
+        __syncwarp();
+        if (!s_last) return;
+        __threadfence();
+        bv = lane < P ? __ldcg(&g_am_val[row * AM_CTAS + lane]) : B8_SNEG; bi = lane < P ? __ldcg(&g_am_idx[row * AM_CTAS + lane]) : -1;
+        warp_best();
+        if (lane == 0) g_am_done[row] = 0u;
     }
-    if (store_capped && cap > 0.f)
-        for (int i = threadIdx.x; i < V; i += 1024) lg[i] = tanhf(lg[i] / cap) * cap;
+    if (lane == 0) {
+        const int t = bi < 0 ? 0 : bi;
+        if (tok) tok[row] = t;
+        if (val) val[row] = bv;
+        if (tok_f32) tok_f32[row] = (float)t;
+    }
 }
 
 int launch_argmax_rows(float* logits, int V, int rows, float cap, bool store_capped, int32_t* tok, float* val, float* tok_f32,
                        cudaStream_t st, bool pdl) {
-    launch_k(k_argmax_rows, dim3(rows), dim3(1024), 0, st, pdl, logits, V, cap, store_capped ? 1 : 0, tok, val, tok_f32);
-    count_launch();
+    for (int r0 = 0; r0 < rows; r0 += AM_ROWS) {
+        const int n = rows - r0 < AM_ROWS ? rows - r0 : AM_ROWS;
+        // 8192 logits per CTA and at most two CTAs per SM in all
+        const int P = max(1, min(min(AM_CTAS, (V + 8191) / 8192), 2 * g.sm_count / n));
+        launch_k(k_argmax_rows, dim3(P, n), dim3(1024), 0, st, pdl, logits + (size_t)r0 * V, V, cap, store_capped ? 1 : 0, tok ? tok + r0 : nullptr,
+                 val ? val + r0 : nullptr, tok_f32 ? tok_f32 + r0 : nullptr);
+        count_launch();
+    }
     return ADAMAH_OK;
 }
 

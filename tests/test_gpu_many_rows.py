@@ -133,3 +133,30 @@ def test_large_results_and_uploads(gpu, n):
         assert all(np.array_equal(k, x[:n]) for k in kept) and np.array_equal(again, -x[:n])
     finally:
         gpu.map_destroy(90)
+
+
+@pytest.mark.parametrize("N", [8192, 8193, 70001, 300000])
+def test_argmax_of_one_row_on_several_ctas(gpu, N):
+    """A Q8_0 head's winner, and of equal rows that different CTAs look at the first."""
+    K, first, second = 64, N // 3, N - 1
+    rng = np.random.default_rng(N)
+    raw = gb.random_q8_0_blocks(rng, N, K).reshape(N, -1).copy()
+    x = rng.standard_normal(K).astype(np.float32)
+    y = q4_blocks.dequant(raw.reshape(-1), 8, N, K).astype(np.float64) @ x
+    raw[first] = raw[second] = raw[int(y.argmax())].copy()
+    want = min(first, int(y.argmax()))
+    gpu.map_create_typed(91, A.DTYPE_GGUF_Q8_0, 1, N * K)
+    gpu.upload_gguf_blocks(91, 8, 0, raw.reshape(-1))
+    gpu.map_create_typed(90, A.DTYPE_F32, 1, K + 4)
+    locs = [gpu.upload_dev(np.array([v], np.uint32))[0] for v in (0, 0, K)]
+    try:
+        gpu.scatter_contiguous(90, 0, x)
+        for _ in range(2):
+            with gpu.batch():
+                gpu.map_matvec_argmax_t_xq4_dev(90, 91, locs[0], locs[1], locs[2], locs[2], locs[2], K, N)
+            assert int(gpu.gather(90, np.array([K], np.uint32)).view(np.float32)[0]) == want
+    finally:
+        for h in locs:
+            gpu.free_handle(h)
+        gpu.map_destroy(90)
+        gpu.map_destroy(91)
