@@ -6,12 +6,14 @@
 // Arithmetic.  A row of activations is scaled by a power of two (largest element near 2^15) and split into two fp16
 // terms, x = x_hi + x_lo (22 bits of every element).  A weight is rebuilt exactly as two fp16 terms, w = w_hi + w_lo:
 //   Q4_0  w = d (q - 8): w_hi = RN16(d (q - 8)), w_lo = fma(d, q - 8, -w_hi), exact because d (q - 8) has 14 bits
-//   Q4_K  w = d (sc q) - dmin m: the first product has 21 bits and splits the same way; the second is the same for 32
-//         neighbouring weights, so it becomes one more "weight" per 32 that multiplies the sum of their 32 activations
-//         (a few extra steps of K, 1/32 of the work)
+//   Q4_K  w = d sc (q - 8) + (8 d sc - dmin m): the first product has 20 bits and splits the same way; the second is the
+//         same for 32 neighbouring weights, so it becomes one more "weight" per 32 that multiplies the sum of their 32
+//         activations (a few extra steps of K, 1/32 of the work).  The codes are centred because d sc q is never negative:
+//         taken apart as d sc q and dmin m, activations with a mean make two sums of many times the result, and what
+//         the tensor core rounds off is relative to them (256 x 5376, 9 rows of N(1, 1): 3.7e-5 of the result; the test asks for 5e-6).
 //   Q8_0  w = d q: 19 bits, as Q4_0
 // and w_hi x_hi + w_lo x_hi + w_hi x_lo is accumulated over K in fp32 (w_lo x_lo lies below 2^-22 of the product).
-// Limit: |w| < 65504, what fp16 holds.
+// Limit, what fp16 holds: 8 d (Q4_0), 128 d (Q8_0), 8 d sc and 32 |8 d sc - dmin m| (Q4_K) below 65504.
 //
 // Two kernels:
 //   k_quant_rows  one CTA per activation row: the optional input chain (residual add + RMS norms, as the GEMV prologue),
@@ -181,7 +183,7 @@ __global__ void __launch_bounds__(512) k_quant_rows(const GemvArgs a, uint8_t* _
         const int i = tid + j * nt;
         const float4 f = make_float4(v[j].x * s, v[j].y * s, v[j].z * s, v[j].w * s);
         if (i < n4) put4(4 * i, f);
-        if (n_min) {                                    // sums over 32 neighbouring values (eight lanes), over 32: what Q4_K's block minimum multiplies
+        if (n_min) {                                    // sums over 32 neighbouring values (eight lanes), over 32: what Q4_K's block offset multiplies
             float t = (f.x + f.y) + (f.z + f.w);
             t += __shfl_xor_sync(0xffffffffu, t, 1);
             t += __shfl_xor_sync(0xffffffffu, t, 2);
@@ -277,6 +279,11 @@ template <bool HIGH> __device__ __forceinline__ void nib_pairs(uint32_t w, uint3
     constexpr uint32_t M = HIGH ? 0x00F000F0u : 0x000F000Fu;
     p[0] = (w & M) | 0x64006400u;
     p[1] = ((w >> 8) & M) | 0x64006400u;
+}
+// The high nibbles as 64 + q, in the mantissa of 64.0.
+__device__ __forceinline__ void nib_pairs_64(uint32_t w, uint32_t (&p)[2]) {
+    p[0] = (w & 0x00F000F0u) | 0x54005400u;
+    p[1] = ((w >> 8) & 0x00F000F0u) | 0x54005400u;
 }
 // v * d as w_hi + w_lo (v two exact small integers)
 __device__ __forceinline__ void split_h2(__half2 v, __half2 d, uint32_t& whi, uint32_t& wlo) {
@@ -381,7 +388,7 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
     [[maybe_unused]] __shared__ unsigned long long s_best[HEAD ? NT : 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = warp >> 2;
     const int S = a.S, split = S > 1 ? (int)(blockIdx.x % (uint32_t)S) : 0;     // a cluster's CTAs are neighbours along x
-    // this split's share of the steps: first those of the block minima, then those of the products
+    // this split's share of the steps: first those of the block offsets, then those of the products
     const int mn0 = split * a.n_min / S, mn1 = (split + 1) * a.n_min / S;
     const int ma0 = split * a.n_main / S, ma1 = (split + 1) * a.n_main / S;
     const int nmn = mn1 - mn0, nst = nmn + ma1 - ma0, n_steps = a.n_min + a.n_main;
@@ -818,16 +825,17 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                         tc_st8(col + 40u, wlo);
                     } else {                            // low nibbles = sub-block 2g, high nibbles = sub-block 2g + 1
                         const uint32_t code = sp >> (8 * b) & 0xFFu;
-                        const __half2 sc = __hsub2(as_h2((code * 0x10001u) | 0x64006400u), __float2half2_rn(1024.f)), off = __hmul2(sc, __float2half2_rn(-1024.f));
+                        const __half2 sc = __hsub2(as_h2((code * 0x10001u) | 0x64006400u), __float2half2_rn(1024.f)), off = __hmul2(sc, __float2half2_rn(-72.f));
 #pragma unroll
                         for (int y = 0; y < 2; ++y) {
                             const uint4 p4 = piece_at(y);
-                            const uint32_t qw[4] = {p4.x >> (4 * b), p4.y >> (4 * b), p4.z >> (4 * b), p4.w >> (4 * b)};
+                            const int up = 4 - 4 * b;
+                            const uint32_t qw[4] = {p4.x << up, p4.y << up, p4.z << up, p4.w << up};
 #pragma unroll
                             for (int x = 0; x < 4; ++x) {
-                                nib_pairs<false>(qw[x], v);
+                                nib_pairs_64(qw[x], v);
 #pragma unroll
-                                for (int p = 0; p < 2; ++p)       // sc * q, an integer below 946, exactly
+                                for (int p = 0; p < 2; ++p)       // sc * (q - 8), an integer of at most 504, exactly
                                     split_h2(__hfma2(as_h2(v[p]), sc, off), as_h2(d01), whi[2 * x + p], wlo[2 * x + p]);
                             }
                             tc_st8(col + y * 8u, whi);
@@ -836,7 +844,7 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                     }
                 }
             } else if (WT == WT_Q4_K && st < nmn) {
-                // a step of block minima: -32 dmin m of 64 sub-blocks (the image holds the sums over 32 activations / 32)
+                // a step of block offsets: 32 (8 d sc - dmin m) of 64 sub-blocks (the image holds the sums over 32 activations / 32)
                 const int sb0 = (mn0 + st) * 8, n_sb = a.units >> 3;
                 const uint4* src = w.q + (size_t)row_of(n_of(item_of(c.i)), row) * rpu;
 #pragma unroll 1
@@ -846,12 +854,14 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                     for (int e = 0; e < 2; ++e) {
                         const int sb = sb0 + 2 * b + e;
                         const uint4 h = __ldg(src + (size_t)min(sb, n_sb - 1) * 9);
-                        const float dm = sb < n_sb ? -32.f * __half2float(__ushort_as_half((unsigned short)(h.x >> 16))) : 0.f;
+                        const bool in = sb < n_sb;
+                        const float dm = in ? -32.f * __half2float(__ushort_as_half((unsigned short)(h.x >> 16))) : 0.f;
+                        const float d8 = in ? 256.f * __half2float(__ushort_as_half((unsigned short)(h.x & 0xFFFFu))) : 0.f;
 #pragma unroll
                         for (int gq = 0; gq < 4; ++gq) {
                             uint32_t sp, mp;
                             q4k_codes(h, gq, sp, mp);
-                            const float v0 = dm * (float)(mp & 0xFFu), v1 = dm * (float)(mp >> 8);
+                            const float v0 = fmaf(d8, (float)(sp & 0xFFu), dm * (float)(mp & 0xFFu)), v1 = fmaf(d8, (float)(sp >> 8), dm * (float)(mp >> 8));
                             const __half2 h2 = __floats2half2_rn(v0, v1);
                             const float2 f2 = __half22float2(h2);
                             whi[4 * e + gq] = as_u32(h2);

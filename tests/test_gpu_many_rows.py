@@ -42,6 +42,33 @@ def test_gemm_tiles(gpu, ggml_type, N, K, B):
     assert gpu.device_error() == 0
 
 
+def _gemm_error(gpu, ggml_type, raw, N, K, x):
+    """Errors against float64, as 2-norms over the result's: of the GEMM, and of the GEMV that takes its place where it is refused."""
+    ref = x.astype(np.float64) @ q4_blocks.dequant(raw.reshape(-1), ggml_type, N, K).astype(np.float64).T
+    errors = []
+    for policy in (2, 0):
+        before = gpu.tc_gemm_count()
+        gpu.tc_gemm_policy(policy)
+        try:
+            y = _gemv(gpu, ggml_type, raw, N, K, x, tile=N % 16 == 0 and K % 64 == 0).astype(np.float64)
+        finally:
+            gpu.tc_gemm_policy(1)
+        assert (gpu.tc_gemm_count() > before) == (policy == 2)
+        errors.append(np.linalg.norm(y - ref) / np.linalg.norm(ref))
+    return errors
+
+
+@pytest.mark.parametrize("N,K,B", [(256, 5376, 9), (129, 2304, 40), (256, 21504, 64), (384, 5376, 130)])
+def test_gemm_q4_k_activations_with_a_mean(gpu, N, K, B):
+    """Q4_K codes are not negative and a block's minimum is taken off afterwards: with activations that have a mean, the two
+    parts are some 60 times the result here.  Same bound as for the tiles: the sums must not be larger than the result."""
+    rng = np.random.default_rng(K + B)
+    raw = rng.integers(0, 256, (N * K // 256, 144), dtype=np.uint8)
+    d = ((0.5 + rng.random((len(raw), 1))) * 1e-4).astype(np.float16)
+    raw[:, 0:2], raw[:, 2:4] = d.view(np.uint8), (d * np.float16(7.5)).view(np.uint8)
+    assert _gemm_error(gpu, 12, raw, N, K, rng.standard_normal((B, K), dtype=np.float32) + np.float32(1))[0] < 5e-6
+
+
 @pytest.mark.parametrize("batch", [9, 17, 40])
 def test_batched_head_and_ragged_prefill_match_the_oracle(gpu, batch):
     """Prompts of 1 to 70 tokens through one ragged prefill, then steps whose products and arg-max are the GEMM's."""
