@@ -321,9 +321,14 @@ __device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, u
 //                246 (NT = 128: 878 and 772, the rate of the instructions).  One elected lane issues, but the whole warp
 //                walks the loop: inside a one-lane branch it took half as long again.
 //   rounding     The tensor core rounds its running sum towards zero, an error that grows with the number of instructions
-//                added up (measured: 5e-9 of the result each).  So the cross terms, 2^-11 of the result, have D2 to
-//                themselves, and every `period` stages D1 is added to registers and restarted.  Relative error of a
-//                1152 x 6912 product: 6.1e-6 with one accumulator for all of K, 5e-7 with this.
+//                added up.  So the cross terms, 2^-11 of the result, have D2 to themselves, and every two (NT = 128: three)
+//                steps D1 is added to registers and restarted.  Relative error of a 1152 x 6912 product by the steps
+//                between: all of K 6.1e-6, eight 5.8e-7, four 3.4e-7, three 2.8e-7, two 2.1e-7; the GEMV, which adds
+//                integers up within a block, has 2.9e-7 to 4.7e-7, and two or three steps stay below it for every size.
+//                Up to NT = 64 a stage has a pair D1 | D2 of its own and the reader's arrivals count among those that
+//                fill the stage, so the issuing warp waits for nothing more.  At NT = 128 there is room for one pair:
+//                the stage that restarts D1 issues its products for D2 first, two thirds of its time, while D1 is
+//                read.  32 prompts x 512 at the 1B shape: 141 ms with eight steps, 157 with two and no second pair, 148 so.
 //   work split   Three ways, by an estimate of their times (launch_rows).  Whole tiles, dealt in turn.  Or all stages
 //                of all tiles in a row, dealt out evenly: a tile that several CTAs share is added up by the one that ends
 //                last (atomic ticket, partial sums in a workspace), in the order of K; 168 tiles on 148 SMs take 1.14 tiles'
@@ -337,7 +342,6 @@ __device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, u
 // The request for shared memory is at least 120 KB, so that an SM never holds two of these CTAs: one that waits for
 // tensor memory held by a cluster that waits for it would never end.
 constexpr int TC_SMEM_MIN = 120 * 1024;
-constexpr int TC_PERIOD = 8;                            // most steps (64 values of K) accumulated in D1 before it is read out
 struct TcGemm {
     WeightRef w0, w1;
     float* y; int ldy;
@@ -345,13 +349,14 @@ struct TcGemm {
     int N, units, B;                                    // units = K / 32
     int pair, swiglu;                                   // gate / up tiles, and which activation
     int n_min, n_main, tiles_n, items;                  // items = tiles_n (weight tiles) * tiles of NT rows
-    int S, period, shared;                              // K splits; stages per accumulation period; whether CTAs share tiles
+    int S, shared;                                      // K splits; whether CTAs share tiles
     float* part; unsigned int* tickets;                 // shared tiles: per CTA the sums of its first and last one; arrivals, by the CTA in which a tile begins
     unsigned long long* best; unsigned int* ticket;     // arg-max: one key per activation row (0 between launches), CTAs that are done
     int* out_tok; float *out_val, *out_tok_f32, softcap;
 };
 template <int WT, int NT> struct TcGeo {
     static constexpr int SP = NT == 128 ? 1 : 2, NS = NT == 128 ? 4 : 2;     // steps per stage, stages
+    static constexpr int BANKS = NT == 128 ? 1 : NS, PERIOD = NT == 128 ? 3 : 1;        // pairs of accumulators D1 | D2; stages between two read-outs
     static constexpr int GROUPS = NT == 128 ? 3 : 4, THREADS = (2 + GROUPS) * 128;     // warpgroups that rebuild weights, a step each in turn
     static constexpr int REG_LOW = 40, REG_READ = NT == 128 ? 200 : 120, REG_MAKE = 80;    // sum = what the CTA is launched with
     static constexpr int R = WT == WT_Q8_0 && NT == 128 ? 3 : 4;             // weight ring: tiles ahead per warp
@@ -362,7 +367,7 @@ template <int WT, int NT> struct TcGeo {
     static constexpr int XCOLS = NT < 32 ? NT : 32;                          // so many columns at a time
     static constexpr int SMEM_USED = XCH + XCOLS * 512 + 1024;
     static constexpr int SMEM = SMEM_USED > TC_SMEM_MIN ? SMEM_USED : TC_SMEM_MIN;
-    static_assert(SMEM <= 226 * 1024 && 2 * NT + 64 * NS * SP <= 512 && GROUPS % SP == 0 && GROUPS <= NS * SP, "shared or tensor memory");
+    static_assert(SMEM <= 226 * 1024 && BANKS * 2 * NT + 64 * NS * SP <= 512 && GROUPS % SP == 0 && GROUPS <= NS * SP, "shared or tensor memory");
     static_assert(REG_LOW + REG_READ + GROUPS * REG_MAKE <= 65536 / THREADS / 8 * 8 * (2 + GROUPS), "registers");
 };
 __device__ __forceinline__ bool elect_one() {
@@ -403,7 +408,7 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
     auto m_of = [&](int item) { return item / a.tiles_n * NT; };                // first activation row and weight tile of an item
     auto n_of = [&](int item) { return item % a.tiles_n; };
     if (tid == 0) {
-        for (int i = 0; i < NS; ++i) { mbar_init(&full[i], 4 * SP + 1); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < NS; ++i) { mbar_init(&full[i], 4 * SP + 1 + (G::BANKS > 1 ? 4 : 0)); mbar_init(&empty[i], 1); }
         mbar_init(&d_full, 1); mbar_init(&d_empty, 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -413,7 +418,7 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
-    constexpr uint32_t A_COL = 2 * NT;                  // first column of the weight ring
+    constexpr uint32_t A_COL = G::BANKS * 2 * NT;       // first column of the weight ring
     bool dead = false;
     auto wait_on = [&](uint64_t* bar, uint32_t parity) {
         if (!dead && !mbar_wait(bar, parity)) { dead = true; atomicOr(a.err, DEVERR_WAIT); }
@@ -491,41 +496,63 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
             for (uint32_t i = n > (uint32_t)NS ? n - NS : 0; i < n; ++i) mbar_wait(&full[i % NS], (i / NS) & 1u);
         } else if (warp == 0) {
             // ---- products ----
-            const uint32_t b_lo = (smem_u32(smB) & 0x3FFFFu) >> 4, d1 = tmem, d2 = tmem + NT;
+            const uint32_t b_lo = (smem_u32(smB) & 0x3FFFFu) >> 4;
             auto desc = [&](uint32_t lo) { return ((uint64_t)TC_DESC_HI << 32) | lo; };
             uint32_t s = 0, par = 0, periods = 0;
             for (int q = q0; q < q1;) {
                 const int j0 = q % spi, j1 = min(spi, j0 + q1 - q);
                 q += j1 - j0;
-                int left = 0;                           // stages left in the period
                 for (int j = j0; j < j1; ++j) {
-                    const bool fresh = left == 0;
-                    if (fresh) {                        // D of the period before must have been read
-                        if (periods) wait_on(&d_empty, (periods - 1u) & 1u);
-                        left = min(a.period, j1 - j);
-                        ++periods;
-                    }
-                    --left;
-                    wait_on(&full[s], par);
-                    tc_fence_after();
-                    if (lead) {
+                    if constexpr (G::BANKS > 1) {       // a stage has accumulators of its own
+                        wait_on(&full[s], par);
+                        tc_fence_after();
+                        if (lead) {
+                            const uint32_t d1 = tmem + s * 2 * NT, d2 = d1 + NT;
 #pragma unroll
-                        for (int t = 0; t < SP; ++t) {
-                            if (SP == 2 && t == 1 && 2 * j + 1 >= nst) break;
-                            const uint32_t slot = s * SP + t, ac = tmem + A_COL + slot * 64u, bh = b_lo + slot * (uint32_t)(G::BSTEP / 16);
-                            if (t == 0 && fresh && j > j0) {    // D1 starts again, D2 goes on
-                                tc_mma_ts(d1, ac, desc(bh), TC_IDESC<NT>, 0u);
-                                tc_mma_ts(d2, ac, desc(bh + NT * 8), TC_IDESC<NT>, 1u);
-                            } else tc_mma_ts(d1, ac, desc(bh), TC_IDESC<2 * NT>, (t > 0 || j > j0) ? 1u : 0u);
-                            tc_mma_ts(d2, ac + 32u, desc(bh), TC_IDESC<NT>, 1u);
+                            for (int t = 0; t < SP; ++t) {
+                                if (t == 1 && 2 * j + 1 >= nst) break;
+                                const uint32_t slot = s * SP + t, ac = tmem + A_COL + slot * 64u, bh = b_lo + slot * (uint32_t)(G::BSTEP / 16);
 #pragma unroll
-                            for (uint32_t q = 1; q < 4; ++q) {
-                                tc_mma_ts(d1, ac + q * 8u, desc(bh + q * 2u), TC_IDESC<2 * NT>, 1u);
+                                for (uint32_t q = 0; q < 4; ++q) {
+                                    tc_mma_ts(d1, ac + q * 8u, desc(bh + q * 2u), TC_IDESC<2 * NT>, t + q > 0 ? 1u : 0u);
+                                    tc_mma_ts(d2, ac + 32u + q * 8u, desc(bh + q * 2u), TC_IDESC<NT>, 1u);
+                                }
+                            }
+                            tc_commit(&empty[s]);       // for the reading warpgroup too
+                        }
+                    } else {
+                        const bool fresh = (j - j0) % G::PERIOD == 0;   // D1 starts again; D2 only with an item
+                        if (j == j0 && periods) wait_on(&d_empty, (periods - 1u) & 1u);
+                        wait_on(&full[s], par);
+                        tc_fence_after();
+                        const uint32_t d1 = tmem, d2 = tmem + NT, ac = tmem + A_COL + s * 64u, bh = b_lo + s * (uint32_t)(G::BSTEP / 16);
+                        if (fresh && j > j0) {          // the products for D2 while D1 is read
+                            if (lead) {
+#pragma unroll
+                                for (uint32_t q = 0; q < 4; ++q) {
+                                    tc_mma_ts(d2, ac + q * 8u, desc(bh + NT * 8 + q * 2u), TC_IDESC<NT>, 1u);
+                                    tc_mma_ts(d2, ac + 32u + q * 8u, desc(bh + q * 2u), TC_IDESC<NT>, 1u);
+                                }
+                            }
+                            __syncwarp();
+                            wait_on(&d_empty, (periods - 1u) & 1u);
+                            tc_fence_after();
+                            if (lead) {
+#pragma unroll
+                                for (uint32_t q = 0; q < 4; ++q) tc_mma_ts(d1, ac + q * 8u, desc(bh + q * 2u), TC_IDESC<NT>, q > 0 ? 1u : 0u);
+                            }
+                        } else if (lead) {
+#pragma unroll
+                            for (uint32_t q = 0; q < 4; ++q) {
+                                tc_mma_ts(d1, ac + q * 8u, desc(bh + q * 2u), TC_IDESC<2 * NT>, (q > 0 || j > j0) ? 1u : 0u);
                                 tc_mma_ts(d2, ac + 32u + q * 8u, desc(bh + q * 2u), TC_IDESC<NT>, 1u);
                             }
                         }
-                        tc_commit(&empty[s]);
-                        if (left == 0) tc_commit(&d_full);
+                        periods += fresh ? 1u : 0u;
+                        if (lead) {
+                            tc_commit(&empty[s]);
+                            if ((j - j0) % G::PERIOD == G::PERIOD - 1 || j == j1 - 1) tc_commit(&d_full);
+                        }
                     }
                     __syncwarp();
                     if (++s == (uint32_t)NS) { s = 0; par ^= 1u; }
@@ -539,7 +566,8 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
         reg_inc<G::REG_READ>();
         pdl_wait();
         float* xch = reinterpret_cast<float*>(sm + G::XCH);
-        uint32_t par = 0;
+        uint32_t nth = 0;                               // accumulation period
+        if constexpr (G::BANKS > 1) { if (lane < NS) mbar_arrive(&full[lane]); }        // all accumulators are free
         if constexpr (HEAD) {
             if (tid - 128 < NT) s_best[tid - 128] = 0;
             asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -554,15 +582,16 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
         };
         for (int q = q0; q < q1;) {
             const int i0 = q / spi, j0 = q - i0 * spi, j1 = min(spi, j0 + q1 - q), item = item_of(i0), tn = n_of(item), m0 = m_of(item);
-            const int np = (j1 - j0 + a.period - 1) / a.period;                         // accumulation periods
+            const int np = (j1 - j0 + G::PERIOD - 1) / G::PERIOD;                       // accumulation periods
             q += j1 - j0;
             float acc[NT];
 #pragma unroll
             for (int c = 0; c < NT; ++c) acc[c] = 0.f;
 #pragma unroll 1
-            for (int p = 0; p < np; ++p) {
-                wait_on(&d_full, par);
-                par ^= 1u;
+            for (int p = 0; p < np; ++p, ++nth) {
+                const uint32_t bank = nth % G::BANKS;
+                if constexpr (G::BANKS > 1) wait_on(&empty[bank], (nth / G::BANKS) & 1u);
+                else wait_on(&d_full, nth & 1u);
                 tc_fence_after();
                 auto take = [&](uint32_t col) {         // the tensor core may wait for this: few round trips
                     constexpr int CH = NT < 32 ? NT : 32;
@@ -577,10 +606,10 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                     }
                 };
 #pragma unroll 1
-                for (int h = 0; h < (p == np - 1 ? 2 : 1); ++h) take(tlane + h * NT);
+                for (int h = 0; h < (G::BANKS > 1 || p == np - 1 ? 2 : 1); ++h) take(tlane + bank * 2 * NT + h * NT);
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&d_empty);
+                if (lane == 0) mbar_arrive(G::BANKS > 1 ? &full[bank] : &d_empty);
             }
             if (S > 1) {                                // one item per cluster, and the activation ring is drained: it becomes the exchange
                 float* ex = reinterpret_cast<float*>(smB);
@@ -992,7 +1021,6 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
     t.w0 = a.w0; t.w1 = a.w1; t.y = a.y; t.ldy = a.ldy; t.img = g_tc.img; t.inv = g_tc.inv; t.err = g.dev_err;
     t.N = a.N; t.units = a.K / 32; t.B = a.B; t.swiglu = a.epi == EPI_SWIGLU;
     t.n_min = n_min; t.n_main = n_main; t.S = S;
-    t.period = TC_PERIOD / sp;
     t.tiles_n = tiles_n;
     t.items = (int)items;
     t.part = g_tc.part; t.tickets = g_tc.tickets; t.shared = shared ? 1 : 0;

@@ -69,6 +69,17 @@ def test_gemm_q4_k_activations_with_a_mean(gpu, N, K, B):
     assert _gemm_error(gpu, 12, raw, N, K, rng.standard_normal((B, K), dtype=np.float32) + np.float32(1))[0] < 5e-6
 
 
+@pytest.mark.parametrize("ggml_type,N,K,B", [(2, 512, 1152, 9), (2, 512, 1152, 33), (2, 256, 6912, 64), (2, 512, 1152, 65), (12, 256, 5376, 16), (12, 256, 5376, 40),
+                                             (12, 256, 21504, 129)])
+def test_gemm_is_as_close_as_the_gemv(gpu, ggml_type, N, K, B):
+    """The tensor core rounds its sums towards zero, so the GEMM moves them to registers every few additions; it has to end no
+    further from the exact product than the GEMV (exact integer sums per block) whose calls it takes."""
+    rng = np.random.default_rng(N + K + B)
+    raw = {2: gb.random_q4_0_blocks, 12: gb.random_q4_k_blocks}[ggml_type](rng, N, K)
+    gemm, gemv = _gemm_error(gpu, ggml_type, raw, N, K, rng.standard_normal((B, K), dtype=np.float32))
+    assert gemm <= gemv
+
+
 @pytest.mark.parametrize("batch", [9, 17, 40])
 def test_batched_head_and_ragged_prefill_match_the_oracle(gpu, batch):
     """Prompts of 1 to 70 tokens through one ragged prefill, then steps whose products and arg-max are the GEMM's."""
