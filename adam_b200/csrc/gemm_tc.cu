@@ -923,9 +923,11 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
 // 1.22 against 1.15; 12: 1.35 against 1.16); where they fill the GPU it costs their number (27B shape with every matrix on
 // one path, 4 rows: 1.62 against 2.02 ms, 6: 2.5 against 2.04, 12: 3.9 against 2.08).  An LM head of a narrow model is bound by
 // rebuilding weights here (262144 x 1152: 75 us whatever the rows, the GEMV 43 us at 4 and 71 at 8).
-// Without a row-tiled copy a GEMV takes one launch per four rows (7 us each), and Q8_0 / Q5_0 have no tensor-core GEMV.
+// Without a row-tiled copy a GEMV takes one launch per four rows (7 us each).  Q8_0 / Q5_0 have no tensor-core GEMV; their
+// product in fp32 is 1.2e-7 from the exact one, closer than the 2.1e-7 of this kernel, so a product that is asked for by itself
+// stays there, and the Q8_0 heads of a model come here, whose logits carry 2e-6 from the layers.
 static int tc_rows_from(int wtype, const GemvArgs& a, bool pair, bool tiled) {
-    if (wtype == WT_Q8_0) return 4;
+    if (wtype == WT_Q8_0) return a.epi == EPI_ARGMAX ? 4 : 1 << 30;
     if (!tiled) return 5;
     const double bytes = (double)a.N * a.K * 0.5625 * (pair ? 2 : 1);
     if (a.epi == EPI_ARGMAX && a.K < 4096) return 9;

@@ -80,6 +80,18 @@ def test_gemm_is_as_close_as_the_gemv(gpu, ggml_type, N, K, B):
     assert gemm <= gemv
 
 
+@pytest.mark.parametrize("B", [3, 4, 9, 64, 130])
+def test_q8_0_products_are_fp32_sums(gpu, B):
+    """A Q8_0 product of many rows: 1152 / 32 additions per lane and five between lanes, each rounded to nearest, end about
+    2^-24 * sqrt(41 / 3) * 2/3 = 1.5e-7 from the exact product."""
+    rng = np.random.default_rng(B)
+    N, K = 1024, 1152
+    raw, x = gb.random_q8_0_blocks(rng, N, K), rng.standard_normal((B, K), dtype=np.float32)
+    y = _matmul(gpu, 8, A.DTYPE_GGUF_Q8_0, raw, N, K, x).astype(np.float64)
+    ref = x.astype(np.float64) @ q4_blocks.dequant(raw.reshape(-1), 8, N, K).astype(np.float64).T
+    assert np.linalg.norm(y - ref) < 1.5e-7 * np.linalg.norm(ref)
+
+
 @pytest.mark.parametrize("batch", [9, 17, 40])
 def test_batched_head_and_ragged_prefill_match_the_oracle(gpu, batch):
     """Prompts of 1 to 70 tokens through one ragged prefill, then steps whose products and arg-max are the GEMM's."""
