@@ -1699,8 +1699,8 @@ extern "C" int adam_b200_decoder_prefill_ragged(uint32_t id, const uint32_t* n_t
 // positions go through the layers together like a prompt, then the LM head runs over the chunk's rows, and the logits of
 // one group of rows travel to the host while the next is computed.  Bound by the copy (1 MB per position at the 1B shape)
 // and the latency of the layers' kernels.
-// Leaves the decoder as n_tokens steps would: positions, log, current token, and the last position's rows in the buffers
-// that adam_b200_decoder_read_buffer reads.
+// Leaves the decoder as n_tokens steps with logits would: positions, log, current token, and the last position's logits and
+// rows where adam_b200_decoder_read_logits and adam_b200_decoder_read_buffer read them.
 extern "C" int adam_b200_decoder_score(uint32_t id, uint32_t n_tokens, float* out) {
     Decoder* D = get_dec(id);
     if (!D) return ADAMAH_ERR_NOT_FOUND;
@@ -1742,6 +1742,8 @@ extern "C" int adam_b200_decoder_score(uint32_t id, uint32_t n_tokens, float* ou
     }
     if (rc == ADAMAH_OK) {
         enqueue_prefill_end(D);
+        const float* last = D->score_logits + ((size_t)((n_group - 1) & 1u) * GROUP + in_group) * d.n_vocab;
+        cudaMemcpyAsync(D->logits, last, (size_t)d.n_vocab * 4, cudaMemcpyDeviceToDevice, g.stream);
         cudaMemcpyAsync(D->cur_tok, tok + in_group, 4, cudaMemcpyDeviceToDevice, g.stream);
         cudaMemcpyAsync(D->cur_val, val + in_group, 4, cudaMemcpyDeviceToDevice, g.stream);
         const uint32_t q_dim = d.n_head * d.head_dim, qkv_ld = q_dim + 2 * d.n_head_kv * d.head_dim;

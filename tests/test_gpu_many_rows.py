@@ -157,6 +157,39 @@ def test_score_equals_steps(gpu, n):
         eng.close()
 
 
+@pytest.mark.parametrize("n,embd_type", [(1, None), (64, None), (65, 8), (130, None)])
+def test_score_leaves_the_decoder_as_steps_do(gpu, n, embd_type):
+    """Logits, token, position, log and last rows after scoring, and the step that follows, are those of n single steps."""
+    cfg = replace(tiny_gemma3(n_layer=2), n_vocab=512)
+    tensors = synth.build_model(cfg, gb.GGML_TYPE_Q4_0, seed=64, embd_type=embd_type)
+    toks = synth.random_prompt(cfg.n_vocab, n, seed=6)
+    eng = ADAMEngine(gpu, cfg, tensors, kv_cap=160, kv_dtype="f32")
+
+    def state():
+        pos, tok = eng.read_state()
+        return int(pos[0]), int(tok[0]), eng.read_log(0, 1, n).tolist(), eng.read_logits(0), eng.read_buffer(0, cfg.n_embd)
+
+    try:
+        seen = []
+        for scored in (False, True):
+            eng.begin([synth.random_prompt(cfg.n_vocab, 3, seed=7)], [4])       # other logits in the buffers beforehand
+            eng.step(3, lm_head=True, logits=True)
+            eng.begin([toks], [n + 2])
+            if scored:
+                eng._score(n, True)
+            else:
+                eng.step(n, lm_head=True, logits=True)
+            after = state()
+            eng.step(1, lm_head=True, logits=True)
+            seen.append((after, state()))
+        for (p0, t0, l0, y0, h0), (p1, t1, l1, y1, h1) in zip(*seen):
+            assert (p0, t0, l0) == (p1, t1, l1)
+            assert np.abs(y0 - y1).max() <= 2e-5 * np.abs(y0).max() and np.abs(h0 - h1).max() <= 2e-5 * np.abs(h0).max()
+        assert gpu.device_error() == 0
+    finally:
+        eng.close()
+
+
 @pytest.mark.parametrize("n", [1, 16383, 16384, 262144, 262145, 1200000])
 def test_large_results_and_uploads(gpu, n):
     """Around the sizes where results move to page-locked blocks and uploads leave the ring; neighbouring locs and others; arrays
