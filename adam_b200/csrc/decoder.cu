@@ -65,7 +65,9 @@ struct Decoder {
     // chunked prefill: what the rows of all chunks are (device copy and pinned source of one call; see PrefillPlan)
     uint8_t *plan, *plan_pin; size_t plan_cap; cudaEvent_t plan_read;
     std::vector<PrefillChunk> chunks; const int32_t* plan_n;
-    float* score_logits; cudaEvent_t score_ev[4]; cudaStream_t score_copy;      // adam_b200_decoder_score: two groups of rows of logits, and their copies to the host
+    // adam_b200_decoder_score: two groups of score_rows rows of logits (NULL: none fit, D->logits takes one at a time), the
+    // winners of a group, and the copies to the host
+    float* score_logits; int32_t* score_tok; uint32_t score_rows; cudaEvent_t score_ev[4]; cudaStream_t score_copy;
     uint32_t rows_cap;          // rows the activation buffers hold
     std::vector<uint32_t> hpos, hplen, hres;   // host mirror of positions, prompt lengths and reserved tokens (argument checks)
     std::vector<int32_t> hbt;            // host mirror of the block table
@@ -685,6 +687,12 @@ static void free_graphs(Decoder* D) {
     free_token_kernel(D);
 }
 
+static void score_release(Decoder* D) {
+    cudaFree(D->score_logits); cudaFree(D->score_tok);
+    for (cudaEvent_t& e : D->score_ev) if (e) { cudaEventDestroy(e); e = nullptr; }
+    if (D->score_copy) cudaStreamDestroy(D->score_copy);
+    D->score_logits = nullptr; D->score_tok = nullptr; D->score_copy = nullptr; D->score_rows = 0;
+}
 static void destroy(Decoder* D) {
     cudaStreamSynchronize(g.stream);
     free_graphs(D);
@@ -696,9 +704,7 @@ static void destroy(Decoder* D) {
     for (void* p : ptrs) cudaFree(p);
     cudaFreeHost(D->plan_pin);
     if (D->plan_read) cudaEventDestroy(D->plan_read);
-    cudaFree(D->score_logits);
-    for (cudaEvent_t e : D->score_ev) if (e) cudaEventDestroy(e);
-    if (D->score_copy) cudaStreamDestroy(D->score_copy);
+    score_release(D);
     delete D;
 }
 
@@ -1695,6 +1701,28 @@ extern "C" int adam_b200_decoder_prefill_ragged(uint32_t id, const uint32_t* n_t
     return rc;
 }
 
+// What scoring needs besides the decoder's buffers.  Where two groups of 64 rows of logits (134 MB at the 1B shape) would leave
+// less than 64 MB on the device, smaller groups, and at last the logits buffer that every decoder has.
+static int score_prepare(Decoder* D) {
+    const adam_b200_decoder_desc& d = D->d;
+    constexpr uint32_t ROWS = 64;                       // rows per LM-head call: one arg-max scratch
+    DCU(cudaMalloc((void**)&D->score_tok, ROWS * 8));
+    for (cudaEvent_t& e : D->score_ev) DCU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    DCU(cudaStreamCreateWithFlags(&D->score_copy, cudaStreamNonBlocking));
+    uint32_t rows = ROWS;
+    for (; rows; rows /= 2) {
+        const size_t need = (size_t)2 * rows * d.n_vocab * 4;
+        size_t left = 0, total = 0;
+        DCU(cudaMemGetInfo(&left, &total));
+        if (left < need + (64u << 20)) continue;
+        if (cudaMalloc((void**)&D->score_logits, need) == cudaSuccess) break;
+        cudaGetLastError();
+        D->score_logits = nullptr;
+    }
+    D->score_rows = rows ? rows : std::min(ROWS, d.max_batch);
+    return ADAMAH_OK;
+}
+
 // Logits after every one of the next n_tokens prompt tokens of the single active sequence (a text under evaluation): the
 // positions go through the layers together like a prompt, then the LM head runs over the chunk's rows, and the logits of
 // one group of rows travel to the host while the next is computed.  Bound by the copy (1 MB per position at the 1B shape)
@@ -1710,54 +1738,55 @@ extern "C" int adam_b200_decoder_score(uint32_t id, uint32_t n_tokens, float* ou
     if (d.tp_size > 1) return fail(ADAMAH_ERR_INVALID, "decoder_score: not available with tensor parallelism");
     int rc = check_prefill(D, &n_tokens, "decoder_score");
     if (rc || (rc = plan_prefill(D, &n_tokens))) return rc;
-    constexpr uint32_t GROUP = 64;                      // rows per LM-head call: one arg-max scratch, one buffer of logits
-    if (!D->score_logits) {
-        DCU(cudaMalloc((void**)&D->score_logits, (size_t)2 * GROUP * d.n_vocab * 4 + 2 * GROUP * 8));
-        for (cudaEvent_t& e : D->score_ev) DCU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        DCU(cudaStreamCreateWithFlags(&D->score_copy, cudaStreamNonBlocking));
-    }
-    int32_t* tok = (int32_t*)(D->score_logits + (size_t)2 * GROUP * d.n_vocab);
-    float* val = (float*)(tok + GROUP);
     { float* pv; int* pi; unsigned int* tk; if ((rc = argmax_scratch(&pv, &pi, &tk))) return rc; }
+    if (!D->score_rows && (rc = score_prepare(D))) { score_release(D); return rc; }
+    const uint32_t GROUP = D->score_rows, halves = D->score_logits ? 2 : 1;
+    float* const base = D->score_logits ? D->score_logits : D->logits;
+    int32_t* tok = D->score_tok;
+    float* val = (float*)(tok + GROUP);
+    cudaError_t err = cudaSuccess;
+    auto ok = [&](cudaError_t e) { if (err == cudaSuccess) err = e; };
     uint32_t done = 0, n_group = 0, last_row = 0, in_group = 0;
     const uint32_t p0 = D->hpos[0];
     g.pdl = pdl_allowed();
     for (const PrefillChunk& c : D->chunks) {
         for (uint32_t part = 0; part < 2 * d.n_layer && rc == ADAMAH_OK; ++part) rc = enqueue_prefill_part(D, c, part);
         for (uint32_t r0 = 0; r0 < c.n_rows && rc == ADAMAH_OK; r0 += GROUP, ++n_group) {
-            const uint32_t m = std::min(GROUP, c.n_rows - r0), half = n_group & 1u;
-            float* lg = D->score_logits + (size_t)half * GROUP * d.n_vocab;
-            if (n_group >= 2) cudaStreamWaitEvent(g.stream, D->score_ev[2 + half], 0);      // the half's copy has left
+            const uint32_t m = std::min(GROUP, c.n_rows - r0), half = n_group % halves;
+            float* lg = base + (size_t)half * GROUP * d.n_vocab;
+            if (n_group >= halves) ok(cudaStreamWaitEvent(g.stream, D->score_ev[2 + half], 0));     // the half's copy has left
             if ((rc = enqueue_head(D, r0, m, lg, tok, val))) break;
             // logged as the token of the position behind, as a step's
             const uint32_t fits = p0 + done + 1 < d.kv_cap ? std::min(m, d.kv_cap - p0 - done - 1) : 0;
-            if (fits) cudaMemcpyAsync(D->gen_log + p0 + done + 1, tok, (size_t)fits * 4, cudaMemcpyDeviceToDevice, g.stream);
-            cudaEventRecord(D->score_ev[half], g.stream);
-            cudaStreamWaitEvent(D->score_copy, D->score_ev[half], 0);
-            cudaMemcpyAsync(out + (size_t)done * d.n_vocab, lg, (size_t)m * d.n_vocab * 4, cudaMemcpyDeviceToHost, D->score_copy);
-            cudaEventRecord(D->score_ev[2 + half], D->score_copy);
+            if (fits) ok(cudaMemcpyAsync(D->gen_log + p0 + done + 1, tok, (size_t)fits * 4, cudaMemcpyDeviceToDevice, g.stream));
+            ok(cudaEventRecord(D->score_ev[half], g.stream));
+            ok(cudaStreamWaitEvent(D->score_copy, D->score_ev[half], 0));
+            ok(cudaMemcpyAsync(out + (size_t)done * d.n_vocab, lg, (size_t)m * d.n_vocab * 4, cudaMemcpyDeviceToHost, D->score_copy));
+            ok(cudaEventRecord(D->score_ev[2 + half], D->score_copy));
             done += m; last_row = r0 + m - 1; in_group = m - 1;
         }
-        if (rc) break;
+        if (rc || err != cudaSuccess) break;
     }
-    if (rc == ADAMAH_OK) {
+    if (rc == ADAMAH_OK && err == cudaSuccess) {
         enqueue_prefill_end(D);
-        const float* last = D->score_logits + ((size_t)((n_group - 1) & 1u) * GROUP + in_group) * d.n_vocab;
-        cudaMemcpyAsync(D->logits, last, (size_t)d.n_vocab * 4, cudaMemcpyDeviceToDevice, g.stream);
-        cudaMemcpyAsync(D->cur_tok, tok + in_group, 4, cudaMemcpyDeviceToDevice, g.stream);
-        cudaMemcpyAsync(D->cur_val, val + in_group, 4, cudaMemcpyDeviceToDevice, g.stream);
+        const float* last = base + ((size_t)((n_group - 1) % halves) * GROUP + in_group) * d.n_vocab;
+        if (halves == 1) ok(cudaStreamWaitEvent(g.stream, D->score_ev[2], 0));      // the row is overwritten in place
+        if (last != D->logits) ok(cudaMemcpyAsync(D->logits, last, (size_t)d.n_vocab * 4, cudaMemcpyDeviceToDevice, g.stream));
+        ok(cudaMemcpyAsync(D->cur_tok, tok + in_group, 4, cudaMemcpyDeviceToDevice, g.stream));
+        ok(cudaMemcpyAsync(D->cur_val, val + in_group, 4, cudaMemcpyDeviceToDevice, g.stream));
         const uint32_t q_dim = d.n_head * d.head_dim, qkv_ld = q_dim + 2 * d.n_head_kv * d.head_dim;
         float* bufs[5] = {D->hbuf[0], D->qkv, D->attn_out, D->proj, D->act};
         const uint32_t lds[5] = {d.n_embd, qkv_ld, q_dim, d.n_embd, d.n_ff};
-        if (last_row) for (int i = 0; i < 5; ++i) cudaMemcpyAsync(bufs[i], bufs[i] + (size_t)last_row * lds[i], (size_t)lds[i] * 4, cudaMemcpyDeviceToDevice, g.stream);
+        if (last_row) for (int i = 0; i < 5; ++i) ok(cudaMemcpyAsync(bufs[i], bufs[i] + (size_t)last_row * lds[i], (size_t)lds[i] * 4, cudaMemcpyDeviceToDevice, g.stream));
         rc = check_launch("decoder score");
     }
     g.pdl = false;
     D->chunks.clear();
-    if (rc == ADAMAH_OK) D->hpos[0] += n_tokens;
-    cudaStreamSynchronize(D->score_copy);
-    DCU(cudaStreamSynchronize(g.stream));               // the caller reads `out` on return
+    ok(cudaStreamSynchronize(D->score_copy));
+    ok(cudaStreamSynchronize(g.stream));                // the caller reads `out` on return
     g.submits++;
+    if (rc == ADAMAH_OK && err != cudaSuccess) rc = fail(ADAMAH_ERR_BACKEND, "decoder_score: %s", cudaGetErrorString(err));
+    if (rc == ADAMAH_OK) D->hpos[0] += n_tokens;
     return rc;
 }
 

@@ -190,6 +190,36 @@ def test_score_leaves_the_decoder_as_steps_do(gpu, n, embd_type):
         eng.close()
 
 
+@pytest.mark.parametrize("max_batch,left_mb", [(1, 8), (3, 8), (1, 100)])
+def test_score_without_room_for_its_buffer(gpu, max_batch, left_mb):
+    """Two groups of 64 rows of 131072 logits are 67 MB: with less on the device the groups get smaller, down to the logits
+    buffer of the decoder, which single steps never needed more than."""
+    import torch
+    cfg = replace(tiny_gemma3(n_layer=1), n_vocab=131072)
+    tensors = synth.build_model(cfg, gb.GGML_TYPE_Q4_0, seed=65)
+    toks = synth.random_prompt(cfg.n_vocab, 70, seed=8)
+    want, filler = None, None
+    for full in (False, True):
+        eng = ADAMEngine(gpu, cfg, tensors, kv_cap=80, kv_dtype="f32", max_batch=max_batch)
+        try:
+            if full:
+                eng.begin([toks], [70])
+                eng.prefill(3)                           # the buffers of a prompt exist
+                torch.cuda.empty_cache()
+                filler = torch.empty(torch.cuda.mem_get_info()[0] - (left_mb << 20), dtype=torch.uint8, device="cuda")
+            got = eng.logits_trace(toks)
+            assert np.array_equal(eng.read_logits(0), got[-1])
+            assert gpu.device_error() == 0
+        finally:
+            del filler
+            filler = None
+            torch.cuda.empty_cache()
+            eng.close()
+        if want is None:
+            want = got
+    assert np.abs(got - want).max() <= 2e-5 * np.abs(want).max()
+
+
 @pytest.mark.parametrize("n", [1, 16383, 16384, 262144, 262145, 1200000])
 def test_large_results_and_uploads(gpu, n):
     """Around the sizes where results move to page-locked blocks and uploads leave the ring; neighbouring locs and others; arrays
