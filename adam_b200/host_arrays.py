@@ -3,9 +3,10 @@
 A copy from the device into an ordinary numpy array goes through the driver's staging buffer at a few GB/s and takes a page
 fault for every 4 KB of a fresh array (68 MB of logits: 15 ms and more); into page-locked memory it runs at the link's rate
 (1.3 ms).  Locking pages costs as much as it saves, so blocks are kept when their array is garbage collected: at most
-``LIMIT`` bytes, the rest is given back to the system at once."""
+``LIMIT`` bytes, the rest is given back to the system."""
 from __future__ import annotations
 
+import collections
 import ctypes
 import math
 import threading
@@ -22,6 +23,9 @@ class HostArrays:
 
     def __init__(self, lib):
         self._lib, self._lock = lib, threading.Lock()
+        # Blocks whose array is gone.  The finalizer runs wherever the garbage collector does, also inside `empty` in the
+        # thread that holds the lock, so it never waits for the lock: it leaves the block here.
+        self._returned = collections.deque()
         self._free = []             # (bytes, address)
         self._kept = 0
         self._small = 0             # bytes of the blocks below LARGE
@@ -34,6 +38,7 @@ class HostArrays:
             return np.empty(shape, dtype)
         block = None
         with self._lock:            # the smallest block that holds it and is not half empty
+            self._take_back()
             fits = [b for b in self._free if n <= b[0] <= 2 * n]
             if fits:
                 block = min(fits)
@@ -53,20 +58,32 @@ class HostArrays:
                 return np.empty(shape, dtype)
             block = (size, address)
         raw = (ctypes.c_char * n).from_address(block[1])
-        weakref.finalize(raw, self._give_back, block)        # `raw` lives as long as the array or a view of it
+        # `raw` lives as long as the array or a view of it; at exit the process gives everything back, arrays that live on included
+        weakref.finalize(raw, self._give_back, block).atexit = False
         return np.frombuffer(raw, dtype).reshape(shape)
 
     def _give_back(self, block):
-        with self._lock:
+        self._returned.append(block)
+        if self._lock.acquire(blocking=False):      # else whoever holds it, or the next call, takes the block back
+            try:
+                self._take_back()
+            finally:
+                self._lock.release()
+
+    def _take_back(self):           # under the lock
+        while self._returned:
+            block = self._returned.popleft()
             if not self._closed and self._kept + block[0] <= self.LIMIT:
                 self._free.append(block)
                 self._kept += block[0]
-                return
-            self._small -= block[0] if block[0] < self.LARGE else 0
-        self._lib.adam_b200_host_free(block[1])
+            else:
+                self._small -= block[0] if block[0] < self.LARGE else 0
+                self._lib.adam_b200_host_free(block[1])
 
     def close(self):
         with self._lock:
-            blocks, self._free, self._kept, self._closed = self._free, [], 0, True
+            self._closed = True
+            self._take_back()
+            blocks, self._free, self._kept = self._free, [], 0
         for _, address in blocks:
             self._lib.adam_b200_host_free(address)
