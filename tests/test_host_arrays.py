@@ -76,3 +76,24 @@ def test_blocks_are_used_again_and_live_as_long_as_a_view(arrays):
     assert b.ctypes.data != where and (view == 1).all()
     del view
     assert arrays.empty((299, 1000), np.float32).ctypes.data == where
+
+
+def test_locked_memory_is_bounded(arrays):
+    """Results that a program keeps are ordinary arrays once the bound is reached; unused blocks make room for used ones."""
+    arrays.LOCKED_LIMIT = 8 * MB
+    kept = [arrays.empty((2 * MB,), np.uint8) for _ in range(10)] + [arrays.empty((MB // 2,), np.uint8)]
+    assert arrays._lib.locked() == 8 * MB and arrays._locked == 8 * MB
+    for i, a in enumerate(kept):
+        a[:] = i
+    assert all((a == i).all() for i, a in enumerate(kept))
+    del a, kept
+    big = arrays.empty((7 * MB,), np.uint8)
+    assert big.ctypes.data in arrays._lib.blocks and arrays._lib.locked() <= 8 * MB
+    del big
+
+
+def test_a_library_without_memory_gives_ordinary_arrays(arrays):
+    arrays._lib.adam_b200_host_alloc = lambda n: None
+    a, b = arrays.empty((MB,), np.float32), arrays.empty((MB // 8,), np.float32)
+    a[:], b[:] = 1, 2
+    assert arrays._locked == 0 and arrays._small == 0
