@@ -196,10 +196,12 @@ __device__ __forceinline__ float rcp_newton(float d) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return fmaf(r, fmaf(-d, r, 1.0f), r);
 }
-// x / (1 + e^-z), without branches (z >= -80 keeps the divisor finite).
+// x / (1 + e^-z), without branches.  Below z = -80 it is x * 0 (the true factor, e^-80 and less, is nothing beside any other
+// term, and 1 + tanh is 0 there), which is NaN for an infinite x; an infinite x elsewhere keeps its sign, which div_by would lose.
 __device__ __forceinline__ float gated(float x, float z) {
-    const float d = 1.0f + expf(-fmaxf(z, -80.f));
-    return div_by(x, d, rcp_newton(d));
+    const float d = 1.0f + expf(-fmaxf(z, -80.f)), r = rcp_newton(d);
+    const float q = fabsf(x) <= 3.402823466e+38f ? div_by(x, d, r) : x * r;
+    return z < -80.f ? x * 0.f : q;
 }
 // GELU in its tanh form (tests/diagnostics/diag_inference.py:941-943), 0.5 x (1 + tanh u), written as x / (1 + e^-2u): the
 // same function without tanhf's branches, and without the cancellation in 1 + tanh u for negative u.

@@ -57,6 +57,29 @@ def test_argmax_nan_and_large(gpu):
     assert int(_read(gpu, 8, [70005])[0]) == 60001
 
 
+@pytest.mark.parametrize("act,op", [("gelu", A.OP_GEGLU), ("silu", A.OP_SWIGLU)])
+def test_gates_over_the_whole_range(gpu, act, op):
+    """Infinities, NaN, zeros and the largest and smallest values as the oracle has them.  Elsewhere against float64: the factor
+    1 / (1 + e^-z) carries the rounding of z (three operations) and a few ulp of its own; below z = -80 it counts as 0."""
+    big = np.float32(3.402823466e38)
+    special = np.array([np.inf, -np.inf, np.nan, 0.0, -0.0, big, -big, 1e20, -1e20, 1e-38, -1e-38, 1e-45, 80.0, -80.0, 100.0, -100.0], np.float32)
+    x = np.concatenate([special, np.linspace(-90, 90, 40001), np.linspace(-4, 4, 40001), np.logspace(-38, 38, 2001), -np.logspace(-38, 38, 2001)]).astype(np.float32)
+    n, m = len(x), len(special)
+    _f32map(gpu, 12, 2 * n, np.concatenate([x, np.ones(n, np.float32)]))
+    src, one = _h(gpu, np.arange(n)), _h(gpu, np.arange(n, 2 * n))
+    gpu.map_op2_dev(12, op, src, one, src, n)
+    y = _read(gpu, 12, np.arange(n))
+    gpu.free_handle(src), gpu.free_handle(one)
+    with np.errstate(all="ignore"):
+        want = od.gelu_tanh(special) if act == "gelu" else od.silu(special)
+        np.testing.assert_allclose(y[:m], want, rtol=1e-6, atol=1e-37)
+        x = x[m:].astype(np.float64)
+        z = 2 * np.sqrt(2 / np.pi) * (x + 0.044715 * x ** 3) if act == "gelu" else x.clip(-80, 80)
+        ref = x * np.exp(z - np.logaddexp(0, z))
+        ref[z < -80] = 0
+    assert (np.abs(y[m:] - ref) <= (8 + 4 * np.abs(z).clip(0, 100)) * 2.0 ** -24 * np.abs(ref) + 1e-37 + (np.abs(z + 80) < 1e-3) * 1e-30).all()
+
+
 def test_resolve_idx(gpu):
     # tests/test_decode_primitives.py:63-95 (the resolve step)
     vals = np.zeros(32, np.float32)
