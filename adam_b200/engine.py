@@ -377,7 +377,12 @@ class ADAMEngine:
         else:
             self.begin(prompts, [max_len + config.max_tokens] * len(prompts))
         with g.batch():
-            cached = self.prefill_prompts(prompts, reuse)
+            if mode == "cpu" and min_len < max_len:
+                # the sequences share one random stream: who draws when is settled by all of them stepping from the shortest one's end
+                self.prefill(min_len - 1)
+                cached = [min_len - 1] * len(prompts)
+            else:
+                cached = self.prefill_prompts(prompts, reuse)
         t_pre = time.perf_counter() - tp
         td = time.perf_counter()
         ahead = [n - c for n, c in zip(lens, cached)]              # steps until a sequence's first sampled token

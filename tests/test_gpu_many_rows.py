@@ -110,6 +110,27 @@ def test_batched_head_and_ragged_prefill_match_the_oracle(gpu, batch):
         eng.close()
 
 
+def test_host_sampling_of_a_ragged_batch_draws_in_step_order(gpu):
+    """Sequences that are sampled on the host share one seeded random stream: one whose prompt is longer by n tokens draws its
+    first number n steps later, and within a step they draw in their order."""
+    cfg = tiny_gemma3(n_layer=1, n_vocab=64)
+    tensors = synth.build_model(cfg, gb.GGML_TYPE_Q4_0, seed=66)
+    prompts = [list(synth.random_prompt(cfg.n_vocab, n, seed=n)) for n in (7, 3, 5)]
+    rule = GenerationConfig(max_tokens=5, eos_token_ids=(), temperature=1.0, top_k=0, top_p=1.0, repeat_penalty=1.0, seed=11)
+    eng = ADAMEngine(gpu, cfg, tensors, kv_cap=32, kv_dtype="f32", max_batch=3)
+    try:
+        outs, stats = eng.generate_batch(prompts, rule)
+        assert stats["sampling_mode"] == "cpu"
+        rng, want = np.random.default_rng(11), [[] for _ in prompts]
+        for step in range(4 + 5):
+            for b, p in enumerate(prompts):
+                if len(p) - 3 <= step and len(want[b]) < 5:
+                    want[b].append(eng._sample(eng.logits_trace(p + want[b])[-1], rule, [], rng))
+        assert outs == want
+    finally:
+        eng.close()
+
+
 # Query rows per attention tile: 32 (a chunk that does not fill the GPU), 64 and 128 (it does); windows and pages whose edges
 # lie inside a cache tile; a prompt longer than one chunk of 1024 rows.
 @pytest.mark.parametrize("kv_dtype", ["f16", "f32"])
