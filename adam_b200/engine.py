@@ -277,11 +277,19 @@ class ADAMEngine:
         self._check(self._lib.adam_b200_decoder_step_trace(self._dec, 0, out.ctypes.data, 512), "adam_b200_decoder_step_trace")
         return out[:256].reshape(4, 8, 8), out[256:512].reshape(32, 8)
 
-    def logits_trace(self, tokens: Sequence[int], direct: bool = True) -> np.ndarray:
+    def logits_trace(self, tokens: Sequence[int], direct: bool = True, by_steps: bool = False) -> np.ndarray:
         """Teacher-forced pass over ``tokens``: the soft-capped logits after every
-        position, ``[len(tokens), n_vocab]`` (for parity checks)."""
+        position, ``[len(tokens), n_vocab]`` (for parity checks).  The positions run together where the engine can do that;
+        with ``by_steps`` each is a decode step, ``direct`` (kernels enqueued one by one) or as a graph."""
         self.begin([tokens], [len(tokens)])
-        return self._score(len(tokens), direct)
+        return self._score_by_steps(len(tokens), direct) if by_steps else self._score(len(tokens), direct)
+
+    def _score_by_steps(self, n: int, direct: bool) -> np.ndarray:
+        out = np.empty((n, self.cfg.n_vocab), np.float32)
+        for i in range(n):
+            self.step(1, lm_head=True, logits=True, direct=direct)
+            out[i] = self.read_logits(0)
+        return out
 
     def _score(self, n: int, direct: bool) -> np.ndarray:
         # all positions in one pass: at the 1B shape 65 of them take what six single steps take

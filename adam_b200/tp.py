@@ -305,11 +305,7 @@ class ADAMEngineTP(ADAMEngine):
 
     def _score(self, n, direct):
         """Position by position: the collectives sit between the parts of a step."""
-        out = np.empty((n, self.cfg.n_vocab), np.float32)
-        for i in range(n):
-            self.step(1, lm_head=True, logits=True, direct=direct)
-            out[i] = self.read_logits(0)
-        return out
+        return self._score_by_steps(n, direct)
 
     def begin(self, prompts, reserve):
         super().begin(prompts, reserve)

@@ -116,6 +116,27 @@ def test_sliding_window_matches_oracle_extension(gpu):
         eng.close()
 
 
+@pytest.mark.parametrize("layers,embd_type,tied,window,kv_dtype", [
+    (gb.GGML_TYPE_Q4_0, None, True, 0, "f32"), (gb.GGML_TYPE_Q4_0, None, False, 8, "f16"), (gb.GGML_TYPE_Q4_K, None, True, 8, "f32"), (gb.GGML_TYPE_Q4_K, None, False, 0, "f16"),
+    (gb.GGML_TYPE_Q4_0, gb.GGML_TYPE_Q8_0, True, 8, "f16"), (gb.GGML_TYPE_Q4_K, gb.GGML_TYPE_Q5_0, True, 0, "f32")])
+def test_logits_of_steps_and_of_positions_together_match_the_oracle(gpu, layers, embd_type, tied, window, kv_dtype):
+    """Decode steps, as graphs and kernel by kernel, and the pass that scores all positions together: the same logits."""
+    cfg = _cfg(dict(n_layer=7, sliding_window=8))
+    tensors = synth.build_model(cfg, layers, seed=34, tied=tied, embd_type=embd_type)
+    toks = synth.random_prompt(cfg.n_vocab, 30, seed=6)
+    dec = OracleDecoder(cfg, dequant_model(tensors), kv_cap=32, window=window > 0, kv_dtype=np.float16 if kv_dtype == "f16" else np.float32)
+    ref = np.stack([dec.forward(int(t), i) for i, t in enumerate(toks)])
+    eng = ADAMEngine(gpu, cfg, tensors, kv_cap=32, kv_dtype=kv_dtype, window=window > 0)
+    try:
+        seen = [eng.logits_trace(toks, by_steps=True), eng.logits_trace(toks, direct=False, by_steps=True), eng.logits_trace(toks)]
+        for out in seen:
+            assert _rel(out, ref) < (1e-4 if kv_dtype == "f32" else 1e-3)
+        assert np.array_equal(seen[0], seen[1])          # a graph runs the same kernels
+        assert gpu.device_error() == 0
+    finally:
+        eng.close()
+
+
 def test_long_context_uses_several_attention_splits_and_pages(gpu):
     cfg = _cfg(dict(n_layer=2, n_head=4, n_head_kv=2, head_dim=64))
     tensors = synth.build_model(cfg, gb.GGML_TYPE_Q4_0, seed=34, tied=True)

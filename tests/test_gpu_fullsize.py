@@ -79,10 +79,11 @@ def test_1b_shape_128_prompt_128_greedy_tokens(gpu, golden_dir, case):
         assert got == want
         # teacher-forced logits after positions n_prompt-1 .. n_prompt+n_gen-2 (1e-3 of the largest logit)
         seq = list(prompt) + want[:-1]
-        out = eng.logits_trace(seq)
-        worst = max(_rel(out[n_prompt - 1 + i], want_logits[i]) for i in range(n_gen))
-        assert worst < 1e-3, worst
-        assert all(int(out[n_prompt - 1 + i].argmax()) == want[i] for i in range(n_gen))
+        for by_steps in (False, True):
+            out = eng.logits_trace(seq, by_steps=by_steps)
+            worst = max(_rel(out[n_prompt - 1 + i], want_logits[i]) for i in range(n_gen))
+            assert worst < 1e-3, worst
+            assert all(int(out[n_prompt - 1 + i].argmax()) == want[i] for i in range(n_gen))
         assert gpu.device_error() == 0
     finally:
         eng.close()
@@ -150,9 +151,10 @@ def test_27b_shape_two_layers_and_lm_head(gpu):
     try:
         got, _ = eng.generate(prompt, GenerationConfig(max_tokens=n_gen, **GREEDY))
         assert got == want
-        out = eng.logits_trace(list(prompt) + want[:-1])
-        worst = max(_rel(out[n_prompt - 1 + i], want_logits[i]) for i in range(n_gen))
-        assert worst < 1e-3, worst
+        for by_steps in (False, True):
+            out = eng.logits_trace(list(prompt) + want[:-1], by_steps=by_steps)
+            worst = max(_rel(out[n_prompt - 1 + i], want_logits[i]) for i in range(n_gen))
+            assert worst < 1e-3, worst
         assert gpu.device_error() == 0
     finally:
         eng.close()
