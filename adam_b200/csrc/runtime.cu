@@ -545,9 +545,10 @@ extern "C" int map_gather(uint32_t id, const uint32_t* locs, void* out, uint32_t
     if (m->dtype != ADAMAH_DTYPE_F32 && m->dtype != ADAMAH_DTYPE_Q4)
         return fail(ADAMAH_ERR_INVALID, "gather: map %u holds GGUF blocks; use map_dequant_gguf", id);
     uint64_t n = (uint64_t)n_locs * m->pack_size;
-    if (m->dtype == ADAMAH_DTYPE_F32 && (uint64_t)locs[0] + n_locs <= m->n_packs && locs[n_locs - 1] == locs[0] + n_locs - 1) {
+    const bool in_place = (const uint8_t*)out < (const uint8_t*)(locs + n_locs) && (const uint8_t*)locs < (const uint8_t*)out + n * 4;
+    if (m->dtype == ADAMAH_DTYPE_F32 && !in_place && (uint64_t)locs[0] + n_locs <= m->n_packs && locs[n_locs - 1] == locs[0] + n_locs - 1) {
         // neighbouring packs (a whole result vector): one copy, no locs on the device, no kernel; the locs between the first
-        // and the last are looked at while it is under way
+        // and the last are looked at while it is under way, so the result must not land on them
         bool apart = false;
         CU(download(out, (const float*)m->buf + (uint64_t)locs[0] * m->pack_size, n * 4, [&] {
             const uint32_t first = locs[0];

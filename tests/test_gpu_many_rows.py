@@ -269,6 +269,25 @@ def test_large_results_and_uploads(gpu, n):
         gpu.map_destroy(90)
 
 
+@pytest.mark.parametrize("n", [5, 20000, 1100000])
+def test_gather_onto_its_own_locs(gpu, n):
+    """The result may overwrite the locs: neighbours, and locs that only look like neighbours at both ends; results that go
+    through the staging buffer, and larger ones."""
+    gpu.map_create_typed(90, A.DTYPE_F32, 1, n)
+    try:
+        x = np.random.default_rng(n).standard_normal(n).astype(np.float32)
+        gpu.scatter_contiguous(90, 0, x)
+        swapped = np.arange(n, dtype=np.uint32)
+        swapped[1:-1] = swapped[1:-1][::-1]
+        for locs in (np.arange(n, dtype=np.uint32), swapped):
+            want = x[locs]
+            assert gpu._lib.map_gather(90, locs.ctypes.data, locs.ctypes.data, n) == 0
+            assert np.array_equal(locs.view(np.float32), want)
+        assert gpu.device_error() == 0
+    finally:
+        gpu.map_destroy(90)
+
+
 @pytest.mark.parametrize("N", [8192, 8193, 70001, 300000])
 def test_argmax_of_one_row_on_several_ctas(gpu, N):
     """A Q8_0 head's winner, and of equal rows that different CTAs look at the first."""
