@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 
 namespace ab {
 
@@ -428,8 +429,10 @@ namespace ab { bool capturing(); }
 constexpr size_t RING_BYTES = 4u << 20, RING_MAX = 1u << 20, DOWN_BYTES = 4u << 20, DIRECT_MIN = 64u << 10, SCRATCH_KEEP = 16u << 20;
 struct IoStage { uint8_t* ring; size_t ring_at; uint8_t* down; uint8_t* scratch; size_t scratch_cap; };
 static IoStage g_io = {};
+static std::mutex g_io_lock;        // held by a call from its first use of the stage to its last: the callers may be several threads
 
 static void io_release() {
+    std::lock_guard<std::mutex> stage(g_io_lock);
     cudaFreeHost(g_io.ring); cudaFreeHost(g_io.down); cudaFree(g_io.scratch);
     g_io = IoStage{};
 }
@@ -497,6 +500,7 @@ static int scatter_impl(uint32_t id, const uint32_t* locs, uint32_t start_pack, 
     if (m->dtype != ADAMAH_DTYPE_F32 && m->dtype != ADAMAH_DTYPE_Q4)
         return fail(ADAMAH_ERR_INVALID, "scatter: map %u holds GGUF blocks; use map_upload_gguf_blocks", id);
     uint64_t n = (uint64_t)n_locs * m->pack_size;
+    std::lock_guard<std::mutex> stage(g_io_lock);
     if (!locs && (uint64_t)start_pack + n_locs > m->n_packs) return fail(ADAMAH_ERR_INVALID, "scatter: range beyond map %u", id);
     if (!locs && m->dtype == ADAMAH_DTYPE_F32) {      // contiguous float copy needs no kernel
         CU(upload((float*)m->buf + (uint64_t)start_pack * m->pack_size, data, n * 4));
@@ -545,6 +549,7 @@ extern "C" int map_gather(uint32_t id, const uint32_t* locs, void* out, uint32_t
     if (m->dtype != ADAMAH_DTYPE_F32 && m->dtype != ADAMAH_DTYPE_Q4)
         return fail(ADAMAH_ERR_INVALID, "gather: map %u holds GGUF blocks; use map_dequant_gguf", id);
     uint64_t n = (uint64_t)n_locs * m->pack_size;
+    std::lock_guard<std::mutex> stage(g_io_lock);
     const bool in_place = (const uint8_t*)out < (const uint8_t*)(locs + n_locs) && (const uint8_t*)locs < (const uint8_t*)out + n * 4;
     if (m->dtype == ADAMAH_DTYPE_F32 && !in_place && (uint64_t)locs[0] + n_locs <= m->n_packs && locs[n_locs - 1] == locs[0] + n_locs - 1) {
         // neighbouring packs (a whole result vector): one copy, no locs on the device, no kernel; the locs between the first
@@ -611,6 +616,7 @@ extern "C" uint64_t map_upload_dev(uint32_t handle, const void* data, uint32_t n
             return 0;
         }
     }
+    std::lock_guard<std::mutex> stage(g_io_lock);
     if (upload(g.handles[handle].dev, data, n_bytes) != cudaSuccess) {
         fail(ADAMAH_ERR_BACKEND, "map_upload_dev: copy failed");
         return 0;
@@ -624,6 +630,7 @@ extern "C" int map_download_dev(uint32_t handle, void* out, uint32_t n_bytes) {
     if (!ready()) return ADAMAH_ERR_INVALID;
     if (!out) return fail(ADAMAH_ERR_INVALID, "map_download_dev: null pointer");
     if (!handle_ok(handle, n_bytes)) return ADAMAH_ERR_NOT_FOUND;
+    std::lock_guard<std::mutex> stage(g_io_lock);
     CU(download(out, g.handles[handle].dev, n_bytes));
     return ADAMAH_OK;
 }

@@ -288,6 +288,35 @@ def test_gather_onto_its_own_locs(gpu, n):
         gpu.map_destroy(90)
 
 
+def test_host_io_from_several_threads(gpu):
+    """Each thread writes and reads a map of its own, over all sizes of the staging; the copies run outside Python's lock."""
+    import threading
+    wrong = []
+
+    def work(k):
+        rng = np.random.default_rng(k)
+        for i in range(60):
+            n = int(rng.choice([3, 1000, 20000, 300000]))
+            x, locs = rng.standard_normal(n).astype(np.float32), rng.permutation(n).astype(np.uint32)
+            gpu.scatter(80 + k, locs, x)
+            whole, mixed = gpu.gather(80 + k, np.arange(n, dtype=np.uint32)).view(np.float32), gpu.gather(80 + k, locs).view(np.float32)
+            if not (np.array_equal(whole[locs], x) and np.array_equal(mixed, x)):
+                wrong.append((k, i, n))
+
+    for k in range(4):
+        gpu.map_create_typed(80 + k, A.DTYPE_F32, 1, 300000)
+    try:
+        threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not wrong and gpu.device_error() == 0
+    finally:
+        for k in range(4):
+            gpu.map_destroy(80 + k)
+
+
 @pytest.mark.parametrize("N", [8192, 8193, 70001, 300000])
 def test_argmax_of_one_row_on_several_ctas(gpu, N):
     """A Q8_0 head's winner, and of equal rows that different CTAs look at the first."""
