@@ -26,6 +26,7 @@
 
 #include <cmath>
 #include <cstdlib>
+#include <mutex>
 #include <vector>
 
 namespace ab {
@@ -38,6 +39,7 @@ constexpr int TC_MAX_K = 32768;
 
 struct TcWork { uint8_t* img; size_t img_cap; float* inv; int inv_cap; unsigned long long* best; float* part; unsigned int* tickets; std::vector<void*> retired; };   // best: arg-max keys [inv_cap], then a ticket
 static TcWork g_tc = {};
+static std::mutex g_tc_lock;            // the two kernels of a call are enqueued together: the image is one for all
 static uint64_t g_tc_calls = 0;
 static int g_tc_policy = -1;             // 0 never, 1 where it is expected to be faster, 2 whenever the shape allows; -1 = take it from ADAM_B200_TC
 
@@ -50,6 +52,7 @@ static int tc_pad_rows(int rows) { return (rows + 127) / 128 * 128; }
 // buffers' addresses, so a buffer that is outgrown stays until the release; sizes at least double, which bounds the sum.
 bool gemm_tc_prepare(int rows, int K) {
     if (rows < 1 || K < 1 || K > TC_MAX_K) return false;
+    std::lock_guard<std::mutex> work(g_tc_lock);
     const int pad = tc_pad_rows(rows);
     size_t need = (size_t)(pad / TC_GROUP) * tc_group_bytes(WT_Q4_K, K);
     if (need > TC_IMG_MAX) need = TC_IMG_MAX;
@@ -1048,6 +1051,7 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
 
 // Rows that exceed the workspace run in chunks of whole 128-row tiles.
 int launch_gemm_tc(int wtype, const GemvArgs& a, cudaStream_t stream) {
+    std::lock_guard<std::mutex> work(g_tc_lock);
     const int fit = tc_rows_fit(wtype, a.K);
     for (int b0 = 0; b0 < a.B; b0 += fit) {
         GemvArgs c = a;

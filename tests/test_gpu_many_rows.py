@@ -92,6 +92,45 @@ def test_q8_0_products_are_fp32_sums(gpu, B):
     assert np.linalg.norm(y - ref) < 1.5e-7 * np.linalg.norm(ref)
 
 
+def test_gemm_calls_from_several_threads(gpu):
+    """Products of four threads share one image of activations; each thread has a map, handles and rows of its own."""
+    import threading
+    rng, N, K, B, wrong = np.random.default_rng(9), 256, 512, 16, []
+    raw = gb.random_q4_0_blocks(rng, N, K)
+    W = q4_blocks.dequant(raw.reshape(-1), 2, N, K).astype(np.float64)
+    gpu.map_create_typed(91, A.DTYPE_GGUF_Q4_0, 1, N * K)
+    gpu.upload_gguf_blocks(91, 2, 0, raw)
+    locs = [gpu.upload_dev(np.array([v], np.uint32))[0] for v in (0, 0, B * K)]
+
+    def work(k):
+        rng = np.random.default_rng(k)
+        for i in range(100):
+            x = rng.standard_normal((B, K), dtype=np.float32)
+            gpu.scatter_contiguous(80 + k, 0, x)
+            gpu.map_matmul_t_xq4_dev(80 + k, 91, locs[0], locs[1], locs[2], B, K, N)
+            y = gpu.gather(80 + k, np.arange(B * K, B * K + B * N, dtype=np.uint32)).view(np.float32).reshape(B, N)
+            ref = x.astype(np.float64) @ W.T
+            if np.linalg.norm(y - ref) > 5e-6 * np.linalg.norm(ref):
+                wrong.append((k, i))
+
+    before = gpu.tc_gemm_count()
+    for k in range(4):
+        gpu.map_create_typed(80 + k, A.DTYPE_F32, 1, B * K + B * N)
+    try:
+        threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not wrong and gpu.device_error() == 0 and gpu.tc_gemm_count() == before + 400
+    finally:
+        for k in range(4):
+            gpu.map_destroy(80 + k)
+        gpu.map_destroy(91)
+        for h in locs:
+            gpu.free_handle(h)
+
+
 @pytest.mark.parametrize("batch", [9, 17, 40])
 def test_batched_head_and_ragged_prefill_match_the_oracle(gpu, batch):
     """Prompts of 1 to 70 tokens through one ragged prefill, then steps whose products and arg-max are the GEMM's."""
