@@ -64,7 +64,9 @@ struct Decoder {
     float *part_o, *part_ml; unsigned int* attn_ticket; uint32_t n_splits;
     // chunked prefill: what the rows of all chunks are (device copy and pinned source of one call; see PrefillPlan)
     uint8_t *plan, *plan_pin; size_t plan_cap; cudaEvent_t plan_read;
-    std::vector<PrefillChunk> chunks; const int32_t* plan_n;
+    std::vector<PrefillChunk> chunks; const int32_t* plan_n; std::vector<int32_t> plan_pos;     // chunks of a call, its tokens and first positions
+    int32_t* even_plan;         // the plan of a chunk with the same number of tokens for all, made on the device: row_seq, row_pos, tiles
+    bool pos_shared;            // positions may move without the host's doing: recorded graphs, a caller that has their address
     // adam_b200_decoder_score: two groups of score_rows rows of logits (NULL: none fit, D->logits takes one at a time), the
     // winners of a group, and the copies to the host
     float* score_logits; int32_t* score_tok; uint32_t score_rows; cudaEvent_t score_ev[4]; cudaStream_t score_copy;
@@ -642,12 +644,24 @@ __global__ void __launch_bounds__(256) k_attention(const float* __restrict__ qkv
     if (tid == 0) *tkt = 0u;
 }
 
-// End of a prefill: every sequence moves on by its own number of tokens.
-__global__ void k_advance_by(int32_t* __restrict__ pos, const int32_t* __restrict__ n, uint32_t batch) {
+// End of a prefill: every sequence moves on by its own number of tokens, or all by `even`.
+__global__ void k_advance_by(int32_t* __restrict__ pos, const int32_t* __restrict__ n, int32_t even, uint32_t batch) {
     pdl_launch_dependents();
     pdl_wait();
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b < batch) pos[b] += n[b];
+    if (b < batch) pos[b] += n ? n[b] : even;
+}
+// The plan of a chunk of T tokens for each of `batch` sequences, from where they are now: row r = (sequence r / T, position
+// pos + r % T), and attention tiles of up to `step` positions, those with the longest reach first.
+__global__ void k_even_plan(const int32_t* __restrict__ pos, uint32_t batch, uint32_t T, uint32_t step, int32_t* __restrict__ row_seq,
+                            int32_t* __restrict__ row_pos, AttnTile* __restrict__ tiles) {
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x, per = (T + step - 1) / step;
+    if (r >= batch * T) return;
+    row_seq[r] = (int32_t)(r / T);
+    row_pos[r] = pos[r / T] + (int32_t)(r % T);
+    if (r >= batch * per) return;
+    const uint32_t s = r % batch, first = (per - 1 - r / batch) * step;
+    tiles[r] = AttnTile{(int32_t)(s * T + first), (int32_t)s, pos[s] + (int32_t)first, (int32_t)min(step, T - first)};
 }
 
 // End of a step: advance positions; when the LM head ran, log the sampled token.
@@ -699,7 +713,7 @@ static void destroy(Decoder* D) {
     free_token_kernel(D);
     for (int i = 0; i < 4; ++i) { if (D->tok_ring[i]) cudaFreeHost(D->tok_ring[i]); if (D->tok_event[i]) cudaEventDestroy(D->tok_event[i]); }
     void* ptrs[] = {D->pos, D->cur_tok, D->cur_val, D->prompt_len, D->prompt_tok, D->gen_log, D->block_table, D->kv_pool, D->hbuf[0], D->hbuf[1], D->qkv,
-                    D->attn_out, D->proj, D->act, D->logits, D->part_o, D->part_ml, D->attn_ticket, D->plan,
+                    D->attn_out, D->proj, D->act, D->logits, D->part_o, D->part_ml, D->attn_ticket, D->plan, D->even_plan,
                     D->rope_cos[0], D->rope_sin[0], D->rope_cos[1], D->rope_sin[1]};
     for (void* p : ptrs) cudaFree(p);
     cudaFreeHost(D->plan_pin);
@@ -822,6 +836,16 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
 
 // The embedding kernel takes a full dependency on everything before it (no programmatic launch): later kernels
 // of the step rely on the previous step's position update and cache writes being complete before any of them starts.
+// Is the stream being recorded, by adam_b200_capture_begin or by a caller that lent it?
+static bool stream_recorded() {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(g.stream, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone;
+}
+static bool pdl_allowed() {
+    static const bool allow = !(getenv("ADAM_B200_PDL") && atoi(getenv("ADAM_B200_PDL")) == 0);
+    return allow;
+}
+
 static void launch_embed(Decoder* D, uint32_t rows, const int32_t* row_seq, const int32_t* row_pos) {
     const adam_b200_decoder_desc& d = D->d;
     auto go = [&](auto kern) {
@@ -1195,8 +1219,10 @@ extern "C" int adam_b200_decoder_create(const adam_b200_decoder_desc* desc, uint
     DALLOC(D->part_o, B * d.n_head_kv * D->n_splits * gs * d.head_dim * 4);
     DALLOC(D->part_ml, B * d.n_head_kv * D->n_splits * gs * 2 * 4);
     DALLOC(D->attn_ticket, B * d.n_head * 4);
+    DALLOC(D->even_plan, R * (8 + sizeof(AttnTile)));
 #undef DALLOC
     cudaMemsetAsync(D->attn_ticket, 0, B * d.n_head * 4, g.stream);
+    cudaMemsetAsync(D->even_plan, 0, R * (8 + sizeof(AttnTile)), g.stream);
     cudaMemsetAsync(D->pos, 0, B * 4, g.stream);
     cudaMemsetAsync(D->cur_tok, 0, B * 4, g.stream);
     cudaMemsetAsync(D->cur_val, 0, B * 4, g.stream);
@@ -1402,6 +1428,7 @@ extern "C" int adam_b200_decoder_step(uint32_t id, uint32_t n_steps, uint32_t fl
         if ((uint64_t)D->hpos[b] + n_steps > D->hres[b])
             return fail(ADAMAH_ERR_INVALID, "decoder_step: sequence %u is at position %u of %u reserved, cannot take %u more steps", b, D->hpos[b], D->hres[b], n_steps);
     for (uint32_t& hp : D->hpos) hp += n_steps;
+    if (stream_recorded()) D->pos_shared = true;
     if (D->batch == 1 && !chain && D->tk_state == 0 && !capturing()) { if ((rc = prepare_token_kernel(D))) return rc; }
     if (D->batch == 1 && !chain && D->tk_state == 1 && !capturing()) {
         uint32_t s = 0;
@@ -1534,7 +1561,15 @@ static int plan_prefill(Decoder* D, const uint32_t* n_tokens) {
     uint64_t total = 0;
     for (uint32_t b = 0; b < D->batch; ++b) total += n_tokens[b];
     D->chunks.clear();
+    D->plan_pos.assign(D->hpos.begin(), D->hpos.end());
     if (!total) return ADAMAH_OK;
+    if (D->pos_shared) {
+        DCU(cudaMemcpyAsync(D->plan_pos.data(), D->pos, (size_t)D->batch * 4, cudaMemcpyDeviceToHost, g.stream));
+        DCU(cudaStreamSynchronize(g.stream));
+        for (uint32_t b = 0; b < D->batch; ++b)
+            if (D->plan_pos[b] < 0 || (uint64_t)D->plan_pos[b] + n_tokens[b] > d.kv_cap)
+                return fail(ADAMAH_ERR_INVALID, "decoder_prefill: sequence %u is at position %d of %u", b, D->plan_pos[b], d.kv_cap);
+    }
     const uint64_t n_chunks = (total + D->rows_cap - 1) / D->rows_cap;
     uint64_t size = ((total + n_chunks - 1) / n_chunks + 63) / 64 * 64;
     if (size > D->rows_cap) size = D->rows_cap;
@@ -1550,8 +1585,9 @@ static int plan_prefill(Decoder* D, const uint32_t* n_tokens) {
         std::vector<Run> runs;
         while (c.rows < size && b < D->batch) {
             const uint32_t n = std::min<uint32_t>(n_tokens[b] - at, (uint32_t)size - c.rows);
-            if (n) runs.push_back(Run{c.rows, b, D->hpos[b] + at, n});
-            for (uint32_t i = 0; i < n; ++i) { seq.push_back((int32_t)b); pos.push_back((int32_t)(D->hpos[b] + at + i)); }
+            const uint32_t from = (uint32_t)D->plan_pos[b] + at;
+            if (n) runs.push_back(Run{c.rows, b, from, n});
+            for (uint32_t i = 0; i < n; ++i) { seq.push_back((int32_t)b); pos.push_back((int32_t)(from + i)); }
             c.rows += n; at += n;
             if (at == n_tokens[b]) { ++b; at = 0; }
         }
@@ -1641,21 +1677,35 @@ static int enqueue_prefill_part(Decoder* D, const PrefillChunk& c, uint32_t part
     return check_launch("decoder prefill");
 }
 
-static void enqueue_prefill_end(Decoder* D) {
-    launch_k(k_advance_by, dim3((D->batch + 63) / 64), dim3(64), 0, g.stream, g.pdl, D->pos, D->plan_n, D->batch);
+static void enqueue_prefill_end(Decoder* D, uint32_t even) {       // 0: the plan's numbers of tokens
+    launch_k(k_advance_by, dim3((D->batch + 63) / 64), dim3(64), 0, g.stream, g.pdl, D->pos, even ? (const int32_t*)nullptr : D->plan_n, (int32_t)even, D->batch);
     count_launch();
 }
-
+// A chunk of T tokens of every sequence, planned on the device: it can be recorded and replayed from wherever the sequences are.
+// What reads the plan comes behind the embedding, which is launched with a full dependency.
+static PrefillChunk even_chunk(const Decoder* D, uint32_t T, uint32_t* step) {
+    const adam_b200_decoder_desc& d = D->d;
+    const uint32_t group = d.n_head / d.n_head_kv, rows = D->batch * T, tile_rows = attn_prefill_rows(rows, group, d.n_head_kv, d.head_dim, (uint32_t)g.sm_count);
+    *step = attn_prefill_tokens(group, tile_rows);
+    return PrefillChunk{rows, D->batch * ((T + *step - 1) / *step), tile_rows, D->even_plan, D->even_plan + D->rows_cap, (const AttnTile*)(D->even_plan + 2 * (size_t)D->rows_cap)};
+}
+static int enqueue_even_part(Decoder* D, uint32_t T, uint32_t part) {
+    uint32_t step;
+    const PrefillChunk c = even_chunk(D, T, &step);
+    if (part == 0) {
+        k_even_plan<<<(c.n_rows + 127) / 128, 128, 0, g.stream>>>(D->pos, D->batch, T, step, D->even_plan, D->even_plan + D->rows_cap, (AttnTile*)(D->even_plan + 2 * (size_t)D->rows_cap));
+        count_launch();
+    }
+    if (part < 2 * D->d.n_layer) return enqueue_prefill_part(D, c, part);
+    enqueue_prefill_end(D, T);
+    return check_launch("decoder prefill");
+}
 static int check_prefill(Decoder* D, const uint32_t* n_tokens, const char* name) {
     if (D->batch == 0) return fail(ADAMAH_ERR_INVALID, "%s: call decoder_begin first", name);
     for (uint32_t b = 0; b < D->batch; ++b)
         if ((uint64_t)D->hpos[b] + n_tokens[b] > D->hplen[b])
             return fail(ADAMAH_ERR_INVALID, "%s: sequence %u has only %u prompt tokens left", name, b, D->hplen[b] - D->hpos[b]);
     return ADAMAH_OK;
-}
-static bool pdl_allowed() {
-    static const bool allow = !(getenv("ADAM_B200_PDL") && atoi(getenv("ADAM_B200_PDL")) == 0);
-    return allow;
 }
 
 // One part of one prefill chunk of n_tokens (n_tokens * batch rows, at most what buffer 0 of
@@ -1667,15 +1717,14 @@ extern "C" int adam_b200_decoder_prefill_part(uint32_t id, uint32_t n_tokens, ui
     if (!D) return ADAMAH_ERR_NOT_FOUND;
     if (part > 2 * D->d.n_layer) return fail(ADAMAH_ERR_INVALID, "decoder_prefill_part: part %u of %u", part, 2 * D->d.n_layer + 1);
     if (D->batch && (n_tokens == 0 || (uint64_t)n_tokens * D->batch > D->rows_cap)) return fail(ADAMAH_ERR_INVALID, "decoder_prefill_part: a chunk holds at most %u rows", D->rows_cap);
-    const std::vector<uint32_t> n(D->batch, n_tokens);
     int rc = ADAMAH_OK;
-    if (part == 0 && ((rc = check_prefill(D, n.data(), "decoder_prefill_part")) || (rc = plan_prefill(D, n.data())))) return rc;
-    if (D->chunks.size() != 1 || D->chunks[0].n_rows != n_tokens * D->batch) return fail(ADAMAH_ERR_INVALID, "decoder_prefill_part: begin with part 0");
+    const std::vector<uint32_t> n(D->batch, n_tokens);
+    if ((part == 0 || !D->batch) && (rc = check_prefill(D, n.data(), "decoder_prefill_part"))) return rc;
+    if (stream_recorded()) D->pos_shared = true;
     g.pdl = pdl_allowed();
-    if (part < 2 * D->d.n_layer) rc = enqueue_prefill_part(D, D->chunks[0], part);
-    else { enqueue_prefill_end(D); rc = check_launch("decoder prefill"); }
+    rc = enqueue_even_part(D, n_tokens, part);
     g.pdl = false;
-    if (rc == ADAMAH_OK && part == 2 * D->d.n_layer) { for (uint32_t& hp : D->hpos) hp += n_tokens; D->chunks.clear(); }
+    if (rc == ADAMAH_OK && part == 2 * D->d.n_layer) for (uint32_t& hp : D->hpos) hp += n_tokens;
     end_of_op();
     return rc;
 }
@@ -1687,12 +1736,23 @@ extern "C" int adam_b200_decoder_prefill_ragged(uint32_t id, const uint32_t* n_t
     if (!n_tokens) return fail(ADAMAH_ERR_INVALID, "decoder_prefill: null argument");
     if (capturing()) return fail(ADAMAH_ERR_INVALID, "decoder_prefill: not allowed while a graph is being captured");
     int rc = check_prefill(D, n_tokens, "decoder_prefill");
-    if (rc || (rc = plan_prefill(D, n_tokens))) return rc;
+    if (rc) return rc;
+    if (stream_recorded()) {                    // a caller's own capture of the stream that it lent
+        for (uint32_t b = 1; b < D->batch; ++b) if (n_tokens[b] != n_tokens[0]) return fail(ADAMAH_ERR_INVALID, "decoder_prefill: only equal numbers of tokens can be recorded");
+        D->pos_shared = true;
+        g.pdl = pdl_allowed();
+        const uint32_t most = D->rows_cap / D->batch;
+        for (uint32_t left = n_tokens[0], T; left && rc == ADAMAH_OK; left -= T) {
+            T = std::min(left, most);
+            for (uint32_t part = 0; part <= 2 * D->d.n_layer && rc == ADAMAH_OK; ++part) rc = enqueue_even_part(D, T, part);
+        }
+        g.pdl = false;
+    } else if ((rc = plan_prefill(D, n_tokens))) return rc;
     if (!D->chunks.empty()) {
         g.pdl = pdl_allowed();
         for (const PrefillChunk& c : D->chunks)
             for (uint32_t part = 0; part < 2 * D->d.n_layer && rc == ADAMAH_OK; ++part) rc = enqueue_prefill_part(D, c, part);
-        if (rc == ADAMAH_OK) { enqueue_prefill_end(D); rc = check_launch("decoder prefill"); }
+        if (rc == ADAMAH_OK) { enqueue_prefill_end(D, 0); rc = check_launch("decoder prefill"); }
         g.pdl = false;
         D->chunks.clear();
     }
@@ -1732,7 +1792,7 @@ static int score_prepare(Decoder* D) {
 extern "C" int adam_b200_decoder_score(uint32_t id, uint32_t n_tokens, float* out) {
     Decoder* D = get_dec(id);
     if (!D) return ADAMAH_ERR_NOT_FOUND;
-    if (capturing()) return fail(ADAMAH_ERR_INVALID, "decoder_score: not allowed while a graph is being captured");
+    if (stream_recorded()) return fail(ADAMAH_ERR_INVALID, "decoder_score: not allowed while a graph is being captured");
     if (!out || n_tokens == 0 || D->batch != 1) return fail(ADAMAH_ERR_INVALID, "decoder_score: needs one active sequence, tokens and a destination");
     const adam_b200_decoder_desc& d = D->d;
     if (d.tp_size > 1) return fail(ADAMAH_ERR_INVALID, "decoder_score: not available with tensor parallelism");
@@ -1747,7 +1807,7 @@ extern "C" int adam_b200_decoder_score(uint32_t id, uint32_t n_tokens, float* ou
     cudaError_t err = cudaSuccess;
     auto ok = [&](cudaError_t e) { if (err == cudaSuccess) err = e; };
     uint32_t done = 0, n_group = 0, last_row = 0, in_group = 0;
-    const uint32_t p0 = D->hpos[0];
+    const uint32_t p0 = (uint32_t)D->plan_pos[0];
     g.pdl = pdl_allowed();
     for (const PrefillChunk& c : D->chunks) {
         for (uint32_t part = 0; part < 2 * d.n_layer && rc == ADAMAH_OK; ++part) rc = enqueue_prefill_part(D, c, part);
@@ -1768,7 +1828,7 @@ extern "C" int adam_b200_decoder_score(uint32_t id, uint32_t n_tokens, float* ou
         if (rc || err != cudaSuccess) break;
     }
     if (rc == ADAMAH_OK && err == cudaSuccess) {
-        enqueue_prefill_end(D);
+        enqueue_prefill_end(D, 0);
         const float* last = base + ((size_t)((n_group - 1) % halves) * GROUP + in_group) * d.n_vocab;
         if (halves == 1) ok(cudaStreamWaitEvent(g.stream, D->score_ev[2], 0));      // the row is overwritten in place
         if (last != D->logits) ok(cudaMemcpyAsync(D->logits, last, (size_t)d.n_vocab * 4, cudaMemcpyDeviceToDevice, g.stream));
@@ -1843,8 +1903,8 @@ extern "C" int adam_b200_decoder_step_part(uint32_t id, uint32_t part, uint32_t 
     if (part == 0)
         for (uint32_t b = 0; b < D->batch; ++b)
             if (D->hpos[b] + 1u > D->hres[b]) return fail(ADAMAH_ERR_INVALID, "decoder_step_part: sequence %u has used all %u reserved positions", b, D->hres[b]);
-    static const bool allow = !(getenv("ADAM_B200_PDL") && atoi(getenv("ADAM_B200_PDL")) == 0);
-    g.pdl = allow;
+    if (part + 1 == n_parts(D) && stream_recorded()) D->pos_shared = true;
+    g.pdl = pdl_allowed();
     const int rc = enqueue_part(D, D->batch, part, with_lm, want_logits);
     g.pdl = false;
     if (rc == ADAMAH_OK && part + 1 == n_parts(D)) for (uint32_t& hp : D->hpos) hp += 1;
@@ -1911,7 +1971,7 @@ extern "C" int adam_b200_decoder_buffer_ptr(uint32_t id, uint32_t which, uint64_
     case 0: *ptr_out = (uint64_t)(uintptr_t)D->proj; *bytes_out = (size_t)D->rows_cap * D->d.n_embd * 4; break;
     case 1: *ptr_out = (uint64_t)(uintptr_t)D->cur_tok; *bytes_out = B * 4; break;
     case 2: *ptr_out = (uint64_t)(uintptr_t)D->cur_val; *bytes_out = B * 4; break;
-    case 3: *ptr_out = (uint64_t)(uintptr_t)D->pos; *bytes_out = B * 4; break;
+    case 3: *ptr_out = (uint64_t)(uintptr_t)D->pos; *bytes_out = B * 4; D->pos_shared = true; break;
     default: return fail(ADAMAH_ERR_INVALID, "decoder_buffer_ptr: unknown buffer %u", which);
     }
     return ADAMAH_OK;

@@ -137,6 +137,58 @@ def test_logits_of_steps_and_of_positions_together_match_the_oracle(gpu, layers,
         eng.close()
 
 
+@pytest.mark.parametrize("batch", [1, 3])
+def test_prompts_behind_and_inside_recorded_graphs(gpu, batch):
+    """A recorded graph moves the positions without the host's doing: a prompt chunk behind it starts where the sequences are,
+    and a recorded chunk can be replayed from wherever they are."""
+    cfg = _cfg(dict(n_layer=2))
+    tensors = synth.build_model(cfg, gb.GGML_TYPE_Q4_0, seed=36)
+    prompts = [synth.random_prompt(cfg.n_vocab, 40, seed=20 + b) for b in range(batch)]
+    eng = ADAMEngine(gpu, cfg, tensors, kv_cap=64, kv_dtype="f32", max_batch=batch)
+    graphs = []
+
+    def record(work):
+        gpu.capture_begin()
+        work()
+        graphs.append(gpu.capture_end())
+        return graphs[-1]
+
+    def begin():
+        eng.begin([p[::-1].copy() for p in prompts], [50] * batch)       # other keys and values in the cache beforehand
+        eng.step(40, lm_head=False)
+        eng.begin(prompts, [50] * batch)
+
+    def logits():
+        eng.step(1, lm_head=True, logits=True)
+        return np.stack([eng.read_logits(b) for b in range(batch)])
+
+    def parts():
+        for part in range(2 * cfg.n_layer + 1):
+            assert eng._lib.adam_b200_decoder_prefill_part(eng._dec, 7, part) == 0
+
+    try:
+        begin()
+        eng.step(39, lm_head=False)
+        want = logits()
+        begin()
+        eng.step(1, lm_head=False, direct=True)
+        step = record(lambda: eng.step(1, lm_head=False, direct=True))
+        gpu.graph_launch(step, 9)                        # positions 1 .. 9
+        eng.prefill(29)
+        assert _rel(logits(), want) < 2e-5
+        begin()
+        eng.prefill(4)
+        chunk = record(parts)
+        gpu.graph_launch(chunk, 5)                       # positions 4 .. 38
+        assert eng.read_state()[0][:batch].tolist() == [39] * batch
+        assert _rel(logits(), want) < 2e-5
+        assert gpu.device_error() == 0
+    finally:
+        for g in graphs:
+            gpu.graph_destroy(g)
+        eng.close()
+
+
 def test_long_context_uses_several_attention_splits_and_pages(gpu):
     cfg = _cfg(dict(n_layer=2, n_head=4, n_head_kv=2, head_dim=64))
     tensors = synth.build_model(cfg, gb.GGML_TYPE_Q4_0, seed=34, tied=True)
