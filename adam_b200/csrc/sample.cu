@@ -9,9 +9,9 @@
 // serial insertion list per work group as in the shader:
 //   stage 1  one CTA per group of rows keeps each thread's values in registers and extracts the group's k
 //            best by k rounds of a block-wide arg-max (warp shuffles + one shared-memory hop);
-//   stage 2  (decoder only) one CTA per sequence extracts the k best of all groups' candidates the same
-//            way, which leaves them sorted, then soft-max with temperature, nucleus cut and the draw run on
-//            one warp.
+//   stage 2  (decoder only) one CTA per sequence merges the groups' sorted candidates: k rounds of an arg-max
+//            over the heads of the groups, which leaves the k best sorted; then soft-max with temperature,
+//            nucleus cut and the draw run on one warp.
 // Ties go to the lower row index everywhere (map_argmax.comp `better`), NaN counts as -FLT_MAX.
 #include "common.cuh"
 #include "gemv.cuh"
@@ -152,37 +152,48 @@ __global__ void __launch_bounds__(SEL_T) k_sample_stage1(const float* __restrict
     }
 }
 
-// Stage 2: one CTA per sequence.  The k best of the n_cand candidates (sorted as a by-product), then on warp 0:
+// Stage 2: one CTA per sequence.  The k best of all groups' candidates (`groups` lists of k, each sorted, copied to shared
+// memory where they fit), then on warp 0:
 // p_i = exp((l_i - l_0) / T) / sum, nucleus = the shortest prefix whose probability reaches top_p
 // (np.searchsorted(cumsum, top_p) + 1, engine.py:3724-3726), renormalise, inverse-CDF draw with the uniform u.
 // temperature <= 0 takes the best candidate (engine.py:3719).  Writes the token where the next step reads it and
 // into the log at the sequence's (already advanced) position.
-__global__ void __launch_bounds__(SEL_T) k_sample_stage2(const float* __restrict__ cand_v, const int* __restrict__ cand_i, uint32_t n_cand, uint32_t k,
+__global__ void __launch_bounds__(SEL_T) k_sample_stage2(const float* __restrict__ cand_v, const int* __restrict__ cand_i, uint32_t groups, uint32_t k, int in_shared,
                                                          float temperature, float top_p, uint64_t seed,
                                                          const int32_t* __restrict__ pos, int32_t* __restrict__ cur_tok, float* __restrict__ cur_val,
                                                          int32_t* __restrict__ gen_log, uint32_t ld, float* __restrict__ dbg) {
     __shared__ float sv[SEL_T / 32]; __shared__ int si[SEL_T / 32];
     __shared__ float out_v[TOPK_MAX]; __shared__ int out_i[TOPK_MAX];
     const uint32_t b = blockIdx.x;
+    const uint32_t n_cand = groups * k;
     const float* cv = cand_v + (size_t)b * n_cand;
     const int* ci = cand_i + (size_t)b * n_cand;
-    // candidates beyond SEL_T * SEL_V are folded in by keeping the better of what a slot already holds (they
-    // arrive in groups of k sorted values, so a simple strided pre-pass is enough for the sizes in use)
-    float val[SEL_V]; int key[SEL_V];
-#pragma unroll
-    for (int j = 0; j < SEL_V; ++j) { val[j] = SNEG; key[j] = -1; }
-    // keys must be unique for block_topk: use the row index (unique across groups)
-    for (uint32_t base = 0; base < n_cand; base += SEL_T * SEL_V) {
-#pragma unroll
-        for (int j = 0; j < SEL_V; ++j) {
-            const uint32_t c = base + threadIdx.x + j * SEL_T;
-            if (c < n_cand) {
-                const float v = cv[c]; const int i = ci[c];
-                if (i >= 0 && better(v, i, val[j], key[j])) { val[j] = v; key[j] = i; }
-            }
-        }
+    extern __shared__ unsigned char sel_sm[];
+    unsigned char* head = sel_sm;                       // [groups] candidates of a group that are taken; each thread its own groups
+    if (in_shared) {
+        float* v = reinterpret_cast<float*>(sel_sm + ((groups + 15) & ~15u));
+        int* i = reinterpret_cast<int*>(v + n_cand);
+        for (uint32_t c = threadIdx.x; c < n_cand; c += SEL_T) { v[c] = cv[c]; i[c] = ci[c]; }
+        cv = v; ci = i;
     }
-    block_topk(val, key, k, out_v, out_i, sv, si);
+    for (uint32_t q = threadIdx.x; q < groups; q += SEL_T) head[q] = 0;
+    __syncthreads();
+    float mv = SNEG; int mi = -1; uint32_t mg = 0;      // the best head of this thread's groups
+    auto look = [&]() {
+        mv = SNEG; mi = -1;
+        for (uint32_t q = threadIdx.x; q < groups; q += SEL_T) {
+            const uint32_t c = q * k + head[q];
+            if (head[q] < k && ci[c] >= 0 && better(cv[c], ci[c], mv, mi)) { mv = cv[c]; mi = ci[c]; mg = q; }
+        }
+    };
+    look();
+    for (uint32_t r = 0; r < k; ++r) {
+        float bv = mv; int bi = mi;
+        block_best(bv, bi, sv, si);
+        if (bi >= 0 && bi == mi) { ++head[mg]; look(); }        // rows are unique across groups
+        if (threadIdx.x == 0) { out_v[r] = bi < 0 ? SNEG : bv; out_i[r] = bi; }
+    }
+    __syncthreads();
     if (threadIdx.x >= 32) return;
     const uint32_t lane = threadIdx.x;
     uint32_t n = 0;
@@ -249,7 +260,11 @@ int launch_sample(const float* logits, uint32_t V, uint32_t batch, uint32_t k, f
         s_cand_n = need;
     }
     k_sample_stage1<<<dim3(groups, batch), SEL_T, 0, g.stream>>>(logits, V, k, pos, prompt_len, prompt_tok, gen_log, ld, penalty, on_prompt, s_cand_v, s_cand_i);
-    k_sample_stage2<<<batch, SEL_T, 0, g.stream>>>(s_cand_v, s_cand_i, groups * k, k, temperature, top_p, seed, pos, cur_tok, cur_val, gen_log, ld, nullptr);
+    const size_t heads = (groups + 15) & ~(size_t)15, all = heads + (size_t)groups * k * 8;
+    const bool in_shared = all <= 160 * 1024;           // 82 KB at a vocabulary of 262144 and k = 64
+    if (cudaFuncSetAttribute(k_sample_stage2, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
+        return fail(ADAMAH_ERR_BACKEND, "sampling: cannot raise the shared-memory limit");
+    k_sample_stage2<<<batch, SEL_T, in_shared ? all : heads, g.stream>>>(s_cand_v, s_cand_i, groups, k, in_shared ? 1 : 0, temperature, top_p, seed, pos, cur_tok, cur_val, gen_log, ld, nullptr);
     count_launch(2);
     return check_launch("decoder sampling");
 }

@@ -523,3 +523,27 @@ def test_device_sampling_mode(gpu):
         assert gpu.device_error() == 0
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize("n_vocab,k", [(2048, 64), (131072, 64), (262144, 40), (300032, 64)])
+def test_sampling_ranks_every_candidate(gpu, n_vocab, k):
+    """Vocabularies whose groups of 2048 rows give fewer and more than 2048 candidates: each id is the one that the rule draws
+    from the k best of all logits (nearly equal weights, so that one candidate left out moves the draws behind it)."""
+    cfg = _cfg(dict(n_layer=1, n_vocab=n_vocab))
+    tensors = synth.build_model(cfg, gb.GGML_TYPE_Q4_0, seed=46)
+    prompt = [int(t) for t in synth.random_prompt(cfg.n_vocab, 5, seed=4)]
+    T, seed, n = np.float32(8.0), 77, 24
+    eng = ADAMEngine(gpu, cfg, tensors, kv_cap=32, kv_dtype="f32")
+    try:
+        ids, st = eng.generate(prompt, GenerationConfig(max_tokens=n, temperature=float(T), top_k=k, top_p=1.0, repeat_penalty=1.0, seed=seed, eos_token_ids=()))
+        assert st["sampling_mode"] == "gpu_fused_topk"
+        logits = eng.logits_trace(prompt + ids[:-1], by_steps=True)[len(prompt) - 1:]
+        for i, lg in enumerate(logits):
+            order = np.lexsort((np.arange(lg.size), -lg))[:k]
+            cdf = np.cumsum(np.exp((lg[order] - lg[order[0]]) / T), dtype=np.float32)
+            target = np.float32(_splitmix_uniform(seed, 0, len(prompt) + i) * cdf[-1])
+            if np.abs(cdf - target).min() > 1e-3:            # (a draw that lands on a boundary may round either way)
+                assert ids[i] == order[int(np.argmax(target < cdf))], f"step {i}"
+        assert gpu.device_error() == 0
+    finally:
+        eng.close()
