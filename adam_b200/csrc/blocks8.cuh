@@ -41,5 +41,7 @@ const BlockKind* block_kind(uint32_t ggml_type);                 // NULL if the 
 int check_block_range(const Map* m, uint32_t id, const BlockKind* k, uint32_t ggml_type, uint64_t elem_off, uint64_t n_bytes);
 // Enqueue the placement of n_bytes of file blocks that already lie on the device (2-byte aligned).
 int place_blocks_from_device(Map* m, const BlockKind& k, uint64_t elem_off, const void* dev_src, uint64_t n_bytes);
+// End of an upload of n_bytes of blocks at elem_off: looks their scales over (Map::wide) and waits until all has landed.
+int settle_blocks(Map* m, const BlockKind& k, uint64_t elem_off, uint64_t n_bytes);
 
 }  // namespace ab

@@ -41,6 +41,7 @@ struct Map {
     uint4*    b8_q;        // GGUF_Q8_0 / GGUF_Q5_0 planes (inside buf)
     uint32_t* b8_h;
     __half*   b8_d;
+    bool     wide;         // GGUF blocks: some weights were uploaded that the tcgen05 GEMM's fp16 operands cannot hold
 };
 
 struct Handle {

@@ -13,7 +13,8 @@
 //         the tensor core rounds off is relative to them (256 x 5376, 9 rows of N(1, 1): 3.7e-5 of the result; the test asks for 5e-6).
 //   Q8_0  w = d q: 19 bits, as Q4_0
 // and w_hi x_hi + w_lo x_hi + w_hi x_lo is accumulated over K in fp32 (w_lo x_lo lies below 2^-22 of the product).
-// Limit, what fp16 holds: 8 d (Q4_0), 128 d (Q8_0), 8 d sc and 32 |8 d sc - dmin m| (Q4_K) below 65504.
+// Limit, what fp16 holds: 8 d (Q4_0), 128 d (Q8_0), 8 d sc and 32 |8 d sc - dmin m| (Q4_K) below 65504.  Uploads look for
+// blocks beyond it, and tensors of a map that got one stay on the GEMV kernels.
 //
 // Two kernels:
 //   k_quant_rows  one CTA per activation row: the optional input chain (residual add + RMS norms, as the GEMV prologue),
@@ -937,8 +938,9 @@ static int tc_rows_from(int wtype, const GemvArgs& a, bool pair, bool tiled) {
     return bytes > 10.0e6 ? 6 : 9;
 }
 
-bool gemm_tc_supports(int wtype, const GemvArgs& a, bool tiled) {
+bool gemm_tc_supports(int wtype, const GemvArgs& a, bool tiled, bool wide) {
     const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU;
+    if (wide) return false;
     if (wtype != WT_Q4_0 && wtype != WT_Q4_K && (wtype != WT_Q8_0 || pair)) return false;
     if (a.B < TC_MIN_ROWS || a.K <= 0 || a.K > TC_MAX_K || a.N < 16 || (!a.y && a.epi != EPI_ARGMAX) || (wtype == WT_Q4_K ? (a.K % 256) : (a.K % 32))) return false;
     if (a.epi == EPI_ARGMAX && a.B > tc_rows_fit(wtype, a.K)) return false;

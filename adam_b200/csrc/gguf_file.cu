@@ -81,6 +81,6 @@ extern "C" int adam_b200_upload_gguf_file(uint32_t map_wt, uint32_t ggml_type, u
         done += take;
     }
     close(fd);
-    if (cudaStreamSynchronize(g.stream) != cudaSuccess && rc == ADAMAH_OK) rc = fail(ADAMAH_ERR_BACKEND, "upload_gguf_file: %s", cudaGetErrorString(cudaGetLastError()));
-    return rc ? rc : check_launch("adam_b200_upload_gguf_file");
+    const int end = settle_blocks(m, *k, elem_off, n_bytes);
+    return rc ? rc : end;
 }

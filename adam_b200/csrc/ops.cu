@@ -552,7 +552,7 @@ int run_gemv(uint32_t map_id, uint64_t off, int wtype, GemvArgs& ga) {
         // many rows: the tcgen05 GEMM (its workspace is allocated on first use, never inside a capture)
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(g.stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) gemm_tc_prepare(ga.B, ga.K);
-        if (gemm_tc_supports(wtype, ga, find_tiled(map_id, off, (uint32_t)ga.N, (uint32_t)ga.K) != nullptr)) return launch_gemm_tc(wtype, ga, g.stream);
+        if (gemm_tc_supports(wtype, ga, find_tiled(map_id, off, (uint32_t)ga.N, (uint32_t)ga.K) != nullptr, g.maps[map_id].wide)) return launch_gemm_tc(wtype, ga, g.stream);
     }
     if (wt_is_b8(wtype)) {
         // Q8_0 / Q5_0: plain products from their own kernel; an arg-max is a second small kernel over the logits

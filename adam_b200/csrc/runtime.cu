@@ -749,6 +749,32 @@ int place_blocks_from_device(Map* m, const BlockKind& k, uint64_t elem_off, cons
     }
     return launch_repack_b8(k.ggml_type == 8 ? WT_Q8_0 : WT_Q5_0, dev_src, b8_ref(m, b0), nb, g.stream);
 }
+// Is a block's largest possible weight, or what a Q4_K block is taken apart into, more than fp16 holds (gemm_tc.cu)?  NaN counts.
+__global__ void k_find_wide(const Map m, uint64_t b0, uint64_t n, uint32_t* __restrict__ found) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    bool fits = true;
+    if (m.dtype == ADAMAH_DTYPE_GGUF_Q4_0) fits = 8.f * fabsf(__half2float(m.q40_d[b0 + i])) < 65504.f;
+    else if (m.dtype == ADAMAH_DTYPE_GGUF_Q8_0) fits = 128.f * fabsf(__half2float(m.b8_d[b0 + i])) < 65504.f;
+    else if (m.dtype == ADAMAH_DTYPE_GGUF_Q4_K) {       // codes and minima are 6 bits each
+        const __half2 d = *reinterpret_cast<const __half2*>((const uint8_t*)m.buf + (b0 + i) * 144);
+        fits = 32.f * 63.f * (8.f * fabsf(__low2float(d)) + fabsf(__high2float(d))) < 65504.f;
+    }
+    if (!fits) atomicOr(found, 1u);
+}
+int settle_blocks(Map* m, const BlockKind& k, uint64_t elem_off, uint64_t n_bytes) {
+    const uint64_t nb = n_bytes / k.bytes, b0 = elem_off / k.elems;
+    uint32_t *word = nullptr, found = 0;
+    CU(cudaMallocAsync((void**)&word, 4, g.stream));
+    CU(cudaMemsetAsync(word, 0, 4, g.stream));
+    k_find_wide<<<blocks_for(nb, 256), 256, 0, g.stream>>>(*m, b0, nb, word);
+    count_launch();
+    CU(cudaMemcpyAsync(&found, word, 4, cudaMemcpyDeviceToHost, g.stream));
+    CU(cudaFreeAsync(word, g.stream));
+    CU(cudaStreamSynchronize(g.stream));
+    m->wide |= found != 0;
+    return check_launch("upload of blocks");
+}
 int check_block_range(const Map* m, uint32_t id, const BlockKind* k, uint32_t ggml_type, uint64_t elem_off, uint64_t n_bytes) {
     if (!k || m->dtype != k->dtype) return fail(ADAMAH_ERR_INVALID, "ggml type %u does not match the storage of map %u", ggml_type, id);
     if (elem_off % k->elems || n_bytes % k->bytes) return fail(ADAMAH_ERR_INVALID, "%s upload must cover whole %u-byte blocks", k->name, k->bytes);
@@ -769,8 +795,7 @@ extern "C" int map_upload_gguf_blocks(uint32_t id, uint32_t ggml_type, uint64_t 
     cudaGetLastError();
     if (ggml_type == 12 && !on_dev) {          // file layout kept: straight to its place
         CU(cudaMemcpyAsync((uint8_t*)m->buf + elem_off / 256 * 144, raw, n_bytes, cudaMemcpyHostToDevice, g.stream));
-        CU(cudaStreamSynchronize(g.stream));
-        return ADAMAH_OK;
+        return settle_blocks(m, *k, elem_off, n_bytes);
     }
     void* tmp = nullptr;
     if (!on_dev) {
@@ -779,8 +804,8 @@ extern "C" int map_upload_gguf_blocks(uint32_t id, uint32_t ggml_type, uint64_t 
     }
     rc = place_blocks_from_device(m, *k, elem_off, tmp ? tmp : raw, n_bytes);
     if (tmp) cudaFreeAsync(tmp, g.stream);
-    CU(cudaStreamSynchronize(g.stream));
-    return rc ? rc : check_launch("map_upload_gguf_blocks");
+    const int end = settle_blocks(m, *k, elem_off, n_bytes);
+    return rc ? rc : end;
 }
 
 extern "C" int map_dequant_gguf(uint32_t id, uint64_t elem_off, float* out, uint64_t n_elems) {

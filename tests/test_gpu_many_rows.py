@@ -92,6 +92,20 @@ def test_q8_0_products_are_fp32_sums(gpu, B):
     assert np.linalg.norm(y - ref) < 1.5e-7 * np.linalg.norm(ref)
 
 
+@pytest.mark.parametrize("ggml_type,K,scale", [(2, 256, 9000.0), (2, 256, -65504.0), (12, 512, 200.0), (12, 512, 65504.0)])
+def test_weights_beyond_fp16(gpu, ggml_type, K, scale):
+    """One block whose weights fp16 cannot hold, among ordinary ones: many rows of activations give what the GEMV gives for one."""
+    N, B = 64, 16
+    rng = np.random.default_rng(K)
+    raw = {2: gb.random_q4_0_blocks, 12: gb.random_q4_k_blocks}[ggml_type](rng, N, K).copy()
+    blocks = raw.reshape(-1, {2: 18, 12: 144}[ggml_type])
+    blocks[7, 0:2] = np.array([scale], np.float16).view(np.uint8)
+    x = rng.standard_normal((B, K), dtype=np.float32)
+    y = _gemv(gpu, ggml_type, raw, N, K, x).astype(np.float64)
+    ref = x.astype(np.float64) @ q4_blocks.dequant(raw.reshape(-1), ggml_type, N, K).astype(np.float64).T
+    assert (np.linalg.norm(y - ref, axis=0) <= 2e-5 * np.linalg.norm(ref, axis=0)).all()
+
+
 def test_gemm_calls_from_several_threads(gpu):
     """Products of four threads share one image of activations; each thread has a map, handles and rows of its own."""
     import threading
