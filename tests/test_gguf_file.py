@@ -17,7 +17,7 @@ from adam_b200.gguf_file import GGUFLoader, QUANT_INFO
 
 from tests.golden.make_golden import GGUF_FILE_BUILD, GGUF_FILE_CFG, write_model_gguf
 
-REFERENCE = os.environ.get("ADAM_REFERENCE_DIR", "/root/reference")
+REFERENCE = os.environ.get("ADAM_REFERENCE_DIR", os.path.join(os.path.dirname(__file__), "..", "..", "reference"))
 
 
 @pytest.fixture()

@@ -32,11 +32,13 @@ def test_gemm_tiles(gpu, ggml_type, N, K, B):
     rng = np.random.default_rng(N + K + B)
     raw = {2: gb.random_q4_0_blocks, 8: gb.random_q8_0_blocks, 12: gb.random_q4_k_blocks}[ggml_type](rng, N, K)
     x = rng.standard_normal((B, K), dtype=np.float32) * rng.uniform(0.01, 100.0, (B, 1)).astype(np.float32)
+    before = gpu.tc_gemm_count()
     gpu.tc_gemm_policy(2)
     try:
         y = (_matmul(gpu, 8, A.DTYPE_GGUF_Q8_0, raw, N, K, x) if ggml_type == 8 else _gemv(gpu, ggml_type, raw, N, K, x)).astype(np.float64)
     finally:
         gpu.tc_gemm_policy(1)
+    assert gpu.tc_gemm_count() == before + 1             # it is the GEMM that ran
     ref = x.astype(np.float64) @ q4_blocks.dequant(raw.reshape(-1), ggml_type, N, K).astype(np.float64).T
     assert (np.linalg.norm(y - ref, axis=1) / np.linalg.norm(ref, axis=1)).max() < 5e-6
     assert gpu.device_error() == 0
@@ -155,6 +157,11 @@ def test_batched_head_and_ragged_prefill_match_the_oracle(gpu, batch):
     prompts = [synth.random_prompt(cfg.n_vocab, n, seed=100 + i) for i, n in enumerate(lens)]
     eng = ADAMEngine(gpu, cfg, tensors, kv_cap=80, kv_dtype="f32", max_batch=batch)
     try:
+        eng.begin(prompts, [max(lens) + 3] * batch)
+        eng.step(1, lm_head=False)
+        before = gpu.tc_gemm_count()
+        eng.step(1, lm_head=True, direct=True)
+        assert gpu.tc_gemm_count() == before + 4 * cfg.n_layer + 1          # four products per layer and the head
         outs, _ = eng.generate_batch(prompts, GenerationConfig(max_tokens=3, **GREEDY))
         for p, o in list(zip(prompts, outs))[:: max(1, batch // 8)]:
             assert o == OracleDecoder(cfg, f32, kv_cap=80).generate(p, 3)[0]
@@ -198,16 +205,17 @@ def test_prompt_attention_tiles(gpu, head_dim, n_head, n_kv, window, lens, kv_dt
     prompts = [synth.random_prompt(cfg.n_vocab, n, seed=70 + n) for n in lens]
     eng = ADAMEngine(gpu, cfg, tensors, kv_cap=max(lens) + 8, kv_dtype=kv_dtype, max_batch=len(lens), window=window > 0)
     try:
+        eng.begin(prompts, [max(lens) + 2] * len(lens))  # first: the steps would leave the right keys and values in the cache
+        gpu.batch_begin(); eng.prefill_prompts(prompts, 0); eng.step(1, lm_head=True, logits=True); gpu.batch_end()
+        got = [eng.read_logits(b) for b in range(len(lens))]
         want = []
         for p in prompts:
             eng.begin([p], [len(p) + 2])
             gpu.batch_begin(); eng.step(len(p) - 1, lm_head=False); eng.step(1, lm_head=True, logits=True); gpu.batch_end()
             want.append(eng.read_logits(0))
-        eng.begin(prompts, [max(lens) + 2] * len(lens))
-        gpu.batch_begin(); eng.prefill_prompts(prompts, 0); eng.step(1, lm_head=True, logits=True); gpu.batch_end()
         tol = 1e-3 if kv_dtype == "f16" else 2e-5
-        for b, w in enumerate(want):
-            assert np.abs(eng.read_logits(b) - w).max() <= tol * np.abs(w).max()
+        for g, w in zip(got, want):
+            assert np.abs(g - w).max() <= tol * np.abs(w).max()
         assert gpu.device_error() == 0
     finally:
         eng.close()
@@ -220,12 +228,13 @@ def test_score_equals_steps(gpu, n):
     toks = synth.random_prompt(cfg.n_vocab, n, seed=5)
     eng = ADAMEngine(gpu, cfg, tensors, kv_cap=160, kv_dtype="f32")
     try:
+        got = eng.logits_trace(toks)                     # first: the steps would leave the right keys and values in the cache
         eng.begin([toks], [n])
         want = []
         for _ in range(n):
             eng.step(1, lm_head=True, logits=True)
             want.append(eng.read_logits(0))
-        got, want = eng.logits_trace(toks), np.stack(want)
+        want = np.stack(want)
         assert np.abs(got - want).max() <= 2e-5 * np.abs(want).max()
     finally:
         eng.close()

@@ -1,6 +1,6 @@
 """The reference's OWN ctypes binding (adamah-MAIN/adamah/__init__.py) over libadam_b200.so, selected the way a user
 of the reference would select it: the ADAMAH_LIB_PATH variable (__init__.py:156-161).  CPU only; needs a checkout of the
-reference beside the repository (ADAM_REFERENCE_DIR, default /root/reference) and is skipped without one."""
+reference beside the repository (or at ADAM_REFERENCE_DIR) and is skipped without one."""
 import ctypes
 import importlib.util
 import os
@@ -10,7 +10,7 @@ import pytest
 
 from adam_b200 import _lib
 
-REFERENCE = os.environ.get("ADAM_REFERENCE_DIR", "/root/reference")
+REFERENCE = os.environ.get("ADAM_REFERENCE_DIR", os.path.join(os.path.dirname(__file__), "..", "..", "reference"))
 BINDING = os.path.join(REFERENCE, "adamah-MAIN", "adamah", "__init__.py")
 
 pytestmark = pytest.mark.skipif(not os.path.isfile(BINDING), reason="no checkout of the reference")
