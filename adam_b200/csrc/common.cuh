@@ -70,6 +70,7 @@ struct Context {
     uint64_t     submits;       // stream synchronisations that closed a batch
     uint64_t     flushes;
     uint32_t*    dev_err;       // device error word
+    uint32_t*    wide;          // [MAX_MAPS] device words: what the look at an upload's scales found (settle_blocks)
     bool         pdl;           // launch with programmatic stream serialization (set by the decoder while it enqueues a step)
 };
 

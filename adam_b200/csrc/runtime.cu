@@ -234,6 +234,7 @@ extern "C" int adamah_init_ex(uint64_t, uint64_t) {
     if (!g.handles) return fail(ADAMAH_ERR_MEMORY, "out of host memory");
     CU(cudaMalloc(&g.dev_err, sizeof(uint32_t)));
     CU(cudaMemset(g.dev_err, 0, sizeof(uint32_t)));
+    CU(cudaMalloc(&g.wide, MAX_MAPS * sizeof(uint32_t)));
     g.handle_cursor = 1;
     g.active_dtype = ADAMAH_DTYPE_F32;
     g.sched_mode = 2;
@@ -265,6 +266,7 @@ extern "C" void adamah_shutdown(void) {
     for (uint32_t i = 0; i < MAX_HANDLES; ++i) if (g.handles[i].used) { cudaFree(g.handles[i].dev); free(g.handles[i].shadow); }
     free(g.handles);
     cudaFree(g.dev_err);
+    cudaFree(g.wide);
     cudaStreamDestroy(g.own_stream);
     memset(&g, 0, sizeof g);
 }
@@ -764,13 +766,12 @@ __global__ void k_find_wide(const Map m, uint64_t b0, uint64_t n, uint32_t* __re
 }
 int settle_blocks(Map* m, const BlockKind& k, uint64_t elem_off, uint64_t n_bytes) {
     const uint64_t nb = n_bytes / k.bytes, b0 = elem_off / k.elems;
-    uint32_t *word = nullptr, found = 0;
-    CU(cudaMallocAsync((void**)&word, 4, g.stream));
+    uint32_t* word = g.wide + (m - g.maps);
+    uint32_t found = 0;
     CU(cudaMemsetAsync(word, 0, 4, g.stream));
     k_find_wide<<<blocks_for(nb, 256), 256, 0, g.stream>>>(*m, b0, nb, word);
     count_launch();
     CU(cudaMemcpyAsync(&found, word, 4, cudaMemcpyDeviceToHost, g.stream));
-    CU(cudaFreeAsync(word, g.stream));
     CU(cudaStreamSynchronize(g.stream));
     m->wide |= found != 0;
     return check_launch("upload of blocks");
