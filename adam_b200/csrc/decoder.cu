@@ -88,7 +88,11 @@ struct Decoder {
 constexpr uint32_t MAX_DECODERS = 8;
 constexpr uint32_t ATTN_SPLIT = 64;        // fewest tokens an attention CTA takes before another CTA is added
 constexpr uint32_t ATTN_MAX_SPLITS = 64;   // attention CTAs per (sequence, kv head)
-constexpr uint32_t PREFILL_ROWS = 1024;    // rows (sequences x tokens) of one prefill chunk
+// Rows (sequences x tokens) of one prefill chunk, the same for every shape.  512 / 1024 / 2048 rows: 32 prompts x 512 and their
+// 24 steps at the 1B shape 185 / 147 / 135 ms, one prompt of 1500 tokens with 12 steps 32.3 / 28.5 / 24.5 ms, 64 x 128 at the 27B
+// shape (8 layers) 222 / 222 / 229 ms: the narrow model gains from 2048 (its 1152-row products are 72 tiles on 148 SMs at 1024),
+// the wide one loses.
+constexpr uint32_t PREFILL_ROWS = 1024;
 static Decoder* g_dec[MAX_DECODERS];
 
 static Decoder* get_dec(uint32_t id) {
@@ -1202,10 +1206,8 @@ extern "C" int adam_b200_decoder_create(const adam_b200_decoder_desc* desc, uint
     const uint64_t most = (uint64_t)d.max_batch * d.kv_cap;     // no more prompt rows than that exist
     D->rows_cap = (uint32_t)(most < PREFILL_ROWS ? (most > 64 ? most : 64) : PREFILL_ROWS);
     if (D->rows_cap < d.max_batch) D->rows_cap = d.max_batch;
-    const size_t B = d.max_batch, R = D->rows_cap, E = d.n_embd, q_dim = (size_t)d.n_head * d.head_dim, k_dim = (size_t)d.n_head_kv * d.head_dim;
+    const size_t B = d.max_batch, E = d.n_embd, q_dim = (size_t)d.n_head * d.head_dim, k_dim = (size_t)d.n_head_kv * d.head_dim;
     const uint32_t gs = d.n_head / d.n_head_kv;
-    // workspace of the many-row GEMM (without it those rows run on the GEMV kernels)
-    gemm_tc_prepare((int)D->rows_cap, (int)(d.n_ff > E ? (d.n_ff > q_dim ? d.n_ff : q_dim) : (E > q_dim ? E : q_dim)));
     g_dec[id] = D;
 #define DALLOC(p, bytes) do { cudaError_t e__ = cudaMalloc((void**)&(p), (bytes)); if (e__ != cudaSuccess) { destroy(D); g_dec[id] = nullptr; \
         return fail(ADAMAH_ERR_MEMORY, "decoder_create: cudaMalloc(%zu) failed: %s", (size_t)(bytes), cudaGetErrorString(e__)); } } while (0)
@@ -1213,16 +1215,32 @@ extern "C" int adam_b200_decoder_create(const adam_b200_decoder_desc* desc, uint
     DALLOC(D->prompt_tok, B * d.kv_cap * 4); DALLOC(D->gen_log, B * d.kv_cap * 4);
     DALLOC(D->block_table, B * D->max_pages_per_seq * 4);
     DALLOC(D->kv_pool, (size_t)D->n_pages * D->page_elems * kv_elem_size(d));
-    DALLOC(D->hbuf[0], R * E * 4); DALLOC(D->hbuf[1], R * E * 4); DALLOC(D->qkv, R * (q_dim + 2 * k_dim) * 4);
-    DALLOC(D->attn_out, R * q_dim * 4); DALLOC(D->proj, R * E * 4);
-    DALLOC(D->act, R * d.n_ff * 4); DALLOC(D->logits, B * (size_t)d.n_vocab * 4);
+    DALLOC(D->logits, B * (size_t)d.n_vocab * 4);
     DALLOC(D->part_o, B * d.n_head_kv * D->n_splits * gs * d.head_dim * 4);
     DALLOC(D->part_ml, B * d.n_head_kv * D->n_splits * gs * 2 * 4);
     DALLOC(D->attn_ticket, B * d.n_head * 4);
-    DALLOC(D->even_plan, R * (8 + sizeof(AttnTile)));
+    // Buffers of a chunk's rows: 205 MB at the 27B shape and 1024 rows, fewer rows where that much is not left.
+    struct { void** p; size_t row; } const bufs[7] = {{(void**)&D->hbuf[0], E * 4}, {(void**)&D->hbuf[1], E * 4}, {(void**)&D->qkv, (q_dim + 2 * k_dim) * 4},
+        {(void**)&D->attn_out, q_dim * 4}, {(void**)&D->proj, E * 4}, {(void**)&D->act, (size_t)d.n_ff * 4}, {(void**)&D->even_plan, 8 + sizeof(AttnTile)}};
+    const uint32_t fewest = std::max(64u, d.max_batch);
+    for (;;) {
+        int n = 0;
+        while (n < 7 && cudaMalloc(bufs[n].p, bufs[n].row * D->rows_cap) == cudaSuccess) ++n;
+        if (n == 7) break;
+        cudaGetLastError();
+        for (int i = 0; i < 7; ++i) { if (i < n) cudaFree(*bufs[i].p); *bufs[i].p = nullptr; }
+        if (D->rows_cap == fewest) {
+            const uint32_t rows = D->rows_cap;
+            destroy(D); g_dec[id] = nullptr;
+            return fail(ADAMAH_ERR_MEMORY, "decoder_create: out of device memory for %u rows of activations", rows);
+        }
+        D->rows_cap = std::max(fewest, D->rows_cap / 2);
+    }
 #undef DALLOC
+    // workspace of the many-row GEMM (without it those rows run on the GEMV kernels)
+    gemm_tc_prepare((int)D->rows_cap, (int)std::max(std::max((size_t)d.n_ff, E), q_dim));
     cudaMemsetAsync(D->attn_ticket, 0, B * d.n_head * 4, g.stream);
-    cudaMemsetAsync(D->even_plan, 0, R * (8 + sizeof(AttnTile)), g.stream);
+    cudaMemsetAsync(D->even_plan, 0, D->rows_cap * (8 + sizeof(AttnTile)), g.stream);
     cudaMemsetAsync(D->pos, 0, B * 4, g.stream);
     cudaMemsetAsync(D->cur_tok, 0, B * 4, g.stream);
     cudaMemsetAsync(D->cur_val, 0, B * 4, g.stream);

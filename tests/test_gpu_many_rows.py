@@ -303,6 +303,35 @@ def test_score_without_room_for_its_buffer(gpu, max_batch, left_mb):
     assert np.abs(got - want).max() <= 2e-5 * np.abs(want).max()
 
 
+def test_decoder_where_a_full_chunk_of_rows_does_not_fit(gpu):
+    """1024 rows of this model's activations take 67 MB; with 56 MB left on the device, enough for the model and the 64 rows that a
+    decoder cannot do without, it has smaller chunks and the same results."""
+    import torch
+    cfg = replace(tiny_gemma3(n_layer=1), n_ff=16384)
+    tensors = synth.build_model(cfg, gb.GGML_TYPE_Q4_0, seed=67)
+    toks = synth.random_prompt(cfg.n_vocab, 600, seed=9)
+    seen, filler, eng = [], None, None
+    for full in (False, True):
+        try:
+            if full:
+                torch.cuda.empty_cache()
+                filler = torch.empty(torch.cuda.mem_get_info()[0] - (56 << 20), dtype=torch.uint8, device="cuda")
+            eng = ADAMEngine(gpu, cfg, tensors, kv_cap=1024, kv_dtype="f32")
+            eng.begin([toks], [602])
+            eng.prefill(599)
+            eng.step(1, lm_head=True, logits=True)
+            seen.append(eng.read_logits(0))
+            assert gpu.device_error() == 0
+        finally:
+            del filler
+            filler = None
+            torch.cuda.empty_cache()
+            if eng is not None:
+                eng.close()
+                eng = None
+    assert np.abs(seen[0] - seen[1]).max() <= 2e-5 * np.abs(seen[0]).max()
+
+
 @pytest.mark.parametrize("n", [1, 16383, 16384, 262144, 262145, 1200000])
 def test_large_results_and_uploads(gpu, n):
     """Around the sizes where results move to page-locked blocks and uploads leave the ring; neighbouring locs and others; arrays
