@@ -380,7 +380,7 @@ class Adamah:
         return int(self._lib.adam_b200_kernel_launches())
 
     def tc_gemm_count(self) -> int:
-        """Matrix products enqueued so far on the tcgen05 GEMM (calls with 9..64 activation rows)."""
+        """Matrix products enqueued so far on the tcgen05 GEMM (calls with many activation rows)."""
         return int(self._lib.adam_b200_tc_gemm_count())
 
     def tc_gemm_policy(self, policy: int):

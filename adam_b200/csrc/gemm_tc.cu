@@ -1001,7 +1001,8 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
     }
     // Work split: the cheapest under an estimate in SM cycles.  A step costs the larger of its tensor-core time and what
     // the rebuilding of a weight tile allows.  Dealt out evenly, a CTA costs its stages and, where tiles are shared, the
-    // adding up of P partial results of nt columns; as clusters of S, waves of CTAs and one exchange.
+    // adding up of P partial results of nt columns; as clusters of S, waves of CTAs and one exchange.  One set of figures for
+    // all block types, although rebuilding a Q4_K weight takes longer than a Q4_0 one: they only rank the splits of one call.
     const int nt = a.B <= 16 ? 16 : a.B <= 32 ? 32 : a.B <= 64 ? 64 : 128, sp = nt == 128 ? 1 : 2;
     const int tiles_n = pair ? (a.N + 63) / 64 : (a.N + 127) / 128, tiles_m = (a.B + nt - 1) / nt;
     const long long items = (long long)tiles_n * tiles_m;

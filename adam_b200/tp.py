@@ -278,7 +278,7 @@ class ADAMEngineTP(ADAMEngine):
 
     def prefill(self, n_tokens: int, chunked: bool = True):
         """Consumes ``n_tokens`` prompt positions of every sequence without the LM head, in chunks of
-        up to 64 (sequence, position) rows per pass over this rank's weights, the partial sums of the
+        as many (sequence, position) rows as the projection buffer holds, the partial sums of the
         o- and down-projections (one row per chunk row) all-reduced after each half layer."""
         if n_tokens <= 0:
             return

@@ -67,7 +67,11 @@ uint32_t map_get_dtype(uint32_t id);
 /* adamah.c:4621 -- per-group (scale, zero) of a Q4 map */
 int      map_set_qparams(uint32_t id, const float* scales, const float* zeros, uint32_t n_groups);
 
-/* host <-> map: adamah.c:3087, :2896, :3035, :3374 */
+/* host <-> map: adamah.c:3087, :2896, :3035, :3374.
+ * The host data may be reused when a call returns.  What a scatter or map_upload_dev wrote is there for every later call
+ * of this library, and for the caller's work behind it on a stream lent with adam_b200_set_stream; adamah_sync waits until
+ * it has landed on the device (copies of up to 1 MB may still be under way when the call returns).  A gather or download
+ * has its result on return. */
 int      map_scatter(uint32_t id, const uint32_t* locs, const void* data, uint32_t n_locs);
 int      map_scatter_contiguous(uint32_t id, uint32_t start_pack, const void* data, uint32_t n_locs);
 int      map_scatter_q4_packed_contiguous(uint32_t id, uint32_t start_pack, const void* packed_u8, uint32_t n_locs);
@@ -423,6 +427,8 @@ int adam_b200_decoder_buffer_ptr(uint32_t id, uint32_t which, uint64_t* ptr_out,
 int adam_b200_decoder_read_state(uint32_t id, int32_t* pos_out, int32_t* cur_tok_out);   /* [max_batch] each, may be NULL */
 int adam_b200_decoder_read_log(uint32_t id, uint32_t seq, uint32_t first_pos, uint32_t n, int32_t* out);
 int adam_b200_decoder_read_logits(uint32_t id, uint32_t seq, float* out);                 /* [n_vocab] */
+/* Rows of the last step's buffers (what = 0 hidden state, 2 q/k/v, 4 attention output, 5 projection, 6 activation); behind a
+ * prompt chunk or a scored text the query part of 2 is normalised and rotated. */
 int adam_b200_decoder_read_buffer(uint32_t id, uint32_t what, uint32_t seq, float* out, uint32_t n);
 
 #ifdef __cplusplus
