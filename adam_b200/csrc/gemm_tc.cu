@@ -105,7 +105,9 @@ __device__ __forceinline__ void split_half(float v, __half& hi, __half& lo) {
     lo = __float2half_rn(v - __half2float(hi));
 }
 
-template <int MAXV, bool CHAIN>
+// FEW: the image of gemm_mma.cu instead: per 32 values of K the rows' 2 x 32 halves in the order of its B fragments, for
+// Q4_K (n_min > 0) followed by a float per row, the sum of the 32 values; n_steps is then the number of rows it has room for.
+template <int MAXV, bool CHAIN, bool FEW>
 __global__ void __launch_bounds__(512) k_quant_rows(const GemvArgs a, uint8_t* __restrict__ img, float* __restrict__ inv_out, int n_min, int n_steps) {
     __shared__ float red[66];
     const int r = blockIdx.x, tid = threadIdx.x, K = a.K, n4 = K >> 2, nt = blockDim.x;
@@ -173,6 +175,30 @@ __global__ void __launch_bounds__(512) k_quant_rows(const GemvArgs a, uint8_t* _
     pow2_scale(am, s, inv);                             // largest element in (2^21, 2^22] ...
     s *= 0.0078125f; inv *= 128.f;                      // ... in (2^14, 2^15]
     if (tid == 0) inv_out[r] = inv;
+    if constexpr (FEW) {
+        const int blk = gm_block_bytes(n_min ? WT_Q4_K : WT_Q4_0, n_steps);
+#pragma unroll
+        for (int j = 0; j < MAXV; ++j) {
+            const int i = tid + j * nt;                 // values 4 i .. 4 i + 3: piece i & 3 of the low or high half of block i >> 3
+            const float4 f = make_float4(v[j].x * s, v[j].y * s, v[j].z * s, v[j].w * s);
+            uint8_t* d = img + (size_t)(i >> 3) * blk;
+            if (i < n4) {
+                __half h[4], l[4];
+                split_half(f.x, h[0], l[0]); split_half(f.z, h[1], l[1]); split_half(f.y, h[2], l[2]); split_half(f.w, h[3], l[3]);
+                uint2* q = reinterpret_cast<uint2*>(d) + (r * 8 + (i & 3)) * 2 + ((i >> 2) & 1);
+                q[0] = *reinterpret_cast<const uint2*>(h);
+                q[8] = *reinterpret_cast<const uint2*>(l);
+            }
+            if (n_min) {
+                float t = (f.x + f.y) + (f.z + f.w);
+                t += __shfl_xor_sync(0xffffffffu, t, 1);
+                t += __shfl_xor_sync(0xffffffffu, t, 2);
+                t += __shfl_xor_sync(0xffffffffu, t, 4);
+                if (i < n4 && (i & 7) == 0) reinterpret_cast<float*>(d + 128 * n_steps)[r] = t;
+            }
+        }
+        return;
+    }
     const int r64 = r & 63;
     uint8_t* base = img + (size_t)(r >> 6) * n_steps * (2 * TC_STEP_IMG);
     auto put4 = [&](int k0, float4 f) {                 // values k0 .. k0+3, already scaled
@@ -938,15 +964,33 @@ static int tc_rows_from(int wtype, const GemvArgs& a, bool pair, bool tiled) {
     return bytes > 10.0e6 ? 6 : 9;
 }
 
-bool gemm_tc_supports(int wtype, const GemvArgs& a, bool tiled, bool wide) {
+// Does the call take the mma.sync kernel (gemm_mma.cu)?  Matrices above 10 MB from 3 rows to 16, smaller ones and the heads of
+// narrow models from 5 to 8.  us a call, row kernel included, with it and without (GEMV up to 5 rows, above that k_gemm_tc), by rows:
+//   21504 x 5376 Q4_K   2: 26.7, 24.2   4: 26.7, 32.7   8: 29.8, 46.9   16: 42.2, 47.4   32: 75, 54.5
+//   5376 x 21504 Q4_K   2: 30.3, 36.5   4: 30.6, 60.5   8: 38.2, 54.1   16: 47.8, 55.0   32: 77, 61.9
+//   1152 x 6912 Q4_0    4: 6.1, 8.2     8: 7.7, 10.1    12: 9.3, 9.9    16: 10.7, 10.0
+//   6912 x 1152 Q4_0    4: 4.7, 7.5     8: 5.4, 9.0     16: 7.3, 8.7
+//   262144 x 1152 Q4_0  4: 48.5, 40.9   8: 65.6, 91.2   12: 86, 91.7    16: 108, 92.0
+// and ms a decode step: 1B shape 4 rows 0.887 and 0.894, 5 to 8 rows 1.04 and 1.12 to 1.15, 10 rows 1.226 and 1.220, 16 rows 1.365
+// and 1.242; 27B shape (8 layers) 2 rows 1.16 and 1.05, 3 rows 1.18 and 1.52, 8 rows 1.42 and 2.08, 16 rows 2.16 and 2.25.
+static bool takes_mma(int wtype, const GemvArgs& a, const uint8_t* t0, const uint8_t* t1) {
     const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU;
-    if (wide) return false;
+    if (!t0 || (pair && !t1) || g_tc_policy != 1 || !gemm_mma_supports(wtype, a)) return false;
+    const bool large = (double)a.N * a.K * 0.5625 * (pair ? 2 : 1) > 10.0e6 && !(a.epi == EPI_ARGMAX && a.K < 4096);
+    if (large ? a.B < 3 : a.B < 5 || a.B > 8) return false;
+    return (size_t)(a.K / 32) * gm_block_bytes(wtype, gemm_mma_pad(a.B)) <= g_tc.img_cap && gemm_mma_pad(a.B) <= g_tc.inv_cap;
+}
+
+bool gemm_tc_supports(int wtype, const GemvArgs& a, const uint8_t* t0, const uint8_t* t1, bool wide) {
+    const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU;
+    if (g_tc_policy < 0) g_tc_policy = getenv("ADAM_B200_TC") ? atoi(getenv("ADAM_B200_TC")) : 1;
     if (wtype != WT_Q4_0 && wtype != WT_Q4_K && (wtype != WT_Q8_0 || pair)) return false;
     if (a.B < TC_MIN_ROWS || a.K <= 0 || a.K > TC_MAX_K || a.N < 16 || (!a.y && a.epi != EPI_ARGMAX) || (wtype == WT_Q4_K ? (a.K % 256) : (a.K % 32))) return false;
     if (a.epi == EPI_ARGMAX && a.B > tc_rows_fit(wtype, a.K)) return false;
     if ((a.ldx & 3) || (!a.h_in && (!a.x || ((uintptr_t)a.x & 15)))) return false;
-    if (g_tc_policy < 0) g_tc_policy = getenv("ADAM_B200_TC") ? atoi(getenv("ADAM_B200_TC")) : 1;
-    if (g_tc_policy == 0 || (g_tc_policy == 1 && a.B < tc_rows_from(wtype, a, pair, tiled))) return false;
+    if (takes_mma(wtype, a, t0, t1)) return true;
+    if (wide) return false;
+    if (g_tc_policy == 0 || (g_tc_policy == 1 && a.B < tc_rows_from(wtype, a, pair, t0 && (t1 || !pair)))) return false;
     return tc_rows_fit(wtype, a.K) >= 128;
 }
 
@@ -980,25 +1024,28 @@ static int tc_clusters_at_once(int s) {
     return known[s];
 }
 
+// One CTA per row; the fewest float4 per thread that 512 threads allow.
+template <bool FEW> static void launch_quant_rows(const GemvArgs& a, int n_min, int n_steps, cudaStream_t stream) {
+    const int cand[5] = {1, 2, 4, 8, 16}, n4 = a.K / 4;
+    int mv = 16;
+    for (int c : cand) if ((n4 + c - 1) / c <= 512) { mv = c; break; }
+    const int threads = ((n4 + mv - 1) / mv + 31) / 32 * 32;
+    auto go = [&](auto kern) { launch_k(kern, dim3(a.B), dim3(threads), 0, stream, true, a, g_tc.img, g_tc.inv, n_min, n_steps); };
+    const bool chain = a.h_in != nullptr;
+    switch (mv) {
+    case 1: if (chain) go(k_quant_rows<1, true, FEW>); else go(k_quant_rows<1, false, FEW>); break;
+    case 2: if (chain) go(k_quant_rows<2, true, FEW>); else go(k_quant_rows<2, false, FEW>); break;
+    case 4: if (chain) go(k_quant_rows<4, true, FEW>); else go(k_quant_rows<4, false, FEW>); break;
+    case 8: if (chain) go(k_quant_rows<8, true, FEW>); else go(k_quant_rows<8, false, FEW>); break;
+    default: if (chain) go(k_quant_rows<16, true, FEW>); else go(k_quant_rows<16, false, FEW>); break;
+    }
+    count_launch();
+}
+
 static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
     const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU;
-    const int n_min = tc_min_steps(wtype, a.K), n_main = tc_main_steps(a.K), n4 = a.K / 4;
-    {   // one CTA per row; the fewest float4 per thread that 512 threads allow
-        const int cand[5] = {1, 2, 4, 8, 16};
-        int mv = 16;
-        for (int c : cand) if ((n4 + c - 1) / c <= 512) { mv = c; break; }
-        const int threads = ((n4 + mv - 1) / mv + 31) / 32 * 32;
-        auto go = [&](auto kern) { launch_k(kern, dim3(a.B), dim3(threads), 0, stream, true, a, g_tc.img, g_tc.inv, n_min, n_min + n_main); };
-        const bool chain = a.h_in != nullptr;
-        switch (mv) {
-        case 1: if (chain) go(k_quant_rows<1, true>); else go(k_quant_rows<1, false>); break;
-        case 2: if (chain) go(k_quant_rows<2, true>); else go(k_quant_rows<2, false>); break;
-        case 4: if (chain) go(k_quant_rows<4, true>); else go(k_quant_rows<4, false>); break;
-        case 8: if (chain) go(k_quant_rows<8, true>); else go(k_quant_rows<8, false>); break;
-        default: if (chain) go(k_quant_rows<16, true>); else go(k_quant_rows<16, false>); break;
-        }
-        count_launch();
-    }
+    const int n_min = tc_min_steps(wtype, a.K), n_main = tc_main_steps(a.K);
+    launch_quant_rows<false>(a, n_min, n_min + n_main, stream);
     // Work split: the cheapest under an estimate in SM cycles.  A step costs the larger of its tensor-core time and what
     // the rebuilding of a weight tile allows.  Dealt out evenly, a CTA costs its stages and, where tiles are shared, the
     // adding up of P partial results of nt columns; as clusters of S, waves of CTAs and one exchange.  One set of figures for
@@ -1053,8 +1100,15 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
 }
 
 // Rows that exceed the workspace run in chunks of whole 128-row tiles.
-int launch_gemm_tc(int wtype, const GemvArgs& a, cudaStream_t stream) {
+int launch_gemm_tc(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvArgs& a, cudaStream_t stream) {
     std::lock_guard<std::mutex> work(g_tc_lock);
+    if (takes_mma(wtype, a, t0, t1)) {
+        launch_quant_rows<true>(a, tc_min_steps(wtype, a.K), gemm_mma_pad(a.B), stream);
+        const int rc = launch_gemm_mma(wtype, t0, t1, a, GemmWork{g_tc.img, g_tc.inv, g_tc.part, g_tc.tickets, g_tc.best, (unsigned int*)(g_tc.best + g_tc.inv_cap)}, stream);
+        if (rc) return rc;
+        ++g_tc_calls;
+        return check_launch("gemm_mma");
+    }
     const int fit = tc_rows_fit(wtype, a.K);
     for (int b0 = 0; b0 < a.B; b0 += fit) {
         GemvArgs c = a;

@@ -10,12 +10,21 @@ constexpr int TC_MIN_ROWS = 2;         // fewer rows than this never leave the G
 
 // Does this problem run on the tcgen05 path?  `tiled`: the GEMV kernels would have row-tiled copies of the weights; `wide`:
 // the weights' map says that fp16 may not hold them.
-bool gemm_tc_supports(int wtype, const GemvArgs& a, bool tiled, bool wide);
+bool gemm_tc_supports(int wtype, const GemvArgs& a, const uint8_t* t0, const uint8_t* t1, bool wide);
 // Makes room for calls with up to `rows` activation rows of length K (outside any stream capture; longer calls run in
 // chunks).  The workspace only grows; false when out of memory.
 bool gemm_tc_prepare(int rows, int K);
 void gemm_tc_release();
 // Enqueues the row-quantisation kernel and the GEMM.  Returns ADAMAH_OK or an error code.
-int launch_gemm_tc(int wtype, const GemvArgs& a, cudaStream_t stream);
+int launch_gemm_tc(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvArgs& a, cudaStream_t stream);
+
+// ---- gemm_mma.cu: the second kernel of a call with few rows ----
+constexpr int GM_MAX_ROWS = 16;
+// Bytes of the activation image per 32 values of K, with room for `rows` rows (a multiple of four).
+__host__ __device__ constexpr int gm_block_bytes(int wtype, int rows) { return rows * (wtype == WT_Q4_K ? 132 : 128); }
+struct GemmWork { const uint8_t* img; const float* inv; float* part; unsigned int* tickets; unsigned long long* best; unsigned int* ticket; };
+bool gemm_mma_supports(int wtype, const GemvArgs& a);
+int gemm_mma_pad(int rows);            // rows the image has room for
+int launch_gemm_mma(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvArgs& a, const GemmWork& w, cudaStream_t stream);
 
 }  // namespace ab

@@ -552,7 +552,8 @@ int run_gemv(uint32_t map_id, uint64_t off, int wtype, GemvArgs& ga) {
         // many rows: the tcgen05 GEMM (its workspace is allocated on first use, never inside a capture)
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(g.stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) gemm_tc_prepare(ga.B, ga.K);
-        if (gemm_tc_supports(wtype, ga, find_tiled(map_id, off, (uint32_t)ga.N, (uint32_t)ga.K) != nullptr, g.maps[map_id].wide)) return launch_gemm_tc(wtype, ga, g.stream);
+        const uint8_t* t = (const uint8_t*)find_tiled(map_id, off, (uint32_t)ga.N, (uint32_t)ga.K);
+        if (gemm_tc_supports(wtype, ga, t, nullptr, g.maps[map_id].wide)) return launch_gemm_tc(wtype, t, nullptr, ga, g.stream);
     }
     if (wt_is_b8(wtype)) {
         // Q8_0 / Q5_0: plain products from their own kernel; an arg-max is a second small kernel over the logits

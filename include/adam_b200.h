@@ -387,11 +387,11 @@ void adam_b200_host_free(void* p);
  * this shard's partial sums.  No counterpart in the reference (it has no multi-GPU path). */
 int adam_b200_decoder_n_parts(uint32_t id);                                   /* 2*n_layer + 2, or a negative status */
 int adam_b200_decoder_step_part(uint32_t id, uint32_t part, uint32_t flags);
-/* Number of matrix products enqueued so far on the tcgen05 (tensor memory) GEMM, which takes calls
- * with many activation rows; calls with fewer rows run on the GEMV kernels. */
+/* Number of matrix products enqueued so far on the GEMM kernels: the tcgen05 (tensor memory) one, which takes calls with many
+ * activation rows, and the mma.sync one for a few rows over row-tiled weights; calls with fewer rows run on the GEMV kernels. */
 uint64_t adam_b200_tc_gemm_count(void);
 /* Which calls take it: 0 = none, 1 = those expected to be faster than the GEMV kernels (default; also the
- * initial value of environment variable ADAM_B200_TC), 2 = every call whose shape allows. */
+ * initial value of environment variable ADAM_B200_TC), 2 = every call whose shape allows, on the tcgen05 one. */
 int adam_b200_tc_gemm_policy(int policy);
 /* One part of one prefill chunk of n_tokens (batch * n_tokens rows, at least 64 are accepted) tokens per sequence: parts
  * 0 .. 2*n_layer-1 as above (the projection buffer then holds batch * n_tokens rows of partial

@@ -1,0 +1,73 @@
+"""Products of a few rows over row-tiled weights (the mma.sync GEMM): decode batches and short prompts."""
+import numpy as np
+import pytest
+
+import adam_b200 as A
+from adam_b200 import gguf_blocks as gb
+from oracle import q4_blocks
+
+from tests.test_gpu_gemv import _gemv
+
+pytestmark = pytest.mark.gpu
+
+
+def _error(gpu, ggml_type, raw, N, K, x, policy):
+    gpu.tc_gemm_policy(policy)
+    try:
+        y = _gemv(gpu, ggml_type, raw, N, K, x, tile=True).astype(np.float64)
+    finally:
+        gpu.tc_gemm_policy(1)
+    ref = x.astype(np.float64) @ q4_blocks.dequant(raw.reshape(-1), ggml_type, N, K).astype(np.float64).T
+    return np.linalg.norm(y - ref, axis=1) / np.linalg.norm(ref, axis=1)
+
+
+# Rows around the groups of four the kernel is built for; one row group and many; K of one tile pair, of a partial last
+# stage, and long; items shared between CTAs.
+@pytest.mark.parametrize("mean", [0.0, 1.0])
+@pytest.mark.parametrize("ggml_type,N,K,B", [
+    (2, 16, 64, 5), (2, 1152, 1152, 6), (2, 1536, 1152, 8), (2, 1152, 6912, 8), (2, 2400, 320, 7), (2, 1152, 1024, 5), (2, 4624, 4160, 13), (2, 16400, 1152, 15),
+    (2, 30720, 1152, 3), (12, 16, 256, 7), (12, 5392, 5376, 3), (12, 5376, 5632, 4), (12, 512, 5376, 5), (12, 5376, 1280, 8), (12, 1152, 21504, 9), (12, 5376, 21504, 12), (12, 21504, 1024, 16)])
+def test_few_rows(gpu, ggml_type, N, K, B, mean):
+    """Every row within 5e-7 of the exact product: 22 bits of every activation (2^-23 each, less in a sum), two additions of the
+    tensor core per block rounded towards zero (2^-23 of the block's sum each), fp32 sums over the blocks; and with
+    activations that have a mean within 16 of its units, for the blocks' offsets cancel what the codes' mean adds."""
+    rng = np.random.default_rng(N + K + B)
+    raw = {2: gb.random_q4_0_blocks, 12: gb.random_q4_k_blocks}[ggml_type](rng, N, K)
+    x = (rng.standard_normal((B, K), dtype=np.float32) + np.float32(mean)) * rng.uniform(0.01, 100.0, (B, 1)).astype(np.float32)
+    before = gpu.tc_gemm_count()
+    e = _error(gpu, ggml_type, raw, N, K, x, 1)
+    assert gpu.tc_gemm_count() == before + 1
+    print(f"error {e.max():.2e}, GEMV {_error(gpu, ggml_type, raw, N, K, x, 0).max():.2e}")
+    assert e.max() < 5e-7 and gpu.device_error() == 0
+
+
+def _model(gpu, cfg, batch, policy, prompts):
+    from adam_b200 import synth
+    from adam_b200.config import GenerationConfig
+    from adam_b200.engine import ADAMEngine
+    gpu.tc_gemm_policy(policy)
+    eng = ADAMEngine(gpu, cfg, synth.build_model(cfg, gb.GGML_TYPE_Q4_0, seed=71), kv_cap=48, kv_dtype="f32", max_batch=batch)
+    try:
+        ids, _ = eng.generate_batch(prompts, GenerationConfig(max_tokens=4, eos_token_ids=(), temperature=0.0, top_k=1, repeat_penalty=1.0))
+        eng.begin(prompts, [40] * batch)
+        eng.prefill(len(prompts[0]) - 1)
+        eng.step(1, lm_head=True, logits=True, direct=True)
+        return ids, np.stack([eng.read_logits(b) for b in range(batch)])
+    finally:
+        eng.close()
+        gpu.tc_gemm_policy(1)
+
+
+@pytest.mark.parametrize("batch", [5, 8])
+def test_steps_of_a_few_sequences(gpu, batch):
+    """Gate / up products, the LM head's arg-max and its stored logits against the same steps on the GEMV kernels: a dozen
+    products in a row, each within 7e-7 of the exact one on either path."""
+    from adam_b200 import synth
+    from adam_b200.config import tiny_gemma3
+    cfg = tiny_gemma3(n_layer=2, n_vocab=1008)
+    prompts = [synth.random_prompt(cfg.n_vocab, 9, seed=200 + i) for i in range(batch)]
+    before = gpu.tc_gemm_count()
+    ids, logits = _model(gpu, cfg, batch, 1, prompts)
+    assert gpu.tc_gemm_count() > before
+    want_ids, want = _model(gpu, cfg, batch, 0, prompts)
+    assert ids == want_ids and np.linalg.norm(logits - want) < 1e-5 * np.linalg.norm(want) and gpu.device_error() == 0
