@@ -88,11 +88,11 @@ struct Decoder {
 constexpr uint32_t MAX_DECODERS = 8;
 constexpr uint32_t ATTN_SPLIT = 64;        // fewest tokens an attention CTA takes before another CTA is added
 constexpr uint32_t ATTN_MAX_SPLITS = 64;   // attention CTAs per (sequence, kv head)
-// Rows (sequences x tokens) of one prefill chunk, the same for every shape.  512 / 1024 / 2048 rows: 32 prompts x 512 and their
-// 24 steps at the 1B shape 185 / 147 / 135 ms, one prompt of 1500 tokens with 12 steps 32.3 / 28.5 / 24.5 ms, 64 x 128 at the 27B
-// shape (8 layers) 222 / 222 / 229 ms: the narrow model gains from 2048 (its 1152-row products are 72 tiles on 148 SMs at 1024),
-// the wide one loses.
-constexpr uint32_t PREFILL_ROWS = 1024;
+// Rows (sequences x tokens) of one prefill chunk: 1024, or 2048 where the tiles of an n_embd-wide product (128 x 128) do not
+// give every SM one at 1024.  512 / 1024 / 2048 rows: 32 prompts x 512 and their 24 steps at the 1B shape (n_embd 1152, 72
+// tiles at 1024) 185 / 147 / 135 ms, one prompt of 1500 tokens with 12 steps 32.3 / 28.5 / 24.5 ms, 64 x 128 at the 27B shape
+// (8 layers, 336 tiles) 222 / 222 / 229 ms.
+static uint32_t prefill_rows(uint32_t n_embd) { return (uint64_t)((n_embd + 127) / 128) * (1024 / 128) < (uint64_t)g.sm_count ? 2048u : 1024u; }
 static Decoder* g_dec[MAX_DECODERS];
 
 static Decoder* get_dec(uint32_t id) {
@@ -1204,7 +1204,8 @@ extern "C" int adam_b200_decoder_create(const adam_b200_decoder_desc* desc, uint
     D->n_splits = (d.kv_cap + ATTN_SPLIT - 1) / ATTN_SPLIT;      // ATTN_SPLIT = ATTN_CP * ATTN_CHUNKS_PER_CTA
     if (D->n_splits > ATTN_MAX_SPLITS) D->n_splits = ATTN_MAX_SPLITS;
     const uint64_t most = (uint64_t)d.max_batch * d.kv_cap;     // no more prompt rows than that exist
-    D->rows_cap = (uint32_t)(most < PREFILL_ROWS ? (most > 64 ? most : 64) : PREFILL_ROWS);
+    const uint32_t chunk = prefill_rows(d.n_embd);
+    D->rows_cap = (uint32_t)(most < chunk ? (most > 64 ? most : 64) : chunk);
     if (D->rows_cap < d.max_batch) D->rows_cap = d.max_batch;
     const size_t B = d.max_batch, E = d.n_embd, q_dim = (size_t)d.n_head * d.head_dim, k_dim = (size_t)d.n_head_kv * d.head_dim;
     const uint32_t gs = d.n_head / d.n_head_kv;
