@@ -65,8 +65,8 @@ bool gemm_tc_prepare(int rows, int K) {
         *p = q;
         return true;
     };
-    if (!g_tc.part) {                                   // two tiles of 128 x 128 sums and a ticket per CTA
-        if (!grow((void**)&g_tc.tickets, (size_t)g.sm_count * 4) || !grow((void**)&g_tc.part, (size_t)g.sm_count * 2 * 128 * 128 * 4)) return false;
+    if (!g_tc.part) {                                   // two tiles of 128 x 256 sums and two tickets per CTA
+        if (!grow((void**)&g_tc.tickets, (size_t)g.sm_count * 8) || !grow((void**)&g_tc.part, (size_t)g.sm_count * 2 * 128 * 256 * 4)) return false;
     }
     if (need > g_tc.img_cap) {
         size_t cap = need > 2 * g_tc.img_cap ? need : 2 * g_tc.img_cap;
@@ -331,8 +331,8 @@ __device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, u
 
 // ---- the GEMM ---------------------------------------------------------------------------------------------------
 // One CTA per SM.  A CTA's tile is 128 weight rows (or 64 gate rows in TMEM lanes 0..63 and the same 64 up rows in lanes
-// 64..127) by NT activation rows: D is 2 NT columns of TMEM, the rest a ring of weight tiles (128 rows x 64 values of K as
-// w_hi | w_lo, 64 columns each).  K is walked in stages of SP steps of 64 values, NS stages in flight; a stage has one
+// 64..127) by NT activation rows: D is 2 NT columns of TMEM (NT = 256: NT), the rest a ring of weight tiles (128 rows x 64
+// values of K as w_hi | w_lo, 64 columns each).  K is walked in stages of SP steps of 64 values, NS stages in flight; a stage has one
 // barrier for everything that fills it (its activation tiles, and the warps that rebuild its weight tiles) and one that
 // the tensor core's commit releases.
 //   warp roles   Warpgroup 0: warp 0 issues the tensor-core instructions, warp 1 fetches activation tiles.  Warpgroup 1 reads
@@ -359,6 +359,14 @@ __device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, u
 //                fill the stage, so the issuing warp waits for nothing more.  At NT = 128 there is room for one pair:
 //                the stage that restarts D1 issues its products for D2 first, two thirds of its time, while D1 is
 //                read.  32 prompts x 512 at the 1B shape: 141 ms with eight steps, 157 with two and no second pair, 148 so.
+//   NT = 256     halves the rebuilding per product, which is energy (long prompts run at the power limit).  One accumulator of 256
+//                columns and no D2: a stage of two steps issues the cross terms of both, then both main terms, and is read
+//                out, so the additions at full magnitude are the eight of two steps.  Activations come plane by plane, each slot
+//                given back as soon as its last product is done; a step's weights and planes share one barrier, because a wait of
+//                the issuing warp costs 86 cycles even if satisfied and only some four instructions queue ahead of the tensor
+//                core (a barrier per plane: 640 us instead of 598).  A round trip over the accumulator costs 289 cycles and the
+//                reading of 128 columns 280 more, twice per 3072 cycles of products; two warpgroups read.  Bound by these
+//                trips and the waits (tensor pipe 56 % active), not by rebuilding (leaving it out: -7 %).
 //   work split   Three ways, by an estimate of their times (launch_rows).  Whole tiles, dealt in turn.  Or all stages
 //                of all tiles in a row, dealt out evenly: a tile that several CTAs share is added up by the one that ends
 //                last (atomic ticket, partial sums in a workspace), in the order of K; 168 tiles on 148 SMs take 1.14 tiles'
@@ -385,20 +393,22 @@ struct TcGemm {
     int* out_tok; float *out_val, *out_tok_f32, softcap;
 };
 template <int WT, int NT> struct TcGeo {
+    static constexpr int NH = NT == 256 ? 2 : 1, NC = NT / NH;               // reading warpgroups, columns that each reads
     static constexpr int SP = NT == 128 ? 1 : 2, NS = NT == 128 ? 4 : 2;     // steps per stage, stages
-    static constexpr int BANKS = NT == 128 ? 1 : NS, PERIOD = NT == 128 ? 3 : 1;        // pairs of accumulators D1 | D2; stages between two read-outs
-    static constexpr int GROUPS = NT == 128 ? 3 : 4, THREADS = (2 + GROUPS) * 128;     // warpgroups that rebuild weights, a step each in turn
-    static constexpr int REG_LOW = 40, REG_READ = NT == 128 ? 200 : 120, REG_MAKE = 80;    // sum = what the CTA is launched with
-    static constexpr int R = WT == WT_Q8_0 && NT == 128 ? 3 : 4;             // weight ring: tiles ahead per warp
+    static constexpr int BANKS = NT >= 128 ? 1 : NS, PERIOD = NT == 128 ? 3 : 1;        // sets of accumulators; stages between two read-outs
+    static constexpr int DCOLS = NT == 256 ? NT : BANKS * 2 * NT;            // columns of accumulators
+    static constexpr int GROUPS = NT == 256 ? 2 : NT == 128 ? 3 : 4, THREADS = (1 + NH + GROUPS) * 128;     // warpgroups that rebuild weights, a step each in turn
+    static constexpr int REG_LOW = NT == 256 ? 32 : 40, REG_READ = NT == 256 ? 152 : NT == 128 ? 200 : 120, REG_MAKE = NT == 256 ? 72 : 80;    // sum = what the CTA is launched with
+    static constexpr int R = WT == WT_Q8_0 && NT >= 128 ? 3 : 4;                  // weight ring: tiles ahead per warp
     static constexpr int QB = WT == WT_Q8_0 ? 64 : 32;                       // bytes of a row's codes per step
     static constexpr int SLOT = 32 * QB + (WT == WT_Q4_K ? 512 : 128);       // 32 rows: codes, then block scales / superblock headers
-    static constexpr int BSTEP = NT * 256;                                   // both planes of one step
-    static constexpr int RING = NS * SP * BSTEP, XCH = RING + GROUPS * 4 * R * SLOT;     // offsets: weight rings, columns of results on their way out
-    static constexpr int XCOLS = NT < 32 ? NT : 32;                          // so many columns at a time
-    static constexpr int SMEM_USED = XCH + XCOLS * 512 + 1024;
+    static constexpr int BSTEP = NT * 256, PLANE = NT * 128;                 // both planes of one step, one plane
+    static constexpr int RING = (NT == 256 ? 2 : NS * SP) * BSTEP, XCH = RING + GROUPS * 4 * R * SLOT;     // offsets: weight rings, columns of results on their way out
+    static constexpr int XCOLS = NC < 32 ? NC : 32;                          // so many columns at a time
+    static constexpr int SMEM_USED = XCH + NH * XCOLS * 512 + 1024;
     static constexpr int SMEM = SMEM_USED > TC_SMEM_MIN ? SMEM_USED : TC_SMEM_MIN;
-    static_assert(SMEM <= 226 * 1024 && BANKS * 2 * NT + 64 * NS * SP <= 512 && GROUPS % SP == 0 && GROUPS <= NS * SP, "shared or tensor memory");
-    static_assert(REG_LOW + REG_READ + GROUPS * REG_MAKE <= 65536 / THREADS / 8 * 8 * (2 + GROUPS), "registers");
+    static_assert(SMEM <= 226 * 1024 && DCOLS + 64 * NS * SP <= 512 && GROUPS % SP == 0 && GROUPS <= NS * SP, "shared or tensor memory");
+    static_assert(REG_LOW + NH * REG_READ + GROUPS * REG_MAKE <= 65536 / THREADS / 8 * 8 * (1 + NH + GROUPS), "registers");
 };
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
@@ -412,13 +422,13 @@ template <int WT, int NT, bool HEAD>
 __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcGemm a) {
     using G = TcGeo<WT, NT>;
     const bool pair = !HEAD && WT != WT_Q8_0 && a.pair != 0;
-    constexpr int SP = G::SP, NS = G::NS;
+    constexpr int SP = G::SP, NS = G::NS, NH = G::NH, NC = G::NC;
     extern __shared__ __align__(1024) uint8_t sm_raw[];
     uint8_t* sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);     // the swizzle works on address bits
     uint8_t* smB = sm;
-    __shared__ __align__(8) uint64_t full[NS], empty[NS], d_full, d_empty;
+    __shared__ __align__(8) uint64_t full[NT == 256 ? 2 * NS : NS], empty[NS], d_full, d_empty, p_empty[4];
     __shared__ uint32_t s_tmem;
-    __shared__ bool s_last;
+    __shared__ bool s_last[NH];
     __shared__ float s_inv[NT];
     [[maybe_unused]] __shared__ unsigned long long s_best[HEAD ? NT : 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wg = warp >> 2;
@@ -438,8 +448,9 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
     auto m_of = [&](int item) { return item / a.tiles_n * NT; };                // first activation row and weight tile of an item
     auto n_of = [&](int item) { return item % a.tiles_n; };
     if (tid == 0) {
-        for (int i = 0; i < NS; ++i) { mbar_init(&full[i], 4 * SP + 1 + (G::BANKS > 1 ? 4 : 0)); mbar_init(&empty[i], 1); }
-        mbar_init(&d_full, 1); mbar_init(&d_empty, 4);
+        for (int i = 0; i < NS; ++i) { if (NT != 256) mbar_init(&full[i], 4 * SP + 1 + (G::BANKS > 1 ? 4 : 0)); mbar_init(&empty[i], 1); }
+        mbar_init(&d_full, 1); mbar_init(&d_empty, 4 * NH);
+        if constexpr (NT == 256) for (int i = 0; i < 4; ++i) { mbar_init(&full[i], 4 + 2); mbar_init(&p_empty[i], 1); }      // a step: four warps of weights, two planes
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -448,7 +459,7 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
-    constexpr uint32_t A_COL = G::BANKS * 2 * NT;       // first column of the weight ring
+    constexpr uint32_t A_COL = G::DCOLS;       // first column of the weight ring
     bool dead = false;
     auto wait_on = [&](uint64_t* bar, uint32_t parity) {
         if (!dead && !mbar_wait(bar, parity)) { dead = true; atomicOr(a.err, DEVERR_WAIT); }
@@ -491,132 +502,214 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
         const bool lead = elect_one();
         if (warp == 1) {
             // ---- activation tiles ----
-            uint32_t s = 0, par = 1, n = 0;
-            const size_t group_bytes = (size_t)n_steps * (2 * TC_STEP_IMG);
-            for (int q = q0; q < q1;) {
-                const int i = q / spi, j0 = q - i * spi, j1 = min(spi, j0 + q1 - q);
-                q += j1 - j0;
-                const uint8_t* group = a.img + (size_t)(item_of(i) / a.tiles_n) * (NT == 128 ? 2 : 1) * group_bytes;
-                for (int j = j0; j < j1; ++j, ++n) {
-                    if (n >= (uint32_t)NS) wait_on(&empty[s], par);
-                    const int st0 = j * SP, n_sub = SP == 1 ? 1 : min(SP, nst - st0);
-                    if (lead) {
-                        mbar_expect_tx(&full[s], (uint32_t)(n_sub * G::BSTEP));
-                        for (int t = 0; t < n_sub; ++t) {
-                            const int st = st0 + t;
-                            const uint8_t* src = group + (size_t)(st < nmn ? mn0 + st : a.n_min + ma0 + st - nmn) * (2 * TC_STEP_IMG);
-                            uint8_t* dst = smB + (s * SP + t) * G::BSTEP;
-                            if constexpr (NT == TC_GROUP) bulk_g2s(dst, src, G::BSTEP, &full[s]);
-                            else {                      // both planes of the first NT rows, or of two groups
-                                constexpr int ROWS = NT < TC_GROUP ? NT : TC_GROUP;
-                                bulk_g2s(dst, src, ROWS * 128, &full[s]);
-                                bulk_g2s(dst + NT * 128, src + TC_STEP_IMG, ROWS * 128, &full[s]);
-                                if constexpr (NT > TC_GROUP) {
-                                    bulk_g2s(dst + TC_STEP_IMG, src + group_bytes, TC_STEP_IMG, &full[s]);
-                                    bulk_g2s(dst + NT * 128 + TC_STEP_IMG, src + group_bytes + TC_STEP_IMG, TC_STEP_IMG, &full[s]);
+            if constexpr (NT == 256) {
+                // planes of 256 rows in the order in which they are multiplied and room for them becomes free (see the products)
+                const size_t group_bytes = (size_t)n_steps * (2 * TC_STEP_IMG);
+                uint32_t x[4] = {0, 1, 2, 3}, par = 0xFu;               // slots of a stage's planes lo 0, hi 0, hi 1, lo 1; parities of their waits
+                for (int q = q0; q < q1; ++q) {
+                    const int i = q / spi, st0 = (q - i * spi) * SP, m0 = m_of(item_of(i));
+                    uint64_t* fs = full + ((q - q0) & 1) * 2;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int st = st0 + (k >> 1), lo = k == 0 || k == 3 ? 1 : 0;
+                        const uint32_t s = x[k];
+                        if (st >= nst) {                // no second step: its barrier gets what it counts all the same
+                            if (lead) mbar_arrive(fs + 1);
+                            __syncwarp();
+                            continue;
+                        }
+                        wait_on(&p_empty[s], par >> s & 1u);
+                        par ^= 1u << s;
+                        if (lead) {
+                            mbar_expect_tx(fs + (k >> 1), G::PLANE);
+                            const size_t at = (size_t)(st < nmn ? mn0 + st : a.n_min + ma0 + st - nmn) * (2 * TC_STEP_IMG) + lo * TC_STEP_IMG;
+#pragma unroll
+                            for (int g4 = 0; g4 < 4; ++g4) {            // groups without rows take the first's: their sums are dropped
+                                const int group = m0 / TC_GROUP + (m0 + g4 * TC_GROUP < a.B ? g4 : 0);
+                                bulk_g2s(smB + s * G::PLANE + g4 * TC_STEP_IMG, a.img + group * group_bytes + at, TC_STEP_IMG, fs + (k >> 1));
+                            }
+                        }
+                        __syncwarp();
+                    }
+                    const uint32_t x1 = x[1];
+                    x[1] = x[3]; x[3] = x[2]; x[2] = x1;
+                }
+                // no copy may be in flight when the CTA ends, whatever became of the waits above: the last two stages
+                for (int n = max(0, q1 - q0 - 2); n < q1 - q0; ++n)
+                    for (int t = 0; t < 2; ++t) mbar_wait(&full[(n & 1) * 2 + t], (uint32_t)(n >> 1) & 1u);
+            } else {
+                uint32_t s = 0, par = 1, n = 0;
+                const size_t group_bytes = (size_t)n_steps * (2 * TC_STEP_IMG);
+                for (int q = q0; q < q1;) {
+                    const int i = q / spi, j0 = q - i * spi, j1 = min(spi, j0 + q1 - q);
+                    q += j1 - j0;
+                    const uint8_t* group = a.img + (size_t)(item_of(i) / a.tiles_n) * (NT == 128 ? 2 : 1) * group_bytes;
+                    for (int j = j0; j < j1; ++j, ++n) {
+                        if (n >= (uint32_t)NS) wait_on(&empty[s], par);
+                        const int st0 = j * SP, n_sub = SP == 1 ? 1 : min(SP, nst - st0);
+                        if (lead) {
+                            mbar_expect_tx(&full[s], (uint32_t)(n_sub * G::BSTEP));
+                            for (int t = 0; t < n_sub; ++t) {
+                                const int st = st0 + t;
+                                const uint8_t* src = group + (size_t)(st < nmn ? mn0 + st : a.n_min + ma0 + st - nmn) * (2 * TC_STEP_IMG);
+                                uint8_t* dst = smB + (s * SP + t) * G::BSTEP;
+                                if constexpr (NT == TC_GROUP) bulk_g2s(dst, src, G::BSTEP, &full[s]);
+                                else {                      // both planes of the first NT rows, or of two groups
+                                    constexpr int ROWS = NT < TC_GROUP ? NT : TC_GROUP;
+                                    bulk_g2s(dst, src, ROWS * 128, &full[s]);
+                                    bulk_g2s(dst + NT * 128, src + TC_STEP_IMG, ROWS * 128, &full[s]);
+                                    if constexpr (NT > TC_GROUP) {
+                                        bulk_g2s(dst + TC_STEP_IMG, src + group_bytes, TC_STEP_IMG, &full[s]);
+                                        bulk_g2s(dst + NT * 128 + TC_STEP_IMG, src + group_bytes + TC_STEP_IMG, TC_STEP_IMG, &full[s]);
+                                    }
                                 }
                             }
                         }
+                        __syncwarp();
+                        if (++s == (uint32_t)NS) { s = 0; par ^= 1u; }
                     }
-                    __syncwarp();
-                    if (++s == (uint32_t)NS) { s = 0; par ^= 1u; }
                 }
+                // no copy may be in flight when the CTA ends, whatever became of the waits above
+                for (uint32_t i = n > (uint32_t)NS ? n - NS : 0; i < n; ++i) mbar_wait(&full[i % NS], (i / NS) & 1u);
             }
-            // no copy may be in flight when the CTA ends, whatever became of the waits above
-            for (uint32_t i = n > (uint32_t)NS ? n - NS : 0; i < n; ++i) mbar_wait(&full[i % NS], (i / NS) & 1u);
         } else if (warp == 0) {
             // ---- products ----
             const uint32_t b_lo = (smem_u32(smB) & 0x3FFFFu) >> 4;
             auto desc = [&](uint32_t lo) { return ((uint64_t)TC_DESC_HI << 32) | lo; };
-            uint32_t s = 0, par = 0, periods = 0;
-            for (int q = q0; q < q1;) {
-                const int j0 = q % spi, j1 = min(spi, j0 + q1 - q);
-                q += j1 - j0;
-                for (int j = j0; j < j1; ++j) {
-                    if constexpr (G::BANKS > 1) {       // a stage has accumulators of its own
-                        wait_on(&full[s], par);
+            if constexpr (NT == 256) {
+                // A stage: the cross terms of its (up to) two steps, then their main terms, one accumulator of 256 columns.
+                // A plane x_lo is done with after a third of the stage, x_hi after five sixths: lo 0, lo 1, hi 0, hi 1 in
+                // this order leave their slots to the next stage's lo 0, hi 0, hi 1, lo 1.
+                uint32_t s = 0, par = 0, x[4] = {0, 1, 2, 3};
+                for (int q = q0; q < q1; ++q) {
+                    const int n_sub = min(SP, nst - (q % spi) * SP);
+#pragma unroll
+                    for (int t = 0; t < SP; ++t) {
+                        wait_on(&full[s * 2 + t], par);
+                        if (t == n_sub) break;
+                        if (t == 0 && q > q0) wait_on(&d_empty, (uint32_t)(q - q0 - 1) & 1u);
+                        const uint32_t xl = t ? x[3] : x[0], xh = t ? x[2] : x[1], ac = tmem + A_COL + (s * SP + t) * 64u;
                         tc_fence_after();
                         if (lead) {
-                            const uint32_t d1 = tmem + s * 2 * NT, d2 = d1 + NT;
+                            const uint32_t bl = b_lo + xl * (uint32_t)(G::PLANE / 16), bh = b_lo + xh * (uint32_t)(G::PLANE / 16);
 #pragma unroll
-                            for (int t = 0; t < SP; ++t) {
-                                if (t == 1 && 2 * j + 1 >= nst) break;
-                                const uint32_t slot = s * SP + t, ac = tmem + A_COL + slot * 64u, bh = b_lo + slot * (uint32_t)(G::BSTEP / 16);
+                            for (uint32_t k = 0; k < 4; ++k) tc_mma_ts(tmem, ac + k * 8u, desc(bl + k * 2u), TC_IDESC<NT>, t || k ? 1u : 0u);
+                            tc_commit(&p_empty[xl]);
 #pragma unroll
-                                for (uint32_t q = 0; q < 4; ++q) {
-                                    tc_mma_ts(d1, ac + q * 8u, desc(bh + q * 2u), TC_IDESC<2 * NT>, t + q > 0 ? 1u : 0u);
-                                    tc_mma_ts(d2, ac + 32u + q * 8u, desc(bh + q * 2u), TC_IDESC<NT>, 1u);
-                                }
-                            }
-                            tc_commit(&empty[s]);       // for the reading warpgroup too
+                            for (uint32_t k = 0; k < 4; ++k) tc_mma_ts(tmem, ac + 32u + k * 8u, desc(bh + k * 2u), TC_IDESC<NT>, 1u);
                         }
-                    } else {
-                        const bool fresh = (j - j0) % G::PERIOD == 0;   // D1 starts again; D2 only with an item
-                        if (j == j0 && periods) wait_on(&d_empty, (periods - 1u) & 1u);
-                        wait_on(&full[s], par);
-                        tc_fence_after();
-                        const uint32_t d1 = tmem, d2 = tmem + NT, ac = tmem + A_COL + s * 64u, bh = b_lo + s * (uint32_t)(G::BSTEP / 16);
-                        if (fresh && j > j0) {          // the products for D2 while D1 is read
-                            if (lead) {
+                        __syncwarp();
+                    }
+                    if (lead) {
 #pragma unroll
-                                for (uint32_t q = 0; q < 4; ++q) {
-                                    tc_mma_ts(d2, ac + q * 8u, desc(bh + NT * 8 + q * 2u), TC_IDESC<NT>, 1u);
-                                    tc_mma_ts(d2, ac + 32u + q * 8u, desc(bh + q * 2u), TC_IDESC<NT>, 1u);
-                                }
-                            }
-                            __syncwarp();
-                            wait_on(&d_empty, (periods - 1u) & 1u);
-                            tc_fence_after();
-                            if (lead) {
+                        for (int t = 0; t < SP; ++t) {
+                            if (t == n_sub) break;
+                            const uint32_t xh = t ? x[2] : x[1], ac = tmem + A_COL + (s * SP + t) * 64u, bh = b_lo + xh * (uint32_t)(G::PLANE / 16);
 #pragma unroll
-                                for (uint32_t q = 0; q < 4; ++q) tc_mma_ts(d1, ac + q * 8u, desc(bh + q * 2u), TC_IDESC<NT>, q > 0 ? 1u : 0u);
-                            }
-                        } else if (lead) {
-#pragma unroll
-                            for (uint32_t q = 0; q < 4; ++q) {
-                                tc_mma_ts(d1, ac + q * 8u, desc(bh + q * 2u), TC_IDESC<2 * NT>, (q > 0 || j > j0) ? 1u : 0u);
-                                tc_mma_ts(d2, ac + 32u + q * 8u, desc(bh + q * 2u), TC_IDESC<NT>, 1u);
-                            }
+                            for (uint32_t k = 0; k < 4; ++k) tc_mma_ts(tmem, ac + k * 8u, desc(bh + k * 2u), TC_IDESC<NT>, 1u);
+                            tc_commit(&p_empty[xh]);
                         }
-                        periods += fresh ? 1u : 0u;
-                        if (lead) {
-                            tc_commit(&empty[s]);
-                            if ((j - j0) % G::PERIOD == G::PERIOD - 1 || j == j1 - 1) tc_commit(&d_full);
-                        }
+                        tc_commit(&d_full);
+                        tc_commit(&empty[s]);
                     }
                     __syncwarp();
                     if (++s == (uint32_t)NS) { s = 0; par ^= 1u; }
+                    const uint32_t x1 = x[1];
+                    x[1] = x[3]; x[3] = x[2]; x[2] = x1;
+                }
+            } else {
+                uint32_t s = 0, par = 0, periods = 0;
+                for (int q = q0; q < q1;) {
+                    const int j0 = q % spi, j1 = min(spi, j0 + q1 - q);
+                    q += j1 - j0;
+                    for (int j = j0; j < j1; ++j) {
+                        if constexpr (G::BANKS > 1) {       // a stage has accumulators of its own
+                            wait_on(&full[s], par);
+                            tc_fence_after();
+                            if (lead) {
+                                const uint32_t d1 = tmem + s * 2 * NT, d2 = d1 + NT;
+#pragma unroll
+                                for (int t = 0; t < SP; ++t) {
+                                    if (t == 1 && 2 * j + 1 >= nst) break;
+                                    const uint32_t slot = s * SP + t, ac = tmem + A_COL + slot * 64u, bh = b_lo + slot * (uint32_t)(G::BSTEP / 16);
+#pragma unroll
+                                    for (uint32_t q = 0; q < 4; ++q) {
+                                        tc_mma_ts(d1, ac + q * 8u, desc(bh + q * 2u), TC_IDESC<2 * NT>, t + q > 0 ? 1u : 0u);
+                                        tc_mma_ts(d2, ac + 32u + q * 8u, desc(bh + q * 2u), TC_IDESC<NT>, 1u);
+                                    }
+                                }
+                                tc_commit(&empty[s]);       // for the reading warpgroup too
+                            }
+                        } else {
+                            const bool fresh = (j - j0) % G::PERIOD == 0;   // D1 starts again; D2 only with an item
+                            if (j == j0 && periods) wait_on(&d_empty, (periods - 1u) & 1u);
+                            wait_on(&full[s], par);
+                            tc_fence_after();
+                            const uint32_t d1 = tmem, d2 = tmem + NT, ac = tmem + A_COL + s * 64u, bh = b_lo + s * (uint32_t)(G::BSTEP / 16);
+                            if (fresh && j > j0) {          // the products for D2 while D1 is read
+                                if (lead) {
+#pragma unroll
+                                    for (uint32_t q = 0; q < 4; ++q) {
+                                        tc_mma_ts(d2, ac + q * 8u, desc(bh + NT * 8 + q * 2u), TC_IDESC<NT>, 1u);
+                                        tc_mma_ts(d2, ac + 32u + q * 8u, desc(bh + q * 2u), TC_IDESC<NT>, 1u);
+                                    }
+                                }
+                                __syncwarp();
+                                wait_on(&d_empty, (periods - 1u) & 1u);
+                                tc_fence_after();
+                                if (lead) {
+#pragma unroll
+                                    for (uint32_t q = 0; q < 4; ++q) tc_mma_ts(d1, ac + q * 8u, desc(bh + q * 2u), TC_IDESC<NT>, q > 0 ? 1u : 0u);
+                                }
+                            } else if (lead) {
+#pragma unroll
+                                for (uint32_t q = 0; q < 4; ++q) {
+                                    tc_mma_ts(d1, ac + q * 8u, desc(bh + q * 2u), TC_IDESC<2 * NT>, (q > 0 || j > j0) ? 1u : 0u);
+                                    tc_mma_ts(d2, ac + 32u + q * 8u, desc(bh + q * 2u), TC_IDESC<NT>, 1u);
+                                }
+                            }
+                            periods += fresh ? 1u : 0u;
+                            if (lead) {
+                                tc_commit(&empty[s]);
+                                if ((j - j0) % G::PERIOD == G::PERIOD - 1 || j == j1 - 1) tc_commit(&d_full);
+                            }
+                        }
+                        __syncwarp();
+                        if (++s == (uint32_t)NS) { s = 0; par ^= 1u; }
+                    }
                 }
             }
         }
         __syncwarp();
         if (S > 1) { cl_arrive(); cl_wait(); cl_arrive(); cl_wait(); }
-    } else if (wg == 1) {
-        // ---- results: D1 (and, with an item's last period, D2) into registers; an item's end: scale back, activation, store ----
+    } else if (wg <= NH) {
+        // ---- results: the accumulators into registers; an item's end: scale back, activation, store ----
         reg_inc<G::REG_READ>();
         pdl_wait();
-        float* xch = reinterpret_cast<float*>(sm + G::XCH);
+        const int rd = wg - 1, rt = tid - wg * 128;     // which half it reads, and its thread
+        auto sync_rd = [&]() { asm volatile("bar.sync %0, 128;" :: "r"(wg) : "memory"); };
+        float* xch = reinterpret_cast<float*>(sm + G::XCH) + rd * (G::XCOLS * 128);
         uint32_t nth = 0;                               // accumulation period
         if constexpr (G::BANKS > 1) { if (lane < NS) mbar_arrive(&full[lane]); }        // all accumulators are free
         if constexpr (HEAD) {
-            if (tid - 128 < NT) s_best[tid - 128] = 0;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (rt < NT) s_best[rt] = 0;
+            sync_rd();
         }
         [[maybe_unused]] auto flush_best = [&](int m0) {
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (const int c = tid - 128; c < min(NT, a.B - m0)) {
-                if (s_best[c]) atomicMax(a.best + m0 + c, s_best[c]);
-                s_best[c] = 0;
+            sync_rd();
+            if (rt < min(NT, a.B - m0)) {
+                if (s_best[rt]) atomicMax(a.best + m0 + rt, s_best[rt]);
+                s_best[rt] = 0;
             }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            sync_rd();
         };
         for (int q = q0; q < q1;) {
-            const int i0 = q / spi, j0 = q - i0 * spi, j1 = min(spi, j0 + q1 - q), item = item_of(i0), tn = n_of(item), m0 = m_of(item);
+            const int i0 = q / spi, j0 = q - i0 * spi, j1 = min(spi, j0 + q1 - q), item = item_of(i0), tn = n_of(item), m0 = m_of(item) + rd * NC;
             const int np = (j1 - j0 + G::PERIOD - 1) / G::PERIOD;                       // accumulation periods
             q += j1 - j0;
-            float acc[NT];
+            float acc[NC];
 #pragma unroll
-            for (int c = 0; c < NT; ++c) acc[c] = 0.f;
+            for (int c = 0; c < NC; ++c) acc[c] = 0.f;
 #pragma unroll 1
             for (int p = 0; p < np; ++p, ++nth) {
                 const uint32_t bank = nth % G::BANKS;
@@ -624,27 +717,37 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                 else wait_on(&d_full, nth & 1u);
                 tc_fence_after();
                 auto take = [&](uint32_t col) {         // the tensor core may wait for this: few round trips
-                    constexpr int CH = NT < 32 ? NT : 32;
+                    constexpr int CH = NT == 256 || NC < 32 ? 16 : 32;
 #pragma unroll
-                    for (int ch = 0; ch < NT; ch += CH) {
+                    for (int ch = 0; ch < NC; ch += CH) {
                         float v[CH / 16][16];
 #pragma unroll
                         for (int h = 0; h < CH / 16; ++h) tc_ld16(col + ch + 16 * h, v[h]);
                         tc_ld_wait();
+                        if (NT == 256 && ch == NC - CH) {       // all of it is in registers
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&d_empty);
+                        }
 #pragma unroll
-                        for (int c = 0; c < CH; ++c) acc[ch + c] += v[c / 16][c % 16];
+                        for (int c = 0; c < CH; c += 2) fma2(acc[ch + c], acc[ch + c + 1], v[c / 16][c % 16], v[c / 16][c % 16 + 1], 1.f, 1.f);
                     }
                 };
+                if constexpr (NT == 256) take(tlane + rd * NC);
+                else {
 #pragma unroll 1
-                for (int h = 0; h < (G::BANKS > 1 || p == np - 1 ? 2 : 1); ++h) take(tlane + bank * 2 * NT + h * NT);
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(G::BANKS > 1 ? &full[bank] : &d_empty);
+                    for (int h = 0; h < (G::BANKS > 1 || p == np - 1 ? 2 : 1); ++h) take(tlane + bank * 2 * NT + h * NT);
+                }
+                if constexpr (NT != 256) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(G::BANKS > 1 ? &full[bank] : &d_empty);
+                }
             }
             if (S > 1) {                                // one item per cluster, and the activation ring is drained: it becomes the exchange
                 float* ex = reinterpret_cast<float*>(smB);
 #pragma unroll
-                for (int c = 0; c < NT; ++c) ex[c * 128 + row] = acc[c];
+                for (int c = 0; c < NC; ++c) ex[c * 128 + row] = acc[c];
                 break;
             }
             if (j1 - j0 < spi) {
@@ -656,25 +759,26 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                     return c;
                 };
                 const int c_lo = cta_of(item * spi), c_hi = cta_of(item * spi + spi - 1);
-                auto slot_of = [&](int c) { return a.part + (size_t)(2 * c + (c == c_lo ? 1 : 0)) * (NT * 128) + row; };   // it begins here, or before
+                auto slot_of = [&](int c) { return a.part + (size_t)((2 * c + (c == c_lo ? 1 : 0)) * NH + rd) * (NC * 128) + row; };   // it begins here, or before
                 float* out = slot_of(cta);
 #pragma unroll
-                for (int c = 0; c < NT; ++c) out[c * 128] = acc[c];
+                for (int c = 0; c < NC; ++c) out[c * 128] = acc[c];
                 __threadfence();
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (tid == 128) {
-                    const unsigned int seen = atomicAdd(a.tickets + c_lo, 1u);
-                    s_last = seen == (unsigned int)(c_hi - c_lo);
-                    if (s_last) a.tickets[c_lo] = 0u;
+                sync_rd();
+                if (rt == 0) {
+                    unsigned int* ticket = a.tickets + c_lo * NH + rd;
+                    const unsigned int seen = atomicAdd(ticket, 1u);
+                    s_last[rd] = seen == (unsigned int)(c_hi - c_lo);
+                    if (s_last[rd]) *ticket = 0u;
                 }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                const bool last = s_last;
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+                sync_rd();
+                const bool last = s_last[rd];
+                sync_rd();
                 if (!last) continue;
                 __threadfence();
-                constexpr int CH = NT < 32 ? NT : 32;           // columns whose loads are in flight together
+                constexpr int CH = NT == 256 || NC < 32 ? 16 : 32;     // columns whose loads are in flight together
 #pragma unroll
-                for (int ch = 0; ch < NT; ch += CH) {
+                for (int ch = 0; ch < NC; ch += CH) {
                     const float* in = slot_of(c_lo) + ch * 128;
 #pragma unroll
                     for (int c = 0; c < CH; ++c) acc[ch + c] = __ldcg(in + c * 128);
@@ -683,7 +787,7 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                 for (int other = c_lo + 1; other <= c_hi; ++other) {
                     const float* in = slot_of(other);
 #pragma unroll
-                    for (int ch = 0; ch < NT; ch += CH) {
+                    for (int ch = 0; ch < NC; ch += CH) {
                         float t[CH];
 #pragma unroll
                         for (int c = 0; c < CH; ++c) t[c] = __ldcg(in + (ch + c) * 128);
@@ -694,30 +798,30 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
             }
             // Out through shared memory, XC columns at a time, by rolled loops.
             constexpr int XC = G::XCOLS;
-            const int n_col = min(NT, a.B - m0);
+            const int n_col = min(NC, a.B - m0);
             const int r = pair ? row & 63 : row, n = pair ? tn * 64 + r : tn * 128 + r;
             float* yp = a.y + (size_t)m0 * a.ldy + n;
-            if (tid - 128 < n_col) s_inv[tid - 128] = a.inv[m0 + tid - 128];
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (rt < n_col) s_inv[rd * NC + rt] = a.inv[m0 + rt];
+            sync_rd();
 #pragma unroll 1
             for (int h0 = 0; h0 < n_col; h0 += XC) {
                 const int m = min(XC, n_col - h0);
 #pragma unroll
                 for (int c = 0; c < XC; ++c) xch[c * 128 + row] = acc[c];
                 if (pair) {                             // gate (lanes 0..63) and up rows meet; all lanes share the outputs
-                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    sync_rd();
 #pragma unroll 4
                     for (int c = row >> 6; c < m; c += 2) {
-                        const float sc = s_inv[h0 + c], v = act(xch[c * 128 + r] * sc, xch[c * 128 + 64 + r] * sc);
+                        const float sc = s_inv[rd * NC + h0 + c], v = act(xch[c * 128 + r] * sc, xch[c * 128 + 64 + r] * sc);
                         if (n < a.N) yp[(size_t)(h0 + c) * a.ldy] = v;
                     }
-                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    sync_rd();
                 } else if constexpr (HEAD) {
                     // best of the warp's rows per column: NaN counts as -FLT_MAX, ties go to the lower row
                     unsigned long long mine = 0;        // lane c: column h0 + c
 #pragma unroll 2
                     for (int c = 0; c < m; ++c) {
-                        const float v = xch[c * 128 + row] * s_inv[h0 + c], f = (v == v ? v : -3.402823466e+38f) + 0.f;
+                        const float v = xch[c * 128 + row] * s_inv[rd * NC + h0 + c], f = (v == v ? v : -3.402823466e+38f) + 0.f;
                         const uint32_t bits = __float_as_uint(f), ord = n < a.N ? bits ^ ((uint32_t)((int)bits >> 31) | 0x80000000u) : 0u;
                         const uint32_t top = __reduce_max_sync(0xffffffffu, ord);
                         const uint32_t at = __reduce_min_sync(0xffffffffu, ord == top ? (uint32_t)n : 0xffffffffu);
@@ -727,24 +831,24 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                     if (lane < m) atomicMax(&s_best[h0 + lane], mine);
                 } else if (n < a.N) {
 #pragma unroll 4
-                    for (int c = 0; c < m; ++c) yp[(size_t)(h0 + c) * a.ldy] = xch[c * 128 + row] * s_inv[h0 + c];
+                    for (int c = 0; c < m; ++c) yp[(size_t)(h0 + c) * a.ldy] = xch[c * 128 + row] * s_inv[rd * NC + h0 + c];
                 }
 #pragma unroll
-                for (int c = 0; c < NT - XC; ++c) acc[c] = acc[c + XC];
+                for (int c = 0; c < NC - XC; ++c) acc[c] = acc[c + XC];
             }
             if constexpr (HEAD) { if (a.B > NT) flush_best(m0); }       // the columns change with the next item
-            asm volatile("bar.sync 1, 128;" ::: "memory");              // s_inv is free again
+            sync_rd();              // s_inv is free again
         }
         if (S > 1) finish_split();
         if constexpr (HEAD) {                           // the last CTA to end decodes the winners and clears the keys
             flush_best(0);
             __threadfence();
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (tid == 128) s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (s_last) {
+            sync_rd();
+            if (rt == 0) s_last[0] = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+            sync_rd();
+            if (s_last[0]) {
                 __threadfence();
-                for (int b = tid - 128; b < a.B; b += 128) {
+                for (int b = rt; b < a.B; b += 128) {
                     const unsigned long long key = __ldcg(a.best + b);
                     const uint32_t ord = (uint32_t)(key >> 32);
                     const int tok = (int)(0xffffffffu - (uint32_t)key);
@@ -753,18 +857,18 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                     if (a.out_val) a.out_val[b] = __uint_as_float(ord & 0x80000000u ? ord ^ 0x80000000u : ~ord);
                     a.best[b] = 0;
                 }
-                if (tid == 128) *a.ticket = 0u;
+                if (rt == 0) *a.ticket = 0u;
             }
         }
     } else {
         // ---- weights ----
         reg_set<G::REG_MAKE, 65536 / G::THREADS / 8 * 8>();
-        const int grp = wg - 2, quarter = warp & 3;
+        const int grp = wg - 1 - NH, quarter = warp & 3;
         // This group fills step `sub` of every GROUPS / SP-th stage of the CTA's range.  It waits for a ring slot to be emptied
         // without having followed every phase of it, which is sound because the slots empty in order: it has seen a later
         // one than the slot's last but one use empty (GROUPS <= NS * SP).
         const int sub = grp % SP;
-        uint8_t* ring = sm + G::RING + (warp - 8) * G::R * G::SLOT;
+        uint8_t* ring = sm + G::RING + (warp - 4 * (1 + NH)) * G::R * G::SLOT;
         const uint32_t ring_s = smem_u32(ring);
         const WeightRef w = (pair && quarter >= 2) ? a.w1 : a.w0;                      // lanes 64..127 of a pair: up rows
         const bool scales_async = WT == WT_Q4_K || ((a.units & 1) == 0 && ((uintptr_t)w.d & 3) == 0);
@@ -842,7 +946,7 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
                     q4k_codes(hdr, ks & 3, sp, mp);
                     d01 = (hdr.x & 0xFFFFu) * 0x10001u;
                 }
-#pragma unroll (NT == 128 || WT == WT_Q4_K ? 2 : 1)
+#pragma unroll (NT == 128 || (NT < 128 && WT == WT_Q4_K) ? 2 : 1)
                 for (int b = 0; b < 2; ++b) {           // 32 values of K: columns 16 b .. of w_hi and of w_lo
                     const uint32_t col = acol + b * 16u;
                     uint32_t whi[8], wlo[8], v[2];
@@ -934,7 +1038,7 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
             tc_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&full[stage]);
+            if (lane == 0) mbar_arrive(&full[NT == 256 ? stage * 2 + sub : stage]);
             if (++at == (uint32_t)G::R) at = 0;
             next(c);
         }
@@ -1001,6 +1105,7 @@ template <int WT, int NT, bool HEAD> static TcPick& tc_pick() {
     return p;
 }
 template <int WT, bool HEAD> static TcPick& tc_pick(int nt) {
+    if constexpr (!HEAD && WT != WT_Q8_0) { if (nt == 256) return tc_pick<WT, 256, HEAD>(); }
     return nt == 16 ? tc_pick<WT, 16, HEAD>() : nt == 32 ? tc_pick<WT, 32, HEAD>() : nt == 64 ? tc_pick<WT, 64, HEAD>() : tc_pick<WT, 128, HEAD>();
 }
 template <int WT> static TcPick& tc_pick(int nt, bool head) { return head ? tc_pick<WT, true>(nt) : tc_pick<WT, false>(nt); }
@@ -1050,36 +1155,43 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
     // the rebuilding of a weight tile allows.  Dealt out evenly, a CTA costs its stages and, where tiles are shared, the
     // adding up of P partial results of nt columns; as clusters of S, waves of CTAs and one exchange.  One set of figures for
     // all block types, although rebuilding a Q4_K weight takes longer than a Q4_0 one: they only rank the splits of one call.
-    const int nt = a.B <= 16 ? 16 : a.B <= 32 ? 32 : a.B <= 64 ? 64 : 128, sp = nt == 128 ? 1 : 2;
-    const int tiles_n = pair ? (a.N + 63) / 64 : (a.N + 127) / 128, tiles_m = (a.B + nt - 1) / nt;
-    const long long items = (long long)tiles_n * tiles_m;
-    const double step = nt == 128 ? 900.0 : nt == 64 ? 620.0 : 500.0;
-    const int spi1 = (n_min + n_main + sp - 1) / sp;
-    int S = 1, grid = 1;
+    const bool head = a.epi == EPI_ARGMAX;
+    const int tiles_n = pair ? (a.N + 63) / 64 : (a.N + 127) / 128;
+    int nt = 0, S = 1, grid = 1;
     bool shared = false;
     double best = 1e300;
-    auto offer = [&](double cost, int s, int ctas, bool sh) { if (cost < best * 0.999) { best = cost; S = s; grid = ctas; shared = sh; } };
-    const long long all = items * spi1;
-    const int whole = (int)(items < g.sm_count ? items : g.sm_count);
-    offer((double)((items + whole - 1) / whole) * spi1 * sp * step, 1, whole, false);
-    if (all >= g.sm_count) {
-        const double per = (double)((all + g.sm_count - 1) / g.sm_count), sharers = 2.0 + spi1 / per;
-        offer(per * sp * step + 3000.0 + nt * (20.0 + 40.0 * sharers), 1, g.sm_count, true);
+    auto offer_tiles = [&](int n, double step) {
+        const int sp = n == 128 ? 1 : 2, spi1 = (n_min + n_main + sp - 1) / sp;
+        const long long items = (long long)tiles_n * ((a.B + n - 1) / n), all = items * spi1;
+        auto offer = [&](double cost, int s, int ctas, bool sh) { if (cost < best * 0.999) { best = cost; nt = n; S = s; grid = ctas; shared = sh; } };
+        const int whole = (int)(items < g.sm_count ? items : g.sm_count);
+        offer((double)((items + whole - 1) / whole) * spi1 * sp * step, 1, whole, false);
+        if (all >= g.sm_count) {
+            const double per = (double)((all + g.sm_count - 1) / g.sm_count), sharers = 2.0 + spi1 / per;
+            offer(per * sp * step + 3000.0 + n * (20.0 + 40.0 * sharers), 1, g.sm_count, true);
+        }
+        for (int s = 2; s <= (head || n == 256 ? 1 : 8) && s <= n_main; ++s) {
+            const int at_once = tc_clusters_at_once(s);
+            if (at_once < 1) continue;
+            const int steps = (n_main + s - 1) / s + (n_min + s - 1) / s;
+            offer((double)((items + at_once - 1) / at_once) * ((steps + sp - 1) / sp * sp * step + 2000.0), s, (int)items * s, false);
+        }
+    };
+    // Tiles of 256 rows take 1.9 times a tile of 128 (13824 x 1152 on 2048 rows 166 against 175 us, 21504 x 5376 on 1024 rows 598
+    // against 631), so they are for calls whose tiles still fill the GPU: 1152 x 6912 on 2048 rows, 72 tiles, 121 against 95 us.
+    if (a.B <= 64) offer_tiles(a.B <= 16 ? 16 : a.B <= 32 ? 32 : 64, a.B > 32 ? 620.0 : 500.0);
+    else {
+        offer_tiles(128, 1250.0);
+        if (a.B > 128 && !head && wtype != WT_Q8_0) offer_tiles(256, 2380.0);
     }
-    for (int s = 2; s <= (a.epi == EPI_ARGMAX ? 1 : 8) && s <= n_main; ++s) {
-        const int at_once = tc_clusters_at_once(s);
-        if (at_once < 1) continue;
-        const int steps = (n_main + s - 1) / s + (n_min + s - 1) / s;
-        offer((double)((items + at_once - 1) / at_once) * ((steps + sp - 1) / sp * sp * step + 2000.0), s, (int)items * s, false);
-    }
+    const int tiles_m = (a.B + nt - 1) / nt;
     TcGemm t = {};
     t.w0 = a.w0; t.w1 = a.w1; t.y = a.y; t.ldy = a.ldy; t.img = g_tc.img; t.inv = g_tc.inv; t.err = g.dev_err;
     t.N = a.N; t.units = a.K / 32; t.B = a.B; t.swiglu = a.epi == EPI_SWIGLU;
     t.n_min = n_min; t.n_main = n_main; t.S = S;
     t.tiles_n = tiles_n;
-    t.items = (int)items;
+    t.items = tiles_n * tiles_m;
     t.part = g_tc.part; t.tickets = g_tc.tickets; t.shared = shared ? 1 : 0;
-    const bool head = a.epi == EPI_ARGMAX;
     t.pair = pair;
     if (head) {
         t.best = g_tc.best; t.ticket = (unsigned int*)(g_tc.best + g_tc.inv_cap);

@@ -46,10 +46,10 @@ def _model(gpu, cfg, batch, policy, prompts):
     from adam_b200.config import GenerationConfig
     from adam_b200.engine import ADAMEngine
     gpu.tc_gemm_policy(policy)
-    eng = ADAMEngine(gpu, cfg, synth.build_model(cfg, gb.GGML_TYPE_Q4_0, seed=71), kv_cap=48, kv_dtype="f32", max_batch=batch)
+    eng = ADAMEngine(gpu, cfg, synth.build_model(cfg, gb.GGML_TYPE_Q4_0, seed=71), kv_cap=len(prompts[0]) + 40, kv_dtype="f32", max_batch=batch)
     try:
         ids, _ = eng.generate_batch(prompts, GenerationConfig(max_tokens=4, eos_token_ids=(), temperature=0.0, top_k=1, repeat_penalty=1.0))
-        eng.begin(prompts, [40] * batch)
+        eng.begin(prompts, [len(prompts[0]) + 30] * batch)
         eng.prefill(len(prompts[0]) - 1)
         eng.step(1, lm_head=True, logits=True, direct=True)
         return ids, np.stack([eng.read_logits(b) for b in range(batch)])
@@ -70,4 +70,15 @@ def test_steps_of_a_few_sequences(gpu, batch):
     ids, logits = _model(gpu, cfg, batch, 1, prompts)
     assert gpu.tc_gemm_count() > before
     want_ids, want = _model(gpu, cfg, batch, 0, prompts)
+    assert ids == want_ids and np.linalg.norm(logits - want) < 1e-5 * np.linalg.norm(want) and gpu.device_error() == 0
+
+
+def test_prompt_whose_gate_up_tiles_have_256_rows(gpu):
+    """512 prompt rows on a feed-forward block of 148 gate / up tiles, against the same prompts on the GEMV kernels."""
+    from adam_b200 import synth
+    from adam_b200.config import tiny_gemma3
+    cfg = tiny_gemma3(n_layer=2, n_vocab=1008, n_ff=9472)
+    prompts = [synth.random_prompt(cfg.n_vocab, 257, seed=300 + i) for i in range(2)]
+    ids, logits = _model(gpu, cfg, 2, 1, prompts)
+    want_ids, want = _model(gpu, cfg, 2, 0, prompts)
     assert ids == want_ids and np.linalg.norm(logits - want) < 1e-5 * np.linalg.norm(want) and gpu.device_error() == 0

