@@ -8,8 +8,8 @@ namespace ab {
 
 constexpr int TC_MIN_ROWS = 2;         // fewer rows than this never leave the GEMV kernels
 
-// Does this problem run on the tcgen05 path?  `tiled`: the GEMV kernels would have row-tiled copies of the weights; `wide`:
-// the weights' map says that fp16 may not hold them.
+// Does this problem run on a GEMM?  `t0`, `t1`: row-tiled copies of the weights, where there are any; `wide`: the weights' map
+// says that fp16 may not hold them.
 bool gemm_tc_supports(int wtype, const GemvArgs& a, const uint8_t* t0, const uint8_t* t1, bool wide);
 // Makes room for calls with up to `rows` activation rows of length K (outside any stream capture; longer calls run in
 // chunks).  The workspace only grows; false when out of memory.
