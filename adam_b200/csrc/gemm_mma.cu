@@ -15,7 +15,8 @@
 // where gemm_tc.cu has 2e-7 to 3.4e-7 and the GEMV 1.8e-7 to 7e-7.  (A nibble masked out of its word is a subnormal half, q 2^-24
 // or q 2^-20, and needs no conversion; but the tensor core aligns its products by their nominal exponents: 4e-7 to 1e-6.)
 //
-// One CTA per SM: 16 warps at most that multiply (12 where their sums need the registers) and one that fetches.  A unit is GW row groups of 16 rows (for a gate / up product the same 16 rows of both matrices); warp (r, s) owns unit
+// One CTA per SM: 16 warps at most that multiply (12 where their sums need the registers) and one that fetches.  A unit is GW row
+// groups of 16 rows (for a gate / up product the same 16 rows of both matrices); warp (r, s) owns unit
 // r of the CTA's U and slice s of KS of every stage's K.  A stage is KS * C tile pairs (64 values of K each) of all units and the
 // same K of the activation image, by bulk copies onto one mbarrier.  Work is dealt out as whole items (U units over all of
 // K) or, where those leave SMs idle, as stages of all items in a row; an item that several CTAs share is added up by the one
