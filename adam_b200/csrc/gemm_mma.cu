@@ -307,7 +307,7 @@ __global__ void __launch_bounds__((gm_warps(NTL, GW) + 1) * 32, 1) k_gemm_mma(co
                 return r;
             };
             int c_lo = 0, c_hi = 0;
-            auto slot_of = [&](int c) { return a.part + (size_t)(2 * c + (c == c_lo ? 1 : 0)) * (16 * 16 * BP) + (size_t)r_own * NV * 32 + lane; };     // it begins here, or before
+            auto slot_of = [&](int c) { return a.part + (size_t)(2 * c + (c == c_lo ? 1 : 0)) * GEMM_SLOT + (size_t)r_own * NV * 32 + lane; };     // it begins here, or before
             if (part) {
                 // an item that several CTAs share: leave the partial sums; the CTA that arrives last adds all of them
                 auto cta_of = [&](int qq) {
@@ -392,58 +392,74 @@ bool gemm_mma_supports(int wtype, const GemvArgs& a) {
     return (wtype == WT_Q4_0 || wtype == WT_Q4_K) && a.B <= GM_MAX_ROWS && a.N % 16 == 0 && a.K % (wtype == WT_Q4_0 ? 64 : 256) == 0;
 }
 
+struct GmCall { bool q40, pair, head; int N, K, B; };
 struct GmShape { int gw, U, KS, C, NS, grid; bool shared; };
-
-int launch_gemm_mma(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvArgs& a, const GemmWork& w, cudaStream_t stream) {
-    const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU, head = a.epi == EPI_ARGMAX, q40 = wtype == WT_Q4_0;
-    const int ntl = gemm_mma_pad(a.B) / 4, pairs = a.K / 64, n_rg = a.N / 16;
-    const int tile = mma_tile_bytes(wtype), blk = gm_block_bytes(wtype, 4 * ntl);
+static int gm_groups(const GmCall& p) { return (p.B + 3) / 4; }
+static int gm_wt(const GmCall& p) { return p.q40 ? WT_Q4_0 : WT_Q4_K; }
+static size_t gm_stage_bytes(const GmCall& p, const GmShape& f) {
+    return (size_t)f.KS * f.C * ((size_t)f.U * f.gw * mma_tile_bytes(gm_wt(p)) + 2 * gm_block_bytes(gm_wt(p), 4 * gm_groups(p)));
+}
+static size_t gm_red_bytes(const GmCall& p, const GmShape& f) { return f.KS > 1 || f.shared ? (size_t)f.U * f.KS * gm_groups(p) * 2 * f.gw * 128 : 0; }
+static int gm_steps(const GmCall& p, const GmShape& f) { return (p.K / 64 + f.KS * f.C - 1) / (f.KS * f.C); }      // stages per item
+static int gm_items(const GmCall& p, const GmShape& f) {
+    const int n_rg = p.N / 16, units = p.pair ? n_rg : (n_rg + f.gw - 1) / f.gw;
+    return (units + f.U - 1) / f.U;
+}
+static int gm_item_floats(const GmCall& p, const GmShape& f) { return f.U * gm_groups(p) * 2 * f.gw * 32; }         // sums of one item
+// Number of stages that fit (f.NS); false where that is too few, or where a shared item's sums do not fit the workspace.
+static bool gm_fits(const GmCall& p, GmShape& f) {
+    if (f.shared && gm_item_floats(p, f) > GEMM_SLOT) return false;
+    const size_t room = GM_SMEM - gm_red_bytes(p, f), st = gm_stage_bytes(p, f);
+    f.NS = room < st ? 0 : (int)(room / st);
+    if (f.NS > GM_MAX_STAGES) f.NS = GM_MAX_STAGES;
+    return f.NS >= 2 || (f.NS == 1 && gm_steps(p, f) == 1 && !f.shared);
+}
+// Shape: the cheapest under an estimate in SM cycles, fitted to sweeps of all shapes on 262144 x 1152, 21504 x 5376,
+// 1536 x 1152, 6912 x 1152 and 1152 x 6912 (2, 8 and 16 rows): a warp's tile pair takes 137 cycles of latency and a share of the
+// SM's pipes that grows with the warps and the rows, no less than its bytes from HBM; a stage some 100 cycles and 55 for each
+// of its bulk copies; an item its exchange; sharing items the workspace (about 4 us).
+static GmShape gm_shape(const GmCall& p, int sm_count) {
+    const int ntl = gm_groups(p), pairs = p.K / 64;
     GmShape s = {};
-    auto red_of = [&](const GmShape& f) { return f.KS > 1 || f.shared ? (size_t)f.U * f.KS * ntl * 2 * f.gw * 128 : 0; };
-    auto stage_of = [&](const GmShape& f) { return (size_t)f.U * f.gw * f.KS * f.C * tile + (size_t)f.KS * f.C * 2 * blk; };
-    auto fits = [&](GmShape& f) {
-        const size_t room = GM_SMEM - red_of(f), st = stage_of(f);
-        const int spi = (pairs + f.KS * f.C - 1) / (f.KS * f.C);
-        f.NS = room < st ? 0 : (int)(room / st);
-        if (f.NS > GM_MAX_STAGES) f.NS = GM_MAX_STAGES;
-        return f.NS >= 2 || (f.NS == 1 && spi == 1 && !f.shared);
-    };
-    auto items_of = [&](const GmShape& f) { const int units = pair ? n_rg : (n_rg + f.gw - 1) / f.gw; return (units + f.U - 1) / f.U; };
-    // Shape: the cheapest under an estimate in SM cycles, fitted to sweeps of all shapes on 262144 x 1152, 21504 x 5376,
-    // 1536 x 1152, 6912 x 1152 and 1152 x 6912 (2, 8 and 16 rows): a warp's tile pair takes 137 cycles of latency and a share of the
-    // SM's pipes that grows with the warps and the rows, no less than its bytes from HBM; a stage some 100 cycles and 55 for each
-    // of its bulk copies; an item its exchange; sharing items the workspace (about 4 us).
     double best = 1e300;
-    const double share = (q40 ? 15.0 : 21.0) + (q40 ? 10.0 : 11.0) * ntl, bytes = tile / 23.0;
-    for (int gw = pair ? 2 : 1; gw <= (head ? 1 : 2); ++gw)
+    const double share = (p.q40 ? 15.0 : 21.0) + (p.q40 ? 10.0 : 11.0) * ntl, bytes = mma_tile_bytes(gm_wt(p)) / 23.0;
+    for (int gw = p.pair ? 2 : 1; gw <= (p.head ? 1 : 2); ++gw)
         for (int U = 1; U <= gm_warps(ntl, gw) && U * gw <= 32; ++U)
             for (int ks = 1; U * ks <= gm_warps(ntl, gw) && ks <= pairs && (U <= 8 || ks == 1); ++ks)
                 for (int c = 1; c <= 8 && (c == 1 || ks * (c - 1) < pairs); ++c)
                     for (int sh = 0; sh < 2; ++sh) {
                         GmShape f = {gw, U, ks, c, 0, 0, sh != 0};
-                        if (!fits(f)) continue;
-                        const int step = ks * c, spi = (pairs + step - 1) / step, items = items_of(f), rest = pairs - (spi - 1) * step;
+                        if (!gm_fits(p, f)) continue;
+                        const int step = ks * c, spi = gm_steps(p, f), items = gm_items(p, f), rest = pairs - (spi - 1) * step;
                         const double nw = U * ks, lone = (137.0 + 30.0 * (gw - 1)) + nw * gw * share, mem = nw * gw * bytes;
                         const double per_pair = lone > mem ? lone : mem, fixed = 100.0 + 55.0 * U * gw, finish = 400.0 + (ks > 1 ? 300.0 : 0.0);
                         const double item = (spi - 1) * (c * per_pair + fixed) + (rest < c ? rest : c) * per_pair + fixed;
-                        const int whole = items < g.sm_count ? items : g.sm_count;
+                        const int whole = items < sm_count ? items : sm_count;
                         double cost;
                         if (sh) {
                             const long long all = (long long)items * spi;
-                            if (all <= g.sm_count || items % g.sm_count == 0) continue;
-                            const double per = (double)((all + g.sm_count - 1) / g.sm_count);
+                            if (all <= sm_count || items % sm_count == 0) continue;
+                            const double per = (double)((all + sm_count - 1) / sm_count);
                             cost = per * (c * per_pair + fixed) + (1.0 + per / spi) * finish + 8000.0 + spi / per * 300.0;
-                            f.grid = g.sm_count;
+                            f.grid = sm_count;
                         } else { cost = (double)((items + whole - 1) / whole) * (item + finish); f.grid = whole; }
                         if (cost < best * 0.999) { best = cost; s = f; }
                     }
+    return s;
+}
+
+int launch_gemm_mma(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvArgs& a, const GemmWork& w, cudaStream_t stream) {
+    const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU, head = a.epi == EPI_ARGMAX, q40 = wtype == WT_Q4_0;
+    const GmCall p = {q40, pair, head, a.N, a.K, a.B};
+    const int ntl = gm_groups(p), pairs = a.K / 64, n_rg = a.N / 16;
+    GmShape s = gm_shape(p, g.sm_count);
     if (const char* force = getenv("ADAM_B200_GM_SHAPE")) {
         int v[5];
         if (sscanf(force, "%d,%d,%d,%d,%d", &v[0], &v[1], &v[2], &v[3], &v[4]) == 5) {
             GmShape f = {pair ? 2 : head ? 1 : v[0], v[1], v[2], v[3], 0, 0, v[4] != 0};
-            if (f.U * f.KS <= gm_warps(ntl, f.gw) && f.U * f.gw <= 32 && f.KS <= pairs && (f.U <= 8 || f.KS == 1) && fits(f)) {
-                const int items = items_of(f);
-                if (f.shared && (long long)items * ((pairs + f.KS * f.C - 1) / (f.KS * f.C)) <= g.sm_count) f.shared = false;
+            if (f.U * f.KS <= gm_warps(ntl, f.gw) && f.U * f.gw <= 32 && f.KS <= pairs && (f.U <= 8 || f.KS == 1) && gm_fits(p, f)) {
+                const int items = gm_items(p, f);
+                if (f.shared && (long long)items * gm_steps(p, f) <= g.sm_count) f.shared = false;
                 f.grid = f.shared || items > g.sm_count ? g.sm_count : items;
                 s = f;
             } else s.U = 0;
@@ -453,7 +469,7 @@ int launch_gemm_mma(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvA
     GmArgs m = {};
     m.t0 = t0; m.t1 = t1; m.img = w.img; m.inv = w.inv; m.err = g.dev_err; m.y = a.y; m.ldy = a.ldy;
     m.N = a.N; m.n_rg = n_rg; m.pairs = pairs; m.B = a.B; m.pair = pair; m.swiglu = a.epi == EPI_SWIGLU;
-    m.U = s.U; m.KS = s.KS; m.C = s.C; m.NS = s.NS; m.spi = (pairs + s.KS * s.C - 1) / (s.KS * s.C); m.items = items_of(s); m.shared = s.shared;
+    m.U = s.U; m.KS = s.KS; m.C = s.C; m.NS = s.NS; m.spi = gm_steps(p, s); m.items = gm_items(p, s); m.shared = s.shared;
     m.part = w.part; m.tickets = w.tickets;
     if (head) { m.best = w.best; m.ticket = w.ticket; m.out_tok = a.out_tok; m.out_val = a.out_val; m.out_tok_f32 = a.out_tok_f32; m.softcap = a.softcap; }
     if (getenv("ADAM_B200_DEBUG")) fprintf(stderr, "[gemm_mma] N %d K %d B %d pair %d: %d,%d,%d,%d,%d, %d stages, grid %d\n", a.N, a.K, a.B, (int)pair, s.gw, s.U, s.KS, s.C, (int)s.shared, s.NS, s.grid);
@@ -467,10 +483,29 @@ int launch_gemm_mma(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvA
             return fail(ADAMAH_ERR_BACKEND, "gemm_mma: cannot raise the shared-memory limit");
         known = true;
     }
-    const cudaError_t e = launch_k(k, dim3((unsigned)s.grid), dim3((unsigned)(s.U * s.KS + 1) * 32), s.NS * stage_of(s) + red_of(s), stream, true, m);
+    const cudaError_t e = launch_k(k, dim3((unsigned)s.grid), dim3((unsigned)(s.U * s.KS + 1) * 32), s.NS * gm_stage_bytes(p, s) + gm_red_bytes(p, s), stream, true, m);
     if (e != cudaSuccess) return fail(ADAMAH_ERR_BACKEND, "gemm_mma: launch failed: %s", cudaGetErrorString(e));
     count_launch();
     return ADAMAH_OK;
 }
 
 }  // namespace ab
+
+// The launch shape that a product would get on a GPU of `sm_count` SMs, without a GPU: out[0..9] = row groups per warp, units, K slices,
+// tile pairs per stage and slice, stages, CTAs, items shared (0 / 1), floats of an item's sums, of the room for them in the workspace,
+// bytes of shared memory.
+extern "C" int adam_b200_few_rows_shape(uint32_t ggml_type, uint32_t n, uint32_t k, uint32_t rows, uint32_t kind, uint32_t sm_count, uint32_t* out) {
+    using namespace ab;
+    const int wt = ggml_type == 2 ? WT_Q4_0 : WT_Q4_K;
+    GemvArgs a = {};
+    a.N = (int)n; a.K = (int)k; a.B = (int)rows;
+    if ((ggml_type != 2 && ggml_type != 12) || kind > 2 || !out || !rows || rows > GM_MAX_ROWS || !n || !k || n > (1u << 30) || k > (1u << 30) || !sm_count || sm_count > 1024 ||
+        !gemm_mma_supports(wt, a))
+        return ADAMAH_ERR_INVALID;
+    const GmCall p = {wt == WT_Q4_0, kind == 1, kind == 2, a.N, a.K, a.B};
+    const GmShape s = gm_shape(p, (int)sm_count);
+    const uint32_t v[10] = {(uint32_t)s.gw, (uint32_t)s.U, (uint32_t)s.KS, (uint32_t)s.C, (uint32_t)s.NS, (uint32_t)s.grid, s.shared ? 1u : 0u,
+                            (uint32_t)gm_item_floats(p, s), (uint32_t)GEMM_SLOT, (uint32_t)(s.NS * gm_stage_bytes(p, s) + gm_red_bytes(p, s))};
+    for (int i = 0; i < 10; ++i) out[i] = v[i];
+    return ADAMAH_OK;
+}

@@ -65,8 +65,8 @@ bool gemm_tc_prepare(int rows, int K) {
         *p = q;
         return true;
     };
-    if (!g_tc.part) {                                   // two tiles of 128 x 256 sums and two tickets per CTA
-        if (!grow((void**)&g_tc.tickets, (size_t)g.sm_count * 8) || !grow((void**)&g_tc.part, (size_t)g.sm_count * 2 * 128 * 256 * 4)) return false;
+    if (!g_tc.part) {                                   // two slots of sums and two tickets per CTA
+        if (!grow((void**)&g_tc.tickets, (size_t)g.sm_count * 8) || !grow((void**)&g_tc.part, (size_t)g.sm_count * 2 * GEMM_SLOT * 4)) return false;
     }
     if (need > g_tc.img_cap) {
         size_t cap = need > 2 * g_tc.img_cap ? need : 2 * g_tc.img_cap;

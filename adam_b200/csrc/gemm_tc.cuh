@@ -7,6 +7,8 @@
 namespace ab {
 
 constexpr int TC_MIN_ROWS = 2;         // fewer rows than this never leave the GEMV kernels
+// Floats of one item's partial sums in the workspace; a CTA has two such slots, for its first and its last item.
+constexpr int GEMM_SLOT = 128 * 256;
 
 // Does this problem run on a GEMM?  `t0`, `t1`: row-tiled copies of the weights, where there are any; `wide`: the weights' map
 // says that fp16 may not hold them.

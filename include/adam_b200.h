@@ -390,6 +390,10 @@ int adam_b200_decoder_step_part(uint32_t id, uint32_t part, uint32_t flags);
 /* Number of matrix products enqueued so far on the GEMM kernels: the tcgen05 (tensor memory) one, which takes calls with many
  * activation rows, and the mma.sync one for a few rows over row-tiled weights; calls with fewer rows run on the GEMV kernels. */
 uint64_t adam_b200_tc_gemm_count(void);
+/* The launch shape that the GEMM for a few rows would take for a product (kind 0), a gate / up pair (1) or an arg-max (2) on a
+ * GPU of sm_count SMs; needs no GPU.  out[10]: row groups per warp, units, K slices, tile pairs per stage and slice, stages, CTAs,
+ * items shared between CTAs (0 / 1), floats of an item's sums, floats of a workspace slot, bytes of shared memory. */
+int adam_b200_few_rows_shape(uint32_t ggml_type, uint32_t n, uint32_t k, uint32_t rows, uint32_t kind, uint32_t sm_count, uint32_t* out);
 /* Which calls take it: 0 = none, 1 = those expected to be faster than the GEMV kernels (default; also the
  * initial value of environment variable ADAM_B200_TC), 2 = every call whose shape allows, on the tcgen05 one. */
 int adam_b200_tc_gemm_policy(int policy);

@@ -1,0 +1,50 @@
+"""Launch shapes of the GEMM for a few rows, chosen on the host: no GPU needed."""
+import ctypes
+
+import pytest
+
+from adam_b200 import _lib
+
+GROUPS, UNITS, SLICES, PAIRS, STAGES, CTAS, SHARED, ITEM, SLOT, SMEM = range(10)
+
+
+def _shape(ggml_type, n, k, rows, kind, sms=148):
+    out = (ctypes.c_uint32 * 10)()
+    assert _lib.load().adam_b200_few_rows_shape(ggml_type, n, k, rows, kind, sms, out) == 0
+    return list(out)
+
+
+# Gate / up pairs whose estimate picks shared items of more than 16 row groups, and the widths of the models that are timed.
+@pytest.mark.parametrize("ggml_type,n,k", [(12, 28672, 2560), (2, 28928, 3584), (2, 28672, 4864), (12, 14336, 4864), (12, 7168, 4864), (12, 7168, 5888),
+                                           (2, 6912, 1152), (12, 21504, 5376)])
+def test_a_shared_item_fits_its_slot(ggml_type, n, k):
+    """Two CTAs that share an item leave their sums in slots side by side: one may not reach into the other."""
+    for kind in range(3):
+        for rows in range(3, 17):
+            s = _shape(ggml_type, n, k, rows, kind)
+            assert s[ITEM] <= s[SLOT] or not s[SHARED], (rows, kind, s)
+            assert s[SMEM] <= 227 * 1024 - 2048 and s[STAGES] >= 1 and 1 <= s[CTAS] <= 148
+
+
+def test_shared_items_of_more_than_16_row_groups_are_met():
+    """The case above is not an empty one."""
+    s = _shape(12, 28672, 2560, 13, 1)
+    assert s[SHARED] and s[UNITS] * s[GROUPS] > 16
+
+
+@pytest.mark.parametrize("sms", [1, 3, 132, 148, 160])
+def test_shapes_of_odd_sizes(sms):
+    for ggml_type, step in ((2, 64), (12, 256)):
+        for n in (16, 48, 1008, 14352, 50000):
+            for k in (step, 5 * step, 7168, 32768):
+                for kind in range(3):
+                    for rows in (1, 4, 7, 12, 16):
+                        s = _shape(ggml_type, n, k, rows, kind, sms)
+                        assert s[ITEM] <= s[SLOT] or not s[SHARED], (ggml_type, n, k, rows, kind, s)
+                        assert s[UNITS] * s[SLICES] <= 16 and s[SMEM] <= 227 * 1024 - 2048
+
+
+@pytest.mark.parametrize("args", [(8, 128, 256, 4, 0, 148), (2, 100, 256, 4, 0, 148), (2, 128, 96, 4, 0, 148), (12, 128, 64, 4, 0, 148), (2, 128, 256, 17, 0, 148),
+                                  (2, 128, 256, 0, 0, 148), (2, 0, 256, 4, 0, 148), (2, 128, 256, 4, 3, 148), (2, 128, 256, 4, 0, 0)])
+def test_problems_it_does_not_take(args):
+    assert _lib.load().adam_b200_few_rows_shape(*args, (ctypes.c_uint32 * 10)()) < 0

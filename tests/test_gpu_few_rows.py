@@ -41,12 +41,12 @@ def test_few_rows(gpu, ggml_type, N, K, B, mean):
     assert e.max() < 5e-7 and gpu.device_error() == 0
 
 
-def _model(gpu, cfg, batch, policy, prompts):
+def _model(gpu, cfg, batch, policy, prompts, ggml_type=gb.GGML_TYPE_Q4_0):
     from adam_b200 import synth
     from adam_b200.config import GenerationConfig
     from adam_b200.engine import ADAMEngine
     gpu.tc_gemm_policy(policy)
-    eng = ADAMEngine(gpu, cfg, synth.build_model(cfg, gb.GGML_TYPE_Q4_0, seed=71), kv_cap=len(prompts[0]) + 40, kv_dtype="f32", max_batch=batch)
+    eng = ADAMEngine(gpu, cfg, synth.build_model(cfg, ggml_type, seed=71), kv_cap=len(prompts[0]) + 40, kv_dtype="f32", max_batch=batch)
     try:
         ids, _ = eng.generate_batch(prompts, GenerationConfig(max_tokens=4, eos_token_ids=(), temperature=0.0, top_k=1, repeat_penalty=1.0))
         eng.begin(prompts, [len(prompts[0]) + 30] * batch)
@@ -71,6 +71,19 @@ def test_steps_of_a_few_sequences(gpu, batch):
     assert gpu.tc_gemm_count() > before
     want_ids, want = _model(gpu, cfg, batch, 0, prompts)
     assert ids == want_ids and np.linalg.norm(logits - want) < 1e-5 * np.linalg.norm(want) and gpu.device_error() == 0
+
+
+# Feed-forward blocks whose gate / up items have 20 to 24 row groups and are shared between CTAs (test_few_rows_shapes.py).
+@pytest.mark.parametrize("ggml_type,n_embd,n_ff,batch", [(12, 2560, 28672, 13), (12, 4864, 7168, 16), (2, 3584, 28928, 12)])
+def test_steps_whose_gate_up_items_are_shared(gpu, ggml_type, n_embd, n_ff, batch):
+    """Against the same steps on the GEMV kernels: a dozen products in a row, each within 7e-7 of the exact one on either path."""
+    from adam_b200 import synth
+    from adam_b200.config import tiny_gemma3
+    cfg = tiny_gemma3(n_layer=1, n_embd=n_embd, n_ff=n_ff, n_vocab=256)
+    prompts = [synth.random_prompt(cfg.n_vocab, 3, seed=400 + i) for i in range(batch)]
+    ids, logits = _model(gpu, cfg, batch, 1, prompts, ggml_type)
+    want_ids, want = _model(gpu, cfg, batch, 0, prompts, ggml_type)
+    assert np.linalg.norm(logits - want) < 1e-5 * np.linalg.norm(want) and ids == want_ids and gpu.device_error() == 0
 
 
 def test_prompt_whose_gate_up_tiles_have_256_rows(gpu):
