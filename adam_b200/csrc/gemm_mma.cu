@@ -418,7 +418,7 @@ static bool gm_fits(const GmCall& p, GmShape& f) {
 // 1536 x 1152, 6912 x 1152 and 1152 x 6912 (2, 8 and 16 rows): a warp's tile pair takes 137 cycles of latency and a share of the
 // SM's pipes that grows with the warps and the rows, no less than its bytes from HBM; a stage some 100 cycles and 55 for each
 // of its bulk copies; an item its exchange; sharing items the workspace (about 4 us).
-static GmShape gm_shape(const GmCall& p, int sm_count) {
+static GmShape gm_search(const GmCall& p, int sm_count) {
     const int ntl = gm_groups(p), pairs = p.K / 64;
     GmShape s = {};
     double best = 1e300;
@@ -448,23 +448,39 @@ static GmShape gm_shape(const GmCall& p, int sm_count) {
     return s;
 }
 
+// ADAM_B200_GM_SHAPE="row groups per warp,units,k_slices,tile pairs,shared" (a tuning aid, read once) in place of the estimate
+// wherever a call can be launched so.
+static GmShape gm_forced(const GmCall& p, int sm_count, GmShape s) {
+    struct Force { bool set; int v[5]; };
+    static const Force force = [] {
+        Force f = {};
+        const char* e = getenv("ADAM_B200_GM_SHAPE");
+        f.set = e && sscanf(e, "%d,%d,%d,%d,%d", &f.v[0], &f.v[1], &f.v[2], &f.v[3], &f.v[4]) == 5;
+        return f;
+    }();
+    if (!force.set) return s;
+    GmShape f = {p.pair ? 2 : p.head ? 1 : force.v[0], force.v[1], force.v[2], force.v[3], 0, 0, force.v[4] != 0};
+    const int warps = gm_warps(gm_groups(p), f.gw);
+    if ((f.gw != 1 && f.gw != 2) || f.U < 1 || f.U > warps || f.U * f.gw > 32 || f.KS < 1 || f.KS > warps / f.U || f.KS > p.K / 64 || f.C < 1 || f.C > 8 || (f.U > 8 && f.KS > 1))
+        return s;
+    const int items = gm_items(p, f);
+    if ((long long)items * gm_steps(p, f) <= sm_count) f.shared = false;
+    if (!gm_fits(p, f)) return s;
+    f.grid = f.shared || items > sm_count ? sm_count : items;
+    return f;
+}
+static GmShape gm_shape(const GmCall& p, int sm_count) {
+    const GmShape s = gm_forced(p, sm_count, gm_search(p, sm_count));
+    if (getenv("ADAM_B200_DEBUG"))
+        fprintf(stderr, "[gemm_mma] N %d K %d rows %d pair %d: %d,%d,%d,%d,%d, %d stages, grid %d\n", p.N, p.K, 4 * gm_groups(p), (int)p.pair, s.gw, s.U, s.KS, s.C, (int)s.shared, s.NS, s.grid);
+    return s;
+}
+
 int launch_gemm_mma(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvArgs& a, const GemmWork& w, cudaStream_t stream) {
     const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU, head = a.epi == EPI_ARGMAX, q40 = wtype == WT_Q4_0;
     const GmCall p = {q40, pair, head, a.N, a.K, a.B};
     const int ntl = gm_groups(p), pairs = a.K / 64, n_rg = a.N / 16;
-    GmShape s = gm_shape(p, g.sm_count);
-    if (const char* force = getenv("ADAM_B200_GM_SHAPE")) {
-        int v[5];
-        if (sscanf(force, "%d,%d,%d,%d,%d", &v[0], &v[1], &v[2], &v[3], &v[4]) == 5) {
-            GmShape f = {pair ? 2 : head ? 1 : v[0], v[1], v[2], v[3], 0, 0, v[4] != 0};
-            if (f.U * f.KS <= gm_warps(ntl, f.gw) && f.U * f.gw <= 32 && f.KS <= pairs && (f.U <= 8 || f.KS == 1) && gm_fits(p, f)) {
-                const int items = gm_items(p, f);
-                if (f.shared && (long long)items * gm_steps(p, f) <= g.sm_count) f.shared = false;
-                f.grid = f.shared || items > g.sm_count ? g.sm_count : items;
-                s = f;
-            } else s.U = 0;
-        }
-    }
+    const GmShape s = gm_shape(p, g.sm_count);
     if (!s.U) return fail(ADAMAH_ERR_INVALID, "gemm_mma: shape not supported");
     GmArgs m = {};
     m.t0 = t0; m.t1 = t1; m.img = w.img; m.inv = w.inv; m.err = g.dev_err; m.y = a.y; m.ldy = a.ldy;
@@ -472,7 +488,6 @@ int launch_gemm_mma(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvA
     m.U = s.U; m.KS = s.KS; m.C = s.C; m.NS = s.NS; m.spi = gm_steps(p, s); m.items = gm_items(p, s); m.shared = s.shared;
     m.part = w.part; m.tickets = w.tickets;
     if (head) { m.best = w.best; m.ticket = w.ticket; m.out_tok = a.out_tok; m.out_val = a.out_val; m.out_tok_f32 = a.out_tok_f32; m.softcap = a.softcap; }
-    if (getenv("ADAM_B200_DEBUG")) fprintf(stderr, "[gemm_mma] N %d K %d B %d pair %d: %d,%d,%d,%d,%d, %d stages, grid %d\n", a.N, a.K, a.B, (int)pair, s.gw, s.U, s.KS, s.C, (int)s.shared, s.NS, s.grid);
     const GmKernel k = head ? (q40 ? gm_kernel<WT_Q4_0, 1, true>(ntl) : gm_kernel<WT_Q4_K, 1, true>(ntl))
                      : s.gw == 2 ? (q40 ? gm_kernel<WT_Q4_0, 2, false>(ntl) : gm_kernel<WT_Q4_K, 2, false>(ntl))
                                  : (q40 ? gm_kernel<WT_Q4_0, 1, false>(ntl) : gm_kernel<WT_Q4_K, 1, false>(ntl));
@@ -499,7 +514,7 @@ extern "C" int adam_b200_few_rows_shape(uint32_t ggml_type, uint32_t n, uint32_t
     const int wt = ggml_type == 2 ? WT_Q4_0 : WT_Q4_K;
     GemvArgs a = {};
     a.N = (int)n; a.K = (int)k; a.B = (int)rows;
-    if ((ggml_type != 2 && ggml_type != 12) || kind > 2 || !out || !rows || rows > GM_MAX_ROWS || !n || !k || n > (1u << 30) || k > (1u << 30) || !sm_count || sm_count > 1024 ||
+    if ((ggml_type != 2 && ggml_type != 12) || kind > 2 || !out || !rows || rows > GM_MAX_ROWS || !n || !k || n > (1u << 30) || k > 32768 || !sm_count || sm_count > 1024 ||
         !gemm_mma_supports(wt, a))
         return ADAMAH_ERR_INVALID;
     const GmCall p = {wt == WT_Q4_0, kind == 1, kind == 2, a.N, a.K, a.B};

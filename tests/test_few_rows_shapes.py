@@ -1,5 +1,8 @@
 """Launch shapes of the GEMM for a few rows, chosen on the host: no GPU needed."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import pytest
 
@@ -48,3 +51,14 @@ def test_shapes_of_odd_sizes(sms):
                                   (2, 128, 256, 0, 0, 148), (2, 0, 256, 4, 0, 148), (2, 128, 256, 4, 3, 148), (2, 128, 256, 4, 0, 0)])
 def test_problems_it_does_not_take(args):
     assert _lib.load().adam_b200_few_rows_shape(*args, (ctypes.c_uint32 * 10)()) < 0
+
+
+# 0 and negative units, slices and tile pairs; products of two that are in range though neither is; more than shared memory holds.
+@pytest.mark.parametrize("force", ["1,0,1,1,0", "1,1,0,1,0", "1,1,1,0,1", "1,-2,-3,1,0", "1,1,1,-1,0", "0,1,1,1,0", "3,1,1,1,0", "1,16,1,8,1", "2,16,1,1,1", "1,4,4,2,1"])
+def test_a_forced_shape_is_taken_where_it_can_be(force):
+    code = ("import ctypes; from adam_b200 import _lib; o = (ctypes.c_uint32 * 10)(); f = _lib.load().adam_b200_few_rows_shape\n"
+            "for a in ((2, 1152, 1152, 8, 0, 148), (12, 28672, 2560, 13, 1, 148), (2, 48, 64, 3, 2, 148)):\n"
+            "    assert f(*a, o) == 0; s = list(o); print(s)\n"
+            "    assert s[1] >= 1 and s[2] >= 1 and s[1] * s[2] <= 16 and 1 <= s[3] <= 8 and s[4] >= 1 and 1 <= s[5] <= 148 and (not s[6] or s[7] <= s[8]) and s[9] <= 230000")
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, ADAM_B200_GM_SHAPE=force), capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
