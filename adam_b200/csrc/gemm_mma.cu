@@ -27,6 +27,8 @@
 
 #include <cstdio>
 #include <cstdlib>
+#include <mutex>
+#include <unordered_map>
 
 namespace ab {
 
@@ -469,8 +471,18 @@ static GmShape gm_forced(const GmCall& p, int sm_count, GmShape s) {
     f.grid = f.shared || items > sm_count ? sm_count : items;
     return f;
 }
+// The search takes 4 to 16 us, as long as a small product: a shape is kept for the next call of the same problem.
 static GmShape gm_shape(const GmCall& p, int sm_count) {
+    static std::mutex lock;
+    static std::unordered_map<uint64_t, GmShape> known;
+    const uint64_t key = (uint64_t)(uint32_t)(p.N / 16) | (uint64_t)(p.K / 64) << 28 | (uint64_t)gm_groups(p) << 40 | (uint64_t)(p.q40 ? 1 : 0) << 44 |
+                         (uint64_t)(p.pair ? 1 : p.head ? 2 : 0) << 45 | (uint64_t)sm_count << 48;
+    std::lock_guard<std::mutex> work(lock);
+    const auto it = known.find(key);
+    if (it != known.end()) return it->second;
     const GmShape s = gm_forced(p, sm_count, gm_search(p, sm_count));
+    if (known.size() >= 4096) known.clear();
+    known[key] = s;
     if (getenv("ADAM_B200_DEBUG"))
         fprintf(stderr, "[gemm_mma] N %d K %d rows %d pair %d: %d,%d,%d,%d,%d, %d stages, grid %d\n", p.N, p.K, 4 * gm_groups(p), (int)p.pair, s.gw, s.U, s.KS, s.C, (int)s.shared, s.NS, s.grid);
     return s;

@@ -3,6 +3,7 @@ import ctypes
 import os
 import subprocess
 import sys
+import time
 
 import pytest
 
@@ -51,6 +52,21 @@ def test_shapes_of_odd_sizes(sms):
                                   (2, 128, 256, 0, 0, 148), (2, 0, 256, 4, 0, 148), (2, 128, 256, 4, 3, 148), (2, 128, 256, 4, 0, 0)])
 def test_problems_it_does_not_take(args):
     assert _lib.load().adam_b200_few_rows_shape(*args, (ctypes.c_uint32 * 10)()) < 0
+
+
+def test_a_shape_is_searched_once():
+    """A call that has been made before does not search again: a small part of the time of first calls, with a margin for noise."""
+    f, out = _lib.load().adam_b200_few_rows_shape, (ctypes.c_uint32 * 10)()
+
+    def seconds(sizes):
+        t = time.perf_counter()
+        for n in sizes:
+            assert f(12, n, 5376, 8, 0, 148, out) == 0
+        return time.perf_counter() - t
+
+    first = min(seconds(range(20000 + 16000 * i, 30000 + 16000 * i, 16)) for i in range(3))
+    again = min(seconds([21504] * 625) for _ in range(3))
+    assert again < first / 3
 
 
 # 0 and negative units, slices and tile pairs; products of two that are in range though neither is; more than shared memory holds.
