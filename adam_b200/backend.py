@@ -380,11 +380,18 @@ class Adamah:
         return int(self._lib.adam_b200_kernel_launches())
 
     def tc_gemm_count(self) -> int:
-        """Matrix products enqueued so far on the tcgen05 GEMM (calls with many activation rows)."""
+        """Matrix products enqueued so far on the GEMM kernels, few rows or many."""
         return int(self._lib.adam_b200_tc_gemm_count())
 
+    def gemm_counts(self) -> dict:
+        """Launches of the GEMM kernels so far, by kernel and split."""
+        names = ("few", "few_shared", "tile_16", "tile_32", "tile_64", "tile_128", "tile_256", "shared", "clusters", "cluster_waves")
+        out = (ctypes.c_uint64 * len(names))()
+        self._check(self._lib.adam_b200_gemm_counts(out, len(names)), "adam_b200_gemm_counts")
+        return dict(zip(names, out))
+
     def tc_gemm_policy(self, policy: int):
-        """0 = never take the tcgen05 GEMM, 1 = where it is expected to be faster (default), 2 = whenever the shape allows."""
+        """0 = never take the GEMM kernels, 1 = where they are expected to be faster (default), 2 = the tcgen05 one whenever the shape allows."""
         self._check(self._lib.adam_b200_tc_gemm_policy(int(policy)), "adam_b200_tc_gemm_policy")
 
     def device_error(self) -> int:

@@ -513,6 +513,8 @@ int launch_gemm_mma(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvA
     const cudaError_t e = launch_k(k, dim3((unsigned)s.grid), dim3((unsigned)(s.U * s.KS + 1) * 32), s.NS * gm_stage_bytes(p, s) + gm_red_bytes(p, s), stream, true, m);
     if (e != cudaSuccess) return fail(ADAMAH_ERR_BACKEND, "gemm_mma: launch failed: %s", cudaGetErrorString(e));
     count_launch();
+    ++g_gemm_counts[GC_FEW];
+    if (s.shared) ++g_gemm_counts[GC_FEW_SHARED];
     return ADAMAH_OK;
 }
 

@@ -42,6 +42,7 @@ struct TcWork { uint8_t* img; size_t img_cap; float* inv; int inv_cap; unsigned 
 static TcWork g_tc = {};
 static std::mutex g_tc_lock;            // the two kernels of a call are enqueued together: the image is one for all
 static uint64_t g_tc_calls = 0;
+uint64_t g_gemm_counts[GC_COUNTS] = {};
 static int g_tc_policy = -1;             // 0 never, 1 where it is expected to be faster, 2 whenever the shape allows; -1 = take it from ADAM_B200_TC
 
 static int tc_main_steps(int K) { return (K + 63) / 64; }
@@ -1174,11 +1175,16 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
         }
         for (int s = 2; s <= (head || n == 256 ? 1 : 8) && s <= n_main; ++s) {
             const int at_once = tc_clusters_at_once(s);
-            if (at_once < 1) continue;
+            if (at_once < 1 || (n == 128 && items > at_once)) continue;
             const int steps = (n_main + s - 1) / s + (n_min + s - 1) / s;
             offer((double)((items + at_once - 1) / at_once) * ((steps + sp - 1) / sp * sp * step + 2000.0), s, (int)items * s, false);
         }
     };
+    // Clusters of 128-row tiles only where all of them run at once.  A second wave starts CTAs anew (barriers, tensor memory, an empty
+    // pipeline), which the estimate does not see: us with and without it, 6912 pairs x 1152 on 320 rows 74.6 and 59.2, 1152 x 1024 on
+    // 1280 rows 39.1 and 20.1, 1536 x 1152 on 2048 rows 54.2 and 34.0, 1152 x 6912 on 1280 rows 98.9 and 68.6, 4096 x 2560 on 300
+    // rows 45.7 and 31.5.  Over 242 measured products (14 shapes, 65 to 2048 rows) the split chosen so takes 1.1 % longer than
+    // the best of all, 5.0 % with second waves.
     // Tiles of 256 rows take 1.9 times a tile of 128 (13824 x 1152 on 2048 rows 166 against 175 us, 21504 x 5376 on 1024 rows 598
     // against 631), so they are for calls whose tiles still fill the GPU: 1152 x 6912 on 2048 rows, 72 tiles, 121 against 95 us.
     if (a.B <= 64) offer_tiles(a.B <= 16 ? 16 : a.B <= 32 ? 32 : 64, a.B > 32 ? 620.0 : 500.0);
@@ -1210,6 +1216,9 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
     else e = launch_k_cluster(p.k, dim3((unsigned)grid), dim3(p.threads), (size_t)p.smem, stream, true, (unsigned)S, t);
     if (e != cudaSuccess) return fail(ADAMAH_ERR_BACKEND, "gemm_tc: launch failed: %s", cudaGetErrorString(e));
     count_launch();
+    ++g_gemm_counts[nt == 16 ? GC_TILE_16 : nt == 32 ? GC_TILE_32 : nt == 64 ? GC_TILE_64 : nt == 128 ? GC_TILE_128 : GC_TILE_256];
+    if (shared) ++g_gemm_counts[GC_SHARED];
+    if (S > 1) ++g_gemm_counts[t.items > tc_clusters_at_once(S) ? GC_CLUSTER_WAVES : GC_CLUSTERS];
     return ADAMAH_OK;
 }
 
@@ -1244,6 +1253,13 @@ int launch_gemm_tc(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvAr
 // Number of GEMMs enqueued on the tcgen05 path since the library was loaded (tests use it to
 // see which kernel a call took).
 extern "C" uint64_t adam_b200_tc_gemm_count(void) { return ab::g_tc_calls; }
+// The same by kernel and split: the first n values of the enumeration in gemm_tc.cuh.
+extern "C" int adam_b200_gemm_counts(uint64_t* out, uint32_t n) {
+    if (!out) return ADAMAH_ERR_INVALID;
+    std::lock_guard<std::mutex> work(ab::g_tc_lock);
+    for (uint32_t i = 0; i < n; ++i) out[i] = i < ab::GC_COUNTS ? ab::g_gemm_counts[i] : 0;
+    return ADAMAH_OK;
+}
 // 0 = never use the tcgen05 GEMM, 1 = where it is expected to be faster (default), 2 = whenever the shape allows.
 extern "C" int adam_b200_tc_gemm_policy(int policy) {
     if (policy < 0 || policy > 2) return ADAMAH_ERR_INVALID;

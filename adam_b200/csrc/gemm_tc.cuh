@@ -20,6 +20,11 @@ void gemm_tc_release();
 // Enqueues the row-quantisation kernel and the GEMM.  Returns ADAMAH_OK or an error code.
 int launch_gemm_tc(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvArgs& a, cudaStream_t stream);
 
+// Which kernels calls have taken, counted under the lock that orders them: the few-row kernel (also: with items shared between CTAs),
+// k_gemm_tc by rows of a tile (16 .. 256), with tiles shared, as clusters, and as more clusters than run at once.
+enum { GC_FEW, GC_FEW_SHARED, GC_TILE_16, GC_TILE_32, GC_TILE_64, GC_TILE_128, GC_TILE_256, GC_SHARED, GC_CLUSTERS, GC_CLUSTER_WAVES, GC_COUNTS };
+extern uint64_t g_gemm_counts[GC_COUNTS];
+
 // ---- gemm_mma.cu: the second kernel of a call with few rows ----
 constexpr int GM_MAX_ROWS = 16;
 // Bytes of the activation image per 32 values of K, with room for `rows` rows (a multiple of four).

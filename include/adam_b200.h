@@ -390,6 +390,10 @@ int adam_b200_decoder_step_part(uint32_t id, uint32_t part, uint32_t flags);
 /* Number of matrix products enqueued so far on the GEMM kernels: the tcgen05 (tensor memory) one, which takes calls with many
  * activation rows, and the mma.sync one for a few rows over row-tiled weights; calls with fewer rows run on the GEMV kernels. */
 uint64_t adam_b200_tc_gemm_count(void);
+/* The same by kernel and split, the first n of: few rows; few rows with items shared between CTAs; tcgen05 tiles of 16, 32, 64, 128
+ * and 256 activation rows; of those: tiles shared between CTAs, clusters, more clusters than run at once.  Launches, not calls: a
+ * call beyond the workspace runs in several. */
+int adam_b200_gemm_counts(uint64_t* out, uint32_t n);
 /* The launch shape that the GEMM for a few rows would take for a product (kind 0), a gate / up pair (1) or an arg-max (2) on a
  * GPU of sm_count SMs; needs no GPU.  out[10]: row groups per warp, units, K slices, tile pairs per stage and slice, stages, CTAs,
  * items shared between CTAs (0 / 1), floats of an item's sums, floats of a workspace slot, bytes of shared memory. */

@@ -62,6 +62,22 @@ def test_gemm_tiles_of_256_rows(gpu, ggml_type, N, K, B):
     assert gpu.device_error() == 0
 
 
+# Products that 128-row tiles as clusters would take several waves for.
+@pytest.mark.parametrize("N,K,B", [(1152, 1024, 1280), (1536, 1152, 1800), (1152, 6912, 1280), (4096, 2560, 300), (2560, 2048, 1024)])
+def test_clusters_run_in_one_wave(gpu, N, K, B):
+    """Clusters of CTAs that share a K are for calls whose tiles leave SMs idle: never more of them than run at once.  Error as in
+    test_gemm_tiles."""
+    rng = np.random.default_rng(N + K + B)
+    raw = gb.random_q4_0_blocks(rng, N, K)
+    x = rng.standard_normal((B, K), dtype=np.float32)
+    before = gpu.gemm_counts()
+    y = _gemv(gpu, 2, raw, N, K, x).astype(np.float64)
+    after = gpu.gemm_counts()
+    assert after["tile_128"] + after["tile_256"] > before["tile_128"] + before["tile_256"] and after["cluster_waves"] == before["cluster_waves"]
+    ref = x.astype(np.float64) @ q4_blocks.dequant(raw.reshape(-1), 2, N, K).astype(np.float64).T
+    assert (np.linalg.norm(y - ref, axis=1) / np.linalg.norm(ref, axis=1)).max() < 5e-6 and gpu.device_error() == 0
+
+
 def _gemm_error(gpu, ggml_type, raw, N, K, x):
     """Errors against float64, as 2-norms over the result's: of the GEMM, and of the GEMV that takes its place where it is refused."""
     ref = x.astype(np.float64) @ q4_blocks.dequant(raw.reshape(-1), ggml_type, N, K).astype(np.float64).T
