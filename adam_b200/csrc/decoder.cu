@@ -871,7 +871,11 @@ static int gemv(const Mat& m, const Mat* m2, GemvArgs a, int B, int epi) {
 #endif
     a.w0 = m.w; if (m2) a.w1 = m2->w;
     a.N = (int)m.rows; a.K = (int)m.cols; a.B = B; a.epi = epi;
-    if (B >= TC_MIN_ROWS && (!m2 || m2->wtype == m.wtype) && gemm_tc_supports(m.wtype, a, m.tiled, m2 ? m2->tiled : nullptr, g.maps[m.map_id].wide || (m2 && g.maps[m2->map_id].wide))) return launch_gemm_tc(m.wtype, m.tiled, m2 ? m2->tiled : nullptr, a, g.stream);
+    if (B >= TC_MIN_ROWS && (!m2 || m2->wtype == m.wtype)) {
+        const uint8_t* t1 = m2 ? m2->tiled : nullptr;
+        const GemmRoute route = gemm_route(m.wtype, a, m.tiled, t1, g.maps[m.map_id].wide || (m2 && g.maps[m2->map_id].wide));
+        if (route != GEMM_NONE) return launch_gemm(route, m.wtype, m.tiled, t1, a, g.stream);
+    }
     if (m.tiled && (!m2 || (m2->tiled && m2->wtype == m.wtype)) && gemv_mma_supports(m.wtype, a))
         return launch_gemv_mma(m.wtype, m.tiled, m2 ? m2->tiled : nullptr, a, g.stream);
     return launch_gemv(m.wtype, a, g.stream);
@@ -910,7 +914,7 @@ static int enqueue_head(Decoder* D, uint32_t r0, uint32_t rows, float* logits, i
     a.out_tok = tok; a.out_val = val;
     a.w0 = lm.w; a.N = (int)lm.rows; a.K = (int)lm.cols; a.B = (int)rows; a.epi = EPI_ARGMAX;
     D->h_final = 0;
-    if (gemm_tc_supports(lm.wtype, a, lm.tiled, nullptr, g.maps[lm.map_id].wide)) return launch_gemm_tc(lm.wtype, lm.tiled, nullptr, a, g.stream);
+    if (const GemmRoute route = gemm_route(lm.wtype, a, lm.tiled, nullptr, g.maps[lm.map_id].wide)) return launch_gemm(route, lm.wtype, lm.tiled, nullptr, a, g.stream);
     if (wt_is_b8(lm.wtype)) {
         // Q8_0 / Q5_0 LM head: the norm chain, the products and the arg-max as three kernels; the products land in the
         // logits buffer (soft-capped afterwards only when the caller wants them)

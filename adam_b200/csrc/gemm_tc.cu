@@ -25,6 +25,7 @@
 #include "gemm_tc.cuh"
 #include "gemv_mma.cuh"
 
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <mutex>
@@ -43,7 +44,7 @@ static TcWork g_tc = {};
 static std::mutex g_tc_lock;            // the two kernels of a call are enqueued together: the image is one for all
 static uint64_t g_tc_calls = 0;
 uint64_t g_gemm_counts[GC_COUNTS] = {};
-static int g_tc_policy = -1;             // 0 never, 1 where it is expected to be faster, 2 whenever the shape allows; -1 = take it from ADAM_B200_TC
+static std::atomic<int> g_tc_policy{-1};  // 0 never, 1 where it is expected to be faster, 2 whenever the shape allows; -1 = take it from ADAM_B200_TC
 
 static int tc_main_steps(int K) { return (K + 63) / 64; }
 static int tc_min_steps(int wtype, int K) { return wtype == WT_Q4_K ? (K / 32 + 63) / 64 : 0; }
@@ -1080,25 +1081,29 @@ static int tc_rows_from(int wtype, const GemvArgs& a, bool pair, bool tiled) {
 //   262144 x 1152 Q4_0  4: 48.5, 40.9   8: 65.6, 91.2   12: 86, 91.7    16: 108, 92.0
 // and ms a decode step: 1B shape 4 rows 0.887 and 0.894, 5 to 8 rows 1.04 and 1.12 to 1.15, 10 rows 1.226 and 1.220, 16 rows 1.365
 // and 1.242; 27B shape (8 layers) 2 rows 1.16 and 1.05, 3 rows 1.18 and 1.52, 8 rows 1.42 and 2.08, 16 rows 2.16 and 2.25.
-static bool takes_mma(int wtype, const GemvArgs& a, const uint8_t* t0, const uint8_t* t1) {
+static bool takes_mma(int wtype, const GemvArgs& a, const uint8_t* t0, const uint8_t* t1, int policy) {
     const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU;
-    if (!t0 || (pair && !t1) || g_tc_policy != 1 || !gemm_mma_supports(wtype, a)) return false;
+    if (!t0 || (pair && !t1) || policy != 1 || !gemm_mma_supports(wtype, a)) return false;
     const bool large = (double)a.N * a.K * 0.5625 * (pair ? 2 : 1) > 10.0e6 && !(a.epi == EPI_ARGMAX && a.K < 4096);
     if (large ? a.B < 3 : a.B < 5 || a.B > 8) return false;
     return (size_t)(a.K / 32) * gm_block_bytes(wtype, gemm_mma_pad(a.B)) <= g_tc.img_cap && gemm_mma_pad(a.B) <= g_tc.inv_cap;
 }
 
-bool gemm_tc_supports(int wtype, const GemvArgs& a, const uint8_t* t0, const uint8_t* t1, bool wide) {
+GemmRoute gemm_route(int wtype, const GemvArgs& a, const uint8_t* t0, const uint8_t* t1, bool wide) {
     const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU;
-    if (g_tc_policy < 0) g_tc_policy = getenv("ADAM_B200_TC") ? atoi(getenv("ADAM_B200_TC")) : 1;
-    if (wtype != WT_Q4_0 && wtype != WT_Q4_K && (wtype != WT_Q8_0 || pair)) return false;
-    if (a.B < TC_MIN_ROWS || a.K <= 0 || a.K > TC_MAX_K || a.N < 16 || (!a.y && a.epi != EPI_ARGMAX) || (wtype == WT_Q4_K ? (a.K % 256) : (a.K % 32))) return false;
-    if (a.epi == EPI_ARGMAX && a.B > tc_rows_fit(wtype, a.K)) return false;
-    if ((a.ldx & 3) || (!a.h_in && (!a.x || ((uintptr_t)a.x & 15)))) return false;
-    if (takes_mma(wtype, a, t0, t1)) return true;
-    if (wide) return false;
-    if (g_tc_policy == 0 || (g_tc_policy == 1 && a.B < tc_rows_from(wtype, a, pair, t0 && (t1 || !pair)))) return false;
-    return tc_rows_fit(wtype, a.K) >= 128;
+    int policy = g_tc_policy;
+    if (policy < 0) {
+        const int first = getenv("ADAM_B200_TC") ? atoi(getenv("ADAM_B200_TC")) : 1;
+        if (g_tc_policy.compare_exchange_strong(policy, first)) policy = first;
+    }
+    if (wtype != WT_Q4_0 && wtype != WT_Q4_K && (wtype != WT_Q8_0 || pair)) return GEMM_NONE;
+    if (a.B < TC_MIN_ROWS || a.K <= 0 || a.K > TC_MAX_K || a.N < 16 || (!a.y && a.epi != EPI_ARGMAX) || (wtype == WT_Q4_K ? (a.K % 256) : (a.K % 32))) return GEMM_NONE;
+    if (a.epi == EPI_ARGMAX && a.B > tc_rows_fit(wtype, a.K)) return GEMM_NONE;
+    if ((a.ldx & 3) || (!a.h_in && (!a.x || ((uintptr_t)a.x & 15)))) return GEMM_NONE;
+    if (takes_mma(wtype, a, t0, t1, policy)) return GEMM_FEW;
+    if (wide) return GEMM_NONE;
+    if (policy == 0 || (policy == 1 && a.B < tc_rows_from(wtype, a, pair, t0 && (t1 || !pair)))) return GEMM_NONE;
+    return tc_rows_fit(wtype, a.K) >= 128 ? GEMM_TC : GEMM_NONE;
 }
 
 typedef void (*TcKernel)(const TcGemm);
@@ -1223,9 +1228,9 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
 }
 
 // Rows that exceed the workspace run in chunks of whole 128-row tiles.
-int launch_gemm_tc(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvArgs& a, cudaStream_t stream) {
+int launch_gemm(GemmRoute route, int wtype, const uint8_t* t0, const uint8_t* t1, const GemvArgs& a, cudaStream_t stream) {
     std::lock_guard<std::mutex> work(g_tc_lock);
-    if (takes_mma(wtype, a, t0, t1)) {
+    if (route == GEMM_FEW) {
         launch_quant_rows<true>(a, tc_min_steps(wtype, a.K), gemm_mma_pad(a.B), stream);
         const int rc = launch_gemm_mma(wtype, t0, t1, a, GemmWork{g_tc.img, g_tc.inv, g_tc.part, g_tc.tickets, g_tc.best, (unsigned int*)(g_tc.best + g_tc.inv_cap)}, stream);
         if (rc) return rc;

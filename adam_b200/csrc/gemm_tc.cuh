@@ -10,15 +10,17 @@ constexpr int TC_MIN_ROWS = 2;         // fewer rows than this never leave the G
 // Floats of one item's partial sums in the workspace; a CTA has two such slots, for its first and its last item.
 constexpr int GEMM_SLOT = 128 * 256;
 
-// Does this problem run on a GEMM?  `t0`, `t1`: row-tiled copies of the weights, where there are any; `wide`: the weights' map
-// says that fp16 may not hold them.
-bool gemm_tc_supports(int wtype, const GemvArgs& a, const uint8_t* t0, const uint8_t* t1, bool wide);
+// Which GEMM a problem runs on, none for the GEMV kernels.  `t0`, `t1`: row-tiled copies of the weights, where there are any;
+// `wide`: the weights' map says that fp16 may not hold them.  Asked once per call: the answer goes with it, for the policy may
+// change in between.
+enum GemmRoute { GEMM_NONE, GEMM_FEW, GEMM_TC };
+GemmRoute gemm_route(int wtype, const GemvArgs& a, const uint8_t* t0, const uint8_t* t1, bool wide);
 // Makes room for calls with up to `rows` activation rows of length K (outside any stream capture; longer calls run in
 // chunks).  The workspace only grows; false when out of memory.
 bool gemm_tc_prepare(int rows, int K);
 void gemm_tc_release();
 // Enqueues the row-quantisation kernel and the GEMM.  Returns ADAMAH_OK or an error code.
-int launch_gemm_tc(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvArgs& a, cudaStream_t stream);
+int launch_gemm(GemmRoute route, int wtype, const uint8_t* t0, const uint8_t* t1, const GemvArgs& a, cudaStream_t stream);
 
 // Which kernels calls have taken, counted under the lock that orders them: the few-row kernel (also: with items shared between CTAs),
 // k_gemm_tc by rows of a tile (16 .. 256), with tiles shared, as clusters, and as more clusters than run at once.

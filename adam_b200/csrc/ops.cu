@@ -553,7 +553,7 @@ int run_gemv(uint32_t map_id, uint64_t off, int wtype, GemvArgs& ga) {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(g.stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) gemm_tc_prepare(ga.B, ga.K);
         const uint8_t* t = (const uint8_t*)find_tiled(map_id, off, (uint32_t)ga.N, (uint32_t)ga.K);
-        if (gemm_tc_supports(wtype, ga, t, nullptr, g.maps[map_id].wide)) return launch_gemm_tc(wtype, t, nullptr, ga, g.stream);
+        if (const GemmRoute route = gemm_route(wtype, ga, t, nullptr, g.maps[map_id].wide)) return launch_gemm(route, wtype, t, nullptr, ga, g.stream);
     }
     if (wt_is_b8(wtype)) {
         // Q8_0 / Q5_0: plain products from their own kernel; an arg-max is a second small kernel over the logits

@@ -95,3 +95,45 @@ def test_prompt_whose_gate_up_tiles_have_256_rows(gpu):
     ids, logits = _model(gpu, cfg, 2, 1, prompts)
     want_ids, want = _model(gpu, cfg, 2, 0, prompts)
     assert ids == want_ids and np.linalg.norm(logits - want) < 1e-5 * np.linalg.norm(want) and gpu.device_error() == 0
+
+
+def test_wide_weights_while_the_policy_changes(gpu):
+    """Weights beyond fp16 take the few-row kernel or the GEMV, never the tcgen05 GEMM, whenever another thread sets the policy."""
+    import threading
+    N, K, B, calls = 64, 512, 8, 200
+    rng = np.random.default_rng(5)
+    raw = gb.random_q4_0_blocks(rng, N, K).copy()
+    raw.reshape(-1, 18)[7::9, 0:2] = np.array([65504.0], np.float16).view(np.uint8)
+    x = rng.standard_normal((B, K), dtype=np.float32)
+    ref = x.astype(np.float64) @ q4_blocks.dequant(raw.reshape(-1), 2, N, K).astype(np.float64).T
+    gpu.map_create_typed(81, A.DTYPE_GGUF_Q4_0, 1, N * K)
+    gpu.upload_gguf_blocks(81, 2, 0, raw)
+    gpu.tile_tensor(81, 0, N, K)
+    gpu.map_create_typed(80, A.DTYPE_F32, 1, B * K + calls * B * N)
+    gpu.scatter_contiguous(80, 0, x)
+    zero = gpu.upload_dev(np.array([0], np.uint32))[0]
+    outs = [gpu.upload_dev(np.array([B * K + i * B * N], np.uint32))[0] for i in range(calls)]
+    done = threading.Event()
+
+    def change():
+        while not done.is_set():
+            gpu.tc_gemm_policy(2)
+            gpu.tc_gemm_policy(1)
+
+    thread = threading.Thread(target=change)
+    thread.start()
+    try:
+        for _ in range(20):
+            for h in outs:
+                gpu.map_matmul_t_xq4_dev(80, 81, zero, zero, h, B, K, N)
+            y = gpu.gather(80, np.arange(B * K, B * K + calls * B * N, dtype=np.uint32)).view(np.float32).reshape(calls, B, N).astype(np.float64)
+            assert (np.linalg.norm(y - ref, axis=(1, 2)) < 1e-6 * np.linalg.norm(ref)).all()
+    finally:
+        done.set()
+        thread.join()
+        gpu.tc_gemm_policy(1)
+        for h in [zero] + outs:
+            gpu.free_handle(h)
+        gpu.map_destroy(80)
+        gpu.map_destroy(81)
+    assert gpu.device_error() == 0
