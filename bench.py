@@ -215,9 +215,9 @@ def gemv_shape(gpu, A, t, N, K, B=1, target_bytes=600e6, reps=5, tile=True):
     a_h = gpu.upload_dev(np.array([0], np.uint32))[0]
     c_h = gpu.upload_dev(np.array([B * K], np.uint32))[0]
     bhs = [gpu.upload_dev(np.array([c * N * K], np.uint32))[0] for c in range(copies)]
-    tc0 = gpu.tc_gemm_count()
+    before = gpu.gemm_counts()
     gpu.map_matmul_t_xq4_dev(0, 1, a_h, bhs[0], c_h, B, K, N)       # eager once: workspaces are allocated outside the capture
-    tc_path = gpu.tc_gemm_count() > tc0
+    ran = [k for k, n in gpu.gemm_counts().items() if n > before[k]]
     gpu.capture_begin()
     for c in range(copies):
         gpu.map_matmul_t_xq4_dev(0, 1, a_h, bhs[c], c_h, B, K, N)
@@ -236,7 +236,8 @@ def gemv_shape(gpu, A, t, N, K, B=1, target_bytes=600e6, reps=5, tile=True):
     gpu.graph_launch(gid2, 2)
     gpu.batch_begin(); gpu.timer_begin(); gpu.graph_launch(gid2, 1); ms2 = gpu.timer_end(); gpu.batch_end()
     peak, _ = measured_peaks()
-    kernel = ("mma.sync GEMM" if tile and t in (2, 12) and B <= 16 else "tcgen05 GEMM") if tc_path else ("CUDA-core GEMV (planes)" if t in (8, 6) else "tensor-core GEMV (tiled)" if tile else "CUDA-core GEMV")
+    kernel = ("mma.sync GEMM" if "few" in ran else "tcgen05 GEMM" if ran else "CUDA-core GEMV (planes)" if t in (8, 6) else
+              "tensor-core GEMV (tiled)" if tile else "CUDA-core GEMV")
     out = dict(type=_BLOCK_NAME[t], kernel=kernel,
                N=N, K=K, B=B, copies=copies, bytes_per_launch=int(alg), us_per_launch=round(best * 1e3 / copies, 3), GBs=round(gbs, 1),
                frac_of_measured=round(gbs / peak, 3), frac_of_8TBs=round(gbs / 8000, 3), warm_us_per_launch=round(ms2 * 1e3 / 20, 3))
