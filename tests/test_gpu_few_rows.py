@@ -34,9 +34,9 @@ def test_few_rows(gpu, ggml_type, N, K, B, mean):
     rng = np.random.default_rng(N + K + B)
     raw = {2: gb.random_q4_0_blocks, 12: gb.random_q4_k_blocks}[ggml_type](rng, N, K)
     x = (rng.standard_normal((B, K), dtype=np.float32) + np.float32(mean)) * rng.uniform(0.01, 100.0, (B, 1)).astype(np.float32)
-    before = gpu.tc_gemm_count()
+    before = gpu.gemm_counts()
     e = _error(gpu, ggml_type, raw, N, K, x, 1)
-    assert gpu.tc_gemm_count() == before + 1
+    assert gpu.gemm_counts()["few"] == before["few"] + 1
     print(f"error {e.max():.2e}, GEMV {_error(gpu, ggml_type, raw, N, K, x, 0).max():.2e}")
     assert e.max() < 5e-7 and gpu.device_error() == 0
 
@@ -66,9 +66,9 @@ def test_steps_of_a_few_sequences(gpu, batch):
     from adam_b200.config import tiny_gemma3
     cfg = tiny_gemma3(n_layer=2, n_vocab=1008)
     prompts = [synth.random_prompt(cfg.n_vocab, 9, seed=200 + i) for i in range(batch)]
-    before = gpu.tc_gemm_count()
+    before = gpu.gemm_counts()
     ids, logits = _model(gpu, cfg, batch, 1, prompts)
-    assert gpu.tc_gemm_count() > before
+    assert gpu.gemm_counts()["few"] > before["few"]
     want_ids, want = _model(gpu, cfg, batch, 0, prompts)
     assert ids == want_ids and np.linalg.norm(logits - want) < 1e-5 * np.linalg.norm(want) and gpu.device_error() == 0
 
@@ -81,20 +81,60 @@ def test_steps_whose_gate_up_items_are_shared(gpu, ggml_type, n_embd, n_ff, batc
     from adam_b200.config import tiny_gemma3
     cfg = tiny_gemma3(n_layer=1, n_embd=n_embd, n_ff=n_ff, n_vocab=256)
     prompts = [synth.random_prompt(cfg.n_vocab, 3, seed=400 + i) for i in range(batch)]
+    before = gpu.gemm_counts()
     ids, logits = _model(gpu, cfg, batch, 1, prompts, ggml_type)
+    assert gpu.gemm_counts()["few_shared"] > before["few_shared"]
     want_ids, want = _model(gpu, cfg, batch, 0, prompts, ggml_type)
     assert np.linalg.norm(logits - want) < 1e-5 * np.linalg.norm(want) and ids == want_ids and gpu.device_error() == 0
 
 
-def test_prompt_whose_gate_up_tiles_have_256_rows(gpu):
-    """512 prompt rows on a feed-forward block of 148 gate / up tiles, against the same prompts on the GEMV kernels."""
+@pytest.mark.parametrize("n_embd,n_ff,tokens,shared", [(256, 9472, 257, False), (2560, 10240, 513, True)])
+def test_prompt_whose_gate_up_tiles_have_256_rows(gpu, n_embd, n_ff, tokens, shared):
+    """512 prompt rows on a feed-forward block of 148 gate / up tiles, 1024 on one of 640 that CTAs share, against the same prompts
+    on the GEMV kernels."""
     from adam_b200 import synth
     from adam_b200.config import tiny_gemma3
-    cfg = tiny_gemma3(n_layer=2, n_vocab=1008, n_ff=9472)
-    prompts = [synth.random_prompt(cfg.n_vocab, 257, seed=300 + i) for i in range(2)]
+    cfg = tiny_gemma3(n_layer=1 if shared else 2, n_embd=n_embd, n_vocab=1008, n_ff=n_ff)
+    prompts = [synth.random_prompt(cfg.n_vocab, tokens, seed=300 + i) for i in range(2)]
+    before = gpu.gemm_counts()
     ids, logits = _model(gpu, cfg, 2, 1, prompts)
+    after = gpu.gemm_counts()
+    assert after["tile_256"] > before["tile_256"] and (after["shared"] > before["shared"] or not shared)
     want_ids, want = _model(gpu, cfg, 2, 0, prompts)
     assert ids == want_ids and np.linalg.norm(logits - want) < 1e-5 * np.linalg.norm(want) and gpu.device_error() == 0
+
+
+# Gate / up products and heads of one to four groups of four rows: units of many row groups, items shared between CTAs (the pairs of
+# 7168 x 4864), a last item with fewer row groups than the others.
+@pytest.mark.parametrize("ggml_type,n_embd,n_ff,n_vocab,batch", [
+    (12, 4864, 7168, 8208, 3), (12, 4864, 7168, 8208, 4), (12, 4864, 7168, 8208, 9), (12, 4864, 7168, 8208, 15), (2, 1152, 6912, 40016, 5), (2, 1152, 6976, 40016, 8), (2, 256, 512, 65552, 7)])
+def test_steps_of_wide_blocks(gpu, ggml_type, n_embd, n_ff, n_vocab, batch):
+    """Gate / up products, the arg-max and the stored logits of the few-row kernel against the GEMV kernels', as above."""
+    from adam_b200 import synth
+    from adam_b200.config import tiny_gemma3
+    cfg = tiny_gemma3(n_layer=1, n_embd=n_embd, n_ff=n_ff, n_vocab=n_vocab)
+    prompts = [synth.random_prompt(cfg.n_vocab, 2, seed=500 + i) for i in range(batch)]
+    before = gpu.gemm_counts()
+    ids, logits = _model(gpu, cfg, batch, 1, prompts, ggml_type)
+    assert gpu.gemm_counts()["few"] >= before["few"] + 3
+    want_ids, want = _model(gpu, cfg, batch, 0, prompts, ggml_type)
+    assert ids == want_ids and np.linalg.norm(logits - want) < 1e-5 * np.linalg.norm(want) and gpu.device_error() == 0
+
+
+@pytest.mark.parametrize("ggml_type,N,K,B", [(2, 1152, 1152, 6), (12, 5376, 5632, 4), (12, 21504, 1024, 16)])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_rows_that_are_not_finite(gpu, ggml_type, N, K, B, bad):
+    """A row with an infinity or a NaN has no finite result, and the other rows have the bits that they have without it."""
+    rng = np.random.default_rng(N + B)
+    raw = {2: gb.random_q4_0_blocks, 12: gb.random_q4_k_blocks}[ggml_type](rng, N, K)
+    x = rng.standard_normal((B, K), dtype=np.float32)
+    want = _gemv(gpu, ggml_type, raw, N, K, x, tile=True)
+    x[B // 2, K - 5] = bad
+    before = gpu.gemm_counts()
+    y = _gemv(gpu, ggml_type, raw, N, K, x, tile=True)
+    assert gpu.gemm_counts()["few"] == before["few"] + 1
+    others = np.arange(B) != B // 2
+    assert np.array_equal(y[others], want[others]) and not np.isfinite(y[B // 2]).any()
 
 
 def test_wide_weights_while_the_policy_changes(gpu):
