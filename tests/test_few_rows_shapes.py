@@ -36,6 +36,18 @@ def test_shared_items_of_more_than_16_row_groups_are_met():
     assert s[SHARED] and s[UNITS] * s[GROUPS] > 16
 
 
+@pytest.mark.parametrize("kind", [0, 1, 2])
+def test_a_cta_of_several_items_has_two_stages(kind):
+    """With one stage nothing is fetched while a CTA multiplies: only for CTAs that have one item."""
+    for ggml_type, step in ((2, 64), (12, 256)):
+        for n in (1152, 5376, 16384, 21504, 65536, 131072, 262144):
+            for k in (step, 768, 1536, 2560, 5376, 21504):
+                for rows in (3, 8, 12, 16):
+                    s = _shape(ggml_type, n, k, rows, kind)
+                    items = -(-(-(-n // 16 // (1 if kind == 1 else s[GROUPS]))) // s[UNITS])
+                    assert s[STAGES] >= 2 or items <= s[CTAS], (ggml_type, n, k, rows, s)
+
+
 @pytest.mark.parametrize("sms", [1, 3, 132, 148, 160])
 def test_shapes_of_odd_sizes(sms):
     for ggml_type, step in ((2, 64), (12, 256)):
