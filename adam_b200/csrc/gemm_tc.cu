@@ -688,9 +688,10 @@ __global__ void __launch_bounds__(TcGeo<WT, NT>::THREADS, 1) k_gemm_tc(const TcG
         // ---- results: the accumulators into registers; an item's end: scale back, activation, store ----
         reg_inc<G::REG_READ>();
         pdl_wait();
-        // Which half it reads, and its thread.  Both are constants where one warpgroup reads: with rd and the barrier's number in
-        // registers a text of 65 tokens at the 1B shape is scored in 3950 us instead of 3890.
-        const int rd = NH == 1 ? 0 : wg - 1, rt = tid - (rd + 1) * 128;
+        // Which half it reads, and its thread.  rd and the barrier's number are constants where one warpgroup reads: in registers they
+        // cost spills at NT = 64 (a text of 65 tokens at the 1B shape is scored in 3960 us instead of 3900).  rt comes from wg: from
+        // rd it costs spills in the Q4_K instance of NT = 128 (a 27B prompt of 100 tokens and 24 steps 24.08 ms instead of 23.98).
+        const int rd = NH == 1 ? 0 : wg - 1, rt = tid - wg * 128;
         auto sync_rd = [&]() { asm volatile("bar.sync %0, 128;" :: "r"(rd + 1) : "memory"); };
         float* xch = reinterpret_cast<float*>(sm + G::XCH) + rd * (G::XCOLS * 128);
         uint32_t nth = 0;                               // accumulation period
