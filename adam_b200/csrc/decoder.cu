@@ -89,9 +89,9 @@ constexpr uint32_t MAX_DECODERS = 8;
 constexpr uint32_t ATTN_SPLIT = 64;        // fewest tokens an attention CTA takes before another CTA is added
 constexpr uint32_t ATTN_MAX_SPLITS = 64;   // attention CTAs per (sequence, kv head)
 // Rows (sequences x tokens) of one prefill chunk: 1024, or 2048 where the tiles of an n_embd-wide product (128 x 128) do not
-// give every SM one at 1024.  512 / 1024 / 2048 rows: 32 prompts x 512 and their 24 steps at the 1B shape (n_embd 1152, 72
-// tiles at 1024) 185 / 147 / 135 ms, one prompt of 1500 tokens with 12 steps 32.3 / 28.5 / 24.5 ms, 64 x 128 at the 27B shape
-// (8 layers, 336 tiles) 222 / 222 / 229 ms.
+// give every SM one at 1024.  Prompts and one step, ms with 1024 and with 2048 rows: 1B shape (n_embd 1152, 72 tiles at 1024)
+// 32 prompts x 512 105.4 and 90.8, 8 x 160 12.5 and 8.7, one of 1500 tokens 13.5 and 10.6; 27B shape (8 layers, 336 tiles)
+// 64 x 128 175.6 and 178.0, 16 x 128 45.0 and 45.8, 4 x 900 83.8 and 86.9, one of 900 tokens 22.2 and 22.2.
 static uint32_t prefill_rows(uint32_t n_embd) { return (uint64_t)((n_embd + 127) / 128) * (1024 / 128) < (uint64_t)g.sm_count ? 2048u : 1024u; }
 static Decoder* g_dec[MAX_DECODERS];
 

@@ -418,15 +418,19 @@ static bool gm_fits(const GmCall& p, GmShape& f, int sm_count) {
     if (f.NS > GM_MAX_STAGES) f.NS = GM_MAX_STAGES;
     return f.NS >= 2 || (f.NS == 1 && gm_steps(p, f) == 1 && !f.shared && gm_items(p, f) <= sm_count);
 }
-// Shape: the cheapest under an estimate in SM cycles, fitted to sweeps of all shapes on 262144 x 1152, 21504 x 5376,
-// 1536 x 1152, 6912 x 1152 and 1152 x 6912 (2, 8 and 16 rows): a warp's tile pair takes 137 cycles of latency and a share of the
-// SM's pipes that grows with the warps and the rows, no less than its bytes from HBM; a stage some 100 cycles and 55 for each
-// of its bulk copies; an item its exchange; sharing items the workspace (about 4 us).
+// Shape: the cheapest under an estimate in SM cycles, fitted to sweeps of shapes on 262144 x 1152, 21504 x 5376, 1536 x 1152, 6912 x 1152
+// and 1152 x 6912 (2, 8 and 16 rows) and on ten products with long K (8, 12 and 16 rows, 2520 shapes in all): a warp's tile pair
+// takes 137 cycles of latency and a share of the SM's pipes that grows with the warps and the rows, no less than its bytes from HBM
+// and those of the activation image from L2 (86 a cycle); a stage some 140 cycles, 60 for each of its bulk copies and 60 more where
+// the next one alone is in flight; an item its exchange, the slices of K one after the other; sharing items the workspace (about 8 us).
+// The shapes chosen so are 1.5 % slower than the best measured ones, 5.6 % without the image and with a cheaper exchange and
+// workspace: 2560 x 10240 Q4_K on 12 rows 22.0 us and 19.4, 24576 x 1024
+// Q4_0 on 16 rows 13.2 and 10.6, 131072 x 2560 Q4_0 on 8 rows 71.2 and 56.6; 6912 x 1152 Q4_0 on 8 rows 5.49 and 5.69.
 static GmShape gm_search(const GmCall& p, int sm_count) {
     const int ntl = gm_groups(p), pairs = p.K / 64;
     GmShape s = {};
     double best = 1e300;
-    const double share = (p.q40 ? 15.0 : 21.0) + (p.q40 ? 10.0 : 11.0) * ntl, bytes = mma_tile_bytes(gm_wt(p)) / 23.0;
+    const double share = (p.q40 ? 15.0 : 21.0) + (p.q40 ? 10.0 : 11.0) * ntl, bytes = mma_tile_bytes(gm_wt(p)) / 23.0, img = 2 * gm_block_bytes(gm_wt(p), 4 * ntl) / 86.0;
     for (int gw = p.pair ? 2 : 1; gw <= (p.head ? 1 : 2); ++gw)
         for (int U = 1; U <= gm_warps(ntl, gw) && U * gw <= 32; ++U)
             for (int ks = 1; U * ks <= gm_warps(ntl, gw) && ks <= pairs && (U <= 8 || ks == 1); ++ks)
@@ -435,8 +439,9 @@ static GmShape gm_search(const GmCall& p, int sm_count) {
                         GmShape f = {gw, U, ks, c, 0, 0, sh != 0};
                         if (!gm_fits(p, f, sm_count)) continue;
                         const int step = ks * c, spi = gm_steps(p, f), items = gm_items(p, f), rest = pairs - (spi - 1) * step;
-                        const double nw = U * ks, lone = (137.0 + 30.0 * (gw - 1)) + nw * gw * share, mem = nw * gw * bytes;
-                        const double per_pair = lone > mem ? lone : mem, fixed = 100.0 + 55.0 * U * gw, finish = 400.0 + (ks > 1 ? 300.0 : 0.0);
+                        const double nw = U * ks, lone = (137.0 + 30.0 * (gw - 1)) + nw * gw * share, mem = nw * gw * bytes + ks * img;
+                        const double per_pair = lone > mem ? lone : mem, fixed = 140.0 + 60.0 * U * gw + (f.NS == 2 ? 60.0 : 0.0);
+                        const double finish = 400.0 + (ks > 1 ? 1000.0 + 14.0 * ks * ntl * gw : 0.0);
                         const double item = (spi - 1) * (c * per_pair + fixed) + (rest < c ? rest : c) * per_pair + fixed;
                         const int whole = items < sm_count ? items : sm_count;
                         double cost;
@@ -444,7 +449,7 @@ static GmShape gm_search(const GmCall& p, int sm_count) {
                             const long long all = (long long)items * spi;
                             if (all <= sm_count || items % sm_count == 0) continue;
                             const double per = (double)((all + sm_count - 1) / sm_count);
-                            cost = per * (c * per_pair + fixed) + (1.0 + per / spi) * finish + 8000.0 + spi / per * 300.0;
+                            cost = per * (c * per_pair + fixed) + (1.0 + per / spi) * finish + 15000.0 + spi / per * 300.0;
                             f.grid = sm_count;
                         } else { cost = (double)((items + whole - 1) / whole) * (item + finish); f.grid = whole; }
                         if (cost < best * 0.999) { best = cost; s = f; }

@@ -368,7 +368,7 @@ __device__ __forceinline__ void q4k_codes(const uint4& h, int g, uint32_t& sp, u
 //                the issuing warp costs 86 cycles even if satisfied and only some four instructions queue ahead of the tensor
 //                core (a barrier per plane: 640 us instead of 598).  A round trip over the accumulator costs 289 cycles and the
 //                reading of 128 columns 280 more, twice per 3072 cycles of products; two warpgroups read.  Bound by these
-//                trips and the waits (tensor pipe 56 % active), not by rebuilding (leaving it out: -7 %).
+//                trips and the waits (tensor pipe 63 % active at 21504 x 5376 Q4_K on 1024 rows), not by rebuilding (leaving it out: -7 %).
 //   work split   Three ways, by an estimate of their times (launch_rows).  Whole tiles, dealt in turn.  Or all stages
 //                of all tiles in a row, dealt out evenly: a tile that several CTAs share is added up by the one that ends
 //                last (atomic ticket, partial sums in a workspace), in the order of K; 168 tiles on 148 SMs take 1.14 tiles'
@@ -1192,7 +1192,8 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
     // rows 45.7 and 31.5.  Over 242 measured products (14 shapes, 65 to 2048 rows) the split chosen so takes 1.1 % longer than
     // the best of all, 5.0 % with second waves.
     // Tiles of 256 rows take 1.9 times a tile of 128 (13824 x 1152 on 2048 rows 166 against 175 us, 21504 x 5376 on 1024 rows 598
-    // against 631), so they are for calls whose tiles still fill the GPU: 1152 x 6912 on 2048 rows, 72 tiles, 121 against 95 us.
+    // against 631), so they win where their number suits the SMs as well as that of the smaller ones does: 5376 x 4096 Q4_K on 768 rows,
+    // 126 tiles, 97 against 100 us, but 1152 x 6912 on 2048 rows, 72 tiles, 120 against 92.
     if (a.B <= 64) offer_tiles(a.B <= 16 ? 16 : a.B <= 32 ? 32 : 64, a.B > 32 ? 620.0 : 500.0);
     else {
         offer_tiles(128, 1250.0);

@@ -19,7 +19,7 @@ def _shape(ggml_type, n, k, rows, kind, sms=148):
 
 
 # Gate / up pairs whose estimate picks shared items of more than 16 row groups, and the widths of the models that are timed.
-@pytest.mark.parametrize("ggml_type,n,k", [(12, 28672, 2560), (2, 28928, 3584), (2, 28672, 4864), (12, 14336, 4864), (12, 7168, 4864), (12, 7168, 5888),
+@pytest.mark.parametrize("ggml_type,n,k", [(12, 28672, 2560), (2, 28928, 3584), (12, 28672, 3584), (2, 28672, 4864), (12, 14336, 4864), (12, 7168, 4864), (12, 7168, 5888),
                                            (2, 6912, 1152), (12, 21504, 5376)])
 def test_a_shared_item_fits_its_slot(ggml_type, n, k):
     """Two CTAs that share an item leave their sums in slots side by side: one may not reach into the other."""
@@ -32,7 +32,7 @@ def test_a_shared_item_fits_its_slot(ggml_type, n, k):
 
 def test_shared_items_of_more_than_16_row_groups_are_met():
     """The case above is not an empty one."""
-    s = _shape(12, 28672, 2560, 13, 1)
+    s = _shape(12, 28672, 3584, 12, 1)
     assert s[SHARED] and s[UNITS] * s[GROUPS] > 16
 
 
