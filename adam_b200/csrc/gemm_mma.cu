@@ -495,6 +495,11 @@ static GmShape gm_shape(const GmCall& p, int sm_count) {
     return s;
 }
 
+int gemm_mma_ctas(int wtype, const GemvArgs& a) {
+    const GmCall p = {wtype == WT_Q4_0, a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU, a.epi == EPI_ARGMAX, a.N, a.K, a.B};
+    return gm_shape(p, g.sm_count).grid;
+}
+
 int launch_gemm_mma(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvArgs& a, const GemmWork& w, cudaStream_t stream) {
     const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU, head = a.epi == EPI_ARGMAX, q40 = wtype == WT_Q4_0;
     const GmCall p = {q40, pair, head, a.N, a.K, a.B};

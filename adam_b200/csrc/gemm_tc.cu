@@ -1073,20 +1073,33 @@ static int tc_rows_from(int wtype, const GemvArgs& a, bool pair, bool tiled) {
     return bytes > 10.0e6 ? 6 : 9;
 }
 
+static int tc_clusters_at_once(int s);
 // Does the call take the mma.sync kernel (gemm_mma.cu)?  Matrices above 10 MB from 3 rows to 16, smaller ones and the heads of
 // narrow models from 5 to 8.  us a call, row kernel included, with it and without (GEMV up to 5 rows, above that k_gemm_tc), by rows:
-//   21504 x 5376 Q4_K   2: 26.7, 24.2   4: 26.7, 32.7   8: 29.8, 46.9   16: 42.2, 47.4   32: 75, 54.5
-//   5376 x 21504 Q4_K   2: 30.3, 36.5   4: 30.6, 60.5   8: 38.2, 54.1   16: 47.8, 55.0   32: 77, 61.9
-//   1152 x 6912 Q4_0    4: 6.1, 8.2     8: 7.7, 10.1    12: 9.3, 9.9    16: 10.7, 10.0
-//   6912 x 1152 Q4_0    4: 4.7, 7.5     8: 5.4, 9.0     16: 7.3, 8.7
+//   21504 x 5376 Q4_K   2: 26.7, 24.2   4: 24.1, 32.2   8: 29.4, 47.3   16: 42.1, 47.6   32: 75, 54.5
+//   5376 x 21504 Q4_K   2: 30.3, 36.5   4: 30.1, 59.8   8: 34.2, 54.2   16: 47.9, 55.0   32: 77, 61.9
+//   1152 x 6912 Q4_0    4: 6.1, 8.2     8: 7.7, 9.8     12: 9.3, 9.9    16: 10.7, 10.0
+//   6912 x 1152 Q4_0    4: 4.7, 7.5     8: 5.7, 8.2     16: 7.3, 8.7
 //   262144 x 1152 Q4_0  4: 48.5, 40.9   8: 65.6, 91.2   12: 86, 91.7    16: 108, 92.0
 // and ms a decode step: 1B shape 4 rows 0.887 and 0.894, 5 to 8 rows 1.04 and 1.12 to 1.15, 10 rows 1.226 and 1.220, 16 rows 1.365
 // and 1.242; 27B shape (8 layers) 2 rows 1.16 and 1.05, 3 rows 1.18 and 1.52, 8 rows 1.42 and 2.08, 16 rows 2.16 and 2.25.
+// From 9 rows on only where it has CTAs for the SMs: a long K over few row groups leaves them idle, and k_gemm_tc's clusters do
+// not.  CTAs here and there, us with it and without: 2560 x 10240 Q4_K 80, 120: 12 rows 19.4, 17.8, 16 rows 20.7, 18.0; on 16 rows
+// 3072 x 12288 Q4_0 96, 120: 21.1, 19.8, 1536 x 14336 Q4_0 96, 96: 17.2, 15.5, but 4096 x 14336 Q4_0 128, 128: 23.6, 24.3; on 12 rows
+// 3072 x 12288 Q4_0 17.1, 19.4, 1536 x 14336 Q4_0 14.8, 15.4.
 static bool takes_mma(int wtype, const GemvArgs& a, const uint8_t* t0, const uint8_t* t1, int policy) {
     const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU;
     if (!t0 || (pair && !t1) || policy != 1 || !gemm_mma_supports(wtype, a)) return false;
     const bool large = (double)a.N * a.K * 0.5625 * (pair ? 2 : 1) > 10.0e6 && !(a.epi == EPI_ARGMAX && a.K < 4096);
     if (large ? a.B < 3 : a.B < 5 || a.B > 8) return false;
+    if (a.B > 8 && large) {
+        const int ctas = gemm_mma_ctas(wtype, a), tiles = pair ? (a.N + 63) / 64 : (a.N + 127) / 128;
+        if (a.B > 12 && 3 * ctas <= 2 * g.sm_count) return false;
+        std::lock_guard<std::mutex> work(g_tc_lock);
+        int there = tiles < g.sm_count ? tiles : g.sm_count;
+        for (int s = 2; s <= 8 && a.epi != EPI_ARGMAX; ++s) if (tiles <= tc_clusters_at_once(s)) there = tiles * s;
+        if (10 * ctas < 7 * there) return false;
+    }
     return (size_t)(a.K / 32) * gm_block_bytes(wtype, gemm_mma_pad(a.B)) <= g_tc.img_cap && gemm_mma_pad(a.B) <= g_tc.inv_cap;
 }
 

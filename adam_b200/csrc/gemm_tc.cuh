@@ -34,6 +34,7 @@ __host__ __device__ constexpr int gm_block_bytes(int wtype, int rows) { return r
 struct GemmWork { const uint8_t* img; const float* inv; float* part; unsigned int* tickets; unsigned long long* best; unsigned int* ticket; };
 bool gemm_mma_supports(int wtype, const GemvArgs& a);
 int gemm_mma_pad(int rows);            // rows the image has room for
+int gemm_mma_ctas(int wtype, const GemvArgs& a);        // CTAs that a supported call is launched with
 int launch_gemm_mma(int wtype, const uint8_t* t0, const uint8_t* t1, const GemvArgs& a, const GemmWork& w, cudaStream_t stream);
 
 }  // namespace ab

@@ -41,6 +41,20 @@ def test_few_rows(gpu, ggml_type, N, K, B, mean):
     assert e.max() < 5e-7 and gpu.device_error() == 0
 
 
+@pytest.mark.parametrize("ggml_type,N,K,B,few", [(2, 2560, 10240, 8, True), (2, 2560, 10240, 12, False), (12, 2560, 10240, 9, False), (2, 3072, 12288, 12, True), (2, 3072, 12288, 13, False),
+                                                  (12, 1536, 14336, 16, False), (2, 4096, 14336, 16, True), (12, 21504, 5376, 16, True)])
+def test_long_products_of_few_row_groups(gpu, ggml_type, N, K, B, few):
+    """From 9 rows on the tcgen05 GEMM keeps products whose row groups leave SMs idle here; error as in test_few_rows and test_gemm_tiles."""
+    rng = np.random.default_rng(N + K + B)
+    raw = {2: gb.random_q4_0_blocks, 12: gb.random_q4_k_blocks}[ggml_type](rng, N, K)
+    x = rng.standard_normal((B, K), dtype=np.float32)
+    before = gpu.gemm_counts()
+    e = _error(gpu, ggml_type, raw, N, K, x, 1)
+    after = gpu.gemm_counts()
+    assert after["few"] == before["few"] + few and after["tile_16"] == before["tile_16"] + (not few)
+    assert e.max() < (5e-7 if few else 5e-6) and gpu.device_error() == 0
+
+
 def _model(gpu, cfg, batch, policy, prompts, ggml_type=gb.GGML_TYPE_Q4_0):
     from adam_b200 import synth
     from adam_b200.config import GenerationConfig
