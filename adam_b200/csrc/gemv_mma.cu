@@ -1,5 +1,6 @@
 // Host-side launch logic of the tensor-core Q4_0 GEMV (kernel in gemv_mma.cuh).
 #include "gemv_mma.cuh"
+#include "gemv_row.cuh"
 
 #include <cstdio>
 #include <cstdlib>
@@ -45,6 +46,7 @@ int launch_gemv_mma(int wt, const uint8_t* t0, const uint8_t* t1, GemvArgs a, cu
     if (!gemv_mma_supports(wt, a)) return fail(ADAMAH_ERR_INVALID, "gemv_mma: shape not supported");
     const bool pair = (a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU);
     if (pair && !t1) return fail(ADAMAH_ERR_INVALID, "gemv_mma: second matrix missing");
+    if (gemv_row_takes(wt, a)) return launch_gemv_row(wt, t0, t1, a, stream);
     const int units = a.K / 32, pairs = a.K / 64, n_rg = a.N / 16;
     // batch rows per pass: as many of 4, 2, 1 as shared memory allows
     // Batch rows per pass.  The passes of a launch run side by side (gridDim.x), each re-reading the weights from L2.

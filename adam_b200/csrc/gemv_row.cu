@@ -1,0 +1,74 @@
+// Host-side launch logic of the one-row GEMV (kernel in gemv_row.cuh).
+#include "gemv_row.cuh"
+
+namespace ab {
+
+typedef void (*RowKernel)(const GemvArgs, const uint8_t*, const uint8_t*, float);
+struct RowShape { RowKernel k; int ks; size_t smem; };
+
+// Two tile pairs per warp: its 32 lanes hold one float4 of activations each, the shortest chain there is.  Up to 10 such slices
+// (K <= 1280) a CTA is small enough for three per SM, which is what a matrix of 450 row groups needs to be resident; longer
+// rows have one CTA per SM of up to 32 warps, and four pairs per warp beyond K = 4096.
+constexpr int ROW_THREADS = 320, ROW_CTAS = 3;
+
+template <int WT>
+static RowShape row_shape(const GemvArgs& a) {
+    const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU, chain = a.h_in != nullptr;
+    const int pairs = a.K >> 6;
+    RowShape s = {};
+    int ppw = 2;
+    s.ks = (pairs + 1) / 2;
+    if (s.ks * 32 <= ROW_THREADS) {
+        s.k = pair ? (chain ? k_gemv_row<true, WT, true, 2, ROW_THREADS, ROW_CTAS> : k_gemv_row<true, WT, false, 2, ROW_THREADS, ROW_CTAS>)
+                   : (chain ? k_gemv_row<false, WT, true, 2, ROW_THREADS, ROW_CTAS> : k_gemv_row<false, WT, false, 2, ROW_THREADS, ROW_CTAS>);
+    } else if (pair) {
+        return RowShape{};
+    } else if (s.ks <= ROW_MAX_WARPS) {
+        s.k = chain ? k_gemv_row<false, WT, true, 2, 1024, 1> : k_gemv_row<false, WT, false, 2, 1024, 1>;
+    } else {
+        ppw = 4;
+        s.ks = (pairs + 3) / 4;
+        if (chain || s.ks > ROW_MAX_WARPS) return RowShape{};
+        s.k = k_gemv_row<false, WT, false, 4, 1024, 1>;
+    }
+    s.smem = (size_t)s.ks * ppw * 256;
+    return s;
+}
+
+static bool row_shape_for(int wt, const GemvArgs& a, RowShape* out) {
+    if (a.N <= 0 || a.K <= 0 || a.B != 1 || a.N % 16 || a.K % 64 || a.epi == EPI_ARGMAX) return false;
+    if (wt != WT_Q4_0 && (wt != WT_Q4_K || a.K % 256)) return false;
+    const void* x = a.h_in ? (const void*)a.h_in : (const void*)a.x;
+    if (((uintptr_t)x & 15) || (a.ldx & 3)) return false;
+    const RowShape s = wt == WT_Q4_0 ? row_shape<WT_Q4_0>(a) : row_shape<WT_Q4_K>(a);
+    if (!s.k) return false;
+    // Every CTA resident at once: a second wave would request its weights only when the first is done, which is what the rings
+    // of k_gemv_mma are for.  (The occupancies asked for are kept: a step asks for the same few shapes.)
+    struct Known { RowKernel k; int ks, per_sm; };
+    static thread_local Known known[32]; static thread_local int n_known = 0;
+    int per_sm = -1;
+    for (int i = 0; i < n_known; ++i) if (known[i].k == s.k && known[i].ks == s.ks) per_sm = known[i].per_sm;
+    if (per_sm < 0) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, s.k, s.ks * 32, s.smem) != cudaSuccess) { cudaGetLastError(); return false; }
+        if (n_known < 32) known[n_known++] = Known{s.k, s.ks, per_sm};
+    }
+    if ((long long)(a.N / 16) > (long long)per_sm * g.sm_count) return false;
+    *out = s;
+    return true;
+}
+
+bool gemv_row_takes(int wt, const GemvArgs& a) {
+    RowShape s;
+    return row_shape_for(wt, a, &s);
+}
+
+int launch_gemv_row(int wt, const uint8_t* t0, const uint8_t* t1, GemvArgs a, cudaStream_t stream) {
+    RowShape s;
+    if (!row_shape_for(wt, a, &s)) return fail(ADAMAH_ERR_INVALID, "gemv_row: shape not supported");
+    if (launch_k(s.k, dim3(a.N / 16, a.B), dim3(s.ks * 32), s.smem, stream, g.pdl, a, t0, t1, 1.0f / (float)a.K) != cudaSuccess)
+        return fail(ADAMAH_ERR_BACKEND, "gemv_row: launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+    count_launch();
+    return ADAMAH_OK;
+}
+
+}  // namespace ab

@@ -1,0 +1,279 @@
+// Dequant GEMV for one activation row and a matrix that fits the registers of all SMs at once.
+//
+// One token of one sequence is a chain of products of a few megabytes each, and what such a product takes is not its
+// bytes but the chain of latencies from "the previous kernel is done" to "the last row is stored": the activations' trip
+// through L2, the reductions of the norm chain, the split into bytes, a few MMAs, the sum over K slices.  This kernel
+// keeps that chain as short as it gets; k_gemv_mma (gemv_mma.cuh), whose warps share one staged copy of the activations
+// behind three CTA-wide reductions, is for matrices that have to be streamed.
+//   * A CTA is one group of 16 rows, its warps are the K slices: PPW tile pairs (64 weights each) per warp.  All CTAs are
+//     resident together, so a warp holds its whole share of the matrix in registers, requested ahead of the dependency
+//     wait: no ring, no stage barriers, no loop.
+//   * A warp stages only the 64 * PPW activations that it multiplies, with a power-of-two scale of its own: no CTA-wide
+//     maximum, no CTA barrier between staging and product.  (Its integers are relative to the slice's largest value, so
+//     they are never coarser than those of one scale for the vector.)
+//   * Of the input chain only the branch's RMS is needed ahead of the product.  1 / rms of the stream is a factor of the
+//     whole result and its sum of squares meets the K slices' sums at the one barrier that adds them.
+//   * Q4_0 codes enter the MMA as signed bytes 16 (q - 8): a nibble in a byte's upper half, its top bit flipped, IS that
+//     byte, so nothing is subtracted per block.  (Q4_K: unsigned 16 q, its offsets take the block's activation sums.)
+// Measured on a B200 at the 1B shape (Q4_0), from the end of the dependency wait to the last store, k_gemv_mma -> here: QKV
+// 1536 x 1152 3.3 -> 1.5 us, o-proj 1152 x 1024 2.3 -> 0.9, gate / up 2 x 6912 x 1152 4.1 -> 2.3, down 1152 x 6912 4.5 -> 1.9;
+// a step 0.656 -> 0.450 ms (kernels that stamp their phases).  Relative error of a product 2.8e-7 to 3.3e-7 (N(0, 1)
+// activations; before the same), 5.5e-7 to 8.1e-7 where they have heavy tails (before 8.1e-7 to 2.0e-6).
+// The arithmetic otherwise is that of k_gemv_mma: |x s| <= 2^22, three signed bytes per activation, mma.m16n8k32 in
+// integers, block scale and sums in fp32.
+#pragma once
+#include "gemv_mma.cuh"
+
+namespace ab {
+
+// Shared memory of a warp's slice: per unit of 32 activations four columns (hi, mid, lo, zero) of 32 bytes; column c of
+// unit u stands at place c ^ (u & 3), so that the four units a warp stores at once fall on different banks.
+constexpr int ROW_MAX_WARPS = 32;
+constexpr int ROW_RED_LD = 36;              // floats per row of the K slices' sums: 16-byte rows on different banks
+
+__device__ __forceinline__ void imma16832_s(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0), "r"(0), "r"(0), "r"(0));
+}
+
+__device__ __forceinline__ uint4 ld_weight(const uint8_t* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint2 ld_weight2(const uint8_t* p) {
+    uint2 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+
+// 1 / sqrt(v), the library's approximation and one step of Newton's iteration.
+__device__ __forceinline__ float rsqrt_newton(float v) {
+    const float r = rsqrtf(v);
+    return fmaf(0.5f * r, fmaf(-v * r, r, 1.0f), r);
+}
+
+// The first `n` (<= 32) floats of a 16-byte aligned row whose last group of four is filled up with zeros.
+__device__ __forceinline__ float row_total(const float* p, int n) {
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+    for (int i = 0; i < ROW_MAX_WARPS / 4; ++i) {
+        if (4 * i < n) {
+            const float4 v = reinterpret_cast<const float4*>(p)[i];
+            s0 += v.x; s1 += v.y; s2 += v.z; s3 += v.w;
+        }
+    }
+    return (s0 + s1) + (s2 + s3);
+}
+
+#ifdef ADAM_B200_STEP_TRACE
+#define GR_STAMP(slot) do { if (threadIdx.x == 0 && blockIdx.x < 8 && blockIdx.y == 0) STEP_STAMP(a.trace, blockIdx.x * 8 + (slot)); } while (0)
+#else
+#define GR_STAMP(slot) do { } while (0)
+#endif
+
+// grid (row groups, activation rows), 32 * K slices threads; PPW: tile pairs per warp at most; THREADS, CTAS: the launch bounds.
+template <bool PAIR, int WT, bool CHAIN, int PPW, int THREADS, int CTAS>
+__global__ void __launch_bounds__(THREADS, CTAS) k_gemv_row(const GemvArgs a, const uint8_t* __restrict__ t0, const uint8_t* __restrict__ t1, float inv_k) {
+    GR_STAMP(0);
+    constexpr int NM = PAIR ? 2 : 1, NV = PPW / 2, UNITS = 2 * PPW, TILE = MmaGeo<PAIR, WT>::TILE;
+    static_assert(PPW % 2 == 0, "a warp's 32 lanes load two tile pairs' activations at a time");
+    extern __shared__ __align__(16) unsigned char smem_raw[];               // per warp: UNITS * 128 bytes
+    __shared__ __align__(16) float s_red[NM][16][ROW_RED_LD];
+    __shared__ __align__(16) float s_part[2][ROW_MAX_WARPS];                // the slices' sums of squares: branch, stream
+    __shared__ float s_sx[WT == WT_Q4_K ? ROW_MAX_WARPS * UNITS * 2 : 1];   // Q4_K: activation sums of the units, in the lanes' units
+    const int lane = threadIdx.x & 31, ks = threadIdx.x >> 5, KS = blockDim.x >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int rg = blockIdx.x, b = blockIdx.y;
+    const int pairs = a.K >> 6;
+    const int p0 = ks * pairs / KS, np = (ks + 1) * pairs / KS - p0;
+
+    // ---- ahead of the dependency wait: weights, norm weights, what stays constant in shared memory ----
+    uint4 q[NM][PPW];
+    uint2 sc[NM][PPW], hd[NM][PPW];
+#pragma unroll
+    for (int i = 0; i < PPW; ++i) {
+#pragma unroll
+        for (int m = 0; m < NM; ++m) {
+            const uint8_t* tile = (m ? t1 : t0) + ((size_t)rg * pairs + p0 + i) * TILE;
+            const bool in = i < np;
+            q[m][i] = in ? ld_weight(tile + lane * 16) : make_uint4(0u, 0u, 0u, 0u);
+            sc[m][i] = in ? ld_weight2(tile + 512 + g * 8) : make_uint2(0u, 0u);      // no pair: scale 0, whatever its bytes and activations
+            if (WT == WT_Q4_K) hd[m][i] = in ? ld_weight2(tile + 576 + g * 8) : make_uint2(0u, 0u);
+        }
+    }
+    float4 vp[NV], vw[NV];
+    const int f0 = p0 * 16;                                                 // the slice's first float4
+    if (CHAIN) {
+        const float4 o4 = make_float4(1.f, 1.f, 1.f, 1.f);
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int f = lane + 32 * j;
+            vp[j] = (f < np * 16 && a.add_src && a.w_post) ? reinterpret_cast<const float4*>(a.w_post)[f0 + f] : o4;
+            vw[j] = (f < np * 16 && a.w_pre) ? reinterpret_cast<const float4*>(a.w_pre)[f0 + f] : o4;
+        }
+    }
+    unsigned char* xb = smem_raw + ks * (UNITS * 128);
+    for (int i = lane; i < UNITS * 8; i += 32) {                            // the zero column
+        const int u = i >> 3;
+        reinterpret_cast<uint32_t*>(xb + u * 128 + ((3 ^ (u & 3)) * 32))[i & 7] = 0u;
+    }
+    const int ks4 = (KS + 3) & ~3;                                          // sums are read four at a time: zeros behind the last slice's
+    if (ks == 0) {
+        for (int k = KS; k < ks4; ++k) {
+            if (lane < 16) {
+#pragma unroll
+                for (int m = 0; m < NM; ++m) s_red[m][lane][k] = 0.f;
+            }
+            if (lane < 2) s_part[lane][k] = 0.f;
+        }
+    }
+    GR_STAMP(1);
+    pdl_launch_dependents();
+    pdl_wait();
+    GR_STAMP(2);
+
+    // ---- this warp's activations ----
+    float4 x[NV];
+    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (CHAIN) {
+        const float4* hp = reinterpret_cast<const float4*>(a.h_in + (size_t)b * a.ldx) + f0;
+        const float4* ap = a.add_src ? reinterpret_cast<const float4*>(a.add_src + (size_t)b * a.ldx) + f0 : nullptr;
+        float4 va[NV];
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int f = lane + 32 * j;
+            x[j] = f < np * 16 ? hp[f] : z4;
+            va[j] = (ap && f < np * 16) ? ap[f] : z4;
+        }
+        float ra = 1.f;
+        if (ap && a.w_post) {
+            float s = 0.f;
+#pragma unroll
+            for (int j = 0; j < NV; ++j) s += fmaf(va[j].x, va[j].x, va[j].y * va[j].y) + fmaf(va[j].z, va[j].z, va[j].w * va[j].w);
+            s = warp_sum(s);
+            if (lane == 0) s_part[0][ks] = s;
+            __syncthreads();
+            ra = rsqrt_newton(fmaf(row_total(s_part[0], KS), inv_k, a.eps));
+        }
+        GR_STAMP(5);
+        float s = 0.f;
+        if (ap) {
+#pragma unroll
+            for (int j = 0; j < NV; ++j) {
+                x[j].x = fmaf(va[j].x * ra, vp[j].x, x[j].x); x[j].y = fmaf(va[j].y * ra, vp[j].y, x[j].y);
+                x[j].z = fmaf(va[j].z * ra, vp[j].z, x[j].z); x[j].w = fmaf(va[j].w * ra, vp[j].w, x[j].w);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int f = lane + 32 * j;
+            if (a.h_out && rg == 0 && f < np * 16) reinterpret_cast<float4*>(a.h_out + (size_t)b * a.ldx)[f0 + f] = x[j];
+            s += fmaf(x[j].x, x[j].x, x[j].y * x[j].y) + fmaf(x[j].z, x[j].z, x[j].w * x[j].w);
+            x[j].x *= vw[j].x; x[j].y *= vw[j].y; x[j].z *= vw[j].z; x[j].w *= vw[j].w;
+        }
+        if (a.w_pre) {
+            s = warp_sum(s);
+            if (lane == 0) s_part[1][ks] = s;
+        }
+    } else {
+        const float4* xp = reinterpret_cast<const float4*>(a.x + (size_t)b * a.ldx) + f0;
+#pragma unroll
+        for (int j = 0; j < NV; ++j) { const int f = lane + 32 * j; x[j] = f < np * 16 ? xp[f] : z4; }
+    }
+    float am = 0.f, scale, inv;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) am = fmaxf(am, fmaxf(fmaxf(fabsf(x[j].x), fabsf(x[j].y)), fmaxf(fabsf(x[j].z), fabsf(x[j].w))));
+    am = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(am)));        // not negative: the bits are in the values' order
+    pow2_scale(am, scale, inv);
+    GR_STAMP(6);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int f = lane + 32 * j, u = f >> 3;
+        const float v[4] = {x[j].x * scale, x[j].y * scale, x[j].z * scale, x[j].w * scale};
+        uint32_t wh, wm, wl;
+        split_x4(v, true, wh, wm, wl);
+        unsigned char* p = xb + u * 128 + (f & 3) * 8 + ((f >> 2) & 1) * 4;
+        *reinterpret_cast<uint32_t*>(p + ((0 ^ (u & 3)) * 32)) = wh;
+        *reinterpret_cast<uint32_t*>(p + ((1 ^ (u & 3)) * 32)) = wm;
+        *reinterpret_cast<uint32_t*>(p + ((2 ^ (u & 3)) * 32)) = wl;
+        if (WT == WT_Q4_K) {
+            int sh = __dp4a((int)wh, 0x01010101, 0), sm = __dp4a((int)wm, 0x01010101, 0), sl = __dp4a((int)wl, 0x01010101, 0);
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                sh += __shfl_xor_sync(0xffffffffu, sh, o);
+                sm += __shfl_xor_sync(0xffffffffu, sm, o);
+                sl += __shfl_xor_sync(0xffffffffu, sl, o);
+            }
+            if ((lane & 7) == 0)
+                *reinterpret_cast<float2*>(s_sx + (ks * UNITS + u) * 2) = make_float2(-16.f * (float)(sh * 256 + sm), -16.f * (float)(sl * 256));
+        }
+    }
+    __syncwarp();
+    GR_STAMP(3);
+
+    // ---- products ----
+    float acc[NM][2];
+#pragma unroll
+    for (int m = 0; m < NM; ++m) acc[m][0] = acc[m][1] = 0.f;
+    const int c = g & 3;                                                    // lanes g >= 4 fill columns that nobody reads
+#pragma unroll
+    for (int i = 0; i < PPW; ++i) {
+#pragma unroll
+        for (int blk = 0; blk < 2; ++blk) {
+            const int u = 2 * i + blk;
+            const uint2 bx = *reinterpret_cast<const uint2*>(xb + u * 128 + (c ^ (u & 3)) * 32 + t * 8);
+#pragma unroll
+            for (int m = 0; m < NM; ++m) {
+                const uint32_t w0 = blk ? q[m][i].z : q[m][i].x, w1 = blk ? q[m][i].w : q[m][i].y, s2 = blk ? sc[m][i].y : sc[m][i].x;
+                int dd[4];
+                if constexpr (WT == WT_Q4_0) {
+                    const uint32_t M = 0xF0F0F0F0u, X = 0x80808080u;
+                    imma16832_s(dd, ((w0 << 4) & M) ^ X, ((w1 << 4) & M) ^ X, (w0 & M) ^ X, (w1 & M) ^ X, bx.x, bx.y);
+                    const float2 d = __half22float2(*reinterpret_cast<const __half2*>(&s2));
+                    acc[m][0] = fmaf(d.x, (float)(dd[0] * 256 + dd[1]), acc[m][0]);
+                    acc[m][1] = fmaf(d.y, (float)(dd[2] * 256 + dd[3]), acc[m][1]);
+                } else {
+                    const uint32_t M = 0xF0F0F0F0u;
+                    imma16832(dd, (w0 << 4) & M, (w1 << 4) & M, w0 & M, w1 & M, bx.x, bx.y);
+                    const float2 dm0 = __half22float2(*reinterpret_cast<const __half2*>(&hd[m][i].x)), dm1 = __half22float2(*reinterpret_cast<const __half2*>(&hd[m][i].y));
+                    const float es0 = dm0.x * (float)(s2 & 0xFFu), em0 = dm0.y * (float)((s2 >> 8) & 0xFFu);
+                    const float es1 = dm1.x * (float)((s2 >> 16) & 0xFFu), em1 = dm1.y * (float)(s2 >> 24);
+                    const float sx = s_sx[(ks * UNITS + u) * 2 + (t & 1)];
+                    acc[m][0] = fmaf(es0, (float)(dd[0] * 256 + dd[1]), fmaf(em0, sx, acc[m][0]));
+                    acc[m][1] = fmaf(es1, (float)(dd[2] * 256 + dd[3]), fmaf(em1, sx, acc[m][1]));
+                }
+            }
+        }
+    }
+    // Even lanes hold 16 (256 hi + mid), odd ones 16 * 256 lo: times 65536 / 256 / 16 and 1 / 256 / 16, both exact.
+    const float cm = ((t & 1) ? 1.0f / 4096.0f : 16.0f) * inv;
+#pragma unroll
+    for (int m = 0; m < NM; ++m) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float v = acc[m][h] * cm;
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            if (t == 0) s_red[m][g + 8 * h][ks] = v;
+        }
+    }
+    __syncthreads();
+    // ---- the slices' sums: lane = row (and matrix) ----
+    if (ks == 0) {
+        float v = row_total(s_red[PAIR ? lane >> 4 : 0][lane & 15], KS);
+        if (CHAIN && a.w_pre) v *= rsqrt_newton(fmaf(row_total(s_part[1], KS), inv_k, a.eps));
+        const float up = PAIR ? __shfl_down_sync(0xffffffffu, v, 16) : 0.f;
+        if (lane < 16) {
+            const float r = !PAIR ? v : (a.epi == EPI_GEGLU ? gelu_tanh(v) : silu_clip(v)) * up;
+            a.y[(size_t)b * a.ldy + rg * 16 + lane] = r;
+        }
+    }
+    GR_STAMP(4);
+}
+
+// ADAMAH_ERR_INVALID where gemv_row_takes() says no.
+bool gemv_row_takes(int wtype, const GemvArgs& a);
+int launch_gemv_row(int wtype, const uint8_t* t0, const uint8_t* t1, GemvArgs a, cudaStream_t stream);
+
+}  // namespace ab

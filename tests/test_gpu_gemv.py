@@ -170,6 +170,26 @@ def test_q4_k_gemv_tensor_core_path(gpu, N, K, B):
     assert np.abs(y - y0).max() < 1e-4 * np.abs(y0).max()
 
 
+@pytest.mark.parametrize("ggml_type,N,K", [
+    (2, 16, 64), (2, 32, 192), (2, 7104, 1152), (2, 7120, 1152),       # one slice; a slice of one pair; the most CTAs of 10 slices, one more
+    (2, 48, 1280), (2, 48, 1344), (2, 160, 4096), (2, 160, 4160),      # 10 and 11 slices; 32; slices of up to four pairs
+    (2, 96, 8192), (2, 2368, 6912), (2, 2384, 6912), (2, 96, 8256),    # 32 of four; one CTA per SM and one more; too long
+    (12, 16, 256), (12, 2048, 1280), (12, 48, 1536), (12, 80, 4352), (12, 80, 8192)])
+def test_one_row_gemv_edges(gpu, ggml_type, N, K):
+    """Products of one row whose matrix fits the registers (one warp per K slice), at the edges of what takes them.  A slice's
+    activations are rounded to 23 bits of its own largest value, sums are fp32: 1e-6 of the result's 2-norm for activations
+    whose slices differ by factors of up to 1e6."""
+    rng = np.random.default_rng(N + K)
+    raw = (gb.random_q4_0_blocks if ggml_type == 2 else gb.random_q4_k_blocks)(rng, N, K)
+    x = rng.standard_normal((1, K)).astype(np.float32)
+    W = q4_blocks.dequant(raw.reshape(-1), ggml_type, N, K).astype(np.float64)
+    for scale in (np.ones(K), 10.0 ** rng.integers(-3, 4, K // 64).repeat(64), np.zeros(K)):
+        xs = (x * scale).astype(np.float32)
+        y = _gemv(gpu, ggml_type, raw, N, K, xs, tile=True)
+        ref = xs.astype(np.float64) @ W.T
+        assert np.linalg.norm(y - ref) <= 1e-6 * np.linalg.norm(xs) * np.linalg.norm(W) / np.sqrt(K) * 4
+
+
 @pytest.mark.parametrize("N,K", [(5376, 5376), (512, 21504), (2048, 4096), (3, 256), (9, 768), (64, 1024)])
 def test_q4_k_gemv(gpu, N, K):
     rng = np.random.default_rng(N * 17 + K)
