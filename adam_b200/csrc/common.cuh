@@ -104,6 +104,17 @@ inline cudaError_t launch_k(void (*k)(KArgs...), dim3 grid, dim3 block, size_t s
     return cudaLaunchKernelEx(&cfg, k, KArgs(args)...);
 }
 
+// Shared-memory settings of a kernel of a decode step: its limit, and all of an SM's shared memory whatever it asks for itself.  An
+// SM changes its split between L1 and shared memory only when it is empty, so a kernel whose own choice differs from that of
+// the kernel before it cannot start beside it.
+inline bool carveout_max(const void* k, int smem_limit) {
+    if ((smem_limit > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_limit) != cudaSuccess) ||
+        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return true;
+}
 
 // The same with the CTAs of a launch grouped into thread-block clusters of `cluster_x` along x (gridDim.x a multiple of it).
 template <typename... KArgs, typename... Args>
@@ -197,6 +208,11 @@ __device__ __forceinline__ float rcp_newton(float d) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return fmaf(r, fmaf(-d, r, 1.0f), r);
+}
+// 1 / sqrt(v), the library's approximation and one step of Newton's iteration.
+__device__ __forceinline__ float rsqrt_newton(float v) {
+    const float r = rsqrtf(v);
+    return fmaf(0.5f * r, fmaf(-v * r, r, 1.0f), r);
 }
 // x / (1 + e^-z), without branches.  Below z = -80 it is x * 0 (the true factor, e^-80 and less, is nothing beside any other
 // term, and 1 + tanh is 0 there), which is NaN for an infinite x; an infinite x elsewhere keeps its sign, which div_by would lose.

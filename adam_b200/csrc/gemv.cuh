@@ -75,6 +75,8 @@ struct GemvArgs {
     float softcap;                  // applied to stored logits only (monotone)
     int max_grid;                   // 0 = launcher's choice; otherwise an upper bound on the CTAs launched
     uint32_t* err;                  // device error word (set by launch_gemv_mma)
+    // matrices that later kernels of the step read (16-byte aligned; NULL = none): the one-row kernel asks L2 for them
+    const uint8_t* pf[3]; uint32_t pf_bytes[3], pf_part[3];      // pf_part: a warp's share (set by the launcher)
 #ifdef ADAM_B200_STEP_TRACE
     long long* trace;               // 8 stamps per CTA for the first 8 CTAs of the first batch group (NULL = off)
 #endif

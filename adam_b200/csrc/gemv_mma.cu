@@ -79,7 +79,7 @@ int launch_gemv_mma(int wt, const uint8_t* t0, const uint8_t* t1, GemvArgs a, cu
         MmaKernel k = wt == WT_Q4_0 ? pick_kernel<WT_Q4_0>(vi, pair) : pick_kernel<WT_Q4_K>(vi, pair);
         MmaInfo& ki = g_mma_info[wt == WT_Q4_0 ? 0 : 1][vi][pair ? 1 : 0];
         if (!ki.attr) {
-            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM_LIMIT) != cudaSuccess)
+            if (!carveout_max((const void*)k, MMA_SMEM_LIMIT))
                 return fail(ADAMAH_ERR_BACKEND, "gemv_mma: cannot raise the shared-memory limit");
             ki.attr = true;
         }
@@ -155,7 +155,7 @@ int launch_gemv_mma(int wt, const uint8_t* t0, const uint8_t* t1, GemvArgs a, cu
             k = wt == WT_Q4_0 ? (MmaKernel)k_gemv_mma<4, false, WT_Q4_0, 2> : (MmaKernel)k_gemv_mma<4, false, WT_Q4_K, 2>;
             static bool attr2[2];
             if (!attr2[wt == WT_Q4_0 ? 0 : 1]) {
-                if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM_LIMIT_LONG) != cudaSuccess)
+                if (!carveout_max((const void*)k, MMA_SMEM_LIMIT_LONG))
                     return fail(ADAMAH_ERR_BACKEND, "gemv_mma: cannot raise the shared-memory limit");
                 attr2[wt == WT_Q4_0 ? 0 : 1] = true;
             }

@@ -6,11 +6,10 @@ namespace ab {
 typedef void (*RowKernel)(const GemvArgs, const uint8_t*, const uint8_t*, float);
 struct RowShape { RowKernel k; int ks; size_t smem; };
 
-// Two tile pairs per warp: its 32 lanes hold one float4 of activations each, the shortest chain there is.  Up to 10 such slices
-// (K <= 1280) a CTA is small enough for three per SM, which is what a matrix of 450 row groups needs to be resident; longer
-// rows have one CTA per SM of up to 32 warps, and four pairs per warp beyond K = 4096.
-constexpr int ROW_THREADS = 320, ROW_CTAS = 3;
-
+// Two tile pairs per warp: its 32 lanes hold one float4 of activations each, the shortest chain there is (K <= 4096); four for
+// longer rows.  Up to nine slices (K <= 1152) a thread keeps to 56 registers: three such CTAs, what a matrix of 400 row groups
+// needs of every SM, then leave room in each quarter of the register file for the kernels ahead of them, and all start in time.
+constexpr int ROW_THREADS = 288, ROW_CTAS = 4;
 template <int WT>
 static RowShape row_shape(const GemvArgs& a) {
     const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU, chain = a.h_in != nullptr;
@@ -21,14 +20,13 @@ static RowShape row_shape(const GemvArgs& a) {
     if (s.ks * 32 <= ROW_THREADS) {
         s.k = pair ? (chain ? k_gemv_row<true, WT, true, 2, ROW_THREADS, ROW_CTAS> : k_gemv_row<true, WT, false, 2, ROW_THREADS, ROW_CTAS>)
                    : (chain ? k_gemv_row<false, WT, true, 2, ROW_THREADS, ROW_CTAS> : k_gemv_row<false, WT, false, 2, ROW_THREADS, ROW_CTAS>);
-    } else if (pair) {
-        return RowShape{};
     } else if (s.ks <= ROW_MAX_WARPS) {
-        s.k = chain ? k_gemv_row<false, WT, true, 2, 1024, 1> : k_gemv_row<false, WT, false, 2, 1024, 1>;
+        s.k = pair ? (chain ? k_gemv_row<true, WT, true, 2, 1024, 1> : k_gemv_row<true, WT, false, 2, 1024, 1>)
+                   : (chain ? k_gemv_row<false, WT, true, 2, 1024, 1> : k_gemv_row<false, WT, false, 2, 1024, 1>);
     } else {
         ppw = 4;
         s.ks = (pairs + 3) / 4;
-        if (chain || s.ks > ROW_MAX_WARPS) return RowShape{};
+        if (pair || chain || s.ks > ROW_MAX_WARPS) return RowShape{};
         s.k = k_gemv_row<false, WT, false, 4, 1024, 1>;
     }
     s.smem = (size_t)s.ks * ppw * 256;
@@ -49,7 +47,8 @@ static bool row_shape_for(int wt, const GemvArgs& a, RowShape* out) {
     int per_sm = -1;
     for (int i = 0; i < n_known; ++i) if (known[i].k == s.k && known[i].ks == s.ks) per_sm = known[i].per_sm;
     if (per_sm < 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, s.k, s.ks * 32, s.smem) != cudaSuccess) { cudaGetLastError(); return false; }
+        if (!carveout_max((const void*)s.k, 0) ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, s.k, s.ks * 32, s.smem) != cudaSuccess) { cudaGetLastError(); return false; }
         if (n_known < 32) known[n_known++] = Known{s.k, s.ks, per_sm};
     }
     if ((long long)(a.N / 16) > (long long)per_sm * g.sm_count) return false;
@@ -65,6 +64,11 @@ bool gemv_row_takes(int wt, const GemvArgs& a) {
 int launch_gemv_row(int wt, const uint8_t* t0, const uint8_t* t1, GemvArgs a, cudaStream_t stream) {
     RowShape s;
     if (!row_shape_for(wt, a, &s)) return fail(ADAMAH_ERR_INVALID, "gemv_row: shape not supported");
+    const uint32_t n_w = (uint32_t)(a.N / 16 * s.ks);
+    for (int r = 0; r < 3; ++r) {
+        if (!a.pf[r]) a.pf_bytes[r] = 0;
+        a.pf_part[r] = (a.pf_bytes[r] / n_w + 127u) & ~127u;
+    }
     if (launch_k(s.k, dim3(a.N / 16, a.B), dim3(s.ks * 32), s.smem, stream, g.pdl, a, t0, t1, 1.0f / (float)a.K) != cudaSuccess)
         return fail(ADAMAH_ERR_BACKEND, "gemv_row: launch failed: %s", cudaGetErrorString(cudaGetLastError()));
     count_launch();

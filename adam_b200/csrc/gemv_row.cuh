@@ -16,9 +16,11 @@
 //   * Q4_0 codes enter the MMA as signed bytes 16 (q - 8): a nibble in a byte's upper half, its top bit flipped, IS that
 //     byte, so nothing is subtracted per block.  (Q4_K: unsigned 16 q, its offsets take the block's activation sums.)
 // Measured on a B200 at the 1B shape (Q4_0), from the end of the dependency wait to the last store, k_gemv_mma -> here: QKV
-// 1536 x 1152 3.3 -> 1.5 us, o-proj 1152 x 1024 2.3 -> 0.9, gate / up 2 x 6912 x 1152 4.1 -> 2.3, down 1152 x 6912 4.5 -> 1.9;
-// a step 0.656 -> 0.450 ms (kernels that stamp their phases).  Relative error of a product 2.8e-7 to 3.3e-7 (N(0, 1)
-// activations; before the same), 5.5e-7 to 8.1e-7 where they have heavy tails (before 8.1e-7 to 2.0e-6).
+// 1536 x 1152 3.3 -> 1.6 us, o-proj 1152 x 1024 2.3 -> 0.9, gate / up 2 x 6912 x 1152 4.1 -> 2.1, down 1152 x 6912 4.5 -> 1.7.
+// Relative error of a product 2.8e-7 to 3.3e-7 (N(0, 1) activations; before the same), 5.5e-7 to 8.1e-7 where they have heavy
+// tails (before 8.1e-7 to 2.0e-6).  Tried and not kept: weights in shared memory by bulk copy (+0.3 us per product, an SM takes
+// four CTAs of the gate / up product and another two), three row groups per CTA behind one staging (all 27 warps of an SM in
+// step: products 0.75 -> 1.25 us), the code run once on nothing ahead of the wait (the same times: it is in the instruction cache).
 // The arithmetic otherwise is that of k_gemv_mma: |x s| <= 2^22, three signed bytes per activation, mma.m16n8k32 in
 // integers, block scale and sums in fp32.
 #pragma once
@@ -26,10 +28,7 @@
 
 namespace ab {
 
-// Shared memory of a warp's slice: per unit of 32 activations four columns (hi, mid, lo, zero) of 32 bytes; column c of
-// unit u stands at place c ^ (u & 3), so that the four units a warp stores at once fall on different banks.
 constexpr int ROW_MAX_WARPS = 32;
-constexpr int ROW_RED_LD = 36;              // floats per row of the K slices' sums: 16-byte rows on different banks
 
 __device__ __forceinline__ void imma16832_s(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
@@ -48,156 +47,175 @@ __device__ __forceinline__ uint2 ld_weight2(const uint8_t* p) {
     return v;
 }
 
-// 1 / sqrt(v), the library's approximation and one step of Newton's iteration.
-__device__ __forceinline__ float rsqrt_newton(float v) {
-    const float r = rsqrtf(v);
-    return fmaf(0.5f * r, fmaf(-v * r, r, 1.0f), r);
-}
-
-// The first `n` (<= 32) floats of a 16-byte aligned row whose last group of four is filled up with zeros.
-__device__ __forceinline__ float row_total(const float* p, int n) {
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+// The sum of NG groups of four floats at a 16-byte aligned place.
+template <int NG>
+__device__ __forceinline__ float row_total(const float* p) {
+    float4 t = reinterpret_cast<const float4*>(p)[0];
 #pragma unroll
-    for (int i = 0; i < ROW_MAX_WARPS / 4; ++i) {
-        if (4 * i < n) {
-            const float4 v = reinterpret_cast<const float4*>(p)[i];
-            s0 += v.x; s1 += v.y; s2 += v.z; s3 += v.w;
-        }
+    for (int i = 1; i < NG; ++i) {
+        const float4 v = reinterpret_cast<const float4*>(p)[i];
+        t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
     }
-    return (s0 + s1) + (s2 + s3);
+    return (t.x + t.y) + (t.z + t.w);
 }
 
 #ifdef ADAM_B200_STEP_TRACE
-#define GR_STAMP(slot) do { if (threadIdx.x == 0 && blockIdx.x < 8 && blockIdx.y == 0) STEP_STAMP(a.trace, blockIdx.x * 8 + (slot)); } while (0)
+// CTAs 0 to 6 stamp their own rows, row 7 has the latest stamp of any CTA.
+#define GR_STAMP(slot) do { if (threadIdx.x == 0 && blockIdx.y == 0 && a.trace) { \
+        if (blockIdx.x < 7) STEP_STAMP(a.trace, blockIdx.x * 8 + (slot)); \
+        atomicMax(reinterpret_cast<unsigned long long*>(a.trace) + 56 + (slot), (unsigned long long)step_trace_now()); } } while (0)
 #else
 #define GR_STAMP(slot) do { } while (0)
 #endif
 
-// grid (row groups, activation rows), 32 * K slices threads; PPW: tile pairs per warp at most; THREADS, CTAS: the launch bounds.
+// grid (row groups, activation rows), 32 * slices threads; PPW: tile pairs per warp; THREADS, CTAS: the launch bounds.
+//
+// An SM has up to 27 such warps that all wait for the same event and then run through this code together: what it takes is
+// their instructions.  So no instruction here is about what the launch already knows: slices are PPW pairs (the last may be
+// shorter: it loads its last pair again, with scales of zero), sums are over a fixed number of slices (zeros behind the last),
+// addresses are made ahead of the wait, a value becomes an integer by an addition (1.5 * 2^23: the integer is in the low bits).
 template <bool PAIR, int WT, bool CHAIN, int PPW, int THREADS, int CTAS>
 __global__ void __launch_bounds__(THREADS, CTAS) k_gemv_row(const GemvArgs a, const uint8_t* __restrict__ t0, const uint8_t* __restrict__ t1, float inv_k) {
     GR_STAMP(0);
+    pdl_launch_dependents();
     constexpr int NM = PAIR ? 2 : 1, NV = PPW / 2, UNITS = 2 * PPW, TILE = MmaGeo<PAIR, WT>::TILE;
+    constexpr int NG = (THREADS / 32 + 3) / 4, LD = NG % 2 ? NG * 4 : NG * 4 + 4;          // groups of four slices; floats per row of their sums: rows on different banks
     static_assert(PPW % 2 == 0, "a warp's 32 lanes load two tile pairs' activations at a time");
-    extern __shared__ __align__(16) unsigned char smem_raw[];               // per warp: UNITS * 128 bytes
-    __shared__ __align__(16) float s_red[NM][16][ROW_RED_LD];
-    __shared__ __align__(16) float s_part[2][ROW_MAX_WARPS];                // the slices' sums of squares: branch, stream
+    extern __shared__ __align__(128) unsigned char smem_raw[];              // per warp: UNITS * 128 bytes
+    __shared__ __align__(16) float s_red[NM * 16][LD];
+    __shared__ __align__(16) float s_part[2][NG * 4];                       // the slices' sums of squares: branch, stream
     __shared__ float s_sx[WT == WT_Q4_K ? ROW_MAX_WARPS * UNITS * 2 : 1];   // Q4_K: activation sums of the units, in the lanes' units
     const int lane = threadIdx.x & 31, ks = threadIdx.x >> 5, KS = blockDim.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int rg = blockIdx.x, b = blockIdx.y;
     const int pairs = a.K >> 6;
-    const int p0 = ks * pairs / KS, np = (ks + 1) * pairs / KS - p0;
+    const int p0 = ks * PPW, np = min(PPW, pairs - p0);
 
     // ---- ahead of the dependency wait: weights, norm weights, what stays constant in shared memory ----
     uint4 q[NM][PPW];
     uint2 sc[NM][PPW], hd[NM][PPW];
+    {
+        const size_t off = ((size_t)rg * pairs + p0) * TILE;
 #pragma unroll
-    for (int i = 0; i < PPW; ++i) {
+        for (int i = 0; i < PPW; ++i) {
+            const int at = (i < np ? i : np - 1) * TILE;
 #pragma unroll
-        for (int m = 0; m < NM; ++m) {
-            const uint8_t* tile = (m ? t1 : t0) + ((size_t)rg * pairs + p0 + i) * TILE;
-            const bool in = i < np;
-            q[m][i] = in ? ld_weight(tile + lane * 16) : make_uint4(0u, 0u, 0u, 0u);
-            sc[m][i] = in ? ld_weight2(tile + 512 + g * 8) : make_uint2(0u, 0u);      // no pair: scale 0, whatever its bytes and activations
-            if (WT == WT_Q4_K) hd[m][i] = in ? ld_weight2(tile + 576 + g * 8) : make_uint2(0u, 0u);
+            for (int m = 0; m < NM; ++m) {
+                const uint8_t* tile = (m ? t1 : t0) + off + at;
+                q[m][i] = ld_weight(tile + lane * 16);
+                sc[m][i] = ld_weight2(tile + 512 + g * 8);
+                if (WT == WT_Q4_K) hd[m][i] = ld_weight2(tile + 576 + g * 8);
+            }
         }
     }
+    if (lane == 0) {
+        const uint32_t wi = (uint32_t)(rg * KS + ks);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            const uint32_t at = wi * a.pf_part[r];
+            if (at < a.pf_bytes[r])
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(a.pf[r] + at), "r"(min(a.pf_part[r], a.pf_bytes[r] - at)) : "memory");
+        }
+    }
+    const int f0 = p0 * 16 + lane, nf = np * 16 - lane;                     // this lane's first float4; how far the slice goes from there
     float4 vp[NV], vw[NV];
-    const int f0 = p0 * 16;                                                 // the slice's first float4
     if (CHAIN) {
         const float4 o4 = make_float4(1.f, 1.f, 1.f, 1.f);
 #pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            const int f = lane + 32 * j;
-            vp[j] = (f < np * 16 && a.add_src && a.w_post) ? reinterpret_cast<const float4*>(a.w_post)[f0 + f] : o4;
-            vw[j] = (f < np * 16 && a.w_pre) ? reinterpret_cast<const float4*>(a.w_pre)[f0 + f] : o4;
+        for (int j = 0; j < NV; ++j) vp[j] = vw[j] = o4;
+        if (a.w_post) {
+#pragma unroll
+            for (int j = 0; j < NV; ++j) if (32 * j < nf) vp[j] = reinterpret_cast<const float4*>(a.w_post)[f0 + 32 * j];
+        }
+        if (a.w_pre) {
+#pragma unroll
+            for (int j = 0; j < NV; ++j) if (32 * j < nf) vw[j] = reinterpret_cast<const float4*>(a.w_pre)[f0 + 32 * j];
         }
     }
+    // Unit u of the slice is 128 bytes, column c (hi, mid, lo, zero) of it at c ^ (u & 3).  Stores: lane's unit is lane / 8 (+ 4 per
+    // further float4), its place (lane & 3) * 8 + (lane & 4).  Loads: lane (g, t) reads column g & 3 of every unit.
     unsigned char* xb = smem_raw + ks * (UNITS * 128);
-    for (int i = lane; i < UNITS * 8; i += 32) {                            // the zero column
-        const int u = i >> 3;
-        reinterpret_cast<uint32_t*>(xb + u * 128 + ((3 ^ (u & 3)) * 32))[i & 7] = 0u;
-    }
-    const int ks4 = (KS + 3) & ~3;                                          // sums are read four at a time: zeros behind the last slice's
-    if (ks == 0) {
-        for (int k = KS; k < ks4; ++k) {
-            if (lane < 16) {
+    unsigned char* xs = xb + (lane >> 3) * 128 + (lane & 3) * 8 + (lane & 4);
+    unsigned char *x_hi = xs + ((0 ^ (lane >> 3)) * 32), *x_mid = xs + ((1 ^ (lane >> 3)) * 32), *x_lo = xs + ((2 ^ (lane >> 3)) * 32);
+    const unsigned char* xl = xb + (g & 3) * 32 + t * 8;
+    const int step = ((g & 1) ? -32 : 32), step2 = ((g & 2) ? -64 : 64);    // to column c ^ 1, c ^ 2
 #pragma unroll
-                for (int m = 0; m < NM; ++m) s_red[m][lane][k] = 0.f;
-            }
+    for (int j = 0; j < NV; ++j) *reinterpret_cast<uint32_t*>(xs + j * 512 + ((3 ^ (lane >> 3)) * 32)) = 0u;
+    if (ks == 0) {
+        for (int k = KS; k < NG * 4; ++k) {
+            if (lane < NM * 16) s_red[lane][k] = 0.f;
             if (lane < 2) s_part[lane][k] = 0.f;
         }
     }
+    const float4* hp = reinterpret_cast<const float4*>((CHAIN ? a.h_in : a.x) + (size_t)b * a.ldx) + f0;
+    const float4* ap = reinterpret_cast<const float4*>(a.add_src + (size_t)b * a.ldx) + f0;
     GR_STAMP(1);
-    pdl_launch_dependents();
     pdl_wait();
     GR_STAMP(2);
 
     // ---- this warp's activations ----
     float4 x[NV];
-    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) { x[j] = make_float4(0.f, 0.f, 0.f, 0.f); if (32 * j < nf) x[j] = hp[32 * j]; }
     if (CHAIN) {
-        const float4* hp = reinterpret_cast<const float4*>(a.h_in + (size_t)b * a.ldx) + f0;
-        const float4* ap = a.add_src ? reinterpret_cast<const float4*>(a.add_src + (size_t)b * a.ldx) + f0 : nullptr;
-        float4 va[NV];
+        if (a.add_src) {
+            float4 va[NV];
 #pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            const int f = lane + 32 * j;
-            x[j] = f < np * 16 ? hp[f] : z4;
-            va[j] = (ap && f < np * 16) ? ap[f] : z4;
-        }
-        float ra = 1.f;
-        if (ap && a.w_post) {
-            float s = 0.f;
+            for (int j = 0; j < NV; ++j) { va[j] = make_float4(0.f, 0.f, 0.f, 0.f); if (32 * j < nf) va[j] = ap[32 * j]; }
+            float ra = 1.f;
+            if (a.w_post) {
+                float s = 0.f;
 #pragma unroll
-            for (int j = 0; j < NV; ++j) s += fmaf(va[j].x, va[j].x, va[j].y * va[j].y) + fmaf(va[j].z, va[j].z, va[j].w * va[j].w);
-            s = warp_sum(s);
-            if (lane == 0) s_part[0][ks] = s;
-            __syncthreads();
-            ra = rsqrt_newton(fmaf(row_total(s_part[0], KS), inv_k, a.eps));
-        }
-        GR_STAMP(5);
-        float s = 0.f;
-        if (ap) {
+                for (int j = 0; j < NV; ++j) s += fmaf(va[j].x, va[j].x, va[j].y * va[j].y) + fmaf(va[j].z, va[j].z, va[j].w * va[j].w);
+                s = warp_sum(s);
+                if (lane == 0) s_part[0][ks] = s;
+                __syncthreads();
+                ra = rsqrt_newton(fmaf(row_total<NG>(s_part[0]), inv_k, a.eps));
+            }
 #pragma unroll
             for (int j = 0; j < NV; ++j) {
                 x[j].x = fmaf(va[j].x * ra, vp[j].x, x[j].x); x[j].y = fmaf(va[j].y * ra, vp[j].y, x[j].y);
                 x[j].z = fmaf(va[j].z * ra, vp[j].z, x[j].z); x[j].w = fmaf(va[j].w * ra, vp[j].w, x[j].w);
             }
         }
+        GR_STAMP(5);
+        if (a.h_out && rg == 0) {
+            float4* ho = reinterpret_cast<float4*>(a.h_out + (size_t)b * a.ldx) + f0;
 #pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            const int f = lane + 32 * j;
-            if (a.h_out && rg == 0 && f < np * 16) reinterpret_cast<float4*>(a.h_out + (size_t)b * a.ldx)[f0 + f] = x[j];
-            s += fmaf(x[j].x, x[j].x, x[j].y * x[j].y) + fmaf(x[j].z, x[j].z, x[j].w * x[j].w);
-            x[j].x *= vw[j].x; x[j].y *= vw[j].y; x[j].z *= vw[j].z; x[j].w *= vw[j].w;
+            for (int j = 0; j < NV; ++j) if (32 * j < nf) ho[32 * j] = x[j];
         }
         if (a.w_pre) {
+            float s = 0.f;
+#pragma unroll
+            for (int j = 0; j < NV; ++j) {
+                s += fmaf(x[j].x, x[j].x, x[j].y * x[j].y) + fmaf(x[j].z, x[j].z, x[j].w * x[j].w);
+                x[j].x *= vw[j].x; x[j].y *= vw[j].y; x[j].z *= vw[j].z; x[j].w *= vw[j].w;
+            }
             s = warp_sum(s);
             if (lane == 0) s_part[1][ks] = s;
         }
-    } else {
-        const float4* xp = reinterpret_cast<const float4*>(a.x + (size_t)b * a.ldx) + f0;
-#pragma unroll
-        for (int j = 0; j < NV; ++j) { const int f = lane + 32 * j; x[j] = f < np * 16 ? xp[f] : z4; }
     }
-    float am = 0.f, scale, inv;
+    float am = 0.f;
 #pragma unroll
     for (int j = 0; j < NV; ++j) am = fmaxf(am, fmaxf(fmaxf(fabsf(x[j].x), fabsf(x[j].y)), fmaxf(fabsf(x[j].z), fabsf(x[j].w))));
-    am = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(am)));        // not negative: the bits are in the values' order
-    pow2_scale(am, scale, inv);
+    // The power of two that brings the largest value m * 2^e, 1/2 <= m < 1, to m * 2^22 (2^22 and not more: the largest vector
+    // element of 2^-104 and less is left smaller).  |x|'s bits are in the values' order.
+    const uint32_t eb = max(__reduce_max_sync(0xffffffffu, __float_as_uint(am)) >> 23, 22u);
+    const float scale = __uint_as_float((275u - eb) << 23), inv = __uint_as_float((eb - 21u) << 23);
     GR_STAMP(6);
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
-        const int f = lane + 32 * j, u = f >> 3;
-        const float v[4] = {x[j].x * scale, x[j].y * scale, x[j].z * scale, x[j].w * scale};
-        uint32_t wh, wm, wl;
-        split_x4(v, true, wh, wm, wl);
-        unsigned char* p = xb + u * 128 + (f & 3) * 8 + ((f >> 2) & 1) * 4;
-        *reinterpret_cast<uint32_t*>(p + ((0 ^ (u & 3)) * 32)) = wh;
-        *reinterpret_cast<uint32_t*>(p + ((1 ^ (u & 3)) * 32)) = wm;
-        *reinterpret_cast<uint32_t*>(p + ((2 ^ (u & 3)) * 32)) = wl;
+        const float v[4] = {x[j].x, x[j].y, x[j].z, x[j].w};
+        uint32_t w[4];
+        // x * scale + 1.5 * 2^23 has the integer in its low 23 bits; its three signed bytes as in split_x4
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = (__float_as_uint(fmaf(v[i], scale, 12582912.f)) + (0x00808080u - 0x4B400000u)) ^ 0x00808080u;
+        const uint32_t wl = __byte_perm(__byte_perm(w[0], w[1], 0x0040), __byte_perm(w[2], w[3], 0x0040), 0x5410);
+        const uint32_t wm = __byte_perm(__byte_perm(w[0], w[1], 0x0051), __byte_perm(w[2], w[3], 0x0051), 0x5410);
+        const uint32_t wh = __byte_perm(__byte_perm(w[0], w[1], 0x0062), __byte_perm(w[2], w[3], 0x0062), 0x5410);
+        *reinterpret_cast<uint32_t*>(x_hi + j * 512) = wh;
+        *reinterpret_cast<uint32_t*>(x_mid + j * 512) = wm;
+        *reinterpret_cast<uint32_t*>(x_lo + j * 512) = wl;
         if (WT == WT_Q4_K) {
             int sh = __dp4a((int)wh, 0x01010101, 0), sm = __dp4a((int)wm, 0x01010101, 0), sl = __dp4a((int)wl, 0x01010101, 0);
 #pragma unroll
@@ -207,7 +225,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_gemv_row(const GemvArgs a, co
                 sl += __shfl_xor_sync(0xffffffffu, sl, o);
             }
             if ((lane & 7) == 0)
-                *reinterpret_cast<float2*>(s_sx + (ks * UNITS + u) * 2) = make_float2(-16.f * (float)(sh * 256 + sm), -16.f * (float)(sl * 256));
+                *reinterpret_cast<float2*>(s_sx + (ks * UNITS + (lane >> 3) + 4 * j) * 2) = make_float2(-16.f * (float)(sh * 256 + sm), -16.f * (float)(sl * 256));
         }
     }
     __syncwarp();
@@ -217,16 +235,16 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_gemv_row(const GemvArgs a, co
     float acc[NM][2];
 #pragma unroll
     for (int m = 0; m < NM; ++m) acc[m][0] = acc[m][1] = 0.f;
-    const int c = g & 3;                                                    // lanes g >= 4 fill columns that nobody reads
 #pragma unroll
     for (int i = 0; i < PPW; ++i) {
 #pragma unroll
         for (int blk = 0; blk < 2; ++blk) {
             const int u = 2 * i + blk;
-            const uint2 bx = *reinterpret_cast<const uint2*>(xb + u * 128 + (c ^ (u & 3)) * 32 + t * 8);
+            const uint2 bx = *reinterpret_cast<const uint2*>(xl + u * 128 + ((u & 1) ? step : 0) + ((u & 2) ? step2 : 0));   // lanes g >= 4 fill columns that nobody reads
 #pragma unroll
             for (int m = 0; m < NM; ++m) {
-                const uint32_t w0 = blk ? q[m][i].z : q[m][i].x, w1 = blk ? q[m][i].w : q[m][i].y, s2 = blk ? sc[m][i].y : sc[m][i].x;
+                const uint32_t w0 = blk ? q[m][i].z : q[m][i].x, w1 = blk ? q[m][i].w : q[m][i].y;
+                const uint32_t s2 = i < np ? (blk ? sc[m][i].y : sc[m][i].x) : 0u;
                 int dd[4];
                 if constexpr (WT == WT_Q4_0) {
                     const uint32_t M = 0xF0F0F0F0u, X = 0x80808080u;
@@ -255,14 +273,14 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_gemv_row(const GemvArgs a, co
         for (int h = 0; h < 2; ++h) {
             float v = acc[m][h] * cm;
             v += __shfl_xor_sync(0xffffffffu, v, 1);
-            if (t == 0) s_red[m][g + 8 * h][ks] = v;
+            if (t == 0) s_red[m * 16 + g + 8 * h][ks] = v;
         }
     }
     __syncthreads();
     // ---- the slices' sums: lane = row (and matrix) ----
     if (ks == 0) {
-        float v = row_total(s_red[PAIR ? lane >> 4 : 0][lane & 15], KS);
-        if (CHAIN && a.w_pre) v *= rsqrt_newton(fmaf(row_total(s_part[1], KS), inv_k, a.eps));
+        float v = row_total<NG>(s_red[PAIR ? lane : lane & 15]);
+        if (CHAIN && a.w_pre) v *= rsqrt_newton(fmaf(row_total<NG>(s_part[1]), inv_k, a.eps));
         const float up = PAIR ? __shfl_down_sync(0xffffffffu, v, 16) : 0.f;
         if (lane < 16) {
             const float r = !PAIR ? v : (a.epi == EPI_GEGLU ? gelu_tanh(v) : silu_clip(v)) * up;
