@@ -50,6 +50,14 @@ template <typename T, int DPL> struct KvRow {
             w[0] = *reinterpret_cast<const unsigned short*>(p);
         }
     }
+    __device__ __forceinline__ void store(T* p) const {
+        if constexpr (BYTES == 32) {
+            reinterpret_cast<uint4*>(p)[0] = make_uint4(w[0], w[1], w[2], w[3]); reinterpret_cast<uint4*>(p)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+        } else if constexpr (BYTES == 16) *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+        else if constexpr (BYTES == 8) *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[1]);
+        else if constexpr (BYTES == 4) *reinterpret_cast<uint32_t*>(p) = w[0];
+        else *reinterpret_cast<unsigned short*>(p) = (unsigned short)w[0];
+    }
     __device__ __forceinline__ void from_float(const float* f) {      // values already rounded to T
         if constexpr (sizeof(T) == 4) {
 #pragma unroll

@@ -761,13 +761,16 @@ def step_trace(gpu, args):
         r = prod[k, 0].astype(np.int64)
         out["kernels"][nm] = {"started": (r[0] - t0) / 1e3, "prologue_done": (r[1] - t0) / 1e3, "wait_over": (r[2] - t0) / 1e3,
                               "input_staged": (r[3] - t0) / 1e3, "products_done": (r[4] - t0) / 1e3}
+        m = prod[k, 7].astype(np.int64)             # the latest CTA's stamps
+        if m[4] > 0:
+            out["kernels"][nm]["latest"] = {"started": (m[0] - t0) / 1e3, "wait_over": (m[2] - t0) / 1e3, "input_staged": (m[3] - t0) / 1e3, "products_done": (m[4] - t0) / 1e3}
         if r[5] > 0:        # inside the staging: norm chain -- branch RMS known, stream RMS and maximum known; long plain vector -- bulk copy landed, maximum known
             out["kernels"][nm].update({"staging_mark_1": (r[5] - t0) / 1e3, "staging_mark_2": (r[6] - t0) / 1e3})
     live = att[(att[:, 4] > 0)]
     if len(live):
         last = att[att[:, 7] > 0]
         out["kernels"]["attention"] = {
-            "ctas_with_positions": int(len(live)), "started": float((live[:, 0].min() - t0) / 1e3), "rows_requested": float((live[:, 1].max() - t0) / 1e3),
+            "ctas_with_positions": int(len(live)), "started": float((live[:, 0].min() - t0) / 1e3), "last_started": float((live[:, 0].max() - t0) / 1e3), "rows_requested": float((live[:, 1].max() - t0) / 1e3),
             "wait_over": float((live[:, 2].max() - t0) / 1e3), "rows_normed_rotated": float((live[:, 3].max() - t0) / 1e3),
             "positions_done": float((live[:, 4].max() - t0) / 1e3), "partial_stored": float((live[:, 5].max() - t0) / 1e3) if (live[:, 5] > 0).any() else None,
             "ticket_taken": float((live[:, 6].max() - t0) / 1e3) if (live[:, 6] > 0).any() else None,
