@@ -24,6 +24,7 @@
 // Every wait is bounded: when one runs out the kernel records DEVERR_WAIT, stops waiting, and still frees its tensor memory.
 #include "gemm_tc.cuh"
 #include "gemv_mma.cuh"
+#include "gemv_rows.cuh"
 
 #include <atomic>
 #include <cmath>
@@ -1114,6 +1115,7 @@ GemmRoute gemm_route(int wtype, const GemvArgs& a, const uint8_t* t0, const uint
     if (a.B < TC_MIN_ROWS || a.K <= 0 || a.K > TC_MAX_K || a.N < 16 || (!a.y && a.epi != EPI_ARGMAX) || (wtype == WT_Q4_K ? (a.K % 256) : (a.K % 32))) return GEMM_NONE;
     if (a.epi == EPI_ARGMAX && a.B > tc_rows_fit(wtype, a.K)) return GEMM_NONE;
     if ((a.ldx & 3) || (!a.h_in && (!a.x || ((uintptr_t)a.x & 15)))) return GEMM_NONE;
+    if (policy == 1 && t0 && (t1 || !pair) && gemv_rows_takes(wtype, a)) return GEMM_NONE;
     if (takes_mma(wtype, a, t0, t1, policy)) return GEMM_FEW;
     if (wide) return GEMM_NONE;
     if (policy == 0 || (policy == 1 && a.B < tc_rows_from(wtype, a, pair, t0 && (t1 || !pair)))) return GEMM_NONE;

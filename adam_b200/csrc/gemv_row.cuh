@@ -47,6 +47,18 @@ __device__ __forceinline__ uint2 ld_weight2(const uint8_t* p) {
     return v;
 }
 
+// Four scaled activations (integers of at most 31 bits after rounding) as four words of signed bytes, the highest digits first:
+// the digits of split_x4, of which the top one needs no flip.
+__device__ __forceinline__ void split4_x4(const float (&f)[4], uint32_t (&d)[4]) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = ((uint32_t)__float2int_rn(f[i]) + 0x00808080u) ^ 0x00808080u;
+    const uint32_t l01 = __byte_perm(w[0], w[1], 0x5140), l23 = __byte_perm(w[2], w[3], 0x5140);      // bytes 0, 0, 1, 1
+    const uint32_t h01 = __byte_perm(w[0], w[1], 0x7362), h23 = __byte_perm(w[2], w[3], 0x7362);      // bytes 2, 2, 3, 3
+    d[0] = __byte_perm(h01, h23, 0x7632); d[1] = __byte_perm(h01, h23, 0x5410);
+    d[2] = __byte_perm(l01, l23, 0x7632); d[3] = __byte_perm(l01, l23, 0x5410);
+}
+
 // The sum of NG groups of four floats at a 16-byte aligned place.
 template <int NG>
 __device__ __forceinline__ float row_total(const float* p) {
@@ -68,6 +80,12 @@ __device__ __forceinline__ float row_total(const float* p) {
 #define GR_STAMP(slot) do { } while (0)
 #endif
 
+#ifdef ADAM_B200_STEP_TRACE
+#define GM_STAMP2(slot) do { if (threadIdx.x == 0 && blockIdx.x < 8) STEP_STAMP(a_in.trace, blockIdx.x * 8 + (slot)); } while (0)
+#else
+#define GM_STAMP2(slot) do { } while (0)
+#endif
+
 // grid (row groups, activation rows), 32 * slices threads; PPW: tile pairs per warp; THREADS, CTAS: the launch bounds.
 //
 // An SM has up to 27 such warps that all wait for the same event and then run through this code together: what it takes is
@@ -81,7 +99,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_gemv_row(const GemvArgs a, co
     constexpr int NM = PAIR ? 2 : 1, NV = PPW / 2, UNITS = 2 * PPW, TILE = MmaGeo<PAIR, WT>::TILE;
     constexpr int NG = (THREADS / 32 + 3) / 4, LD = NG % 2 ? NG * 4 : NG * 4 + 4;          // groups of four slices; floats per row of their sums: rows on different banks
     static_assert(PPW % 2 == 0, "a warp's 32 lanes load two tile pairs' activations at a time");
-    extern __shared__ __align__(128) unsigned char smem_raw[];              // per warp: UNITS * 128 bytes
+    extern __shared__ __align__(16) unsigned char smem_raw[];               // per warp: UNITS * 128 bytes
     __shared__ __align__(16) float s_red[NM * 16][LD];
     __shared__ __align__(16) float s_part[2][NG * 4];                       // the slices' sums of squares: branch, stream
     __shared__ float s_sx[WT == WT_Q4_K ? ROW_MAX_WARPS * UNITS * 2 : 1];   // Q4_K: activation sums of the units, in the lanes' units

@@ -190,6 +190,27 @@ def test_one_row_gemv_edges(gpu, ggml_type, N, K):
         assert np.linalg.norm(y - ref) <= 1e-6 * np.linalg.norm(xs) * np.linalg.norm(W) / np.sqrt(K) * 4
 
 
+@pytest.mark.parametrize("ggml_type,N,K,B", [
+    (2, 16, 64, 2), (2, 48, 192, 3), (2, 2368, 1024, 4), (2, 2384, 1152, 3),       # one row group per CTA, one more than the SMs
+    (2, 6912, 1152, 2), (2, 7120, 1152, 4), (2, 4752, 2048, 2), (2, 160, 2048, 4),  # three per CTA, the last CTA not full; 16 slices
+    (2, 160, 2112, 3), (2, 1152, 6912, 4), (2, 96, 8192, 4), (2, 96, 8256, 2),      # slices of four pairs; the most; too long
+    (12, 16, 256, 4), (12, 6912, 1280, 3), (12, 96, 4352, 2), (12, 2064, 1536, 4)])
+def test_few_row_gemv_edges(gpu, ggml_type, N, K, B):
+    """Products of two to four rows over matrices that the SMs hold at once, at the edges of what takes them.  Activations keep 31 bits
+    of their slice's largest value, sums are fp32: 5e-7 of the norms' product, rows and slices of any scale."""
+    rng = np.random.default_rng(N + K + B)
+    raw = (gb.random_q4_0_blocks if ggml_type == 2 else gb.random_q4_k_blocks)(rng, N, K)
+    x = rng.standard_normal((B, K)).astype(np.float32) * rng.uniform(0.01, 100.0, (B, 1)).astype(np.float32)
+    W = q4_blocks.dequant(raw.reshape(-1), ggml_type, N, K).astype(np.float64)
+    for scale in (np.ones(K), 10.0 ** rng.integers(-3, 4, K // 64).repeat(64)):
+        xs = (x * scale).astype(np.float32)
+        xs[B - 1, : K // 2] = 0.0
+        y = _gemv(gpu, ggml_type, raw, N, K, xs, tile=True)
+        for b in range(B):
+            ref = W @ xs[b].astype(np.float64)
+            assert np.linalg.norm(y[b] - ref) <= 5e-7 * np.linalg.norm(xs[b]) * np.linalg.norm(W) / np.sqrt(K) * 4
+
+
 @pytest.mark.parametrize("N,K", [(5376, 5376), (512, 21504), (2048, 4096), (3, 256), (9, 768), (64, 1024)])
 def test_q4_k_gemv(gpu, N, K):
     rng = np.random.default_rng(N * 17 + K)
