@@ -2,6 +2,7 @@
 #include "gemv_mma.cuh"
 #include "gemv_row.cuh"
 #include "gemv_rows.cuh"
+#include "gemv_ring.cuh"
 
 #include <cstdio>
 #include <cstdlib>
@@ -48,6 +49,7 @@ int launch_gemv_mma(int wt, const uint8_t* t0, const uint8_t* t1, GemvArgs a, cu
     const bool pair = (a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU);
     if (pair && !t1) return fail(ADAMAH_ERR_INVALID, "gemv_mma: second matrix missing");
     if (gemv_row_takes(wt, a)) return launch_gemv_row(wt, t0, t1, a, stream);
+    if (gemv_ring_takes(wt, a)) return launch_gemv_ring(wt, t0, t1, a, stream);
     if (gemv_rows_takes(wt, a)) return launch_gemv_rows(wt, t0, t1, a, stream);
     const int units = a.K / 32, pairs = a.K / 64, n_rg = a.N / 16;
     // batch rows per pass: as many of 4, 2, 1 as shared memory allows

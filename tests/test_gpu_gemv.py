@@ -190,6 +190,25 @@ def test_one_row_gemv_edges(gpu, ggml_type, N, K):
         assert np.linalg.norm(y - ref) <= 1e-6 * np.linalg.norm(xs) * np.linalg.norm(W) / np.sqrt(K) * 4
 
 
+@pytest.mark.parametrize("ggml_type,N,K", [
+    (2, 2384, 5376), (2, 4752, 4160), (2, 2400, 8192), (2, 16, 8256), (2, 48, 12352),      # uneven slices, CTAs of one and two row groups
+    (2, 32, 21504), (2, 16, 24576), (2, 16, 24640),                                        # two ring stages; the longest slices; longer
+    (12, 2384, 5376), (12, 2400, 4352), (12, 32, 21504), (12, 16, 24576)])
+def test_streamed_one_row_gemv_edges(gpu, ggml_type, N, K):
+    """Products of one row over matrices that are streamed, at the edges of what takes them; the bound of test_few_row_gemv_edges
+    (1e-6 where the matrix is too long for slices of their own scale: 23 bits of the vector's largest value)."""
+    rng = np.random.default_rng(N + K)
+    raw = (gb.random_q4_0_blocks if ggml_type == 2 else gb.random_q4_k_blocks)(rng, N, K)
+    x = rng.standard_normal((1, K)).astype(np.float32)
+    W = q4_blocks.dequant(raw.reshape(-1), ggml_type, N, K).astype(np.float64)
+    tol = 5e-7 if K <= 24576 else 1e-6
+    for scale in (np.ones(K), 10.0 ** rng.integers(-3, 4, K // 64).repeat(64)):
+        xs = (x * scale).astype(np.float32)
+        y = _gemv(gpu, ggml_type, raw, N, K, xs, tile=True)
+        ref = xs.astype(np.float64) @ W.T
+        assert np.linalg.norm(y - ref) <= tol * np.linalg.norm(xs) * np.linalg.norm(W) / np.sqrt(K) * 4
+
+
 @pytest.mark.parametrize("ggml_type,N,K,B", [
     (2, 16, 64, 2), (2, 48, 192, 3), (2, 2368, 1024, 4), (2, 2384, 1152, 3),       # one row group per CTA, one more than the SMs
     (2, 6912, 1152, 2), (2, 7120, 1152, 4), (2, 4752, 2048, 2), (2, 160, 2048, 4),  # three per CTA, the last CTA not full; 16 slices
