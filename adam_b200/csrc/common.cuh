@@ -108,7 +108,7 @@ inline cudaError_t launch_k(void (*k)(KArgs...), dim3 grid, dim3 block, size_t s
 // SM changes its split between L1 and shared memory only when it is empty, so a kernel whose own choice differs from that of
 // the kernel before it cannot start beside it.
 inline bool carveout_max(const void* k, int smem_limit) {
-    if ((smem_limit > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_limit) != cudaSuccess) ||
+    if ((smem_limit > 0 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_limit) != cudaSuccess) ||
         cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess) {
         cudaGetLastError();
         return false;
@@ -116,17 +116,24 @@ inline bool carveout_max(const void* k, int smem_limit) {
     return true;
 }
 
-// The same with the CTAs of a launch grouped into thread-block clusters of `cluster_x` along x (gridDim.x a multiple of it).
+// The same with the CTAs of a launch grouped into thread-block clusters of `cluster_x` along x (gridDim.x a multiple of it), and
+// with `all_shared` under the split of carveout_max for this launch alone.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_k_cluster(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, unsigned cluster_x, Args... args) {
+inline cudaError_t launch_k_cluster(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl, unsigned cluster_x, bool all_shared, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
-    cudaLaunchAttribute at[2];
+    cudaLaunchAttribute at[3];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = cluster_x; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at; cfg.numAttrs = pdl ? 2 : 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    if (pdl) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (all_shared) {
+        at[cfg.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        at[cfg.numAttrs++].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+    }
     return cudaLaunchKernelEx(&cfg, k, KArgs(args)...);
 }
 

@@ -242,9 +242,11 @@ __global__ void __launch_bounds__(256) k_attention(const float* __restrict__ qkv
     __shared__ bool s_last;
     __shared__ __align__(8) uint64_t s_bar[16][2], s_mb;                // a slot's keys and values; the cluster's partial results
     AT_STAMP(0);
-    // Asked for at once, by the CTAs without positions too: the next kernel starts when every CTA has asked (one that leaves
-    // a cluster early counts only when the whole cluster is done, which held the o-proj back until the merge).
-    pdl_launch_dependents();
+    // In a cluster asked for at once, by the CTAs without positions too: the next kernel starts when every CTA has asked (one that
+    // leaves a cluster early counts only when the whole cluster is done, which held the o-proj back until the merge).  Large
+    // grids of independent splits ask late and keep their own shared-memory split: the kernels around them fill the SMs (64
+    // sequences of the 27B shape, 8 layers: 3.30 ms per step, 3.42 when asked at once, 3.57 with the largest split, too).
+    if (n_splits_max == 0) pdl_launch_dependents();
     // n_splits_max == 0: the gridDim.x splits of a (sequence, head group) are one thread-block cluster and merge
     // through CTA 0's shared memory instead of global memory, a ticket and the last CTA to arrive.
     const bool cmerge = n_splits_max == 0;
@@ -364,6 +366,7 @@ __global__ void __launch_bounds__(256) k_attention(const float* __restrict__ qkv
         sn[j] = i < half ? st[i] : 0.f;
     }
     AT_STAMP(1);
+    if (n_splits_max != 0) pdl_launch_dependents();
     pdl_wait();                                 // this step's q/k/v rows come from the previous kernel
     AT_STAMP(2);
     const float* row_q = qkv + (size_t)b * qkv_ld + (size_t)head0 * hd;
@@ -803,11 +806,6 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
     const uint32_t hpc_auto = work <= 12u ? 1u : (work <= 32u ? (gs >= 2u ? 2u : 1u) : gs);
     const uint32_t hpc = (hpc_env && gs % hpc_env == 0 && hpc_env <= 8u) ? hpc_env : hpc_auto;
     const uint32_t window = ((d.flags & 1u) && d.sliding_window > 0 && !is_global_layer(d, L)) ? d.sliding_window : 0;
-    // Chunks in flight per CTA: one per warp, or up to two where few CTAs run and a context just beyond 8 chunks per CTA (a window of
-    // 512) would have a warp wait for memory a second time.
-    const size_t slot_bytes = (size_t)2 * ATTN_CP * d.head_dim * sizeof(T);
-    const uint32_t n_slots = work <= 64u ? (uint32_t)std::min<size_t>(16, std::max<size_t>(8, (192u << 10) / slot_bytes)) : 8u;
-    const size_t smem = n_slots * slot_bytes + ((size_t)hpc * d.head_dim + 2 * (size_t)d.head_dim) * 4;
     const int which = is_global_layer(d, L) ? 1 : 0;
     const Layer& ly = D->layers[L];
     const uint32_t qkv_ld = (d.n_head + 2 * d.n_head_kv) * d.head_dim;
@@ -831,31 +829,35 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
         bool done = false;
         for (int i = 0; i < n_set; ++i) done |= set[i] == kern;
         if (!done) {
-            if (!carveout_max((const void*)kern, ATTN_SMEM_LIMIT)) return fail(ADAMAH_ERR_BACKEND, "attention: cannot raise the shared-memory limit");
+            if (cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ATTN_SMEM_LIMIT) != cudaSuccess) return fail(ADAMAH_ERR_BACKEND, "attention: cannot raise the shared-memory limit");
             if (n_set < 32) set[n_set++] = kern;
         }
     }
-    // Few (sequence, head) pairs in flight (at most 12): the position splits of a pair form one thread-block cluster of 8 CTAs and merge
-    // through shared memory (no partial results in global memory, no ticket, no last-CTA pass: 3 us less per launch at the
+    // Few (sequence, head group) pairs in flight (at most 16): the position splits of a pair form one thread-block cluster of 8 CTAs and
+    // merge through shared memory (no partial results in global memory, no ticket, no last-CTA pass: 3 us less per launch at the
     // 1B shape).  A cluster covers any context, its CTAs taking more chunks each, so layers that may attend to more than
     // 2048 positions keep the wider grid of independent splits.  (Clusters of 16 were measured slower: they start later,
     // and so does every kernel behind them.)  ADAM_B200_ATTN_CLUSTER=0 turns the path off, =16 allows clusters of 16.
     static const int cluster_env = getenv("ADAM_B200_ATTN_CLUSTER") ? atoi(getenv("ADAM_B200_ATTN_CLUSTER")) : 8;
-    static const uint32_t cluster_work = getenv("ADAM_B200_ATTN_CLUSTER_WORK") ? (uint32_t)atoi(getenv("ADAM_B200_ATTN_CLUSTER_WORK")) : 12u;
-    // The kernels behind a cluster launch start later (their prologues no longer overlap it); that costs more than the merge
-    // saves once the o-proj behind it has more than about a megabyte of tiles to request (27B shape, 4-way shard: 2 % slower).
-    const size_t o_bytes = (size_t)ly.m[MAT_O].rows * ly.m[MAT_O].cols * 9 / 16;
-    if (cluster_env != 0 && work <= cluster_work && reach <= 2048u && o_bytes <= (1u << 20)) {
-        struct Known { AttnKernel k; unsigned cs; };
+    static const uint32_t cluster_pairs = getenv("ADAM_B200_ATTN_CLUSTER_WORK") ? (uint32_t)atoi(getenv("ADAM_B200_ATTN_CLUSTER_WORK")) : 16u;
+    const bool cluster = cluster_env != 0 && pairs <= cluster_pairs && reach <= 2048u;
+    // Chunks in flight per CTA: one per warp; up to two in a cluster of splits, where a context just beyond 8 chunks per CTA (a window
+    // of 512) would have a warp wait for memory a second time.  (Elsewhere CTAs without positions would hold that much, too.)
+    const size_t slot_bytes = (size_t)2 * ATTN_CP * d.head_dim * sizeof(T);
+    const uint32_t n_slots = cluster ? (uint32_t)std::min<size_t>(16, std::max<size_t>(8, (192u << 10) / slot_bytes)) : 8u;
+    const size_t smem = n_slots * slot_bytes + ((size_t)hpc * d.head_dim + 2 * (size_t)d.head_dim) * 4;
+    if (cluster) {
+        // clusters of a size that run at once, by kernel (0: none of that size)
+        struct Known { AttnKernel k; unsigned cs; int n; };
         static Known known[16]; static int n_known = 0;
-        int cs = -1;
-        for (int i = 0; i < n_known; ++i) if (known[i].k == kern) cs = (int)known[i].cs;
+        const Known* kn = nullptr;
+        for (int i = 0; i < n_known; ++i) if (known[i].k == kern) kn = &known[i];
         const auto smem_for = [&](unsigned c) { return smem + (size_t)c * hpc * (d.head_dim + 4) * 4; };
-        if (cs < 0) {
-            cs = 0;
+        Known fresh = {kern, 0u, 0};
+        if (!kn) {
             const unsigned c_max = cluster_env == 16 ? 16u : 8u;
             if (c_max > 8 && cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) cudaGetLastError();
-            for (unsigned c = c_max; c >= 8 && !cs; c >>= 1) {
+            for (unsigned c = c_max; c >= 8 && !fresh.n; c >>= 1) {
                 cudaLaunchConfig_t cfg = {};
                 cfg.gridDim = dim3(c, grid.y, 1); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = smem_for(c);
                 cudaLaunchAttribute at[1];
@@ -864,13 +866,15 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
                 cfg.attrs = at; cfg.numAttrs = 1;
                 int n = 0;
                 if (cudaOccupancyMaxActiveClusters(&n, (const void*)kern, &cfg) != cudaSuccess) { cudaGetLastError(); continue; }
-                if (n >= (int)(grid.y * grid.z)) cs = (int)c;
+                fresh.cs = c; fresh.n = n;
             }
-            if (n_known < 16) { known[n_known].k = kern; known[n_known].cs = (unsigned)cs; ++n_known; }
+            if (n_known < 16) known[n_known++] = fresh;
+            kn = &fresh;
         }
+        const unsigned cs = kn->n >= (int)pairs ? kn->cs : 0u;
         if (cs > 0) {
-            grid.x = (unsigned)cs;
-            if (launch_k_cluster(kern, grid, dim3(256), smem_for((unsigned)cs), g.stream, g.pdl, (unsigned)cs, D->qkv, qkv_ld, ly.norm[NORM_Q], ly.norm[NORM_K], d.norm_eps,
+            grid.x = cs;
+            if (launch_k_cluster(kern, grid, dim3(256), smem_for(cs), g.stream, g.pdl, cs, true, D->qkv, qkv_ld, ly.norm[NORM_Q], ly.norm[NORM_K], d.norm_eps,
                                  D->rope_cos[which], D->rope_sin[which], D->rope_pos[which],
                                  D->kv_pool, geo, D->block_table, D->pos, d.n_head, L, window, d.attn_scale,
                                  d.attn_softcap, D->attn_out, D->part_o, D->part_ml, D->attn_ticket, 0u, hpc | (cpc << 16), n_slots, g.dev_err STEP_TRACE_ARG((g_step_trace && L == g_step_trace_layer) ? g_step_trace + 4 * 64 : nullptr)) != cudaSuccess)

@@ -1235,7 +1235,7 @@ static int launch_rows(int wtype, const GemvArgs& a, cudaStream_t stream) {
     }
     cudaError_t e;
     if (S == 1) e = launch_k(p.k, dim3((unsigned)grid), dim3(p.threads), (size_t)p.smem, stream, true, t);
-    else e = launch_k_cluster(p.k, dim3((unsigned)grid), dim3(p.threads), (size_t)p.smem, stream, true, (unsigned)S, t);
+    else e = launch_k_cluster(p.k, dim3((unsigned)grid), dim3(p.threads), (size_t)p.smem, stream, true, (unsigned)S, false, t);
     if (e != cudaSuccess) return fail(ADAMAH_ERR_BACKEND, "gemm_tc: launch failed: %s", cudaGetErrorString(e));
     count_launch();
     ++g_gemm_counts[nt == 16 ? GC_TILE_16 : nt == 32 ? GC_TILE_32 : nt == 64 ? GC_TILE_64 : nt == 128 ? GC_TILE_128 : GC_TILE_256];
