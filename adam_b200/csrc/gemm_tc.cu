@@ -97,8 +97,9 @@ static int tc_rows_fit(int wtype, int K) {              // rows of one pass: who
 }
 
 // ---- activations: chain, scale, two fp16 planes in B-operand order -------------------------------------------
-// Bound by the latency of its chain (one row per CTA: load, up to three reductions, store), not by its 12 bytes per
-// value; the row stays in registers (MAXV float4 per thread) and all loads are issued before the first use.
+// Bound by the latency of its chain (one row per CTA: load, up to two reductions of one barrier each, store), not by its 12
+// bytes per value; the row stays in registers (MAXV float4 per thread), all loads are issued before the first use, the norm
+// weights ahead of the dependency wait.
 // Four consecutive values of K are stored in the order 0, 2, 1, 3: the order in which a word of nibbles is taken apart
 // two at a time (see k_gemm_tc); K order is free as long as both operands agree.
 __device__ __forceinline__ uint32_t swz_off(int r, int kb) { return (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((((kb >> 4) ^ r) & 7) << 4) + (kb & 15)); }
@@ -112,55 +113,53 @@ __device__ __forceinline__ void split_half(float v, __half& hi, __half& lo) {
 // Q4_K (n_min > 0) followed by a float per row, the sum of the 32 values; n_steps is then the number of rows it has room for.
 template <int MAXV, bool CHAIN, bool FEW>
 __global__ void __launch_bounds__(512) k_quant_rows(const GemvArgs a, uint8_t* __restrict__ img, float* __restrict__ inv_out, int n_min, int n_steps) {
-    __shared__ float red[66];
+    __shared__ __align__(16) float red[3][16];          // the warps' sums: branch, stream; their maxima
     const int r = blockIdx.x, tid = threadIdx.x, K = a.K, n4 = K >> 2, nt = blockDim.x;
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f), o4 = make_float4(1.f, 1.f, 1.f, 1.f);
     const bool post = CHAIN && a.add_src && a.w_post, pre = CHAIN && a.w_pre;
-    float4 v[MAXV];
+    float4 v[MAXV], vp[CHAIN ? MAXV : 1], vw[CHAIN ? MAXV : 1];
     pdl_launch_dependents();
+    // ahead of the wait: the norm weights (a step's matrices have pushed them out of L2), zeros behind the last warp's sum
+    if constexpr (CHAIN) {
+#pragma unroll
+        for (int j = 0; j < MAXV; ++j) {
+            const int i = tid + j * nt;
+            vp[j] = (i < n4 && post) ? reinterpret_cast<const float4*>(a.w_post)[i] : o4;
+            vw[j] = (i < n4 && pre) ? reinterpret_cast<const float4*>(a.w_pre)[i] : o4;
+        }
+    }
+    if (tid < 16) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) if (tid >= nt >> 5) red[k][tid] = 0.f;
+    }
+    const float inv_k = 1.0f / (float)K;
     pdl_wait();
     const size_t row = (size_t)r * a.ldx;
     if constexpr (CHAIN) {
         const float* ap = a.add_src ? a.add_src + row : nullptr;
-        float4 va[MAXV], vp[MAXV], vw[MAXV];
+        float4 va[MAXV];
 #pragma unroll
         for (int j = 0; j < MAXV; ++j) {
             const int i = tid + j * nt;
             const bool in = i < n4;
             v[j] = in ? reinterpret_cast<const float4*>(a.h_in + row)[i] : z4;
             va[j] = (in && ap) ? reinterpret_cast<const float4*>(ap)[i] : z4;
-            vp[j] = (in && post) ? reinterpret_cast<const float4*>(a.w_post)[i] : o4;
-            vw[j] = (in && pre) ? reinterpret_cast<const float4*>(a.w_pre)[i] : o4;
         }
-        float rms_a = 1.f;
+        float ra = 1.f;
         if (post) {
             float ss = 0.f;
 #pragma unroll
-            for (int j = 0; j < MAXV; ++j) { ss = fmaf(va[j].x, va[j].x, ss); ss = fmaf(va[j].y, va[j].y, ss); ss = fmaf(va[j].z, va[j].z, ss); ss = fmaf(va[j].w, va[j].w, ss); }
-            ss = block_sum(ss, red);
-            rms_a = sqrtf(ss / (float)K + a.eps);
+            for (int j = 0; j < MAXV; ++j) ss += fmaf(va[j].x, va[j].x, va[j].y * va[j].y) + fmaf(va[j].z, va[j].z, va[j].w * va[j].w);
+            ss = warp_sum(ss);
+            if ((tid & 31) == 0) red[0][tid >> 5] = ss;
+            __syncthreads();
+            ra = rsqrt_newton(fmaf(row_total<4>(red[0]), inv_k, a.eps));
         }
-        const float rcp_a = __frcp_rn(rms_a);
-        float ss = 0.f;
-#pragma unroll
-        for (int j = 0; j < MAXV; ++j) {
-            if (ap) {
-                if (post) {
-                    v[j].x += div_by(va[j].x, rms_a, rcp_a) * vp[j].x; v[j].y += div_by(va[j].y, rms_a, rcp_a) * vp[j].y;
-                    v[j].z += div_by(va[j].z, rms_a, rcp_a) * vp[j].z; v[j].w += div_by(va[j].w, rms_a, rcp_a) * vp[j].w;
-                } else { v[j].x += va[j].x; v[j].y += va[j].y; v[j].z += va[j].z; v[j].w += va[j].w; }
-            }
-            ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss); ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
-            const int i = tid + j * nt;
-            if (i < n4 && a.h_out) reinterpret_cast<float4*>(a.h_out + row)[i] = v[j];
-        }
-        if (pre) {
-            ss = block_sum(ss, red);
-            const float rms = sqrtf(ss / (float)K + a.eps), rcp = __frcp_rn(rms);
+        if (ap) {
 #pragma unroll
             for (int j = 0; j < MAXV; ++j) {
-                v[j].x = div_by(v[j].x, rms, rcp) * vw[j].x; v[j].y = div_by(v[j].y, rms, rcp) * vw[j].y;
-                v[j].z = div_by(v[j].z, rms, rcp) * vw[j].z; v[j].w = div_by(v[j].w, rms, rcp) * vw[j].w;
+                v[j].x = fmaf(va[j].x * ra, vp[j].x, v[j].x); v[j].y = fmaf(va[j].y * ra, vp[j].y, v[j].y);
+                v[j].z = fmaf(va[j].z * ra, vp[j].z, v[j].z); v[j].w = fmaf(va[j].w * ra, vp[j].w, v[j].w);
             }
         }
     } else {
@@ -170,13 +169,36 @@ __global__ void __launch_bounds__(512) k_quant_rows(const GemvArgs a, uint8_t* _
             v[j] = i < n4 ? reinterpret_cast<const float4*>(a.x + row)[i] : z4;
         }
     }
-    float am = 0.f;
+    // the stream's sum of squares and the largest value (ahead of the division by the RMS) in one round
+    float ss = 0.f, am = 0.f;
 #pragma unroll
-    for (int j = 0; j < MAXV; ++j) am = fmaxf(am, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
-    am = block_max(am, red);
+    for (int j = 0; j < MAXV; ++j) {
+        if constexpr (CHAIN) {
+            const int i = tid + j * nt;
+            if (i < n4 && a.h_out) reinterpret_cast<float4*>(a.h_out + row)[i] = v[j];
+            ss += fmaf(v[j].x, v[j].x, v[j].y * v[j].y) + fmaf(v[j].z, v[j].z, v[j].w * v[j].w);
+            v[j].x *= vw[j].x; v[j].y *= vw[j].y; v[j].z *= vw[j].z; v[j].w *= vw[j].w;
+        }
+        am = fmaxf(am, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
+    }
+    am = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(am)));          // not negative: the bits are in the values' order
+    if (pre) ss = warp_sum(ss);
+    if ((tid & 31) == 0) { red[1][tid >> 5] = ss; red[2][tid >> 5] = am; }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float4 m = reinterpret_cast<const float4*>(red[2])[k];
+        am = fmaxf(am, fmaxf(fmaxf(m.x, m.y), fmaxf(m.z, m.w)));
+    }
+    float rp = 1.f;                                     // 1 / RMS of the stream, a factor of every value
+    if (pre) { rp = rsqrt_newton(fmaf(row_total<4>(red[1]), inv_k, a.eps)); am = am * rp * 1.000001f; }
     float s, inv;
     pow2_scale(am, s, inv);                             // largest element in (2^21, 2^22] ...
     s *= 0.0078125f; inv *= 128.f;                      // ... in (2^14, 2^15]
+    if (pre) {
+#pragma unroll
+        for (int j = 0; j < MAXV; ++j) { v[j].x *= rp; v[j].y *= rp; v[j].z *= rp; v[j].w *= rp; }
+    }
     if (tid == 0) inv_out[r] = inv;
     if constexpr (FEW) {
         const int blk = gm_block_bytes(n_min ? WT_Q4_K : WT_Q4_0, n_steps);
