@@ -8,8 +8,8 @@
 // dequant GEMV and stay in L2; selection then works on them in two short parallel stages instead of a
 // serial insertion list per work group as in the shader:
 //   stage 1  one CTA per group of rows keeps each thread's values in registers and extracts the group's k
-//            best by k rounds of a block-wide arg-max (warp shuffles + one shared-memory hop);
-//   stage 2  (decoder only) one CTA per sequence merges the groups' sorted candidates: k rounds of an arg-max
+//            best: every warp its own, then one warp merges the warps' lists (no barrier per candidate);
+//   stage 2  (decoder only) one CTA per sequence merges the groups' sorted candidates: k rounds of a warp's arg-max
 //            over the heads of the groups, which leaves the k best sorted; then soft-max with temperature,
 //            nucleus cut and the draw run on one warp.
 // Ties go to the lower row index everywhere (map_argmax.comp `better`), NaN counts as -FLT_MAX.
@@ -30,34 +30,60 @@ constexpr int SEL_T = 256;                 // threads of a selection CTA
 constexpr int SEL_V = 8;                   // values a thread keeps in registers (a group has at most SEL_T * SEL_V rows)
 constexpr uint32_t TOPK_MAX = 64;
 
-// Block-wide arg-max of (v, i) over SEL_T threads; every thread gets the winner.  sv/si: SEL_T / 32 slots.
-__device__ __forceinline__ void block_best(float& v, int& i, float* sv, int* si) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, i, o);
-        if (better(ov, oi, v, i)) { v = ov; i = oi; }
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) { sv[warp] = v; si[warp] = i; }
-    __syncthreads();
-    v = sv[0]; i = si[0];
-#pragma unroll
-    for (int w = 1; w < SEL_T / 32; ++w) if (better(sv[w], si[w], v, i)) { v = sv[w]; i = si[w]; }
+// A value as an unsigned number in the order of `better` (both zeros are one number; nothing is 0).
+__device__ __forceinline__ uint32_t rank_of(float v) {
+    const uint32_t u = __float_as_uint(v + 0.0f);
+    return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
+// The warp's best of (rank, row), ties to the lower row; rank 0: there is none.  True on the lane that holds it.
+__device__ __forceinline__ bool warp_best(uint32_t o, uint32_t row, uint32_t& best, uint32_t& best_row) {
+    best = __reduce_max_sync(0xffffffffu, o);
+    best_row = __reduce_min_sync(0xffffffffu, o == best ? row : 0xffffffffu);
+    return best != 0u && o == best && row == best_row;
 }
 
-// The k best of this CTA's values: thread t holds values val[j] with keys key[j] (key < 0 = empty slot).
-// Round r leaves the r-th best in (out_v[r], out_i[r]) (shared memory, k <= 64); a slot is emptied once taken.
-__device__ __forceinline__ void block_topk(float (&val)[SEL_V], int (&key)[SEL_V], uint32_t k, float* out_v, int* out_i, float* sv, int* si) {
+// The k best of this CTA's values, sorted: thread t holds values val[j] of rows key[j], ascending with j (key < 0 = empty slot).
+// Every warp sorts out its own k best (a round is two warp reductions and, on the winner's lane, a look at its eight values; no
+// barrier), then one warp merges the warps' lists the same way.  As k rounds of an arg-max over the CTA it took 1 us per round.
+struct TopkLists { float v[SEL_T / 32][TOPK_MAX]; int i[SEL_T / 32][TOPK_MAX]; };
+__device__ __forceinline__ void block_topk(float (&val)[SEL_V], int (&key)[SEL_V], uint32_t k, float* out_v, int* out_i, TopkLists& l) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t rank[SEL_V];
+#pragma unroll
+    for (int j = 0; j < SEL_V; ++j) rank[j] = key[j] >= 0 ? rank_of(val[j]) : 0u;
+    uint32_t o = 0u, best, row;
+    int at = 0;
+    auto look = [&]() {
+        o = 0u;
+#pragma unroll
+        for (int j = 0; j < SEL_V; ++j) if (rank[j] > o) { o = rank[j]; at = key[j]; }
+    };
+    look();
     for (uint32_t r = 0; r < k; ++r) {
-        float bv = SNEG; int bi = -1;
+        const bool mine = warp_best(o, (uint32_t)at, best, row);
+        if (mine) {
+            float v = 0.f;
 #pragma unroll
-        for (int j = 0; j < SEL_V; ++j) if (key[j] >= 0 && better(val[j], key[j], bv, bi)) { bv = val[j]; bi = key[j]; }
-        block_best(bv, bi, sv, si);
-#pragma unroll
-        for (int j = 0; j < SEL_V; ++j) if (key[j] >= 0 && key[j] == bi) key[j] = -1;
-        if (threadIdx.x == 0) { out_v[r] = bi < 0 ? SNEG : bv; out_i[r] = bi; }
+            for (int j = 0; j < SEL_V; ++j) if (key[j] == at) { v = val[j]; rank[j] = 0u; }
+            l.v[warp][r] = v; l.i[warp][r] = at;
+            look();
+        }
+        if (best == 0u && lane == 0) { l.v[warp][r] = SNEG; l.i[warp][r] = -1; }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t next = 0;
+        auto head = [&]() {
+            const bool in = lane < SEL_T / 32 && next < k && l.i[lane][next] >= 0;
+            o = in ? rank_of(l.v[lane][next]) : 0u;
+            at = in ? l.i[lane][next] : 0;
+        };
+        head();
+        for (uint32_t r = 0; r < k; ++r) {
+            const bool mine = warp_best(o, (uint32_t)at, best, row);
+            if (mine) { out_v[r] = l.v[lane][next]; out_i[r] = at; ++next; head(); }
+            if (best == 0u && lane == 0) { out_v[r] = SNEG; out_i[r] = -1; }
+        }
     }
     __syncthreads();
 }
@@ -76,7 +102,7 @@ __global__ void __launch_bounds__(SEL_T) k_group_topk(const float* __restrict__ 
                                                       float* __restrict__ cand_v, int* __restrict__ cand_i,
                                                       float* __restrict__ map, uint64_t n_el, const uint32_t* __restrict__ li,
                                                       const uint32_t* __restrict__ lv, uint32_t* err) {
-    __shared__ float sv[SEL_T / 32]; __shared__ int si[SEL_T / 32];
+    __shared__ TopkLists lists;
     __shared__ float out_v[TOPK_MAX]; __shared__ int out_i[TOPK_MAX];
     const uint32_t g = blockIdx.x, r0 = g * rpg, r1 = min(N, r0 + rpg);
     float val[SEL_V]; int key[SEL_V];
@@ -86,7 +112,7 @@ __global__ void __launch_bounds__(SEL_T) k_group_topk(const float* __restrict__ 
         key[j] = row < r1 ? (int)row : -1;
         val[j] = row < r1 ? penalised(logits[row], (int)row, pen, n_pen, penalty) : SNEG;
     }
-    block_topk(val, key, k, out_v, out_i, sv, si);
+    block_topk(val, key, k, out_v, out_i, lists);
     if (threadIdx.x < k) {
         const uint32_t o = g * k + threadIdx.x;
         if (map) {
@@ -107,35 +133,26 @@ __host__ __device__ inline float sample_uniform(uint64_t seed, uint32_t seq, uin
     return (float)(z >> 40) * (1.0f / 16777216.0f);
 }
 
-// The ids whose logits get the repeat penalty: the distinct tokens among the last 64 of the history (prompt
-// included with on_prompt, else generated tokens only), as the reference's `set(prev[-64:])` (engine.py:3713).
+// The ids whose logits get the repeat penalty: the tokens among the last 64 of the history (prompt included with on_prompt, else
+// generated tokens only), as the reference's `set(prev[-64:])` (engine.py:3713): a thread each, an id may stand there twice.
 // Position q of sequence b holds prompt_tok[q] for q < prompt_len and the logged sample otherwise.
 __device__ __forceinline__ uint32_t history_ids(const int32_t* prompt_tok, const int32_t* gen_log, int32_t plen, int32_t pos_new,
                                                 int on_prompt, uint32_t* ids) {
-    const int32_t lo = max(on_prompt ? 0 : plen, pos_new - 64);
-    uint32_t n = 0;
-    for (int32_t q = lo; q < pos_new; ++q) {
-        const int32_t t = q < plen ? prompt_tok[q] : gen_log[q];
-        if (t < 0) continue;
-        bool seen = false;
-        for (uint32_t j = 0; j < n; ++j) seen |= ids[j] == (uint32_t)t;
-        if (!seen) ids[n++] = (uint32_t)t;
-    }
-    return n;
+    const int32_t lo = max(on_prompt ? 0 : plen, pos_new - 64), q = lo + (int32_t)threadIdx.x;
+    if (q < pos_new) ids[threadIdx.x] = (uint32_t)(q < plen ? prompt_tok[q] : gen_log[q]);      // none: negative, no row's number
+    return (uint32_t)max(pos_new - lo, 0);
 }
 
-// Stage 1 for the decoder: grid (groups, batch); the penalty list is rebuilt by every CTA (<= 64 short loops).
+// Stage 1 for the decoder: grid (groups, batch); every CTA reads the history for itself.
 __global__ void __launch_bounds__(SEL_T) k_sample_stage1(const float* __restrict__ logits, uint32_t V, uint32_t k,
                                                          const int32_t* __restrict__ pos, const int32_t* __restrict__ prompt_len,
                                                          const int32_t* __restrict__ prompt_tok, const int32_t* __restrict__ gen_log, uint32_t ld,
                                                          float penalty, int on_prompt, float* __restrict__ cand_v, int* __restrict__ cand_i) {
-    __shared__ float sv[SEL_T / 32]; __shared__ int si[SEL_T / 32];
+    __shared__ TopkLists lists;
     __shared__ float out_v[TOPK_MAX]; __shared__ int out_i[TOPK_MAX];
-    __shared__ uint32_t s_pen[64]; __shared__ uint32_t s_np;
+    __shared__ uint32_t s_pen[64];
     const uint32_t g = blockIdx.x, b = blockIdx.y, groups = gridDim.x;
-    if (threadIdx.x == 0)
-        s_np = penalty != 1.0f ? history_ids(prompt_tok + (size_t)b * ld, gen_log + (size_t)b * ld, prompt_len[b], pos[b], on_prompt, s_pen) : 0u;
-    __syncthreads();
+    const uint32_t n_pen = penalty != 1.0f ? history_ids(prompt_tok + (size_t)b * ld, gen_log + (size_t)b * ld, prompt_len[b], pos[b], on_prompt, s_pen) : 0u;
     const float* lg = logits + (size_t)b * V;
     const uint32_t rpg = SEL_T * SEL_V, r0 = g * rpg, r1 = min(V, r0 + rpg);
     float val[SEL_V]; int key[SEL_V];
@@ -143,9 +160,20 @@ __global__ void __launch_bounds__(SEL_T) k_sample_stage1(const float* __restrict
     for (int j = 0; j < SEL_V; ++j) {
         const uint32_t row = r0 + threadIdx.x + j * SEL_T;
         key[j] = row < r1 ? (int)row : -1;
-        val[j] = row < r1 ? penalised(lg[row], (int)row, s_pen, s_np, penalty) : SNEG;
+        val[j] = row < r1 ? lg[row] : SNEG;
+        if (!(val[j] == val[j])) val[j] = SNEG;
     }
-    block_topk(val, key, k, out_v, out_i, sv, si);
+    __syncthreads();
+    uint32_t seen = 0;                                  // this thread's values that have had their penalty
+    for (uint32_t i = 0; i < n_pen; ++i) {
+        const uint32_t d = s_pen[i] - r0;
+        if (d < rpg && (d & (SEL_T - 1)) == threadIdx.x) {
+#pragma unroll
+            for (int j = 0; j < SEL_V; ++j)
+                if ((d / SEL_T) == (uint32_t)j && !(seen >> j & 1u)) { seen |= 1u << j; val[j] = val[j] > 0.f ? __fdiv_rn(val[j], penalty) : val[j] * penalty; }
+        }
+    }
+    block_topk(val, key, k, out_v, out_i, lists);
     if (threadIdx.x < k) {
         const size_t o = ((size_t)b * groups + g) * k + threadIdx.x;
         cand_v[o] = out_v[threadIdx.x]; cand_i[o] = out_i[threadIdx.x];
@@ -162,68 +190,84 @@ __global__ void __launch_bounds__(SEL_T) k_sample_stage2(const float* __restrict
                                                          float temperature, float top_p, uint64_t seed,
                                                          const int32_t* __restrict__ pos, int32_t* __restrict__ cur_tok, float* __restrict__ cur_val,
                                                          int32_t* __restrict__ gen_log, uint32_t ld, float* __restrict__ dbg) {
-    __shared__ float sv[SEL_T / 32]; __shared__ int si[SEL_T / 32];
     __shared__ float out_v[TOPK_MAX]; __shared__ int out_i[TOPK_MAX];
     const uint32_t b = blockIdx.x;
     const uint32_t n_cand = groups * k;
     const float* cv = cand_v + (size_t)b * n_cand;
     const int* ci = cand_i + (size_t)b * n_cand;
     extern __shared__ unsigned char sel_sm[];
-    unsigned char* head = sel_sm;                       // [groups] candidates of a group that are taken; each thread its own groups
+    // [groups] the rank and row of a group's head, [groups] candidates of it that are taken; then the candidates
+    uint2* hd = reinterpret_cast<uint2*>(sel_sm);
+    unsigned char* head = sel_sm + (size_t)groups * 8;
     if (in_shared) {
-        float* v = reinterpret_cast<float*>(sel_sm + ((groups + 15) & ~15u));
+        float* v = reinterpret_cast<float*>(sel_sm + (((size_t)groups * 9 + 15) & ~(size_t)15));
         int* i = reinterpret_cast<int*>(v + n_cand);
+#pragma unroll 8
         for (uint32_t c = threadIdx.x; c < n_cand; c += SEL_T) { v[c] = cv[c]; i[c] = ci[c]; }
         cv = v; ci = i;
+        __syncthreads();
     }
-    for (uint32_t q = threadIdx.x; q < groups; q += SEL_T) head[q] = 0;
+    auto head_of = [&](uint32_t q, uint32_t taken) {
+        const uint32_t c = q * k + taken;
+        return taken < k && ci[c] >= 0 ? make_uint2(rank_of(cv[c]), (uint32_t)ci[c]) : make_uint2(0u, 0u);
+    };
+    for (uint32_t q = threadIdx.x; q < groups; q += SEL_T) { head[q] = 0; hd[q] = head_of(q, 0u); }
     __syncthreads();
-    float mv = SNEG; int mi = -1; uint32_t mg = 0;      // the best head of this thread's groups
+    if (threadIdx.x >= 32) return;
+    const uint32_t lane = threadIdx.x;
+    // one warp: a lane's groups by their heads
+    uint32_t o = 0u, at = 0u, mg = 0u, best, row;
     auto look = [&]() {
-        mv = SNEG; mi = -1;
-        for (uint32_t q = threadIdx.x; q < groups; q += SEL_T) {
-            const uint32_t c = q * k + head[q];
-            if (head[q] < k && ci[c] >= 0 && better(cv[c], ci[c], mv, mi)) { mv = cv[c]; mi = ci[c]; mg = q; }
+        o = 0u;
+#pragma unroll 4
+        for (uint32_t q = lane; q < groups; q += 32) {
+            const uint2 h = hd[q];
+            if (h.x > o || (h.x == o && h.y < at)) { o = h.x; at = h.y; mg = q; }
         }
     };
     look();
     for (uint32_t r = 0; r < k; ++r) {
-        float bv = mv; int bi = mi;
-        block_best(bv, bi, sv, si);
-        if (bi >= 0 && bi == mi) { ++head[mg]; look(); }        // rows are unique across groups
-        if (threadIdx.x == 0) { out_v[r] = bi < 0 ? SNEG : bv; out_i[r] = bi; }
+        if (warp_best(o, at, best, row)) {
+            out_v[r] = cv[mg * k + head[mg]]; out_i[r] = (int)at;
+            hd[mg] = head_of(mg, ++head[mg]);
+            look();
+        }
+        if (best == 0u && lane == 0) { out_v[r] = SNEG; out_i[r] = -1; }
     }
-    __syncthreads();
-    if (threadIdx.x >= 32) return;
-    const uint32_t lane = threadIdx.x;
+    __syncwarp();
     uint32_t n = 0;
     for (uint32_t r = 0; r < k; ++r) if (out_i[r] >= 0) n = r + 1;
     int chosen = 0;
     if (n > 1 && temperature > 0.f) {
-        // two candidates per lane
+        // two candidates per lane; every sum in candidate order, as a sequential cumulative sum
+        __shared__ float s_p[TOPK_MAX], s_q[TOPK_MAX];
         const float l0 = out_v[0];
-        float p[2];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) { const uint32_t r = lane + 32 * h; p[h] = r < n ? expf(__fdiv_rn(out_v[r] - l0, temperature)) : 0.f; }
-        // sums in candidate order (lane 0 walks the values): the same order as a sequential cumulative sum
+        for (int h = 0; h < 2; ++h) { const uint32_t r = lane + 32 * h; s_p[r] = r < n ? expf(__fdiv_rn(out_v[r] - l0, temperature)) : 0.f; }
+        __syncwarp();
         float sum = 0.f;
-        for (uint32_t r = 0; r < n; ++r) sum += __shfl_sync(0xffffffffu, p[r >> 5], r & 31);
+#pragma unroll 8
+        for (uint32_t r = 0; r < n; ++r) sum += s_p[r];
         uint32_t keep = n;
         if (top_p < 1.0f) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) { const uint32_t r = lane + 32 * h; s_q[r] = __fdiv_rn(s_p[r], sum); }
+            __syncwarp();
             float cs = 0.f;
             for (uint32_t r = 0; r < n; ++r) {
-                cs += __fdiv_rn(__shfl_sync(0xffffffffu, p[r >> 5], r & 31), sum);
+                cs += s_q[r];
                 if (cs >= top_p) { keep = r + 1; break; }
             }
         }
         float ks = 0.f;
-        for (uint32_t r = 0; r < keep; ++r) ks += __shfl_sync(0xffffffffu, p[r >> 5], r & 31);
+#pragma unroll 8
+        for (uint32_t r = 0; r < keep; ++r) ks += s_p[r];
         const float u = sample_uniform(seed, b, (uint32_t)pos[b]);
         const float target = u * ks;
         float acc = 0.f;
         chosen = (int)keep - 1;
         for (uint32_t r = 0; r < keep; ++r) {
-            acc += __shfl_sync(0xffffffffu, p[r >> 5], r & 31);
+            acc += s_p[r];
             if (target < acc) { chosen = (int)r; break; }
         }
         if (dbg && lane == 0) { dbg[b * 4] = (float)keep; dbg[b * 4 + 1] = u; dbg[b * 4 + 2] = sum; dbg[b * 4 + 3] = (float)n; }
@@ -260,7 +304,7 @@ int launch_sample(const float* logits, uint32_t V, uint32_t batch, uint32_t k, f
         s_cand_n = need;
     }
     k_sample_stage1<<<dim3(groups, batch), SEL_T, 0, g.stream>>>(logits, V, k, pos, prompt_len, prompt_tok, gen_log, ld, penalty, on_prompt, s_cand_v, s_cand_i);
-    const size_t heads = (groups + 15) & ~(size_t)15, all = heads + (size_t)groups * k * 8;
+    const size_t heads = ((size_t)groups * 9 + 15) & ~(size_t)15, all = heads + (size_t)groups * k * 8;
     const bool in_shared = all <= 160 * 1024;           // 82 KB at a vocabulary of 262144 and k = 64
     if (cudaFuncSetAttribute(k_sample_stage2, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
         return fail(ADAMAH_ERR_BACKEND, "sampling: cannot raise the shared-memory limit");
