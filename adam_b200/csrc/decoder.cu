@@ -833,14 +833,14 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
             if (n_set < 32) set[n_set++] = kern;
         }
     }
-    // Few (sequence, head group) pairs in flight (at most 16): the position splits of a pair form one thread-block cluster of 8 CTAs and
-    // merge through shared memory (no partial results in global memory, no ticket, no last-CTA pass: 3 us less per launch at the
+    // Few (sequence, head group) pairs in flight: the position splits of a pair form one thread-block cluster -- of 8 CTAs up to 16
+    // pairs, of 4 up to 32, of 2 up to 64: one CTA per SM -- and merge through shared memory (no partial results in global memory, no ticket, no last-CTA pass: 3 us less per launch at the
     // 1B shape).  A cluster covers any context, its CTAs taking more chunks each, so layers that may attend to more than
     // 2048 positions keep the wider grid of independent splits.  (Clusters of 16 were measured slower: they start later,
     // and so does every kernel behind them.)  ADAM_B200_ATTN_CLUSTER=0 turns the path off, =16 allows clusters of 16.
     static const int cluster_env = getenv("ADAM_B200_ATTN_CLUSTER") ? atoi(getenv("ADAM_B200_ATTN_CLUSTER")) : 8;
-    static const uint32_t cluster_pairs = getenv("ADAM_B200_ATTN_CLUSTER_WORK") ? (uint32_t)atoi(getenv("ADAM_B200_ATTN_CLUSTER_WORK")) : 16u;
-    const bool cluster = cluster_env != 0 && pairs <= cluster_pairs && reach <= 2048u;
+    static const uint32_t cluster_pairs = getenv("ADAM_B200_ATTN_CLUSTER_WORK") ? (uint32_t)atoi(getenv("ADAM_B200_ATTN_CLUSTER_WORK")) : 64u;
+    const bool cluster = cluster_env != 0 && pairs <= cluster_pairs && (pairs <= 32u || pairs >= 56u) && reach <= 2048u;
     // Chunks in flight per CTA: one per warp; up to two in a cluster of splits, where a context just beyond 8 chunks per CTA (a window
     // of 512) would have a warp wait for memory a second time.  (Elsewhere CTAs without positions would hold that much, too.)
     const size_t slot_bytes = (size_t)2 * ATTN_CP * d.head_dim * sizeof(T);
@@ -848,16 +848,16 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
     const size_t smem = n_slots * slot_bytes + ((size_t)hpc * d.head_dim + 2 * (size_t)d.head_dim) * 4;
     if (cluster) {
         // clusters of a size that run at once, by kernel (0: none of that size)
-        struct Known { AttnKernel k; unsigned cs; int n; };
-        static Known known[16]; static int n_known = 0;
+        struct Known { AttnKernel k; unsigned want, cs; int n; };
+        static Known known[64]; static int n_known = 0;
+        const unsigned want = pairs > 32u ? 2u : pairs > 16u ? 4u : cluster_env == 16 ? 16u : 8u;
         const Known* kn = nullptr;
-        for (int i = 0; i < n_known; ++i) if (known[i].k == kern) kn = &known[i];
+        for (int i = 0; i < n_known; ++i) if (known[i].k == kern && known[i].want == want) kn = &known[i];
         const auto smem_for = [&](unsigned c) { return smem + (size_t)c * hpc * (d.head_dim + 4) * 4; };
-        Known fresh = {kern, 0u, 0};
+        Known fresh = {kern, want, 0u, 0};
         if (!kn) {
-            const unsigned c_max = cluster_env == 16 ? 16u : 8u;
-            if (c_max > 8 && cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) cudaGetLastError();
-            for (unsigned c = c_max; c >= 8 && !fresh.n; c >>= 1) {
+            if (want > 8 && cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) cudaGetLastError();
+            for (unsigned c = want; c >= std::min(want, 8u) && !fresh.n; c >>= 1) {
                 cudaLaunchConfig_t cfg = {};
                 cfg.gridDim = dim3(c, grid.y, 1); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = smem_for(c);
                 cudaLaunchAttribute at[1];
@@ -868,12 +868,13 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
                 if (cudaOccupancyMaxActiveClusters(&n, (const void*)kern, &cfg) != cudaSuccess) { cudaGetLastError(); continue; }
                 fresh.cs = c; fresh.n = n;
             }
-            if (n_known < 16) known[n_known++] = fresh;
+            if (n_known < 64) known[n_known++] = fresh;
             kn = &fresh;
         }
         const unsigned cs = kn->n >= (int)pairs ? kn->cs : 0u;
         if (cs > 0) {
             grid.x = cs;
+            const uint32_t cpc = cpc_env ? cpc_env : 8u;
             if (launch_k_cluster(kern, grid, dim3(256), smem_for(cs), g.stream, g.pdl, cs, true, D->qkv, qkv_ld, ly.norm[NORM_Q], ly.norm[NORM_K], d.norm_eps,
                                  D->rope_cos[which], D->rope_sin[which], D->rope_pos[which],
                                  D->kv_pool, geo, D->block_table, D->pos, d.n_head, L, window, d.attn_scale,
