@@ -1,4 +1,5 @@
-// Host-side launch logic of the tensor-core Q4_0 GEMV (kernel in gemv_mma.cuh).
+// Host-side launch logic of the tensor-core GEMV over row-tiled weights: one row whose matrix fits the registers (gemv_row.cuh), one
+// row that streams (gemv_ring.cuh), two to four rows (gemv_rows.cuh); else the kernel of gemv_mma.cuh.
 #include "gemv_mma.cuh"
 #include "gemv_row.cuh"
 #include "gemv_rows.cuh"
@@ -52,11 +53,10 @@ int launch_gemv_mma(int wt, const uint8_t* t0, const uint8_t* t1, GemvArgs a, cu
     if (gemv_ring_takes(wt, a)) return launch_gemv_ring(wt, t0, t1, a, stream);
     if (gemv_rows_takes(wt, a)) return launch_gemv_rows(wt, t0, t1, a, stream);
     const int units = a.K / 32, pairs = a.K / 64, n_rg = a.N / 16;
-    // batch rows per pass: as many of 4, 2, 1 as shared memory allows
-    // Batch rows per pass.  The passes of a launch run side by side (gridDim.x), each re-reading the weights from L2.
-    // Matrices of a few MB are bound by latency, not by bytes: there more, thinner passes (more CTAs in flight) win --
-    // measured at the 1B shape: 4 rows as 4 passes of one (0.94 against 1.41 ms per step), 8..32 rows as passes of two
-    // (batch 8: 1.21 against 1.48 ms).  Large matrices (27B shapes, LM heads) and prefill chunks keep four rows per pass.
+    // Batch rows per pass: as many of 4, 2, 1 as shared memory allows.  The passes of a launch run side by side (gridDim.x), each
+    // re-reading the weights from L2.  Matrices of a few MB that the kernels above do not take are bound by latency: there more,
+    // thinner passes (more CTAs in flight) win -- at the 1B shape 4 rows as 4 passes of one took 0.94 against 1.41 ms per step, 8
+    // rows as passes of two 1.21 against 1.48.  Large matrices (27B shapes, LM heads) and prefill chunks keep four rows per pass.
     static const int nb_env = getenv("ADAM_B200_MMA_ROWS") ? atoi(getenv("ADAM_B200_MMA_ROWS")) : 0;
     const double w_bytes = (double)a.N * a.K * 0.5625 * (pair ? 2 : 1);
     int nb_max = (nb_env == 1 || nb_env == 2 || nb_env == 4) ? nb_env : (w_bytes > 16.0e6 ? 4 : (a.B <= 4 ? 1 : (a.B <= 32 ? 2 : 4)));

@@ -1,5 +1,8 @@
 // Tensor-core variant of the Q4_0 / Q4_K dequant GEMV over row-tiled weights (tile.cu).
 //
+// What takes it: LM heads with their arg-max, two to four rows over large matrices, and shapes that the kernels of gemv_row.cuh,
+// gemv_rows.cuh and gemv_ring.cuh (same arithmetic, activations staged slice by slice) leave.
+//
 // Why tensor cores in a memory-bound GEMV: on the plain CUDA-core path the unpack
 // (one byte-permute per weight, on the half-rate integer pipe) and one FMA per weight
 // cap the kernel at about half of HBM bandwidth.  Here a 16-row x 32-weight block is

@@ -16,7 +16,7 @@ static RingKernel pick(bool pair, bool chain, int nv, int nst) {
 }
 
 struct RingShape { RingKernel k; size_t smem; };
-// Rows of at least one tile pair per slice, at most 128 values per lane (32 where the norm chain holds four vectors), beside which
+// Rows of at least two tile pairs per slice (a set of sums costs a barrier), at most 128 values per lane (32 where the norm chain holds four vectors), beside which
 // the rings fit.
 static bool ring_shape(int wt, const GemvArgs& a, RingShape* out) {
     if (a.N <= 0 || a.K <= 0 || a.B != 1 || a.N % 16 || a.K % 64 || a.epi == EPI_ARGMAX) return false;
@@ -24,7 +24,7 @@ static bool ring_shape(int wt, const GemvArgs& a, RingShape* out) {
     const void* x = a.h_in ? (const void*)a.h_in : (const void*)a.x;
     if ((uintptr_t)x & 15) return false;
     const int pairs = a.K >> 6, np = (pairs + RING_WARPS - 1) / RING_WARPS, nv = (np + 1) / 2;
-    if (pairs < RING_WARPS) return false;
+    if (pairs < 2 * RING_WARPS) return false;
     const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU, chain = a.h_in != nullptr;
     RingShape s;
     int nst = 3;

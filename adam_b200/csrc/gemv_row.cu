@@ -52,6 +52,9 @@ static bool row_shape_for(int wt, const GemvArgs& a, RowShape* out) {
         if (n_known < 32) known[n_known++] = Known{s.k, s.ks, per_sm};
     }
     if ((long long)(a.N / 16) > (long long)per_sm * g.sm_count) return false;
+    // and at most 48 warps per SM: more of them take the instructions of as many stagings (9472 x 1152, 36 warps per SM, 5.2 us by
+    // k_gemv_mma and 3.4 here; 20000 x 1024, 68 warps, 7.4 and 7.7)
+    if ((long long)(a.N / 16) * s.ks > 48ll * g.sm_count) return false;
     *out = s;
     return true;
 }

@@ -171,8 +171,8 @@ def test_q4_k_gemv_tensor_core_path(gpu, N, K, B):
 
 
 @pytest.mark.parametrize("ggml_type,N,K", [
-    (2, 16, 64), (2, 32, 192), (2, 7104, 1152), (2, 7120, 1152),       # one slice; a slice of one pair; the most CTAs of 10 slices, one more
-    (2, 48, 1280), (2, 48, 1344), (2, 160, 4096), (2, 160, 4160),      # 10 and 11 slices; 32; slices of up to four pairs
+    (2, 16, 64), (2, 32, 192), (2, 11840, 1152), (2, 11856, 1152),     # one slice; a slice of one pair; five CTAs per SM, one more
+    (2, 48, 1280), (2, 14208, 1024), (2, 14224, 1024), (2, 160, 4096), (2, 160, 4160),      # 10 slices; 48 warps per SM, more; 32 slices; slices of up to four pairs
     (2, 96, 8192), (2, 2368, 6912), (2, 2384, 6912), (2, 96, 8256),    # 32 of four; one CTA per SM and one more; too long
     (12, 16, 256), (12, 2048, 1280), (12, 48, 1536), (12, 80, 4352), (12, 80, 8192)])
 def test_one_row_gemv_edges(gpu, ggml_type, N, K):
