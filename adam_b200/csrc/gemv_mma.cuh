@@ -7,17 +7,17 @@
 // (one byte-permute per weight, on the half-rate integer pipe) and one FMA per weight
 // cap the kernel at about half of HBM bandwidth.  Here a 16-row x 32-weight block is
 // ONE integer MMA (mma.sync.m16n8k32, u8 x s8 -> s32):
-//   * weights enter as the raw nibbles 0..15 (u8): three logic ops split a 32-bit word
-//     into its four low and four high nibbles, which are exactly the A registers;
+//   * three logic ops split a 32-bit word of weights into its four low and four high nibbles,
+//     which are exactly the A registers: Q4_0 as signed bytes 16 (q - 8), so that no offset is
+//     left to subtract, Q4_K as the codes 0..15;
 //   * the activation vector is scaled by a power of two s (chosen per vector so that
 //     |x*s| <= 2^22), rounded to an integer and split into three signed bytes
 //     x*s = hi*65536 + mid*256 + lo, i.e. 23 bits of every activation are kept.  The
 //     8-wide B operand holds, for up to two batch rows, the columns (hi, mid, lo, 0);
 //   * lane (g, t) = (lane/4, lane%4) receives rows g and g+8 of column pair t: an even
 //     t sees (hi, mid), an odd t sees (lo, 0), and both form v = d0*256 + d1 in integer
-//     arithmetic (exact), convert it once, remove the -8 offset of Q4_0 with the block's
-//     pre-summed activations (kept in the same units), scale by the block scale d and
-//     accumulate in fp32.  Even and odd lanes differ by the constant factor 65536, which
+//     arithmetic (exact), convert it once, scale by the block scale d and accumulate in fp32
+//     (Q4_K: its offsets take the block's pre-summed activations, kept in the same units).  Even and odd lanes differ by the constant factor 65536, which
 //     is applied once per row group when the two are added.
 // The tensor pipe stays almost idle: the kernel is a stream over the weight bytes.
 //
@@ -40,6 +40,13 @@ namespace ab {
 // D = A(u8, 16x32) * B(s8, 32x8) with a zero accumulator input.
 __device__ __forceinline__ void imma16832(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0), "r"(0), "r"(0), "r"(0));
+}
+
+// The same with A signed: Q4_0's codes as 16 (q - 8), a nibble in a byte's upper half with its top bit flipped.
+__device__ __forceinline__ void imma16832_s(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0), "r"(0), "r"(0), "r"(0));
 }
@@ -241,7 +248,6 @@ __global__ void __launch_bounds__(512, 1) k_gemv_mma(const GemvArgs a_in, const 
     constexpr int CH = MmaGeo<PAIR, WT>::CH;
     constexpr int STAGE_BYTES = MmaGeo<PAIR, WT>::STAGE_BYTES;
     constexpr int MMA_TILE = MmaGeo<PAIR, WT>::TILE;
-    constexpr float SXF = WT == WT_Q4_0 ? -8.0f : -1.0f;    // Q4_0: d*(q-8); Q4_K: (d*sc)*q - (dmin*m)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ float s_red[2][MMA_MAX_WARPS][NM][NI][16][2];
     __shared__ __align__(8) uint64_t s_bar[MMA_MAX_WARPS][NST];
@@ -265,7 +271,7 @@ __global__ void __launch_bounds__(512, 1) k_gemv_mma(const GemvArgs a_in, const 
     // Stage = up to CH consecutive tile pairs of the warp's row group (contiguous in memory),
     // one cp.async.bulk per matrix, completion counted on the stage's mbarrier.
     signed char* xb = reinterpret_cast<signed char*>(smem_raw);                            // [units][NCOL][32]
-    float* s_sx = reinterpret_cast<float*>(smem_raw + (size_t)units * NCOL * 32);          // [units][NPR], already times -8
+    float* s_sx = reinterpret_cast<float*>(smem_raw + (size_t)units * NCOL * 32);          // [units][NPR], Q4_K only
     unsigned char* ring = smem_raw + (((size_t)units * (NCOL * 32 + NPR * 4) + 127) & ~(size_t)127) + (size_t)warp * NST * STAGE_BYTES;
     const int nch = (np + CH - 1) / CH;                     // chunks per row group for this warp
     const int n_chunks = my_sets * nch;
@@ -321,6 +327,10 @@ __global__ void __launch_bounds__(512, 1) k_gemv_mma(const GemvArgs a_in, const 
     {
         const int n4 = a.K >> 2;
         const int nj = (n4 + (int)blockDim.x - 1) / (int)blockDim.x;          // float4 per thread
+        auto put = [&](int i, int b, float4 v) {                              // called by whole warps
+            if constexpr (WT == WT_Q4_0) { if (i < n4) put_x4<NCOL>(xb, 4 * i, b, v); }
+            else put_x4_sums<NCOL>(xb, s_sx, 4 * i, b, v, i < n4, -1.0f);
+        };
         for (int b = 0; b < NBR && b < a.B; ++b) {
             const size_t row = (size_t)b * a.ldx;
             float (*rd)[32] = s_rd[b & 1];
@@ -386,7 +396,7 @@ __global__ void __launch_bounds__(512, 1) k_gemv_mma(const GemvArgs a_in, const 
                 for (int j = 0; j < 3; ++j) {
                     if (j < nj) {
                         const int i = threadIdx.x + j * blockDim.x;
-                        put_x4_sums<NCOL>(xb, s_sx, 4 * i, b, make_float4(vh[j].x * s, vh[j].y * s, vh[j].z * s, vh[j].w * s), i < n4, SXF);
+                        put(i, b, make_float4(vh[j].x * s, vh[j].y * s, vh[j].z * s, vh[j].w * s));
                     }
                 }
             } else {
@@ -410,7 +420,7 @@ __global__ void __launch_bounds__(512, 1) k_gemv_mma(const GemvArgs a_in, const 
                     for (int j = 0; j < 8; ++j) {
                         if (j < nj) {
                             const int i = threadIdx.x + j * blockDim.x;
-                            put_x4_sums<NCOL>(xb, s_sx, 4 * i, b, make_float4(v[j].x * s, v[j].y * s, v[j].z * s, v[j].w * s), i < n4, SXF);
+                            put(i, b, make_float4(v[j].x * s, v[j].y * s, v[j].z * s, v[j].w * s));
                         }
                     }
                 } else {
@@ -450,7 +460,7 @@ __global__ void __launch_bounds__(512, 1) k_gemv_mma(const GemvArgs a_in, const 
                             for (int u = 0; u < 4; ++u) {
                                 if (j0 + u < nj) {
                                     const int i = threadIdx.x + (j0 + u) * blockDim.x;
-                                    put_x4_sums<NCOL>(xb, s_sx, 4 * i, b, make_float4(v4[u].x * s, v4[u].y * s, v4[u].z * s, v4[u].w * s), i < n4, SXF);
+                                    put(i, b, make_float4(v4[u].x * s, v4[u].y * s, v4[u].z * s, v4[u].w * s));
                                 }
                             }
                         }
@@ -474,7 +484,7 @@ __global__ void __launch_bounds__(512, 1) k_gemv_mma(const GemvArgs a_in, const 
                             for (int u = 0; u < 4; ++u) {
                                 if (j0 + u < nj) {
                                     const int i = threadIdx.x + (j0 + u) * blockDim.x;
-                                    put_x4_sums<NCOL>(xb, s_sx, 4 * i, b, make_float4(v4[u].x * s, v4[u].y * s, v4[u].z * s, v4[u].w * s), i < n4, SXF);
+                                    put(i, b, make_float4(v4[u].x * s, v4[u].y * s, v4[u].z * s, v4[u].w * s));
                                 }
                             }
                         }
@@ -505,21 +515,21 @@ __global__ void __launch_bounds__(512, 1) k_gemv_mma(const GemvArgs a_in, const 
     const uint2* xq = reinterpret_cast<const uint2*>(xb) + (g % (NCOL < 8 ? NCOL : 8)) * 4 + t;
     constexpr int xstep = NCOL * 4;                            // uint2 per block
     const float* sxp = s_sx + (t % (NPR < 4 ? NPR : 4));
-    const float cm = (t & 1) ? (1.0f / 256.0f) : 256.0f;      // even lanes hold (hi, mid), odd lanes (lo, 0)
+    // even lanes hold (hi, mid), odd lanes (lo, 0); Q4_0's codes count 16
+    const float cm = ((t & 1) ? (1.0f / 256.0f) : 256.0f) * (WT == WT_Q4_0 ? 0.0625f : 1.0f);
 
     // One 16x32 block of one matrix against the staged columns.
-    auto block_imma = [&](uint32_t wg, uint32_t wh, const uint2* xu, const float* sxu, uint32_t sc2, float (&ac)[NI][2]) {
-        const uint32_t a0 = wg & 0x0F0F0F0Fu, a2 = (wg >> 4) & 0x0F0F0F0Fu;
-        const uint32_t a1 = wh & 0x0F0F0F0Fu, a3 = (wh >> 4) & 0x0F0F0F0Fu;
+    auto block_imma = [&](uint32_t wg, uint32_t wh, const uint2* xu, uint32_t sc2, float (&ac)[NI][2]) {
+        const uint32_t M = 0xF0F0F0F0u, X = 0x80808080u;
+        const uint32_t a0 = ((wg << 4) & M) ^ X, a2 = (wg & M) ^ X, a1 = ((wh << 4) & M) ^ X, a3 = (wh & M) ^ X;
         const float2 d = __half22float2(*reinterpret_cast<const __half2*>(&sc2));
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
             const uint2 b = xu[i * 32];
             int dd[4];
-            imma16832(dd, a0, a1, a2, a3, b.x, b.y);
-            const float sx = sxu[i * 4];
-            ac[i][0] = fmaf(d.x, (float)(dd[0] * 256 + dd[1]) + sx, ac[i][0]);
-            ac[i][1] = fmaf(d.y, (float)(dd[2] * 256 + dd[3]) + sx, ac[i][1]);
+            imma16832_s(dd, a0, a1, a2, a3, b.x, b.y);
+            ac[i][0] = fmaf(d.x, (float)(dd[0] * 256 + dd[1]), ac[i][0]);
+            ac[i][1] = fmaf(d.y, (float)(dd[2] * 256 + dd[3]), ac[i][1]);
         }
     };
     // Same for Q4_K: sc4 = { sc[g], m[g], sc[g+8], m[g+8] } of this block as bytes, (d, dmin) of the two rows.
@@ -548,8 +558,8 @@ __global__ void __launch_bounds__(512, 1) k_gemv_mma(const GemvArgs a_in, const 
             const uint4 q = reinterpret_cast<const uint4*>(tile)[lane];
             const uint2 sc = reinterpret_cast<const uint2*>(tile + 512)[g];
             if constexpr (WT == WT_Q4_0) {
-                block_imma(q.x, q.y, xu0, sx0, sc.x, acc[m]);
-                block_imma(q.z, q.w, xu0 + xstep, sx0 + NPR, sc.y, acc[m]);
+                block_imma(q.x, q.y, xu0, sc.x, acc[m]);
+                block_imma(q.z, q.w, xu0 + xstep, sc.y, acc[m]);
             } else {
                 const uint2 hd = reinterpret_cast<const uint2*>(tile + 576)[g];
                 const float2 dm0 = __half22float2(*reinterpret_cast<const __half2*>(&hd.x));
