@@ -4,6 +4,10 @@
 namespace ab {
 
 typedef void (*RingKernel)(const GemvArgs, const uint8_t*, const uint8_t*, float);
+// Row groups per CTA at most: beyond, the staging that this kernel saves is less than its barrier per row group costs.  us by k_gemv_mma
+// and here, cold, Q4_0 / Q4_K: 12000 x 5376 (5.1 per CTA) 14.3 and 11.4 / 16.8 and 14.8; 16000 x 5376 (6.8) 15.1 and 13.5 / 17.7
+// and 17.3; 21504 x 5376 (9.1) 18.5 and 16.8 / 21.8 and 22.9; 32768 x 5376 (13.8) 22.7 and 23.0 / 27.9 and 31.0.
+constexpr int RING_SETS = 7;
 constexpr int RING_SMEM_LIMIT = 220 * 1024;
 
 // Ring stages: three, two beside the staged form of a very long row (86 KB at K = 21504) where three do not fit.
@@ -24,7 +28,7 @@ static bool ring_shape(int wt, const GemvArgs& a, RingShape* out) {
     const void* x = a.h_in ? (const void*)a.h_in : (const void*)a.x;
     if ((uintptr_t)x & 15) return false;
     const int pairs = a.K >> 6, np = (pairs + RING_WARPS - 1) / RING_WARPS, nv = (np + 1) / 2;
-    if (pairs < 2 * RING_WARPS) return false;
+    if (pairs < 2 * RING_WARPS || a.N / 16 > RING_SETS * g.sm_count) return false;
     const bool pair = a.epi == EPI_GEGLU || a.epi == EPI_SWIGLU, chain = a.h_in != nullptr;
     RingShape s;
     int nst = 3;

@@ -4,9 +4,8 @@
 // The warps of a CTA are the K slices of one 16-row group at a time; every warp stages only the activations of its slice, with
 // a scale of its own (31 bits, four signed bytes), and its weights stream through its own ring.  k_gemv_mma stages the whole
 // vector in every CTA behind three CTA-wide reductions, and while that runs a ring takes no more than it holds (25 MB over all
-// SMs): at the 27B shape 16 of a layer's 72 us.  Here it takes 2.3 us per product: one layer 68.5 us (QKV 8.3 -> 7.3 us behind its
-// wait, o-proj 6.3 -> 3.7, gate / up 26 -> 27 with its start 2 us earlier, down 20.4 -> 17.5), a request on the 27B shape (8
-// layers) 23.9 -> 22.4 ms with the attention's splits in clusters.
+// SMs): at the 27B shape 16 of a layer's 72 us.  Here it takes 2.3 us per product (QKV 8.3 -> 7.3 us behind its wait, o-proj 6.3
+// -> 3.7, down 20.4 -> 14.5).  Matrices of many row groups per CTA stay with k_gemv_mma (gemv_ring.cu).
 #pragma once
 #include "gemv_row.cuh"
 
