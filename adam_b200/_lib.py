@@ -97,6 +97,7 @@ _SIGS = {
     "adam_b200_last_error": (c_char_p, []),
     "adam_b200_device_info": (c_int, [POINTER(c_int), POINTER(c_int), POINTER(u64)]),
     "adam_b200_kernel_launches": (u64, []),
+    "adam_b200_step_kernel_counts": (c_int, [POINTER(u64), u32]),
     "adam_b200_device_error": (u32, []),
     "adam_b200_handle_free": (c_int, [u32]),
     "adam_b200_timer_begin": (c_int, []),

@@ -390,6 +390,13 @@ class Adamah:
         self._check(self._lib.adam_b200_gemm_counts(out, len(names)), "adam_b200_gemm_counts")
         return dict(zip(names, out))
 
+    def step_kernel_counts(self) -> dict:
+        """Launches of the GEMV kernels and of the decode attention so far, by kernel (a graph's when it is recorded)."""
+        names = ("row", "ring", "rows", "mma", "blocks", "attn_splits", "attn_cluster_2", "attn_cluster_4", "attn_cluster_8", "attn_cluster_16")
+        out = (ctypes.c_uint64 * len(names))()
+        self._check(self._lib.adam_b200_step_kernel_counts(out, len(names)), "adam_b200_step_kernel_counts")
+        return dict(zip(names, out))
+
     def tc_gemm_policy(self, policy: int):
         """0 = never take the GEMM kernels, 1 = where they are expected to be faster (default), 2 = the tcgen05 one whenever the shape allows."""
         self._check(self._lib.adam_b200_tc_gemm_policy(int(policy)), "adam_b200_tc_gemm_policy")

@@ -51,6 +51,10 @@ struct Handle {
     uint32_t* shadow;      // host copy of what the host uploaded (NULL for device-produced data)
 };
 
+// Kernels of a decode step, counted by launch: the GEMVs, the decode attention as independent splits and as clusters of a size.
+enum { RAN_GEMV_ROW, RAN_GEMV_RING, RAN_GEMV_ROWS, RAN_GEMV_MMA, RAN_GEMV, RAN_ATTN_SPLITS, RAN_ATTN_CLUSTER_2, RAN_ATTN_CLUSTER_4, RAN_ATTN_CLUSTER_8,
+       RAN_ATTN_CLUSTER_16, RAN_COUNTS };
+
 struct Context {
     bool         inited;
     int          device;
@@ -67,6 +71,7 @@ struct Context {
     int          sched_mode;
     uint64_t     ticket;
     uint64_t     launches;      // kernels launched (graph nodes counted one by one)
+    uint64_t     ran[RAN_COUNTS];   // of those, by kernel
     uint64_t     submits;       // stream synchronisations that closed a batch
     uint64_t     flushes;
     uint32_t*    dev_err;       // device error word
@@ -88,6 +93,7 @@ bool hfirst(uint32_t h, uint32_t* out);
 uint32_t handle_alloc(uint32_t n_bytes);            // 0 on failure
 int  check_launch(const char* what);                // cudaGetLastError -> status
 inline void count_launch(uint64_t n = 1) { g.launches += n; }
+inline void count_ran(int kernel) { ++g.launches; ++g.ran[kernel]; }
 void end_of_op();                                   // sync when not inside a batch
 
 // Launch `k` on `st`; with `pdl` the launch may begin before the previous kernel in the

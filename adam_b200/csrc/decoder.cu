@@ -880,7 +880,7 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
                                  D->kv_pool, geo, D->block_table, D->pos, d.n_head, L, window, d.attn_scale,
                                  d.attn_softcap, D->attn_out, D->part_o, D->part_ml, D->attn_ticket, 0u, hpc | (cpc << 16), n_slots, g.dev_err STEP_TRACE_ARG((g_step_trace && L == g_step_trace_layer) ? g_step_trace + 4 * 64 : nullptr)) != cudaSuccess)
                 return fail(ADAMAH_ERR_BACKEND, "attention: cluster launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-            count_launch();
+            count_ran(cs == 2 ? RAN_ATTN_CLUSTER_2 : cs == 4 ? RAN_ATTN_CLUSTER_4 : cs == 8 ? RAN_ATTN_CLUSTER_8 : RAN_ATTN_CLUSTER_16);
             return ADAMAH_OK;
         }
     }
@@ -888,7 +888,7 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
              D->rope_cos[which], D->rope_sin[which], D->rope_pos[which],
              D->kv_pool, geo, D->block_table, D->pos, d.n_head, L, window, d.attn_scale,
              d.attn_softcap, D->attn_out, D->part_o, D->part_ml, D->attn_ticket, D->n_splits, hpc | (cpc << 16), n_slots, g.dev_err STEP_TRACE_ARG((g_step_trace && L == g_step_trace_layer) ? g_step_trace + 4 * 64 : nullptr));
-    count_launch();
+    count_ran(RAN_ATTN_SPLITS);
     return ADAMAH_OK;
 }
 

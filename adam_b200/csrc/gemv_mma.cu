@@ -166,7 +166,7 @@ int launch_gemv_mma(int wt, const uint8_t* t0, const uint8_t* t1, GemvArgs a, cu
         }
         if (launch_k(k, dim3(n_pass, grid), dim3(n_warps * 32), smem, stream, g.pdl, g1, t0, t1, KS) != cudaSuccess)
             return fail(ADAMAH_ERR_BACKEND, "gemv_mma: launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-        count_launch();
+        count_ran(RAN_GEMV_MMA);
     }
     return ADAMAH_OK;
 }

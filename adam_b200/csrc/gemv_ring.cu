@@ -60,7 +60,7 @@ int launch_gemv_ring(int wt, const uint8_t* t0, const uint8_t* t1, GemvArgs a, c
     const int n_rg = a.N / 16;
     if (launch_k(s.k, dim3(n_rg < g.sm_count ? n_rg : g.sm_count), dim3(RING_WARPS * 32), s.smem, stream, g.pdl, a, t0, t1, 1.0f / (float)a.K) != cudaSuccess)
         return fail(ADAMAH_ERR_BACKEND, "gemv_ring: launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-    count_launch();
+    count_ran(RAN_GEMV_RING);
     return ADAMAH_OK;
 }
 

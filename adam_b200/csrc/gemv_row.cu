@@ -74,7 +74,7 @@ int launch_gemv_row(int wt, const uint8_t* t0, const uint8_t* t1, GemvArgs a, cu
     }
     if (launch_k(s.k, dim3(a.N / 16, a.B), dim3(s.ks * 32), s.smem, stream, g.pdl, a, t0, t1, 1.0f / (float)a.K) != cudaSuccess)
         return fail(ADAMAH_ERR_BACKEND, "gemv_row: launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-    count_launch();
+    count_ran(RAN_GEMV_ROW);
     return ADAMAH_OK;
 }
 

@@ -70,7 +70,7 @@ int launch_gemv_rows(int wt, const uint8_t* t0, const uint8_t* t1, GemvArgs a, c
     a.err = g.dev_err;
     if (launch_k(s.k, dim3((a.N / 16 + s.rgs - 1) / s.rgs), dim3(s.ks * s.rgs * 32), s.smem, stream, g.pdl, a, t0, t1, s.ks, 1.0f / (float)a.K) != cudaSuccess)
         return fail(ADAMAH_ERR_BACKEND, "gemv_rows: launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-    count_launch();
+    count_ran(RAN_GEMV_ROWS);
     return ADAMAH_OK;
 }
 

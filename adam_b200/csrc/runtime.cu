@@ -303,6 +303,11 @@ extern "C" int adam_b200_device_info(int* device, int* sm_count, uint64_t* total
     return ADAMAH_OK;
 }
 extern "C" uint64_t adam_b200_kernel_launches(void) { return g.launches; }
+extern "C" int adam_b200_step_kernel_counts(uint64_t* out, uint32_t n) {
+    if (!out) return ADAMAH_ERR_INVALID;
+    for (uint32_t i = 0; i < n; ++i) out[i] = i < RAN_COUNTS ? g.ran[i] : 0;
+    return ADAMAH_OK;
+}
 // Reads and clears the device error word (bits: 1 = a loc fell outside its map,
 // 2 = a bounded device wait ran out, 4 = bad token id).
 extern "C" uint32_t adam_b200_device_error(void) {

@@ -224,6 +224,10 @@ int         adam_b200_device_info(int* device, int* sm_count, uint64_t* total_me
 /* Number of kernel launches (graph nodes count individually) since the last
  * adamah_stats_reset; also reported as dispatch_count by adamah_stats_get. */
 uint64_t    adam_b200_kernel_launches(void);
+/* The kernels of a decode step by launch since adamah_init, the first n of: the GEMVs for one row over a matrix that
+ * the registers hold, one row over a streamed one, two to four rows, the tensor-core GEMV of any of them, the one over GGUF blocks as
+ * they are; decode attention as independent splits, as clusters of 2, 4, 8 and 16. */
+int         adam_b200_step_kernel_counts(uint64_t* out, uint32_t n);
 
 /* Reads and clears the device error word: bit 0 = a loc fell outside its map,
  * bit 1 = a bounded device-side wait ran out, bit 2 = token id out of range.
