@@ -222,10 +222,11 @@ __device__ __forceinline__ float rcp_newton(float d) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return fmaf(r, fmaf(-d, r, 1.0f), r);
 }
-// 1 / sqrt(v), the library's approximation and one step of Newton's iteration.
+// 1 / sqrt(v), the library's approximation and one step of Newton's iteration; 0 for an infinite v, as a quotient by its root
+// would be (squares overflow long before values do).
 __device__ __forceinline__ float rsqrt_newton(float v) {
     const float r = rsqrtf(v);
-    return fmaf(0.5f * r, fmaf(-v * r, r, 1.0f), r);
+    return r == 0.f ? r : fmaf(0.5f * r, fmaf(-v * r, r, 1.0f), r);
 }
 // x / (1 + e^-z), without branches.  Below z = -80 it is x * 0 (the true factor, e^-80 and less, is nothing beside any other
 // term, and 1 + tanh is 0 there), which is NaN for an infinite x; an infinite x elsewhere keeps its sign, which div_by would lose.

@@ -1,0 +1,41 @@
+"""The kernels of a decode step at the edges of the rules that choose them; a test says which kernel it is about and sees that it ran."""
+import numpy as np
+import pytest
+
+from adam_b200 import synth
+from adam_b200.config import tiny_gemma3
+from adam_b200.engine import ADAMEngine
+from oracle.decoder import OracleDecoder, dequant_model
+
+pytestmark = pytest.mark.gpu
+
+
+def _ran(gpu, before):
+    return {k: n - before[k] for k, n in gpu.step_kernel_counts().items() if n > before[k]}
+
+
+def _model(ggml_type=2, seed=0, **kw):
+    kw = dict(dict(n_layer=2, n_embd=128, n_head=2, n_head_kv=1, head_dim=128, n_ff=128, n_vocab=256, sliding_window=0), **kw)
+    act, post = kw.pop("act", "gelu"), kw.pop("post_norms", True)
+    cfg = tiny_gemma3(**kw)
+    cfg.ffn_act = act
+    return cfg, synth.build_model(cfg, ggml_type, seed=seed, post_norms=post)
+
+
+# ---- products behind the norm chain, gate / up pairs -------------------------------------------------------------------
+
+@pytest.mark.parametrize("batch", [1, 3, 8])
+def test_rows_whose_squares_overflow(gpu, batch):
+    """x / sqrt(inf) is 0 for finite x, in every kernel that norms its input."""
+    cfg, tensors = _model(seed=3, n_layer=1)
+    tensors["blk.0.post_attention_norm.weight"] *= np.float32(1e25)
+    eng = ADAMEngine(gpu, cfg, tensors, kv_cap=16, kv_dtype="f32", max_batch=batch)
+    try:
+        eng.begin([[7]] * batch, [4] * batch)
+        with np.errstate(over="ignore"):
+            want = OracleDecoder(cfg, dequant_model(tensors), kv_cap=16).forward(7, 0)
+        eng.step(1, lm_head=True, logits=True, direct=True)
+        for b in range(batch):
+            assert np.array_equal(eng.read_logits(b), want)
+    finally:
+        eng.close()
