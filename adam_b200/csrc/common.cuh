@@ -222,6 +222,12 @@ __device__ __forceinline__ float rcp_newton(float d) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return fmaf(r, fmaf(-d, r, 1.0f), r);
 }
+// The larger value, NaN where either is one (fmaxf drops a NaN).
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
 // 1 / sqrt(v), the library's approximation and one step of Newton's iteration; 0 for an infinite v, as a quotient by its root
 // would be (squares overflow long before values do).
 __device__ __forceinline__ float rsqrt_newton(float v) {

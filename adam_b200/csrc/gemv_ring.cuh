@@ -124,11 +124,8 @@ __global__ void __launch_bounds__(RING_WARPS * 32, 1) k_gemv_ring(const GemvArgs
             if (lane == 0) s_part[1][ks] = s;
         }
     }
-    float am = 0.f;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) am = fmaxf(am, fmaxf(fmaxf(fabsf(x[j].x), fabsf(x[j].y)), fmaxf(fabsf(x[j].z), fabsf(x[j].w))));
-    const uint32_t eb = max(__reduce_max_sync(0xffffffffu, __float_as_uint(am)) >> 23, 30u);
-    const float scale = __uint_as_float((283u - eb) << 23), inv = __uint_as_float((eb - 29u) << 23);
+    float scale, inv;
+    slice_scale<30>(largest(x), scale, inv);
     GM_STAMP2(6);
     unsigned char* xs = xb + (lane >> 3) * 128 + (lane & 3) * 8 + (lane & 4);
 #pragma unroll

@@ -65,6 +65,24 @@ __device__ __forceinline__ float row_total(const float* p) {
     return (t.x + t.y) + (t.z + t.w);
 }
 
+// The largest absolute value of a lane's activations, NaN if one of them is.
+template <int NV>
+__device__ __forceinline__ float largest(const float4 (&x)[NV]) {
+    float am = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) am = max_nan(am, max_nan(max_nan(fabsf(x[j].x), fabsf(x[j].y)), max_nan(fabsf(x[j].z), fabsf(x[j].w))));
+    return am;
+}
+// The power of two that brings a slice's largest value m * 2^e, 1/2 <= m < 1, to m * 2^BITS (less for values below 2^(BITS - 126)) and
+// what undoes it.  |x|'s bits are in the values' order, infinity and NaN last: a slice that has one has no finite result,
+// whatever its integers are.
+template <int BITS>
+__device__ __forceinline__ void slice_scale(float am, float& scale, float& inv) {
+    const uint32_t eb = max(__reduce_max_sync(0xffffffffu, __float_as_uint(am)) >> 23, (uint32_t)BITS);
+    scale = __uint_as_float((253u + BITS - eb) << 23);
+    inv = __uint_as_float(eb == 255u ? 0x7FFFFFFFu : (eb - (BITS - 1)) << 23);
+}
+
 #ifdef ADAM_B200_STEP_TRACE
 // CTAs 0 to 6 stamp their own rows, row 7 has the latest stamp of any CTA.
 #define GR_STAMP(slot) do { if (threadIdx.x == 0 && blockIdx.y == 0 && a.trace) { \
@@ -207,13 +225,8 @@ __global__ void __launch_bounds__(THREADS, CTAS) k_gemv_row(const GemvArgs a, co
             if (lane == 0) s_part[1][ks] = s;
         }
     }
-    float am = 0.f;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) am = fmaxf(am, fmaxf(fmaxf(fabsf(x[j].x), fabsf(x[j].y)), fmaxf(fabsf(x[j].z), fabsf(x[j].w))));
-    // The power of two that brings the largest value m * 2^e, 1/2 <= m < 1, to m * 2^22 (2^22 and not more: the largest vector
-    // element of 2^-104 and less is left smaller).  |x|'s bits are in the values' order.
-    const uint32_t eb = max(__reduce_max_sync(0xffffffffu, __float_as_uint(am)) >> 23, 22u);
-    const float scale = __uint_as_float((275u - eb) << 23), inv = __uint_as_float((eb - 21u) << 23);
+    float scale, inv;
+    slice_scale<22>(largest(x), scale, inv);
     GR_STAMP(6);
 #pragma unroll
     for (int j = 0; j < NV; ++j) {

@@ -151,13 +151,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemv_rows(const GemvArgs a, cons
                     if (lane == 0) s_part[1][r][ks] = s;
                 }
             }
-            float am = 0.f;
-#pragma unroll
-            for (int j = 0; j < NV; ++j) am = fmaxf(am, fmaxf(fmaxf(fabsf(x[q][j].x), fabsf(x[q][j].y)), fmaxf(fabsf(x[q][j].z), fabsf(x[q][j].w))));
-            // The power of two that brings the largest value m * 2^e, 1/2 <= m < 1, to m * 2^30 (less for values below 2^-96).
-            const uint32_t eb = max(__reduce_max_sync(0xffffffffu, __float_as_uint(am)) >> 23, 30u);
-            const float scale = __uint_as_float((283u - eb) << 23);
-            if (lane == 0) s_inv[r][ks] = __uint_as_float((eb - 29u) << 23);
+            float scale, inv;
+            slice_scale<30>(largest(x[q]), scale, inv);
+            if (lane == 0) s_inv[r][ks] = inv;
             unsigned char* xs = xb + (lane >> 3) * (NR * 128) + r * 128 + (lane & 3) * 8 + (lane & 4);
 #pragma unroll
             for (int j = 0; j < NV; ++j) {

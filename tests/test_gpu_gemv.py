@@ -230,6 +230,31 @@ def test_few_row_gemv_edges(gpu, ggml_type, N, K, B):
             assert np.linalg.norm(y[b] - ref) <= 5e-7 * np.linalg.norm(xs[b]) * np.linalg.norm(W) / np.sqrt(K) * 4
 
 
+# A row's own element is at both ends of the product; kernels with K slices, rings, rows side by side.
+@pytest.mark.parametrize("ggml_type,N,K,B,policy,kernel", [
+    (2, 1152, 1152, 1, 1, "row"), (12, 2048, 1280, 1, 1, "row"), (2, 96, 8192, 1, 1, "row"), (2, 2384, 5376, 1, 1, "ring"), (12, 32, 21504, 1, 1, "ring"),
+    (2, 6912, 1152, 2, 1, "rows"), (12, 6912, 1280, 3, 1, "rows"), (2, 2368, 8192, 4, 1, "rows")])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_rows_that_are_not_finite(gpu, ggml_type, N, K, B, policy, kernel, bad):
+    """A row with an infinity or a NaN has no finite result, and the other rows have the bits that they have without it."""
+    rng = np.random.default_rng(N + B)
+    raw = (gb.random_q4_0_blocks if ggml_type == 2 else gb.random_q4_k_blocks)(rng, N, K)
+    x = rng.standard_normal((B, K), dtype=np.float32)
+    gpu.tc_gemm_policy(policy)
+    try:
+        want = _gemv(gpu, ggml_type, raw, N, K, x, tile=True)
+        for at in (0, K - 5):
+            y = x.copy()
+            y[B // 2, at] = bad
+            before = gpu.step_kernel_counts()
+            got = _gemv(gpu, ggml_type, raw, N, K, y, tile=True)
+            assert [k for k, n in gpu.step_kernel_counts().items() if n > before[k]] == [kernel]
+            others = np.arange(B) != B // 2
+            assert np.array_equal(got[others], want[others]) and not np.isfinite(got[B // 2]).any()
+    finally:
+        gpu.tc_gemm_policy(1)
+
+
 @pytest.mark.parametrize("N,K", [(5376, 5376), (512, 21504), (2048, 4096), (3, 256), (9, 768), (64, 1024)])
 def test_q4_k_gemv(gpu, N, K):
     rng = np.random.default_rng(N * 17 + K)
