@@ -228,6 +228,8 @@ __device__ __forceinline__ float max_nan(float a, float b) {
     asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
 }
+// The warp's largest of values that are not negative, NaN if one of them is: their bits are in their order, NaN last.
+__device__ __forceinline__ float warp_max_abs(float v) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v))); }
 // 1 / sqrt(v), the library's approximation and one step of Newton's iteration; 0 for an infinite v, as a quotient by its root
 // would be (squares overflow long before values do).
 __device__ __forceinline__ float rsqrt_newton(float v) {

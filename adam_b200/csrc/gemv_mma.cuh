@@ -89,34 +89,31 @@ __device__ __forceinline__ void put_x4(signed char* xb, int k0, int b, float4 v)
     *reinterpret_cast<uint32_t*>(xb + i0 + 96) = 0u;
 }
 
-// Power-of-two scale that brings amax to at most 2^22 (and its inverse).
+// Power-of-two scale that brings amax to at most 2^22 (and its inverse).  A row with an infinity or a NaN has no finite result,
+// whatever its integers are.
 __device__ __forceinline__ void pow2_scale(float amax, float& s, float& inv) {
-    if (!(amax > 0.f) || !(amax < 3.0e38f)) { s = 1.f; inv = 1.f; return; }
-    // amax = m * 2^e with m in [0.5, 1)  (denormals count as e = -126)
-    int e = (int)((__float_as_uint(amax) >> 23) & 0xFFu) - 126;
-    e = max(-100, min(100, 22 - e));
+    // amax = m * 2^e with m in [0.5, 1)  (denormals count as e = -126); 128 and more: infinity, NaN
+    const int top = (int)(__float_as_uint(amax) >> 23) - 126;
+    const int e = amax == 0.f ? 0 : max(-106, min(100, 22 - top));
     s = __uint_as_float((uint32_t)(127 + e) << 23);
-    inv = __uint_as_float((uint32_t)(127 - e) << 23);
+    inv = __uint_as_float(top > 128 ? 0x7FFFFFFFu : (uint32_t)(127 - e) << 23);
 }
 
-// Block-wide sum of `sv` and maximum of `mv` in one pass (red: 66 floats).
+// Block-wide sum of `sv` and maximum of `mv` (not negative; NaN if one is) in one pass (red: 66 floats).
 __device__ __forceinline__ void block_sum_max(float& sv, float& mv, float* red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        sv += __shfl_xor_sync(0xffffffffu, sv, o);
-        mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, o));
-    }
+    sv = warp_sum(sv);
+    mv = warp_max_abs(mv);
     __syncthreads();
     if (lane == 0) { red[warp] = sv; red[33 + warp] = mv; }
     __syncthreads();
-    float a = 0.f, m = -3.402823466e+38f;
-    for (int w = 0; w < nw; ++w) { a += red[w]; m = fmaxf(m, red[33 + w]); }
+    float a = 0.f, m = 0.f;
+    for (int w = 0; w < nw; ++w) { a += red[w]; m = max_nan(m, red[33 + w]); }
     sv = a; mv = m;
 }
 
 // CTA-wide reductions with ONE barrier each: warp results go to `buf` (32 floats that no other reduction in
-// flight uses), every warp then folds them itself.
+// flight uses), every warp then folds them itself.  Maxima: of values that are not negative, NaN if one is.
 __device__ __forceinline__ float cta_sum1(float v, float* buf) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
     v = warp_sum(v);
@@ -126,26 +123,19 @@ __device__ __forceinline__ float cta_sum1(float v, float* buf) {
 }
 __device__ __forceinline__ float cta_max1(float v, float* buf) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    v = warp_max(v);
+    v = warp_max_abs(v);
     if (lane == 0) buf[warp] = v;
     __syncthreads();
-    return warp_max(lane < nw ? buf[lane] : -3.402823466e+38f);
+    return warp_max_abs(lane < nw ? buf[lane] : 0.f);
 }
 __device__ __forceinline__ void cta_sum_max1(float& sv, float& mv, float* bs, float* bm) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        sv += __shfl_xor_sync(0xffffffffu, sv, o);
-        mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, o));
-    }
+    sv = warp_sum(sv);
+    mv = warp_max_abs(mv);
     if (lane == 0) { bs[warp] = sv; bm[warp] = mv; }
     __syncthreads();
-    sv = lane < nw ? bs[lane] : 0.f; mv = lane < nw ? bm[lane] : -3.402823466e+38f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        sv += __shfl_xor_sync(0xffffffffu, sv, o);
-        mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, o));
-    }
+    sv = warp_sum(lane < nw ? bs[lane] : 0.f);
+    mv = warp_max_abs(lane < nw ? bm[lane] : 0.f);
 }
 
 // put_x4 plus the block's pre-summed columns: the eight lanes that hold the 32 activations of one block add
@@ -369,7 +359,7 @@ __global__ void __launch_bounds__(512, 1) k_gemv_mma(const GemvArgs a_in, const 
                             } else { vh[j].x += va[j].x; vh[j].y += va[j].y; vh[j].z += va[j].z; vh[j].w += va[j].w; }
                         }
                         ss = fmaf(vh[j].x, vh[j].x, ss); ss = fmaf(vh[j].y, vh[j].y, ss); ss = fmaf(vh[j].z, vh[j].z, ss); ss = fmaf(vh[j].w, vh[j].w, ss);
-                        am = fmaxf(am, fmaxf(fmaxf(fabsf(vh[j].x * vw[j].x), fabsf(vh[j].y * vw[j].y)), fmaxf(fabsf(vh[j].z * vw[j].z), fabsf(vh[j].w * vw[j].w))));
+                        am = max_nan(am, max_nan(max_nan(fabsf(vh[j].x * vw[j].x), fabsf(vh[j].y * vw[j].y)), max_nan(fabsf(vh[j].z * vw[j].z), fabsf(vh[j].w * vw[j].w))));
                         const int i = threadIdx.x + j * blockDim.x;
                         if (i < n4 && a.h_out && bx == 0) reinterpret_cast<float4*>(a.h_out + row)[i] = vh[j];
                     }
@@ -413,7 +403,7 @@ __global__ void __launch_bounds__(512, 1) k_gemv_mma(const GemvArgs a_in, const 
                     }
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
-                        if (j < nj) am = fmaxf(am, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
+                        if (j < nj) am = max_nan(am, max_nan(max_nan(fabsf(v[j].x), fabsf(v[j].y)), max_nan(fabsf(v[j].z), fabsf(v[j].w))));
                     am = cta_max1(am, rd[0]);
                     pow2_scale(am, s, inv);
 #pragma unroll
@@ -442,7 +432,7 @@ __global__ void __launch_bounds__(512, 1) k_gemv_mma(const GemvArgs a_in, const 
 #pragma unroll 4
                         for (int i = threadIdx.x; i < n4; i += blockDim.x) {
                             const float4 v = park[i];
-                            am = fmaxf(am, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+                            am = max_nan(am, max_nan(max_nan(fabsf(v.x), fabsf(v.y)), max_nan(fabsf(v.z), fabsf(v.w))));
                         }
                         am = cta_max1(am, rd[0]);
                         GM_STAMP(6);
@@ -468,7 +458,7 @@ __global__ void __launch_bounds__(512, 1) k_gemv_mma(const GemvArgs a_in, const 
 #pragma unroll 4
                         for (int i = threadIdx.x; i < n4; i += blockDim.x) {
                             const float4 v = src[i];
-                            am = fmaxf(am, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+                            am = max_nan(am, max_nan(max_nan(fabsf(v.x), fabsf(v.y)), max_nan(fabsf(v.z), fabsf(v.w))));
                         }
                         am = cta_max1(am, rd[0]);
                         pow2_scale(am, s, inv);

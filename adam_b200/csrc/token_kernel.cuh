@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(TK_THREADS, 1) k_token(const __grid_constant__
             if (stage) {
                 const float4 vw = i == tid ? vw_first : (w_pre ? reinterpret_cast<const float4*>(w_pre)[i] : one4);
                 ss = fmaf(vh.x, vh.x, ss); ss = fmaf(vh.y, vh.y, ss); ss = fmaf(vh.z, vh.z, ss); ss = fmaf(vh.w, vh.w, ss);
-                am = fmaxf(am, fmaxf(fmaxf(fabsf(vh.x * vw.x), fabsf(vh.y * vw.y)), fmaxf(fabsf(vh.z * vw.z), fabsf(vh.w * vw.w))));
+                am = max_nan(am, max_nan(max_nan(fabsf(vh.x * vw.x), fabsf(vh.y * vw.y)), max_nan(fabsf(vh.z * vw.z), fabsf(vh.w * vw.w))));
             }
         }
         if (!stage) { __syncthreads(); return; }             // s_a may be rewritten by the next gather
@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(TK_THREADS, 1) k_token(const __grid_constant__
 #pragma unroll
                 for (int k = 0; k < 16; ++k) {
                     const int idx = lane + 32 * k;
-                    if (idx < nv) { saw[idx] = val[k]; am = fmaxf(am, fabsf(val[k])); }
+                    if (idx < nv) { saw[idx] = val[k]; am = max_nan(am, fabsf(val[k])); }
                 }
             } else {
                 constexpr int HSH = HD == 32 ? 5 : HD == 64 ? 6 : HD == 128 ? 7 : 8;
@@ -586,12 +586,12 @@ __global__ void __launch_bounds__(TK_THREADS, 1) k_token(const __grid_constant__
                         }
                         const float x = num / den;
                         saw[q * 64 + lane + 32 * k] = x;
-                        am = fmaxf(am, fabsf(x));
+                        am = max_nan(am, fabsf(x));
                     }
                 }
             }
             __syncwarp();
-            am = warp_max(am);
+            am = warp_max_abs(am);
             float sc;
             pow2_scale(am, sc, inv);
 #pragma unroll 1

@@ -230,10 +230,11 @@ def test_few_row_gemv_edges(gpu, ggml_type, N, K, B):
             assert np.linalg.norm(y[b] - ref) <= 5e-7 * np.linalg.norm(xs[b]) * np.linalg.norm(W) / np.sqrt(K) * 4
 
 
-# A row's own element is at both ends of the product; kernels with K slices, rings, rows side by side.
+# A row's own element is at both ends of the product; kernels with K slices, rings, rows side by side, and one scale per row.
 @pytest.mark.parametrize("ggml_type,N,K,B,policy,kernel", [
     (2, 1152, 1152, 1, 1, "row"), (12, 2048, 1280, 1, 1, "row"), (2, 96, 8192, 1, 1, "row"), (2, 2384, 5376, 1, 1, "ring"), (12, 32, 21504, 1, 1, "ring"),
-    (2, 6912, 1152, 2, 1, "rows"), (12, 6912, 1280, 3, 1, "rows"), (2, 2368, 8192, 4, 1, "rows")])
+    (2, 6912, 1152, 2, 1, "rows"), (12, 6912, 1280, 3, 1, "rows"), (2, 2368, 8192, 4, 1, "rows"),
+    (2, 20000, 1024, 1, 1, "mma"), (2, 16, 24640, 1, 1, "mma"), (12, 96, 8448, 3, 0, "mma"), (2, 1152, 1152, 5, 0, "mma")])
 @pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
 def test_rows_that_are_not_finite(gpu, ggml_type, N, K, B, policy, kernel, bad):
     """A row with an infinity or a NaN has no finite result, and the other rows have the bits that they have without it."""
@@ -251,6 +252,27 @@ def test_rows_that_are_not_finite(gpu, ggml_type, N, K, B, policy, kernel, bad):
             assert [k for k, n in gpu.step_kernel_counts().items() if n > before[k]] == [kernel]
             others = np.arange(B) != B // 2
             assert np.array_equal(got[others], want[others]) and not np.isfinite(got[B // 2]).any()
+    finally:
+        gpu.tc_gemm_policy(1)
+
+
+@pytest.mark.parametrize("N,K,B,policy,kernel", [(1152, 1152, 1, 1, "row"), (2384, 5376, 1, 1, "ring"), (6912, 1152, 3, 1, "rows"),
+                                                 (20000, 1024, 1, 1, "mma"), (16, 24640, 1, 1, "mma"), (1152, 1152, 5, 0, "mma")])
+@pytest.mark.parametrize("top", [1e36, 1e37, 3.3e38])
+def test_rows_near_the_end_of_fp32(gpu, N, K, B, policy, kernel, top):
+    """Activations up to `top`, finite results: the bound of the same products of ordinary rows."""
+    rng = np.random.default_rng(N)
+    raw = gb.random_q4_0_blocks(rng, N, K)
+    W = q4_blocks.dequant(raw.reshape(-1), 2, N, K).astype(np.float64)
+    x = rng.standard_normal((B, K))
+    x = (x * (top / np.abs(x).max())).astype(np.float32)
+    gpu.tc_gemm_policy(policy)
+    try:
+        before = gpu.step_kernel_counts()
+        y = _gemv(gpu, 2, raw, N, K, x, tile=True).astype(np.float64) / top
+        assert [k for k, n in gpu.step_kernel_counts().items() if n > before[k]] == [kernel]
+        ref = (x.astype(np.float64) / top) @ W.T
+        assert np.linalg.norm(y - ref) <= 4e-6 * np.linalg.norm(x.astype(np.float64) / top) * np.linalg.norm(W) / np.sqrt(K)
     finally:
         gpu.tc_gemm_policy(1)
 
