@@ -325,8 +325,8 @@ __global__ void __launch_bounds__(256) k_attention(const float* __restrict__ qkv
     float* s_vn = s_kn + hd;                    // [hd] newest value (as stored)
     float* s_cp = s_vn + hd;                    // cluster merge, CTA 0 only: [split][gs * hd + 4 * gs] (16-byte aligned rows)
     // Rows of chunk c: keys (kv = 0), values (1) or both (2).  A chunk whose rows are all there and consecutive is one copy,
-    // otherwise a lane fetches a row each.  Positions outside [start, seq) then read the nearest valid row instead (their
-    // scores are masked later, but what an earlier sequence left there need not be finite).
+    // otherwise a lane fetches a row each.  Positions outside [start, seq) then read the nearest row inside; their scores and value
+    // rows are masked later.
     const bool whole = geo.page % CP == 0;
     auto request = [&](uint32_t c, uint32_t kv, uint32_t slot) {
         const uint32_t j = lane % CP, k = kv == 2 ? lane / CP : kv;
@@ -506,6 +506,15 @@ __global__ void __launch_bounds__(256) k_attention(const float* __restrict__ qkv
         }
         if (!landed(slot, 1, extra ? 0u : ph)) break;
         if (c == c_new) { row.from_float(s_vn + lane * DPL); row.store(reinterpret_cast<T*>(s_kv + (CP + jn) * ROWB) + lane * DPL); }
+        // Value rows outside [start, seq) count with probability 0, and 0 times what stands there (an earlier sequence's infinities) need
+        // not be 0.  The fence: a bulk copy writes the slot next.
+        if (c * CP < start || c * CP + CP > seq) {
+            row.zero();
+#pragma unroll
+            for (int j = 0; j < CP; ++j)
+                if (c * CP + j < start || c * CP + j >= seq) row.store(reinterpret_cast<T*>(s_kv + (CP + j) * ROWB) + lane * DPL);
+            if (late) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
 #pragma unroll
         for (int j = 0; j < CP; ++j) {
             float vf[DPL];

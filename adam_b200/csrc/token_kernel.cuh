@@ -809,6 +809,10 @@ __global__ void __launch_bounds__(TK_THREADS, 1) k_token(const __grid_constant__
 #pragma unroll
                 for (int j = 0; j < CP; ++j) if (j == jn) { kr[j] = nk; vr[j] = nv; }
             }
+            if (c * CP < sp.start || c * CP + CP > seq) {        // probability 0 times whatever an earlier sequence left there need not be 0
+#pragma unroll
+                for (int j = 0; j < CP; ++j) if (c * CP + j < sp.start || c * CP + j >= seq) vr[j].zero();
+            }
             float sc[CP];
 #pragma unroll
             for (int j = 0; j < CP; ++j) {

@@ -2,6 +2,7 @@
 import numpy as np
 import pytest
 
+from adam_b200 import gguf_blocks as gb
 from adam_b200 import synth
 from adam_b200.config import tiny_gemma3
 from adam_b200.engine import ADAMEngine
@@ -39,3 +40,35 @@ def test_rows_whose_squares_overflow(gpu, batch):
             assert np.array_equal(eng.read_logits(b), want)
     finally:
         eng.close()
+
+
+# ---- attention ---------------------------------------------------------------------------------------------------------
+
+def _overflowing(n_layer):
+    """A model whose token 5 has values in the first layer that fp16 does not hold, and whose other tokens do not: dimension 0 is
+    nothing in their embeddings."""
+    cfg, tensors = _model(seed=9, n_layer=n_layer)
+    raw = tensors["token_embd.weight"].raw.reshape(cfg.n_vocab, -1, gb.Q4_0_BYTES)
+    raw[:, 0, 2] = (raw[:, 0, 2] & 0xF0) | 8                    # the code of weight 0: zero
+    raw[5, 0, 2] = (raw[5, 0, 2] & 0xF0) | 15
+    tensors["blk.0.attn_norm.weight"][0] = 1e9
+    return cfg, tensors
+
+
+@pytest.mark.parametrize("single_launch", [False, True])
+def test_pages_of_a_sequence_that_was_not_finite(gpu, single_launch):
+    """What an earlier sequence left behind the newest position does not count."""
+    cfg, tensors = _overflowing(2)
+    toks = synth.random_prompt(cfg.n_vocab, 70, seed=1)
+    toks[toks == 5] = 6
+    outs = []
+    for first in ([], [5] * 80):
+        eng = ADAMEngine(gpu, cfg, tensors, kv_cap=96, kv_dtype="f16", single_launch=single_launch)
+        try:
+            if first:
+                eng.begin([first], [len(first)])
+                eng.step(len(first), lm_head=False)
+            outs.append(eng.logits_trace(toks, by_steps=True))
+        finally:
+            eng.close()
+    assert np.isfinite(outs[0]).all() and np.array_equal(outs[0], outs[1])
