@@ -236,11 +236,17 @@ __device__ __forceinline__ float rsqrt_newton(float v) {
     const float r = rsqrtf(v);
     return r == 0.f ? r : fmaf(0.5f * r, fmaf(-v * r, r, 1.0f), r);
 }
+// x / d with r = rcp_newton(d): an infinite x stays one (div_by makes it a NaN).
+__device__ __forceinline__ float quotient(float x, float d, float r) { return fabsf(x) <= 3.402823466e+38f ? div_by(x, d, r) : x * r; }
+__device__ __forceinline__ float4 quotient4(float4 num, float d) {
+    const float r = rcp_newton(d);
+    return make_float4(quotient(num.x, d, r), quotient(num.y, d, r), quotient(num.z, d, r), quotient(num.w, d, r));
+}
 // x / (1 + e^-z), without branches.  Below z = -80 it is x * 0 (the true factor, e^-80 and less, is nothing beside any other
 // term, and 1 + tanh is 0 there), which is NaN for an infinite x; an infinite x elsewhere keeps its sign, which div_by would lose.
 __device__ __forceinline__ float gated(float x, float z) {
     const float d = 1.0f + expf(-fmaxf(z, -80.f)), r = rcp_newton(d);
-    const float q = fabsf(x) <= 3.402823466e+38f ? div_by(x, d, r) : x * r;
+    const float q = quotient(x, d, r);
     return z < -80.f ? x * 0.f : q;
 }
 // GELU in its tanh form (tests/diagnostics/diag_inference.py:941-943), 0.5 x (1 + tanh u), written as x / (1 + e^-2u): the

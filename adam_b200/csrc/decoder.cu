@@ -603,8 +603,7 @@ __global__ void __launch_bounds__(256) k_attention(const float* __restrict__ qkv
             L = fmaf(ww, s_l[w][g], L);
         }
         if (n_act == 1) {
-            const float r = rcp_newton(L);
-            reinterpret_cast<float4*>(orow)[i4] = make_float4(div_by(v.x, L, r), div_by(v.y, L, r), div_by(v.z, L, r), div_by(v.w, L, r));
+            reinterpret_cast<float4*>(orow)[i4] = quotient4(v, L);
         }
         else if (cmerge) {
             if (split != 0) {
@@ -634,14 +633,16 @@ __global__ void __launch_bounds__(256) k_attention(const float* __restrict__ qkv
                     num.x *= a0; num.y *= a0; num.z *= a0; num.w *= a0; den *= a0;
 #pragma unroll
                     for (int k = 0; k < 7; ++k) {
-                        const float w = s0 + k < n_act ? expf(ml[k].x - Mn) : 0.f;
-                        num.x = fmaf(w, x[k].x, num.x); num.y = fmaf(w, x[k].y, num.y); num.z = fmaf(w, x[k].z, num.z); num.w = fmaf(w, x[k].w, num.w);
-                        den = fmaf(w, ml[k].y, den);
+                        // (a weight of 0 for the repeated ones would make NaN of an infinity)
+                        const bool in = s0 + k < n_act;
+                        const float w = expf(ml[k].x - Mn);
+                        num.x = in ? fmaf(w, x[k].x, num.x) : num.x; num.y = in ? fmaf(w, x[k].y, num.y) : num.y;
+                        num.z = in ? fmaf(w, x[k].z, num.z) : num.z; num.w = in ? fmaf(w, x[k].w, num.w) : num.w;
+                        den = in ? fmaf(w, ml[k].y, den) : den;
                     }
                     M = Mn;
                 }
-                const float r = rcp_newton(den);
-                reinterpret_cast<float4*>(orow)[i4] = make_float4(div_by(num.x, den, r), div_by(num.y, den, r), div_by(num.z, den, r), div_by(num.w, den, r));
+                reinterpret_cast<float4*>(orow)[i4] = quotient4(num, den);
             }
         } else {
             reinterpret_cast<float4*>(po)[i4] = v;
@@ -691,8 +692,7 @@ __global__ void __launch_bounds__(256) k_attention(const float* __restrict__ qkv
             }
             M = Mn;
         }
-        const float r = rcp_newton(den);
-        reinterpret_cast<float4*>(orow)[i4] = make_float4(div_by(num.x, den, r), div_by(num.y, den, r), div_by(num.z, den, r), div_by(num.w, den, r));
+        reinterpret_cast<float4*>(orow)[i4] = quotient4(num, den);
     }
     AT_STAMP(7);
     if (tid == 0) *tkt = 0u;

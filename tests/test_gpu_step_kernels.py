@@ -72,3 +72,28 @@ def test_pages_of_a_sequence_that_was_not_finite(gpu, single_launch):
         finally:
             eng.close()
     assert np.isfinite(outs[0]).all() and np.array_equal(outs[0], outs[1])
+
+
+# One split, a cluster's two splits, the independent splits of many sequences.
+@pytest.mark.parametrize("before,batch", [(3, 1), (150, 1), (150, 40)])
+def test_values_beyond_fp16_are_infinite(gpu, before, batch):
+    """The newest position's value row holds infinities: so does the attention's output, there and with their signs."""
+    cfg, tensors = _overflowing(1)
+    toks = synth.random_prompt(cfg.n_vocab, before, seed=2)
+    toks[toks == 5] = 6
+    prompt = list(toks) + [5]
+    eng = ADAMEngine(gpu, cfg, tensors, kv_cap=256, kv_dtype="f16", max_batch=batch)
+    try:
+        eng.begin([prompt] * batch, [len(prompt) + 1] * batch)
+        eng.step(before, lm_head=False, direct=True)
+        eng.step(1, lm_head=False, direct=True)
+        q_dim, hd = cfg.n_head * cfg.head_dim, cfg.head_dim
+        for b in {0, batch - 1}:
+            v = eng.read_buffer(2, q_dim + 2 * hd, b)[q_dim + hd:]
+            want = np.where(np.abs(v) >= 65520.0, np.copysign(np.inf, v), 0.0)
+            got = eng.read_buffer(4, q_dim, b).reshape(cfg.n_head, hd)
+            assert np.isinf(want).any() and not np.isnan(got).any()
+            for h in got:
+                assert np.array_equal(np.where(np.isinf(h), h, 0.0), want)
+    finally:
+        eng.close()
