@@ -812,7 +812,7 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
     // head are then read once instead of once per query head).
     static const uint32_t hpc_env = getenv("ADAM_B200_ATTN_HPC") ? (uint32_t)atoi(getenv("ADAM_B200_ATTN_HPC")) : 0u;
     const uint32_t work = batch * d.n_head;                    // CTAs per position split with one head each
-    const uint32_t hpc_auto = work <= 12u ? 1u : (work <= 32u ? (gs >= 2u ? 2u : 1u) : gs);
+    const uint32_t hpc_auto = work <= 12u ? 1u : (work <= 32u ? (gs % 2u == 0u ? 2u : 1u) : gs);       // a divisor of the group
     const uint32_t hpc = (hpc_env && gs % hpc_env == 0 && hpc_env <= 8u) ? hpc_env : hpc_auto;
     const uint32_t window = ((d.flags & 1u) && d.sliding_window > 0 && !is_global_layer(d, L)) ? d.sliding_window : 0;
     const int which = is_global_layer(d, L) ? 1 : 0;

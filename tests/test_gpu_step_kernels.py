@@ -44,6 +44,31 @@ def test_rows_whose_squares_overflow(gpu, batch):
 
 # ---- attention ---------------------------------------------------------------------------------------------------------
 
+# Groups of three, five and seven query heads.
+@pytest.mark.parametrize("head_dim,n_head,n_kv,window,page,batch,length,kv_dtype,kernel", [
+    (32, 3, 1, 0, 64, 6, 200, "f32", "attn_cluster_4"), (64, 5, 1, 0, 64, 5, 90, "f16", "attn_cluster_4"),
+    (32, 6, 2, 0, 64, 4, 150, "f32", "attn_cluster_4"), (128, 7, 1, 0, 64, 2, 200, "f32", "attn_cluster_8")])
+def test_attention_of_a_step(gpu, head_dim, n_head, n_kv, window, page, batch, length, kv_dtype, kernel):
+    """The logits of a step behind prompts are those of the prompt kernels.  f32 cache: 2e-5 (both sides sum in fp32, in different
+    orders); f16: a last-bit difference can move a cached value by one f16 step."""
+    cfg, tensors = _model(seed=length, n_head=n_head, n_head_kv=n_kv, head_dim=head_dim, sliding_window=window)
+    prompts = [synth.random_prompt(cfg.n_vocab, max(2, length - 3 * b), seed=70 + b) for b in range(batch)]
+    eng = ADAMEngine(gpu, cfg, tensors, kv_cap=length + 8, kv_dtype=kv_dtype, max_batch=batch, window=window > 0, page_size=page)
+    try:
+        eng.begin(prompts, [len(p) + 2 for p in prompts])
+        eng.prefill_prompts(prompts, 0)
+        before = gpu.step_kernel_counts()
+        eng.step(1, lm_head=True, logits=True, direct=True)
+        assert {k: n for k, n in _ran(gpu, before).items() if k.startswith("attn")} == {kernel: cfg.n_layer}
+        got = {b: eng.read_logits(b) for b in sorted({0, 1 % batch, batch // 3, batch // 2, batch - 1})}
+        for b, g in got.items():
+            want = eng.logits_trace(prompts[b])[-1]
+            assert np.abs(g - want).max() <= (1e-3 if kv_dtype == "f16" else 2e-5) * np.abs(want).max(), b
+        assert gpu.device_error() == 0
+    finally:
+        eng.close()
+
+
 def _overflowing(n_layer):
     """A model whose token 5 has values in the first layer that fp16 does not hold, and whose other tokens do not: dimension 0 is
     nothing in their embeddings."""
