@@ -856,14 +856,14 @@ static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
     const uint32_t n_slots = cluster ? (uint32_t)std::min<size_t>(16, std::max<size_t>(8, (192u << 10) / slot_bytes)) : 8u;
     const size_t smem = n_slots * slot_bytes + ((size_t)hpc * d.head_dim + 2 * (size_t)d.head_dim) * 4;
     if (cluster) {
-        // clusters of a size that run at once, by kernel (0: none of that size)
-        struct Known { AttnKernel k; unsigned want, cs; int n; };
+        // clusters of a size that run at once, by kernel and shared memory, which the heads per CTA change (0: none of that size)
+        struct Known { AttnKernel k; size_t smem; unsigned want, cs; int n; };
         static Known known[64]; static int n_known = 0;
         const unsigned want = pairs > 32u ? 2u : pairs > 16u ? 4u : cluster_env == 16 ? 16u : 8u;
         const Known* kn = nullptr;
-        for (int i = 0; i < n_known; ++i) if (known[i].k == kern && known[i].want == want) kn = &known[i];
+        for (int i = 0; i < n_known; ++i) if (known[i].k == kern && known[i].smem == smem && known[i].want == want) kn = &known[i];
         const auto smem_for = [&](unsigned c) { return smem + (size_t)c * hpc * (d.head_dim + 4) * 4; };
-        Known fresh = {kern, want, 0u, 0};
+        Known fresh = {kern, smem, want, 0u, 0};
         if (!kn) {
             if (want > 8 && cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) cudaGetLastError();
             for (unsigned c = want; c >= std::min(want, 8u) && !fresh.n; c >>= 1) {

@@ -44,8 +44,9 @@ def test_rows_whose_squares_overflow(gpu, batch):
 
 # ---- attention ---------------------------------------------------------------------------------------------------------
 
-# Groups of three, five and seven query heads.
+# Groups of three, five and seven query heads; two groups that share a kernel and differ in shared memory, one behind the other.
 @pytest.mark.parametrize("head_dim,n_head,n_kv,window,page,batch,length,kv_dtype,kernel", [
+    (256, 5, 1, 0, 64, 20, 90, "f32", "attn_cluster_4"), (256, 6, 1, 0, 64, 20, 90, "f32", None),
     (32, 3, 1, 0, 64, 6, 200, "f32", "attn_cluster_4"), (64, 5, 1, 0, 64, 5, 90, "f16", "attn_cluster_4"),
     (32, 6, 2, 0, 64, 4, 150, "f32", "attn_cluster_4"), (128, 7, 1, 0, 64, 2, 200, "f32", "attn_cluster_8")])
 def test_attention_of_a_step(gpu, head_dim, n_head, n_kv, window, page, batch, length, kv_dtype, kernel):
@@ -59,7 +60,7 @@ def test_attention_of_a_step(gpu, head_dim, n_head, n_kv, window, page, batch, l
         eng.prefill_prompts(prompts, 0)
         before = gpu.step_kernel_counts()
         eng.step(1, lm_head=True, logits=True, direct=True)
-        assert {k: n for k, n in _ran(gpu, before).items() if k.startswith("attn")} == {kernel: cfg.n_layer}
+        assert kernel is None or {k: n for k, n in _ran(gpu, before).items() if k.startswith("attn")} == {kernel: cfg.n_layer}
         got = {b: eng.read_logits(b) for b in sorted({0, 1 % batch, batch // 3, batch // 2, batch - 1})}
         for b, g in got.items():
             want = eng.logits_trace(prompts[b])[-1]
