@@ -125,6 +125,7 @@ _SIGS = {
     "adam_b200_tc_gemm_count": (ctypes.c_uint64, []),
     "adam_b200_gemm_counts": (c_int, [POINTER(u64), u32]),
     "adam_b200_few_rows_shape": (c_int, [u32, u32, u32, u32, u32, u32, POINTER(u32)]),
+    "adam_b200_attention_shape": (c_int, [u32, u32, u32, u32, u32, u32, POINTER(u32)]),
     "adam_b200_tc_gemm_policy": (c_int, [c_int]),
     "adam_b200_decoder_n_parts": (c_int, [u32]),
     "adam_b200_decoder_prefill_part": (c_int, [u32, u32, u32]),

@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 namespace ab {
@@ -800,104 +801,120 @@ static AttnKernel pick_attn_hd(uint32_t hd) {
     }
 }
 
-template <typename T>
-static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
-    const adam_b200_decoder_desc& d = D->d;
-    KvGeom geo{d.n_layer, d.n_head_kv, d.head_dim, d.page_size, D->max_pages_per_seq, D->page_elems};
-    const uint32_t gs = d.n_head / d.n_head_kv;
+// Launch shape of a decode attention.
+struct AttnShape {
+    uint32_t gs, hpc, work, pairs;      // query heads per kv head and per CTA; (sequence, head), (sequence, head group) pairs
+    uint32_t cluster;                   // CTAs of a cluster of position splits; 0: independent splits, 8 slots each
+    uint32_t slots;                     // chunks in flight per CTA of a cluster
+    size_t smem, smem_cluster;          // of a CTA of independent splits, of a cluster
+};
+static AttnShape attn_shape(uint32_t n_head, uint32_t n_kv, uint32_t head_dim, uint32_t kv_bytes, uint32_t batch, uint32_t reach, uint32_t most = 16) {
+    AttnShape s = {};
+    s.gs = n_head / n_kv;
     // Query heads per CTA: one while that still leaves SMs idle (lowest latency; the CTAs
     // of a kv head re-read its rows from L2), the whole group once the grid is large.
     // Measured at the 1B shape (4 query heads on 1 kv head): up to three sequences are fastest with a CTA per query head, eight
     // sequences with two heads per CTA, 16 or more sequences and prefill chunks with the whole group per CTA (the rows of a kv
     // head are then read once instead of once per query head).
     static const uint32_t hpc_env = getenv("ADAM_B200_ATTN_HPC") ? (uint32_t)atoi(getenv("ADAM_B200_ATTN_HPC")) : 0u;
-    const uint32_t work = batch * d.n_head;                    // CTAs per position split with one head each
-    const uint32_t hpc_auto = work <= 12u ? 1u : (work <= 32u ? (gs % 2u == 0u ? 2u : 1u) : gs);       // a divisor of the group
-    const uint32_t hpc = (hpc_env && gs % hpc_env == 0 && hpc_env <= 8u) ? hpc_env : hpc_auto;
-    const uint32_t window = ((d.flags & 1u) && d.sliding_window > 0 && !is_global_layer(d, L)) ? d.sliding_window : 0;
-    const int which = is_global_layer(d, L) ? 1 : 0;
-    const Layer& ly = D->layers[L];
-    const uint32_t qkv_ld = (d.n_head + 2 * d.n_head_kv) * d.head_dim;
-    dim3 grid(D->n_splits, d.n_head_kv * (gs / hpc), batch);
-    // Chunks of 8 positions a CTA takes before another CTA joins: with few (sequence, head) pairs the SMs are idle and a
-    // CTA's chain of dependent chunk loads is the attention's whole time, so the positions are spread thinly (one chunk
-    // per warp); with many pairs the grid is full anyway and every extra CTA only repeats the query prologue.
-    static const uint32_t cpc_env = getenv("ADAM_B200_ATTN_CPC") ? (uint32_t)atoi(getenv("ADAM_B200_ATTN_CPC")) : 0u;
-    const uint32_t pairs = grid.y * grid.z;
-    const uint32_t cpc = cpc_env ? cpc_env : (work <= 64u ? 8u : ATTN_CHUNKS_PER_CTA);
-    // Position splits launched: no more than this layer can reach (a split without positions still costs a CTA its start and the
-    // read of the position: 15 of 16 CTAs of the 27B shape's 64 sequences, 60 of the launch's 75 us), and no more than four
-    // CTAs per SM in all -- beyond that the pairs alone fill the GPU and a CTA takes more chunks instead.
-    const uint32_t reach = window ? (window < d.kv_cap ? window : d.kv_cap) : d.kv_cap;
-    const uint32_t useful = ((reach + ATTN_CP - 1) / ATTN_CP + 1 + cpc - 1) / cpc, fill = (4u * (uint32_t)g.sm_count + pairs - 1) / pairs;
-    grid.x = std::min(D->n_splits, std::min(useful, fill));
-    AttnKernel kern = hpc <= 1 ? pick_attn_hd<T, 1>(d.head_dim) : hpc <= 2 ? pick_attn_hd<T, 2>(d.head_dim)
-                    : hpc <= 4 ? pick_attn_hd<T, 4>(d.head_dim) : pick_attn_hd<T, 8>(d.head_dim);
-    {
-        static AttnKernel set[32]; static int n_set = 0;
-        bool done = false;
-        for (int i = 0; i < n_set; ++i) done |= set[i] == kern;
-        if (!done) {
-            if (cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ATTN_SMEM_LIMIT) != cudaSuccess) return fail(ADAMAH_ERR_BACKEND, "attention: cannot raise the shared-memory limit");
-            if (n_set < 32) set[n_set++] = kern;
-        }
-    }
-    // Few (sequence, head group) pairs in flight: the position splits of a pair form one thread-block cluster -- of 8 CTAs up to 16
+    s.work = batch * n_head;
+    const uint32_t hpc_auto = s.work <= 12u ? 1u : (s.work <= 32u ? (s.gs % 2u == 0u ? 2u : 1u) : s.gs);      // a divisor of the group
+    s.hpc = (hpc_env && s.gs % hpc_env == 0 && hpc_env <= 8u) ? hpc_env : hpc_auto;
+    s.pairs = n_kv * (s.gs / s.hpc) * batch;
+    // Few pairs in flight: the position splits of a pair form one thread-block cluster -- of 8 CTAs up to 16
     // pairs, of 4 up to 32, of 2 up to 64: one CTA per SM -- and merge through shared memory (no partial results in global memory, no ticket, no last-CTA pass: 3 us less per launch at the
     // 1B shape).  A cluster covers any context, its CTAs taking more chunks each, so layers that may attend to more than
     // 2048 positions keep the wider grid of independent splits.  (Clusters of 16 were measured slower: they start later,
     // and so does every kernel behind them.)  ADAM_B200_ATTN_CLUSTER=0 turns the path off, =16 allows clusters of 16.
     static const int cluster_env = getenv("ADAM_B200_ATTN_CLUSTER") ? atoi(getenv("ADAM_B200_ATTN_CLUSTER")) : 8;
     static const uint32_t cluster_pairs = getenv("ADAM_B200_ATTN_CLUSTER_WORK") ? (uint32_t)atoi(getenv("ADAM_B200_ATTN_CLUSTER_WORK")) : 64u;
-    const bool cluster = cluster_env != 0 && pairs <= cluster_pairs && (pairs <= 32u || pairs >= 56u) && reach <= 2048u;
+    if (cluster_env != 0 && s.pairs <= cluster_pairs && (s.pairs <= 32u || s.pairs >= 56u) && reach <= 2048u)
+        s.cluster = s.pairs > 32u ? 2u : s.pairs > 16u ? 4u : cluster_env == 16 ? std::min(most, 16u) : 8u;
     // Chunks in flight per CTA: one per warp; up to two in a cluster of splits, where a context just beyond 8 chunks per CTA (a window
-    // of 512) would have a warp wait for memory a second time.  (Elsewhere CTAs without positions would hold that much, too.)
-    const size_t slot_bytes = (size_t)2 * ATTN_CP * d.head_dim * sizeof(T);
-    const uint32_t n_slots = cluster ? (uint32_t)std::min<size_t>(16, std::max<size_t>(8, (192u << 10) / slot_bytes)) : 8u;
-    const size_t smem = n_slots * slot_bytes + ((size_t)hpc * d.head_dim + 2 * (size_t)d.head_dim) * 4;
-    if (cluster) {
-        // clusters of a size that run at once, by kernel and shared memory, which the heads per CTA change (0: none of that size)
-        struct Known { AttnKernel k; size_t smem; unsigned want, cs; int n; };
-        static Known known[64]; static int n_known = 0;
-        const unsigned want = pairs > 32u ? 2u : pairs > 16u ? 4u : cluster_env == 16 ? 16u : 8u;
-        const Known* kn = nullptr;
-        for (int i = 0; i < n_known; ++i) if (known[i].k == kern && known[i].smem == smem && known[i].want == want) kn = &known[i];
-        const auto smem_for = [&](unsigned c) { return smem + (size_t)c * hpc * (d.head_dim + 4) * 4; };
-        Known fresh = {kern, smem, want, 0u, 0};
-        if (!kn) {
-            if (want > 8 && cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) cudaGetLastError();
-            for (unsigned c = want; c >= std::min(want, 8u) && !fresh.n; c >>= 1) {
-                cudaLaunchConfig_t cfg = {};
-                cfg.gridDim = dim3(c, grid.y, 1); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = smem_for(c);
-                cudaLaunchAttribute at[1];
-                at[0].id = cudaLaunchAttributeClusterDimension;
-                at[0].val.clusterDim.x = c; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-                cfg.attrs = at; cfg.numAttrs = 1;
-                int n = 0;
-                if (cudaOccupancyMaxActiveClusters(&n, (const void*)kern, &cfg) != cudaSuccess) { cudaGetLastError(); continue; }
-                fresh.cs = c; fresh.n = n;
-            }
-            if (n_known < 64) known[n_known++] = fresh;
-            kn = &fresh;
-        }
-        const unsigned cs = kn->n >= (int)pairs ? kn->cs : 0u;
-        if (cs > 0) {
-            grid.x = cs;
-            const uint32_t cpc = cpc_env ? cpc_env : 8u;
-            if (launch_k_cluster(kern, grid, dim3(256), smem_for(cs), g.stream, g.pdl, cs, true, D->qkv, qkv_ld, ly.norm[NORM_Q], ly.norm[NORM_K], d.norm_eps,
-                                 D->rope_cos[which], D->rope_sin[which], D->rope_pos[which],
-                                 D->kv_pool, geo, D->block_table, D->pos, d.n_head, L, window, d.attn_scale,
-                                 d.attn_softcap, D->attn_out, D->part_o, D->part_ml, D->attn_ticket, 0u, hpc | (cpc << 16), n_slots, g.dev_err STEP_TRACE_ARG((g_step_trace && L == g_step_trace_layer) ? g_step_trace + 4 * 64 : nullptr)) != cudaSuccess)
-                return fail(ADAMAH_ERR_BACKEND, "attention: cluster launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-            count_ran(cs == 2 ? RAN_ATTN_CLUSTER_2 : cs == 4 ? RAN_ATTN_CLUSTER_4 : cs == 8 ? RAN_ATTN_CLUSTER_8 : RAN_ATTN_CLUSTER_16);
-            return ADAMAH_OK;
-        }
+    // of 512) would have a warp wait for memory a second time: as many as fit beside the queries and, in the first CTA, the splits' partial
+    // results.  (Elsewhere CTAs without positions would hold that much, too.)
+    const size_t slot = (size_t)2 * ATTN_CP * head_dim * kv_bytes, rows = ((size_t)s.hpc + 2) * head_dim * 4, merge = (size_t)s.cluster * s.hpc * (head_dim + 4) * 4;
+    s.smem = 8 * slot + rows;
+    if (s.cluster) {
+        const size_t fit = rows + merge < (size_t)ATTN_SMEM_LIMIT ? (ATTN_SMEM_LIMIT - rows - merge) / slot : 0;
+        s.slots = (uint32_t)std::min<size_t>(16, std::min<size_t>((192u << 10) / slot, fit));
+        if (s.slots < 8u) s.cluster = 0;
+        s.smem_cluster = s.slots * slot + rows + merge;
     }
-    launch_k(kern, grid, dim3(256), smem, g.stream, g.pdl, D->qkv, qkv_ld, ly.norm[NORM_Q], ly.norm[NORM_K], d.norm_eps,
-             D->rope_cos[which], D->rope_sin[which], D->rope_pos[which],
-             D->kv_pool, geo, D->block_table, D->pos, d.n_head, L, window, d.attn_scale,
-             d.attn_softcap, D->attn_out, D->part_o, D->part_ml, D->attn_ticket, D->n_splits, hpc | (cpc << 16), n_slots, g.dev_err STEP_TRACE_ARG((g_step_trace && L == g_step_trace_layer) ? g_step_trace + 4 * 64 : nullptr));
-    count_ran(RAN_ATTN_SPLITS);
+    return s;
+}
+
+template <typename T>
+static int launch_attn_t(Decoder* D, uint32_t L, uint32_t batch) {
+    const adam_b200_decoder_desc& d = D->d;
+    KvGeom geo{d.n_layer, d.n_head_kv, d.head_dim, d.page_size, D->max_pages_per_seq, D->page_elems};
+    const uint32_t window = ((d.flags & 1u) && d.sliding_window > 0 && !is_global_layer(d, L)) ? d.sliding_window : 0;
+    const uint32_t reach = window ? (window < d.kv_cap ? window : d.kv_cap) : d.kv_cap;
+    AttnShape s = attn_shape(d.n_head, d.n_head_kv, d.head_dim, sizeof(T), batch, reach);
+    const int which = is_global_layer(d, L) ? 1 : 0;
+    const Layer& ly = D->layers[L];
+    const uint32_t qkv_ld = (d.n_head + 2 * d.n_head_kv) * d.head_dim;
+    AttnKernel kern = s.hpc <= 1 ? pick_attn_hd<T, 1>(d.head_dim) : s.hpc <= 2 ? pick_attn_hd<T, 2>(d.head_dim)
+                    : s.hpc <= 4 ? pick_attn_hd<T, 4>(d.head_dim) : pick_attn_hd<T, 8>(d.head_dim);
+    // Chunks of 8 positions a CTA takes before another CTA joins: with few (sequence, head) pairs the SMs are idle and a
+    // CTA's chain of dependent chunk loads is the attention's whole time, so the positions are spread thinly (one chunk
+    // per warp); with many pairs the grid is full anyway and every extra CTA only repeats the query prologue.
+    static const uint32_t cpc_env = getenv("ADAM_B200_ATTN_CPC") ? (uint32_t)atoi(getenv("ADAM_B200_ATTN_CPC")) : 0u;
+    const uint32_t cpc = cpc_env ? cpc_env : (s.work <= 64u ? 8u : ATTN_CHUNKS_PER_CTA);
+    // Position splits launched: no more than this layer can reach (a split without positions still costs a CTA its start and the
+    // read of the position: 15 of 16 CTAs of the 27B shape's 64 sequences, 60 of the launch's 75 us), and no more than four
+    // CTAs per SM in all -- beyond that the pairs alone fill the GPU and a CTA takes more chunks instead.
+    const uint32_t useful = ((reach + ATTN_CP - 1) / ATTN_CP + 1 + cpc - 1) / cpc, fill = (4u * (uint32_t)g.sm_count + s.pairs - 1) / s.pairs;
+    dim3 grid(std::min(D->n_splits, std::min(useful, fill)), d.n_head_kv * (s.gs / s.hpc), batch);
+    // Per kernel: whether its limit is raised, and how many clusters of a size run at once (which the heads per CTA change, too).
+    struct Known { AttnKernel k; size_t smem; uint32_t cs; int n; };
+    static std::mutex lock;
+    static Known known[64]; static int n_known = 0;
+    const auto at_once = [&](uint32_t cs, size_t smem) -> int {          // clusters, or 0 for independent splits; negative: no launch
+        std::lock_guard<std::mutex> hold(lock);
+        bool raised = false;
+        for (int i = 0; i < n_known; ++i) {
+            if (known[i].k != kern) continue;
+            if (known[i].cs == cs && known[i].smem == smem) return known[i].n;
+            raised = true;
+        }
+        if (!raised && cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ATTN_SMEM_LIMIT) != cudaSuccess) return -1;
+        int n = 0;
+        if (cs) {
+            if (cs > 8 && cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) cudaGetLastError();
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(cs, grid.y, 1); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = smem;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+            cfg.attrs = at; cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&n, (const void*)kern, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+        }
+        if (n_known == 64) n_known = 0;
+        known[n_known++] = Known{kern, smem, cs, n};
+        return n;
+    };
+    int n = at_once(s.cluster, s.smem_cluster);
+    if (s.cluster == 16 && n >= 0 && n < (int)s.pairs) {
+        s = attn_shape(d.n_head, d.n_head_kv, d.head_dim, sizeof(T), batch, reach, 8);
+        n = at_once(s.cluster, s.smem_cluster);
+    }
+    if (n < 0) return fail(ADAMAH_ERR_BACKEND, "attention: cannot raise the shared-memory limit");
+    const uint32_t cs = n >= (int)s.pairs ? s.cluster : 0u;
+    cudaError_t e;
+    const auto args = [&](auto launch, uint32_t n_splits, uint32_t per_cta, uint32_t slots) {
+        return launch(D->qkv, qkv_ld, ly.norm[NORM_Q], ly.norm[NORM_K], d.norm_eps, D->rope_cos[which], D->rope_sin[which], D->rope_pos[which],
+                      D->kv_pool, geo, D->block_table, D->pos, d.n_head, L, window, d.attn_scale, d.attn_softcap, D->attn_out, D->part_o, D->part_ml,
+                      D->attn_ticket, n_splits, s.hpc | (per_cta << 16), slots, g.dev_err STEP_TRACE_ARG((g_step_trace && L == g_step_trace_layer) ? g_step_trace + 4 * 64 : nullptr));
+    };
+    if (cs) {
+        grid.x = cs;
+        e = args([&](auto... a) -> cudaError_t { return launch_k_cluster(kern, grid, dim3(256), s.smem_cluster, g.stream, g.pdl, cs, true, a...); }, 0u, cpc_env ? cpc_env : 8u, s.slots);
+    } else {
+        e = args([&](auto... a) -> cudaError_t { return launch_k(kern, grid, dim3(256), s.smem, g.stream, g.pdl, a...); }, D->n_splits, cpc, 8u);
+    }
+    if (e != cudaSuccess) return fail(ADAMAH_ERR_BACKEND, "attention: launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+    count_ran(!cs ? RAN_ATTN_SPLITS : cs == 2 ? RAN_ATTN_CLUSTER_2 : cs == 4 ? RAN_ATTN_CLUSTER_4 : cs == 8 ? RAN_ATTN_CLUSTER_8 : RAN_ATTN_CLUSTER_16);
     return ADAMAH_OK;
 }
 
@@ -2110,6 +2127,17 @@ extern "C" int adam_b200_decoder_read_logits(uint32_t id, uint32_t seq, float* o
     DCU(cudaStreamSynchronize(g.stream));
     return ADAMAH_OK;
 }
+// The launch shape that a step's attention asks for (the device may not run that many clusters at once): heads per CTA, (sequence,
+// head group) pairs, CTAs per cluster or 0, a cluster's slots and bytes of shared memory, bytes of a CTA of independent splits.
+extern "C" int adam_b200_attention_shape(uint32_t n_head, uint32_t n_head_kv, uint32_t head_dim, uint32_t kv_dtype, uint32_t batch, uint32_t reach, uint32_t* out) {
+    if (!out || !n_head_kv || n_head < n_head_kv || n_head % n_head_kv || n_head / n_head_kv > 8 || !batch || !reach || kv_dtype > 1 ||
+        (head_dim != 32 && head_dim != 64 && head_dim != 128 && head_dim != 256)) return fail(ADAMAH_ERR_INVALID, "attention_shape: bad arguments");
+    const AttnShape s = attn_shape(n_head, n_head_kv, head_dim, kv_dtype ? 2u : 4u, batch, reach);
+    out[0] = s.hpc; out[1] = s.pairs; out[2] = s.cluster; out[3] = s.cluster ? s.slots : 8u;
+    out[4] = s.cluster ? (uint32_t)s.smem_cluster : 0u; out[5] = (uint32_t)s.smem;
+    return ADAMAH_OK;
+}
+
 // Debug/verification read of an activation buffer of the last step:
 // what = 0 hidden after the last layer [E] (steps that ran the LM head), 2 qkv, 4 attn_out, 5 proj [E], 6 act [FF].
 extern "C" int adam_b200_decoder_read_buffer(uint32_t id, uint32_t what, uint32_t seq, float* out, uint32_t n) {

@@ -402,6 +402,10 @@ int adam_b200_gemm_counts(uint64_t* out, uint32_t n);
  * GPU of sm_count SMs; needs no GPU.  out[10]: row groups per warp, units, K slices, tile pairs per stage and slice, stages, CTAs,
  * items shared between CTAs (0 / 1), floats of an item's sums, floats of a workspace slot, bytes of shared memory. */
 int adam_b200_few_rows_shape(uint32_t ggml_type, uint32_t n, uint32_t k, uint32_t rows, uint32_t kind, uint32_t sm_count, uint32_t* out);
+/* The launch shape that the attention of a decode step asks for, `reach` positions per sequence at most (kv_dtype as in the
+ * decoder's description); needs no GPU.  out[6]: query heads per CTA, (sequence, head group) pairs, CTAs per cluster of position
+ * splits (0 = independent splits), chunks of 8 positions in flight per CTA, bytes of shared memory as clusters, as independent splits. */
+int adam_b200_attention_shape(uint32_t n_head, uint32_t n_head_kv, uint32_t head_dim, uint32_t kv_dtype, uint32_t batch, uint32_t reach, uint32_t* out);
 /* Which calls take it: 0 = none, 1 = those expected to be faster than the GEMV kernels (default; also the
  * initial value of environment variable ADAM_B200_TC), 2 = every call whose shape allows, on the tcgen05 one. */
 int adam_b200_tc_gemm_policy(int policy);

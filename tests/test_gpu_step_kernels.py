@@ -44,9 +44,17 @@ def test_rows_whose_squares_overflow(gpu, batch):
 
 # ---- attention ---------------------------------------------------------------------------------------------------------
 
-# Groups of three, five and seven query heads; two groups that share a kernel and differ in shared memory, one behind the other.
+# Heads per CTA 1, 2, 4, 8 and the odd groups; clusters of 2, 4 and 8 whose CTAs have more chunks than slots (16, 12 and fewer of them),
+# splits; a window, pages that chunks of eight do not divide.
 @pytest.mark.parametrize("head_dim,n_head,n_kv,window,page,batch,length,kv_dtype,kernel", [
-    (256, 5, 1, 0, 64, 20, 90, "f32", "attn_cluster_4"), (256, 6, 1, 0, 64, 20, 90, "f32", None),
+    (256, 4, 1, 0, 64, 60, 300, "f16", "attn_cluster_2"), (256, 4, 1, 0, 64, 64, 300, "f32", "attn_cluster_2"),
+    (128, 8, 1, 100, 16, 56, 260, "f16", "attn_cluster_2"), (128, 4, 4, 60, 12, 14, 420, "f32", "attn_cluster_2"),
+    (256, 4, 1, 0, 64, 20, 1100, "f16", "attn_cluster_4"), (256, 4, 1, 0, 64, 17, 700, "f32", "attn_cluster_4"),
+    (64, 4, 2, 0, 12, 10, 500, "f32", "attn_cluster_4"), (256, 8, 1, 0, 64, 24, 700, "f32", "attn_cluster_4"),
+    (256, 4, 1, 0, 64, 12, 1100, "f32", "attn_cluster_8"), (256, 1, 1, 0, 64, 1, 2000, "f32", "attn_cluster_8"),
+    (128, 2, 1, 300, 20, 5, 1000, "f16", "attn_cluster_8"), (256, 8, 2, 0, 64, 5, 1100, "f32", "attn_cluster_8"),
+    (256, 4, 1, 0, 64, 40, 300, "f16", "attn_splits"), (256, 4, 1, 0, 64, 70, 200, "f32", "attn_splits"),
+    (256, 5, 1, 0, 64, 20, 90, "f32", "attn_cluster_4"), (256, 6, 1, 0, 64, 20, 90, "f32", "attn_cluster_4"),
     (32, 3, 1, 0, 64, 6, 200, "f32", "attn_cluster_4"), (64, 5, 1, 0, 64, 5, 90, "f16", "attn_cluster_4"),
     (32, 6, 2, 0, 64, 4, 150, "f32", "attn_cluster_4"), (128, 7, 1, 0, 64, 2, 200, "f32", "attn_cluster_8")])
 def test_attention_of_a_step(gpu, head_dim, n_head, n_kv, window, page, batch, length, kv_dtype, kernel):
@@ -60,7 +68,7 @@ def test_attention_of_a_step(gpu, head_dim, n_head, n_kv, window, page, batch, l
         eng.prefill_prompts(prompts, 0)
         before = gpu.step_kernel_counts()
         eng.step(1, lm_head=True, logits=True, direct=True)
-        assert kernel is None or {k: n for k, n in _ran(gpu, before).items() if k.startswith("attn")} == {kernel: cfg.n_layer}
+        assert {k: n for k, n in _ran(gpu, before).items() if k.startswith("attn")} == {kernel: cfg.n_layer}
         got = {b: eng.read_logits(b) for b in sorted({0, 1 % batch, batch // 3, batch // 2, batch - 1})}
         for b, g in got.items():
             want = eng.logits_trace(prompts[b])[-1]
