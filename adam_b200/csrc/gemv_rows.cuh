@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemv_rows(const GemvArgs a, cons
         bulk_g2s(wb, t0 + off, (uint32_t)(np * TILE), &s_bar[warp]);
         if (PAIR) bulk_g2s(wb + PPW * TILE, t1 + off, (uint32_t)(np * TILE), &s_bar[warp]);
     }
+    __syncwarp();                                                           // every lane waits on the barrier, a warp without rows with nothing in between
     const int f0 = p0 * 16 + lane, nf = np * 16 - lane;                     // this lane's first float4; how far the slice goes from there
     float4 vp[NV], vw[NV];
     if (CHAIN) {
