@@ -930,19 +930,20 @@ static bool pdl_allowed() {
     return allow;
 }
 
-static void launch_embed(Decoder* D, uint32_t rows, const int32_t* row_seq, const int32_t* row_pos) {
+template <int WT>
+static void launch_embed_t(Decoder* D, uint32_t rows, const int32_t* row_seq, const int32_t* row_pos) {
     const adam_b200_decoder_desc& d = D->d;
-    auto go = [&](auto kern) {
-        static bool set = false;
-        if (!set) { carveout_max((const void*)kern, 0); set = true; }
-        launch_k(kern, dim3(rows), dim3(256), 0, g.stream, false, D->embd.w, d.n_embd, D->embd.rows, d.emb_scale, D->pos, D->prompt_len, D->prompt_tok,
-                 d.kv_cap, D->cur_tok, D->hbuf[0], row_seq, row_pos, g.dev_err);
-    };
+    static const bool set = carveout_max((const void*)k_embed<WT>, 0);        // once for each of the kernels
+    (void)set;
+    launch_k(k_embed<WT>, dim3(rows), dim3(256), 0, g.stream, false, D->embd.w, d.n_embd, D->embd.rows, d.emb_scale, D->pos, D->prompt_len, D->prompt_tok,
+             d.kv_cap, D->cur_tok, D->hbuf[0], row_seq, row_pos, g.dev_err);
+}
+static void launch_embed(Decoder* D, uint32_t rows, const int32_t* row_seq, const int32_t* row_pos) {
     switch (D->embd.wtype) {
-    case WT_Q4_0: go(k_embed<WT_Q4_0>); break;
-    case WT_Q4_K: go(k_embed<WT_Q4_K>); break;
-    case WT_Q8_0: go(k_embed<WT_Q8_0>); break;
-    default:      go(k_embed<WT_Q5_0>); break;
+    case WT_Q4_0: launch_embed_t<WT_Q4_0>(D, rows, row_seq, row_pos); break;
+    case WT_Q4_K: launch_embed_t<WT_Q4_K>(D, rows, row_seq, row_pos); break;
+    case WT_Q8_0: launch_embed_t<WT_Q8_0>(D, rows, row_seq, row_pos); break;
+    default:      launch_embed_t<WT_Q5_0>(D, rows, row_seq, row_pos); break;
     }
     count_launch();
 }
