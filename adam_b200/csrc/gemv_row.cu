@@ -1,10 +1,13 @@
 // Host-side launch logic of the one-row GEMV (kernel in gemv_row.cuh).
 #include "gemv_row.cuh"
 
+#include <atomic>
+
 namespace ab {
 
 typedef void (*RowKernel)(const GemvArgs, const uint8_t*, const uint8_t*, float);
-struct RowShape { RowKernel k; int ks; size_t smem; };
+struct RowShape { RowKernel k; int id, ks; size_t smem; };        // id: which of a type's instances
+constexpr int ROW_IDS = 9;
 
 // Two tile pairs per warp: its 32 lanes hold one float4 of activations each, the shortest chain there is (K <= 4096); four for
 // longer rows.  Up to nine slices (K <= 1152) a thread keeps to 56 registers: three such CTAs, what a matrix of 400 row groups
@@ -17,14 +20,17 @@ static RowShape row_shape(const GemvArgs& a) {
     RowShape s = {};
     int ppw = 2;
     s.ks = (pairs + 1) / 2;
+    s.id = (pair ? 1 : 0) + (chain ? 2 : 0);
     if (s.ks * 32 <= ROW_THREADS) {
         s.k = pair ? (chain ? k_gemv_row<true, WT, true, 2, ROW_THREADS, ROW_CTAS> : k_gemv_row<true, WT, false, 2, ROW_THREADS, ROW_CTAS>)
                    : (chain ? k_gemv_row<false, WT, true, 2, ROW_THREADS, ROW_CTAS> : k_gemv_row<false, WT, false, 2, ROW_THREADS, ROW_CTAS>);
     } else if (s.ks <= ROW_MAX_WARPS) {
+        s.id += 4;
         s.k = pair ? (chain ? k_gemv_row<true, WT, true, 2, 1024, 1> : k_gemv_row<true, WT, false, 2, 1024, 1>)
                    : (chain ? k_gemv_row<false, WT, true, 2, 1024, 1> : k_gemv_row<false, WT, false, 2, 1024, 1>);
     } else {
         ppw = 4;
+        s.id = 8;
         s.ks = (pairs + 3) / 4;
         if (pair || chain || s.ks > ROW_MAX_WARPS) return RowShape{};
         s.k = k_gemv_row<false, WT, false, 4, 1024, 1>;
@@ -41,15 +47,14 @@ static bool row_shape_for(int wt, const GemvArgs& a, RowShape* out) {
     const RowShape s = wt == WT_Q4_0 ? row_shape<WT_Q4_0>(a) : row_shape<WT_Q4_K>(a);
     if (!s.k) return false;
     // Every CTA resident at once: a second wave would request its weights only when the first is done, which is what the rings
-    // of k_gemv_mma are for.  (The occupancies asked for are kept: a step asks for the same few shapes.)
-    struct Known { RowKernel k; int ks, per_sm; };
-    static thread_local Known known[32]; static thread_local int n_known = 0;
-    int per_sm = -1;
-    for (int i = 0; i < n_known; ++i) if (known[i].k == s.k && known[i].ks == s.ks) per_sm = known[i].per_sm;
+    // of k_gemv_mma are for.  (Asked for once per instance and number of slices.)
+    static std::atomic<int> known[2][ROW_IDS][ROW_MAX_WARPS + 1];           // CTAs per SM plus one, 0 = not asked yet
+    std::atomic<int>& kn = known[wt == WT_Q4_0 ? 0 : 1][s.id][s.ks];
+    int per_sm = kn - 1;
     if (per_sm < 0) {
         if (!carveout_max((const void*)s.k, 0) ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, s.k, s.ks * 32, s.smem) != cudaSuccess) { cudaGetLastError(); return false; }
-        if (n_known < 32) known[n_known++] = Known{s.k, s.ks, per_sm};
+        kn = per_sm + 1;
     }
     if ((long long)(a.N / 16) > (long long)per_sm * g.sm_count) return false;
     // and at most 48 warps per SM: more of them take the instructions of as many stagings (9472 x 1152, 36 warps per SM, 5.2 us by
