@@ -189,16 +189,17 @@ __global__ void __launch_bounds__(SEL_T) k_sample_stage1(const float* __restrict
 __global__ void __launch_bounds__(SEL_T) k_sample_stage2(const float* __restrict__ cand_v, const int* __restrict__ cand_i, uint32_t groups, uint32_t k, int in_shared,
                                                          float temperature, float top_p, uint64_t seed,
                                                          const int32_t* __restrict__ pos, int32_t* __restrict__ cur_tok, float* __restrict__ cur_val,
-                                                         int32_t* __restrict__ gen_log, uint32_t ld, float* __restrict__ dbg) {
+                                                         int32_t* __restrict__ gen_log, uint32_t ld, uint2* __restrict__ far_heads, float* __restrict__ dbg) {
     __shared__ float out_v[TOPK_MAX]; __shared__ int out_i[TOPK_MAX];
     const uint32_t b = blockIdx.x;
     const uint32_t n_cand = groups * k;
     const float* cv = cand_v + (size_t)b * n_cand;
     const int* ci = cand_i + (size_t)b * n_cand;
     extern __shared__ unsigned char sel_sm[];
-    // [groups] the rank and row of a group's head, [groups] candidates of it that are taken; then the candidates
-    uint2* hd = reinterpret_cast<uint2*>(sel_sm);
-    unsigned char* head = sel_sm + (size_t)groups * 8;
+    // [groups] the rank and row of a group's head (in `far_heads` where there are too many), [groups] candidates of it that are taken;
+    // then the candidates
+    uint2* hd = far_heads ? far_heads + (size_t)b * groups : reinterpret_cast<uint2*>(sel_sm);
+    unsigned char* head = sel_sm + (far_heads ? 0 : (size_t)groups * 8);
     if (in_shared) {
         float* v = reinterpret_cast<float*>(sel_sm + (((size_t)groups * 9 + 15) & ~(size_t)15));
         int* i = reinterpret_cast<int*>(v + n_cand);
@@ -282,6 +283,7 @@ __global__ void __launch_bounds__(SEL_T) k_sample_stage2(const float* __restrict
 }
 
 static float* s_cand_v = nullptr; static int* s_cand_i = nullptr; static size_t s_cand_n = 0;
+static uint2* s_heads = nullptr; static size_t s_heads_n = 0;
 
 // Enqueue the sampling step for `batch` sequences whose soft-capped logits lie at logits[b * V .. ) and whose
 // positions were already advanced.  k = 1..64.
@@ -290,25 +292,36 @@ int launch_sample(const float* logits, uint32_t V, uint32_t batch, uint32_t k, f
                   int32_t* cur_tok, float* cur_val) {
     if (k == 0 || k > TOPK_MAX) return fail(ADAMAH_ERR_INVALID, "sampling: top_k must be 1..64 on the device");
     const uint32_t groups = (V + SEL_T * SEL_V - 1) / (SEL_T * SEL_V);
-    const size_t need = (size_t)batch * groups * k;
-    if (s_cand_n < need) {
+    // Heads, candidates taken and the candidates in shared memory where they fit (82 KB at a vocabulary of 262144 and k = 64); the heads
+    // alone as far as 37 million rows, beyond which they are in global memory, too.
+    constexpr size_t LIMIT = 160 * 1024;
+    const size_t near = ((size_t)groups * 9 + 15) & ~(size_t)15, all = near + (size_t)groups * k * 8;
+    const bool in_shared = all <= LIMIT, far = near > LIMIT;
+    const size_t need = (size_t)batch * groups * k, need_heads = far ? (size_t)batch * groups : 0;
+    if (s_cand_n < need || s_heads_n < need_heads) {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(g.stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
             return fail(ADAMAH_ERR_INVALID, "sampling: the first sampled step must run outside a graph capture");
         cudaStreamSynchronize(g.stream);
-        cudaFree(s_cand_v); cudaFree(s_cand_i); s_cand_v = nullptr; s_cand_i = nullptr; s_cand_n = 0;
-        if (cudaMalloc((void**)&s_cand_v, need * 4) != cudaSuccess || cudaMalloc((void**)&s_cand_i, need * 4) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(ADAMAH_ERR_MEMORY, "sampling: out of device memory");
+        if (s_cand_n < need) {
+            cudaFree(s_cand_v); cudaFree(s_cand_i); s_cand_v = nullptr; s_cand_i = nullptr; s_cand_n = 0;
+            if (cudaMalloc((void**)&s_cand_v, need * 4) != cudaSuccess || cudaMalloc((void**)&s_cand_i, need * 4) != cudaSuccess) {
+                cudaGetLastError();
+                return fail(ADAMAH_ERR_MEMORY, "sampling: out of device memory");
+            }
+            s_cand_n = need;
         }
-        s_cand_n = need;
+        if (s_heads_n < need_heads) {
+            cudaFree(s_heads); s_heads = nullptr; s_heads_n = 0;
+            if (cudaMalloc((void**)&s_heads, need_heads * sizeof(uint2)) != cudaSuccess) { cudaGetLastError(); return fail(ADAMAH_ERR_MEMORY, "sampling: out of device memory"); }
+            s_heads_n = need_heads;
+        }
     }
     k_sample_stage1<<<dim3(groups, batch), SEL_T, 0, g.stream>>>(logits, V, k, pos, prompt_len, prompt_tok, gen_log, ld, penalty, on_prompt, s_cand_v, s_cand_i);
-    const size_t heads = ((size_t)groups * 9 + 15) & ~(size_t)15, all = heads + (size_t)groups * k * 8;
-    const bool in_shared = all <= 160 * 1024;           // 82 KB at a vocabulary of 262144 and k = 64
-    if (cudaFuncSetAttribute(k_sample_stage2, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
+    if (cudaFuncSetAttribute(k_sample_stage2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LIMIT) != cudaSuccess)
         return fail(ADAMAH_ERR_BACKEND, "sampling: cannot raise the shared-memory limit");
-    k_sample_stage2<<<batch, SEL_T, in_shared ? all : heads, g.stream>>>(s_cand_v, s_cand_i, groups, k, in_shared ? 1 : 0, temperature, top_p, seed, pos, cur_tok, cur_val, gen_log, ld, nullptr);
+    k_sample_stage2<<<batch, SEL_T, in_shared ? all : far ? (size_t)groups : near, g.stream>>>(s_cand_v, s_cand_i, groups, k, in_shared ? 1 : 0, temperature, top_p, seed, pos, cur_tok, cur_val, gen_log, ld,
+                                                                                              far ? s_heads : nullptr, nullptr);
     count_launch(2);
     return check_launch("decoder sampling");
 }
@@ -325,7 +338,8 @@ int logits_scratch(size_t n, float** out) {
 }
 void sample_free_all() {
     cudaFree(s_logits); s_logits = nullptr; s_logits_n = 0;
-    cudaFree(s_cand_v); cudaFree(s_cand_i); s_cand_v = nullptr; s_cand_i = nullptr; s_cand_n = 0;
+    cudaFree(s_cand_v); cudaFree(s_cand_i); cudaFree(s_heads);
+    s_cand_v = nullptr; s_cand_i = nullptr; s_heads = nullptr; s_cand_n = s_heads_n = 0;
 }
 
 }  // namespace ab

@@ -4,7 +4,7 @@ import pytest
 
 from adam_b200 import gguf_blocks as gb
 from adam_b200 import synth
-from adam_b200.config import tiny_gemma3
+from adam_b200.config import GenerationConfig, tiny_gemma3
 from adam_b200.engine import ADAMEngine
 from oracle.decoder import OracleDecoder, dequant_model
 
@@ -129,5 +129,27 @@ def test_values_beyond_fp16_are_infinite(gpu, before, batch):
             assert np.isinf(want).any() and not np.isnan(got).any()
             for h in got:
                 assert np.array_equal(np.where(np.isinf(h), h, 0.0), want)
+    finally:
+        eng.close()
+
+
+# ---- sampling ----------------------------------------------------------------------------------------------------------
+
+def test_sampling_over_a_very_large_vocabulary(gpu):
+    """More groups of candidates than shared memory has room for the heads of."""
+    V, hot = 37_400_000, 37_399_999
+    cfg, tensors = _model(seed=4, n_layer=1, n_embd=64, n_ff=64, head_dim=32, n_vocab=64)
+    small = tensors["token_embd.weight"].raw.reshape(64, -1)
+    raw = np.zeros((V, small.shape[1]), np.uint8)
+    raw[:8], raw[hot] = small[:8], small[8]
+    tensors["token_embd.weight"] = synth.QTensor(2, V, 64, raw.reshape(-1))
+    cfg.n_vocab = V
+    eng = ADAMEngine(gpu, cfg, tensors, kv_cap=16, kv_dtype="f32")
+    try:
+        rule = dict(max_tokens=1, eos_token_ids=(), repeat_penalty=1.0)
+        for prompt in ([1], [hot], [3, hot]):
+            best, _ = eng.generate(prompt, GenerationConfig(top_k=1, temperature=0.0, **rule))
+            drawn, stats = eng.generate(prompt, GenerationConfig(top_k=40, top_p=0.95, temperature=1e-4, seed=1, **rule))
+            assert stats["sampling_mode"] == "gpu_fused_topk" and drawn == best
     finally:
         eng.close()
