@@ -170,12 +170,20 @@ def test_q4_k_gemv_tensor_core_path(gpu, N, K, B):
     assert np.abs(y - y0).max() < 1e-4 * np.abs(y0).max()
 
 
-@pytest.mark.parametrize("ggml_type,N,K", [
-    (2, 16, 64), (2, 32, 192), (2, 11840, 1152), (2, 11856, 1152),     # one slice; a slice of one pair; five CTAs per SM, one more
-    (2, 48, 1280), (2, 14208, 1024), (2, 14224, 1024), (2, 160, 4096), (2, 160, 4160),      # 10 slices; 48 warps per SM, more; 32 slices; slices of up to four pairs
-    (2, 96, 8192), (2, 2368, 6912), (2, 2384, 6912), (2, 96, 8256),    # 32 of four; one CTA per SM and one more; too long
-    (12, 16, 256), (12, 2048, 1280), (12, 48, 1536), (12, 80, 4352), (12, 80, 8192)])
-def test_one_row_gemv_edges(gpu, ggml_type, N, K):
+def _gemv_on(gpu, kernel, *args):
+    """The product over a row-tiled copy, which has to run on that kernel alone."""
+    before, gemms = gpu.step_kernel_counts(), gpu.gemm_counts()
+    y = _gemv(gpu, *args, tile=True)
+    assert [k for k, n in gpu.step_kernel_counts().items() if n > before[k]] == [kernel] and gpu.gemm_counts() == gemms
+    return y
+
+
+@pytest.mark.parametrize("ggml_type,N,K,kernel", [
+    (2, 16, 64, "row"), (2, 32, 192, "row"), (2, 11840, 1152, "row"), (2, 11856, 1152, "mma"),     # one slice; a slice of one pair; five CTAs per SM, one more
+    (2, 48, 1280, "row"), (2, 14208, 1024, "row"), (2, 14224, 1024, "mma"), (2, 160, 4096, "row"), (2, 160, 4160, "row"),      # 10 slices; 48 warps per SM, more; 32 slices; slices of up to four pairs
+    (2, 96, 8192, "row"), (2, 2368, 6912, "row"), (2, 2384, 6912, "ring"), (2, 96, 8256, "ring"),  # 32 of four; one CTA per SM and one more; too long
+    (12, 16, 256, "row"), (12, 2048, 1280, "row"), (12, 48, 1536, "row"), (12, 80, 4352, "row"), (12, 80, 8192, "row")])
+def test_one_row_gemv_edges(gpu, ggml_type, N, K, kernel):
     """Products of one row whose matrix fits the registers (one warp per K slice), at the edges of what takes them.  A slice's
     activations are rounded to 23 bits of its own largest value, sums are fp32: 1e-6 of the result's 2-norm for activations
     whose slices differ by factors of up to 1e6."""
@@ -185,36 +193,38 @@ def test_one_row_gemv_edges(gpu, ggml_type, N, K):
     W = q4_blocks.dequant(raw.reshape(-1), ggml_type, N, K).astype(np.float64)
     for scale in (np.ones(K), 10.0 ** rng.integers(-3, 4, K // 64).repeat(64), np.zeros(K)):
         xs = (x * scale).astype(np.float32)
-        y = _gemv(gpu, ggml_type, raw, N, K, xs, tile=True)
+        y = _gemv_on(gpu, kernel, ggml_type, raw, N, K, xs)
         ref = xs.astype(np.float64) @ W.T
         assert np.linalg.norm(y - ref) <= 1e-6 * np.linalg.norm(xs) * np.linalg.norm(W) / np.sqrt(K) * 4
 
 
-@pytest.mark.parametrize("ggml_type,N,K", [
-    (2, 2384, 5376), (2, 4752, 4160), (2, 2400, 8192), (2, 16, 8256), (2, 48, 12352),      # uneven slices, CTAs of one and two row groups
-    (2, 32, 21504), (2, 16, 24576), (2, 16, 24640),                                        # two ring stages; the longest slices; longer
-    (12, 2384, 5376), (12, 2400, 4352), (12, 32, 21504), (12, 16, 24576)])
-def test_streamed_one_row_gemv_edges(gpu, ggml_type, N, K):
+@pytest.mark.parametrize("ggml_type,N,K,kernel", [
+    (2, 2384, 5376, "ring"), (2, 4752, 4160, "ring"), (2, 2400, 8192, "ring"), (2, 16, 8256, "ring"), (2, 48, 12352, "ring"),      # uneven slices, CTAs of one to three row groups
+    (2, 16576, 2048, "ring"), (2, 16592, 2048, "mma"),                                     # seven row groups per CTA, two pairs per slice; more groups
+    (2, 32, 21504, "ring"), (2, 16, 24576, "ring"), (2, 16, 24640, "mma"),                 # two ring stages; the longest slices; longer
+    (12, 2384, 5376, "ring"), (12, 2400, 4352, "ring"), (12, 32, 21504, "ring"), (12, 16, 24576, "ring")])
+def test_streamed_one_row_gemv_edges(gpu, ggml_type, N, K, kernel):
     """Products of one row over matrices that are streamed, at the edges of what takes them; the bound of test_few_row_gemv_edges
     (1e-6 where the matrix is too long for slices of their own scale: 23 bits of the vector's largest value)."""
     rng = np.random.default_rng(N + K)
     raw = (gb.random_q4_0_blocks if ggml_type == 2 else gb.random_q4_k_blocks)(rng, N, K)
     x = rng.standard_normal((1, K)).astype(np.float32)
     W = q4_blocks.dequant(raw.reshape(-1), ggml_type, N, K).astype(np.float64)
-    tol = 5e-7 if K <= 24576 else 1e-6
+    tol = 5e-7 if kernel == "ring" else 1e-6
     for scale in (np.ones(K), 10.0 ** rng.integers(-3, 4, K // 64).repeat(64)):
         xs = (x * scale).astype(np.float32)
-        y = _gemv(gpu, ggml_type, raw, N, K, xs, tile=True)
+        y = _gemv_on(gpu, kernel, ggml_type, raw, N, K, xs)
         ref = xs.astype(np.float64) @ W.T
         assert np.linalg.norm(y - ref) <= tol * np.linalg.norm(xs) * np.linalg.norm(W) / np.sqrt(K) * 4
 
 
-@pytest.mark.parametrize("ggml_type,N,K,B", [
-    (2, 16, 64, 2), (2, 48, 192, 3), (2, 2368, 1024, 4), (2, 2384, 1152, 3),       # one row group per CTA, one more than the SMs
-    (2, 6912, 1152, 2), (2, 7120, 1152, 4), (2, 4752, 2048, 2), (2, 160, 2048, 4),  # three per CTA, the last CTA not full; 16 slices
-    (2, 160, 2112, 3), (2, 1152, 6912, 4), (2, 96, 8192, 4), (2, 96, 8256, 2),      # slices of four pairs; the most; too long
-    (12, 16, 256, 4), (12, 6912, 1280, 3), (12, 96, 4352, 2), (12, 2064, 1536, 4)])
-def test_few_row_gemv_edges(gpu, ggml_type, N, K, B):
+@pytest.mark.parametrize("ggml_type,N,K,B,kernel", [
+    (2, 16, 64, 2, "rows"), (2, 48, 192, 3, "rows"), (2, 2368, 1024, 4, "rows"), (2, 2384, 1152, 3, "rows"),       # one row group per CTA, one more than the SMs
+    (2, 6912, 1152, 2, "rows"), (2, 7040, 1152, 4, "rows"), (2, 7120, 1152, 4, "mma"),      # three per CTA, the last CTA not full; more warps than a CTA has
+    (2, 4720, 2048, 2, "rows"), (2, 4752, 2048, 2, "mma"), (2, 160, 2048, 4, "rows"),       # 16 slices
+    (2, 160, 2112, 3, "rows"), (2, 1152, 6912, 4, "rows"), (2, 96, 8192, 4, "rows"), (2, 96, 8256, 2, "mma"),      # slices of four pairs; the most; too long
+    (12, 16, 256, 4, "rows"), (12, 6912, 1280, 3, "rows"), (12, 96, 4352, 2, "rows"), (12, 2064, 1536, 4, "rows")])
+def test_few_row_gemv_edges(gpu, ggml_type, N, K, B, kernel):
     """Products of two to four rows over matrices that the SMs hold at once, at the edges of what takes them.  Activations keep 31 bits
     of their slice's largest value, sums are fp32: 5e-7 of the norms' product, rows and slices of any scale."""
     rng = np.random.default_rng(N + K + B)
@@ -224,7 +234,7 @@ def test_few_row_gemv_edges(gpu, ggml_type, N, K, B):
     for scale in (np.ones(K), 10.0 ** rng.integers(-3, 4, K // 64).repeat(64)):
         xs = (x * scale).astype(np.float32)
         xs[B - 1, : K // 2] = 0.0
-        y = _gemv(gpu, ggml_type, raw, N, K, xs, tile=True)
+        y = _gemv_on(gpu, kernel, ggml_type, raw, N, K, xs)
         for b in range(B):
             ref = W @ xs[b].astype(np.float64)
             assert np.linalg.norm(y[b] - ref) <= 5e-7 * np.linalg.norm(xs[b]) * np.linalg.norm(W) / np.sqrt(K) * 4
@@ -247,9 +257,7 @@ def test_rows_that_are_not_finite(gpu, ggml_type, N, K, B, policy, kernel, bad):
         for at in (0, K - 5):
             y = x.copy()
             y[B // 2, at] = bad
-            before = gpu.step_kernel_counts()
-            got = _gemv(gpu, ggml_type, raw, N, K, y, tile=True)
-            assert [k for k, n in gpu.step_kernel_counts().items() if n > before[k]] == [kernel]
+            got = _gemv_on(gpu, kernel, ggml_type, raw, N, K, y)
             others = np.arange(B) != B // 2
             assert np.array_equal(got[others], want[others]) and not np.isfinite(got[B // 2]).any()
     finally:
@@ -268,9 +276,7 @@ def test_rows_near_the_end_of_fp32(gpu, N, K, B, policy, kernel, top):
     x = (x * (top / np.abs(x).max())).astype(np.float32)
     gpu.tc_gemm_policy(policy)
     try:
-        before = gpu.step_kernel_counts()
-        y = _gemv(gpu, 2, raw, N, K, x, tile=True).astype(np.float64) / top
-        assert [k for k, n in gpu.step_kernel_counts().items() if n > before[k]] == [kernel]
+        y = _gemv_on(gpu, kernel, 2, raw, N, K, x).astype(np.float64) / top
         ref = (x.astype(np.float64) / top) @ W.T
         assert np.linalg.norm(y - ref) <= 4e-6 * np.linalg.norm(x.astype(np.float64) / top) * np.linalg.norm(W) / np.sqrt(K)
     finally:

@@ -25,6 +25,37 @@ def _model(ggml_type=2, seed=0, **kw):
 
 # ---- products behind the norm chain, gate / up pairs -------------------------------------------------------------------
 
+# One row: a slice of one tile pair, ten slices and 32, the last of one pair; rows that are streamed, in uneven slices and the longest.
+# Two to four: one row group per CTA and three with a CTA that is not full, 16 slices.  Kernels per layer.
+@pytest.mark.parametrize("ggml_type,n_embd,n_ff,batch,act,post_norms,kernels", [
+    (2, 192, 320, 1, "gelu", True, {"row": 4}), (2, 1216, 640, 1, "silu", True, {"row": 4}), (2, 4032, 192, 1, "gelu", False, {"row": 4}),
+    (12, 1280, 768, 1, "silu", False, {"row": 4}), (12, 3840, 256, 1, "gelu", True, {"row": 4}),
+    (2, 4160, 384, 1, "gelu", True, {"row": 2, "ring": 2}), (2, 6144, 320, 1, "silu", False, {"row": 2, "ring": 2}),
+    (12, 4352, 512, 1, "gelu", True, {"row": 2, "ring": 2}),
+    (2, 192, 320, 2, "gelu", True, {"rows": 4}), (2, 1152, 7040, 3, "gelu", True, {"rows": 4}), (2, 1216, 640, 4, "silu", False, {"rows": 4}),
+    (2, 2048, 384, 2, "silu", True, {"rows": 4}), (12, 1280, 3328, 4, "gelu", True, {"rows": 4}), (12, 1536, 512, 3, "gelu", False, {"rows": 4})])
+def test_products_of_a_step(gpu, ggml_type, n_embd, n_ff, batch, act, post_norms, kernels):
+    """Logits of five steps against the oracle's: fp32 sums on both sides, in different orders."""
+    cfg, tensors = _model(ggml_type, seed=n_embd, n_embd=n_embd, n_ff=n_ff, act=act, post_norms=post_norms)
+    f32 = dequant_model(tensors)
+    prompts = [synth.random_prompt(cfg.n_vocab, 5, seed=b) for b in range(batch)]
+    eng = ADAMEngine(gpu, cfg, tensors, kv_cap=16, kv_dtype="f32", max_batch=batch)
+    try:
+        eng.begin(prompts, [8] * batch)
+        oracles = [OracleDecoder(cfg, f32, kv_cap=16) for _ in prompts]
+        for i in range(5):
+            before = gpu.step_kernel_counts()
+            eng.step(1, lm_head=True, logits=True, direct=True)
+            ran = _ran(gpu, before)
+            assert {k: ran.get(k, 0) for k in ("row", "ring", "rows")} == {k: cfg.n_layer * kernels.get(k, 0) for k in ("row", "ring", "rows")}
+            for b, p in enumerate(prompts):
+                want = oracles[b].forward(int(p[i]), i)
+                assert np.abs(eng.read_logits(b) - want).max() <= 2e-5 * np.abs(want).max()
+        assert gpu.device_error() == 0
+    finally:
+        eng.close()
+
+
 @pytest.mark.parametrize("batch", [1, 3, 8])
 def test_rows_whose_squares_overflow(gpu, batch):
     """x / sqrt(inf) is 0 for finite x, in every kernel that norms its input."""
