@@ -821,18 +821,21 @@ static AttnShape attn_shape(uint32_t n_head, uint32_t n_kv, uint32_t head_dim, u
     const uint32_t hpc_auto = s.work <= 12u ? 1u : (s.work <= 32u ? (s.gs % 2u == 0u ? 2u : 1u) : s.gs);      // a divisor of the group
     s.hpc = (hpc_env && s.gs % hpc_env == 0 && hpc_env <= 8u) ? hpc_env : hpc_auto;
     s.pairs = n_kv * (s.gs / s.hpc) * batch;
-    // Few pairs in flight: the position splits of a pair form one thread-block cluster -- of 8 CTAs up to 16
-    // pairs, of 4 up to 32, of 2 up to 64: one CTA per SM -- and merge through shared memory (no partial results in global memory, no ticket, no last-CTA pass: 3 us less per launch at the
-    // 1B shape).  A cluster covers any context, its CTAs taking more chunks each, so layers that may attend to more than
-    // 2048 positions keep the wider grid of independent splits.  (Clusters of 16 were measured slower: they start later,
-    // and so does every kernel behind them.)  ADAM_B200_ATTN_CLUSTER=0 turns the path off, =16 allows clusters of 16.
+    // Few pairs in flight: the position splits of a pair form one thread-block cluster -- of 8 CTAs up to 16 pairs, of 4 up to 32, of 2
+    // up to 64: one CTA per SM -- and merge through shared memory (no partial results in global memory, no ticket, no last-CTA pass:
+    // 3 us less per launch at the 1B shape).  The lines at 32 and 56 rest on 48 sequences (clusters of 2 slower), 56 and 64 (faster)
+    // of that shape at a context of 512.  With an fp32 cache 9 sequences take 1.14 ms per step as clusters of 8 with 11 slots and 1.17
+    // as independent splits, 12 take 1.17 and 1.19, 16 the same.  A cluster covers any context, its CTAs taking more chunks each, so
+    // layers that may attend to more than 2048 positions keep the wider grid of independent splits.  (Clusters of 16 were measured
+    // slower: they start later, and so does every kernel behind them.)  ADAM_B200_ATTN_CLUSTER=0 turns the path off, =16 allows
+    // clusters of 16.
     static const int cluster_env = getenv("ADAM_B200_ATTN_CLUSTER") ? atoi(getenv("ADAM_B200_ATTN_CLUSTER")) : 8;
     static const uint32_t cluster_pairs = getenv("ADAM_B200_ATTN_CLUSTER_WORK") ? (uint32_t)atoi(getenv("ADAM_B200_ATTN_CLUSTER_WORK")) : 64u;
     if (cluster_env != 0 && s.pairs <= cluster_pairs && (s.pairs <= 32u || s.pairs >= 56u) && reach <= 2048u)
         s.cluster = s.pairs > 32u ? 2u : s.pairs > 16u ? 4u : cluster_env == 16 ? std::min(most, 16u) : 8u;
     // Chunks in flight per CTA: one per warp; up to two in a cluster of splits, where a context just beyond 8 chunks per CTA (a window
-    // of 512) would have a warp wait for memory a second time: as many as fit beside the queries and, in the first CTA, the splits' partial
-    // results.  (Elsewhere CTAs without positions would hold that much, too.)
+    // of 512) would have a warp wait for memory a second time: as many as fit beside the queries and, in the first CTA, the splits'
+    // partial results.  (Elsewhere CTAs without positions would hold that much, too.)
     const size_t slot = (size_t)2 * ATTN_CP * head_dim * kv_bytes, rows = ((size_t)s.hpc + 2) * head_dim * 4, merge = (size_t)s.cluster * s.hpc * (head_dim + 4) * 4;
     s.smem = 8 * slot + rows;
     if (s.cluster) {

@@ -22,8 +22,7 @@
 // The tensor pipe stays almost idle: the kernel is a stream over the weight bytes.
 //
 // Q4_K blocks go through the same MMA; their tile carries the 6-bit scale and min as bytes
-// and the superblock's (d, dmin) per row, the block scale is d*sc and the offset term
-// -(dmin*m)*sum(x) replaces -8*d*sum(x).
+// and the superblock's (d, dmin) per row; the block scale is d*sc, the offset term -(dmin*m)*sum(x).
 //
 // Batch rows 2i and 2i+1 use MMA i of a block (NI = 1 or 2 MMAs per block, four rows per
 // group); a call with more rows runs its groups as the fast grid dimension of one launch.

@@ -6,7 +6,8 @@ namespace ab {
 typedef void (*RingKernel)(const GemvArgs, const uint8_t*, const uint8_t*, float);
 // Row groups per CTA at most: beyond, the staging that this kernel saves is less than its barrier per row group costs.  us by k_gemv_mma
 // and here, cold, Q4_0 / Q4_K: 12000 x 5376 (5.1 per CTA) 14.3 and 11.4 / 16.8 and 14.8; 16000 x 5376 (6.8) 15.1 and 13.5 / 17.7
-// and 17.3; 21504 x 5376 (9.1) 18.5 and 16.8 / 21.8 and 22.9; 32768 x 5376 (13.8) 22.7 and 23.0 / 27.9 and 31.0.
+// and 17.3; 21504 x 5376 (9.1) 18.5 and 16.8 / 21.8 and 22.9; 32768 x 5376 (13.8) 22.7 and 23.0 / 27.9 and 31.0.  One line for both
+// types, where Q4_K turns; Q4_0 turns between 9 and 14.
 constexpr int RING_SETS = 7;
 constexpr int RING_SMEM_LIMIT = 220 * 1024;
 
@@ -20,8 +21,8 @@ static RingKernel pick(bool pair, bool chain, int nv, int nst) {
 }
 
 struct RingShape { RingKernel k; size_t smem; };
-// Rows of at least two tile pairs per slice (a set of sums costs a barrier), at most 128 values per lane (32 where the norm chain holds four vectors), beside which
-// the rings fit.
+// Rows of at least two tile pairs per slice (a set of sums costs a barrier), at most twelve float4 per lane (four where the norm chain
+// holds four vectors: such rows come up to K = 6144, what gemv_mma_supports takes), beside which the rings fit.
 static bool ring_shape(int wt, const GemvArgs& a, RingShape* out) {
     if (a.N <= 0 || a.K <= 0 || a.B != 1 || a.N % 16 || a.K % 64 || a.epi == EPI_ARGMAX) return false;
     if (wt != WT_Q4_0 && (wt != WT_Q4_K || a.K % 256)) return false;

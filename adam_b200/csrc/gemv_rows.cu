@@ -5,8 +5,8 @@ namespace ab {
 
 typedef void (*RowsKernel)(const GemvArgs, const uint8_t*, const uint8_t*, int, float);
 struct RowsShape { RowsKernel k; int ks, rgs; size_t smem; };
-// 1B shape, ms per step with k_gemv_mma (from five rows on the few-row GEMM) and with this kernel: 2 rows 0.727 and 0.503, 3 0.836 and
-// 0.637, 4 0.906 and 0.750; 5 1.051 and 0.960, 6 1.029 and 0.974, 8 1.023 and 1.051: there the few-row GEMM keeps its calls.
+// 1B shape, ms per step with k_gemv_mma and with this kernel: 2 rows 0.730 and 0.502, 3 0.838 and 0.643, 4 0.901 and 0.694.  Instances
+// for eight rows took 0.960 at 5 rows, 0.974 at 6 and 1.051 at 8, the few-row GEMM takes 0.927, 0.934 and 0.960: it keeps those calls.
 constexpr int ROWS_MAX = 4;
 constexpr int ROWS_SMEM_LIMIT = 220 * 1024;
 

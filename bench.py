@@ -202,6 +202,15 @@ def _gemv_weights(gpu, A, t, N, K, copies, tile):
     return rng
 
 
+STEP_KERNELS = {"row": "k_gemv_row", "ring": "k_gemv_ring", "rows": "k_gemv_rows", "mma": "k_gemv_mma", "blocks": "k_gemv", "attn_splits": "k_attention (independent splits)",
+                **{f"attn_cluster_{n}": f"k_attention (clusters of {n})" for n in (2, 4, 8, 16)}}
+
+
+def _ran(gpu, before):
+    """Names of the step's kernels that were launched since, with their counts."""
+    return {STEP_KERNELS[k]: int(n - before[k]) for k, n in gpu.step_kernel_counts().items() if n > before[k]}
+
+
 def gemv_shape(gpu, A, t, N, K, B=1, target_bytes=600e6, reps=5, tile=True):
     """Cold-HBM bandwidth of y = W x for one shape: a CUDA graph whose launches walk over enough distinct
     copies of W to exceed L2, timed with CUDA events on the library stream (best of ``reps``); plus the warm
@@ -215,9 +224,10 @@ def gemv_shape(gpu, A, t, N, K, B=1, target_bytes=600e6, reps=5, tile=True):
     a_h = gpu.upload_dev(np.array([0], np.uint32))[0]
     c_h = gpu.upload_dev(np.array([B * K], np.uint32))[0]
     bhs = [gpu.upload_dev(np.array([c * N * K], np.uint32))[0] for c in range(copies)]
-    before = gpu.gemm_counts()
+    before, before_step = gpu.gemm_counts(), gpu.step_kernel_counts()
     gpu.map_matmul_t_xq4_dev(0, 1, a_h, bhs[0], c_h, B, K, N)       # eager once: workspaces are allocated outside the capture
     ran = [k for k, n in gpu.gemm_counts().items() if n > before[k]]
+    gemvs = ", ".join(_ran(gpu, before_step))
     gpu.capture_begin()
     for c in range(copies):
         gpu.map_matmul_t_xq4_dev(0, 1, a_h, bhs[c], c_h, B, K, N)
@@ -237,7 +247,7 @@ def gemv_shape(gpu, A, t, N, K, B=1, target_bytes=600e6, reps=5, tile=True):
     gpu.batch_begin(); gpu.timer_begin(); gpu.graph_launch(gid2, 1); ms2 = gpu.timer_end(); gpu.batch_end()
     peak, _ = measured_peaks()
     kernel = ("mma.sync GEMM" if "few" in ran else "tcgen05 GEMM" if ran else "CUDA-core GEMV (planes)" if t in (8, 6) else
-              "tensor-core GEMV (tiled)" if tile else "CUDA-core GEMV")
+              "CUDA-core GEMV" if gemvs == "k_gemv" else f"tensor-core GEMV ({gemvs})")
     out = dict(type=_BLOCK_NAME[t], kernel=kernel,
                N=N, K=K, B=B, copies=copies, bytes_per_launch=int(alg), us_per_launch=round(best * 1e3 / copies, 3), GBs=round(gbs, 1),
                frac_of_measured=round(gbs / peak, 3), frac_of_8TBs=round(gbs / 8000, 3), warm_us_per_launch=round(ms2 * 1e3 / 20, 3))
@@ -585,6 +595,12 @@ def main():
     e2e_tps = st["n_gen"] / st["total_s"]
     same_ids = [int(t) for t in tokens_kernel] == out[warmup:warmup + steps]
 
+    # ---- what a step of the chain of kernels launches --------------------------------------------------
+    eng.begin([prompt[:2]], [4])
+    before = gpu.step_kernel_counts()
+    eng.step(1, lm_head=True, direct=True, chain=True)
+    step_kernels = ", ".join(f"{n} {k}" for k, n in _ran(gpu, before).items())
+
     # ---- dominant kernel: the dequant GEMV on the LM-head shape, alone on the stream --------
     hbm_peak, peak_kind = measured_peaks()
     m_embd = eng._mat_loc["token_embd.weight"]
@@ -594,10 +610,12 @@ def main():
     a_h = gpu.upload_dev(np.array([0], np.uint32))[0]; b_h = gpu.upload_dev(np.array([m_embd[1]], np.uint32))[0]
     d_h = gpu.upload_dev(np.array([K + 8], np.uint32))[0]; t_h = gpu.upload_dev(np.zeros(4, np.uint32))[0]
     reps = 20
+    before = gpu.step_kernel_counts()
     gpu.capture_begin()
     for _ in range(reps):
         gpu.map_matvec_argmax_t_xq4_dev(200, m_embd[0], a_h, b_h, t_h, t_h, d_h, K, N, 256)
     gid = gpu.capture_end()
+    head_kernel = ", ".join(_ran(gpu, before))
     gpu.graph_launch(gid, 2)
     best = 1e30
     for _ in range(5):
@@ -661,14 +679,14 @@ def main():
             "roofline": {"bound": "hbm", "achieved": token_bytes / (ms / steps * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                          "frac": token_bytes / (ms / steps * 1e-3) / 1e9 / hbm_peak, "traffic": TOKEN_DRAM_TRAFFIC if token_kernel else CHAIN_DRAM_TRAFFIC,
                          "kernel": ("k_token<Q4_0, fp16 KV, head 256> (one launch per token: every layer, LM head, arg-max)" if token_kernel
-                                    else "all %d kernels of a token step together (CUDA graph: 105 k_gemv_mma, 26 k_attention, embed, advance); "
-                                         "the largest single kernel is under lm_head_gemv" % (launches // max(1, steps))),
+                                    else "all %d kernels of a token step together (CUDA graph: %s, embed, advance); "
+                                         "the largest single kernel is under lm_head_gemv" % (launches // max(1, steps), step_kernels)),
                          "bytes_per_step": token_bytes, "us_per_step": ms / steps * 1e3,
                          "launches_in_timed_region": int(launches), "peak_kind": peak_kind,
                          "frac_of_8TBs": token_bytes / (ms / steps * 1e-3) / 1e9 / 8000.0,
                          "note": "latency-bound: 26 layers x 5 dependent kernels (or hand-overs between SMs inside the single launch); the bytes stream at this rate only on average"},
             "lm_head_gemv": {"bound": "hbm", "achieved": gemv_gbs, "peak": hbm_peak, "unit": "GB/s", "frac": gemv_gbs / hbm_peak,
-                             "traffic": LMHEAD_DRAM_TRAFFIC, "kernel": "k_gemv_mma<4,false> (LM head %dx%d Q4_0 + arg-max, tensor-core path), alone on the stream" % (N, K),
+                             "traffic": LMHEAD_DRAM_TRAFFIC, "kernel": "%s (LM head %dx%d Q4_0 + arg-max, tensor-core path), alone on the stream" % (head_kernel, N, K),
                              "bytes_per_launch": gemv_bytes, "us_per_launch": best / reps * 1e3, "frac_of_8TBs": gemv_gbs / 8000.0},
             "step_hbm": {"bytes_per_step": step_bytes, "achieved_GBs": step_bytes / (ms / steps * 1e-3) / 1e9,
                          "frac": step_bytes / (ms / steps * 1e-3) / 1e9 / hbm_peak},
